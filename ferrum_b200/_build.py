@@ -4,13 +4,16 @@
     every ``.cu`` / ``.cpp`` under ``csrc/`` except ``csrc/host`` — the sm_100a
     kernels and the CUDA runtime wrappers, compiled with
     ``nvcc -gencode arch=compute_100a,code=sm_100a`` (cross-compiles without a GPU).
+``lib/_native.so``
+    ``csrc/native/*.cpp`` — the host path of the differentiable ops (autograd nodes, launch code) as a Python
+    module against torch's C++ interface; it calls the kernel library's C ABI.
 ``lib/libferrum_b200_host.so``
     ``csrc/host/*.cpp`` — checkpoint serializer, samplers, bucket planner and the
     plain-C++ CPU reference loops; no CUDA dependency, so it loads anywhere.
 
-Both expose a C ABI that the Python layer reaches through :mod:`ctypes`, which
-keeps the build free of framework headers (a full rebuild takes well under a
-minute) and lets non-Python callers link the same entry points.
+The first and the last expose a C ABI, free of framework headers, which lets
+non-Python callers link the same entry points; Python reaches both through
+:mod:`ctypes` as well.
 
 Objects are cached by a hash of the source, the headers under ``csrc/`` and the
 flags, so ``build()`` is incremental.  Run ``python -m ferrum_b200._build``.
@@ -33,6 +36,7 @@ CUDA_LIB = LIB / "libferrum_b200_cuda.so"
 OBJ_BOUNDS = ROOT / "_obj_bounds"
 CUDA_LIB_BOUNDS = LIB / "libferrum_b200_cuda_bounds.so"  # debug build with device-side index checks
 HOST_LIB = LIB / "libferrum_b200_host.so"
+NATIVE_LIB = LIB / "_native.so"  # Python module: host path of the ops (csrc/native)
 
 CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.environ.get("NVCC") or shutil.which("nvcc") or f"{CUDA_HOME}/bin/nvcc"
@@ -49,15 +53,33 @@ CXX_FLAGS = ["-O3", "-std=c++17", "-fPIC", "-Wall", "-Wno-unused-function"]
 def _headers_digest() -> str:
     h = hashlib.sha256()
     for p in sorted(CSRC.rglob("*")):
-        if p.suffix in (".h", ".cuh", ".hpp"):
+        if p.suffix in (".h", ".cuh", ".hpp") and p.parent.name != "native":
             h.update(p.name.encode())
             h.update(p.read_bytes())
     return h.hexdigest()
 
 
+def _torch_flags() -> tuple[list[str], list[str]]:
+    """(compile, link) flags of the sources under ``csrc/native``."""
+    import sysconfig
+
+    import torch
+
+    root = Path(torch.__file__).resolve().parent
+    inc = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include"]
+    cflags = [*(f"-I{p}" for p in inc), f"-I{sysconfig.get_paths()['include']}",
+              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DTORCH_EXTENSION_NAME=_native",
+              "-fvisibility=hidden", "-Wno-deprecated-declarations"]
+    lflags = [f"-L{root / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+    return cflags, lflags
+
+
 def _compile_one(src: Path, flags_key: str, hdr: str, verbose: bool, bounds: bool = False) -> Path:
     rel = src.relative_to(CSRC)
     extra = ["-DFERRUM_BOUNDS=1"] if bounds else []
+    if rel.parts[0] == "native":
+        extra = _torch_flags()[0]
+        hdr += (CSRC / "native" / "native.h").read_text()
     flags_key += " ".join(extra)
     obj = (OBJ_BOUNDS if bounds else OBJ) / (str(rel).replace("/", "__") + ".o")
     stamp = obj.with_suffix(".hash")
@@ -96,8 +118,19 @@ def _link(objs: list[Path], out: Path, cuda: bool) -> None:
 
 def sources() -> tuple[list[Path], list[Path]]:
     host = sorted(p for p in (CSRC / "host").glob("*.cpp") if p.name != "selftest.cpp")
-    cuda = sorted(p for p in CSRC.rglob("*") if p.suffix in (".cu", ".cpp") and (CSRC / "host") not in p.parents)
+    cuda = sorted(p for p in CSRC.rglob("*") if p.suffix in (".cu", ".cpp") and (CSRC / "host") not in p.parents
+                  and (CSRC / "native") not in p.parents)
     return cuda, host
+
+
+def _link_native(objs: list[Path]) -> None:
+    tmp = NATIVE_LIB.with_suffix(".so.tmp")
+    # the fb_* symbols stay undefined: the kernel library (normal or index-checking) is loaded globally first
+    r = subprocess.run([CXX, "-shared", "-o", str(tmp), *map(str, objs), *_torch_flags()[1]], capture_output=True,
+                       text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"link failed: {NATIVE_LIB}\n{r.stdout}\n{r.stderr}")
+    os.replace(tmp, NATIVE_LIB)
 
 
 def build_bounds(verbose: bool = True, jobs: int | None = None) -> None:
@@ -118,7 +151,7 @@ def build_bounds(verbose: bool = True, jobs: int | None = None) -> None:
 
 
 def build(verbose: bool = True, jobs: int | None = None) -> None:
-    """Compile every native source for sm_100a and link the two libraries."""
+    """Compile every native source for sm_100a and link the libraries."""
     OBJ.mkdir(exist_ok=True)
     cuda_src, host_src = sources()
     hdr = _headers_digest()
@@ -129,7 +162,10 @@ def build(verbose: bool = True, jobs: int | None = None) -> None:
         cuda_futs = [ex.submit(_compile_one, s, nv_key if s.suffix == ".cu" else cx_key, hdr, verbose)
                      for s in cuda_src]
         host_futs = [ex.submit(_compile_one, s, cx_key, hdr, verbose) for s in host_src]
+        native_futs = [ex.submit(_compile_one, s, cx_key, hdr, verbose)
+                       for s in sorted((CSRC / "native").glob("*.cpp"))]
         cuda_objs = [f.result() for f in cuda_futs]
+        native_objs = [f.result() for f in native_futs]
         host_objs = [f.result() for f in host_futs]
 
     def newer(objs: list[Path], lib: Path) -> bool:
@@ -139,6 +175,10 @@ def build(verbose: bool = True, jobs: int | None = None) -> None:
         _link(cuda_objs, CUDA_LIB, cuda=True)
         if verbose:
             print(f"[ferrum_b200 build] linked {CUDA_LIB.name}")
+    if newer(native_objs, NATIVE_LIB):
+        _link_native(native_objs)
+        if verbose:
+            print(f"[ferrum_b200 build] linked {NATIVE_LIB.name}")
     if host_objs and newer(host_objs, HOST_LIB):
         _link(host_objs, HOST_LIB, cuda=False)
         if verbose:

@@ -18,6 +18,7 @@ from . import _build
 _lock = threading.Lock()
 _cuda = None
 _host = None
+_native = None
 
 
 class NativeLibraryError(RuntimeError):
@@ -226,8 +227,8 @@ class _CountingLib:
 
 
 def launch_count() -> int:
-    """Number of kernel-launcher calls made through this module so far."""
-    return _launches
+    """Number of kernel-launcher calls made so far, from Python and from the native host path."""
+    return _launches + (_native.launch_count() if _native is not None else 0)
 
 
 def cuda():
@@ -244,6 +245,30 @@ def cuda():
                 _bind(lib, _lib_dist.SIGS)
                 _cuda = _CountingLib(lib)
     return _cuda
+
+
+def native():
+    """The host path of the differentiable ops (``lib/_native.so``); its kernels are those of :func:`cuda`."""
+    global _native
+    if _native is None:
+        cuda()
+        with _lock:
+            if _native is None:
+                import importlib.machinery
+                import importlib.util
+
+                import torch  # noqa: F401 - the module links against torch's libraries
+
+                from . import config
+
+                _ensure(_build.NATIVE_LIB)
+                loader = importlib.machinery.ExtensionFileLoader("_native", str(_build.NATIVE_LIB))
+                mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_native", loader))
+                loader.exec_module(mod)
+                mod.set_use_2cta(os.environ.get("FERRUM_GEMM_2CTA", "1") == "1")
+                mod.set_tf32(config.matmul_precision() == "tf32")
+                _native = mod
+    return _native
 
 
 def host():

@@ -21,6 +21,8 @@ import threading
 
 import torch
 
+from . import _lib
+
 _state = threading.local()
 _default_precision = os.environ.get("FERRUM_MATMUL_PRECISION", "fp32").lower()
 
@@ -33,6 +35,8 @@ def matmul_precision(value: str | None = None) -> str:
         if value not in ("fp32", "tf32", "bf16"):
             raise ValueError("matmul precision must be 'fp32', 'tf32' or 'bf16'")
         _default_precision = value
+        if _lib._native is not None:  # backward passes read the setting in native code
+            _lib._native.set_tf32(value == "tf32")
     return _default_precision
 
 

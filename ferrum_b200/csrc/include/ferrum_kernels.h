@@ -139,6 +139,20 @@ int fb_softmax_bwd(const void* dy, const void* y, void* dx, long long rows, int 
 // dlogits != NULL the gradient (softmax - onehot) * grad_scale in `dlogits_dtype`.
 int fb_ce_fwd_bwd(const void* logits, const long long* labels, float* row_loss, void* dlogits, long long rows,
                   int cols, float grad_scale, int dtype, int dlogits_dtype, cudaStream_t stream);
+// Mean losses (kernels/mean_loss.cu): the scalar scale * sum lands in `loss`; workspace = fb_mean_loss_workspace(n)
+// floats.  row_stats (optional) [rows][2]: row maximum and sum of exponentials, what the backward pass reads.
+// gout: the incoming scalar gradient, read on the device.
+long long fb_mean_loss_workspace(long long n);
+int fb_ce_fwd(const void* logits, const long long* labels, float* row_stats, float* loss, float* workspace,
+              long long rows, int cols, float scale, int dtype, cudaStream_t stream);
+int fb_ce_bwd(const void* logits, const long long* labels, const float* row_stats, const float* gout, void* dlogits,
+              long long rows, int cols, float scale, int dtype, cudaStream_t stream);
+int fb_nll_fwd(const void* log_probs, const long long* target, float* loss, float* workspace, long long rows, int cols,
+               float scale, int dtype, cudaStream_t stream);
+int fb_nll_bwd(const long long* target, const float* gout, void* dlog_probs, long long rows, int cols, float scale,
+               int dtype, cudaStream_t stream);
+int fb_loss_mean_fwd(const float* pred, const float* target, float* loss, float* workspace, long long n, int kind,
+                     float scale, cudaStream_t stream);
 // Elementwise losses: sum of per-element loss into out[0] (pre-zeroed), scaled by `scale`.
 int fb_loss_fwd(const float* pred, const float* target, float* out, long long n, int kind, float scale,
                 cudaStream_t stream);

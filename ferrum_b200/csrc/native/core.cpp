@@ -1,0 +1,213 @@
+// Launch accounting, the GEMM dispatch and the module itself.
+#include "native.h"
+
+#include <c10/cuda/CUDAFunctions.h>
+#include <mutex>
+#include <vector>
+
+extern "C" {
+int32_t* fb_rt_status_ptr(void);
+const char* fb_rt_error_string(int);
+void* fb_rt_event_create(int timing);
+int fb_rt_event_record(void* event, void* stream);
+int fb_rt_event_synchronize(void* event);
+int fb_rt_event_destroy(void* event);
+float fb_rt_event_elapsed_ms(void* start, void* stop);
+}
+
+namespace fbn {
+
+std::atomic<ll> g_launches{0};
+std::atomic<bool> g_profiling{false};
+std::atomic<bool> g_tf32{false}, g_use_2cta{true};
+std::atomic<int> g_max_ctas{0};
+
+// ------------------------------------------------------------------------------------------------ launches
+struct Record {
+  const char* name;
+  void *e0, *e1;
+};
+static std::mutex g_prof_mutex;
+static std::vector<Record> g_records;
+static thread_local Record t_record;
+
+void profile_begin(const char* name) {
+  t_record.name = name;
+  t_record.e0 = fb_rt_event_create(1);
+  t_record.e1 = fb_rt_event_create(1);
+  fb_rt_event_record(t_record.e0, cur_stream());
+}
+void profile_end() {
+  fb_rt_event_record(t_record.e1, cur_stream());
+  std::lock_guard<std::mutex> lock(g_prof_mutex);
+  g_records.push_back(t_record);
+}
+
+void launch_failed(const char* name, int rc) {
+  TORCH_CHECK(rc < 0, name, ": CUDA error ", rc, ": ", fb_rt_error_string(rc));
+  TORCH_CHECK_VALUE(false, name, ": invalid argument (code ", rc, ")");
+}
+
+int32_t* status() {
+  static std::atomic<int32_t*> ptrs[64];
+  const int dev = c10::cuda::current_device();
+  std::atomic<int32_t*>& slot = ptrs[dev & 63];
+  int32_t* p = slot.load(std::memory_order_acquire);
+  if (p == nullptr) {
+    p = fb_rt_status_ptr();
+    TORCH_CHECK(p != nullptr, "could not allocate the device status block");
+    fb_layernorm_set_status(p);  // kernels without a status argument report here (one device per process)
+    slot.store(p, std::memory_order_release);
+  }
+  return p;
+}
+
+Tensor cast(const Tensor& t, at::ScalarType st) {
+  if (t.scalar_type() == st) return t;
+  if (!((is_f32(t) && st == at::kBFloat16) || (is_bf16(t) && st == at::kFloat))) return t.to(st);
+  Tensor x = contig(t), y = empty(x.sizes(), x, st);
+  FB_CALL(fb_cast, x.data_ptr(), y.data_ptr(), x.numel(), dt(x), dt(y), cur_stream());
+  return y;
+}
+
+// ---------------------------------------------------------------------------------------------------- GEMM
+bool tma_ok(const Op& a) {
+  const ll unit = a.bf16 ? 8 : 4;  // elements per 16 bytes
+  if (reinterpret_cast<uintptr_t>(a.p) % 16) return false;
+  if (a.s_k == 1) return a.s_row % unit == 0 && a.s_row >= a.k;
+  if (a.s_row == 1) return a.s_k % unit == 0 && a.s_k >= a.rows;
+  return false;
+}
+
+void gemm(const Op& a, const Op& b, const float* bias, int act, void* out, ll ldc, bool out_bf16, bool accumulate,
+          void* act_grad, const Tensor* like, bool tf32) {
+  const int M = static_cast<int>(a.rows), N = static_cast<int>(b.rows), K = static_cast<int>(a.k);
+  TORCH_CHECK(a.k == b.k, "inner dimensions differ: [", a.rows, ", ", a.k, "] x [", b.rows, ", ", b.k, "]^T");
+  if (M == 0 || N == 0) return;
+  const bool ok = tma_ok(a) && tma_ok(b);
+  const int a_mn = a.s_k == 1 ? 0 : 1, b_mn = b.s_k == 1 ? 0 : 1;
+  const ll lda = a_mn ? a.s_k : a.s_row, ldb = b_mn ? b.s_k : b.s_row;
+  if (a.bf16 && ok) {
+    int rc = -3;
+    if (g_use_2cta.load(std::memory_order_relaxed) && M >= 512 && N >= 128)
+      launch("fb_gemm_bf16", [&] {
+        rc = fb_gemm_bf16_2cta(a.p, b.p, out, act_grad, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_bf16, act,
+                               accumulate, g_max_ctas, status(), cur_stream());
+        return rc == -3 ? 0 : rc;  // -3: CTA pairs cannot be scheduled on this device
+      });
+    if (rc == -3)
+      FB_CALL(fb_gemm_bf16, a.p, b.p, out, act_grad, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_bf16, act,
+              accumulate, g_max_ctas, status(), cur_stream());
+    return;
+  }
+  TORCH_CHECK(act_grad == nullptr, "activation derivatives need operands that a TMA map describes");
+  if (!a.bf16 && tf32 && ok) {
+    int rc = -3;
+    if (M >= 512 && N >= 256)
+      launch("fb_gemm_tf32", [&] {
+        rc = fb_gemm_tf32_2cta(static_cast<const float*>(a.p), static_cast<const float*>(b.p), static_cast<float*>(out),
+                               bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, act, accumulate, g_max_ctas, status(), cur_stream());
+        return rc == -3 ? 0 : rc;
+      });
+    if (rc == -3)
+      FB_CALL(fb_gemm_tf32, static_cast<const float*>(a.p), static_cast<const float*>(b.p), static_cast<float*>(out),
+              bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, act, accumulate, g_max_ctas, status(), cur_stream());
+    return;
+  }
+  if (!a.bf16 && !out_bf16) {
+    FB_CALL(fb_gemm_f32_simt, static_cast<const float*>(a.p), static_cast<const float*>(b.p), static_cast<float*>(out),
+            bias, M, N, K, a.s_row, a.s_k, b.s_k, b.s_row, ldc, act, accumulate, 1, 0, 0, 0, cur_stream());
+    return;
+  }
+  // bf16 operands whose row pitch is not a multiple of 16 bytes: exact fp32 kernel on fp32 copies
+  TORCH_CHECK(like != nullptr, "gemm: missing tensor options");
+  auto wide = [&](const Op& o) {
+    Tensor v = at::from_blob(const_cast<void*>(o.p), {o.rows, o.k}, {o.s_row, o.s_k},
+                             like->options().dtype(o.bf16 ? at::kBFloat16 : at::kFloat));
+    return f32c(v);
+  };
+  Tensor af = wide(a), bf = wide(b);
+  if (out_bf16) {
+    Tensor res = empty({M, N}, *like, at::kFloat);
+    FB_CALL(fb_gemm_f32_simt, af.data_ptr<float>(), bf.data_ptr<float>(), res.data_ptr<float>(), bias, M, N, K, K, 1, 1,
+            K, N, act, 0, 1, 0, 0, 0, cur_stream());
+    Tensor o = at::from_blob(out, {M, N}, {ldc, 1}, like->options().dtype(at::kBFloat16));
+    if (ldc == N)
+      FB_CALL(fb_cast, res.data_ptr(), out, res.numel(), FB_DT_F32, FB_DT_BF16, cur_stream());
+    else
+      o.copy_(res);
+  } else {
+    FB_CALL(fb_gemm_f32_simt, af.data_ptr<float>(), bf.data_ptr<float>(), static_cast<float*>(out), bias, M, N, K, K, 1,
+            1, K, ldc, act, accumulate, 1, 0, 0, 0, cur_stream());
+  }
+}
+
+// --------------------------------------------------------------------------------------------------- sinks
+Sink::~Sink() {
+  if (sink != nullptr && Py_IsInitialized()) {
+    py::gil_scoped_acquire gil;
+    Py_XDECREF(sink);
+    Py_XDECREF(param);
+  }
+}
+std::shared_ptr<Sink> make_sink(py::handle sink, py::handle param) {
+  if (sink.is_none()) return nullptr;
+  auto s = std::make_shared<Sink>();
+  s->sink = sink.inc_ref().ptr();
+  s->param = param.inc_ref().ptr();
+  return s;
+}
+void wgrad_to_sink(Sink& s, const Tensor& g2, const Tensor& x2) {
+  Tensor buf;
+  bool acc = false;
+  {
+    py::gil_scoped_acquire gil;
+    py::handle sink(s.sink), param(s.param);
+    if (is_bf16(g2) && is_bf16(x2) && py::hasattr(sink, "try_push") &&
+        sink.attr("try_push")(param, g2.t(), x2.t()).cast<bool>())
+      return;
+    py::tuple r = sink.attr("acquire")(param);
+    buf = r[0].cast<Tensor>();
+    acc = r[1].cast<bool>();
+  }
+  gemm(op2d(g2).t(), op2d(x2).t(), nullptr, 0, buf.data_ptr(), buf.stride(0), false, acc, nullptr, &g2,
+       g_tf32.load(std::memory_order_relaxed));
+}
+void sink_ready(Sink& s) {
+  py::gil_scoped_acquire gil;
+  py::handle(s.sink).attr("ready")(py::handle(s.param));
+}
+
+}  // namespace fbn
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  using namespace fbn;
+  m.def("launch_count", [] { return g_launches.load(); });
+  m.def("set_tf32", [](bool f) { g_tf32 = f; });
+  m.def("set_use_2cta", [](bool f) { g_use_2cta = f; });
+  m.def("set_max_ctas", [](int n) { g_max_ctas = n; });
+  m.def("profile_start", [] {
+    std::lock_guard<std::mutex> lock(g_prof_mutex);
+    for (auto& r : g_records) {
+      fb_rt_event_destroy(r.e0);
+      fb_rt_event_destroy(r.e1);
+    }
+    g_records.clear();
+    g_profiling = true;
+  });
+  m.def("profile_stop", [] { g_profiling = false; });
+  m.def("profile_records", [] {  // (launcher, milliseconds) of every call since profile_start; synchronizes
+    std::vector<std::pair<std::string, float>> out;
+    std::lock_guard<std::mutex> lock(g_prof_mutex);
+    for (auto& r : g_records) {
+      fb_rt_event_synchronize(r.e1);
+      out.emplace_back(r.name, fb_rt_event_elapsed_ms(r.e0, r.e1));
+    }
+    return out;
+  });
+  m.def("cast", [](const Tensor& t, const Tensor& like) { return cast(t, like.scalar_type()); });
+  bind_linear(m);
+  bind_elementwise(m);
+  bind_layers(m);
+  bind_optim(m);
+}

@@ -1,0 +1,285 @@
+// Linear layers: act(x W^T + b), LayerNorm(act(x W^T + b)) as one node, LayerNorm.
+#include "native.h"
+
+extern "C" int fb_rt_memset(void* p, int value, unsigned long long bytes, cudaStream_t stream);
+
+namespace fbn {
+namespace {
+
+constexpr int kNone = FB_ACT_NONE;
+
+// The operands of a Linear in the precision of the call: bf16 (cast of x, cached or cast copy of W) or fp32.
+struct Operands {
+  Tensor x2, w;
+  Tensor saved;  // what the backward pass keeps of x: x itself (its version is checked) or the converted copy
+};
+Operands operands(const Tensor& x, const Tensor& weight, const Tensor& w_low, bool low) {
+  TORCH_CHECK_VALUE(weight.is_cuda(), "the weight is not on the input's device");
+  Operands o;
+  Tensor x2 = as2d(x);
+  if (low) {
+    o.x2 = is_bf16(x2) ? x2 : cast(x2, at::kBFloat16);
+    if (!tma_ok(op2d(o.x2))) o.x2 = contig(o.x2);
+    o.w = w_low.defined() ? w_low : cast(weight, at::kBFloat16);
+  } else {
+    o.x2 = is_f32(x2) ? x2 : cast(x2, at::kFloat);
+    o.w = cast(weight, at::kFloat);
+  }
+  o.saved = o.x2.is_alias_of(x) ? x : o.x2;
+  return o;
+}
+
+std::vector<int64_t> out_sizes(const Tensor& x, int64_t last) {
+  std::vector<int64_t> s(x.sizes().begin(), x.sizes().end());
+  s.back() = last;
+  return s;
+}
+
+// Gradient of a Linear's input, weight and bias from g2 [M, N], in the precision of the forward pass.
+void linear_grads(const Tensor& g2, const Tensor& x2, const Tensor& w, bool low, at::ScalarType x_dtype,
+                  at::IntArrayRef x_sizes, const std::shared_ptr<Sink>& sink, bool need_x, bool need_w, bool need_b,
+                  variable_list& out) {
+  const bool tf32 = !low && g_tf32.load(std::memory_order_relaxed);
+  const int64_t N = w.size(0), K = w.size(1);
+  if (need_x) {  // before the weight gradient: the weight may be overwritten once its bucket is reduced
+    Tensor gx = empty(x_sizes, g2, low ? at::kBFloat16 : at::kFloat);
+    gemm(op2d(g2), op2d(w).t(), nullptr, kNone, gx.data_ptr(), K, low, false, nullptr, &g2, tf32);
+    out[0] = cast(gx, x_dtype);
+  }
+  if (need_w) {
+    if (sink) {
+      wgrad_to_sink(*sink, g2, x2);
+    } else {
+      Tensor gw = empty({N, K}, g2, at::kFloat);
+      gemm(op2d(g2).t(), op2d(x2).t(), nullptr, kNone, gw.data_ptr(), K, false, false, nullptr, &g2, tf32);
+      out[1] = gw;
+    }
+  }
+  if (need_b) {
+    Tensor gb = empty({N}, g2, at::kFloat);
+    FB_CALL(fb_colsum, g2.data_ptr(), gb.data_ptr<float>(), g2.size(0), N, dt(g2), 0, cur_stream());
+    out[2] = gb;
+  }
+  if (need_w && sink) sink_ready(*sink);
+}
+
+struct LinearNode : Node {
+  SavedVariable x_, w_, y_;
+  bool low = false, has_bias = false;
+  int act = kNone;
+  at::ScalarType x_dtype = at::kFloat;
+  std::vector<int64_t> x_sizes;
+  std::shared_ptr<Sink> sink;
+  std::string name() const override { return "FerrumLinearBackward"; }
+  void release_variables() override {
+    x_.reset_data();
+    w_.reset_data();
+    y_.reset_data();
+  }
+  variable_list apply(variable_list&& grads) override {
+    NoAutograd below;
+    variable_list out(3);
+    if (!grads[0].defined()) return out;
+    Tensor x2 = as2d(x_.unpack()), w = w_.unpack();
+    Tensor g2 = contig(as2d(grads[0]));
+    g2 = low ? cast(g2, at::kBFloat16) : cast(g2, at::kFloat);
+    if (act != kNone) {  // only activations whose derivative is a function of the output are fused
+      Tensor y = as2d(y_.unpack(shared_from_this()));
+      Tensor d = empty(g2.sizes(), g2, g2.scalar_type());
+      FB_CALL(fb_unary_bwd, g2.data_ptr(), y.data_ptr(), d.data_ptr(), g2.numel(), act, 0.f, 0.f, dt(g2), cur_stream());
+      g2 = d;
+    }
+    linear_grads(g2, x2, w, low, x_dtype, x_sizes, sink, task_should_compute_output(0), task_should_compute_output(1),
+                 has_bias && task_should_compute_output(2), out);
+    return out;
+  }
+};
+
+Tensor linear(const Tensor& x, const Tensor& weight, const c10::optional<Tensor>& bias_, int act, bool low, bool tf32,
+              const c10::optional<Tensor>& w_low, py::object sink) {
+  NoAutograd below;
+  const Tensor bias = bias_.value_or(Tensor());
+  Operands o = operands(x, weight, w_low.value_or(Tensor()), low);
+  const int64_t N = weight.size(0);
+  Tensor y = empty(out_sizes(x, N), o.x2, low ? at::kBFloat16 : at::kFloat);
+  Tensor b = bias.defined() ? f32c(bias) : bias;
+  gemm(op2d(o.x2), op2d(o.w), fptr(b), act, y.data_ptr(), N, low, false, nullptr, &o.x2, tf32 && !low);
+  if (wants_grad({&x, &weight, &bias})) {
+    auto n = make_node<LinearNode>(x, weight, bias);
+    n->low = low;
+    n->act = act;
+    n->has_bias = bias.defined();
+    n->x_dtype = x.scalar_type();
+    n->x_sizes.assign(x.sizes().begin(), x.sizes().end());
+    n->sink = make_sink(sink, py::cast(weight));
+    n->x_ = SavedVariable(o.saved, false);
+    n->w_ = SavedVariable(o.w, false);
+    torch::autograd::set_history(y, n);
+    if (act != kNone) n->y_ = SavedVariable(y, true);
+  }
+  return y;
+}
+
+// ---------------------------------------------------------------------------------------------- LayerNorm
+struct NormStats {
+  Tensor mean, rstd;
+};
+NormStats norm_fwd(const Tensor& x2, const Tensor& gamma, const Tensor& beta, const Tensor& y, float eps, int pre) {
+  NormStats s{empty({x2.size(0)}, x2, at::kFloat), empty({x2.size(0)}, x2, at::kFloat)};
+  status();  // the wide-row kernels report bounded-wait failures to the status block
+  FB_CALL(fb_layernorm_fwd, x2.data_ptr(), fptr(gamma), fptr(beta), y.data_ptr(), s.mean.data_ptr<float>(),
+          s.rstd.data_ptr<float>(), x2.size(0), static_cast<int>(x2.size(1)), eps, pre, dt(x2), cur_stream());
+  return s;
+}
+// stats [3, cols]: d_gamma, d_beta, column sum of dx
+Tensor norm_bwd(const Tensor& gy2, const Tensor& x2, const Tensor& dact, const Tensor& gamma, const NormStats& s,
+                const Tensor& dx, int pre, bool colsum) {
+  const int64_t rows = x2.size(0), cols = x2.size(1);
+  const int nblk = fb_layernorm_bwd_blocks(rows, static_cast<int>(cols));
+  Tensor partial = empty({std::max(nblk, 1), 3, cols}, x2, at::kFloat);
+  Tensor stats = empty({3, cols}, x2, at::kFloat);
+  fb_rt_memset(stats.data_ptr(), 0, stats.numel() * 4, cur_stream());
+  FB_CALL(fb_layernorm_bwd, gy2.data_ptr(), x2.data_ptr(), ptr(dact), fptr(gamma), s.mean.data_ptr<float>(),
+          s.rstd.data_ptr<float>(), dx.data_ptr(), partial.data_ptr<float>(), stats.data_ptr<float>(), rows,
+          static_cast<int>(cols), pre, dt(x2), nblk, colsum ? 1 : 0, cur_stream());
+  return stats;
+}
+
+struct LayerNormNode : Node {
+  SavedVariable x_, g_;
+  NormStats st;
+  int pre = kNone;
+  bool has_gamma = false, has_beta = false;
+  std::string name() const override { return "FerrumLayerNormBackward"; }
+  void release_variables() override {
+    x_.reset_data();
+    g_.reset_data();
+    st = NormStats();
+  }
+  variable_list apply(variable_list&& grads) override {
+    NoAutograd below;
+    variable_list out(3);
+    if (!grads[0].defined()) return out;
+    Tensor x = contig(x_.unpack()), g = g_.unpack();
+    Tensor x2 = as2d(x), gy = contig(cast(grads[0], x.scalar_type()));
+    Tensor dx = empty(x.sizes(), x, x.scalar_type());
+    Tensor stats = norm_bwd(as2d(gy), x2, Tensor(), g, st, dx, pre, false);
+    out[0] = dx;
+    if (has_gamma) out[1] = stats[0];
+    if (has_beta) out[2] = stats[1];
+    return out;
+  }
+};
+
+Tensor layer_norm(const Tensor& x, const c10::optional<Tensor>& gamma_, const c10::optional<Tensor>& beta_, double eps,
+                  int pre) {
+  NoAutograd below;
+  const Tensor gamma = gamma_.value_or(Tensor()), beta = beta_.value_or(Tensor());
+  Tensor xc = contig(x);
+  Tensor g = gamma.defined() ? contig(gamma) : gamma, b = beta.defined() ? contig(beta) : beta;
+  Tensor y = empty(xc.sizes(), xc, xc.scalar_type());
+  NormStats st = norm_fwd(as2d(xc), g, b, as2d(y), static_cast<float>(eps), pre);
+  if (wants_grad({&x, &gamma, &beta})) {
+    auto n = make_node<LayerNormNode>(x, gamma, beta);
+    n->st = st;
+    n->pre = pre;
+    n->has_gamma = gamma.defined();
+    n->has_beta = beta.defined();
+    n->x_ = SavedVariable(xc.is_alias_of(x) ? x : xc, false);
+    if (g.defined()) n->g_ = SavedVariable(g, false);
+    torch::autograd::set_history(y, n);
+  }
+  return y;
+}
+
+// ---------------------------------------------------------------- LayerNorm(act(x W^T + b)) as one node
+// Tensor-core path: the GEMM epilogue writes act(z) and, where a backward pass follows, act'(z); the normalisation
+// reads act(z).  Backward: one streaming kernel turns dy into dz and yields d_gamma, d_beta and the bias gradient,
+// then the two products run on dz.  fp32 path: z is stored, the activation is evaluated inside the normalisation.
+struct LinearActNormNode : Node {
+  SavedVariable x_, w_, g_;
+  Tensor z, dact;
+  NormStats st;
+  bool low = false, has_bias = false;
+  int pre = kNone;
+  at::ScalarType x_dtype = at::kFloat;
+  std::vector<int64_t> x_sizes;
+  std::shared_ptr<Sink> sink;
+  std::string name() const override { return "FerrumLinearActNormBackward"; }
+  void release_variables() override {
+    x_.reset_data();
+    w_.reset_data();
+    g_.reset_data();
+    z = dact = Tensor();
+    st = NormStats();
+  }
+  variable_list apply(variable_list&& grads) override {
+    NoAutograd below;
+    variable_list out(5);
+    if (!grads[0].defined()) return out;
+    Tensor x2 = as2d(x_.unpack()), w = w_.unpack(), g = g_.unpack();
+    Tensor gy2 = contig(as2d(cast(grads[0], z.scalar_type())));
+    Tensor dz = empty(z.sizes(), z, z.scalar_type());
+    Tensor stats = norm_bwd(gy2, z, dact, g, st, dz, pre, true);
+    linear_grads(dz, x2, w, low, x_dtype, x_sizes, sink, task_should_compute_output(0), task_should_compute_output(1),
+                 false, out);
+    if (has_bias) out[2] = stats[2];
+    out[3] = stats[0];
+    out[4] = stats[1];
+    return out;
+  }
+};
+
+Tensor linear_act_norm(const Tensor& x, const Tensor& weight, const c10::optional<Tensor>& bias_, const Tensor& gamma,
+                       const Tensor& beta, double eps, int act, bool low, bool tf32,
+                       const c10::optional<Tensor>& w_low, py::object sink) {
+  NoAutograd below;
+  const Tensor bias = bias_.value_or(Tensor());
+  Operands o = operands(x, weight, w_low.value_or(Tensor()), low);
+  const int64_t N = weight.size(0), M = o.x2.size(0);
+  const bool grad = wants_grad({&x, &weight, &bias, &gamma, &beta});
+  Tensor b = bias.defined() ? f32c(bias) : bias;
+  Tensor g = contig(gamma), be = contig(beta);
+  Tensor z = empty({M, N}, o.x2, low ? at::kBFloat16 : at::kFloat), dact;
+  const bool fused = low && act != kNone && tma_ok(op2d(o.x2)) && tma_ok(op2d(o.w));
+  if (fused && grad) dact = empty({M, N}, o.x2, at::kBFloat16);
+  gemm(op2d(o.x2), op2d(o.w), fptr(b), fused ? act : kNone, z.data_ptr(), N, low, false, ptr(dact), &o.x2,
+       tf32 && !low);
+  const int pre = fused ? kNone : act;
+  Tensor y = empty(out_sizes(x, N), o.x2, z.scalar_type());
+  NormStats st = norm_fwd(z, g, be, y, static_cast<float>(eps), pre);
+  if (grad) {
+    auto n = make_node<LinearActNormNode>(x, weight, bias, gamma, beta);
+    n->low = low;
+    n->pre = pre;
+    n->has_bias = bias.defined();
+    n->x_dtype = x.scalar_type();
+    n->x_sizes.assign(x.sizes().begin(), x.sizes().end());
+    n->sink = make_sink(sink, py::cast(weight));
+    n->x_ = SavedVariable(o.saved, false);
+    n->w_ = SavedVariable(o.w, false);
+    n->g_ = SavedVariable(g, false);
+    n->z = z;
+    n->dact = dact;
+    n->st = st;
+    torch::autograd::set_history(y, n);
+  }
+  return y;
+}
+
+}  // namespace
+
+void bind_linear(py::module_& m) {
+  m.def("linear", &linear);
+  m.def("layer_norm", &layer_norm);
+  m.def("linear_act_norm", &linear_act_norm);
+  m.def("gemm_nt",  // out = act(a b^T + bias) without a graph; see ops/functional.py
+        [](const Tensor& a, const Tensor& b, const c10::optional<Tensor>& bias, int act, const Tensor& out,
+           bool accumulate, bool tf32) {
+          Tensor bb = bias.has_value() ? *bias : Tensor();
+          gemm(op2d(a), op2d(b), fptr(bb), act, out.data_ptr(), out.stride(0), is_bf16(out), accumulate, nullptr, &out,
+               tf32);
+        });
+}
+
+}  // namespace fbn

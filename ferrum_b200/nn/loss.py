@@ -47,6 +47,8 @@ def _ce_onehot(log_probs, targets):
 
 
 def _nll_index(log_probs, targets):
+    if F._native(log_probs) and log_probs.numel() > 0:
+        return F.nll_index(log_probs, targets)
     C = log_probs.shape[-1]
     lp2 = log_probs.reshape(-1, C)
     onehot = torch.zeros(lp2.shape, device=lp2.device, dtype=lp2.dtype)

@@ -15,7 +15,7 @@ from collections import OrderedDict
 
 import torch
 
-from .. import config
+from .. import _lib, config
 from ..core import DType, Device, FerrumError, IndexOutOfBounds, InvalidShape, ShapeMismatch, Tensor, _as_device
 from ..ops import functional as F
 from . import init as _init
@@ -111,23 +111,7 @@ def low_precision_weight(p: torch.nn.Parameter):
     modification of the parameter (torch in-place op, ``.data`` swap) is detected
     through the version counter / data pointer and triggers one re-cast.
     """
-    if not (p.is_cuda and p.dtype == torch.float32 and config.low_precision_active()):
-        return None
-    d = p.__dict__
-    sh = d.get("_fb_shadow")
-    key = (p._version, p.data_ptr())
-    if sh is None or sh.shape != p.shape or sh.device != p.device:
-        sh = torch.empty_like(p, dtype=torch.bfloat16)
-        d["_fb_shadow"] = sh
-        d["_fb_shadow_key"] = None
-    if d.get("_fb_shadow_key") != key:
-        from .. import _lib
-
-        src = p.detach().contiguous()
-        _lib.check(_lib.cuda().fb_cast(src.data_ptr(), sh.data_ptr(), p.numel(), F.F32, F.BF16, F._stream()),
-                   "fb_cast")
-        d["_fb_shadow_key"] = key
-    return sh
+    return _lib.native().low_weight(p) if p.is_cuda and config.low_precision_active() else None
 
 
 class Linear(Module):

@@ -2,7 +2,7 @@
 
 Every function here takes and returns plain torch tensors.  For CUDA tensors
 (fp32 / bf16) the forward and the backward both run this package's sm_100a
-kernels through ``torch.autograd.Function`` subclasses; for CPU tensors the
+kernels through autograd nodes (most of them native, ``csrc/native``); for CPU tensors the
 same mathematics is expressed with torch CPU ops so that the torch autograd
 engine differentiates it.  There is no second GPU implementation: if the
 native library is missing on a GPU machine the launchers raise.
@@ -31,8 +31,6 @@ UNARY = {
     "exp": 9, "log": 10, "sqrt": 11, "abs": 12, "sin": 13, "cos": 14, "pow": 15, "add_scalar": 16,
     "mul_scalar": 17, "rsub_scalar": 18, "rdiv_scalar": 19, "affine": 20, "clamp": 21,
 }
-_SAVES_OUTPUT = {"tanh", "sigmoid", "exp", "sqrt"}
-_SAVES_NOTHING = {"neg", "add_scalar", "mul_scalar", "rsub_scalar", "affine", "none"}
 BINARY = {"add": 0, "sub": 1, "mul": 2, "div": 3, "pow": 4, "max": 5, "min": 6}
 REDUCE = {"sum": 0, "mean": 1, "max": 2, "min": 3, "prod": 4}
 LOSS = {"mse": 0, "bce": 1, "l1": 2, "smooth_l1": 3}
@@ -228,28 +226,9 @@ def _unary_cpu(x, op, a, b):
     raise ValueError(op)
 
 
-class _UnaryFn(Function):
-    @staticmethod
-    def forward(ctx, x, op, alpha, beta):
-        y = raw_unary(x, op, alpha, beta)
-        ctx.op, ctx.alpha, ctx.beta = op, alpha, beta
-        if op in _SAVES_NOTHING:
-            ctx.save_for_backward()
-        elif op in _SAVES_OUTPUT:
-            ctx.save_for_backward(y)
-        else:
-            ctx.save_for_backward(x)
-        return y
-
-    @staticmethod
-    def backward(ctx, g):
-        saved = ctx.saved_tensors[0] if ctx.saved_tensors else None
-        return raw_unary_bwd(g, saved, ctx.op, ctx.alpha, ctx.beta), None, None, None
-
-
 def unary(x: torch.Tensor, op: str, alpha: float = 0.0, beta: float = 0.0) -> torch.Tensor:
     if _native(x):
-        return _UnaryFn.apply(x, op, float(alpha), float(beta))
+        return _lib.native().unary(x, UNARY[op], alpha, beta)
     return _unary_cpu(x, op, alpha, beta)
 
 
@@ -347,6 +326,8 @@ def _binary_cpu(a, b, op):
 
 def binary(a: torch.Tensor, b: torch.Tensor, op: str) -> torch.Tensor:
     if _native(a) and _native(b):
+        if op == "add" and a.shape == b.shape:
+            return _lib.native().add(a, b)
         return _BinaryFn.apply(a, b, op)
     return _binary_cpu(a, b, op)
 
@@ -448,30 +429,14 @@ def arg_reduce(x: torch.Tensor, is_max: bool, dim: int | None = None, keepdim: b
 def _gemm_nt(a: torch.Tensor, b_nt: torch.Tensor, bias=None, act=None, low: bool = False, out=None,
              out_dtype=None, accumulate=False) -> torch.Tensor:
     """out = act(a @ b_nt^T + bias) with a [M,K], b_nt [N,K] (any strides)."""
-    if low:
-        ab = a if a.dtype == torch.bfloat16 else raw_cast(a.contiguous(), torch.bfloat16)
-        bb = b_nt if b_nt.dtype == torch.bfloat16 else raw_cast(b_nt.contiguous(), torch.bfloat16)
-        if not _gemm.bf16_operand_ok(ab):
-            ab = ab.contiguous()
-        if not _gemm.bf16_operand_ok(bb):
-            bb = bb.contiguous()
-        if _gemm.bf16_operand_ok(ab) and _gemm.bf16_operand_ok(bb):
-            return _gemm.gemm_bf16(ab, bb, bias=bias, act=act, out=out,
-                                   out_dtype=out_dtype or torch.bfloat16, accumulate=accumulate)
-        # row pitch not a multiple of 16 bytes: exact SIMT kernel on fp32 copies
-        res = _gemm.gemm_f32(_f32(ab), _f32(bb), bias=bias, act=act, out=out if out is not None and
-                             out.dtype == torch.float32 else None, accumulate=accumulate and out is not None)
-        if out is not None and out.dtype != torch.float32:
-            out.copy_(res)
-            return out
-        return raw_cast(res, out_dtype or torch.bfloat16)
-    af, bf = _f32(a), _f32(b_nt)
-    if (config.tf32_active() and _gemm.tf32_operand_ok(af) and _gemm.tf32_operand_ok(bf)
-            and (out is None or (out.dtype == torch.float32 and out.stride(-1) == 1))
-            and (bias is None or bias.dtype == torch.float32)):
-        return _gemm.gemm_tf32(af, bf, bias=bias, act=act, out=out, accumulate=accumulate)
-    res = _gemm.gemm_f32(af, bf, bias=bias, act=act, out=out, accumulate=accumulate)
-    return res
+    dt = torch.bfloat16 if low else torch.float32
+    ab = a if a.dtype == dt else raw_cast(a.contiguous(), dt)
+    bb = b_nt if b_nt.dtype == dt else raw_cast(b_nt.contiguous(), dt)
+    if out is None:
+        out = torch.empty((a.shape[0], b_nt.shape[0]), device=a.device, dtype=out_dtype or dt)
+        accumulate = False
+    _lib.native().gemm_nt(ab, bb, bias, UNARY[act or "none"], out, accumulate, not low and config.tf32_active())
+    return out
 
 
 class _MatmulFn(Function):
@@ -729,71 +694,6 @@ class GradSink:
         raise NotImplementedError
 
 
-def _wgrad_to_sink(sink, weight_ref, g_t: torch.Tensor, x_t: torch.Tensor, low: bool) -> None:
-    """dW = g_t @ x_t^T written where the sink wants it: pushed to the shard owners from the GEMM epilogue when the
-    sink supports that (data-parallel engine in push mode, bf16 operands), else into the sink's buffer."""
-    push = getattr(sink, "try_push", None)
-    if push is not None and low and g_t.dtype == torch.bfloat16 and x_t.dtype == torch.bfloat16 and push(
-            weight_ref, g_t, x_t):
-        return
-    buf, acc = sink.acquire(weight_ref)
-    _gemm_nt(g_t, x_t, low=low, out=buf, out_dtype=torch.float32, accumulate=acc)
-
-
-class _LinearFn(Function):
-    @staticmethod
-    def forward(ctx, x, weight, bias, act, low, w_low, sink):
-        lead = x.shape[:-1]
-        x2 = x.reshape(-1, x.shape[-1])
-        ctx.low, ctx.act, ctx.sink = low, act, sink
-        ctx.x_dtype, ctx.lead = x.dtype, lead
-        ctx.has_bias = bias is not None
-        ctx.weight_ref = weight
-        if low:
-            xb = x2 if x2.dtype == torch.bfloat16 else raw_cast(x2.contiguous(), torch.bfloat16)
-            wb = w_low if w_low is not None else raw_cast(weight.detach().contiguous(), torch.bfloat16)
-            y = _gemm_nt(xb, wb, bias=bias, act=act, low=True)
-            saved_x, saved_w = xb, wb
-        else:
-            xf = _f32(x2)
-            y = _gemm_nt(xf, weight.detach(), bias=bias, act=act, low=False)
-            saved_x, saved_w = xf, weight.detach()
-        if act is None:
-            ctx.save_for_backward(saved_x, saved_w)
-        else:
-            ctx.save_for_backward(saved_x, saved_w, y)
-        return y.reshape(*lead, weight.shape[0])
-
-    @staticmethod
-    def backward(ctx, g):
-        low, act = ctx.low, ctx.act
-        saved = ctx.saved_tensors
-        x2, w = saved[0], saved[1]
-        g2 = g.reshape(-1, g.shape[-1]).contiguous()
-        if low and g2.dtype != torch.bfloat16:
-            g2 = raw_cast(g2, torch.bfloat16)
-        if not low:
-            g2 = _f32(g2)
-        if act is not None:
-            # only activations whose derivative is a function of the output are fused here
-            g2 = raw_unary_bwd(g2, saved[2], act)
-        gx = gw = gb = None
-        if ctx.needs_input_grad[0]:  # dgrad first: the weight may be overwritten once its bucket is reduced
-            gx = _gemm_nt(g2, w.t(), low=low)
-            gx = raw_cast(gx, ctx.x_dtype).reshape(*ctx.lead, w.shape[1])
-        if ctx.needs_input_grad[1]:
-            sink = ctx.sink
-            if sink is not None:
-                _wgrad_to_sink(sink, ctx.weight_ref, g2.t(), x2.t(), low)
-            else:
-                gw = _gemm_nt(g2.t(), x2.t(), low=low, out_dtype=torch.float32)
-        if ctx.has_bias and ctx.needs_input_grad[2]:
-            gb = raw_colsum(g2)
-        if ctx.needs_input_grad[1] and ctx.sink is not None:
-            ctx.sink.ready(ctx.weight_ref)
-        return gx, gw, gb, None, None, None, None
-
-
 _FUSABLE_ACT = {"relu", "tanh", "sigmoid"}  # derivative expressible from the output
 
 
@@ -808,57 +708,14 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
         y = torch.nn.functional.linear(x, weight, bias)
         return _unary_cpu(y, act, 0.0, 0.0) if act else y
     low = config.low_precision_active()
-    needs_grad = torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad)
-    if act is not None and act not in _FUSABLE_ACT and needs_grad:
-        y = _LinearFn.apply(x, weight, bias, None, low, w_low, sink)
-        return unary(y, act)
-    return _LinearFn.apply(x, weight, bias, act, low, w_low, sink)
+    tf32 = not low and config.tf32_active()
+    if act is not None and act not in _FUSABLE_ACT and torch.is_grad_enabled() and (
+            x.requires_grad or weight.requires_grad):
+        return unary(_lib.native().linear(x, weight, bias, 0, low, tf32, w_low, sink), act)
+    return _lib.native().linear(x, weight, bias, UNARY[act or "none"], low, tf32, w_low, sink)
 
 
 # =============================================================================== normalisation
-class _LayerNormFn(Function):
-    @staticmethod
-    def forward(ctx, x, gamma, beta, eps, pre_act, want_colsum):
-        cols = x.shape[-1]
-        x2 = x.reshape(-1, cols).contiguous()
-        rows = x2.shape[0]
-        y = torch.empty_like(x2)
-        mean = torch.empty(rows, device=x.device, dtype=torch.float32)
-        rstd = torch.empty(rows, device=x.device, dtype=torch.float32)
-        g = gamma.detach().contiguous() if gamma is not None else None
-        b = beta.detach().contiguous() if beta is not None else None
-        _rt.status_ptr()  # the wide-row kernels report bounded-wait failures to the status block
-        _lib.check(_lib.cuda().fb_layernorm_fwd(x2.data_ptr(), _ptr(g), _ptr(b), y.data_ptr(), mean.data_ptr(),
-                                                rstd.data_ptr(), rows, cols, eps, UNARY[pre_act or "none"],
-                                                _dt(x2), _stream()), "fb_layernorm_fwd")
-        ctx.save_for_backward(x2, g, mean, rstd)
-        ctx.pre_act, ctx.shape, ctx.want_colsum = pre_act, x.shape, want_colsum
-        ctx.has_gamma, ctx.has_beta = gamma is not None, beta is not None
-        return y.reshape(x.shape)
-
-    @staticmethod
-    def backward(ctx, gy):
-        x2, g, mean, rstd = ctx.saved_tensors
-        rows, cols = x2.shape
-        gy2 = gy.reshape(rows, cols).contiguous()
-        if gy2.dtype != x2.dtype:
-            gy2 = raw_cast(gy2, x2.dtype)
-        lib = _lib.cuda()
-        dx = torch.empty_like(x2)
-        nblk = lib.fb_layernorm_bwd_blocks(rows, cols)
-        partial = torch.empty((max(nblk, 1), 3, cols), device=x2.device, dtype=torch.float32)
-        stats = torch.zeros((3, cols), device=x2.device, dtype=torch.float32)
-        _lib.check(lib.fb_layernorm_bwd(gy2.data_ptr(), x2.data_ptr(), None, _ptr(g), mean.data_ptr(), rstd.data_ptr(),
-                                        dx.data_ptr(), partial.data_ptr(), stats.data_ptr(), rows, cols,
-                                        UNARY[ctx.pre_act or "none"], _dt(x2), nblk, 1 if ctx.want_colsum else 0,
-                                        _stream()), "fb_layernorm_bwd")
-        dgamma = stats[0] if ctx.has_gamma else None
-        dbeta = stats[1] if ctx.has_beta else None
-        dcol = stats[2] if ctx.want_colsum else None
-        ctx.colsum = dcol
-        return dx.reshape(ctx.shape), dgamma, dbeta, None, None, None
-
-
 def layer_norm(x: torch.Tensor, gamma=None, beta=None, eps: float = 1e-5, pre_act: str | None = None,
                n_norm_dims: int = 1) -> torch.Tensor:
     """Normalise over the last ``n_norm_dims`` dimensions; optional fused GELU before the statistics."""
@@ -869,7 +726,7 @@ def layer_norm(x: torch.Tensor, gamma=None, beta=None, eps: float = 1e-5, pre_ac
         b = beta.reshape(-1) if beta is not None else None
         return layer_norm(flat, g, b, eps, pre_act, 1).reshape(x.shape)
     if _native(x):
-        return _LayerNormFn.apply(x, gamma, beta, float(eps), pre_act, False)
+        return _lib.native().layer_norm(x, gamma, beta, eps, UNARY[pre_act or "none"])
     a = _unary_cpu(x, pre_act, 0.0, 0.0) if pre_act else x
     mu = a.mean(-1, keepdim=True)
     var = ((a - mu) ** 2).mean(-1, keepdim=True)
@@ -881,94 +738,13 @@ def layer_norm(x: torch.Tensor, gamma=None, beta=None, eps: float = 1e-5, pre_ac
     return y
 
 
-class _LinearActNormFn(Function):
-    """One autograd node for the block ``LayerNorm(act(x W^T + b))``.
-
-    Forward (tensor-core path): the GEMM epilogue writes act(z) and act'(z) in bf16, the LayerNorm kernel reads
-    act(z) and writes y.  Backward: one streaming kernel turns dy into dz (using the stored derivative) and also
-    yields d_gamma, d_beta and the column sum of dz (= the bias gradient), then the dgrad and wgrad GEMMs run on
-    dz.  On the fp32 path z itself is stored and the activation is evaluated inside the normalisation kernels.
-    """
-
-    @staticmethod
-    def forward(ctx, x, weight, bias, gamma, beta, eps, act, low, w_low, sink):
-        lead = x.shape[:-1]
-        x2 = x.reshape(-1, x.shape[-1])
-        if low:
-            xs = x2 if x2.dtype == torch.bfloat16 else raw_cast(x2.contiguous(), torch.bfloat16)
-            ws = w_low if w_low is not None else raw_cast(weight.detach().contiguous(), torch.bfloat16)
-        else:
-            xs, ws = _f32(x2), weight.detach()
-        # Tensor-core path: the GEMM epilogue stores act(z) and act'(z), so the normalisation kernels are pure
-        # streaming code.  fp32 path: z is stored and the GELU is evaluated inside the normalisation kernels.
-        dual = low and act is not None and xs.dtype == torch.bfloat16 and _gemm.bf16_operand_ok(xs) \
-            and _gemm.bf16_operand_ok(ws)
-        if dual:
-            z = torch.empty((xs.shape[0], ws.shape[0]), device=xs.device, dtype=torch.bfloat16)
-            dact = torch.empty_like(z)
-            _gemm.gemm_bf16(xs, ws, bias=bias, act=act, out=z, act_grad=dact)
-            pre = "none"
-        else:
-            z = _gemm_nt(xs, ws, bias=bias, act=None, low=low)
-            dact, pre = None, act or "none"
-        rows, cols = z.shape
-        y = torch.empty_like(z)
-        mean = torch.empty(rows, device=z.device, dtype=torch.float32)
-        rstd = torch.empty(rows, device=z.device, dtype=torch.float32)
-        g = gamma.detach().contiguous()
-        b = beta.detach().contiguous()
-        _rt.status_ptr()  # the wide-row kernels report bounded-wait failures to the status block
-        _lib.check(_lib.cuda().fb_layernorm_fwd(z.data_ptr(), g.data_ptr(), b.data_ptr(), y.data_ptr(),
-                                                mean.data_ptr(), rstd.data_ptr(), rows, cols, eps, UNARY[pre], _dt(z),
-                                                _stream()), "fb_layernorm_fwd")
-        if dual:
-            ctx.save_for_backward(xs, ws, z, g, mean, rstd, dact)
-        else:
-            ctx.save_for_backward(xs, ws, z, g, mean, rstd)
-        ctx.dual = dual
-        ctx.low, ctx.act, ctx.sink, ctx.weight_ref = low, pre, sink, weight
-        ctx.x_dtype, ctx.lead, ctx.has_bias = x.dtype, lead, bias is not None
-        return y.reshape(*lead, cols)
-
-    @staticmethod
-    def backward(ctx, gy):
-        if ctx.dual:
-            xs, ws, z, g, mean, rstd, dact = ctx.saved_tensors
-        else:
-            xs, ws, z, g, mean, rstd = ctx.saved_tensors
-            dact = None
-        rows, cols = z.shape
-        low = ctx.low
-        gy2 = gy.reshape(rows, cols).contiguous()
-        if gy2.dtype != z.dtype:
-            gy2 = raw_cast(gy2, z.dtype)
-        lib = _lib.cuda()
-        dz = torch.empty_like(z)
-        nblk = lib.fb_layernorm_bwd_blocks(rows, cols)
-        partial = torch.empty((max(nblk, 1), 3, cols), device=z.device, dtype=torch.float32)
-        stats = torch.zeros((3, cols), device=z.device, dtype=torch.float32)  # d_gamma, d_beta, colsum(dz)
-        _lib.check(lib.fb_layernorm_bwd(gy2.data_ptr(), z.data_ptr(), _ptr(dact), g.data_ptr(), mean.data_ptr(),
-                                        rstd.data_ptr(), dz.data_ptr(), partial.data_ptr(), stats.data_ptr(), rows,
-                                        cols, UNARY[ctx.act], _dt(z), nblk, 1, _stream()), "fb_layernorm_bwd")
-        gx = gw = None
-        if ctx.needs_input_grad[0]:
-            gx = raw_cast(_gemm_nt(dz, ws.t(), low=low), ctx.x_dtype).reshape(*ctx.lead, ws.shape[1])
-        if ctx.needs_input_grad[1]:
-            if ctx.sink is not None:
-                _wgrad_to_sink(ctx.sink, ctx.weight_ref, dz.t(), xs.t(), low)
-                ctx.sink.ready(ctx.weight_ref)
-            else:
-                gw = _gemm_nt(dz.t(), xs.t(), low=low, out_dtype=torch.float32)
-        gb = stats[2] if ctx.has_bias else None
-        return gx, gw, gb, stats[0], stats[1], None, None, None, None, None
-
-
 def linear_act_layernorm(x, weight, bias, gamma, beta, eps: float = 1e-5, act: str = "gelu", w_low=None,
                          sink: GradSink | None = None):
     """``LayerNorm(act(x @ weight^T + bias)) * gamma + beta`` as one fused block (CUDA); composed ops on CPU."""
     if _native(x) and gamma is not None and beta is not None:
-        return _LinearActNormFn.apply(x, weight, bias, gamma, beta, float(eps), act, config.low_precision_active(),
-                                      w_low, sink)
+        low = config.low_precision_active()
+        return _lib.native().linear_act_norm(x, weight, bias, gamma, beta, eps, UNARY[act or "none"], low,
+                                             not low and config.tf32_active(), w_low, sink)
     return layer_norm(linear(x, weight, bias, None, w_low, sink), gamma, beta, eps, act)
 
 
@@ -1044,31 +820,6 @@ def batch_norm(x: torch.Tensor, gamma, beta, running_mean, running_var, training
 
 
 # =============================================================================== softmax / losses
-class _SoftmaxFn(Function):
-    @staticmethod
-    def forward(ctx, x, log_mode):
-        cols = x.shape[-1]
-        x2 = x.reshape(-1, cols).contiguous()
-        y = torch.empty_like(x2)
-        _lib.check(_lib.cuda().fb_softmax_fwd(x2.data_ptr(), y.data_ptr(), x2.shape[0], cols, 1 if log_mode else 0,
-                                              _dt(x2), _stream()), "fb_softmax_fwd")
-        ctx.save_for_backward(y)
-        ctx.log_mode, ctx.shape = log_mode, x.shape
-        return y.reshape(x.shape)
-
-    @staticmethod
-    def backward(ctx, g):
-        (y,) = ctx.saved_tensors
-        rows, cols = y.shape
-        g2 = g.reshape(rows, cols).contiguous()
-        if g2.dtype != y.dtype:
-            g2 = raw_cast(g2, y.dtype)
-        dx = torch.empty_like(y)
-        _lib.check(_lib.cuda().fb_softmax_bwd(g2.data_ptr(), y.data_ptr(), dx.data_ptr(), rows, cols,
-                                              1 if ctx.log_mode else 0, _dt(y), _stream()), "fb_softmax_bwd")
-        return dx.reshape(ctx.shape), None
-
-
 def _softmax_any_dim(x, dim, log_mode):
     nd = x.dim()
     if nd == 0:
@@ -1077,8 +828,8 @@ def _softmax_any_dim(x, dim, log_mode):
     d = dim + nd if dim < 0 else dim
     if _native(x):
         if d != nd - 1:
-            return _SoftmaxFn.apply(x.transpose(d, -1), log_mode).transpose(d, -1)
-        return _SoftmaxFn.apply(x, log_mode)
+            return _lib.native().softmax(x.transpose(d, -1), log_mode).transpose(d, -1)
+        return _lib.native().softmax(x, log_mode)
     return torch.log_softmax(x, d) if log_mode else torch.softmax(x, d)
 
 
@@ -1091,34 +842,6 @@ def log_softmax(x: torch.Tensor, dim: int = -1) -> torch.Tensor:
     return _softmax_any_dim(x, dim, True)
 
 
-class _CEFn(Function):
-    """Fused log-softmax + NLL over integer labels: one kernel yields loss rows and the logit gradient."""
-
-    @staticmethod
-    def forward(ctx, logits, labels, scale):
-        rows, cols = logits.shape
-        lg = logits.contiguous()
-        row_loss = torch.empty(rows, device=lg.device, dtype=torch.float32)
-        need_grad = ctx.needs_input_grad[0]
-        dl = torch.empty_like(lg) if need_grad else None
-        _lib.check(_lib.cuda().fb_ce_fwd_bwd(lg.data_ptr(), labels.data_ptr(), row_loss.data_ptr(), _ptr(dl), rows,
-                                             cols, scale, _dt(lg), _dt(lg), _stream()), "fb_ce_fwd_bwd")
-        if need_grad:
-            ctx.save_for_backward(dl)
-        loss = raw_reduce(row_loss, "sum", None)
-        return raw_unary(loss, "mul_scalar", scale)
-
-    @staticmethod
-    def backward(ctx, g):
-        (dl,) = ctx.saved_tensors
-        # dl already carries the 1/rows factor; scale by the incoming scalar gradient
-        gf = _f32(g).reshape(1).contiguous()
-        out = torch.empty_like(dl)
-        _lib.check(_lib.cuda().fb_scale_by_device_scalar(dl.data_ptr(), gf.data_ptr(), out.data_ptr(), dl.numel(),
-                                                         _dt(dl), _stream()), "fb_scale_by_device_scalar")
-        return out, None, None
-
-
 def cross_entropy_logits(logits: torch.Tensor, labels: torch.Tensor) -> torch.Tensor:
     """Mean over the batch of ``-log softmax(logits)[label]`` for integer ``labels`` (fused kernel on CUDA)."""
     if logits.dim() != 2:
@@ -1126,35 +849,14 @@ def cross_entropy_logits(logits: torch.Tensor, labels: torch.Tensor) -> torch.Te
         labels = labels.reshape(-1)
     labels = labels.to(torch.int64)
     if _native(logits):
-        x = logits
-        if not torch.is_grad_enabled():
-            x = logits.detach()
-        return _CEFn.apply(x, labels.contiguous(), 1.0 / logits.shape[0])
+        return _lib.native().cross_entropy(logits, labels)
     lp = torch.log_softmax(logits.float(), -1)
     return -lp.gather(1, labels.unsqueeze(1)).mean()
 
 
-class _ElemLossFn(Function):
-    @staticmethod
-    def forward(ctx, pred, target, kind):
-        p, t = _f32(pred).contiguous(), _f32(target).contiguous()
-        out = torch.zeros((), device=p.device, dtype=torch.float32)
-        n = p.numel()
-        _lib.check(_lib.cuda().fb_loss_fwd(p.data_ptr(), t.data_ptr(), out.data_ptr(), n, LOSS[kind], 1.0 / n,
-                                           _stream()), "fb_loss_fwd")
-        ctx.save_for_backward(p, t)
-        ctx.kind, ctx.shape, ctx.dtype = kind, pred.shape, pred.dtype
-        return out
-
-    @staticmethod
-    def backward(ctx, g):
-        p, t = ctx.saved_tensors
-        gf = _f32(g).contiguous()
-        dp = torch.empty_like(p)
-        n = p.numel()
-        _lib.check(_lib.cuda().fb_loss_bwd(p.data_ptr(), t.data_ptr(), gf.data_ptr(), dp.data_ptr(), n,
-                                           LOSS[ctx.kind], 1.0 / n, _stream()), "fb_loss_bwd")
-        return raw_cast(dp.reshape(ctx.shape), ctx.dtype), None, None
+def nll_index(log_probs: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
+    """Mean over the rows of ``-log_probs[i, targets[i]]`` for integer ``targets`` on the GPU."""
+    return _lib.native().nll(log_probs, targets.reshape(-1).to(torch.int64))
 
 
 def elementwise_loss(pred: torch.Tensor, target: torch.Tensor, kind: str) -> torch.Tensor:
@@ -1162,7 +864,7 @@ def elementwise_loss(pred: torch.Tensor, target: torch.Tensor, kind: str) -> tor
     if tuple(pred.shape) != tuple(target.shape):
         target = target.expand_as(pred)
     if _native(pred) and pred.numel() > 0:
-        return _ElemLossFn.apply(pred, target.detach(), kind)
+        return _lib.native().elementwise_loss(pred, target, LOSS[kind])
     d = pred - target
     if kind == "mse":
         return (d * d).mean()
@@ -1236,67 +938,13 @@ def dropout(x: torch.Tensor, p: float, training: bool, seed: int | None = None) 
     return torch.nn.functional.dropout(x, p, True)
 
 
-def _sorted_indices(idx_flat: torch.Tensor):
-    """(sorted indices, original positions): a radix sort of the looked-up ids."""
-    return torch.sort(idx_flat, stable=True)
-
-
-class _EmbeddingFn(Function):
-    @staticmethod
-    def forward(ctx, weight, idx, padding_idx, out_dtype, pool, sink=None):
-        ctx.sink, ctx.weight_ref = sink, weight
-        w = weight.detach().contiguous()
-        V, D = w.shape
-        idx_c = idx.contiguous()
-        lib = _lib.cuda()
-        if pool:
-            B, S = idx_c.shape
-            out = torch.empty((B, D), device=w.device, dtype=out_dtype)
-            _lib.check(lib.fb_embedding_meanpool_fwd(w.data_ptr(), idx_c.data_ptr(), out.data_ptr(), B, S, D, V,
-                                                     F32 if out_dtype == torch.float32 else BF16, _stream()),
-                       "fb_embedding_meanpool_fwd")
-            ctx.group = S
-        else:
-            out = torch.empty((*idx_c.shape, D), device=w.device, dtype=out_dtype)
-            _lib.check(lib.fb_embedding_fwd(w.data_ptr(), idx_c.data_ptr(), out.data_ptr(), idx_c.numel(), D, V,
-                                            -1 if padding_idx is None else padding_idx,
-                                            F32 if out_dtype == torch.float32 else BF16, _rt.status_ptr(),
-                                            _stream()), "fb_embedding_fwd")
-            ctx.group = 1
-        ctx.save_for_backward(idx_c)
-        ctx.wshape, ctx.padding_idx, ctx.pool = (V, D), padding_idx, pool
-        return out
-
-    @staticmethod
-    def backward(ctx, g):
-        (idx,) = ctx.saved_tensors
-        V, D = ctx.wshape
-        g2 = g.reshape(-1, D).contiguous()
-        flat = idx.reshape(-1)
-        sidx, perm = _sorted_indices(flat)
-        if ctx.sink is not None:  # accumulate straight into the data-parallel gradient arena
-            dw, acc = ctx.sink.acquire(ctx.weight_ref)
-            if not acc:
-                dw.zero_()
-        else:
-            dw = torch.zeros((V, D), device=g.device, dtype=torch.float32)
-        scale = 1.0 / ctx.group if ctx.pool else 1.0
-        _lib.check(_lib.cuda().fb_embedding_bwd_sorted(g2.data_ptr(), sidx.data_ptr(), perm.data_ptr(),
-                                                       dw.data_ptr(), flat.numel(), D, ctx.group, scale,
-                                                       -1 if ctx.padding_idx is None else ctx.padding_idx, V,
-                                                       _dt(g2), _stream()), "fb_embedding_bwd_sorted")
-        if ctx.sink is not None:
-            ctx.sink.ready(ctx.weight_ref)
-            return None, None, None, None, None, None
-        return dw, None, None, None, None, None
-
-
 def embedding(weight: torch.Tensor, idx: torch.Tensor, padding_idx: int | None = None,
               out_dtype: torch.dtype | None = None, sink: GradSink | None = None) -> torch.Tensor:
     """Row gather ``weight[idx]`` -> ``[*idx.shape, D]``; rows at ``padding_idx`` are zero (embedding.rs:122-208)."""
     idx = idx.to(torch.int64)
     if weight.is_cuda and weight.dtype == torch.float32:
-        return _EmbeddingFn.apply(weight, idx, padding_idx, out_dtype or torch.float32, False, sink)
+        return _lib.native().embedding(weight, idx, -1 if padding_idx is None else padding_idx, False,
+                                       out_dtype == torch.bfloat16, sink)
     out = torch.nn.functional.embedding(idx, weight)
     if padding_idx is not None:
         out = out * (idx != padding_idx).unsqueeze(-1).to(out.dtype)
@@ -1308,7 +956,7 @@ def embedding_mean_pool(weight: torch.Tensor, idx: torch.Tensor, out_dtype: torc
     """``mean_s weight[idx[b, s]]`` for ``idx [B, S]`` without materialising ``[B, S, D]``."""
     idx = idx.to(torch.int64)
     if weight.is_cuda and weight.dtype == torch.float32 and idx.dim() == 2 and idx.shape[1] * 8 <= 48 * 1024:
-        return _EmbeddingFn.apply(weight, idx, None, out_dtype or torch.float32, True, sink)
+        return _lib.native().embedding(weight, idx, -1, True, out_dtype == torch.bfloat16, sink)
     return torch.nn.functional.embedding(idx, weight).mean(1)
 
 

@@ -28,12 +28,14 @@ def set_gemm_2cta(flag: bool) -> None:
     """Choose between the CTA-pair kernel (large shapes) and the single-CTA kernel."""
     global _use_2cta
     _use_2cta = bool(flag)
+    _lib.native().set_use_2cta(_use_2cta)
 
 
 def set_gemm_cta_limit(n: int) -> None:
     """Cap the persistent GEMM grid (0 = one CTA per SM)."""
     global _max_ctas
     _max_ctas = int(n)
+    _lib.native().set_max_ctas(_max_ctas)
 
 
 def _stream() -> int:

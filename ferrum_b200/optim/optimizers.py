@@ -13,7 +13,6 @@ waits for the reduction kernels, which have already applied the update.
 """
 from __future__ import annotations
 
-import ctypes
 from dataclasses import dataclass, replace
 
 import torch
@@ -141,6 +140,9 @@ class Optimizer:
         if self._engine is not None:
             self._engine.zero_grad()
             return
+        if set_to_none and _lib._native is not None:
+            _lib._native.clear_grads(self.params)
+            return
         for p in self.params:
             if set_to_none:
                 p.grad = None
@@ -157,28 +159,11 @@ class Optimizer:
         self._step_local()
 
     # -- helpers
-    def _split(self):
-        cuda, cpu = [], []
-        for i, p in enumerate(self.params):
-            if p.grad is None:
-                continue
-            (cuda if (p.is_cuda and p.dtype == torch.float32 and p.grad.dtype == torch.float32
-                      and p.is_contiguous() and p.grad.is_contiguous()) else cpu).append(i)
-        return cuda, cpu
+    def _on_gpu(self) -> bool:
+        return any(p.is_cuda for p in self.params)
 
-    @staticmethod
-    def _ptr_array(vals):
-        arr = (ctypes.c_void_p * len(vals))()
-        for i, v in enumerate(vals):
-            arr[i] = v
-        return arr
-
-    @staticmethod
-    def _shadow_ptr(p):
-        sh = p.__dict__.get("_fb_shadow")
-        if sh is None or sh.shape != p.shape or p.__dict__.get("_fb_shadow_key") != (p._version, p.data_ptr()):
-            return None  # absent or stale: the owning layer re-casts on its next forward
-        return sh.data_ptr()
+    def _with_grad(self) -> list:
+        return [i for i, p in enumerate(self.params) if p.grad is not None]
 
 
 class SGD(Optimizer):
@@ -201,31 +186,9 @@ class SGD(Optimizer):
 
     def _step_local(self) -> None:
         c = self.config
-        cuda_idx, cpu_idx = self._split()
-        if cuda_idx:
-            ps, gs, bs, shs, ns = [], [], [], [], []
-            for i in cuda_idx:
-                p = self.params[i]
-                first = self.velocity[i] is None
-                if c.momentum != 0.0 and first:
-                    self.velocity[i] = torch.zeros_like(p)
-                ps.append(p.data_ptr())
-                gs.append(p.grad.data_ptr())
-                bs.append(self.velocity[i].data_ptr() if c.momentum != 0.0 else None)
-                shs.append(self._shadow_ptr(p))
-                ns.append(p.numel())
-            # buffers start at zero, so mu * 0 + g == g reproduces the reference's first step (sgd.rs:95-104)
-            h = self.hparams()
-            n = len(ps)
-            st = torch.cuda.current_stream().cuda_stream
-            if self._dyn is not None:
-                _lib.check(_lib.cuda().fb_sgd_multi_dyn(self._ptr_array(ps), self._ptr_array(gs), self._ptr_array(bs),
-                                                        self._ptr_array(shs), (ctypes.c_longlong * n)(*ns), n, h,
-                                                        self._dyn.data_ptr(), st), "fb_sgd_multi_dyn")
-            else:
-                _lib.check(_lib.cuda().fb_sgd_multi(self._ptr_array(ps), self._ptr_array(gs), self._ptr_array(bs),
-                                                    self._ptr_array(shs), (ctypes.c_longlong * n)(*ns), n, h, st),
-                           "fb_sgd_multi")
+        cpu_idx = _lib.native().sgd_step(self.params, self.velocity if c.momentum != 0.0 else None, c.lr, c.momentum,
+                                         c.weight_decay, c.nesterov, self.step_count == 0,
+                                         self._dyn) if self._on_gpu() else self._with_grad()
         with torch.no_grad():
             for i in cpu_idx:
                 p = self.params[i]
@@ -288,34 +251,8 @@ class Adam(Optimizer):
         self.step_count += 1
         t = self.step_count
         bc1, bc2 = 1.0 - c.beta1 ** t, 1.0 - c.beta2 ** t
-        cuda_idx, cpu_idx = self._split()
-        if cuda_idx:
-            ps, gs, ms, vs, shs, ns = [], [], [], [], [], []
-            for i in cuda_idx:
-                p = self.params[i]
-                if self.m[i] is None:
-                    self.m[i] = torch.zeros_like(p)
-                    self.v[i] = torch.zeros_like(p)
-                ps.append(p.data_ptr())
-                gs.append(p.grad.data_ptr())
-                ms.append(self.m[i].data_ptr())
-                vs.append(self.v[i].data_ptr())
-                shs.append(self._shadow_ptr(p))
-                ns.append(p.numel())
-            n = len(ps)
-            st = torch.cuda.current_stream().cuda_stream
-            if self._dyn is not None:
-                lib = _lib.cuda()
-                _lib.check(lib.fb_optim_advance(self._dyn.data_ptr(), c.beta1, c.beta2, st), "fb_optim_advance")
-                _lib.check(lib.fb_adam_multi_dyn(self._ptr_array(ps), self._ptr_array(gs), self._ptr_array(ms),
-                                                 self._ptr_array(vs), self._ptr_array(shs),
-                                                 (ctypes.c_longlong * n)(*ns), n, self.hparams(t),
-                                                 self._dyn.data_ptr(), st), "fb_adam_multi_dyn")
-            else:
-                _lib.check(_lib.cuda().fb_adam_multi(self._ptr_array(ps), self._ptr_array(gs), self._ptr_array(ms),
-                                                     self._ptr_array(vs), self._ptr_array(shs),
-                                                     (ctypes.c_longlong * n)(*ns), n, self.hparams(t), st),
-                           "fb_adam_multi")
+        cpu_idx = _lib.native().adam_step(self.params, self.m, self.v, c.lr, c.beta1, c.beta2, c.eps, c.weight_decay,
+                                          bc1, bc2, self._dyn) if self._on_gpu() else self._with_grad()
         with torch.no_grad():
             for i in cpu_idx:
                 p = self.params[i]

@@ -46,14 +46,15 @@ class _TimedLib:
 class Profile:
     def __init__(self):
         self.records = []
+        self.native = []  # (launcher, milliseconds) of the native host path
 
     def report(self) -> dict:
         """{entry point: {"calls", "total_ms", "mean_us"}} sorted by total time (synchronizes)."""
         torch.cuda.synchronize()
         agg = defaultdict(lambda: [0, 0.0])
-        for name, e0, e1 in self.records:
+        for name, ms in [(n, e0.elapsed_time(e1)) for n, e0, e1 in self.records] + self.native:
             agg[name][0] += 1
-            agg[name][1] += e0.elapsed_time(e1)
+            agg[name][1] += ms
         out = {k: {"calls": c, "total_ms": t, "mean_us": 1e3 * t / c} for k, (c, t) in agg.items()}
         return dict(sorted(out.items(), key=lambda kv: -kv[1]["total_ms"]))
 
@@ -72,11 +73,15 @@ def profile(nvtx: bool = True):
     """Time every kernel launcher called inside the block."""
     prof = Profile()
     real = _lib.cuda()
+    native = _lib.native()
     _lib._cuda = _TimedLib(real, prof.records, nvtx)
+    native.profile_start()
     try:
         yield prof
     finally:
         _lib._cuda = real
+        native.profile_stop()
+        prof.native = native.profile_records()
 
 
 def measured_peaks() -> dict | None:
