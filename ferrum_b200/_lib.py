@@ -113,6 +113,7 @@ _CUDA_SIGS = {
     "fb_gemm_bf16_2cta_set_profile": (None, [P]),
     "fb_gemm_bf16_2cta_set_group_m": (I, [I]),
     "fb_gemm_bf16_batched": (I, [P, P, P, I, I, I, LL, LL, LL, I, I, LL, LL, LL, LL, LL, LL, I, I, I, I, F, P, P]),
+    "fb_gemm_f32_tensor": (I, [P, P, P, P, I, I, I, LL, LL, LL, LL, LL, I, I, F, I, I, LL, LL, LL, LL, LL, LL, P, P]),
     "fb_gemm_f32_simt": (I, [P, P, P, P, I, I, I, LL, LL, LL, LL, LL, I, I, I, LL, LL, LL, P]),
     # secondary layers
     "fb_lstm_gates_fwd": (I, [P, P, P, P, P, P, LL, I, P]),

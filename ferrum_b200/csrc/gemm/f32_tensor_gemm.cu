@@ -1,0 +1,495 @@
+// fp32 GEMM on the tensor cores without giving up fp32 precision (sm_100a).
+//
+// Every fp32 operand element is split into three bf16 numbers a = a0 + a1 + a2, each the value that was left rounded
+// to nearest (8 + 8 + 8 significant bits: the sum is exact), and six of the nine products are accumulated in fp32 by
+// tcgen05.mma: a0 b0, a0 b1, a1 b0, a1 b1, a0 b2, a2 b0.  The three that are left out are below 2^-26 of |a b|, less
+// than the rounding of one fp32 multiply-add.  The tensor core truncates where it adds (2048 x 2048 x 4096 of
+// normal numbers summed there alone: relative error 2.8e-5), so each k-block of 64 gets a fresh accumulator and the
+// k-blocks are added in registers, rounded to nearest: 1.7e-7, against 1.1e-6 of a chain of fp32 multiply-adds.
+//
+// What bounds it: six bf16 MMAs per fp32 product (271 TFLOP/s at the measured bf16 rate), and beside it the split:
+// about seven instructions per operand element in eight warps, in the shadow of the MMAs.  The split happens on the
+// way from global memory (registers) to shared memory (three bf16 planes, 128-byte swizzle, K-major), so any element
+// strides are accepted, nothing is staged in global memory and no second launch is needed.
+//
+// One CTA per 128 x BN output tile and K split.  The splits of a tile are one thread-block cluster: the partial tiles
+// meet through distributed shared memory in a fixed order, so small outputs fill the chip without a workspace.
+//
+// Infinities, NaNs and values that would round to infinity do not survive the split (inf - inf, 0 * inf) and always
+// end in a result that is not finite; such a result is computed again with fp32 multiply-adds when the tile is written.
+//
+// The issue of a k-block's MMAs takes as long as the MMAs themselves (the queue is short), so it has a warp of its own;
+// a loader warp that issued them held up the next stage (5200 instead of 2300 cycles per k-block).
+#include <cooperative_groups.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include <cfloat>
+#include <cstdint>
+
+#include "../common/ptx.cuh"
+#include "../common/status.h"
+#include "../include/ferrum_kernels.h"
+
+namespace fb {
+namespace {
+
+namespace cg = cooperative_groups;
+
+constexpr int kBM = 128;
+constexpr int kLoaders = 512;
+constexpr int kThreads = kLoaders + 32;  // 16 warps load, split, add up and write; one issues the MMAs
+
+template <int BN>
+struct Cfg {
+  static constexpr int kBK = 64;                   // fp32 elements of K per stage
+  static constexpr int kRow = kBK * 2;             // bytes of a row of a bf16 plane = its swizzle width
+  static constexpr int kPieces = kBK / 8;          // 8-element pieces per row
+  static constexpr int kPlaneA = kBM * kRow, kPlaneB = BN * kRow;
+  static constexpr int kStage = 3 * (kPlaneA + kPlaneB);
+  static constexpr int kStages = BN == 64 ? 3 : 2;
+  static constexpr int kPitch = BN + 4;   // floats per row of the tile in shared memory: conflict-free 16-byte rows
+  static constexpr int kTile = kBM * kPitch * 4;
+  static constexpr int kBody = kStages * kStage > kTile ? kStages * kStage : kTile;
+  static constexpr int kSmem = kBody + 1024 + 256;
+  static constexpr int kTmemCols = 2 * BN;
+  static constexpr int kPerThread = (kBM + BN) * kPieces / kLoaders;  // pieces of a stage per thread
+  static constexpr int kAcc = kBM * BN / kLoaders;                    // accumulators per thread: a quarter of a tile row
+  // 16-byte chunk of a row, as the 128- / 64-byte swizzle of the matrix descriptors places it
+  __device__ static uint32_t at(int row, int kc) {
+    return row * kRow + ((kc ^ (kRow == 128 ? row & 7 : (row >> 1) & 3)) << 4);
+  }
+  __device__ static uint64_t desc(uint32_t addr) {
+    return ptx::make_smem_desc_sw128(addr, 16, 8 * kRow, kRow == 128 ? 2 : 4);
+  }
+};
+
+struct Operand {
+  const float* p;
+  long long s_row, s_k, s_bo, s_bi;  // element strides; slices of the batch (outer, inner)
+  int rows;
+};
+
+// How an operand lies in memory: K contiguous with 16-byte aligned rows (two vector loads per piece), K contiguous
+// with any alignment, or anything else (lanes follow the rows).
+enum Layout { kVecK = 0, kScalarK = 1, kRowFast = 2 };
+
+struct Args {
+  Operand a, b;
+  float* out;
+  const float* bias;
+  long long ldc, sc_bo, sc_bi;
+  int M, N, K;
+  int act, beta;
+  float alpha;
+  int batch_inner;
+  int kb_total, kb_per_split;
+  int32_t* status;
+  unsigned long long timeout_ns;
+};
+
+__device__ __forceinline__ float act_f(float x, int act) {
+  switch (act) {
+    case FB_ACT_RELU: return fmaxf(x, 0.f);
+    case FB_ACT_GELU: {
+      const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
+      return 0.5f * x * (1.f + tanhf(u));
+    }
+    case FB_ACT_SILU: return x / (1.f + expf(-x));
+    case FB_ACT_TANH: return tanhf(x);
+    case FB_ACT_SIGMOID: return 1.f / (1.f + expf(-x));
+    default: return x;
+  }
+}
+
+// Where piece `c` of an operand tile (row, 8 consecutive k) lies: neighbouring lanes follow the contiguous direction.
+template <int ROWS, int L, int PIECES>
+__device__ __forceinline__ void piece(int c, int& row, int& kc) {
+  if (L == kRowFast) {
+    row = c % ROWS;
+    kc = c / ROWS;
+  } else {
+    row = c / PIECES;
+    kc = c % PIECES;
+  }
+}
+
+// Rows past the edge read the last row (their products are dropped with the tile's edge), so whole k-blocks load
+// without a condition and stay in flight until they are split; only the last k-block of a ragged K is guarded.
+template <int ROWS, int L, int PIECES>
+__device__ __forceinline__ void load_piece(const Operand& o, const float* base, int row0, int k0, int K, int c,
+                                           float (&v)[8]) {
+  int row, kc;
+  piece<ROWS, L, PIECES>(c, row, kc);
+  const int r = min(row0 + row, o.rows - 1), k = k0 + kc * 8;
+  if (k0 + PIECES * 8 <= K) {
+    if constexpr (L == kVecK) {
+      const float* p = base + r * o.s_row + k;
+      const float4 x = __ldg(reinterpret_cast<const float4*>(p)), y = __ldg(reinterpret_cast<const float4*>(p) + 1);
+      v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+      v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+    } else if constexpr (L == kScalarK) {
+      const float* p = base + r * o.s_row + k;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = __ldg(p + j);
+    } else {
+      const float* p = base + r * o.s_row + k * o.s_k;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = __ldg(p + j * o.s_k);
+    }
+  } else {
+    const float* p = base + r * o.s_row;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v[j] = 0.f;
+      if (k + j < K) v[j] = __ldg(p + (k + j) * o.s_k);
+    }
+  }
+}
+
+__device__ __forceinline__ float2 sub2(float2 x, float2 y) {  // x - y with one packed instruction: y * -1 is exact
+  float2 r;
+  asm("{\n.reg .b64 a, b, c, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmov.b64 c, {%6, %6};\n"
+      "fma.rn.f32x2 d, b, c, a;\nmov.b64 {%0, %1}, d;\n}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y), "f"(-1.f));
+  return r;
+}
+__device__ __forceinline__ float2 add2(float2 x, float2 y) {
+  float2 r;
+  asm("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nadd.rn.f32x2 d, a, b;\nmov.b64 {%0, %1}, d;\n}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
+  return r;
+}
+__device__ __forceinline__ uint32_t bf16_pair(float2 x) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(x.x, x.y);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ float2 wide_pair(uint32_t w) {
+  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+}
+
+// Splits eight values and stores them into the three planes.
+__device__ __forceinline__ void store_piece(uint32_t at, uint32_t plane_bytes, const float (&v)[8]) {
+  uint32_t w0[4], w1[4], w2[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 x = make_float2(v[2 * j], v[2 * j + 1]);
+    w0[j] = bf16_pair(x);
+    const float2 r = sub2(x, wide_pair(w0[j]));
+    w1[j] = bf16_pair(r);
+    w2[j] = bf16_pair(sub2(r, wide_pair(w1[j])));
+  }
+  ptx::st_shared_v4(at, w0[0], w0[1], w0[2], w0[3]);
+  ptx::st_shared_v4(at + plane_bytes, w1[0], w1[1], w1[2], w1[3]);
+  ptx::st_shared_v4(at + 2 * plane_bytes, w2[0], w2[1], w2[2], w2[3]);
+}
+
+template <int BN, int LA, int LB>
+__global__ void __launch_bounds__(kThreads, 1) gemm_f32_tensor_kernel(const __grid_constant__ Args p) {
+  using C = Cfg<BN>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + C::kBody);
+  uint64_t* empty_bar = full_bar + C::kStages;
+  uint64_t* acc_full = empty_bar + C::kStages;   // accumulator buffer complete
+  uint64_t* acc_empty = acc_full + 2;            // accumulator buffer read out
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int splits = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
+
+  const int n0 = static_cast<int>(blockIdx.x / splits) * BN, m0 = static_cast<int>(blockIdx.y) * kBM;
+  const int bo = static_cast<int>(blockIdx.z) / p.batch_inner, bi = static_cast<int>(blockIdx.z) % p.batch_inner;
+  const float* a = p.a.p + bo * p.a.s_bo + bi * p.a.s_bi;
+  const float* b = p.b.p + bo * p.b.s_bo + bi * p.b.s_bi;
+  float* out = p.out + bo * p.sc_bo + bi * p.sc_bi;
+
+  const int kb_lo = min(p.kb_total, rank * p.kb_per_split), kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
+  const int nkb = kb_hi - kb_lo;
+
+  if (threadIdx.x == 0) {
+    *abort_flag = 0;
+    for (int s = 0; s < C::kStages; ++s) {
+      ptx::mbar_init(&full_bar[s], kLoaders / 32);
+      ptx::mbar_init(&empty_bar[s], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      ptx::mbar_init(&acc_full[i], 1);
+      ptx::mbar_init(&acc_empty[i], kLoaders / 32);
+    }
+    ptx::fence_mbar_init();
+  }
+  if (warp == 0) {
+    ptx::tmem_alloc(tmem_slot, C::kTmemCols);
+    ptx::tmem_relinquish();
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  float acc[C::kAcc];
+  if (warp < kLoaders / 32) {
+    // -------------------------------------------------------- load, split, add up
+    constexpr int kPA = kBM * C::kPieces / kLoaders;  // pieces of A per thread; the rest are B's
+    float v[C::kPerThread][8];
+    auto fetch = [&](int i, int kb) {
+      const int k0 = kb * C::kBK;
+      if (i < kPA)
+        load_piece<kBM, LA, C::kPieces>(p.a, a, m0, k0, p.K, i * kLoaders + threadIdx.x, v[i]);
+      else
+        load_piece<BN, LB, C::kPieces>(p.b, b, n0, k0, p.K, (i - kPA) * kLoaders + threadIdx.x, v[i]);
+    };
+    if (nkb > 0) {
+#pragma unroll
+      for (int i = 0; i < C::kPerThread; ++i) fetch(i, kb_lo);
+    }
+#pragma unroll
+    for (int i = 0; i < C::kAcc; ++i) acc[i] = 0.f;
+    const uint32_t taddr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + (warp >> 2) * C::kAcc;
+    int blocks_read = 0;
+    bool ok = true;
+    auto read_block = [&]() {  // adds a finished k-block's accumulator to the registers
+      const int buf = blocks_read & 1;
+      const bool ready = ptx::mbar_wait(&acc_full[buf], (blocks_read >> 1) & 1, abort_flag, p.timeout_ns);
+      if (!__all_sync(0xffffffffu, ready)) {
+        ok = false;
+        return;
+      }
+      ptx::tc_fence_after();
+#pragma unroll
+      for (int j = 0; j < C::kAcc / 16; ++j) {
+        uint32_t r[16];
+        ptx::tmem_ld_32x32b_x16(taddr + buf * BN + j * 16, r);
+        ptx::tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+          const float2 s = add2(make_float2(acc[j * 16 + i], acc[j * 16 + i + 1]),
+                                make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])));
+          acc[j * 16 + i] = s.x;
+          acc[j * 16 + i + 1] = s.y;
+        }
+      }
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&acc_empty[buf]);
+      ++blocks_read;
+    };
+    for (int kb = 0; kb < nkb && ok; ++kb) {
+      const int s = kb % C::kStages;
+      const bool free_slot = ptx::mbar_wait(&empty_bar[s], ((kb / C::kStages) & 1) ^ 1, abort_flag, p.timeout_ns);
+      if (!__all_sync(0xffffffffu, free_slot)) {
+        ok = false;
+        break;
+      }
+      const uint32_t sa = ptx::smem_u32(smem + s * C::kStage), sb = sa + 3 * C::kPlaneA;
+      const bool more = kb + 1 < nkb;
+#pragma unroll
+      for (int i = 0; i < C::kPerThread; ++i) {
+        int row, kc;
+        if (i < kPA) {
+          piece<kBM, LA, C::kPieces>(i * kLoaders + threadIdx.x, row, kc);
+          store_piece(sa + C::at(row, kc), C::kPlaneA, v[i]);
+        } else {
+          piece<BN, LB, C::kPieces>((i - kPA) * kLoaders + threadIdx.x, row, kc);
+          store_piece(sb + C::at(row, kc), C::kPlaneB, v[i]);
+        }
+        if (more) fetch(i, kb_lo + kb + 1);
+      }
+      ptx::fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&full_bar[s]);
+      if (kb > 0) read_block();  // the k-block before: added up while the MMAs of this one run
+    }
+    if (ok && nkb > 0) read_block();
+    if (!ok) {
+      if (lane == 0) report_status(p.status, kStatusGemmTimeout, 50, blockIdx.x, warp);
+    }
+  } else if (lane == 0) {
+    // ---------------------------------------------------------------- MMA issue
+    const uint32_t idesc = ptx::make_idesc(1u, kBM, BN, 0, 0);
+    for (int kb = 0; kb < nkb; ++kb) {
+      const int s = kb % C::kStages, buf = kb & 1;
+      if (!ptx::mbar_wait(&acc_empty[buf], ((kb >> 1) & 1) ^ 1, abort_flag, p.timeout_ns) ||
+          !ptx::mbar_wait(&full_bar[s], (kb / C::kStages) & 1, abort_flag, p.timeout_ns)) {
+        report_status(p.status, kStatusGemmTimeout, 51, blockIdx.x, kb);
+        break;
+      }
+      ptx::tc_fence_after();
+      const uint32_t sa = ptx::smem_u32(smem + s * C::kStage), sb = sa + 3 * C::kPlaneA;
+      const uint32_t d = tmem + buf * BN;
+      constexpr int ia[6] = {2, 0, 1, 1, 0, 0}, ib[6] = {0, 2, 1, 0, 1, 0};  // small products first
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+#pragma unroll
+        for (int k = 0; k < C::kBK / 16; ++k) {
+          const uint64_t ad = C::desc(sa + ia[q] * C::kPlaneA + k * 32);
+          const uint64_t bd = C::desc(sb + ib[q] * C::kPlaneB + k * 32);
+          ptx::umma_f16(d, ad, bd, idesc, (q | k) != 0 ? 1u : 0u);
+        }
+      }
+      ptx::umma_commit(&empty_bar[s]);
+      ptx::umma_commit(&acc_full[buf]);
+    }
+  }
+
+  // ------------------------------------------------------------------ partial tiles meet
+  __syncthreads();  // every MMA has completed (the loaders waited for the last one): the stages are free
+  float* tile = reinterpret_cast<float*>(smem);
+  if (warp < kLoaders / 32) {
+    const int row = (warp & 3) * 32 + lane, c0 = (warp >> 2) * C::kAcc;
+    float4* t4 = reinterpret_cast<float4*>(tile + row * C::kPitch + c0);
+#pragma unroll
+    for (int i = 0; i < C::kAcc / 4; ++i)
+      t4[i] = make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
+  }
+  cluster.sync();
+  const int rows_per = kBM / splits;
+  const bool vec = p.N % 4 == 0 && p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+  constexpr int kVec = BN / 4;
+  for (int i = threadIdx.x; i < rows_per * kVec; i += kThreads) {
+    const int row = rank * rows_per + i / kVec, c = (i % kVec) * 4;
+    const int m = m0 + row, n = n0 + c;
+    if (m >= p.M || n >= p.N) continue;
+    float f[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int r = 0; r < splits; ++r) {
+      const float4 t = *reinterpret_cast<const float4*>(cluster.map_shared_rank(tile, r) + row * C::kPitch + c);
+      f[0] += t.x; f[1] += t.y; f[2] += t.z; f[3] += t.w;
+    }
+    for (int j = 0; j < 4; ++j) {
+      if (fabsf(f[j]) <= FLT_MAX || n + j >= p.N) continue;
+      // not finite: an operand that does not survive the split, or a result that is not finite in fp32 either
+      float s = 0.f;
+      for (int k = 0; k < p.K; ++k)
+        s = fmaf(a[m * p.a.s_row + k * p.a.s_k], b[(n + j) * p.b.s_row + k * p.b.s_k], s);
+      f[j] = s;
+    }
+    float* o = out + m * p.ldc + n;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (n + j < p.N) {
+        float x = f[j] * p.alpha;
+        if (p.bias != nullptr) x += __ldg(p.bias + n + j);
+        f[j] = act_f(x, p.act);
+      }
+    if (vec) {
+      float4 x = make_float4(f[0], f[1], f[2], f[3]);
+      if (p.beta) {
+        const float4 old = *reinterpret_cast<float4*>(o);
+        x.x += old.x; x.y += old.y; x.z += old.z; x.w += old.w;
+      }
+      *reinterpret_cast<float4*>(o) = x;
+    } else {
+      for (int j = 0; j < 4 && n + j < p.N; ++j) o[j] = p.beta ? o[j] + f[j] : f[j];
+    }
+  }
+  ptx::tc_fence_before();
+  cluster.sync();  // no CTA leaves while another one still reads its tile
+  if (warp == 0) {
+    ptx::tc_fence_after();
+    ptx::tmem_dealloc(tmem, C::kTmemCols);
+  }
+}
+
+int sm_count() {
+  static int n = 0;
+  if (n == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  }
+  return n;
+}
+
+template <int BN, int LA, int LB>
+int launch_one(const Args& args, int batch, int splits, cudaStream_t st) {
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(gemm_f32_tensor_kernel<BN, LA, LB>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::kSmem);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    configured = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>((args.N + BN - 1) / BN * splits), static_cast<unsigned>((args.M + kBM - 1) / kBM),
+                     static_cast<unsigned>(batch));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = Cfg<BN>::kSmem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = splits;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, gemm_f32_tensor_kernel<BN, LA, LB>, args));
+}
+
+template <int BN, int LA>
+int launch_b(int lb, const Args& args, int batch, int splits, cudaStream_t st) {
+  if (lb == kVecK) return launch_one<BN, LA, kVecK>(args, batch, splits, st);
+  if (lb == kScalarK) return launch_one<BN, LA, kScalarK>(args, batch, splits, st);
+  return launch_one<BN, LA, kRowFast>(args, batch, splits, st);
+}
+template <int BN>
+int launch(int la, int lb, const Args& args, int batch, int splits, cudaStream_t st) {
+  if (la == kVecK) return launch_b<BN, kVecK>(lb, args, batch, splits, st);
+  if (la == kScalarK) return launch_b<BN, kScalarK>(lb, args, batch, splits, st);
+  return launch_b<BN, kRowFast>(lb, args, batch, splits, st);
+}
+
+int layout_of(const float* p, long long s_row, long long s_k, long long s_bo, long long s_bi) {
+  if (s_k == 1)
+    return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && s_row % 4 == 0 && s_bo % 4 == 0 && s_bi % 4 == 0 ? kVecK : kScalarK;
+  return kRowFast;
+}
+
+}  // namespace
+}  // namespace fb
+
+using namespace fb;
+
+extern "C" int fb_gemm_f32_tensor(const float* a, const float* b, float* out, const float* bias, int M, int N, int K,
+                                  long long sam, long long sak, long long sbn, long long sbk, long long ldc, int act,
+                                  int beta, float alpha, int batch_outer, int batch_inner, long long sa_outer,
+                                  long long sa_inner, long long sb_outer, long long sb_inner, long long sc_outer,
+                                  long long sc_inner, int32_t* status, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || batch_outer <= 0 || batch_inner <= 0) return 0;
+  const long long batch = static_cast<long long>(batch_outer) * batch_inner;
+  if (K < 0 || batch > 65535 || (M + kBM - 1) / kBM > 65535) return -1;
+  Args g;
+  g.a = Operand{a, sam, sak, sa_outer, sa_inner, M};
+  g.b = Operand{b, sbn, sbk, sb_outer, sb_inner, N};
+  g.out = out;
+  g.bias = bias;
+  g.ldc = ldc;
+  g.sc_bo = sc_outer;
+  g.sc_bi = sc_inner;
+  g.M = M;
+  g.N = N;
+  g.K = K;
+  g.act = act;
+  g.beta = beta;
+  g.alpha = alpha;
+  g.batch_inner = batch_inner;
+  g.status = status;
+  g.timeout_ns = 2000000000ull;
+    // Tile width and K splits: the wide tile where it alone fills the chip, else the narrow one; then as many splits
+  // as there are idle SMs, each with at least one k-block.
+  const long long tm = (M + kBM - 1) / kBM;
+  const long long wide = tm * ((N + 127) / 128) * batch, narrow = tm * ((N + 63) / 64) * batch;
+  const int bk_wide = Cfg<128>::kBK;
+  const bool use_wide = N > 64 && wide * 8 > sm_count() && wide * (K + 127) / 128 >= sm_count();
+  const long long tiles = use_wide ? wide : narrow;
+  g.kb_total = (K + (use_wide ? bk_wide : Cfg<64>::kBK) - 1) / (use_wide ? bk_wide : Cfg<64>::kBK);
+  int splits = 1;
+  while (splits < 8 && tiles * splits * 2 <= sm_count() && splits * 2 <= g.kb_total) splits *= 2;
+  g.kb_per_split = (g.kb_total + splits - 1) / splits;
+  const int la = layout_of(a, sam, sak, sa_outer, sa_inner), lb = layout_of(b, sbn, sbk, sb_outer, sb_inner);
+  return use_wide ? launch<128>(la, lb, g, static_cast<int>(batch), splits, stream)
+                  : launch<64>(la, lb, g, static_cast<int>(batch), splits, stream);
+}

@@ -77,6 +77,13 @@ int fb_gemm_bf16_batched(const void* a, const void* b, void* out, int M, int N, 
                          long long sb_outer, long long sb_inner, long long sc_outer, long long sc_inner,
                          int a_mn_major, int b_mn_major, int out_bf16, int beta, float alpha, int32_t* status,
                          cudaStream_t stream);
+// fp32 GEMM of fp32 precision on the tensor cores (three bf16 parts per operand element, gemm/f32_tensor_gemm.cu):
+// out[s] = act(alpha * A[s] B[s]^T + bias) (+= when beta), any element strides; s = (outer, inner) batch slice.
+int fb_gemm_f32_tensor(const float* a, const float* b, float* out, const float* bias, int M, int N, int K,
+                       long long sam, long long sak, long long sbn, long long sbk, long long ldc, int act, int beta,
+                       float alpha, int batch_outer, int batch_inner, long long sa_outer, long long sa_inner,
+                       long long sb_outer, long long sb_inner, long long sc_outer, long long sc_inner,
+                       int32_t* status, cudaStream_t stream);
 // fp32 SIMT GEMM with arbitrary element strides (parity runs, odd shapes):
 // out[m,n] = act(sum_k A[m*sam + k*sak] * B[k*sbk + n*sbn] + bias[n]) (+= out when beta).
 int fb_gemm_f32_simt(const float* a, const float* b, float* out, const float* bias, int M, int N, int K,

@@ -79,6 +79,9 @@ bool tma_ok(const Op& a) {
   return false;
 }
 
+// fp32 products with a reduction this short do not repay the tensor-core kernel's set-up (7 us against 2 - 3).
+constexpr int kSimtK = 32;
+
 void gemm(const Op& a, const Op& b, const float* bias, int act, void* out, ll ldc, bool out_bf16, bool accumulate,
           void* act_grad, const Tensor* like, bool tf32) {
   const int M = static_cast<int>(a.rows), N = static_cast<int>(b.rows), K = static_cast<int>(a.k);
@@ -112,6 +115,12 @@ void gemm(const Op& a, const Op& b, const float* bias, int act, void* out, ll ld
     if (rc == -3)
       FB_CALL(fb_gemm_tf32, static_cast<const float*>(a.p), static_cast<const float*>(b.p), static_cast<float*>(out),
               bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, act, accumulate, g_max_ctas, status(), cur_stream());
+    return;
+  }
+  if (!a.bf16 && !out_bf16 && K > kSimtK) {
+    FB_CALL(fb_gemm_f32_tensor, static_cast<const float*>(a.p), static_cast<const float*>(b.p), static_cast<float*>(out),
+            bias, M, N, K, a.s_row, a.s_k, b.s_row, b.s_k, ldc, act, accumulate, 1.f, 1, 1, 0, 0, 0, 0, 0, 0, status(),
+            cur_stream());
     return;
   }
   if (!a.bf16 && !out_bf16) {

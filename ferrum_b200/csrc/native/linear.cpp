@@ -267,12 +267,101 @@ Tensor linear_act_norm(const Tensor& x, const Tensor& weight, const c10::optiona
   return y;
 }
 
+// ------------------------------------------------------------------------------------- batched products
+// alpha * a b for [Bo, Bi, M, K] x [Bo, Bi, K, N] views (heads interleaved in the feature dimension, transposes):
+// fp32 operands on the fp32 tensor-core kernel with any strides, bf16 ones through 4-D TMA maps.
+bool batched_tma_ok(const Tensor& t) {
+  if (reinterpret_cast<uintptr_t>(t.data_ptr()) % 16) return false;
+  const ll s0 = t.stride(2), s1 = t.stride(3);
+  ll ld;
+  if (s1 == 1) ld = s0 >= t.size(3) ? s0 : 1;
+  else if (s0 == 1) ld = s1 >= t.size(2) ? s1 : 1;
+  else return false;
+  if (ld % 8) return false;
+  for (int d = 0; d < 2; ++d)
+    if (t.size(d) != 1 && (t.stride(d) <= 0 || t.stride(d) % 8)) return false;
+  return true;
+}
+Tensor batched_operand(const Tensor& t, bool low) {
+  if (!low) return cast(t, at::kFloat);
+  Tensor b = cast(t, at::kBFloat16);
+  return batched_tma_ok(b) ? b : b.contiguous();
+}
+// out = alpha * a b^T with a [.., M, K], b [.., N, K]
+void batched_nt(const Tensor& a, const Tensor& b, const Tensor& out, float alpha) {
+  const int M = static_cast<int>(a.size(2)), N = static_cast<int>(b.size(2)), K = static_cast<int>(a.size(3));
+  const int Bo = static_cast<int>(a.size(0)), Bi = static_cast<int>(a.size(1));
+  if (is_f32(a)) {
+    FB_CALL(fb_gemm_f32_tensor, a.data_ptr<float>(), b.data_ptr<float>(), out.data_ptr<float>(), nullptr, M, N, K,
+            a.stride(2), a.stride(3), b.stride(2), b.stride(3), out.stride(2), 0, 0, alpha, Bo, Bi, a.stride(0),
+            a.stride(1), b.stride(0), b.stride(1), out.stride(0), out.stride(1), status(), cur_stream());
+    return;
+  }
+  const int a_mn = a.stride(3) == 1 ? 0 : 1, b_mn = b.stride(3) == 1 ? 0 : 1;
+  FB_CALL(fb_gemm_bf16_batched, a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a_mn ? a.stride(3) : a.stride(2),
+          b_mn ? b.stride(3) : b.stride(2), out.stride(2), Bo, Bi, a.stride(0), a.stride(1), b.stride(0), b.stride(1),
+          out.stride(0), out.stride(1), a_mn, b_mn, 1, 0, alpha, status(), cur_stream());
+}
+Tensor batched_usable(const Tensor& t) { return is_f32(t) || batched_tma_ok(t) ? t : t.contiguous(); }
+
+struct BmmNode : Node {
+  SavedVariable a_, b_;
+  float alpha = 1.f;
+  at::ScalarType da = at::kFloat, db = at::kFloat;
+  std::string name() const override { return "FerrumBmmBackward"; }
+  void release_variables() override {
+    a_.reset_data();
+    b_.reset_data();
+  }
+  variable_list apply(variable_list&& grads) override {
+    NoAutograd below;
+    variable_list out(2);
+    if (!grads[0].defined()) return out;
+    Tensor a = a_.unpack(), b = b_.unpack(), g = batched_operand(grads[0], is_bf16(a));
+    if (task_should_compute_output(0)) {
+      Tensor ga = empty(a.sizes(), a, a.scalar_type());
+      batched_nt(g, b, ga, alpha);
+      out[0] = cast(ga, da);
+    }
+    if (task_should_compute_output(1)) {
+      Tensor gb = empty(b.sizes(), b, b.scalar_type());
+      batched_nt(a.transpose(-1, -2), g.transpose(-1, -2), gb, alpha);
+      out[1] = cast(gb, db);
+    }
+    return out;
+  }
+};
+
+Tensor bmm(const Tensor& a, const Tensor& b, double alpha, bool heads_inner, bool low) {
+  NoAutograd below;
+  TORCH_CHECK_VALUE(a.dim() == 4 && b.dim() == 4 && a.size(0) == b.size(0) && a.size(1) == b.size(1) &&
+                        a.size(3) == b.size(2),
+                    "bmm: [Bo, Bi, M, K] x [Bo, Bi, K, N] expected, got ", a.sizes(), " x ", b.sizes());
+  Tensor ac = batched_operand(a, low), bc = batched_operand(b, low);
+  const auto st = low ? at::kBFloat16 : at::kFloat;
+  const int64_t Bo = a.size(0), Bi = a.size(1), M = a.size(2), N = b.size(3);
+  // heads_inner: stored [Bo, M, Bi, N], so that merging the heads afterwards is a view
+  Tensor y = heads_inner ? empty({Bo, M, Bi, N}, ac, st).permute({0, 2, 1, 3}) : empty({Bo, Bi, M, N}, ac, st);
+  if (y.numel() > 0) batched_nt(ac, batched_usable(bc.transpose(-1, -2)), y, static_cast<float>(alpha));
+  if (wants_grad({&a, &b})) {
+    auto n = make_node<BmmNode>(a, b);
+    n->alpha = static_cast<float>(alpha);
+    n->da = a.scalar_type();
+    n->db = b.scalar_type();
+    n->a_ = SavedVariable(ac, false);
+    n->b_ = SavedVariable(bc, false);
+    torch::autograd::set_history(y, n);
+  }
+  return y;
+}
+
 }  // namespace
 
 void bind_linear(py::module_& m) {
   m.def("linear", &linear);
   m.def("layer_norm", &layer_norm);
   m.def("linear_act_norm", &linear_act_norm);
+  m.def("bmm", &bmm);
   m.def("gemm_nt",  // out = act(a b^T + bias) without a graph; see ops/functional.py
         [](const Tensor& a, const Tensor& b, const c10::optional<Tensor>& bias, int act, const Tensor& out,
            bool accumulate, bool tf32) {

@@ -466,64 +466,15 @@ class _MatmulFn(Function):
         return ga, gb, None
 
 
-class _BmmFn(Function):
-    """Batched fp32 matmul on the SIMT kernel (grid.z = batch)."""
-
-    @staticmethod
-    def forward(ctx, a, b):
-        ctx.save_for_backward(a, b)
-        return _gemm.gemm_f32(a, b.transpose(1, 2))
-
-    @staticmethod
-    def backward(ctx, g):
-        a, b = ctx.saved_tensors
-        g = g.contiguous()
-        ga = _gemm.gemm_f32(g, b) if ctx.needs_input_grad[0] else None
-        gb = _gemm.gemm_f32(a.transpose(1, 2), g.transpose(1, 2)) if ctx.needs_input_grad[1] else None
-        return ga, gb
-
-
-def _bmm_operand(t):
-    t = t if t.dtype == torch.bfloat16 else raw_cast(t, torch.bfloat16)
-    return t if _gemm.batched_operand_ok(t) else t.contiguous()
-
-
-class _BmmLowFn(Function):
-    """Batched ``alpha * a @ b`` over 4-D operands on the tcgen05 kernel (bf16 in, bf16 out, fp32 accumulate);
-    strided views (heads interleaved in the feature dimension, transposes) are consumed without copies."""
-
-    @staticmethod
-    def forward(ctx, a, b, alpha, heads_inner=False):
-        a, b = _bmm_operand(a), _bmm_operand(b)
-        ctx.save_for_backward(a, b)
-        ctx.alpha = alpha
-        bt = b.transpose(-1, -2)
-        out = None
-        if heads_inner:  # result stored [Bo, M, Bi, N] so that merging the heads afterwards is a view
-            Bo, Bi, M, _ = a.shape
-            out = torch.empty((Bo, M, Bi, b.shape[-1]), device=a.device, dtype=torch.bfloat16).permute(0, 2, 1, 3)
-        return _gemm.gemm_bf16_batched(a, bt if _gemm.batched_operand_ok(bt) else bt.contiguous(), out=out,
-                                       alpha=alpha)
-
-    @staticmethod
-    def backward(ctx, g):
-        a, b = ctx.saved_tensors
-        g = _bmm_operand(g)
-        ga = gb = None
-        if ctx.needs_input_grad[0]:   # dA = alpha * g @ b^T
-            ga = _gemm.gemm_bf16_batched(g, b, alpha=ctx.alpha)
-        if ctx.needs_input_grad[1]:   # dB = alpha * a^T @ g
-            gb = _gemm.gemm_bf16_batched(a.transpose(-1, -2), g.transpose(-1, -2), alpha=ctx.alpha)
-        return ga, gb, None, None
-
-
 def bmm_scaled(a: torch.Tensor, b: torch.Tensor, alpha: float = 1.0, heads_inner: bool = False) -> torch.Tensor:
     """``alpha * a @ b`` for 4-D ``[Bo, Bi, M, K] @ [Bo, Bi, K, N]``: tensor cores under autocast for TMA-describable
     operands (feature extents multiples of 8), the fp32 batched kernel otherwise.  ``heads_inner`` stores the
     result as ``[Bo, M, Bi, N]`` (returned as the permuted view)."""
-    if (_native(a) and _native(b) and config.low_precision_active() and a.shape[-1] % 8 == 0
-            and b.shape[-1] % 8 == 0):
-        return _BmmLowFn.apply(a, b, float(alpha), heads_inner)
+    if _native(a) and _native(b):
+        low = config.low_precision_active()
+        if (a.shape[-1] % 8 == 0 and b.shape[-1] % 8 == 0) if low else (
+                a.dtype == b.dtype == torch.float32 and a.shape[:2] == b.shape[:2]):
+            return _lib.native().bmm(a, b, alpha, heads_inner, low)
     out = matmul(a, b)
     return scalar_op(out, "mul", float(alpha)) if alpha != 1.0 else out
 
@@ -671,10 +622,10 @@ def matmul(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     if low and a.shape[-1] % 8 == 0 and b.shape[-1] % 8 == 0:
         a4 = a.expand(*bs, *a.shape[-2:]).reshape(1, -1, *a.shape[-2:])
         b4 = b.expand(*bs, *b.shape[-2:]).reshape(1, -1, *b.shape[-2:])
-        return _BmmLowFn.apply(a4, b4, 1.0).reshape(*bs, a.shape[-2], b.shape[-1])
-    a3 = _f32(a.expand(*bs, *a.shape[-2:]).reshape(-1, *a.shape[-2:]).contiguous())
-    b3 = _f32(b.expand(*bs, *b.shape[-2:]).reshape(-1, *b.shape[-2:]).contiguous())
-    out = _BmmFn.apply(a3, b3)
+        return _lib.native().bmm(a4, b4, 1.0, False, True).reshape(*bs, a.shape[-2], b.shape[-1])
+    a4 = _f32(a.expand(*bs, *a.shape[-2:])).reshape(1, -1, *a.shape[-2:])
+    b4 = _f32(b.expand(*bs, *b.shape[-2:])).reshape(1, -1, *b.shape[-2:])
+    out = _lib.native().bmm(a4, b4, 1.0, False, False)
     return raw_cast(out.reshape(*bs, a.shape[-2], b.shape[-1]), torch.promote_types(a.dtype, b.dtype))
 
 

@@ -1,7 +1,7 @@
 """Raw (non-autograd) GEMM launchers.
 
 ``gemm_bf16``  — the tcgen05/TMEM kernel (``csrc/gemm/tcgen05_gemm.cu``).
-``gemm_f32``   — the fp32 SIMT kernel with arbitrary strides (``csrc/gemm/simt_gemm.cu``).
+``gemm_f32``   — fp32 with arbitrary strides (``csrc/gemm/f32_tensor_gemm.cu``, ``simt_gemm.cu``).
 
 Both compute ``out = act(A @ B^T + bias)`` in the "NT" convention used by
 ``Linear`` (reference forward: ferrum-nn/src/linear.rs:78-89), where operand
@@ -214,8 +214,10 @@ def gemm_bf16_batched(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None
 
 
 def gemm_f32(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None = None, act: str | None = None,
-             out: torch.Tensor | None = None, accumulate: bool = False) -> torch.Tensor:
-    """fp32 ``out = act(a @ b^T + bias)`` with arbitrary strides; ``a``/``b`` may be 2-D or batched 3-D."""
+             out: torch.Tensor | None = None, accumulate: bool = False, simt: bool = False) -> torch.Tensor:
+    """fp32 ``out = act(a @ b^T + bias)`` with arbitrary strides; ``a``/``b`` may be 2-D or batched 3-D.  Runs on the
+    tensor cores with three bf16 parts per operand element, which keeps fp32 precision; ``simt`` selects the fp32
+    multiply-add kernel (short reductions, oracle)."""
     assert a.is_cuda and a.dtype == torch.float32 and b.dtype == torch.float32
     batched = a.dim() == 3
     if batched:
@@ -236,6 +238,12 @@ def gemm_f32(a: torch.Tensor, b: torch.Tensor, bias: torch.Tensor | None = None,
     ldc = out.stride(-2)
     bsc = out.stride(0) if batched else 0
     lib = _lib.cuda()
+    if not simt and K > 32:
+        _lib.check(lib.fb_gemm_f32_tensor(a.data_ptr(), b.data_ptr(), out.data_ptr(),
+                                          bias.data_ptr() if bias is not None else None, M, N, K, sam, sak, sbn, sbk,
+                                          ldc, ACT[act], 1 if accumulate else 0, 1.0, 1, Bt, 0, bsa, 0, bsb, 0, bsc,
+                                          _rt.status_ptr(), _stream()), "fb_gemm_f32_tensor")
+        return out
     rc = lib.fb_gemm_f32_simt(a.data_ptr(), b.data_ptr(), out.data_ptr(),
                               bias.data_ptr() if bias is not None else None, M, N, K, sam, sak, sbk, sbn, ldc,
                               ACT[act], 1 if accumulate else 0, Bt, bsa, bsb, bsc, _stream())
