@@ -69,8 +69,105 @@ Tensor embedding(const Tensor& weight, const Tensor& idx_, ll padding, bool pool
   return y;
 }
 
+// ------------------------------------------------------------------------------------ recurrent sequences
+// One LSTM (gates = 4) or GRU (gates = 3) layer over proj [T, B, gates H]; returns hs [T, B, H] and, for LSTM, the
+// last cell state [B, H].  The recurrence runs in one launch per direction; the weight gradient of all steps is one
+// product over T B rows.
+struct RnnSeqNode : Node {
+  SavedVariable w_, h0_, c0_, hs_;
+  Tensor cs, saved;
+  int gates = 4;
+  bool has_bias = false;
+  std::string name() const override { return "FerrumRnnSeqBackward"; }
+  void release_variables() override {
+    w_.reset_data();
+    h0_.reset_data();
+    c0_.reset_data();
+    hs_.reset_data();
+    cs = saved = Tensor();
+  }
+  variable_list apply(variable_list&& grads) override {
+    NoAutograd below;
+    variable_list out(5);  // proj, w, bias, h0, c0
+    Tensor w = contig(w_.unpack()), h0 = h0_.unpack(), c0 = c0_.unpack(), hs = hs_.unpack(shared_from_this());
+    if (h0.defined()) h0 = f32c(h0);
+    if (c0.defined()) c0 = f32c(c0);
+    Tensor dhs = grads[0].defined() ? f32c(grads[0]) : Tensor();
+    Tensor dc = grads.size() > 1 && grads[1].defined() ? f32c(grads[1]) : Tensor();
+    if (!dhs.defined() && !dc.defined()) return out;
+    const int64_t T = hs.size(0), B = hs.size(1), H = hs.size(2), GH = gates * H;
+    Tensor dxi = empty({T, B, GH}, hs, at::kFloat), dhh = gates == 3 ? empty({T, B, GH}, hs, at::kFloat) : dxi;
+    Tensor dh0 = task_should_compute_output(3) ? empty({B, H}, hs, at::kFloat) : Tensor();
+    Tensor dc0 = gates == 4 && task_should_compute_output(4) ? empty({B, H}, hs, at::kFloat) : Tensor();
+    FB_CALL(fb_rnn_seq_bwd, gates, w.data_ptr<float>(), fptr(h0), fptr(c0), hs.data_ptr<float>(), fptr(cs),
+            saved.data_ptr<float>(), fptr(dhs), fptr(dc), dxi.data_ptr<float>(),
+            gates == 3 ? dhh.data_ptr<float>() : nullptr, fptr_mut(dh0), fptr_mut(dc0), static_cast<int>(T),
+            static_cast<int>(B), static_cast<int>(H), status(), cur_stream());
+    out[0] = dxi;
+    if (task_should_compute_output(1)) {
+      Tensor dw = empty({GH, H}, hs, at::kFloat);
+      const float* d = dhh.data_ptr<float>();
+      const bool first = h0.defined();  // the step from a zero state contributes nothing
+      if (T > 1)
+        gemm(Op{d + B * GH, GH, (T - 1) * B, 1, GH, false}, Op{hs.data_ptr(), H, (T - 1) * B, 1, H, false}, nullptr, 0,
+             dw.data_ptr(), H, false);
+      if (first)
+        gemm(Op{d, GH, B, 1, GH, false}, Op{h0.data_ptr(), H, B, 1, H, false}, nullptr, 0, dw.data_ptr(), H, false,
+             T > 1);
+      if (T == 1 && !first) dw.zero_();
+      out[1] = dw;
+    }
+    if (has_bias && task_should_compute_output(2)) {
+      Tensor db = empty({GH}, hs, at::kFloat);
+      FB_CALL(fb_colsum, dhh.data_ptr(), db.data_ptr<float>(), T * B, GH, FB_DT_F32, 0, cur_stream());
+      out[2] = db;
+    }
+    out[3] = dh0;
+    out[4] = dc0;
+    return out;
+  }
+};
+
+std::vector<Tensor> rnn_seq(int gates, const Tensor& proj, const Tensor& w, const c10::optional<Tensor>& bias_,
+                            const c10::optional<Tensor>& h0_, const c10::optional<Tensor>& c0_) {
+  NoAutograd below;
+  const Tensor bias = bias_.value_or(Tensor()), h0 = h0_.value_or(Tensor()), c0 = c0_.value_or(Tensor());
+  Tensor x = f32c(proj), wc = contig(w);
+  const int64_t T = x.size(0), B = x.size(1), H = wc.size(1), GH = gates * H;
+  TORCH_CHECK_VALUE(x.size(2) == GH && wc.size(0) == GH, "rnn_seq: sizes do not match");
+  Tensor b = bias.defined() ? contig(bias) : bias, h = h0.defined() ? f32c(h0) : h0, c = c0.defined() ? f32c(c0) : c0;
+  const bool grad = wants_grad({&proj, &w, &bias, &h0, &c0});
+  Tensor wt = empty({H, GH}, x, at::kFloat), hs = empty({T, B, H}, x, at::kFloat);
+  Tensor cs = gates == 4 && grad ? empty({T, B, H}, x, at::kFloat) : Tensor();
+  Tensor saved = grad ? empty({T, B, 4 * H}, x, at::kFloat) : Tensor();
+  Tensor c_last = gates == 4 ? empty({B, H}, x, at::kFloat) : Tensor();
+  FB_CALL(fb_transpose_2d, wc.data_ptr(), wt.data_ptr(), static_cast<int>(GH), static_cast<int>(H), 4, cur_stream());
+  FB_CALL(fb_rnn_seq_fwd, gates, x.data_ptr<float>(), wt.data_ptr<float>(), fptr(b), fptr(h), fptr(c),
+          hs.data_ptr<float>(), fptr_mut(cs), fptr_mut(saved), fptr_mut(c_last), static_cast<int>(T),
+          static_cast<int>(B), static_cast<int>(H), status(), cur_stream());
+  std::vector<Tensor> out{hs};
+  if (gates == 4) out.push_back(c_last);
+  if (grad) {
+    auto n = make_node<RnnSeqNode>(proj, w, bias, h0, c0);
+    n->gates = gates;
+    n->has_bias = bias.defined();
+    n->w_ = SavedVariable(w, false);
+    if (h0.defined()) n->h0_ = SavedVariable(h0, false);
+    if (c0.defined()) n->c0_ = SavedVariable(c0, false);
+    n->cs = cs;
+    n->saved = saved;
+    torch::autograd::set_history(out, n);
+    n->hs_ = SavedVariable(out[0], true);
+  }
+  return out;
+}
+
 }  // namespace
 
-void bind_layers(py::module_& m) { m.def("embedding", &embedding); }
+void bind_layers(py::module_& m) {
+  m.def("embedding", &embedding);
+  m.def("rnn_seq", &rnn_seq);
+  m.def("rnn_seq_supported", [](int gates, int batch, int hidden) { return fb_rnn_seq_supported(gates, batch, hidden) != 0; });
+}
 
 }  // namespace fbn

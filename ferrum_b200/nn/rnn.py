@@ -2,8 +2,8 @@
 
 Input is sequence-first ``[T, B, F]``.  The reference executes only layer 0 in the forward direction and computes
 the LSTM / GRU gates on host vectors without autograd; here every layer runs, the per-step projections are GEMMs
-of this package (the input projection of a whole sequence is one GEMM), the gate arithmetic of an LSTM / GRU step
-is one fused kernel forward and one backward, and everything is differentiable.
+of this package (the input projection of a whole sequence is one GEMM), an fp32 LSTM / GRU layer's recurrence is one
+launch per direction (other precisions: one fused gate kernel per step), and everything is differentiable.
 """
 from __future__ import annotations
 
@@ -155,10 +155,15 @@ class RNN(_SeqBase):
         wrapped = isinstance(input, Tensor)
         x = _unwrap(input)
         self._check(x)
-        h0 = _unwrap(h_0) if h_0 is not None else self._zeros(x)
+        fused = self.cell_cls is GRUCell and F.rnn_sequence_ok(3, x, self.cells[0].weight_hh)
+        h0 = _unwrap(h_0) if h_0 is not None else (None if fused else self._zeros(x))
         finals, layer_in = [], x
         for l, cell in enumerate(self.cells):
             proj = cell.input_projection(layer_in)  # one GEMM for the whole sequence
+            if fused:
+                layer_in = F.rnn_sequence(3, proj, cell.weight_hh, cell.bias_hh, None if h0 is None else h0[l])[0]
+                finals.append(layer_in[-1])
+                continue
             h, outs = h0[l], []
             for t in range(x.shape[0]):
                 h = cell.step(proj[t], h)
@@ -191,11 +196,18 @@ class LSTM(_SeqBase):
         wrapped = isinstance(input, Tensor)
         x = _unwrap(input)
         self._check(x)
-        h0 = _unwrap(hx[0]) if hx is not None else self._zeros(x)
-        c0 = _unwrap(hx[1]) if hx is not None else self._zeros(x)
+        fused = F.rnn_sequence_ok(4, x, self.cells[0].weight_hh)
+        h0 = _unwrap(hx[0]) if hx is not None else (None if fused else self._zeros(x))
+        c0 = _unwrap(hx[1]) if hx is not None else (None if fused else self._zeros(x))
         hs, cs, layer_in = [], [], x
         for l, cell in enumerate(self.cells):
             proj = cell.input_projection(layer_in)
+            if fused:
+                layer_in, c = F.rnn_sequence(4, proj, cell.weight_hh, cell.bias_hh, None if h0 is None else h0[l],
+                                             None if c0 is None else c0[l])
+                hs.append(layer_in[-1])
+                cs.append(c)
+                continue
             h, c, outs = h0[l], c0[l], []
             for t in range(x.shape[0]):
                 h, c = cell.step(proj[t], h, c)

@@ -1013,6 +1013,20 @@ def gru_gates(xi, hh, h_prev):
     return (1 - z) * n + z * h_prev
 
 
+def rnn_sequence_ok(gates: int, x: torch.Tensor, weight_hh: torch.Tensor) -> bool:
+    """True when a whole layer's recurrence over ``x [T, B, F]`` can run in one launch per direction
+    (csrc/kernels/rnn_seq.cu): fp32 on the GPU, the recurrent matrix within a cluster's shared memory."""
+    return (x.is_cuda and x.dtype == weight_hh.dtype == torch.float32 and x.shape[0] > 0 and x.shape[1] > 0
+            and not config.low_precision_active() and not config.tf32_active()
+            and _lib.native().rnn_seq_supported(gates, x.shape[1], weight_hh.shape[1]))
+
+
+def rnn_sequence(gates: int, proj, weight_hh, bias_hh, h0=None, c0=None):
+    """``[hs]`` (GRU, gates = 3) or ``[hs, c_last]`` (LSTM, gates = 4) from the input projections ``[T, B, gates H]``;
+    absent initial states are zero."""
+    return _lib.native().rnn_seq(gates, proj, weight_hh, bias_hh, h0, c0)
+
+
 def conv_out_size(size, k, stride, pad, dil):
     return (size + 2 * pad - dil * (k - 1) - 1) // stride + 1
 

@@ -1,0 +1,50 @@
+"""Whole-sequence LSTM / GRU kernels against torch's fp64 recurrence, at the edges of their plans.
+
+Bound: fp32 sums over at most a few hundred terms per step and a contracting recurrence: 2e-5 of each result's norm."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kind", ["LSTM", "GRU"])
+@pytest.mark.parametrize("T,B,I,H,L,state", [(1, 1, 3, 8, 1, False), (1, 3, 5, 40, 1, True), (5, 33, 7, 33, 2, True),
+                                             (9, 130, 16, 64, 1, False), (4, 37, 12, 257, 1, True),
+                                             (3, 150, 8, 512, 1, True), (6, 2, 8, 376, 2, False)])
+def test_sequence(kind, T, B, I, H, L, state):
+    import ferrum_b200 as fb
+    from ferrum_b200 import nn
+
+    torch.manual_seed(T + B + H)
+    m = getattr(nn, kind)(I, H, L, device=fb.Device.Cuda(0))
+    assert fb.ops.functional.rnn_sequence_ok(4 if kind == "LSTM" else 3, torch.empty(T, B, I, device="cuda"),
+                                             m.cells[0].weight_hh)
+    ref = getattr(torch.nn, kind)(I, H, L, device="cuda", dtype=torch.float64)
+    with torch.no_grad():
+        for l, c in enumerate(m.cells):
+            for n in ("weight_ih", "weight_hh", "bias_ih", "bias_hh"):
+                getattr(ref, f"{n}_l{l}").copy_(getattr(c, n))
+    x = torch.randn(T, B, I, device="cuda", requires_grad=True)
+    h0 = torch.randn(L, B, H, device="cuda", requires_grad=True) if state else None
+    c0 = torch.randn(L, B, H, device="cuda", requires_grad=True) if state and kind == "LSTM" else None
+    xd, hd, cd = (t.detach().double().requires_grad_(True) if t is not None else None for t in (x, h0, c0))
+    if kind == "LSTM":
+        y, (hn, cn) = m.forward_seq(x, (h0, c0) if state else None)
+        yr, (hr, cr) = ref(xd, (hd, cd) if state else None)
+    else:
+        y, hn = m.forward_seq(x, h0)
+        yr, hr = ref(xd, hd)
+        cn, cr = hn, hr
+    g = torch.randn_like(y)
+    ((y * g).sum() + (hn * 0.5).sum() + (cn * 0.3).sum()).backward()
+    ((yr * g.double()).sum() + (hr * 0.5).sum() + (cr * 0.3).sum()).backward()
+    pairs = [(y, yr), (hn, hr), (cn, cr), (x.grad, xd.grad)]
+    pairs += [(t.grad, r.grad) for t, r in ((h0, hd), (c0, cd)) if t is not None]
+    for l, c in enumerate(m.cells):
+        pairs += [(getattr(c, n).grad, getattr(ref, f"{n}_l{l}").grad) for n in
+                  ("weight_ih", "weight_hh", "bias_ih", "bias_hh")]
+    for got, want in pairs:
+        assert (got.double() - want).norm() <= 2e-5 * want.norm() + 1e-6
+    with torch.no_grad():
+        again = m.forward_seq(x.detach(), None if not state else ((h0, c0) if kind == "LSTM" else h0))[0]
+    assert torch.equal(again, y)
