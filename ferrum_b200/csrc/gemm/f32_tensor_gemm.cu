@@ -18,6 +18,12 @@
 // Infinities, NaNs and values that would round to infinity do not survive the split (inf - inf, 0 * inf) and always
 // end in a result that is not finite; such a result is computed again with fp32 multiply-adds when the tile is written.
 //
+// bf16 operands whose rows a TMA map cannot describe (a pitch that is no multiple of 16 bytes, an odd base) take the
+// same kernel with one plane and one product: no padded copies, no fp32 copies.  Rows at any 2-byte address are read
+// with aligned 16-byte loads and shifted into place; the loads and the shifts bound it, not the MMAs.  Against fp32
+// copies on the multiply-add kernel: 777 x 1001 x 1001 23 instead of 148 us, 8191 x 4095 x 4095 1.3 (both K-major) to
+// 1.8 ms (both row-major) instead of 12.4; relative error 9e-8 instead of 2.5e-7 at K = 1001.
+//
 // The issue of a k-block's MMAs takes as long as the MMAs themselves (the queue is short), so it has a warp of its own;
 // a loader warp that issued them held up the next stage (5200 instead of 2300 cycles per k-block).
 #include <cooperative_groups.h>
@@ -40,14 +46,33 @@ constexpr int kBM = 128;
 constexpr int kLoaders = 512;
 constexpr int kThreads = kLoaders + 32;  // 16 warps load, split, add up and write; one issues the MMAs
 
-template <int BN>
+// The element type of the operands: fp32 in three bf16 planes, or bf16 in one.
+template <typename T>
+struct El;
+template <>
+struct El<float> {
+  struct Piece {
+    float v[8];
+  };
+  static constexpr int kPlanes = 3, kProducts = 6;
+};
+template <>
+struct El<__nv_bfloat16> {
+  struct Piece {
+    uint32_t w[8];  // as loaded: words, the two words that cover a piece at an odd address, or single elements
+    uint32_t off;   // byte offset of the piece in w
+  };
+  static constexpr int kPlanes = 1, kProducts = 1;
+};
+
+template <typename T, int BN>
 struct Cfg {
-  static constexpr int kBK = 64;                   // fp32 elements of K per stage
+  static constexpr int kBK = 64;                   // elements of K per stage
   static constexpr int kRow = kBK * 2;             // bytes of a row of a bf16 plane = its swizzle width
   static constexpr int kPieces = kBK / 8;          // 8-element pieces per row
   static constexpr int kPlaneA = kBM * kRow, kPlaneB = BN * kRow;
-  static constexpr int kStage = 3 * (kPlaneA + kPlaneB);
-  static constexpr int kStages = BN == 64 ? 3 : 2;
+  static constexpr int kStage = El<T>::kPlanes * (kPlaneA + kPlaneB);
+  static constexpr int kStages = El<T>::kPlanes == 1 ? 4 : BN == 64 ? 3 : 2;
   static constexpr int kPitch = BN + 4;   // floats per row of the tile in shared memory: conflict-free 16-byte rows
   static constexpr int kTile = kBM * kPitch * 4;
   static constexpr int kBody = kStages * kStage > kTile ? kStages * kStage : kTile;
@@ -65,9 +90,10 @@ struct Cfg {
 };
 
 struct Operand {
-  const float* p;
+  const void* p;
   long long s_row, s_k, s_bo, s_bi;  // element strides; slices of the batch (outer, inner)
   int rows;
+  uintptr_t end;                     // address past the last element
 };
 
 // How an operand lies in memory: K contiguous with 16-byte aligned rows (two vector loads per piece), K contiguous
@@ -76,11 +102,11 @@ enum Layout { kVecK = 0, kScalarK = 1, kRowFast = 2 };
 
 struct Args {
   Operand a, b;
-  float* out;
+  void* out;
   const float* bias;
   long long ldc, sc_bo, sc_bi;
   int M, N, K;
-  int act, beta;
+  int act, beta, out_bf16;
   float alpha;
   int batch_inner;
   int kb_total, kb_per_split;
@@ -118,7 +144,8 @@ __device__ __forceinline__ void piece(int c, int& row, int& kc) {
 // without a condition and stay in flight until they are split; only the last k-block of a ragged K is guarded.
 template <int ROWS, int L, int PIECES>
 __device__ __forceinline__ void load_piece(const Operand& o, const float* base, int row0, int k0, int K, int c,
-                                           float (&v)[8]) {
+                                           El<float>::Piece& out) {
+  float(&v)[8] = out.v;
   int row, kc;
   piece<ROWS, L, PIECES>(c, row, kc);
   const int r = min(row0 + row, o.rows - 1), k = k0 + kc * 8;
@@ -147,6 +174,53 @@ __device__ __forceinline__ void load_piece(const Operand& o, const float* base, 
   }
 }
 
+__device__ __forceinline__ uint32_t u16_at(const __nv_bfloat16* p) {
+  return __ldg(reinterpret_cast<const unsigned short*>(p));
+}
+
+// The same for bf16.  A row at an odd address: the two aligned 16-byte words that cover the piece, if both lie inside
+// the operand; element by element at the operand's first and last bytes.  Words are kept as they arrive and put
+// together when they are stored, so that nothing waits for a load here.
+template <int ROWS, int L, int PIECES>
+__device__ __forceinline__ void load_piece(const Operand& o, const __nv_bfloat16* base, int row0, int k0, int K, int c,
+                                           El<__nv_bfloat16>::Piece& v) {
+  int row, kc;
+  piece<ROWS, L, PIECES>(c, row, kc);
+  const int r = min(row0 + row, o.rows - 1), k = k0 + kc * 8;
+  const __nv_bfloat16* p = base + r * o.s_row + k * o.s_k;
+  auto quad = [&](int i, uintptr_t at) {
+    const uint4 x = __ldg(reinterpret_cast<const uint4*>(at));
+    v.w[i] = x.x; v.w[i + 1] = x.y; v.w[i + 2] = x.z; v.w[i + 3] = x.w;
+  };
+  const bool whole = k0 + PIECES * 8 <= K;
+  if (L == kVecK && whole) {
+    quad(0, reinterpret_cast<uintptr_t>(p));
+  } else if (L == kRowFast) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v.w[j] = 0;
+      if (whole || k + j < K) v.w[j] = u16_at(p + j * o.s_k);
+    }
+  } else {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(p), lo = at & ~uintptr_t(15);
+    if (L == kScalarK && whole && lo >= reinterpret_cast<uintptr_t>(o.p) && lo + 32 <= o.end) {
+      quad(0, lo);
+      quad(4, lo + 16);
+      v.off = static_cast<uint32_t>(at & 15);
+    } else {
+      uint32_t e[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        e[j] = 0;
+        if (whole || k + j < K) e[j] = u16_at(p + j);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v.w[j] = e[2 * j] | e[2 * j + 1] << 16;
+      v.off = 0;
+    }
+  }
+}
+
 __device__ __forceinline__ float2 sub2(float2 x, float2 y) {  // x - y with one packed instruction: y * -1 is exact
   float2 r;
   asm("{\n.reg .b64 a, b, c, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmov.b64 c, {%6, %6};\n"
@@ -171,7 +245,9 @@ __device__ __forceinline__ float2 wide_pair(uint32_t w) {
 }
 
 // Splits eight values and stores them into the three planes.
-__device__ __forceinline__ void store_piece(uint32_t at, uint32_t plane_bytes, const float (&v)[8]) {
+template <int L>
+__device__ __forceinline__ void store_piece(uint32_t at, uint32_t plane_bytes, const El<float>::Piece& in) {
+  const float(&v)[8] = in.v;
   uint32_t w0[4], w1[4], w2[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -186,9 +262,28 @@ __device__ __forceinline__ void store_piece(uint32_t at, uint32_t plane_bytes, c
   ptx::st_shared_v4(at + 2 * plane_bytes, w2[0], w2[1], w2[2], w2[3]);
 }
 
-template <int BN, int LA, int LB>
-__global__ void __launch_bounds__(kThreads, 1) gemm_f32_tensor_kernel(const __grid_constant__ Args p) {
-  using C = Cfg<BN>;
+template <int L>
+__device__ __forceinline__ void store_piece(uint32_t at, uint32_t, const El<__nv_bfloat16>::Piece& v) {
+  if constexpr (L == kVecK) {
+    ptx::st_shared_v4(at, v.w[0], v.w[1], v.w[2], v.w[3]);
+  } else if constexpr (L == kRowFast) {
+    ptx::st_shared_v4(at, v.w[0] | v.w[1] << 16, v.w[2] | v.w[3] << 16, v.w[4] | v.w[5] << 16, v.w[6] | v.w[7] << 16);
+  } else {
+    uint32_t t[6], s[5];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) t[i] = v.off & 8 ? v.w[i + 2] : v.w[i];
+#pragma unroll
+    for (int i = 0; i < 5; ++i) s[i] = v.off & 4 ? t[i + 1] : t[i];
+    const uint32_t sh = (v.off & 2) * 8;
+    ptx::st_shared_v4(at, __funnelshift_r(s[0], s[1], sh), __funnelshift_r(s[1], s[2], sh),
+                      __funnelshift_r(s[2], s[3], sh), __funnelshift_r(s[3], s[4], sh));
+  }
+}
+
+template <typename T, int BN, int LA, int LB>
+__global__ void __launch_bounds__(kThreads, 1) gemm_split_kernel(const __grid_constant__ Args p) {
+  using C = Cfg<T, BN>;
+  constexpr int kPlanes = El<T>::kPlanes;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + C::kBody);
@@ -204,9 +299,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_tensor_kernel(const __gr
 
   const int n0 = static_cast<int>(blockIdx.x / splits) * BN, m0 = static_cast<int>(blockIdx.y) * kBM;
   const int bo = static_cast<int>(blockIdx.z) / p.batch_inner, bi = static_cast<int>(blockIdx.z) % p.batch_inner;
-  const float* a = p.a.p + bo * p.a.s_bo + bi * p.a.s_bi;
-  const float* b = p.b.p + bo * p.b.s_bo + bi * p.b.s_bi;
-  float* out = p.out + bo * p.sc_bo + bi * p.sc_bi;
+  const T* a = static_cast<const T*>(p.a.p) + bo * p.a.s_bo + bi * p.a.s_bi;
+  const T* b = static_cast<const T*>(p.b.p) + bo * p.b.s_bo + bi * p.b.s_bi;
+  const long long out_at = bo * p.sc_bo + bi * p.sc_bi;
 
   const int kb_lo = min(p.kb_total, rank * p.kb_per_split), kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
   const int nkb = kb_hi - kb_lo;
@@ -236,7 +331,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_tensor_kernel(const __gr
   if (warp < kLoaders / 32) {
     // -------------------------------------------------------- load, split, add up
     constexpr int kPA = kBM * C::kPieces / kLoaders;  // pieces of A per thread; the rest are B's
-    float v[C::kPerThread][8];
+    typename El<T>::Piece v[C::kPerThread];
     auto fetch = [&](int i, int kb) {
       const int k0 = kb * C::kBK;
       if (i < kPA)
@@ -286,17 +381,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_tensor_kernel(const __gr
         ok = false;
         break;
       }
-      const uint32_t sa = ptx::smem_u32(smem + s * C::kStage), sb = sa + 3 * C::kPlaneA;
+      const uint32_t sa = ptx::smem_u32(smem + s * C::kStage), sb = sa + kPlanes * C::kPlaneA;
       const bool more = kb + 1 < nkb;
 #pragma unroll
       for (int i = 0; i < C::kPerThread; ++i) {
         int row, kc;
         if (i < kPA) {
           piece<kBM, LA, C::kPieces>(i * kLoaders + threadIdx.x, row, kc);
-          store_piece(sa + C::at(row, kc), C::kPlaneA, v[i]);
+          store_piece<LA>(sa + C::at(row, kc), C::kPlaneA, v[i]);
         } else {
           piece<BN, LB, C::kPieces>((i - kPA) * kLoaders + threadIdx.x, row, kc);
-          store_piece(sb + C::at(row, kc), C::kPlaneB, v[i]);
+          store_piece<LB>(sb + C::at(row, kc), C::kPlaneB, v[i]);
         }
         if (more) fetch(i, kb_lo + kb + 1);
       }
@@ -320,16 +415,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_tensor_kernel(const __gr
         break;
       }
       ptx::tc_fence_after();
-      const uint32_t sa = ptx::smem_u32(smem + s * C::kStage), sb = sa + 3 * C::kPlaneA;
+      const uint32_t sa = ptx::smem_u32(smem + s * C::kStage), sb = sa + kPlanes * C::kPlaneA;
       const uint32_t d = tmem + buf * BN;
       constexpr int ia[6] = {2, 0, 1, 1, 0, 0}, ib[6] = {0, 2, 1, 0, 1, 0};  // small products first
+      constexpr int kFirst = 6 - El<T>::kProducts;
 #pragma unroll
-      for (int q = 0; q < 6; ++q) {
+      for (int q = kFirst; q < 6; ++q) {
 #pragma unroll
         for (int k = 0; k < C::kBK / 16; ++k) {
           const uint64_t ad = C::desc(sa + ia[q] * C::kPlaneA + k * 32);
           const uint64_t bd = C::desc(sb + ib[q] * C::kPlaneB + k * 32);
-          ptx::umma_f16(d, ad, bd, idesc, (q | k) != 0 ? 1u : 0u);
+          ptx::umma_f16(d, ad, bd, idesc, (q != kFirst || k != 0) ? 1u : 0u);
         }
       }
       ptx::umma_commit(&empty_bar[s]);
@@ -349,7 +445,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_tensor_kernel(const __gr
   }
   cluster.sync();
   const int rows_per = kBM / splits;
-  const bool vec = p.N % 4 == 0 && p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+  const int esz = p.out_bf16 ? 2 : 4;
+  const bool vec = p.N % 4 == 0 && p.ldc % 4 == 0 && out_at % 4 == 0 && reinterpret_cast<uintptr_t>(p.out) % (4 * esz) == 0;
   constexpr int kVec = BN / 4;
   for (int i = threadIdx.x; i < rows_per * kVec; i += kThreads) {
     const int row = rank * rows_per + i / kVec, c = (i % kVec) * 4;
@@ -360,15 +457,16 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_tensor_kernel(const __gr
       const float4 t = *reinterpret_cast<const float4*>(cluster.map_shared_rank(tile, r) + row * C::kPitch + c);
       f[0] += t.x; f[1] += t.y; f[2] += t.z; f[3] += t.w;
     }
-    for (int j = 0; j < 4; ++j) {
-      if (fabsf(f[j]) <= FLT_MAX || n + j >= p.N) continue;
-      // not finite: an operand that does not survive the split, or a result that is not finite in fp32 either
-      float s = 0.f;
-      for (int k = 0; k < p.K; ++k)
-        s = fmaf(a[m * p.a.s_row + k * p.a.s_k], b[(n + j) * p.b.s_row + k * p.b.s_k], s);
-      f[j] = s;
+    if constexpr (kPlanes > 1) {
+      for (int j = 0; j < 4; ++j) {
+        if (fabsf(f[j]) <= FLT_MAX || n + j >= p.N) continue;
+        // not finite: an operand that does not survive the split, or a result that is not finite in fp32 either
+        float s = 0.f;
+        for (int k = 0; k < p.K; ++k)
+          s = fmaf(a[m * p.a.s_row + k * p.a.s_k], b[(n + j) * p.b.s_row + k * p.b.s_k], s);
+        f[j] = s;
+      }
     }
-    float* o = out + m * p.ldc + n;
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (n + j < p.N) {
@@ -376,6 +474,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_tensor_kernel(const __gr
         if (p.bias != nullptr) x += __ldg(p.bias + n + j);
         f[j] = act_f(x, p.act);
       }
+    const long long at = out_at + m * p.ldc + n;
+    if (p.out_bf16) {
+      __nv_bfloat16* o = static_cast<__nv_bfloat16*>(p.out) + at;
+      if (vec) {
+        *reinterpret_cast<uint2*>(o) = make_uint2(bf16_pair(make_float2(f[0], f[1])), bf16_pair(make_float2(f[2], f[3])));
+      } else {
+        for (int j = 0; j < 4 && n + j < p.N; ++j) o[j] = __float2bfloat16_rn(f[j]);
+      }
+      continue;
+    }
+    float* o = static_cast<float*>(p.out) + at;
     if (vec) {
       float4 x = make_float4(f[0], f[1], f[2], f[3]);
       if (p.beta) {
@@ -405,12 +514,13 @@ int sm_count() {
   return n;
 }
 
-template <int BN, int LA, int LB>
+template <typename T, int BN, int LA, int LB>
 int launch_one(const Args& args, int batch, int splits, cudaStream_t st) {
+  constexpr int kSmem = Cfg<T, BN>::kSmem;
   static bool configured = false;
   if (!configured) {
     const cudaError_t e =
-        cudaFuncSetAttribute(gemm_f32_tensor_kernel<BN, LA, LB>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::kSmem);
+        cudaFuncSetAttribute(gemm_split_kernel<T, BN, LA, LB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
     if (e != cudaSuccess) return static_cast<int>(e);
     configured = true;
   }
@@ -418,7 +528,7 @@ int launch_one(const Args& args, int batch, int splits, cudaStream_t st) {
   cfg.gridDim = dim3(static_cast<unsigned>((args.N + BN - 1) / BN * splits), static_cast<unsigned>((args.M + kBM - 1) / kBM),
                      static_cast<unsigned>(batch));
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = Cfg<BN>::kSmem;
+  cfg.dynamicSmemBytes = kSmem;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -426,45 +536,49 @@ int launch_one(const Args& args, int batch, int splits, cudaStream_t st) {
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, gemm_f32_tensor_kernel<BN, LA, LB>, args));
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, gemm_split_kernel<T, BN, LA, LB>, args));
 }
 
-template <int BN, int LA>
+template <typename T, int BN, int LA>
 int launch_b(int lb, const Args& args, int batch, int splits, cudaStream_t st) {
-  if (lb == kVecK) return launch_one<BN, LA, kVecK>(args, batch, splits, st);
-  if (lb == kScalarK) return launch_one<BN, LA, kScalarK>(args, batch, splits, st);
-  return launch_one<BN, LA, kRowFast>(args, batch, splits, st);
+  if (lb == kVecK) return launch_one<T, BN, LA, kVecK>(args, batch, splits, st);
+  if (lb == kScalarK) return launch_one<T, BN, LA, kScalarK>(args, batch, splits, st);
+  return launch_one<T, BN, LA, kRowFast>(args, batch, splits, st);
 }
-template <int BN>
+template <typename T, int BN>
 int launch(int la, int lb, const Args& args, int batch, int splits, cudaStream_t st) {
-  if (la == kVecK) return launch_b<BN, kVecK>(lb, args, batch, splits, st);
-  if (la == kScalarK) return launch_b<BN, kScalarK>(lb, args, batch, splits, st);
-  return launch_b<BN, kRowFast>(lb, args, batch, splits, st);
+  if (la == kVecK) return launch_b<T, BN, kVecK>(lb, args, batch, splits, st);
+  if (la == kScalarK) return launch_b<T, BN, kScalarK>(lb, args, batch, splits, st);
+  return launch_b<T, BN, kRowFast>(lb, args, batch, splits, st);
 }
 
-int layout_of(const float* p, long long s_row, long long s_k, long long s_bo, long long s_bi) {
-  if (s_k == 1)
-    return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && s_row % 4 == 0 && s_bo % 4 == 0 && s_bi % 4 == 0 ? kVecK : kScalarK;
-  return kRowFast;
+template <typename T>
+int layout_of(const Operand& o) {
+  constexpr int kUnit = 16 / sizeof(T);
+  if (o.s_k != 1) return kRowFast;
+  return reinterpret_cast<uintptr_t>(o.p) % 16 == 0 && o.s_row % kUnit == 0 && o.s_bo % kUnit == 0 && o.s_bi % kUnit == 0
+             ? kVecK
+             : kScalarK;
 }
 
-}  // namespace
-}  // namespace fb
-
-using namespace fb;
-
-extern "C" int fb_gemm_f32_tensor(const float* a, const float* b, float* out, const float* bias, int M, int N, int K,
-                                  long long sam, long long sak, long long sbn, long long sbk, long long ldc, int act,
-                                  int beta, float alpha, int batch_outer, int batch_inner, long long sa_outer,
-                                  long long sa_inner, long long sb_outer, long long sb_inner, long long sc_outer,
-                                  long long sc_inner, int32_t* status, cudaStream_t stream) {
+// Strides as the callers give them: a (rows M), b (rows N); K, batch and output strides.
+template <typename T>
+int gemm_split(const T* a, const T* b, void* out, int out_bf16, const float* bias, int M, int N, int K, long long sam,
+               long long sak, long long sbn, long long sbk, long long ldc, int act, int beta, float alpha,
+               int batch_outer, int batch_inner, long long sa_outer, long long sa_inner, long long sb_outer,
+               long long sb_inner, long long sc_outer, long long sc_inner, int32_t* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || batch_outer <= 0 || batch_inner <= 0) return 0;
   const long long batch = static_cast<long long>(batch_outer) * batch_inner;
   if (K < 0 || batch > 65535 || (M + kBM - 1) / kBM > 65535) return -1;
+  auto operand = [&](const T* p, int rows, long long s_row, long long s_k, long long s_bo, long long s_bi) {
+    const long long last = (rows - 1) * s_row + (K > 0 ? K - 1 : 0) * s_k + (batch_outer - 1) * s_bo + (batch_inner - 1) * s_bi;
+    return Operand{p, s_row, s_k, s_bo, s_bi, rows, reinterpret_cast<uintptr_t>(p + last + 1)};
+  };
   Args g;
-  g.a = Operand{a, sam, sak, sa_outer, sa_inner, M};
-  g.b = Operand{b, sbn, sbk, sb_outer, sb_inner, N};
+  g.a = operand(a, M, sam, sak, sa_outer, sa_inner);
+  g.b = operand(b, N, sbn, sbk, sb_outer, sb_inner);
   g.out = out;
+  g.out_bf16 = out_bf16;
   g.bias = bias;
   g.ldc = ldc;
   g.sc_bo = sc_outer;
@@ -478,18 +592,41 @@ extern "C" int fb_gemm_f32_tensor(const float* a, const float* b, float* out, co
   g.batch_inner = batch_inner;
   g.status = status;
   g.timeout_ns = 2000000000ull;
-    // Tile width and K splits: the wide tile where it alone fills the chip, else the narrow one; then as many splits
+  // Tile width and K splits: the wide tile where it alone fills the chip, else the narrow one; then as many splits
   // as there are idle SMs, each with at least one k-block.
   const long long tm = (M + kBM - 1) / kBM;
   const long long wide = tm * ((N + 127) / 128) * batch, narrow = tm * ((N + 63) / 64) * batch;
-  const int bk_wide = Cfg<128>::kBK;
+  constexpr int kBK = Cfg<T, 128>::kBK;
   const bool use_wide = N > 64 && wide * 8 > sm_count() && wide * (K + 127) / 128 >= sm_count();
   const long long tiles = use_wide ? wide : narrow;
-  g.kb_total = (K + (use_wide ? bk_wide : Cfg<64>::kBK) - 1) / (use_wide ? bk_wide : Cfg<64>::kBK);
+  g.kb_total = (K + kBK - 1) / kBK;
   int splits = 1;
   while (splits < 8 && tiles * splits * 2 <= sm_count() && splits * 2 <= g.kb_total) splits *= 2;
   g.kb_per_split = (g.kb_total + splits - 1) / splits;
-  const int la = layout_of(a, sam, sak, sa_outer, sa_inner), lb = layout_of(b, sbn, sbk, sb_outer, sb_inner);
-  return use_wide ? launch<128>(la, lb, g, static_cast<int>(batch), splits, stream)
-                  : launch<64>(la, lb, g, static_cast<int>(batch), splits, stream);
+  const int la = layout_of<T>(g.a), lb = layout_of<T>(g.b);
+  return use_wide ? launch<T, 128>(la, lb, g, static_cast<int>(batch), splits, stream)
+                  : launch<T, 64>(la, lb, g, static_cast<int>(batch), splits, stream);
+}
+
+}  // namespace
+}  // namespace fb
+
+using namespace fb;
+
+extern "C" int fb_gemm_f32_tensor(const float* a, const float* b, float* out, const float* bias, int M, int N, int K,
+                                  long long sam, long long sak, long long sbn, long long sbk, long long ldc, int act,
+                                  int beta, float alpha, int batch_outer, int batch_inner, long long sa_outer,
+                                  long long sa_inner, long long sb_outer, long long sb_inner, long long sc_outer,
+                                  long long sc_inner, int32_t* status, cudaStream_t stream) {
+  return gemm_split<float>(a, b, out, 0, bias, M, N, K, sam, sak, sbn, sbk, ldc, act, beta, alpha, batch_outer,
+                           batch_inner, sa_outer, sa_inner, sb_outer, sb_inner, sc_outer, sc_inner, status, stream);
+}
+
+extern "C" int fb_gemm_bf16_any(const void* a, const void* b, void* out, const float* bias, int M, int N, int K,
+                                long long sam, long long sak, long long sbn, long long sbk, long long ldc, int out_bf16,
+                                int act, int beta, int32_t* status, cudaStream_t stream) {
+  if (out_bf16 && beta) return -1;
+  return gemm_split<__nv_bfloat16>(static_cast<const __nv_bfloat16*>(a), static_cast<const __nv_bfloat16*>(b), out,
+                                   out_bf16, bias, M, N, K, sam, sak, sbn, sbk, ldc, act, beta, 1.f, 1, 1, 0, 0, 0, 0, 0,
+                                   0, status, stream);
 }

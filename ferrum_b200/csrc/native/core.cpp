@@ -117,6 +117,11 @@ void gemm(const Op& a, const Op& b, const float* bias, int act, void* out, ll ld
               bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, act, accumulate, g_max_ctas, status(), cur_stream());
     return;
   }
+  if (a.bf16 && b.bf16 && !(out_bf16 && accumulate)) {  // operands that a TMA map cannot describe
+    FB_CALL(fb_gemm_bf16_any, a.p, b.p, out, bias, M, N, K, a.s_row, a.s_k, b.s_row, b.s_k, ldc, out_bf16, act,
+            accumulate, status(), cur_stream());
+    return;
+  }
   if (!a.bf16 && !out_bf16 && K > kSimtK) {
     FB_CALL(fb_gemm_f32_tensor, static_cast<const float*>(a.p), static_cast<const float*>(b.p), static_cast<float*>(out),
             bias, M, N, K, a.s_row, a.s_k, b.s_row, b.s_k, ldc, act, accumulate, 1.f, 1, 1, 0, 0, 0, 0, 0, 0, status(),
