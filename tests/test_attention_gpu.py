@@ -159,6 +159,30 @@ def test_flash_attention_forward_matches_softmax_attention(B, H, Sq, Skv, D):
     assert out.permute(0, 2, 1, 3).is_contiguous()  # stored [B, Sq, H, D]
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("B,H,Sq,Skv", [(4, 20, 300, 333), (1, 30, 700, 900), (150, 1, 100, 129), (1, 19, 1025, 1025),
+                                        (1, 149, 1, 1)])
+def test_flash_attention_two_query_tiles_per_block(B, H, Sq, Skv, causal, D):
+    """More query tiles than SMs: blocks own two tiles; odd tile counts leave the last block half empty.  Bound: bf16
+    probabilities and a bf16 result, 2^-9 each of values below 4, against the same softmax in fp64."""
+    from ferrum_b200.ops import functional as F
+    from ferrum_b200.utils.runtime import check_status
+
+    g = torch.Generator(device="cuda").manual_seed(Sq + Skv)
+    q = torch.randn(B, H, Sq, D, device="cuda", generator=g).bfloat16()
+    k, v = (torch.randn(B, H, Skv, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    out, lse = F.flash_attention(q, k, v, D ** -0.5, return_lse=True, causal=causal)
+    check_status()
+    s = (q.double() @ k.double().transpose(-1, -2)) * D ** -0.5
+    if causal:
+        i, j = torch.arange(Sq, device="cuda")[:, None], torch.arange(Skv, device="cuda")[None, :]
+        s = s.masked_fill(j > i + (Skv - Sq), float("-inf"))
+    ref = torch.softmax(s, -1) @ v.double()
+    assert (out.double() - ref).abs().max().item() < 2 * 2.0 ** -9 * 4 + 1e-3
+    assert torch.allclose(lse.double(), torch.logsumexp(s, -1), atol=2e-3, rtol=1e-4)
+
+
 def test_attention_module_uses_the_blockwise_kernel_without_gradients():
     import ferrum_b200 as fb
     from ferrum_b200 import _lib, nn
