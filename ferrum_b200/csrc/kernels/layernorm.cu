@@ -222,7 +222,10 @@ __device__ __forceinline__ void ld_pairs_f32(const float* p, float2 (&o)[4]);
 // all K loads are issued back to back (up to 8 KB in flight per warp), the statistics are one pass of shifted sums
 // (x - c with c = the row's first element) reduced by warp shuffles, and there is no block barrier at all: warps
 // stream rows independently.  Packed fp32x2 arithmetic; gamma / beta come through L1.
-template <int K>
+// W > 1, few rows: a block per row.  Latency is all there is then, so W warps find the same statistics (the same sums in
+// the same order: the same bits) and each writes the vectors k % W of its number, whose gamma and beta it asks for
+// beforehand.
+template <int K, int W = 1>
 __global__ void __launch_bounds__(256, 2)
 ln_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
                    __nv_bfloat16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out,
@@ -230,8 +233,11 @@ ln_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
   const int lane = threadIdx.x & 31;
   const int nvec = cols >> 3;
   const float inv_n = 1.f / static_cast<float>(cols);
-  const long long warp_id = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const long long nwarps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
+  const int part = W > 1 ? threadIdx.x >> 5 : 0;
+  const long long warp_id = W > 1 ? blockIdx.x : (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const long long nwarps = W > 1 ? gridDim.x : (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
+  constexpr int kOwn = W > 1 ? K / W : 1;
+  float2 own_g[kOwn][4], own_b[kOwn][4];
   for (long long row = warp_id; row < rows; row += nwarps) {
     const __nv_bfloat16* xr = x + row * cols;
     uint4 raw[K];
@@ -239,6 +245,14 @@ ln_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
     for (int k = 0; k < K; ++k) {
       const int vi = lane + 32 * k;
       raw[k] = vi < nvec ? *reinterpret_cast<const uint4*>(xr + vi * 8) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    if constexpr (W > 1) {
+#pragma unroll
+      for (int i = 0; i < kOwn; ++i) {
+        const int vi = lane + 32 * (part + W * i);
+        if (gamma && vi < nvec) ld_pairs_f32(gamma + vi * 8, own_g[i]);
+        if (beta && vi < nvec) ld_pairs_f32(beta + vi * 8, own_b[i]);
+      }
     }
     // c = element 0 of the row = low half of lane 0's first word
     const float c = __uint_as_float(__shfl_sync(0xffffffffu, raw[0].x, 0) << 16);
@@ -267,7 +281,7 @@ ln_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
     const float var = fmaxf(q * inv_n - ms * ms, 0.f);
     const float mu = c + ms;
     const float rs = rsqrtf(var + eps);
-    if (lane == 0) {
+    if (lane == 0 && part == 0) {
       if (mean_out) mean_out[row] = mu;
       if (rstd_out) rstd_out[row] = rs;
     }
@@ -276,7 +290,7 @@ ln_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       const int vi = lane + 32 * k;
-      if (vi < nvec) {
+      if (vi < nvec && (W == 1 || k % W == part)) {
         const uint32_t w[4] = {raw[k].x, raw[k].y, raw[k].z, raw[k].w};
         float2 g[4], b[4];
 #pragma unroll
@@ -284,8 +298,16 @@ ln_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
           g[e] = make_float2(1.f, 1.f);
           b[e] = make_float2(0.f, 0.f);
         }
-        if (gamma) ld_pairs_f32(gamma + vi * 8, g);
-        if (beta) ld_pairs_f32(beta + vi * 8, b);
+        if constexpr (W > 1) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            if (gamma) g[e] = own_g[k / W][e];
+            if (beta) b[e] = own_b[k / W][e];
+          }
+        } else {
+          if (gamma) ld_pairs_f32(gamma + vi * 8, g);
+          if (beta) ld_pairs_f32(beta + vi * 8, b);
+        }
         uint4 out;
         uint32_t* ow = reinterpret_cast<uint32_t*>(&out);
 #pragma unroll
@@ -979,6 +1001,18 @@ bool launch_fwd_warp<__nv_bfloat16>(const __nv_bfloat16* xp, const float* gamma,
   static const int enabled = env_int("FERRUM_LN_WARP_FWD", 1);
   if (!enabled || pre_act != FB_ACT_NONE || cols < 1024 || cols > 4096) return false;
   const int k = (cols / 8 + 31) / 32;
+  // A block per row while two blocks per SM hold them all: 16 x 4096 6.9 -> 3.5 us, 296 x 2048 4.4 -> 3.2, 296 x 1024
+  // 3.0 -> 2.3; at 592 rows the warps are as fast (4096 columns: 7.1 against 7.2 us), at 1184 almost twice as fast.
+  if (rows <= 2LL * sm_count()) {
+    const int few = static_cast<int>(rows);
+    if (k <= 4)
+      ln_fwd_warp_kernel<4, 4><<<few, 128, 0, st>>>(xp, gamma, beta, yp, mean, rstd, rows, cols, eps);
+    else if (k <= 8)
+      ln_fwd_warp_kernel<8, 8><<<few, 256, 0, st>>>(xp, gamma, beta, yp, mean, rstd, rows, cols, eps);
+    else
+      ln_fwd_warp_kernel<16, 8><<<few, 256, 0, st>>>(xp, gamma, beta, yp, mean, rstd, rows, cols, eps);
+    return true;
+  }
   const long long want = (rows + 7) / 8;  // eight warps per block
   const long long cap = static_cast<long long>(sm_count()) * 2;
   const int grid = static_cast<int>(want < cap ? want : cap);
