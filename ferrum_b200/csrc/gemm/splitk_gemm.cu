@@ -1,0 +1,449 @@
+// bf16 GEMM for outputs of few tiles and a long reduction (sm_100a): a small batch of requests, weight gradients of
+// small layers over many rows.  The persistent kernels give such an output to a handful of SMs, each walking the whole
+// reduction alone: 16 x 4096 x 4096 took 33 us on 16 SMs where the weights stream from HBM in 5.  Here the K splits of a
+// tile are one thread-block cluster: every CTA multiplies its share of the k-blocks, the partial tiles meet in
+// distributed shared memory in a fixed order, and the epilogue (bias, activation, its derivative, accumulation) runs
+// once on the sum.  No workspace, no second launch, no atomics.
+//
+// What bounds it: one read of the larger operand from HBM.  Two CTAs share an SM with 98 KB of stages each, 29 MB in
+// flight over the chip.  Operands in L2, against the persistent kernels: 16 x 4096 x 4096 22.3 -> 9.3 us, 512 x 512 x
+// 4096 25.9 -> 11.9, 1024 x 1024 x 8192 (weight gradient) 47.4 -> 25.4.
+//
+// The tensor core multiplies 128 rows at a time whatever their use.  With up to 64 rows of A the operands change
+// places: 128 rows of B (the weights) against a tile of 16, 32 or 64 rows of A, so almost nothing is padding and the
+// weights are read once; the tile is turned round on its way to shared memory.
+//
+// 192 threads: warp 0 TMA producer, warp 1 MMA issue, warps 2 - 5 read the accumulator; all of them write the output.
+#include <cooperative_groups.h>
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "../common/ptx.cuh"
+#include "../common/status.h"
+#include "../include/ferrum_kernels.h"
+#include "epilogue.cuh"
+
+namespace fb {
+namespace {
+
+namespace cg = cooperative_groups;
+
+constexpr int kRowsP = 128;   // rows of the operand on the 128-row side of the MMA
+constexpr int kBK = 64;       // one 128-byte swizzle row of bf16
+constexpr int kThreads = 192;
+constexpr int kMaxStages = 12;
+constexpr int kSmemAlone = 200 * 1024, kSmemShared = 98 * 1024;  // stages of a CTA that has its SM alone, or half of it
+constexpr int kChunk = 64 * 128;  // 64 rows of 128 bytes: one block of an MN-major operand
+
+template <int BN>
+struct Cfg {
+  static constexpr int kP = kRowsP * 128;
+  static constexpr int kQ = (BN < 64 ? 64 : BN) * 128;  // an MN-major operand arrives in blocks of 64 columns
+  static constexpr int kTile = (kRowsP + 4) * (BN + 4) * 4;
+  static constexpr int kTmemCols = BN < 32 ? 32 : BN;
+};
+
+struct Args {
+  void* out;
+  void* out2;  // act'(z), stored like out
+  const float* bias;
+  int M, N;
+  long long ldc;
+  int p_mn, q_mn;  // operand stored with its rows contiguous
+  int out_bf16, act, beta;
+  int kb_total, kb_per_split, tiles_p;
+  int stages, stage_bytes, body_bytes;
+  int32_t* status;
+  unsigned long long timeout_ns;
+};
+
+__device__ __forceinline__ float act_of(float x, int act) {
+  switch (act) {
+    case FB_ACT_RELU: return act_value<FB_ACT_RELU>(x);
+    case FB_ACT_GELU: return act_value<FB_ACT_GELU>(x);
+    case FB_ACT_SILU: return act_value<FB_ACT_SILU>(x);
+    case FB_ACT_TANH: return act_value<FB_ACT_TANH>(x);
+    case FB_ACT_SIGMOID: return act_value<FB_ACT_SIGMOID>(x);
+    default: return x;
+  }
+}
+
+__device__ __forceinline__ void store_bf16(void* out, long long at, const float (&f)[4], int count, bool vec) {
+  __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out) + at;
+  const __nv_bfloat162 lo = __floats2bfloat162_rn(f[0], f[1]), hi = __floats2bfloat162_rn(f[2], f[3]);
+  if (vec) {
+    *reinterpret_cast<uint2*>(o) =
+        make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+  } else {
+    const __nv_bfloat16 h[4] = {lo.x, lo.y, hi.x, hi.y};
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (j < count) o[j] = h[j];
+  }
+}
+
+// kSwap: P = B (rows are output columns), Q = A.
+template <int BN, bool kSwap>
+__global__ void __launch_bounds__(kThreads, 2)
+gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q,
+                   const __grid_constant__ Args p) {
+  using C = Cfg<BN>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + p.body_bytes);
+  uint64_t* empty_bar = full_bar + kMaxStages;
+  uint64_t* acc_full = empty_bar + kMaxStages;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int splits = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
+  const int tile_id = static_cast<int>(blockIdx.x) / splits;
+  const int p0 = (tile_id % p.tiles_p) * kRowsP, q0 = (tile_id / p.tiles_p) * BN;
+  const int kb_lo = min(p.kb_total, rank * p.kb_per_split), kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
+
+  if (threadIdx.x == 0) {
+    *abort_flag = 0;
+    for (int s = 0; s < p.stages; ++s) {
+      ptx::mbar_init(&full_bar[s], 1);
+      ptx::mbar_init(&empty_bar[s], 1);
+    }
+    ptx::mbar_init(acc_full, 1);
+    ptx::fence_mbar_init();
+    ptx::prefetch_tensormap(&map_p);
+    ptx::prefetch_tensormap(&map_q);
+  }
+  if (warp == 1) {
+    ptx::tmem_alloc(tmem_slot, C::kTmemCols);
+    ptx::tmem_relinquish();
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int issued = 0, s = 0;
+      uint32_t phase = 1;
+      bool ok = true;
+      for (int kb = kb_lo; kb < kb_hi; ++kb, ++issued) {
+        if (!ptx::mbar_wait(&empty_bar[s], phase, abort_flag, p.timeout_ns)) {
+          report_status(p.status, kStatusGemmTimeout, 60, blockIdx.x, kb);
+          ok = false;
+          break;
+        }
+        uint8_t* sp = smem + s * p.stage_bytes;
+        uint8_t* sq = sp + C::kP;
+        ptx::mbar_arrive_expect_tx(&full_bar[s], p.stage_bytes);
+        const int k0 = kb * kBK;
+        if (p.p_mn) {
+#pragma unroll
+          for (int c = 0; c < kRowsP / 64; ++c) ptx::tma_load_2d(sp + c * kChunk, &map_p, &full_bar[s], p0 + c * 64, k0);
+        } else {
+          ptx::tma_load_2d(sp, &map_p, &full_bar[s], k0, p0);
+        }
+        if (p.q_mn) {
+#pragma unroll
+          for (int c = 0; c < C::kQ / kChunk; ++c) ptx::tma_load_2d(sq + c * kChunk, &map_q, &full_bar[s], q0 + c * 64, k0);
+        } else {
+          ptx::tma_load_2d(sq, &map_q, &full_bar[s], k0, q0);
+        }
+        if (++s == p.stages) {
+          s = 0;
+          phase ^= 1;
+        }
+      }
+      if (!ok) {  // no copy may still be writing shared memory when the CTA goes on: wait (bounded) for those in flight
+        for (int i = 0; i < p.stages && i < issued; ++i) {
+          const int last = (issued - 1 - i) / p.stages;
+          const uint64_t t0 = ptx::globaltimer();
+          while (!ptx::mbar_try_wait(&full_bar[i], last & 1))
+            if (ptx::globaltimer() - t0 > p.timeout_ns) break;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && kb_hi > kb_lo) {
+      const uint32_t idesc = ptx::make_idesc(1u, kRowsP, BN, p.p_mn, p.q_mn);
+      const uint32_t p_lbo = p.p_mn ? kChunk : 16, q_lbo = p.q_mn ? kChunk : 16;
+      const uint32_t p_step = p.p_mn ? 16 * 128 : 32, q_step = p.q_mn ? 16 * 128 : 32;
+      int s = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int i = 0; i < kb_hi - kb_lo; ++i) {
+        if (!ptx::mbar_wait(&full_bar[s], phase, abort_flag, p.timeout_ns)) {
+          report_status(p.status, kStatusGemmTimeout, 61, blockIdx.x, i);
+          ok = false;
+          break;
+        }
+        ptx::tc_fence_after();
+        const uint32_t sp = ptx::smem_u32(smem + s * p.stage_bytes), sq = sp + C::kP;
+#pragma unroll
+        for (int k = 0; k < kBK / 16; ++k)
+          ptx::umma_f16(tmem, ptx::make_smem_desc_sw128(sp + k * p_step, p_lbo, 1024),
+                        ptx::make_smem_desc_sw128(sq + k * q_step, q_lbo, 1024), idesc, (i | k) != 0 ? 1u : 0u);
+        ptx::umma_commit(&empty_bar[s]);
+        if (++s == p.stages) {
+          s = 0;
+          phase ^= 1;
+        }
+      }
+      if (ok) ptx::umma_commit(acc_full);
+    }
+  }
+
+  // ------------------------------------------------------------------ the accumulator as an [m][n] tile of fp32
+  constexpr int kRows = kSwap ? BN : kRowsP, kCols = kSwap ? kRowsP : BN, kPitch = kCols + 4;
+  float* tile = reinterpret_cast<float*>(smem);
+  if (warp >= 2) {
+    bool have = kb_hi > kb_lo;
+    if (have) {  // every MMA has completed, hence every copy too: the stages are free
+      const bool ready = ptx::mbar_wait(acc_full, 0, abort_flag, p.timeout_ns);
+      if (!__all_sync(0xffffffffu, ready)) {
+        if (lane == 0) report_status(p.status, kStatusGemmTimeout, 62, blockIdx.x, warp);
+        have = false;
+      }
+      ptx::tc_fence_after();
+    }
+    const int row = (warp & 3) * 32 + lane;
+    const uint32_t taddr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+#pragma unroll
+    for (int j = 0; j < BN / 16; ++j) {
+      uint32_t r[16];
+      if (have) {
+        ptx::tmem_ld_32x32b_x16(taddr + j * 16, r);
+        ptx::tmem_wait_ld();
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) r[i] = 0;
+      }
+      if constexpr (kSwap) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) tile[(j * 16 + i) * kPitch + row] = __uint_as_float(r[i]);
+      } else {
+        float4* t4 = reinterpret_cast<float4*>(tile + row * kPitch + j * 16);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          t4[i] = make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]), __uint_as_float(r[4 * i + 2]),
+                              __uint_as_float(r[4 * i + 3]));
+      }
+    }
+  }
+  cluster.sync();
+
+  // ------------------------------------------------------------------ add the splits, epilogue
+  const int m0 = kSwap ? q0 : p0, n0 = kSwap ? p0 : q0;
+  const int esz = p.out_bf16 ? 2 : 4;
+  const bool vec = p.N % 4 == 0 && p.ldc % 4 == 0 && reinterpret_cast<uintptr_t>(p.out) % (4 * esz) == 0 &&
+                   reinterpret_cast<uintptr_t>(p.out2) % 8 == 0;
+  constexpr int kVec = kCols / 4, kAll = kRows * kVec;
+  const int share = (kAll + splits - 1) / splits;
+  for (int i = rank * share + threadIdx.x; i < min(kAll, (rank + 1) * share); i += kThreads) {
+    const int row = i / kVec, c = (i % kVec) * 4;
+    const int m = m0 + row, n = n0 + c;
+    if (m >= p.M || n >= p.N) continue;
+    float f[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int r = 0; r < splits; ++r) {
+      const float4 t = *reinterpret_cast<const float4*>(cluster.map_shared_rank(tile, r) + row * kPitch + c);
+      f[0] += t.x; f[1] += t.y; f[2] += t.z; f[3] += t.w;
+    }
+    const int count = min(4, p.N - n);
+    if (p.bias != nullptr) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j < count) f[j] += __ldg(p.bias + n + j);
+    }
+    const long long at = m * p.ldc + n;
+    if (p.out2 != nullptr) {
+      float d[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) act_both(f[j], p.act, f[j], d[j]);
+      store_bf16(p.out2, at, d, count, vec);
+    } else if (p.act != FB_ACT_NONE) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) f[j] = act_of(f[j], p.act);
+    }
+    if (p.out_bf16) {
+      store_bf16(p.out, at, f, count, vec);
+      continue;
+    }
+    float* o = static_cast<float*>(p.out) + at;
+    if (vec) {
+      float4 x = make_float4(f[0], f[1], f[2], f[3]);
+      if (p.beta) {
+        const float4 old = *reinterpret_cast<float4*>(o);
+        x.x += old.x; x.y += old.y; x.z += old.z; x.w += old.w;
+      }
+      *reinterpret_cast<float4*>(o) = x;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j < count) o[j] = p.beta ? o[j] + f[j] : f[j];
+    }
+  }
+  ptx::tc_fence_before();
+  cluster.sync();  // no CTA leaves while another one still reads its tile
+  if (warp == 1) {
+    ptx::tc_fence_after();
+    ptx::tmem_dealloc(tmem, C::kTmemCols);
+  }
+}
+
+// ------------------------------------------------------------ host side
+typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                             const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                             CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeFn encoder() {
+  // The encoder wants a current context; an autograd worker entering its first backward has none yet.
+  static thread_local bool bound = false;
+  if (!bound) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaSetDevice(dev);
+    bound = true;
+  }
+  static const EncodeFn fn = [] {
+    void* sym = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      sym = nullptr;
+    return reinterpret_cast<EncodeFn>(sym);
+  }();
+  return fn;
+}
+
+// `rows` x K operand: boxes of 64 k x `box_rows` rows (K-major) or 64 rows x 64 k (MN-major), 128-byte swizzle.
+bool make_map(CUtensorMap* map, const void* ptr, int rows, int K, long long ld, bool mn, int box_rows) {
+  const EncodeFn enc = encoder();
+  if (enc == nullptr || (reinterpret_cast<uintptr_t>(ptr) & 15) != 0 || ld % 8 != 0) return false;
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(mn ? rows : K), static_cast<cuuint64_t>(mn ? K : rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 2};
+  const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(mn ? 64 : box_rows)}, estr[2] = {1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+int sm_count() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v;
+  }();
+  return n;
+}
+
+int tiles_of(int rows, int per) { return (rows + per - 1) / per; }
+
+// Tile: 16, 32, 64 = rows of A against 128 rows of B; 128 + 64 or 128 + 128 = 128 rows of A against 64 or 128 of B,
+// the wide one where the narrow one leaves no room for four splits (1024 x 1024 x 4096: 18 against 20 us).
+int choose_tile(int M, int N) {
+  if (M <= 64) return M <= 16 ? 16 : M <= 32 ? 32 : 64;
+  return static_cast<long long>(tiles_of(M, kRowsP)) * tiles_of(N, 64) * 4 <= 2 * sm_count() ? 192 : 256;
+}
+
+long long tile_count(int M, int N, int tile) {
+  return tile <= 64 ? static_cast<long long>(tiles_of(N, kRowsP)) * tiles_of(M, tile)
+                    : static_cast<long long>(tiles_of(M, kRowsP)) * tiles_of(N, tile - 128);
+}
+
+// As many splits as the two CTAs per SM have room for, each with at least two k-blocks to overlap.
+int choose_splits(long long tiles, int kb_total) {
+  int splits = 1;
+  while (splits < 8 && tiles * splits * 2 <= 2 * sm_count() && splits * 4 <= kb_total) splits *= 2;
+  return splits;
+}
+
+template <int BN, bool kSwap>
+int launch(const CUtensorMap& mp, const CUtensorMap& mq, Args& g, int rows_p, int rows_q, cudaStream_t st) {
+  using C = Cfg<BN>;
+  constexpr int kExtra = 1024 + 256;  // alignment, barriers
+  static const cudaError_t configured = cudaFuncSetAttribute(
+      gemm_splitk_kernel<BN, kSwap>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAlone + kExtra);
+  if (configured != cudaSuccess) return static_cast<int>(configured);
+  g.tiles_p = tiles_of(rows_p, kRowsP);
+  const long long tiles = static_cast<long long>(g.tiles_p) * tiles_of(rows_q, BN);
+  if (tiles > (1 << 27)) return -1;
+  const int splits = choose_splits(tiles, g.kb_total);
+  g.kb_per_split = (g.kb_total + splits - 1) / splits;
+  g.stage_bytes = C::kP + (g.q_mn ? C::kQ : BN * 128);
+  const int room = (tiles * splits <= sm_count() ? kSmemAlone : kSmemShared) / g.stage_bytes;
+  g.stages = room < kMaxStages ? room : kMaxStages;
+  if (g.stages > g.kb_per_split) g.stages = g.kb_per_split;
+  g.body_bytes = g.stages * g.stage_bytes;
+  if (g.body_bytes < C::kTile) g.body_bytes = (C::kTile + 1023) / 1024 * 1024;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(tiles * splits));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = g.body_bytes + kExtra;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = splits;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, gemm_splitk_kernel<BN, kSwap>, mp, mq, g));
+}
+
+}  // namespace
+}  // namespace fb
+
+// Where this kernel is the faster one by enough to repay another order of summation.  The persistent kernels take
+// 4.6 us and 4.3 ns per unit of K for any output that fits one wave (a chain of MMAs on one accumulator advances by
+// 16 of K in 69 ns however narrow the tile); this one has 5 to 6 us of launch, cluster and epilogue and then divides K
+// by the splits.  K 256: 6 against 5.7 us; K 1024: 7 against 9 at best; K 2048: 8 against 13.5 us with eight splits
+// (8 x 4096), 10.8 against 14 with four (96 x 4096); with two splits it needs a very long reduction
+// (512 x 4096 x 8192: 43 against 49 us, but 300 x 4096 x 4096: 26 against 24).
+extern "C" int fb_gemm_bf16_splitk_use(int M, int N, int K) {
+  using namespace fb;
+  if (M <= 0 || N <= 0 || K < 2048) return 0;
+  const int kb = (K + kBK - 1) / kBK;
+  const int splits = choose_splits(tile_count(M, N, choose_tile(M, N)), kb);
+  return splits >= 4 || (kb >= 128 && splits >= 2);
+}
+
+extern "C" int fb_gemm_bf16_splitk(const void* a, const void* b, void* out, void* out2, const float* bias, int M, int N,
+                                   int K, long long lda, long long ldb, long long ldc, int a_mn_major, int b_mn_major,
+                                   int out_bf16, int act, int beta, int tile, int32_t* status, cudaStream_t stream) {
+  using namespace fb;
+  if (M <= 0 || N <= 0 || K <= 0) return -1;
+  if ((out2 != nullptr && !out_bf16) || (out_bf16 && beta)) return -1;
+  if (tile == 0) tile = choose_tile(M, N);
+  if (tile != 16 && tile != 32 && tile != 64 && tile != 192 && tile != 256) return -1;
+  const bool swap = tile <= 64;
+  const int bn = swap ? tile : tile - 128;
+  CUtensorMap ma, mb;
+  if (!make_map(&ma, a, M, K, lda, a_mn_major != 0, swap ? bn : kRowsP) ||
+      !make_map(&mb, b, N, K, ldb, b_mn_major != 0, swap ? kRowsP : bn))
+    return -2;
+  Args g;
+  g.out = out;
+  g.out2 = out2;
+  g.bias = bias;
+  g.M = M;
+  g.N = N;
+  g.ldc = ldc;
+  g.p_mn = swap ? b_mn_major : a_mn_major;
+  g.q_mn = swap ? a_mn_major : b_mn_major;
+  g.out_bf16 = out_bf16;
+  g.act = act;
+  g.beta = beta;
+  g.kb_total = (K + kBK - 1) / kBK;
+  g.status = status;
+  g.timeout_ns = 2000000000ull;
+  switch (tile) {
+    case 16: return launch<16, true>(mb, ma, g, N, M, stream);
+    case 32: return launch<32, true>(mb, ma, g, N, M, stream);
+    case 64: return launch<64, true>(mb, ma, g, N, M, stream);
+    case 192: return launch<64, false>(ma, mb, g, M, N, stream);
+    default: return launch<128, false>(ma, mb, g, M, N, stream);
+  }
+}

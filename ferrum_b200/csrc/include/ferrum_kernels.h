@@ -89,6 +89,13 @@ int fb_gemm_f32_tensor(const float* a, const float* b, float* out, const float* 
 int fb_gemm_bf16_any(const void* a, const void* b, void* out, const float* bias, int M, int N, int K, long long sam,
                      long long sak, long long sbn, long long sbk, long long ldc, int out_bf16, int act, int beta,
                      int32_t* status, cudaStream_t stream);
+// bf16 products of few output tiles: the K splits of a tile meet in a cluster (gemm/splitk_gemm.cu).  Arguments as
+// fb_gemm_bf16; tile: 0 = chosen by size, 16 / 32 / 64 = rows of A against 128 rows of B, 192 / 256 = 128 rows of A
+// against 64 / 128 rows of B.
+int fb_gemm_bf16_splitk_use(int M, int N, int K);  // 1: faster than fb_gemm_bf16 / _2cta for this product
+int fb_gemm_bf16_splitk(const void* a, const void* b, void* out, void* out2, const float* bias, int M, int N, int K,
+                        long long lda, long long ldb, long long ldc, int a_mn_major, int b_mn_major, int out_bf16,
+                        int act, int beta, int tile, int32_t* status, cudaStream_t stream);
 // fp32 SIMT GEMM with arbitrary element strides (parity runs, odd shapes):
 // out[m,n] = act(sum_k A[m*sam + k*sak] * B[k*sbk + n*sbn] + bias[n]) (+= out when beta).
 int fb_gemm_f32_simt(const float* a, const float* b, float* out, const float* bias, int M, int N, int K,

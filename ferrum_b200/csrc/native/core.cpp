@@ -83,7 +83,7 @@ bool tma_ok(const Op& a) {
 constexpr int kSimtK = 32;
 
 void gemm(const Op& a, const Op& b, const float* bias, int act, void* out, ll ldc, bool out_bf16, bool accumulate,
-          void* act_grad, const Tensor* like, bool tf32) {
+          void* act_grad, const Tensor* like, bool tf32, bool splits) {
   const int M = static_cast<int>(a.rows), N = static_cast<int>(b.rows), K = static_cast<int>(a.k);
   TORCH_CHECK(a.k == b.k, "inner dimensions differ: [", a.rows, ", ", a.k, "] x [", b.rows, ", ", b.k, "]^T");
   if (M == 0 || N == 0) return;
@@ -91,6 +91,12 @@ void gemm(const Op& a, const Op& b, const float* bias, int act, void* out, ll ld
   const int a_mn = a.s_k == 1 ? 0 : 1, b_mn = b.s_k == 1 ? 0 : 1;
   const ll lda = a_mn ? a.s_k : a.s_row, ldb = b_mn ? b.s_k : b.s_row;
   if (a.bf16 && ok) {
+    if (splits && g_max_ctas.load(std::memory_order_relaxed) == 0 && !(out_bf16 && accumulate) &&
+        fb_gemm_bf16_splitk_use(M, N, K)) {
+      FB_CALL(fb_gemm_bf16_splitk, a.p, b.p, out, act_grad, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_bf16, act,
+              accumulate, 0, status(), cur_stream());
+      return;
+    }
     int rc = -3;
     if (g_use_2cta.load(std::memory_order_relaxed) && M >= 512 && N >= 128)
       launch("fb_gemm_bf16", [&] {
@@ -185,7 +191,7 @@ void wgrad_to_sink(Sink& s, const Tensor& g2, const Tensor& x2) {
     acc = r[1].cast<bool>();
   }
   gemm(op2d(g2).t(), op2d(x2).t(), nullptr, 0, buf.data_ptr(), buf.stride(0), false, acc, nullptr, &g2,
-       g_tf32.load(std::memory_order_relaxed));
+       g_tf32.load(std::memory_order_relaxed), true);
 }
 void sink_ready(Sink& s) {
   py::gil_scoped_acquire gil;

@@ -51,7 +51,7 @@ void linear_grads(const Tensor& g2, const Tensor& x2, const Tensor& w, bool low,
       wgrad_to_sink(*sink, g2, x2);
     } else {
       Tensor gw = empty({N, K}, g2, at::kFloat);
-      gemm(op2d(g2).t(), op2d(x2).t(), nullptr, kNone, gw.data_ptr(), K, false, false, nullptr, &g2, tf32);
+      gemm(op2d(g2).t(), op2d(x2).t(), nullptr, kNone, gw.data_ptr(), K, false, false, nullptr, &g2, tf32, true);
       out[1] = gw;
     }
   }
@@ -103,8 +103,9 @@ Tensor linear(const Tensor& x, const Tensor& weight, const c10::optional<Tensor>
   const int64_t N = weight.size(0);
   Tensor y = empty(out_sizes(x, N), o.x2, low ? at::kBFloat16 : at::kFloat);
   Tensor b = bias.defined() ? f32c(bias) : bias;
-  gemm(op2d(o.x2), op2d(o.w), fptr(b), act, y.data_ptr(), N, low, false, nullptr, &o.x2, tf32 && !low);
-  if (wants_grad({&x, &weight, &bias})) {
+  const bool grad = wants_grad({&x, &weight, &bias});
+  gemm(op2d(o.x2), op2d(o.w), fptr(b), act, y.data_ptr(), N, low, false, nullptr, &o.x2, tf32 && !low, !grad);
+  if (grad) {
     auto n = make_node<LinearNode>(x, weight, bias);
     n->low = low;
     n->act = act;
@@ -244,7 +245,7 @@ Tensor linear_act_norm(const Tensor& x, const Tensor& weight, const c10::optiona
   const bool fused = low && act != kNone && tma_ok(op2d(o.x2)) && tma_ok(op2d(o.w));
   if (fused && grad) dact = empty({M, N}, o.x2, at::kBFloat16);
   gemm(op2d(o.x2), op2d(o.w), fptr(b), fused ? act : kNone, z.data_ptr(), N, low, false, ptr(dact), &o.x2,
-       tf32 && !low);
+       tf32 && !low, !grad);
   const int pre = fused ? kNone : act;
   Tensor y = empty(out_sizes(x, N), o.x2, z.scalar_type());
   NormStats st = norm_fwd(z, g, be, y, static_cast<float>(eps), pre);
