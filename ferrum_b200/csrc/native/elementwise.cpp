@@ -116,18 +116,19 @@ Tensor softmax(const Tensor& x, bool log_mode) {
 // Mean cross-entropy of logits and integer labels.  The forward pass keeps the maximum and the sum of exponentials of each row; the logit
 // gradient is written once, in the backward pass, with the incoming gradient applied (read on the device).
 struct CrossEntropyNode : Node {
-  SavedVariable x_;
-  Tensor labels, lse;
+  SavedVariable x_, labels_;  // saved, so that labels changed before the backward pass are noticed
+  Tensor lse;
   std::string name() const override { return "FerrumCrossEntropyBackward"; }
   void release_variables() override {
     x_.reset_data();
-    labels = lse = Tensor();
+    labels_.reset_data();
+    lse = Tensor();
   }
   variable_list apply(variable_list&& grads) override {
     NoAutograd below;
     variable_list out(1);
     if (!grads[0].defined()) return out;
-    Tensor x = contig(x_.unpack()), g = f32c(grads[0]);
+    Tensor x = contig(x_.unpack()), labels = labels_.unpack(), g = f32c(grads[0]);
     Tensor dx = empty(x.sizes(), x, x.scalar_type());
     FB_CALL(fb_ce_bwd, x.data_ptr(), reinterpret_cast<const ll*>(labels.data_ptr<int64_t>()), lse.data_ptr<float>(),
             g.data_ptr<float>(), dx.data_ptr(), x.size(0), static_cast<int>(x.size(1)),
@@ -150,7 +151,7 @@ Tensor cross_entropy(const Tensor& logits, const Tensor& labels) {
   if (grad) {
     auto n = make_node<CrossEntropyNode>(logits);
     n->x_ = SavedVariable(x.is_alias_of(logits) ? logits : x, false);
-    n->labels = lab;
+    n->labels_ = SavedVariable(lab, false);
     n->lse = lse;
     torch::autograd::set_history(loss, n);
   }
@@ -159,18 +160,17 @@ Tensor cross_entropy(const Tensor& logits, const Tensor& labels) {
 
 // Mean of -log_probs[i, target_i].
 struct NllNode : Node {
-  Tensor target;
+  SavedVariable target_;
   int64_t rows = 0, cols = 0;
   at::ScalarType st = at::kFloat;
   std::vector<int64_t> sizes;
   std::string name() const override { return "FerrumNllBackward"; }
-  void release_variables() override { target = Tensor(); }
+  void release_variables() override { target_.reset_data(); }
   variable_list apply(variable_list&& grads) override {
     NoAutograd below;
     variable_list out(1);
     if (!grads[0].defined()) return out;
-    TORCH_CHECK(target.defined(), "Trying to backward through the graph a second time");
-    Tensor g = f32c(grads[0]), dx = empty(sizes, g, st);
+    Tensor target = target_.unpack(), g = f32c(grads[0]), dx = empty(sizes, g, st);
     FB_CALL(fb_nll_bwd, reinterpret_cast<const ll*>(target.data_ptr<int64_t>()), g.data_ptr<float>(), dx.data_ptr(),
             rows, static_cast<int>(cols), -1.f / static_cast<float>(rows), dt(dx), cur_stream());
     out[0] = dx;
@@ -188,7 +188,7 @@ Tensor nll(const Tensor& log_probs, const Tensor& target) {
   if (!is_f32(x)) loss = cast(loss, x.scalar_type());
   if (wants_grad({&log_probs})) {
     auto n = make_node<NllNode>(log_probs);
-    n->target = t;
+    n->target_ = SavedVariable(t, false);
     n->rows = rows;
     n->cols = cols;
     n->st = x.scalar_type();
@@ -200,19 +200,18 @@ Tensor nll(const Tensor& log_probs, const Tensor& target) {
 
 // mse / bce / l1 / smooth_l1, mean over all elements; predictions fp32 or bf16, targets likewise.
 struct ElemLossNode : Node {
-  SavedVariable p_;
-  Tensor t;
+  SavedVariable p_, t_;
   int kind = 0;
   std::string name() const override { return "FerrumElementwiseLossBackward"; }
   void release_variables() override {
     p_.reset_data();
-    t = Tensor();
+    t_.reset_data();
   }
   variable_list apply(variable_list&& grads) override {
     NoAutograd below;
     variable_list out(1);
     if (!grads[0].defined()) return out;
-    Tensor p = p_.unpack(), pc = f32c(p), g = f32c(grads[0]);
+    Tensor p = p_.unpack(), t = t_.unpack(), pc = f32c(p), g = f32c(grads[0]);
     Tensor dp = empty(p.sizes(), pc, at::kFloat);
     FB_CALL(fb_loss_bwd, pc.data_ptr<float>(), t.data_ptr<float>(), g.data_ptr<float>(), dp.data_ptr<float>(),
             pc.numel(), kind, 1.f / static_cast<float>(pc.numel()), cur_stream());
@@ -231,7 +230,7 @@ Tensor elementwise_loss(const Tensor& pred, const Tensor& target, int kind) {
   if (wants_grad({&pred})) {
     auto nd = make_node<ElemLossNode>(pred);
     nd->p_ = SavedVariable(pred, false);
-    nd->t = t;
+    nd->t_ = SavedVariable(t, false);
     nd->kind = kind;
     torch::autograd::set_history(loss, nd);
   }

@@ -5,17 +5,16 @@ namespace fbn {
 namespace {
 
 struct EmbeddingNode : Node {
-  Tensor idx;
+  SavedVariable idx_;
   int64_t vocab = 0, dim = 0, group = 1;
   ll padding = -1;
   std::shared_ptr<Sink> sink;
   std::string name() const override { return "FerrumEmbeddingBackward"; }
-  void release_variables() override { idx = Tensor(); }
+  void release_variables() override { idx_.reset_data(); }
   variable_list apply(variable_list&& grads) override {
     variable_list out(1);
     if (!grads[0].defined()) return out;
-    TORCH_CHECK(idx.defined(), "Trying to backward through the graph a second time");
-    Tensor dw, sorted, perm, g2;
+    Tensor idx = idx_.unpack(), dw, sorted, perm, g2;
     {
       NoAutograd below;
       g2 = contig(grads[0]).reshape({-1, dim});
@@ -58,7 +57,7 @@ Tensor embedding(const Tensor& weight, const Tensor& idx_, ll padding, bool pool
   }
   if (wants_grad({&weight})) {
     auto n = make_node<EmbeddingNode>(weight);
-    n->idx = idx;
+    n->idx_ = SavedVariable(idx, false);
     n->vocab = V;
     n->dim = D;
     n->group = pool ? idx.size(1) : 1;
