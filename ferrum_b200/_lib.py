@@ -108,6 +108,7 @@ _CUDA_SIGS = {
     "fb_gemm_bf16": (I, [P, P, P, P, P, I, I, I, LL, LL, LL, I, I, I, I, I, I, P, P]),
     "fb_gemm_bf16_2cta": (I, [P, P, P, P, P, I, I, I, LL, LL, LL, I, I, I, I, I, I, P, P]),
     "fb_gemm_bf16_splitk": (I, [P, P, P, P, P, I, I, I, LL, LL, LL, I, I, I, I, I, I, P, P]),
+    "fb_gemm_bf16_narrow": (I, [P, P, P, P, P, I, I, I, LL, LL, LL, I, I, I, I, I, I, P, P]),
     "fb_gemm_bf16_2cta_pairs": (I, []),
     "fb_gemm_tf32": (I, [P, P, P, P, I, I, I, LL, LL, LL, I, I, I, I, I, P, P]),
     "fb_gemm_tf32_2cta": (I, [P, P, P, P, I, I, I, LL, LL, LL, I, I, I, I, I, P, P]),

@@ -1,6 +1,6 @@
-// bf16 GEMM for outputs of few tiles and a long reduction (sm_100a): a small batch of requests, weight gradients of
-// small layers over many rows.  The persistent kernels give such an output to a handful of SMs, each walking the whole
-// reduction alone: 16 x 4096 x 4096 took 33 us on 16 SMs where the weights stream from HBM in 5.  Here the K splits of a
+// bf16 GEMM for outputs of few tiles and a long reduction (sm_100a): weight gradients of small layers over many rows.
+// The persistent kernels give such an output to a handful of SMs, each walking the whole reduction alone: 16 x 4096 x
+// 4096 took 33 us on 16 SMs where the larger operand streams from HBM in 5.  Here the K splits of a
 // tile are one thread-block cluster: every CTA multiplies its share of the k-blocks, the partial tiles meet in
 // distributed shared memory in a fixed order, and the epilogue (bias, activation, its derivative, accumulation) runs
 // once on the sum.  No workspace, no second launch, no atomics.
@@ -9,9 +9,9 @@
 // flight over the chip.  Operands in L2, against the persistent kernels: 16 x 4096 x 4096 22.3 -> 9.3 us, 512 x 512 x
 // 4096 25.9 -> 11.9, 1024 x 1024 x 8192 (weight gradient) 47.4 -> 25.4.
 //
-// The tensor core multiplies 128 rows at a time whatever their use.  With up to 64 rows of A the operands change
-// places: 128 rows of B (the weights) against a tile of 16, 32 or 64 rows of A, so almost nothing is padding and the
-// weights are read once; the tile is turned round on its way to shared memory.
+// The tensor core multiplies 128 rows at a time whatever their use.  With up to 64 rows of A (a head of few classes) the
+// operands change places: 128 rows of B against a tile of 16, 32 or 64 rows of A, so almost nothing is padding and B is
+// read once; the tile is turned round on its way to shared memory.
 //
 // 192 threads: warp 0 TMA producer, warp 1 MMA issue, warps 2 - 5 read the accumulator; all of them write the output.
 #include <cooperative_groups.h>
@@ -362,7 +362,7 @@ int choose_splits(long long tiles, int kb_total) {
 }
 
 template <int BN, bool kSwap>
-int launch(const CUtensorMap& mp, const CUtensorMap& mq, Args& g, int rows_p, int rows_q, cudaStream_t st) {
+int launch(const CUtensorMap& mp, const CUtensorMap& mq, Args& g, int rows_p, int rows_q, bool split, cudaStream_t st) {
   using C = Cfg<BN>;
   constexpr int kExtra = 1024 + 256;  // alignment, barriers
   static const cudaError_t configured = cudaFuncSetAttribute(
@@ -371,7 +371,7 @@ int launch(const CUtensorMap& mp, const CUtensorMap& mq, Args& g, int rows_p, in
   g.tiles_p = tiles_of(rows_p, kRowsP);
   const long long tiles = static_cast<long long>(g.tiles_p) * tiles_of(rows_q, BN);
   if (tiles > (1 << 27)) return -1;
-  const int splits = choose_splits(tiles, g.kb_total);
+  const int splits = split ? choose_splits(tiles, g.kb_total) : 1;
   g.kb_per_split = (g.kb_total + splits - 1) / splits;
   g.stage_bytes = C::kP + (g.q_mn ? C::kQ : BN * 128);
   const int room = (tiles * splits <= sm_count() ? kSmemAlone : kSmemShared) / g.stage_bytes;
@@ -410,10 +410,12 @@ extern "C" int fb_gemm_bf16_splitk_use(int M, int N, int K) {
   return splits >= 4 || (kb >= 128 && splits >= 2);
 }
 
-extern "C" int fb_gemm_bf16_splitk(const void* a, const void* b, void* out, void* out2, const float* bias, int M, int N,
-                                   int K, long long lda, long long ldb, long long ldc, int a_mn_major, int b_mn_major,
-                                   int out_bf16, int act, int beta, int tile, int32_t* status, cudaStream_t stream) {
-  using namespace fb;
+namespace fb {
+namespace {
+
+int run(bool split, const void* a, const void* b, void* out, void* out2, const float* bias, int M, int N, int K,
+        long long lda, long long ldb, long long ldc, int a_mn_major, int b_mn_major, int out_bf16, int act, int beta,
+        int tile, int32_t* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return -1;
   if ((out2 != nullptr && !out_bf16) || (out_bf16 && beta)) return -1;
   if (tile == 0) tile = choose_tile(M, N);
@@ -440,10 +442,36 @@ extern "C" int fb_gemm_bf16_splitk(const void* a, const void* b, void* out, void
   g.status = status;
   g.timeout_ns = 2000000000ull;
   switch (tile) {
-    case 16: return launch<16, true>(mb, ma, g, N, M, stream);
-    case 32: return launch<32, true>(mb, ma, g, N, M, stream);
-    case 64: return launch<64, true>(mb, ma, g, N, M, stream);
-    case 192: return launch<64, false>(ma, mb, g, M, N, stream);
-    default: return launch<128, false>(ma, mb, g, M, N, stream);
+    case 16: return launch<16, true>(mb, ma, g, N, M, split, stream);
+    case 32: return launch<32, true>(mb, ma, g, N, M, split, stream);
+    case 64: return launch<64, true>(mb, ma, g, N, M, split, stream);
+    case 192: return launch<64, false>(ma, mb, g, M, N, split, stream);
+    default: return launch<128, false>(ma, mb, g, M, N, split, stream);
   }
+}
+
+}  // namespace
+}  // namespace fb
+
+extern "C" int fb_gemm_bf16_splitk(const void* a, const void* b, void* out, void* out2, const float* bias, int M, int N,
+                                   int K, long long lda, long long ldb, long long ldc, int a_mn_major, int b_mn_major,
+                                   int out_bf16, int act, int beta, int tile, int32_t* status, cudaStream_t stream) {
+  return fb::run(true, a, b, out, out2, bias, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, out_bf16, act, beta, tile,
+                 status, stream);
+}
+
+// Results of up to 64 rows whose sums may not change with the shape (forward passes, input gradients): narrow tiles and
+// one chain of MMAs over the whole reduction, the persistent kernels' bits.  They leave a 16 x 4096 product to 16 CTAs,
+// each of which reads 2 MB of weights alone; here it is 32 or 64.  Operands from HBM: 16 x 4096 x 4096 38.9 -> 29.6 us,
+// 16 x 1000 x 1024 20.5 -> 16.4, 64 x 4096 x 4096 39.0 -> 32.8; 16 x 128 x 512 12.3 -> 14.3, 128 x 512 x 512 18.4 both.
+extern "C" int fb_gemm_bf16_narrow_use(int M, int N, int K) {
+  return M > 0 && M <= 64 && N >= 512 && N <= fb::kRowsP * fb::sm_count() && K >= 512;
+}
+
+extern "C" int fb_gemm_bf16_narrow(const void* a, const void* b, void* out, void* out2, const float* bias, int M, int N,
+                                   int K, long long lda, long long ldb, long long ldc, int a_mn_major, int b_mn_major,
+                                   int out_bf16, int act, int beta, int tile, int32_t* status, cudaStream_t stream) {
+  if (tile == 0) tile = M <= 32 ? fb::choose_tile(M, N) : 192;
+  return fb::run(false, a, b, out, out2, bias, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, out_bf16, act, beta, tile,
+                 status, stream);
 }

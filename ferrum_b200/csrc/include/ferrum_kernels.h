@@ -96,6 +96,11 @@ int fb_gemm_bf16_splitk_use(int M, int N, int K);  // 1: faster than fb_gemm_bf1
 int fb_gemm_bf16_splitk(const void* a, const void* b, void* out, void* out2, const float* bias, int M, int N, int K,
                         long long lda, long long ldb, long long ldc, int a_mn_major, int b_mn_major, int out_bf16,
                         int act, int beta, int tile, int32_t* status, cudaStream_t stream);
+// The same tiles without the splits: the bits of fb_gemm_bf16.
+int fb_gemm_bf16_narrow_use(int M, int N, int K);  // 1: faster than fb_gemm_bf16 for this product
+int fb_gemm_bf16_narrow(const void* a, const void* b, void* out, void* out2, const float* bias, int M, int N, int K,
+                        long long lda, long long ldb, long long ldc, int a_mn_major, int b_mn_major, int out_bf16,
+                        int act, int beta, int tile, int32_t* status, cudaStream_t stream);
 // fp32 SIMT GEMM with arbitrary element strides (parity runs, odd shapes):
 // out[m,n] = act(sum_k A[m*sam + k*sak] * B[k*sbk + n*sbn] + bias[n]) (+= out when beta).
 int fb_gemm_f32_simt(const float* a, const float* b, float* out, const float* bias, int M, int N, int K,

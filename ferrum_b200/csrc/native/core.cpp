@@ -91,11 +91,17 @@ void gemm(const Op& a, const Op& b, const float* bias, int act, void* out, ll ld
   const int a_mn = a.s_k == 1 ? 0 : 1, b_mn = b.s_k == 1 ? 0 : 1;
   const ll lda = a_mn ? a.s_k : a.s_row, ldb = b_mn ? b.s_k : b.s_row;
   if (a.bf16 && ok) {
-    if (splits && g_max_ctas.load(std::memory_order_relaxed) == 0 && !(out_bf16 && accumulate) &&
-        fb_gemm_bf16_splitk_use(M, N, K)) {
-      FB_CALL(fb_gemm_bf16_splitk, a.p, b.p, out, act_grad, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_bf16, act,
-              accumulate, 0, status(), cur_stream());
-      return;
+    if (g_max_ctas.load(std::memory_order_relaxed) == 0 && !(out_bf16 && accumulate)) {
+      if (splits && fb_gemm_bf16_splitk_use(M, N, K)) {
+        FB_CALL(fb_gemm_bf16_splitk, a.p, b.p, out, act_grad, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_bf16, act,
+                accumulate, 0, status(), cur_stream());
+        return;
+      }
+      if (fb_gemm_bf16_narrow_use(M, N, K)) {
+        FB_CALL(fb_gemm_bf16_narrow, a.p, b.p, out, act_grad, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_bf16, act,
+                accumulate, 0, status(), cur_stream());
+        return;
+      }
     }
     int rc = -3;
     if (g_use_2cta.load(std::memory_order_relaxed) && M >= 512 && N >= 128)

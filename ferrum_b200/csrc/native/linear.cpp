@@ -104,7 +104,7 @@ Tensor linear(const Tensor& x, const Tensor& weight, const c10::optional<Tensor>
   Tensor y = empty(out_sizes(x, N), o.x2, low ? at::kBFloat16 : at::kFloat);
   Tensor b = bias.defined() ? f32c(bias) : bias;
   const bool grad = wants_grad({&x, &weight, &bias});
-  gemm(op2d(o.x2), op2d(o.w), fptr(b), act, y.data_ptr(), N, low, false, nullptr, &o.x2, tf32 && !low, !grad);
+  gemm(op2d(o.x2), op2d(o.w), fptr(b), act, y.data_ptr(), N, low, false, nullptr, &o.x2, tf32 && !low);
   if (grad) {
     auto n = make_node<LinearNode>(x, weight, bias);
     n->low = low;
@@ -245,7 +245,7 @@ Tensor linear_act_norm(const Tensor& x, const Tensor& weight, const c10::optiona
   const bool fused = low && act != kNone && tma_ok(op2d(o.x2)) && tma_ok(op2d(o.w));
   if (fused && grad) dact = empty({M, N}, o.x2, at::kBFloat16);
   gemm(op2d(o.x2), op2d(o.w), fptr(b), fused ? act : kNone, z.data_ptr(), N, low, false, ptr(dact), &o.x2,
-       tf32 && !low, !grad);
+       tf32 && !low);
   const int pre = fused ? kNone : act;
   Tensor y = empty(out_sizes(x, N), o.x2, z.scalar_type());
   NormStats st = norm_fwd(z, g, be, y, static_cast<float>(eps), pre);

@@ -53,7 +53,7 @@ def test_tiles(tile, M, N, K, a_mn, b_mn):
     assert (der.double() - s * (1 - s)).norm() <= 2.0 ** -8 * s.norm() + bound * ref.norm()
 
 
-def test_no_grad_linear_takes_it():
+def test_linear_of_few_rows_in_either_grad_mode():
     import ferrum_b200 as fb
     from ferrum_b200 import nn
 
@@ -65,5 +65,6 @@ def test_no_grad_linear_takes_it():
         with fb.no_grad():
             z = lin(x)
     ref = x.bfloat16().double() @ lin.weight.detach().bfloat16().double().t() + lin.bias.detach().double()
+    assert torch.equal(y.detach(), z)
     for out in (y, z):
         assert (out.detach().double() - ref).norm() <= 2.0 ** -8 * ref.norm()
