@@ -131,9 +131,21 @@ std::vector<Tensor> rnn_seq(int gates, const Tensor& proj, const Tensor& w, cons
                             const c10::optional<Tensor>& h0_, const c10::optional<Tensor>& c0_) {
   NoAutograd below;
   const Tensor bias = bias_.value_or(Tensor()), h0 = h0_.value_or(Tensor()), c0 = c0_.value_or(Tensor());
+  TORCH_CHECK_VALUE(proj.dim() == 3 && w.dim() == 2, "rnn_seq: [T, B, gates H] and [gates H, H] expected, got ",
+                    proj.sizes(), " and ", w.sizes());
+  const int64_t T = proj.size(0), B = proj.size(1), H = w.size(1), GH = gates * H;
+  TORCH_CHECK_VALUE(proj.size(2) == GH && w.size(0) == GH, "rnn_seq: sizes do not match: ", proj.sizes(), " and ", w.sizes());
+  TORCH_CHECK_VALUE(!bias.defined() || bias.sizes() == at::IntArrayRef({GH}), "rnn_seq: bias of [", GH, "] expected, got ",
+                    bias.sizes());
+  for (const Tensor* s : {&h0, &c0})
+    TORCH_CHECK_VALUE(!s->defined() || s->sizes() == at::IntArrayRef({B, H}), "rnn_seq: initial state of [", B, ", ", H,
+                      "] expected, got ", s->sizes());
+  check_on(proj, w, "the recurrent matrix");
+  if (bias.defined()) check_on(proj, bias, "the bias");
+  if (h0.defined()) check_on(proj, h0, "the initial hidden state");
+  if (c0.defined()) check_on(proj, c0, "the initial cell state");
+  TORCH_CHECK_VALUE(proj.is_cuda(), "rnn_seq: a CUDA input expected");
   Tensor x = f32c(proj), wc = contig(w);
-  const int64_t T = x.size(0), B = x.size(1), H = wc.size(1), GH = gates * H;
-  TORCH_CHECK_VALUE(x.size(2) == GH && wc.size(0) == GH, "rnn_seq: sizes do not match");
   Tensor b = bias.defined() ? contig(bias) : bias, h = h0.defined() ? f32c(h0) : h0, c = c0.defined() ? f32c(c0) : c0;
   const bool grad = wants_grad({&proj, &w, &bias, &h0, &c0});
   Tensor wt = empty({H, GH}, x, at::kFloat), hs = empty({T, B, H}, x, at::kFloat);

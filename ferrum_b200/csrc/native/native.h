@@ -66,6 +66,10 @@ inline ll rows_of(const Tensor& t) {
 }
 Tensor cast(const Tensor& t, at::ScalarType st);  // the cast kernel for fp32 <-> bf16, contiguous result
 inline Tensor f32c(const Tensor& t) { return contig(is_f32(t) ? t : cast(t, at::kFloat)); }
+// The kernels get bare pointers: what they read must be on the input's device and of the size they go by.
+inline void check_on(const Tensor& input, const Tensor& t, const char* what) {
+  TORCH_CHECK_VALUE(t.device() == input.device(), what, " is on ", t.device(), ", the input on ", input.device());
+}
 inline Tensor as2d(const Tensor& t) { return t.dim() == 2 ? t : t.reshape({-1, t.size(-1)}); }
 
 // ------------------------------------------------------------------------------------------------ autograd

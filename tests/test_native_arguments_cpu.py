@@ -1,0 +1,30 @@
+"""Arguments that the native host path refuses before any kernel gets a pointer (sizes and devices; no GPU needed)."""
+import pytest
+import torch
+
+
+def _native():
+    from ferrum_b200 import _lib
+
+    return _lib.native()
+
+
+@pytest.mark.parametrize("gates", [3, 4])
+@pytest.mark.parametrize("state,what", [((2, 8), "initial state"), ((1, 8), "initial state"), ((3, 9), "initial state"),
+                                        ((8,), "initial state"), ("meta", "on meta")])
+def test_initial_states(gates, state, what):
+    """An input of batch 3, hidden size 8: other sizes and devices of the hidden or the cell state."""
+    proj, w = torch.zeros(2, 3, gates * 8), torch.zeros(gates * 8, 8)
+    bad = torch.zeros(3, 8, device="meta") if state == "meta" else torch.zeros(*state)
+    with pytest.raises(ValueError, match=what):
+        _native().rnn_seq(gates, proj, w, None, bad, None)
+    with pytest.raises(ValueError, match=what):
+        _native().rnn_seq(gates, proj, w, None, None, bad)
+
+
+def test_recurrent_matrix_and_bias():
+    proj, w = torch.zeros(2, 3, 32), torch.zeros(32, 8)
+    for args in ((proj, torch.zeros(32, 7), None), (proj[0], w, None), (proj, w, torch.zeros(31)),
+                 (proj, w.to("meta"), None), (proj, w, torch.zeros(32, device="meta")), (proj, w, None)):
+        with pytest.raises(ValueError):
+            _native().rnn_seq(4, *args, None, None)
