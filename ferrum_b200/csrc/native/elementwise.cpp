@@ -180,8 +180,11 @@ struct NllNode : Node {
 
 Tensor nll(const Tensor& log_probs, const Tensor& target) {
   NoAutograd below;
+  const int64_t cols = log_probs.size(-1), rows = rows_of(log_probs);
+  TORCH_CHECK_VALUE(rows > 0 && target.numel() == rows, "nll: one target per row expected, got ", target.sizes(), " for ",
+                    log_probs.sizes());
+  check_on(log_probs, target, "the target");
   Tensor x = contig(log_probs), t = contig(target);
-  const int64_t cols = x.size(-1), rows = rows_of(x);
   Tensor loss = empty({}, x, at::kFloat), ws = empty({fb_mean_loss_workspace(rows)}, x, at::kFloat);
   FB_CALL(fb_nll_fwd, x.data_ptr(), reinterpret_cast<const ll*>(t.data_ptr<int64_t>()), loss.data_ptr<float>(),
           ws.data_ptr<float>(), rows, static_cast<int>(cols), -1.f / static_cast<float>(rows), dt(x), cur_stream());

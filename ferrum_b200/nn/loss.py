@@ -47,9 +47,10 @@ def _ce_onehot(log_probs, targets):
 
 
 def _nll_index(log_probs, targets):
-    if F._native(log_probs) and log_probs.numel() > 0:
-        return F.nll_index(log_probs, targets)
     C = log_probs.shape[-1]
+    if (F._native(log_probs) and targets.device == log_probs.device and log_probs.numel() > 0
+            and targets.numel() * C == log_probs.numel()):
+        return F.nll_index(log_probs, targets)
     lp2 = log_probs.reshape(-1, C)
     onehot = torch.zeros(lp2.shape, device=lp2.device, dtype=lp2.dtype)
     onehot.scatter_(1, targets.reshape(-1, 1).to(torch.int64), 1.0)

@@ -34,3 +34,17 @@ def test_elementwise_loss_sum(n):
     p, t = (torch.randn(n, device="cuda", generator=g) for _ in range(2))
     want = ((p.double() - t.double()) ** 2).mean().item()
     assert abs(nn.mse_loss(p, t).item() - want) <= 1e-5 * want
+
+
+def test_nll_targets_of_another_number_or_device():
+    """More targets than rows and targets on the CPU are errors; rows past the last target add nothing to the sum."""
+    from ferrum_b200 import nn
+
+    lp = torch.log_softmax(torch.randn(6, 5, device="cuda"), -1)
+    t = torch.randint(0, 5, (8,), device="cuda")
+    for bad in (t, t[:6].cpu()):
+        for fn in (nn.nll_loss, nn.cross_entropy_loss):
+            with pytest.raises((RuntimeError, ValueError)):
+                fn(lp, bad)
+    want = -lp[:4].gather(1, t[:4, None]).sum() / 6
+    assert abs(nn.nll_loss(lp, t[:4]).item() - want.item()) < 1e-6

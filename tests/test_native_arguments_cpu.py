@@ -28,3 +28,14 @@ def test_recurrent_matrix_and_bias():
                  (proj, w.to("meta"), None), (proj, w, torch.zeros(32, device="meta")), (proj, w, None)):
         with pytest.raises(ValueError):
             _native().rnn_seq(4, *args, None, None)
+
+
+def test_nll_targets():
+    lp = torch.zeros(4, 5)
+    for bad in (torch.zeros(3, dtype=torch.int64), torch.zeros(5, dtype=torch.int64)):
+        with pytest.raises(ValueError, match="one target per row"):
+            _native().nll(lp, bad)
+    with pytest.raises(ValueError, match="on meta"):
+        _native().nll(lp, torch.zeros(4, dtype=torch.int64, device="meta"))
+    with pytest.raises(ValueError, match="one target per row"):
+        _native().nll(lp[:0], torch.zeros(0, dtype=torch.int64))
