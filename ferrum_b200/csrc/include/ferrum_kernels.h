@@ -171,8 +171,9 @@ int fb_ce_fwd(const void* logits, const long long* labels, float* row_stats, flo
               long long rows, int cols, float scale, int dtype, cudaStream_t stream);
 int fb_ce_bwd(const void* logits, const long long* labels, const float* row_stats, const float* gout, void* dlogits,
               long long rows, int cols, float scale, int dtype, cudaStream_t stream);
+// a target outside [0, cols) is reported to the status block and makes the loss NaN
 int fb_nll_fwd(const void* log_probs, const long long* target, float* loss, float* workspace, long long rows, int cols,
-               float scale, int dtype, cudaStream_t stream);
+               float scale, int dtype, int32_t* status, cudaStream_t stream);
 int fb_nll_bwd(const long long* target, const float* gout, void* dlog_probs, long long rows, int cols, float scale,
                int dtype, cudaStream_t stream);
 int fb_loss_mean_fwd(const float* pred, const float* target, float* loss, float* workspace, long long n, int kind,

@@ -268,13 +268,13 @@ ce_bwd_kernel(const T* __restrict__ x, const long long* __restrict__ labels, con
 template <typename T, bool kClustered>
 __global__ void __launch_bounds__(kThreads)
 nll_fwd_kernel(const T* __restrict__ lp, const long long* __restrict__ target, float* __restrict__ loss,
-               float* __restrict__ partial, long long rows, int cols, float scale, int32_t* bstatus) {
+               float* __restrict__ partial, long long rows, int cols, float scale, int32_t* status) {
   float acc = 0.f;
   const long long stride = static_cast<long long>(gridDim.x) * kThreads;
   for (long long r = static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x; r < rows; r += stride) {
     const long long t = target[r];
-    if (t >= 0 && t < cols) acc += to_f(lp[r * cols + t]);
-    else (void)FB_INDEX_OK(bstatus, 42, t, cols);
+    // a class outside the range is an error: in the status block (every build), and the loss shows it
+    acc += check_index(status, 42, t, cols) ? to_f(lp[r * cols + t]) : __int_as_float(0x7fffffff);
   }
   finish<kClustered>(acc, scale, loss, partial);
 }
@@ -433,17 +433,16 @@ extern "C" int fb_ce_bwd(const void* logits, const long long* labels, const floa
 }
 
 extern "C" int fb_nll_fwd(const void* log_probs, const long long* target, float* loss, float* workspace, long long rows,
-                          int cols, float scale, int dtype, cudaStream_t stream) {
+                          int cols, float scale, int dtype, int32_t* status, cudaStream_t stream) {
   if (rows <= 0 || cols <= 0) return 0;
   const long long blocks = (rows + kThreads - 1) / kThreads;
   if (dtype == FB_DT_F32)
     return run_mean(nll_fwd_kernel<float, true>, nll_fwd_kernel<float, false>, rows, blocks, loss, workspace, scale,
-                    stream, static_cast<const float*>(log_probs), target, loss, workspace, rows, cols, scale,
-                    bounds_status_ref());
+                    stream, static_cast<const float*>(log_probs), target, loss, workspace, rows, cols, scale, status);
   if (dtype == FB_DT_BF16)
     return run_mean(nll_fwd_kernel<__nv_bfloat16, true>, nll_fwd_kernel<__nv_bfloat16, false>, rows, blocks, loss,
                     workspace, scale, stream, static_cast<const __nv_bfloat16*>(log_probs), target, loss, workspace,
-                    rows, cols, scale, bounds_status_ref());
+                    rows, cols, scale, status);
   return -1;
 }
 

@@ -187,7 +187,7 @@ Tensor nll(const Tensor& log_probs, const Tensor& target) {
   Tensor x = contig(log_probs), t = contig(target);
   Tensor loss = empty({}, x, at::kFloat), ws = empty({fb_mean_loss_workspace(rows)}, x, at::kFloat);
   FB_CALL(fb_nll_fwd, x.data_ptr(), reinterpret_cast<const ll*>(t.data_ptr<int64_t>()), loss.data_ptr<float>(),
-          ws.data_ptr<float>(), rows, static_cast<int>(cols), -1.f / static_cast<float>(rows), dt(x), cur_stream());
+          ws.data_ptr<float>(), rows, static_cast<int>(cols), -1.f / static_cast<float>(rows), dt(x), status(), cur_stream());
   if (!is_f32(x)) loss = cast(loss, x.scalar_type());
   if (wants_grad({&log_probs})) {
     auto n = make_node<NllNode>(log_probs);

@@ -48,3 +48,22 @@ def test_nll_targets_of_another_number_or_device():
                 fn(lp, bad)
     want = -lp[:4].gather(1, t[:4, None]).sum() / 6
     assert abs(nn.nll_loss(lp, t[:4]).item() - want.item()) < 1e-6
+
+
+@pytest.mark.parametrize("bad", [-1, 5])
+@pytest.mark.parametrize("rows", [6, 300000])
+def test_nll_class_out_of_range(rows, bad):
+    """Reported in the status block and by the loss itself; nothing is read outside the row."""
+    from ferrum_b200 import nn
+    from ferrum_b200.utils.runtime import DeviceStatusError, check_status
+
+    lp = torch.log_softmax(torch.randn(rows, 5, device="cuda"), -1).requires_grad_(True)
+    t = torch.randint(0, 5, (rows,), device="cuda")
+    t[rows // 2] = bad
+    check_status()
+    loss = nn.nll_loss(lp, t)
+    with pytest.raises(DeviceStatusError, match="bounds_violation"):
+        check_status()
+    assert loss.isnan()
+    loss.backward()
+    check_status()
