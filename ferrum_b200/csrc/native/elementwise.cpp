@@ -140,6 +140,9 @@ struct CrossEntropyNode : Node {
 
 Tensor cross_entropy(const Tensor& logits, const Tensor& labels) {
   NoAutograd below;
+  TORCH_CHECK_VALUE(logits.dim() == 2 && labels.numel() == logits.size(0),
+                    "cross_entropy: one label per row expected, got ", labels.sizes(), " for ", logits.sizes());
+  check_on(logits, labels, "the label tensor");
   Tensor x = contig(logits), lab = contig(labels);
   const int64_t rows = x.size(0);
   const bool grad = wants_grad({&logits});
@@ -225,6 +228,8 @@ struct ElemLossNode : Node {
 
 Tensor elementwise_loss(const Tensor& pred, const Tensor& target, int kind) {
   NoAutograd below;
+  TORCH_CHECK_VALUE(pred.sizes() == target.sizes(), "loss: predictions ", pred.sizes(), " and targets ", target.sizes());
+  check_on(pred, target, "the target");
   Tensor p = f32c(pred), t = f32c(target);
   const int64_t n = p.numel();
   Tensor loss = empty({}, p, at::kFloat), ws = empty({fb_mean_loss_workspace(n)}, p, at::kFloat);

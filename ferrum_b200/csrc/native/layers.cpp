@@ -40,6 +40,9 @@ struct EmbeddingNode : Node {
 
 Tensor embedding(const Tensor& weight, const Tensor& idx_, ll padding, bool pool, bool out_bf16, py::object sink) {
   NoAutograd below;
+  TORCH_CHECK_VALUE(weight.dim() == 2 && (!pool || idx_.dim() == 2), "embedding: a table of two dimensions expected, got ",
+                    weight.sizes(), " and indices ", idx_.sizes());
+  if (idx_.numel() > 0) check_on(weight, idx_, "the index tensor");
   Tensor w = contig(weight), idx = contig(idx_);
   const int64_t V = w.size(0), D = w.size(1);
   const auto st = out_bf16 ? at::kBFloat16 : at::kFloat;

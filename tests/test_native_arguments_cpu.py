@@ -39,3 +39,22 @@ def test_nll_targets():
         _native().nll(lp, torch.zeros(4, dtype=torch.int64, device="meta"))
     with pytest.raises(ValueError, match="one target per row"):
         _native().nll(lp[:0], torch.zeros(0, dtype=torch.int64))
+
+
+def test_cross_entropy_labels():
+    x = torch.zeros(4, 5)
+    for n in (3, 5):
+        with pytest.raises(ValueError, match="one label per row"):
+            _native().cross_entropy(x, torch.zeros(n, dtype=torch.int64))
+    with pytest.raises(ValueError, match="on meta"):
+        _native().cross_entropy(x, torch.zeros(4, dtype=torch.int64, device="meta"))
+
+
+def test_elementwise_targets_and_embedding_indices():
+    x, i = torch.zeros(4, 5), torch.zeros(2, 3, dtype=torch.int64)
+    for bad in (torch.zeros(4, 4), torch.zeros(20), torch.zeros(4, 5, device="meta")):
+        with pytest.raises(ValueError):
+            _native().elementwise_loss(x, bad, 0)
+    for weight, idx, pool in ((x, i.to("meta"), False), (x, i.to("meta"), True), (x, i[0], True), (x[0], i, False)):
+        with pytest.raises(ValueError):
+            _native().embedding(weight, idx, -1, pool, False, None)
