@@ -405,7 +405,7 @@ extern "C" long long fb_mean_loss_workspace(long long) { return kMaxPartials; }
 
 extern "C" int fb_ce_fwd(const void* logits, const long long* labels, float* row_stats, float* loss, float* workspace,
                          long long rows, int cols, float scale, int dtype, cudaStream_t stream) {
-  if (rows <= 0 || cols <= 0) return 0;
+  if (rows <= 0 || cols <= 0) return -1;  // no mean over nothing: `loss` stays unwritten
   if (dtype == FB_DT_F32) return ce_fwd<float>(logits, labels, row_stats, loss, workspace, rows, cols, scale, stream);
   if (dtype == FB_DT_BF16)
     return ce_fwd<__nv_bfloat16>(logits, labels, row_stats, loss, workspace, rows, cols, scale, stream);
@@ -434,7 +434,7 @@ extern "C" int fb_ce_bwd(const void* logits, const long long* labels, const floa
 
 extern "C" int fb_nll_fwd(const void* log_probs, const long long* target, float* loss, float* workspace, long long rows,
                           int cols, float scale, int dtype, int32_t* status, cudaStream_t stream) {
-  if (rows <= 0 || cols <= 0) return 0;
+  if (rows <= 0 || cols <= 0) return -1;  // no mean over nothing: `loss` stays unwritten
   const long long blocks = (rows + kThreads - 1) / kThreads;
   if (dtype == FB_DT_F32)
     return run_mean(nll_fwd_kernel<float, true>, nll_fwd_kernel<float, false>, rows, blocks, loss, workspace, scale,
@@ -466,7 +466,7 @@ extern "C" int fb_nll_bwd(const long long* target, const float* gout, void* dlog
 
 extern "C" int fb_loss_mean_fwd(const float* pred, const float* target, float* loss, float* workspace, long long n,
                                 int kind, float scale, cudaStream_t stream) {
-  if (n <= 0) return 0;
+  if (n <= 0) return -1;
   return run_mean(elem_loss_kernel<true>, elem_loss_kernel<false>, n, (n + 4 * kThreads - 1) / (4 * kThreads), loss,
                   workspace, scale, stream, pred, target, loss, workspace, n, kind, scale);
 }

@@ -142,6 +142,7 @@ Tensor cross_entropy(const Tensor& logits, const Tensor& labels) {
   NoAutograd below;
   TORCH_CHECK_VALUE(logits.dim() == 2 && labels.numel() == logits.size(0),
                     "cross_entropy: one label per row expected, got ", labels.sizes(), " for ", logits.sizes());
+  TORCH_CHECK_VALUE(logits.numel() > 0, "cross_entropy: no mean over an empty batch, got ", logits.sizes());
   check_on(logits, labels, "the label tensor");
   Tensor x = contig(logits), lab = contig(labels);
   const int64_t rows = x.size(0);

@@ -58,3 +58,16 @@ def test_elementwise_targets_and_embedding_indices():
     for weight, idx, pool in ((x, i.to("meta"), False), (x, i.to("meta"), True), (x, i[0], True), (x[0], i, False)):
         with pytest.raises(ValueError):
             _native().embedding(weight, idx, -1, pool, False, None)
+
+
+@pytest.mark.parametrize("shape", [(0, 5), (4, 0), (0, 0)])
+def test_no_mean_over_nothing(shape):
+    """The native op refuses, and so do the C entry points, which return before they touch their pointers."""
+    from ferrum_b200 import _lib
+
+    with pytest.raises(ValueError, match="empty"):
+        _native().cross_entropy(torch.zeros(shape), torch.zeros(shape[0], dtype=torch.int64))
+    lib = _lib.cuda()
+    assert lib.fb_ce_fwd(None, None, None, None, None, *shape, 1.0, 0, None) != 0
+    assert lib.fb_nll_fwd(None, None, None, None, *shape, 1.0, 0, None, None) != 0
+    assert lib.fb_loss_mean_fwd(None, None, None, None, 0, 0, 1.0, None) != 0
