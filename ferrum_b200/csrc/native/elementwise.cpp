@@ -231,6 +231,7 @@ Tensor elementwise_loss(const Tensor& pred, const Tensor& target, int kind) {
   NoAutograd below;
   TORCH_CHECK_VALUE(pred.sizes() == target.sizes(), "loss: predictions ", pred.sizes(), " and targets ", target.sizes());
   check_on(pred, target, "the target");
+  refuse_tangents({&target});
   Tensor p = f32c(pred), t = f32c(target);
   const int64_t n = p.numel();
   Tensor loss = empty({}, p, at::kFloat), ws = empty({fb_mean_loss_workspace(n)}, p, at::kFloat);

@@ -73,7 +73,14 @@ inline void check_on(const Tensor& input, const Tensor& t, const char* what) {
 inline Tensor as2d(const Tensor& t) { return t.dim() == 2 ? t : t.reshape({-1, t.size(-1)}); }
 
 // ------------------------------------------------------------------------------------------------ autograd
+// The ops run below the autograd keys: a tangent would be lost there without a word.
+inline void refuse_tangents(std::initializer_list<const Tensor*> ts) {
+  for (const Tensor* t : ts)
+    TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->_fw_grad(/*level=*/0).defined(),
+                                "this op has no forward-mode derivative (a dual tensor was given)");
+}
 inline bool wants_grad(std::initializer_list<const Tensor*> ts) {
+  refuse_tangents(ts);
   if (!at::GradMode::is_enabled()) return false;
   for (const Tensor* t : ts)
     if (t->defined() && t->requires_grad()) return true;

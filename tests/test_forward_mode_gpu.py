@@ -1,0 +1,40 @@
+"""The native ops have no forward-mode derivative: a dual input is refused, in either grad mode, instead of losing its
+tangent."""
+import pytest
+import torch
+import torch.autograd.forward_ad as fwd
+
+pytestmark = pytest.mark.gpu
+
+
+def _calls(d):
+    from ferrum_b200.ops import functional as F
+
+    w, b, one = (torch.randn(*s, device="cuda") for s in ((6, 8), (6,), (8,)))
+    t = torch.zeros(4, dtype=torch.int64, device="cuda")
+    q = torch.randn(1, 1, 8, 4, device="cuda")
+    return {
+        "linear": lambda: F.linear(d, w, b),
+        "linear_act_layernorm": lambda: F.linear_act_layernorm(d, w, b, b, b),
+        "layer_norm": lambda: F.layer_norm(d, one, one),
+        "unary": lambda: F.unary(d, "exp"),
+        "add": lambda: F.binary(d, d, "add"),
+        "softmax": lambda: F.softmax(d),
+        "cross_entropy": lambda: F.cross_entropy_logits(d, t),
+        "nll": lambda: F.nll_index(d, t),
+        "mse": lambda: F.elementwise_loss(d, torch.zeros_like(w[:4, :1]).expand(4, 8), "mse"),
+        "mse_target": lambda: F.elementwise_loss(torch.zeros(4, 8, device="cuda"), d, "mse"),
+        "bmm": lambda: F.bmm_scaled(d.reshape(1, 1, 4, 8), q),
+        "embedding": lambda: F.embedding(d, t),
+        "rnn": lambda: F.rnn_sequence(4, d.reshape(4, 1, 8), torch.randn(8, 2, device="cuda"), None),
+    }
+
+
+@pytest.mark.parametrize("grad", [True, False])
+def test_dual_inputs_are_refused(grad):
+    with fwd.dual_level(), torch.set_grad_enabled(grad):
+        d = fwd.make_dual(torch.randn(4, 8, device="cuda"), torch.ones(4, 8, device="cuda"))
+        for name, call in _calls(d).items():
+            with pytest.raises(NotImplementedError):
+                call()
+                pytest.fail(name)
