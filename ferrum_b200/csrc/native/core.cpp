@@ -86,6 +86,7 @@ void gemm(const Op& a, const Op& b, const float* bias, int act, void* out, ll ld
           void* act_grad, const Tensor* like, bool tf32, bool splits) {
   const int M = static_cast<int>(a.rows), N = static_cast<int>(b.rows), K = static_cast<int>(a.k);
   TORCH_CHECK(a.k == b.k, "inner dimensions differ: [", a.rows, ", ", a.k, "] x [", b.rows, ", ", b.k, "]^T");
+  TORCH_CHECK(act <= FB_ACT_SIGMOID, "gemm: no epilogue evaluates activation ", act);
   if (M == 0 || N == 0) return;
   const bool ok = tma_ok(a) && tma_ok(b);
   const int a_mn = a.s_k == 1 ? 0 : 1, b_mn = b.s_k == 1 ? 0 : 1;

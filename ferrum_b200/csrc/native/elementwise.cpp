@@ -32,6 +32,8 @@ struct UnaryNode : Node {
   }
 };
 
+}  // namespace
+
 Tensor unary(const Tensor& x, int op, double alpha, double beta) {
   NoAutograd below;
   Tensor xc = contig(x), y = empty(x.sizes(), x, x.scalar_type());
@@ -48,6 +50,8 @@ Tensor unary(const Tensor& x, int op, double alpha, double beta) {
   }
   return y;
 }
+
+namespace {
 
 // Same-shape add, the residual connection: fp32 result of any mix of fp32 and bf16 operands (bf16 of two bf16 ones).
 struct AddNode : Node {

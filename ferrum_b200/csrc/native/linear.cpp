@@ -172,8 +172,12 @@ struct LayerNormNode : Node {
   }
 };
 
+// The normalisation kernels evaluate a GELU in front of the statistics; any other activation is an op of its own.
+bool norm_evaluates(int act) { return act == kNone || act == FB_ACT_GELU; }
+
 Tensor layer_norm(const Tensor& x, const c10::optional<Tensor>& gamma_, const c10::optional<Tensor>& beta_, double eps,
                   int pre) {
+  if (!norm_evaluates(pre)) return layer_norm(unary(x, pre, 0., 0.), gamma_, beta_, eps, kNone);
   NoAutograd below;
   const Tensor gamma = gamma_.value_or(Tensor()), beta = beta_.value_or(Tensor());
   Tensor xc = contig(x);
@@ -234,6 +238,8 @@ struct LinearActNormNode : Node {
 Tensor linear_act_norm(const Tensor& x, const Tensor& weight, const c10::optional<Tensor>& bias_, const Tensor& gamma,
                        const Tensor& beta, double eps, int act, bool low, bool tf32,
                        const c10::optional<Tensor>& w_low, py::object sink) {
+  if (!low && !norm_evaluates(act))
+    return layer_norm(linear(x, weight, bias_, kNone, low, tf32, w_low, sink), gamma, beta, eps, act);
   NoAutograd below;
   const Tensor bias = bias_.value_or(Tensor());
   Operands o = operands(x, weight, w_low.value_or(Tensor()), low);
@@ -243,6 +249,9 @@ Tensor linear_act_norm(const Tensor& x, const Tensor& weight, const c10::optiona
   Tensor g = contig(gamma), be = contig(beta);
   Tensor z = empty({M, N}, o.x2, low ? at::kBFloat16 : at::kFloat), dact;
   const bool fused = low && act != kNone && tma_ok(op2d(o.x2)) && tma_ok(op2d(o.w));
+  if (fused && act > FB_ACT_SIGMOID) throw py::key_error("linear_act_layernorm: an activation that no epilogue evaluates");
+  if (!fused && !norm_evaluates(act))
+    return layer_norm(linear(x, weight, bias_, kNone, low, tf32, w_low, sink), gamma, beta, eps, act);
   if (fused && grad) dact = empty({M, N}, o.x2, at::kBFloat16);
   gemm(op2d(o.x2), op2d(o.w), fptr(b), fused ? act : kNone, z.data_ptr(), N, low, false, ptr(dact), &o.x2,
        tf32 && !low);

@@ -95,6 +95,8 @@ inline std::shared_ptr<N> make_node(const T&... inputs) {
 // Inside an op and inside a node's apply: the tensor methods used there record nothing of their own.
 typedef at::AutoDispatchBelowADInplaceOrView NoAutograd;
 
+Tensor unary(const Tensor& x, int op, double alpha, double beta);
+
 // ---------------------------------------------------------------------------------------------------- GEMM
 // A GEMM operand as an [rows, K] view given by element strides.
 struct Op {

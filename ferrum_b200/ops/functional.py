@@ -435,7 +435,7 @@ def _gemm_nt(a: torch.Tensor, b_nt: torch.Tensor, bias=None, act=None, low: bool
     if out is None:
         out = torch.empty((a.shape[0], b_nt.shape[0]), device=a.device, dtype=out_dtype or dt)
         accumulate = False
-    _lib.native().gemm_nt(ab, bb, bias, UNARY[act or "none"], out, accumulate, not low and config.tf32_active())
+    _lib.native().gemm_nt(ab, bb, bias, _gemm.ACT[act], out, accumulate, not low and config.tf32_active())
     return out
 
 
@@ -663,7 +663,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
     if act is not None and act not in _FUSABLE_ACT and torch.is_grad_enabled() and (
             x.requires_grad or weight.requires_grad):
         return unary(_lib.native().linear(x, weight, bias, 0, low, tf32, w_low, sink), act)
-    return _lib.native().linear(x, weight, bias, UNARY[act or "none"], low, tf32, w_low, sink)
+    # the activations a GEMM epilogue evaluates; another name is a KeyError
+    return _lib.native().linear(x, weight, bias, _gemm.ACT[act], low, tf32, w_low, sink)
 
 
 # =============================================================================== normalisation
