@@ -47,7 +47,9 @@ def test_linear_act_layernorm(act, K, low):
     leaves = [t.detach().double().requires_grad_(True) for t in (x, w, b, gamma, beta)]
     z = torch.nn.functional.linear(*leaves[:3])
     z = z if act is None else {"gelu": lambda t: torch.nn.functional.gelu(t, approximate="tanh"),
-                               "leaky_relu": lambda t: torch.nn.functional.leaky_relu(t, 0.0)}.get(
+                               # a name carries no parameter: alpha = 0 in both
+                               "leaky_relu": lambda t: torch.nn.functional.leaky_relu(t, 0.0),
+                               "elu": lambda t: torch.nn.functional.elu(t, 0.0)}.get(
         act, getattr(torch.nn.functional, act))(z)
     r = torch.nn.functional.layer_norm(z, (40,), leaves[3], leaves[4])
     r.backward(up.double())
