@@ -661,7 +661,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
     low = config.low_precision_active()
     tf32 = not low and config.tf32_active()
     if act is not None and act not in _FUSABLE_ACT and torch.is_grad_enabled() and (
-            x.requires_grad or weight.requires_grad):
+            x.requires_grad or weight.requires_grad or (bias is not None and bias.requires_grad)):
         return unary(_lib.native().linear(x, weight, bias, 0, low, tf32, w_low, sink), act)
     # the activations a GEMM epilogue evaluates; another name is a KeyError
     return _lib.native().linear(x, weight, bias, _gemm.ACT[act], low, tf32, w_low, sink)

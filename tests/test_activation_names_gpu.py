@@ -56,3 +56,17 @@ def test_linear_act_layernorm(act, K, low):
     bound = 3e-2 if low else 2e-5
     for got, want in [(y, r)] + [(t.grad, s.grad) for t, s in zip((x, w, b, gamma, beta), leaves)]:
         assert (got.double() - want).norm() <= bound * want.norm() + 1e-5
+
+
+@pytest.mark.parametrize("act", ["gelu", "silu", "relu"])
+def test_bias_alone_trained(act):
+    """The derivative of a GELU is no function of its output, whichever of the operands is trained."""
+    from ferrum_b200.ops import functional as F
+
+    x, w, b = (torch.randn(*s, device="cuda") for s in ((16, 32), (24, 32), (24,)))
+    b.requires_grad_(True)
+    F.linear(x, w, b, act).sum().backward()
+    d = b.detach().double().requires_grad_(True)
+    z = torch.nn.functional.linear(x.double(), w.double(), d)
+    (torch.nn.functional.gelu(z, approximate="tanh") if act == "gelu" else getattr(torch.nn.functional, act)(z)).sum().backward()
+    assert (b.grad.double() - d.grad).norm() <= 1e-5 * d.grad.norm()
