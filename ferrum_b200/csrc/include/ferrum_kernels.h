@@ -164,13 +164,11 @@ int fb_softmax_bwd(const void* dy, const void* y, void* dx, long long rows, int 
 int fb_ce_fwd_bwd(const void* logits, const long long* labels, float* row_loss, void* dlogits, long long rows,
                   int cols, float grad_scale, int dtype, int dlogits_dtype, cudaStream_t stream);
 // Mean losses (kernels/mean_loss.cu): the scalar scale * sum lands in `loss`; workspace = fb_mean_loss_workspace(n)
-// floats.  row_stats (optional) [rows][2]: row maximum and sum of exponentials, what the backward pass reads.
-// gout: the incoming scalar gradient, read on the device.
+// floats.  dlogits (optional, of the logits' type): (softmax - onehot) * scale.  gout: the incoming scalar gradient, read
+// on the device.
 long long fb_mean_loss_workspace(long long n);
-int fb_ce_fwd(const void* logits, const long long* labels, float* row_stats, float* loss, float* workspace,
-              long long rows, int cols, float scale, int dtype, cudaStream_t stream);
-int fb_ce_bwd(const void* logits, const long long* labels, const float* row_stats, const float* gout, void* dlogits,
-              long long rows, int cols, float scale, int dtype, cudaStream_t stream);
+int fb_ce_fwd(const void* logits, const long long* labels, void* dlogits, float* loss, float* workspace, long long rows,
+              int cols, float scale, int dtype, cudaStream_t stream);
 // a target outside [0, cols) is reported to the status block and makes the loss NaN
 int fb_nll_fwd(const void* log_probs, const long long* target, float* loss, float* workspace, long long rows, int cols,
                float scale, int dtype, int32_t* status, cudaStream_t stream);

@@ -6,9 +6,8 @@
 // blocks leave one partial sum each and a one-block kernel adds them in order.  The line between the two lies where
 // eight SMs stream the input in about the time that the second launch takes (256 K elements).
 //
-// The cross-entropy keeps {row maximum, sum of exponentials} per row and writes the logit gradient once, in the
-// backward pass, with the incoming gradient applied; writing it in the forward pass and scaling it afterwards read
-// and wrote the whole matrix one more time (8192 x 1000 bf16: 11.4 + 2.0 + 2.0 + 6.3 us in four launches).
+// The cross-entropy writes the logit gradient of a unit loss in the forward pass, from the exponentials it has at hand,
+// and the backward pass scales it by the incoming gradient: the logits are the caller's again once the loss is known.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -132,10 +131,10 @@ struct Vec {
 // Rows of 264 .. 4096 bf16 logits (multiples of 8, 16-byte aligned): a warp owns a row and keeps it in registers (K
 // vectors of 8 per lane), so the row is read once and both reductions are warp shuffles.
 template <int K, bool kClustered>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, K <= 4 ? 4 : (K <= 8 ? 2 : 1))
 ce_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const long long* __restrict__ labels,
-                   float2* __restrict__ row_stats, float* __restrict__ loss, float* __restrict__ partial,
-                   long long rows, int cols, float scale, int32_t* bstatus) {
+                   __nv_bfloat16* __restrict__ dx, float* __restrict__ loss, float* __restrict__ partial, long long rows,
+                   int cols, float scale, int32_t* bstatus) {
   const int lane = threadIdx.x & 31;
   const int nvec = cols >> 3;
   const long long nwarps = static_cast<long long>(gridDim.x) * (kThreads / 32);
@@ -163,23 +162,40 @@ ce_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const long long* __restr
 #pragma unroll
     for (int k = 0; k < K; ++k)
 #pragma unroll
-      for (int e = 0; e < 8; ++e) s += __expf(v[k][e] - m);  // padded lanes: exp(-huge) = 0
+      for (int e = 0; e < 8; ++e) {
+        v[k][e] = __expf(v[k][e] - m);  // padded lanes: exp(-huge) = 0
+        s += v[k][e];
+      }
     s = warp_sum(s);
+    const long long lab = labels[row];
+    const bool valid = lab >= 0 && lab < cols;  // out-of-range labels contribute nothing
     if (lane == 0) {
-      const long long lab = labels[row];
-      const bool valid = lab >= 0 && lab < cols;  // out-of-range labels contribute nothing
       if (!valid) (void)FB_INDEX_OK(bstatus, 41, lab, cols);
       if (valid) acc += m + logf(s) - __bfloat162float(xr[lab]);
-      if (row_stats != nullptr) row_stats[row] = make_float2(m, s);
+    }
+    if (dx != nullptr) {
+      const float inv = valid ? scale / s : 0.f;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const int vi = lane + 32 * k;
+        if (vi >= nvec) continue;
+        float d[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          d[e] = v[k][e] * inv;
+          if (valid && vi * 8 + e == lab) d[e] -= scale;
+        }
+        Vec<__nv_bfloat16>::store(dx + row * cols + vi * 8, d);
+      }
     }
   }
   finish<kClustered>(acc, scale, loss, partial);
 }
 
-// Any other row: TPR threads per row, the row is read again from L1 for the sum.
+// Any other row: TPR threads per row, the row is read again from L1 for the sum and for the gradient.
 template <typename T, int TPR, bool kClustered>
 __global__ void __launch_bounds__(kThreads)
-ce_fwd_kernel(const T* __restrict__ x, const long long* __restrict__ labels, float2* __restrict__ row_stats,
+ce_fwd_kernel(const T* __restrict__ x, const long long* __restrict__ labels, T* __restrict__ dx,
               float* __restrict__ loss, float* __restrict__ partial, long long rows, int cols, float scale,
               int32_t* bstatus) {
   __shared__ float smem[kThreads / 32];
@@ -198,71 +214,22 @@ ce_fwd_kernel(const T* __restrict__ x, const long long* __restrict__ labels, flo
     if (live)
       for (int c = t; c < cols; c += TPR) s += expf(to_f(xr[c]) - m);
     s = group_reduce<TPR, false>(s, smem);
+    const long long lab = live ? labels[row] : -1;
+    const bool valid = lab >= 0 && lab < cols;
     if (live && t == 0) {
-      const long long lab = labels[row];
-      const bool valid = lab >= 0 && lab < cols;
       if (!valid) (void)FB_INDEX_OK(bstatus, 41, lab, cols);
       if (valid) acc += m + logf(s) - to_f(xr[lab]);
-      if (row_stats != nullptr) row_stats[row] = make_float2(m, s);
+    }
+    if (live && dx != nullptr) {
+      const float inv = 1.f / s;
+      for (int c = t; c < cols; c += TPR) {
+        float f = expf(to_f(xr[c]) - m) * inv;
+        if (c == lab) f -= 1.f;
+        put(dx + row * cols + c, valid ? f * scale : 0.f);
+      }
     }
   }
   finish<kClustered>(acc, scale, loss, partial);
-}
-
-// One warp per row; the exponential and the order of the factors are those of the forward kernel's row class.
-template <typename T>
-__global__ void __launch_bounds__(kThreads)
-ce_bwd_kernel(const T* __restrict__ x, const long long* __restrict__ labels, const float2* __restrict__ row_stats,
-              const float* __restrict__ gout, T* __restrict__ dx, long long rows, int cols, float scale, int vec) {
-  const int lane = threadIdx.x & 31;
-  const long long nwarps = static_cast<long long>(gridDim.x) * (kThreads / 32);
-  const float g = gout[0];
-  for (long long row = static_cast<long long>(blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5); row < rows;
-       row += nwarps) {
-    const T* xr = x + row * cols;
-    T* dr = dx + row * cols;
-    const float2 st = row_stats[row];
-    const long long lab = labels[row];
-    const bool valid = lab >= 0 && lab < cols;
-    if (sizeof(T) == 2 && vec) {
-      const float inv = valid ? scale / st.y : 0.f;
-      constexpr int N = Vec<T>::n;
-#pragma unroll 4
-      for (int c = lane * N; c < cols; c += 32 * N) {
-        float f[N];
-        Vec<T>::load(xr + c, f);
-#pragma unroll
-        for (int e = 0; e < N; ++e) {
-          f[e] = __expf(f[e] - st.x) * inv;
-          if (valid && c + e == lab) f[e] -= scale;
-          f[e] *= g;
-        }
-        Vec<T>::store(dr + c, f);
-      }
-    } else if (vec) {
-      const float inv = 1.f / st.y;
-      constexpr int N = Vec<T>::n;
-#pragma unroll 4
-      for (int c = lane * N; c < cols; c += 32 * N) {
-        float f[N];
-        Vec<T>::load(xr + c, f);
-#pragma unroll
-        for (int e = 0; e < N; ++e) {
-          f[e] = expf(f[e] - st.x) * inv;
-          if (c + e == lab) f[e] -= 1.f;
-          f[e] = valid ? f[e] * scale * g : 0.f;
-        }
-        Vec<T>::store(dr + c, f);
-      }
-    } else {
-      const float inv = 1.f / st.y;
-      for (int c = lane; c < cols; c += 32) {
-        float f = expf(to_f(xr[c]) - st.x) * inv;
-        if (c == lab) f -= 1.f;
-        put(dr + c, valid ? f * scale * g : 0.f);
-      }
-    }
-  }
 }
 
 template <typename T, bool kClustered>
@@ -368,19 +335,19 @@ bool vec_ok(const void* a, const void* b, int cols, size_t elem) {
   return cols % static_cast<int>(16 / elem) == 0 &&
          ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0;
 }
-// Rows that the register-resident warp kernel takes; the backward pass follows the same line.
-bool warp_row(const void* x, int cols) { return cols >= 264 && cols <= 4096 && vec_ok(x, nullptr, cols, 2); }
+// Rows that the register-resident warp kernel takes.
+bool warp_row(const void* x, const void* dx, int cols) { return cols >= 264 && cols <= 4096 && vec_ok(x, dx, cols, 2); }
 
 template <typename T>
-int ce_fwd(const void* x, const long long* labels, float* row_stats, float* loss, float* partial, long long rows,
-           int cols, float scale, cudaStream_t st) {
-  float2* stats = reinterpret_cast<float2*>(row_stats);
+int ce_fwd(const void* x, const long long* labels, void* dlogits, float* loss, float* partial, long long rows, int cols,
+           float scale, cudaStream_t st) {
+  T* dx = static_cast<T*>(dlogits);
   if constexpr (sizeof(T) == 2) {
-    if (warp_row(x, cols)) {
+    if (warp_row(x, dx, cols)) {
       const int k = (cols / 8 + 31) / 32;
 #define FB_CE_WARP(K)                                                                                                  \
   return run_mean(ce_fwd_warp_kernel<K, true>, ce_fwd_warp_kernel<K, false>, rows * cols, (rows + 7) / 8, loss, partial, \
-                  scale, st, static_cast<const __nv_bfloat16*>(x), labels, stats, loss, partial, rows, cols, scale,      \
+                  scale, st, static_cast<const __nv_bfloat16*>(x), labels, dx, loss, partial, rows, cols, scale,      \
                   bounds_status_ref())
       if (k <= 4) FB_CE_WARP(4);
       if (k <= 8) FB_CE_WARP(8);
@@ -390,10 +357,10 @@ int ce_fwd(const void* x, const long long* labels, float* row_stats, float* loss
   }
   if (cols <= 512)
     return run_mean(ce_fwd_kernel<T, 32, true>, ce_fwd_kernel<T, 32, false>, rows * cols, (rows + 7) / 8, loss, partial,
-                    scale, st, static_cast<const T*>(x), labels, stats, loss, partial, rows, cols, scale,
+                    scale, st, static_cast<const T*>(x), labels, dx, loss, partial, rows, cols, scale,
                     bounds_status_ref());
   return run_mean(ce_fwd_kernel<T, 256, true>, ce_fwd_kernel<T, 256, false>, rows * cols, rows, loss, partial, scale, st,
-                  static_cast<const T*>(x), labels, stats, loss, partial, rows, cols, scale, bounds_status_ref());
+                  static_cast<const T*>(x), labels, dx, loss, partial, rows, cols, scale, bounds_status_ref());
 }
 
 }  // namespace
@@ -403,33 +370,13 @@ using namespace fb;
 
 extern "C" long long fb_mean_loss_workspace(long long) { return kMaxPartials; }
 
-extern "C" int fb_ce_fwd(const void* logits, const long long* labels, float* row_stats, float* loss, float* workspace,
+extern "C" int fb_ce_fwd(const void* logits, const long long* labels, void* dlogits, float* loss, float* workspace,
                          long long rows, int cols, float scale, int dtype, cudaStream_t stream) {
   if (rows <= 0 || cols <= 0) return -1;  // no mean over nothing: `loss` stays unwritten
-  if (dtype == FB_DT_F32) return ce_fwd<float>(logits, labels, row_stats, loss, workspace, rows, cols, scale, stream);
+  if (dtype == FB_DT_F32) return ce_fwd<float>(logits, labels, dlogits, loss, workspace, rows, cols, scale, stream);
   if (dtype == FB_DT_BF16)
-    return ce_fwd<__nv_bfloat16>(logits, labels, row_stats, loss, workspace, rows, cols, scale, stream);
+    return ce_fwd<__nv_bfloat16>(logits, labels, dlogits, loss, workspace, rows, cols, scale, stream);
   return -1;
-}
-
-extern "C" int fb_ce_bwd(const void* logits, const long long* labels, const float* row_stats, const float* gout,
-                         void* dlogits, long long rows, int cols, float scale, int dtype, cudaStream_t stream) {
-  if (rows <= 0 || cols <= 0) return 0;
-  long long nb = (rows + 7) / 8;
-  const long long cap = static_cast<long long>(sm_count()) * 8;
-  if (nb > cap) nb = cap;
-  const float2* st = reinterpret_cast<const float2*>(row_stats);
-  if (dtype == FB_DT_F32)
-    ce_bwd_kernel<float><<<static_cast<int>(nb), kThreads, 0, stream>>>(
-        static_cast<const float*>(logits), labels, st, gout, static_cast<float*>(dlogits), rows, cols, scale,
-        vec_ok(logits, dlogits, cols, 4));
-  else if (dtype == FB_DT_BF16)
-    ce_bwd_kernel<__nv_bfloat16><<<static_cast<int>(nb), kThreads, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(logits), labels, st, gout, static_cast<__nv_bfloat16*>(dlogits), rows, cols,
-        scale, warp_row(logits, cols) && vec_ok(logits, dlogits, cols, 2));
-  else
-    return -1;
-  return static_cast<int>(cudaGetLastError());
 }
 
 extern "C" int fb_nll_fwd(const void* log_probs, const long long* target, float* loss, float* workspace, long long rows,

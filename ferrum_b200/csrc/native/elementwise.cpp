@@ -117,27 +117,23 @@ Tensor softmax(const Tensor& x, bool log_mode) {
 }
 
 // -------------------------------------------------------------------------------------------------- losses
-// Mean cross-entropy of logits and integer labels.  The forward pass keeps the maximum and the sum of exponentials of each row; the logit
-// gradient is written once, in the backward pass, with the incoming gradient applied (read on the device).
+// Mean cross-entropy of logits and integer labels.  The forward pass writes the logit gradient of a unit loss, the
+// backward pass multiplies it by the incoming gradient (read on the device).
 struct CrossEntropyNode : Node {
-  SavedVariable x_, labels_;  // saved, so that labels changed before the backward pass are noticed
-  Tensor lse;
+  SavedVariable dx_, labels_;  // labels: saved, so that labels changed before the backward pass are noticed
   std::string name() const override { return "FerrumCrossEntropyBackward"; }
   void release_variables() override {
-    x_.reset_data();
+    dx_.reset_data();
     labels_.reset_data();
-    lse = Tensor();
   }
   variable_list apply(variable_list&& grads) override {
     NoAutograd below;
     variable_list out(1);
     if (!grads[0].defined()) return out;
-    Tensor x = contig(x_.unpack()), labels = labels_.unpack(), g = f32c(grads[0]);
-    Tensor dx = empty(x.sizes(), x, x.scalar_type());
-    FB_CALL(fb_ce_bwd, x.data_ptr(), reinterpret_cast<const ll*>(labels.data_ptr<int64_t>()), lse.data_ptr<float>(),
-            g.data_ptr<float>(), dx.data_ptr(), x.size(0), static_cast<int>(x.size(1)),
-            1.f / static_cast<float>(x.size(0)), dt(x), cur_stream());
-    out[0] = dx;
+    labels_.unpack();
+    Tensor dx = dx_.unpack(), g = f32c(grads[0]), y = empty(dx.sizes(), dx, dx.scalar_type());
+    FB_CALL(fb_scale_by_device_scalar, dx.data_ptr(), g.data_ptr<float>(), y.data_ptr(), dx.numel(), dt(dx), cur_stream());
+    out[0] = y;
     return out;
   }
 };
@@ -151,16 +147,14 @@ Tensor cross_entropy(const Tensor& logits, const Tensor& labels) {
   Tensor x = contig(logits), lab = contig(labels);
   const int64_t rows = x.size(0);
   const bool grad = wants_grad({&logits});
-  Tensor loss = empty({}, x, at::kFloat), lse = grad ? empty({rows, 2}, x, at::kFloat) : Tensor();
+  Tensor loss = empty({}, x, at::kFloat), dx = grad ? empty(x.sizes(), x, x.scalar_type()) : Tensor();
   Tensor ws = empty({fb_mean_loss_workspace(rows)}, x, at::kFloat);
-  FB_CALL(fb_ce_fwd, x.data_ptr(), reinterpret_cast<const ll*>(lab.data_ptr<int64_t>()), fptr_mut(lse),
-          loss.data_ptr<float>(), ws.data_ptr<float>(), rows, static_cast<int>(x.size(1)),
-          1.f / static_cast<float>(rows), dt(x), cur_stream());
+  FB_CALL(fb_ce_fwd, x.data_ptr(), reinterpret_cast<const ll*>(lab.data_ptr<int64_t>()), ptr(dx), loss.data_ptr<float>(),
+          ws.data_ptr<float>(), rows, static_cast<int>(x.size(1)), 1.f / static_cast<float>(rows), dt(x), cur_stream());
   if (grad) {
     auto n = make_node<CrossEntropyNode>(logits);
-    n->x_ = SavedVariable(x.is_alias_of(logits) ? logits : x, false);
+    n->dx_ = SavedVariable(dx, false);
     n->labels_ = SavedVariable(lab, false);
-    n->lse = lse;
     torch::autograd::set_history(loss, n);
   }
   return loss;

@@ -1,0 +1,26 @@
+"""What a backward pass keeps: results and inputs that a user may change in place, and tensors that saved-tensor hooks
+see."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_logits_changed_after_cross_entropy(dtype):
+    from ferrum_b200 import nn
+
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(40, 304, device="cuda", generator=g).to(dtype).requires_grad_(True)
+    t = torch.randint(0, 304, (40,), device="cuda", generator=g)
+    grads = []
+    for change in (False, True):
+        x.grad = None
+        logits = x * 1
+        loss = nn.cross_entropy(logits, t)
+        if change:
+            logits.detach().zero_()
+            logits.sigmoid_()
+        loss.backward()
+        grads.append(x.grad)
+    assert torch.equal(*grads)
