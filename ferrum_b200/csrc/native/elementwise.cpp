@@ -205,8 +205,9 @@ Tensor nll(const Tensor& log_probs, const Tensor& target) {
 
 // mse / bce / l1 / smooth_l1, mean over all elements; predictions fp32 or bf16, targets likewise.
 struct ElemLossNode : Node {
-  SavedVariable p_, t_;
+  SavedVariable p_, t_;  // as the kernels read them: the arguments themselves only where they were not converted
   int kind = 0;
+  at::ScalarType st = at::kFloat;
   std::string name() const override { return "FerrumElementwiseLossBackward"; }
   void release_variables() override {
     p_.reset_data();
@@ -216,11 +217,11 @@ struct ElemLossNode : Node {
     NoAutograd below;
     variable_list out(1);
     if (!grads[0].defined()) return out;
-    Tensor p = p_.unpack(), t = t_.unpack(), pc = f32c(p), g = f32c(grads[0]);
-    Tensor dp = empty(p.sizes(), pc, at::kFloat);
-    FB_CALL(fb_loss_bwd, pc.data_ptr<float>(), t.data_ptr<float>(), g.data_ptr<float>(), dp.data_ptr<float>(),
-            pc.numel(), kind, 1.f / static_cast<float>(pc.numel()), cur_stream());
-    out[0] = cast(dp, p.scalar_type());
+    Tensor p = p_.unpack(), t = t_.unpack(), g = f32c(grads[0]);
+    Tensor dp = empty(p.sizes(), p, at::kFloat);
+    FB_CALL(fb_loss_bwd, p.data_ptr<float>(), t.data_ptr<float>(), g.data_ptr<float>(), dp.data_ptr<float>(), p.numel(),
+            kind, 1.f / static_cast<float>(p.numel()), cur_stream());
+    out[0] = cast(dp, st);
     return out;
   }
 };
@@ -237,9 +238,10 @@ Tensor elementwise_loss(const Tensor& pred, const Tensor& target, int kind) {
           kind, 1.f / static_cast<float>(n), cur_stream());
   if (wants_grad({&pred})) {
     auto nd = make_node<ElemLossNode>(pred);
-    nd->p_ = SavedVariable(pred, false);
+    nd->p_ = SavedVariable(p, false);
     nd->t_ = SavedVariable(t, false);
     nd->kind = kind;
+    nd->st = pred.scalar_type();
     torch::autograd::set_history(loss, nd);
   }
   return loss;

@@ -24,3 +24,21 @@ def test_logits_changed_after_cross_entropy(dtype):
         loss.backward()
         grads.append(x.grad)
     assert torch.equal(*grads)
+
+
+@pytest.mark.parametrize("kind", ["mse", "l1"])
+def test_bf16_predictions_changed_after_the_loss(kind):
+    from ferrum_b200 import nn
+
+    x, t = (torch.randn(6, 5, device="cuda").bfloat16() for _ in range(2))
+    x.requires_grad_(True)
+    grads = []
+    for change in (False, True):
+        x.grad = None
+        p = x * 1
+        loss = getattr(nn, f"{kind}_loss")(p, t.clone())
+        if change:
+            p.mul_(2)
+        loss.backward()
+        grads.append(x.grad)
+    assert torch.equal(*grads)
