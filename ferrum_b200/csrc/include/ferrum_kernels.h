@@ -195,12 +195,12 @@ int fb_gru_gates_fwd(const float* xi, const float* hh, const float* h_prev, floa
 int fb_gru_gates_bwd(const float* dh, const float* saved, const float* h_prev, float* dxi, float* dhh,
                      float* dh_prev, long long B, int H, cudaStream_t stream);
 // Whole sequences (kernels/rnn_seq.cu), gates = 4 (LSTM) or 3 (GRU): xi [T, B, gates H] input projections, w_t [H,
-// gates H] transposed recurrent matrix, hs [T, B, H]; cs / saved / c_last as the backward call reads them (NULL: not
-// kept).  Backward: w [gates H, H]; dxi and, for GRU, dhh [T, B, gates H].  h0, c0 and the incoming gradients may be NULL.
+// gates H] transposed recurrent matrix, hs [T, B, H]; hs_kept (a second hs, so that the first is the caller's) / cs /
+// saved / c_last as the backward call reads them (NULL: not kept).  Backward: w [gates H, H]; dxi and, for GRU, dhh [T, B, gates H].  h0, c0 and the incoming gradients may be NULL.
 int fb_rnn_seq_supported(int gates, int B, int H);
 int fb_rnn_seq_fwd(int gates, const float* xi, const float* w_t, const float* bias, const float* h0, const float* c0,
-                   float* hs, float* cs, float* saved, float* c_last, int T, int B, int H, int32_t* status,
-                   cudaStream_t stream);
+                   float* hs, float* hs_kept, float* cs, float* saved, float* c_last, int T, int B, int H,
+                   int32_t* status, cudaStream_t stream);
 int fb_rnn_seq_bwd(int gates, const float* w, const float* h0, const float* c0, const float* hs, const float* cs,
                    const float* saved, const float* d_hs, const float* d_c_last, float* dxi, float* dhh, float* dh0,
                    float* dc0, int T, int B, int H, int32_t* status, cudaStream_t stream);

@@ -36,7 +36,7 @@ __device__ __forceinline__ void cp_async4(float* smem_dst, const float* src) {
 
 struct SeqArgs {
   const float *xi, *w, *bias, *h0, *c0;   // xi [T, B, G H]; w [K, ...] as the direction reads it; bias [G H] or NULL
-  float *hs, *cs, *saved, *c_last;        // [T, B, H], [T, B, H] (NULL: not kept), [T, B, 4 H] (NULL), [B, H]
+  float *hs, *hs_kept, *cs, *saved, *c_last;  // [T, B, H], the same and [T, B, H], [T, B, 4 H] (NULL: not kept), [B, H]
   const float *d_hs, *d_c_last, *hs_in, *cs_in, *saved_in;  // backward inputs (d_* may be NULL)
   float *dxi, *dhh, *dh0, *dc0;           // [T, B, G H], GRU: the hidden side's gradient, [B, H], [B, H] (NULL)
   int T, B, H, hs_units, rows4, k_res;
@@ -326,6 +326,7 @@ __global__ void __launch_bounds__(kT, 1) seq_fwd_kernel(const SeqArgs a) {
       }
       // what the others do not wait for
       a.hs[e_mine + t * e_step] = h;
+      if (a.hs_kept != nullptr) a.hs_kept[e_mine + t * e_step] = h;
       if (G == 4 && a.cs != nullptr) a.cs[e_mine + t * e_step] = c;
       if (a.saved != nullptr) {
         float* sv = a.saved + e4_mine + 4 * t * e_step;
@@ -585,14 +586,14 @@ extern "C" int fb_rnn_seq_supported(int gates, int B, int H) {
 }
 
 extern "C" int fb_rnn_seq_fwd(int gates, const float* xi, const float* w_t, const float* bias, const float* h0,
-                              const float* c0, float* hs, float* cs, float* saved, float* c_last, int T, int B, int H,
-                              int32_t* status, cudaStream_t stream) {
+                              const float* c0, float* hs, float* hs_kept, float* cs, float* saved, float* c_last, int T,
+                              int B, int H, int32_t* status, cudaStream_t stream) {
   if (T <= 0 || B <= 0 || H <= 0) return 0;
   Plan p;
   if ((gates != 3 && gates != 4) || !plan(gates, B, H, false, &p)) return -1;
   SeqArgs a = {};
   a.xi = xi; a.w = w_t; a.bias = bias; a.h0 = h0; a.c0 = c0;
-  a.hs = hs; a.cs = cs; a.saved = saved; a.c_last = c_last;
+  a.hs = hs; a.hs_kept = hs_kept; a.cs = cs; a.saved = saved; a.c_last = c_last;
   a.T = T; a.B = B; a.H = H; a.status = status; a.timeout_ns = 2000000000ull;
   a.hs_units = p.hs_units; a.rows4 = p.rows4; a.k_res = p.k_res;
   return gates == 4 ? run_bs<4>(false, a, p, stream) : run_bs<3>(false, a, p, stream);

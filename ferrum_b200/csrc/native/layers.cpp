@@ -91,7 +91,7 @@ struct RnnSeqNode : Node {
   variable_list apply(variable_list&& grads) override {
     NoAutograd below;
     variable_list out(5);  // proj, w, bias, h0, c0
-    Tensor w = contig(w_.unpack()), h0 = h0_.unpack(), c0 = c0_.unpack(), hs = hs_.unpack(shared_from_this());
+    Tensor w = contig(w_.unpack()), h0 = h0_.unpack(), c0 = c0_.unpack(), hs = hs_.unpack();
     if (h0.defined()) h0 = f32c(h0);
     if (c0.defined()) c0 = f32c(c0);
     Tensor dhs = grads[0].defined() ? f32c(grads[0]) : Tensor();
@@ -152,12 +152,14 @@ std::vector<Tensor> rnn_seq(int gates, const Tensor& proj, const Tensor& w, cons
   Tensor b = bias.defined() ? contig(bias) : bias, h = h0.defined() ? f32c(h0) : h0, c = c0.defined() ? f32c(c0) : c0;
   const bool grad = wants_grad({&proj, &w, &bias, &h0, &c0});
   Tensor wt = empty({H, GH}, x, at::kFloat), hs = empty({T, B, H}, x, at::kFloat);
+  // what the backward pass reads of the outputs is kept apart from them: a caller may change those in place
+  Tensor kept = grad ? empty({T, B, H}, x, at::kFloat) : Tensor();
   Tensor cs = gates == 4 && grad ? empty({T, B, H}, x, at::kFloat) : Tensor();
   Tensor saved = grad ? empty({T, B, 4 * H}, x, at::kFloat) : Tensor();
   Tensor c_last = gates == 4 ? empty({B, H}, x, at::kFloat) : Tensor();
   FB_CALL(fb_transpose_2d, wc.data_ptr(), wt.data_ptr(), static_cast<int>(GH), static_cast<int>(H), 4, cur_stream());
   FB_CALL(fb_rnn_seq_fwd, gates, x.data_ptr<float>(), wt.data_ptr<float>(), fptr(b), fptr(h), fptr(c),
-          hs.data_ptr<float>(), fptr_mut(cs), fptr_mut(saved), fptr_mut(c_last), static_cast<int>(T),
+          hs.data_ptr<float>(), fptr_mut(kept), fptr_mut(cs), fptr_mut(saved), fptr_mut(c_last), static_cast<int>(T),
           static_cast<int>(B), static_cast<int>(H), status(), cur_stream());
   std::vector<Tensor> out{hs};
   if (gates == 4) out.push_back(c_last);
@@ -170,8 +172,8 @@ std::vector<Tensor> rnn_seq(int gates, const Tensor& proj, const Tensor& w, cons
     if (c0.defined()) n->c0_ = SavedVariable(c0, false);
     n->cs = cs;
     n->saved = saved;
+    n->hs_ = SavedVariable(kept, false);
     torch::autograd::set_history(out, n);
-    n->hs_ = SavedVariable(out[0], true);
   }
   return out;
 }

@@ -2,6 +2,7 @@
 see."""
 import pytest
 import torch
+import torch.utils.checkpoint
 
 pytestmark = pytest.mark.gpu
 
@@ -42,3 +43,22 @@ def test_bf16_predictions_changed_after_the_loss(kind):
         loss.backward()
         grads.append(x.grad)
     assert torch.equal(*grads)
+
+
+@pytest.mark.parametrize("kind", ["LSTM", "GRU"])
+def test_sequence_output_changed_in_place(kind):
+    import ferrum_b200 as fb
+    from ferrum_b200 import nn
+
+    torch.manual_seed(3)
+    m = getattr(nn, kind)(8, 40, 2, device=fb.Device.Cuda(0))
+    x, mask = torch.randn(5, 3, 8, device="cuda"), (torch.rand(5, 3, 40, device="cuda") > 0.5).float()
+    grads = []
+    for inplace in (False, True):
+        m.zero_grad()
+        y, last = m.forward_seq(x)
+        y = y.mul_(mask) if inplace else y * mask
+        (y.sum() + sum(t.sum() for t in (last if kind == "LSTM" else (last,)))).backward()
+        grads.append([p.grad.clone() for _, p in m.named_parameters()])
+    for a, b in zip(*grads):
+        assert torch.equal(a, b)
