@@ -5,6 +5,7 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
 #include <c10/core/GradMode.h>
+#include <torch/csrc/autograd/forward_grad.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
@@ -75,6 +76,7 @@ inline Tensor as2d(const Tensor& t) { return t.dim() == 2 ? t : t.reshape({-1, t
 // ------------------------------------------------------------------------------------------------ autograd
 // The ops run below the autograd keys: a tangent would be lost there without a word.
 inline void refuse_tangents(std::initializer_list<const Tensor*> ts) {
+  if (!torch::autograd::ForwardADLevel::try_get_by_idx(0)) return;  // nobody is in a dual level
   for (const Tensor* t : ts)
     TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->_fw_grad(/*level=*/0).defined(),
                                 "this op has no forward-mode derivative (a dual tensor was given)");
