@@ -17,14 +17,13 @@ struct UnaryNode : Node {
   std::string name() const override { return "FerrumUnaryBackward"; }
   void release_variables() override { s_.reset_data(); }
   variable_list apply(variable_list&& grads) override {
-    NoAutograd below;
     variable_list out(1);
     if (!grads[0].defined()) return out;
-    Tensor g = contig(grads[0]), s;
-    if (!saves_nothing(op)) {
-      s = contig(s_.unpack(saves_output(op) ? shared_from_this() : nullptr));
-      s = cast(s, g.scalar_type());
-    }
+    Tensor s;
+    if (!saves_nothing(op)) s = s_.unpack(saves_output(op) ? shared_from_this() : nullptr);
+    NoAutograd below;
+    Tensor g = contig(grads[0]);
+    if (s.defined()) s = cast(contig(s), g.scalar_type());
     Tensor dx = empty(g.sizes(), g, g.scalar_type());
     FB_CALL(fb_unary_bwd, g.data_ptr(), ptr(s), dx.data_ptr(), g.numel(), op, alpha, beta, dt(g), cur_stream());
     out[0] = dx;
@@ -45,8 +44,8 @@ Tensor unary(const Tensor& x, int op, double alpha, double beta) {
     n->alpha = static_cast<float>(alpha);
     n->beta = static_cast<float>(beta);
     torch::autograd::set_history(y, n);
-    if (saves_output(op)) n->s_ = SavedVariable(y, true);
-    else if (!saves_nothing(op)) n->s_ = SavedVariable(x, false);
+    if (saves_output(op)) n->s_ = below.keep(y, true);
+    else if (!saves_nothing(op)) n->s_ = below.keep(x);
   }
   return y;
 }
@@ -90,10 +89,10 @@ struct SoftmaxNode : Node {
   std::string name() const override { return "FerrumSoftmaxBackward"; }
   void release_variables() override { y_.reset_data(); }
   variable_list apply(variable_list&& grads) override {
-    NoAutograd below;
     variable_list out(1);
     if (!grads[0].defined()) return out;
     Tensor y = y_.unpack(shared_from_this());
+    NoAutograd below;
     Tensor g = contig(cast(grads[0], y.scalar_type())), dx = empty(y.sizes(), y, y.scalar_type());
     FB_CALL(fb_softmax_bwd, g.data_ptr(), y.data_ptr(), dx.data_ptr(), rows_of(y), static_cast<int>(y.size(-1)),
             log_mode, dt(y), cur_stream());
@@ -111,7 +110,7 @@ Tensor softmax(const Tensor& x, bool log_mode) {
     auto n = make_node<SoftmaxNode>(x);
     n->log_mode = log_mode;
     torch::autograd::set_history(y, n);
-    n->y_ = SavedVariable(y, true);
+    n->y_ = below.keep(y, true);
   }
   return y;
 }
@@ -127,11 +126,12 @@ struct CrossEntropyNode : Node {
     labels_.reset_data();
   }
   variable_list apply(variable_list&& grads) override {
-    NoAutograd below;
     variable_list out(1);
     if (!grads[0].defined()) return out;
     labels_.unpack();
-    Tensor dx = dx_.unpack(), g = f32c(grads[0]), y = empty(dx.sizes(), dx, dx.scalar_type());
+    Tensor dx = dx_.unpack();
+    NoAutograd below;
+    Tensor g = f32c(grads[0]), y = empty(dx.sizes(), dx, dx.scalar_type());
     FB_CALL(fb_scale_by_device_scalar, dx.data_ptr(), g.data_ptr<float>(), y.data_ptr(), dx.numel(), dt(dx), cur_stream());
     out[0] = y;
     return out;
@@ -153,8 +153,8 @@ Tensor cross_entropy(const Tensor& logits, const Tensor& labels) {
           ws.data_ptr<float>(), rows, static_cast<int>(x.size(1)), 1.f / static_cast<float>(rows), dt(x), cur_stream());
   if (grad) {
     auto n = make_node<CrossEntropyNode>(logits);
-    n->dx_ = SavedVariable(dx, false);
-    n->labels_ = SavedVariable(lab, false);
+    n->dx_ = below.keep(dx);
+    n->labels_ = below.keep(lab);
     torch::autograd::set_history(loss, n);
   }
   return loss;
@@ -169,10 +169,11 @@ struct NllNode : Node {
   std::string name() const override { return "FerrumNllBackward"; }
   void release_variables() override { target_.reset_data(); }
   variable_list apply(variable_list&& grads) override {
-    NoAutograd below;
     variable_list out(1);
     if (!grads[0].defined()) return out;
-    Tensor target = target_.unpack(), g = f32c(grads[0]), dx = empty(sizes, g, st);
+    Tensor target = target_.unpack();
+    NoAutograd below;
+    Tensor g = f32c(grads[0]), dx = empty(sizes, g, st);
     FB_CALL(fb_nll_bwd, reinterpret_cast<const ll*>(target.data_ptr<int64_t>()), g.data_ptr<float>(), dx.data_ptr(),
             rows, static_cast<int>(cols), -1.f / static_cast<float>(rows), dt(dx), cur_stream());
     out[0] = dx;
@@ -193,7 +194,7 @@ Tensor nll(const Tensor& log_probs, const Tensor& target) {
   if (!is_f32(x)) loss = cast(loss, x.scalar_type());
   if (wants_grad({&log_probs})) {
     auto n = make_node<NllNode>(log_probs);
-    n->target_ = SavedVariable(t, false);
+    n->target_ = below.keep(t);
     n->rows = rows;
     n->cols = cols;
     n->st = x.scalar_type();
@@ -214,11 +215,11 @@ struct ElemLossNode : Node {
     t_.reset_data();
   }
   variable_list apply(variable_list&& grads) override {
-    NoAutograd below;
     variable_list out(1);
     if (!grads[0].defined()) return out;
-    Tensor p = p_.unpack(), t = t_.unpack(), g = f32c(grads[0]);
-    Tensor dp = empty(p.sizes(), p, at::kFloat);
+    Tensor p = p_.unpack(), t = t_.unpack();
+    NoAutograd below;
+    Tensor g = f32c(grads[0]), dp = empty(p.sizes(), p, at::kFloat);
     FB_CALL(fb_loss_bwd, p.data_ptr<float>(), t.data_ptr<float>(), g.data_ptr<float>(), dp.data_ptr<float>(), p.numel(),
             kind, 1.f / static_cast<float>(p.numel()), cur_stream());
     out[0] = cast(dp, st);
@@ -238,8 +239,8 @@ Tensor elementwise_loss(const Tensor& pred, const Tensor& target, int kind) {
           kind, 1.f / static_cast<float>(n), cur_stream());
   if (wants_grad({&pred})) {
     auto nd = make_node<ElemLossNode>(pred);
-    nd->p_ = SavedVariable(p, false);
-    nd->t_ = SavedVariable(t, false);
+    nd->p_ = below.keep(p);
+    nd->t_ = below.keep(t);
     nd->kind = kind;
     nd->st = pred.scalar_type();
     torch::autograd::set_history(loss, nd);

@@ -60,7 +60,7 @@ Tensor embedding(const Tensor& weight, const Tensor& idx_, ll padding, bool pool
   }
   if (wants_grad({&weight})) {
     auto n = make_node<EmbeddingNode>(weight);
-    n->idx_ = SavedVariable(idx, false);
+    n->idx_ = below.keep(idx);
     n->vocab = V;
     n->dim = D;
     n->group = pool ? idx.size(1) : 1;
@@ -76,22 +76,19 @@ Tensor embedding(const Tensor& weight, const Tensor& idx_, ll padding, bool pool
 // last cell state [B, H].  The recurrence runs in one launch per direction; the weight gradient of all steps is one
 // product over T B rows.
 struct RnnSeqNode : Node {
-  SavedVariable w_, h0_, c0_, hs_;
-  Tensor cs, saved;
+  SavedVariable w_, h0_, c0_, hs_, cs_, saved_;
   int gates = 4;
   bool has_bias = false;
   std::string name() const override { return "FerrumRnnSeqBackward"; }
   void release_variables() override {
-    w_.reset_data();
-    h0_.reset_data();
-    c0_.reset_data();
-    hs_.reset_data();
-    cs = saved = Tensor();
+    for (SavedVariable* s : {&w_, &h0_, &c0_, &hs_, &cs_, &saved_}) s->reset_data();
   }
   variable_list apply(variable_list&& grads) override {
-    NoAutograd below;
     variable_list out(5);  // proj, w, bias, h0, c0
-    Tensor w = contig(w_.unpack()), h0 = h0_.unpack(), c0 = c0_.unpack(), hs = hs_.unpack();
+    Tensor w = w_.unpack(), h0 = h0_.unpack(), c0 = c0_.unpack(), hs = hs_.unpack(), cs = cs_.unpack(),
+           saved = saved_.unpack();
+    NoAutograd below;
+    w = contig(w);
     if (h0.defined()) h0 = f32c(h0);
     if (c0.defined()) c0 = f32c(c0);
     Tensor dhs = grads[0].defined() ? f32c(grads[0]) : Tensor();
@@ -167,12 +164,12 @@ std::vector<Tensor> rnn_seq(int gates, const Tensor& proj, const Tensor& w, cons
     auto n = make_node<RnnSeqNode>(proj, w, bias, h0, c0);
     n->gates = gates;
     n->has_bias = bias.defined();
-    n->w_ = SavedVariable(w, false);
-    if (h0.defined()) n->h0_ = SavedVariable(h0, false);
-    if (c0.defined()) n->c0_ = SavedVariable(c0, false);
-    n->cs = cs;
-    n->saved = saved;
-    n->hs_ = SavedVariable(kept, false);
+    n->w_ = below.keep(w);
+    n->h0_ = below.keep(h0);
+    n->c0_ = below.keep(c0);
+    n->cs_ = below.keep(cs);
+    n->saved_ = below.keep(saved);
+    n->hs_ = below.keep(kept);
     torch::autograd::set_history(out, n);
   }
   return out;

@@ -77,14 +77,14 @@ struct LinearNode : Node {
     y_.reset_data();
   }
   variable_list apply(variable_list&& grads) override {
-    NoAutograd below;
     variable_list out(3);
     if (!grads[0].defined()) return out;
-    Tensor x2 = as2d(x_.unpack()), w = w_.unpack();
-    Tensor g2 = contig(as2d(grads[0]));
+    Tensor x = x_.unpack(), w = w_.unpack(), y = act != kNone ? y_.unpack(shared_from_this()) : Tensor();
+    NoAutograd below;
+    Tensor x2 = as2d(x), g2 = contig(as2d(grads[0]));
     g2 = low ? cast(g2, at::kBFloat16) : cast(g2, at::kFloat);
     if (act != kNone) {  // only activations whose derivative is a function of the output are fused
-      Tensor y = as2d(y_.unpack(shared_from_this()));
+      y = as2d(y);
       Tensor d = empty(g2.sizes(), g2, g2.scalar_type());
       FB_CALL(fb_unary_bwd, g2.data_ptr(), y.data_ptr(), d.data_ptr(), g2.numel(), act, 0.f, 0.f, dt(g2), cur_stream());
       g2 = d;
@@ -113,10 +113,10 @@ Tensor linear(const Tensor& x, const Tensor& weight, const c10::optional<Tensor>
     n->x_dtype = x.scalar_type();
     n->x_sizes.assign(x.sizes().begin(), x.sizes().end());
     n->sink = make_sink(sink, py::cast(weight));
-    n->x_ = SavedVariable(o.saved, false);
-    n->w_ = SavedVariable(o.w, false);
+    n->x_ = below.keep(o.saved);
+    n->w_ = below.keep(o.w);
     torch::autograd::set_history(y, n);
-    if (act != kNone) n->y_ = SavedVariable(y, true);
+    if (act != kNone) n->y_ = below.keep(y, true);
   }
   return y;
 }
@@ -147,21 +147,23 @@ Tensor norm_bwd(const Tensor& gy2, const Tensor& x2, const Tensor& dact, const T
 }
 
 struct LayerNormNode : Node {
-  SavedVariable x_, g_;
-  NormStats st;
+  SavedVariable x_, g_, mean_, rstd_;
   int pre = kNone;
   bool has_gamma = false, has_beta = false;
   std::string name() const override { return "FerrumLayerNormBackward"; }
   void release_variables() override {
     x_.reset_data();
     g_.reset_data();
-    st = NormStats();
+    mean_.reset_data();
+    rstd_.reset_data();
   }
   variable_list apply(variable_list&& grads) override {
-    NoAutograd below;
     variable_list out(3);
     if (!grads[0].defined()) return out;
-    Tensor x = contig(x_.unpack()), g = g_.unpack();
+    Tensor x = x_.unpack(), g = g_.unpack();
+    const NormStats st{mean_.unpack(), rstd_.unpack()};
+    NoAutograd below;
+    x = contig(x);
     Tensor x2 = as2d(x), gy = contig(cast(grads[0], x.scalar_type()));
     Tensor dx = empty(x.sizes(), x, x.scalar_type());
     Tensor stats = norm_bwd(as2d(gy), x2, Tensor(), g, st, dx, pre, false);
@@ -186,12 +188,13 @@ Tensor layer_norm(const Tensor& x, const c10::optional<Tensor>& gamma_, const c1
   NormStats st = norm_fwd(as2d(xc), g, b, as2d(y), static_cast<float>(eps), pre);
   if (wants_grad({&x, &gamma, &beta})) {
     auto n = make_node<LayerNormNode>(x, gamma, beta);
-    n->st = st;
+    n->mean_ = below.keep(st.mean);
+    n->rstd_ = below.keep(st.rstd);
     n->pre = pre;
     n->has_gamma = gamma.defined();
     n->has_beta = beta.defined();
-    n->x_ = SavedVariable(xc.is_alias_of(x) ? x : xc, false);
-    if (g.defined()) n->g_ = SavedVariable(g, false);
+    n->x_ = below.keep(xc.is_alias_of(x) ? x : xc);
+    n->g_ = below.keep(g);
     torch::autograd::set_history(y, n);
   }
   return y;
@@ -202,9 +205,7 @@ Tensor layer_norm(const Tensor& x, const c10::optional<Tensor>& gamma_, const c1
 // reads act(z).  Backward: one streaming kernel turns dy into dz and yields d_gamma, d_beta and the bias gradient,
 // then the two products run on dz.  fp32 path: z is stored, the activation is evaluated inside the normalisation.
 struct LinearActNormNode : Node {
-  SavedVariable x_, w_, g_;
-  Tensor z, dact;
-  NormStats st;
+  SavedVariable x_, w_, g_, z_, dact_, mean_, rstd_;
   bool low = false, has_bias = false;
   int pre = kNone;
   at::ScalarType x_dtype = at::kFloat;
@@ -212,17 +213,15 @@ struct LinearActNormNode : Node {
   std::shared_ptr<Sink> sink;
   std::string name() const override { return "FerrumLinearActNormBackward"; }
   void release_variables() override {
-    x_.reset_data();
-    w_.reset_data();
-    g_.reset_data();
-    z = dact = Tensor();
-    st = NormStats();
+    for (SavedVariable* s : {&x_, &w_, &g_, &z_, &dact_, &mean_, &rstd_}) s->reset_data();
   }
   variable_list apply(variable_list&& grads) override {
-    NoAutograd below;
     variable_list out(5);
     if (!grads[0].defined()) return out;
-    Tensor x2 = as2d(x_.unpack()), w = w_.unpack(), g = g_.unpack();
+    Tensor x = x_.unpack(), w = w_.unpack(), g = g_.unpack(), z = z_.unpack(), dact = dact_.unpack();
+    const NormStats st{mean_.unpack(), rstd_.unpack()};
+    NoAutograd below;
+    Tensor x2 = as2d(x);
     Tensor gy2 = contig(as2d(cast(grads[0], z.scalar_type())));
     Tensor dz = empty(z.sizes(), z, z.scalar_type());
     Tensor stats = norm_bwd(gy2, z, dact, g, st, dz, pre, true);
@@ -240,18 +239,22 @@ Tensor linear_act_norm(const Tensor& x, const Tensor& weight, const c10::optiona
                        const c10::optional<Tensor>& w_low, py::object sink) {
   if (!low && !norm_evaluates(act))
     return layer_norm(linear(x, weight, bias_, kNone, low, tf32, w_low, sink), gamma, beta, eps, act);
-  NoAutograd below;
   const Tensor bias = bias_.value_or(Tensor());
-  Operands o = operands(x, weight, w_low.value_or(Tensor()), low);
+  Operands o;
+  {
+    NoAutograd below;
+    o = operands(x, weight, w_low.value_or(Tensor()), low);
+  }
+  const bool fused = low && act != kNone && tma_ok(op2d(o.x2)) && tma_ok(op2d(o.w));
+  if (fused && act > FB_ACT_SIGMOID) throw py::key_error("linear_act_layernorm: an activation that no epilogue evaluates");
+  if (!fused && !norm_evaluates(act))
+    return layer_norm(linear(x, weight, bias_, kNone, low, tf32, w_low, sink), gamma, beta, eps, act);
+  NoAutograd below;
   const int64_t N = weight.size(0), M = o.x2.size(0);
   const bool grad = wants_grad({&x, &weight, &bias, &gamma, &beta});
   Tensor b = bias.defined() ? f32c(bias) : bias;
   Tensor g = contig(gamma), be = contig(beta);
   Tensor z = empty({M, N}, o.x2, low ? at::kBFloat16 : at::kFloat), dact;
-  const bool fused = low && act != kNone && tma_ok(op2d(o.x2)) && tma_ok(op2d(o.w));
-  if (fused && act > FB_ACT_SIGMOID) throw py::key_error("linear_act_layernorm: an activation that no epilogue evaluates");
-  if (!fused && !norm_evaluates(act))
-    return layer_norm(linear(x, weight, bias_, kNone, low, tf32, w_low, sink), gamma, beta, eps, act);
   if (fused && grad) dact = empty({M, N}, o.x2, at::kBFloat16);
   gemm(op2d(o.x2), op2d(o.w), fptr(b), fused ? act : kNone, z.data_ptr(), N, low, false, ptr(dact), &o.x2,
        tf32 && !low);
@@ -266,12 +269,13 @@ Tensor linear_act_norm(const Tensor& x, const Tensor& weight, const c10::optiona
     n->x_dtype = x.scalar_type();
     n->x_sizes.assign(x.sizes().begin(), x.sizes().end());
     n->sink = make_sink(sink, py::cast(weight));
-    n->x_ = SavedVariable(o.saved, false);
-    n->w_ = SavedVariable(o.w, false);
-    n->g_ = SavedVariable(g, false);
-    n->z = z;
-    n->dact = dact;
-    n->st = st;
+    n->x_ = below.keep(o.saved);
+    n->w_ = below.keep(o.w);
+    n->g_ = below.keep(g);
+    n->z_ = below.keep(z);
+    n->dact_ = below.keep(dact);
+    n->mean_ = below.keep(st.mean);
+    n->rstd_ = below.keep(st.rstd);
     torch::autograd::set_history(y, n);
   }
   return y;
@@ -324,10 +328,11 @@ struct BmmNode : Node {
     b_.reset_data();
   }
   variable_list apply(variable_list&& grads) override {
-    NoAutograd below;
     variable_list out(2);
     if (!grads[0].defined()) return out;
-    Tensor a = a_.unpack(), b = b_.unpack(), g = batched_operand(grads[0], is_bf16(a));
+    Tensor a = a_.unpack(), b = b_.unpack();
+    NoAutograd below;
+    Tensor g = batched_operand(grads[0], is_bf16(a));
     if (task_should_compute_output(0)) {
       Tensor ga = empty(a.sizes(), a, a.scalar_type());
       batched_nt(g, b, ga, alpha);
@@ -358,8 +363,8 @@ Tensor bmm(const Tensor& a, const Tensor& b, double alpha, bool heads_inner, boo
     n->alpha = static_cast<float>(alpha);
     n->da = a.scalar_type();
     n->db = b.scalar_type();
-    n->a_ = SavedVariable(ac, false);
-    n->b_ = SavedVariable(bc, false);
+    n->a_ = below.keep(ac);
+    n->b_ = below.keep(bc);
     torch::autograd::set_history(y, n);
   }
   return y;

@@ -5,11 +5,13 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
 #include <c10/core/GradMode.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <torch/csrc/autograd/forward_grad.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/utils/pybind.h>
 
 #include <atomic>
@@ -95,7 +97,22 @@ inline std::shared_ptr<N> make_node(const T&... inputs) {
   return n;
 }
 // Inside an op and inside a node's apply: the tensor methods used there record nothing of their own.
-typedef at::AutoDispatchBelowADInplaceOrView NoAutograd;
+struct NoAutograd {
+  const c10::impl::LocalDispatchKeySet outer = c10::impl::tls_local_dispatch_key_set();
+  at::AutoDispatchBelowADInplaceOrView guard;
+  // A tensor that the backward pass reads.  Saved-tensor hooks are the user's code (the recomputation of a checkpoint
+  // among them): they run with the dispatch state of the op's caller, and an apply unpacks before it sets its guard.
+  SavedVariable keep(const Tensor& t, bool is_output = false) const {
+    if (!t.defined()) return SavedVariable();
+    c10::impl::ForceDispatchKeyGuard user(outer);
+    try {
+      return SavedVariable(t, is_output);
+    } catch (python_error& e) {  // raised by a hook, by way of pybind
+      e.restore();
+      throw py::error_already_set();
+    }
+  }
+};
 
 Tensor unary(const Tensor& x, int op, double alpha, double beta);
 
