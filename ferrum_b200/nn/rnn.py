@@ -138,6 +138,10 @@ class _SeqBase(Module):
     def _zeros(self, x):
         return torch.zeros(self.num_layers, x.shape[1], self._hidden, device=x.device, dtype=x.dtype)
 
+    def _one_launch(self, cell_cls, x) -> bool:
+        """True when the layers' recurrences can run as whole-sequence launches: cells whose step is ``cell_cls``'s own."""
+        return all(type(c) is cell_cls and F.rnn_sequence_ok(cell_cls.gates, x, c.weight_hh) for c in self.cells)
+
     def _check(self, x):
         if x.dim() != 3 or x.shape[2] != self.input_size:
             raise ShapeMismatch(type(self).__name__, f"[T, B, {self.input_size}]", list(x.shape))
@@ -155,7 +159,7 @@ class RNN(_SeqBase):
         wrapped = isinstance(input, Tensor)
         x = _unwrap(input)
         self._check(x)
-        fused = self.cell_cls is GRUCell and F.rnn_sequence_ok(3, x, self.cells[0].weight_hh)
+        fused = self._one_launch(GRUCell, x)
         h0 = _unwrap(h_0) if h_0 is not None else (None if fused else self._zeros(x))
         finals, layer_in = [], x
         for l, cell in enumerate(self.cells):
@@ -196,7 +200,7 @@ class LSTM(_SeqBase):
         wrapped = isinstance(input, Tensor)
         x = _unwrap(input)
         self._check(x)
-        fused = F.rnn_sequence_ok(4, x, self.cells[0].weight_hh)
+        fused = self._one_launch(LSTMCell, x)
         h0 = _unwrap(hx[0]) if hx is not None else (None if fused else self._zeros(x))
         c0 = _unwrap(hx[1]) if hx is not None else (None if fused else self._zeros(x))
         hs, cs, layer_in = [], [], x

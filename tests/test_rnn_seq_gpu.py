@@ -48,3 +48,37 @@ def test_sequence(kind, T, B, I, H, L, state):
     with torch.no_grad():
         again = m.forward_seq(x.detach(), None if not state else ((h0, c0) if kind == "LSTM" else h0))[0]
     assert torch.equal(again, y)
+
+
+@pytest.mark.parametrize("kind", ["LSTM", "GRU"])
+@pytest.mark.parametrize("how", ["cell_cls", "one_cell", "other_type"])
+def test_cells_of_the_users_own(kind, how):
+    """A cell class with its own step, in every layer or in one, and a layer of another type than fp32: step by step."""
+    import ferrum_b200 as fb
+    from ferrum_b200 import nn
+    from ferrum_b200.nn import rnn
+
+    calls = []
+
+    class Cell(getattr(rnn, f"{kind}Cell")):
+        def step(self, *a):
+            calls.append(1)
+            return super().step(*a)
+
+    dev = fb.Device.Cuda(0)
+    base = getattr(nn, kind)
+    torch.manual_seed(4)
+    want = base(8, 40, 2, device=dev)
+    model = type("Own", (base,), {"cell_cls": Cell})(8, 40, 2, device=dev) if how == "cell_cls" else base(8, 40, 2, device=dev)
+    model.load_state_dict(want.state_dict())
+    if how == "one_cell":
+        model.cells[1].__class__ = Cell
+    x = torch.randn(5, 3, 8, device="cuda")
+    ref = want.forward_seq(x)[0]
+    if how == "other_type":
+        with torch.no_grad():
+            for n in ("weight_hh", "weight_ih"):
+                setattr(model.cells[1], n, torch.nn.Parameter(getattr(model.cells[1], n).to(torch.bfloat16)))
+    got = model.forward_seq(x)[0]
+    assert len(calls) == {"cell_cls": 10, "one_cell": 5, "other_type": 0}[how]
+    assert (got - ref).norm() <= (2e-2 if how == "other_type" else 1e-6) * ref.norm()
