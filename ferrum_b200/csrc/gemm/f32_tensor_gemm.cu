@@ -1,22 +1,24 @@
 // fp32 GEMM on the tensor cores without giving up fp32 precision (sm_100a).
 //
 // Every fp32 operand element is split into three bf16 numbers a = a0 + a1 + a2, each the value that was left rounded
-// to nearest (8 + 8 + 8 significant bits: the sum is exact), and six of the nine products are accumulated in fp32 by
-// tcgen05.mma: a0 b0, a0 b1, a1 b0, a1 b1, a0 b2, a2 b0.  The three that are left out are below 2^-26 of |a b|, less
-// than the rounding of one fp32 multiply-add.  The tensor core truncates where it adds (2048 x 2048 x 4096 of
+// to nearest (8 + 8 + 8 significant bits), and six of the nine products are accumulated in fp32 by tcgen05.mma: a0 b0,
+// a0 b1, a1 b0, a1 b1, a0 b2, a2 b0.  The three that are left out are below 2^-26 of |a b|, less than the rounding of one
+// fp32 multiply-add.  bf16 ends at 2^-133, fp32 at 2^-149: operands are multiplied by 2^16 before the split and sums by
+// 2^-32 after it (both exact), so that a = a0 + a1 + a2 holds for every finite value down to the last subnormal.  The tensor core truncates where it adds (2048 x 2048 x 4096 of
 // normal numbers summed there alone: relative error 2.8e-5), so each k-block of 64 gets a fresh accumulator and the
 // k-blocks are added in registers, rounded to nearest: 1.7e-7, against 1.1e-6 of a chain of fp32 multiply-adds.
 //
 // What bounds it: six bf16 MMAs per fp32 product (271 TFLOP/s at the measured bf16 rate), and beside it the split:
-// about seven instructions per operand element in eight warps, in the shadow of the MMAs.  The split happens on the
+// about eight instructions per operand element in sixteen warps, in the shadow of the MMAs.  The split happens on the
 // way from global memory (registers) to shared memory (three bf16 planes, 128-byte swizzle, K-major), so any element
 // strides are accepted, nothing is staged in global memory and no second launch is needed.
 //
 // One CTA per 128 x BN output tile and K split.  The splits of a tile are one thread-block cluster: the partial tiles
 // meet through distributed shared memory in a fixed order, so small outputs fill the chip without a workspace.
 //
-// Infinities, NaNs and values that would round to infinity do not survive the split (inf - inf, 0 * inf) and always
-// end in a result that is not finite; such a result is computed again with fp32 multiply-adds when the tile is written.
+// Infinities, NaNs and values that would round to infinity (from 2^112) do not survive the split (inf - inf, 0 * inf) and
+// always end in a result that is not finite, and so do sums above 2^96; such a result is computed again with fp32
+// multiply-adds when the tile is written.
 //
 // bf16 operands whose rows a TMA map cannot describe (a pitch that is no multiple of 16 bytes, an odd base) take the
 // same kernel with one plane and one product: no padded copies, no fp32 copies.  Rows at any 2-byte address are read
@@ -41,6 +43,8 @@ namespace fb {
 namespace {
 
 namespace cg = cooperative_groups;
+
+constexpr float kUp = 65536.f, kDown = 1.f / (kUp * kUp);  // of an operand before the split, of a sum after it
 
 constexpr int kBM = 128;
 constexpr int kLoaders = 512;
@@ -236,6 +240,13 @@ __device__ __forceinline__ float2 add2(float2 x, float2 y) {
       : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
   return r;
 }
+__device__ __forceinline__ float2 scale2(float2 x, float s) {
+  float2 r;
+  asm("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %4};\nmul.rn.f32x2 d, a, b;\nmov.b64 {%0, %1}, d;\n}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(x.x), "f"(x.y), "f"(s));
+  return r;
+}
 __device__ __forceinline__ uint32_t bf16_pair(float2 x) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(x.x, x.y);
   return *reinterpret_cast<const uint32_t*>(&h);
@@ -251,7 +262,7 @@ __device__ __forceinline__ void store_piece(uint32_t at, uint32_t plane_bytes, c
   uint32_t w0[4], w1[4], w2[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const float2 x = make_float2(v[2 * j], v[2 * j + 1]);
+    const float2 x = scale2(make_float2(v[2 * j], v[2 * j + 1]), kUp);
     w0[j] = bf16_pair(x);
     const float2 r = sub2(x, wide_pair(w0[j]));
     w1[j] = bf16_pair(r);
@@ -459,7 +470,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split_kernel(const __grid_co
     }
     if constexpr (kPlanes > 1) {
       for (int j = 0; j < 4; ++j) {
-        if (fabsf(f[j]) <= FLT_MAX || n + j >= p.N) continue;
+        const bool finite = fabsf(f[j]) <= FLT_MAX;
+        f[j] *= kDown;
+        if (finite || n + j >= p.N) continue;
         // not finite: an operand that does not survive the split, or a result that is not finite in fp32 either
         float s = 0.f;
         for (int k = 0; k < p.K; ++k)

@@ -57,3 +57,30 @@ def test_values_outside_the_split(value):
     fine = torch.isfinite(ref.float())
     assert torch.equal(fine, torch.isfinite(out)) and torch.equal(ref.isnan(), out.isnan())
     assert (out - ref)[fine].abs().max() <= 1e-6 * ref[fine].abs().max()
+
+
+@pytest.mark.parametrize("ea,eb", [(-120, 100), (100, -120), (-126, 90), (-140, 100),
+                                   (-148, 110), (-60, -60), (100, -100), (60, 30), (115, -20), (55, 50)])
+def test_operands_of_any_exponent(ea, eb):
+    """The smallest operands decide the result, the largest leave the split: the bound is that of ordinary values of one
+    sign (100 terms: a truncation per 16 products and k-block, or 100 roundings of a chain: below 2e-6)."""
+    from ferrum_b200.ops.gemm import gemm_f32
+
+    g = torch.Generator(device="cuda").manual_seed(11)
+    a = torch.ldexp(1 + torch.rand(70, 100, device="cuda", generator=g), torch.tensor(ea, device="cuda"))
+    b = torch.ldexp(1 + torch.rand(130, 100, device="cuda", generator=g), torch.tensor(eb, device="cuda"))
+    ref, out = a.double() @ b.double().t(), gemm_f32(a, b).double()
+    assert (out - ref).abs().max() <= 2e-6 * ref.abs().max()
+
+
+@pytest.mark.parametrize("K", [33, 64, 100, 784, 4096])
+def test_operands_of_one_sign(K):
+    """Truncation is a bias that shows where all products have one sign: no further from fp64 than a chain of fp32
+    multiply-adds (K / 2 roundings at random, and never below two roundings of the result)."""
+    from ferrum_b200.ops.gemm import gemm_f32
+
+    g = torch.Generator(device="cuda").manual_seed(K)
+    a, b = torch.rand(300, K, device="cuda", generator=g), torch.rand(200, K, device="cuda", generator=g)
+    ref = a.double() @ b.double().t()
+    err = lambda o: ((o.double() - ref).norm() / ref.norm()).item()
+    assert err(gemm_f32(a, b)) <= max(err(gemm_f32(a, b, simt=True)), 2.0 ** -23)
