@@ -473,7 +473,7 @@ def bmm_scaled(a: torch.Tensor, b: torch.Tensor, alpha: float = 1.0, heads_inner
     if _native(a) and _native(b):
         low = config.low_precision_active()
         if (a.shape[-1] % 8 == 0 and b.shape[-1] % 8 == 0) if low else (
-                a.dtype == b.dtype == torch.float32 and a.shape[:2] == b.shape[:2]):
+                a.dim() == b.dim() == 4 and a.dtype == b.dtype == torch.float32 and a.shape[:2] == b.shape[:2]):
             return _lib.native().bmm(a, b, alpha, heads_inner, low)
     out = matmul(a, b)
     return scalar_op(out, "mul", float(alpha)) if alpha != 1.0 else out

@@ -84,3 +84,14 @@ def test_operands_of_one_sign(K):
     ref = a.double() @ b.double().t()
     err = lambda o: ((o.double() - ref).norm() / ref.norm()).item()
     assert err(gemm_f32(a, b)) <= max(err(gemm_f32(a, b, simt=True)), 2.0 ** -23)
+
+
+@pytest.mark.parametrize("lead_a,lead_b", [((3,), (3,)), ((), ()), ((2, 3), (3,)), ((3, 2, 2), (3, 2, 2))])
+def test_scaled_products_of_other_ranks(lead_a, lead_b):
+    """``bmm_scaled`` takes in fp32 what ``matmul`` takes."""
+    from ferrum_b200.ops import functional as F
+
+    g = torch.Generator(device="cuda").manual_seed(4)
+    a, b = (torch.randn(*l, *s, device="cuda", generator=g) for l, s in ((lead_a, (5, 40)), (lead_b, (40, 7))))
+    ref = 0.5 * (a.double() @ b.double())
+    assert (F.bmm_scaled(a, b, 0.5).double() - ref).norm() <= 5e-7 * ref.norm()
