@@ -498,6 +498,16 @@ int smem_limit() {
   return v;
 }
 
+int sm_count() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v;
+  }();
+  return n;
+}
+
 struct Plan {
   int ncl, bs, hs_units, rows4, k_res;
   bool reg;  // weights in registers
@@ -508,7 +518,7 @@ struct Plan {
 bool plan(int G, int B, int H, bool backward, Plan* p) {
   if (H < 1 || H > 1024) return false;
   p->ncl = H >= 256 ? 8 : (H >= 128 ? 4 : (H >= 64 ? 2 : 1));
-  const int slots = 148 / p->ncl;
+  const int slots = sm_count() / p->ncl;
   p->bs = B <= slots ? 1 : (B <= 2 * slots ? 2 : (B <= 4 * slots ? 4 : 8));
   p->hs_units = (H + p->ncl - 1) / p->ncl;
   const int rows = backward ? p->hs_units : G * p->hs_units, K = backward ? G * H : H;
