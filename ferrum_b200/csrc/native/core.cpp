@@ -79,6 +79,39 @@ bool tma_ok(const Op& a) {
   return false;
 }
 
+// A bf16 operand that no TMA map describes, laid out again with its reduction (a multiple of 8) contiguous.
+static Op aligned_copy(const Op& o, const at::TensorOptions& opt, Tensor& keep) {
+  if (o.s_row == 1 && o.s_k == o.rows) {  // a contiguous matrix seen transposed: the operands of a weight gradient
+    keep = at::empty({o.rows, o.k}, opt);
+    FB_CALL(fb_transpose_2d, o.p, keep.data_ptr(), static_cast<int>(o.k), static_cast<int>(o.rows), 2, cur_stream());
+  } else {
+    keep = at::from_blob(const_cast<void*>(o.p), {o.rows, o.k}, {o.s_row, o.s_k}, opt)
+               .clone(at::MemoryFormat::Contiguous);
+  }
+  return op2d(keep);
+}
+// Where the copies repay.  The kernel that reads such operands in place does 70 products (multiply-adds) per ns, the
+// aligned kernels many times that; a copy takes 6 us and 1.6 TB/s, and 5 us are left to be sure.  Behind a single
+// transpose, where the TMA unit can store the result's rows, the aligned kernels also start earlier and store 3 us per
+// million elements faster.  Weight gradients [N, K] of M rows, in place against copies and product: M 8192, 4095 x 4095
+// 1679 / 417 us; 1024, 2049 x 2049 88 / 65; 4096, 1001 x 1001 74 / 69; 1024, 1001 x 1001 31 / 36; 8192, 37 x 4095 74 /
+// 140; with bias gradient 64, 1001 x 2048 27 / 24; 512, 333 x 1024 27 / 30.
+static bool copies_repay(const Op& a, const Op& b, bool rows_tma) {
+  if (a.k % 8 != 0) return false;
+  double us = static_cast<double>(a.rows) * b.rows * a.k / 7e7, cost = 0.;
+  int copies = 0;
+  bool transposes = true;
+  for (const Op* o : {&a, &b})
+    if (!tma_ok(*o)) {
+      cost += 6. + static_cast<double>(o->rows) * o->k * 4 / 1.6e6;
+      transposes &= o->s_row == 1;
+      ++copies;
+    }
+  if (copies != 1 || !transposes || !rows_tma) return us > cost + 5.;
+  us += static_cast<double>(a.rows) * b.rows * 3e-6;
+  return us > cost - 2.;
+}
+
 // fp32 products with a reduction this short do not repay the tensor-core kernel's set-up (7 us against 2 - 3).
 constexpr int kSimtK = 32;
 
@@ -131,6 +164,14 @@ void gemm(const Op& a, const Op& b, const float* bias, int act, void* out, ll ld
     return;
   }
   if (a.bf16 && b.bf16 && !(out_bf16 && accumulate)) {  // operands that a TMA map cannot describe
+    const bool rows_tma = reinterpret_cast<uintptr_t>(out) % 16 == 0 && ldc * (out_bf16 ? 2 : 4) % 16 == 0;
+    if (like != nullptr && copies_repay(a, b, rows_tma)) {
+      Tensor ka, kb;
+      const auto opt = like->options().dtype(at::kBFloat16).requires_grad(false);
+      gemm(tma_ok(a) ? a : aligned_copy(a, opt, ka), tma_ok(b) ? b : aligned_copy(b, opt, kb), bias, act, out, ldc,
+           out_bf16, accumulate, nullptr, like, tf32, splits);
+      return;
+    }
     FB_CALL(fb_gemm_bf16_any, a.p, b.p, out, bias, M, N, K, a.s_row, a.s_k, b.s_row, b.s_k, ldc, out_bf16, act,
             accumulate, status(), cur_stream());
     return;

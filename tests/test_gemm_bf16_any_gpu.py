@@ -36,3 +36,32 @@ def test_layouts_and_edges(la, lb, M, N, K):
     low = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
     _lib.native().gemm_nt(a, b, bias, 0, low, False, False)
     assert (low.double() - ref).norm() <= 2.0 ** -8 * ref.norm()
+
+
+@pytest.mark.parametrize("la,lb", [("rows", "rows"), ("rows", "even"), ("odd", "odd"), ("odd", "even"), ("step", "rows"),
+                                   ("flat", "flat"), ("flat", "even")])
+@pytest.mark.parametrize("M,N,K", [(2049, 2049, 1024), (1001, 1200, 4096), (1601, 1603, 1000), (513, 333, 8192), (1001, 2000, 64)])
+def test_large_products_of_aligned_reduction(la, lb, M, N, K):
+    """Sizes where unaligned operands are copied first (the last one is not): the persistent kernels' bits, whose tensor
+    core truncates K / 16 times: K / 16 * 2^-23 of the norm."""
+    from ferrum_b200 import _lib
+    from ferrum_b200.utils.runtime import check_status
+
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    make = lambda rows, l: (torch.randn(K, rows, device="cuda", generator=g).bfloat16().t() if l == "flat"
+                            else _operand(rows, K, l, g))
+    a, b = make(M, la), make(N, lb)
+    bias = torch.randn(N, device="cuda", generator=g)
+    ref = a.double() @ b.double().t() + bias.double()
+    bound = (K / 16 * 2.0 ** -23 + 1e-6)
+    out = torch.full((M, N), 2.0, device="cuda")
+    _lib.native().gemm_nt(a, b, bias, 1, out, True, False)
+    check_status()
+    assert (out.double() - 2 - ref.clamp_min(0)).norm() <= bound * (ref.norm() + 2 * (M * N) ** 0.5)
+    low = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    _lib.native().gemm_nt(a, b, bias, 0, low, False, False)
+    assert (low.double() - ref).norm() <= 2.0 ** -8 * ref.norm()
+    if M * N > 2e6 and "step" not in (la, lb):
+        aligned = torch.empty_like(low)
+        _lib.native().gemm_nt(a.contiguous().clone(), b.contiguous().clone(), bias, 0, aligned, False, False)
+        assert torch.equal(aligned, low)
