@@ -119,13 +119,16 @@ void gemm(const Op& a, const Op& b, const float* bias, int act, void* out, ll ld
           void* act_grad, const Tensor* like, bool tf32, bool splits) {
   const int M = static_cast<int>(a.rows), N = static_cast<int>(b.rows), K = static_cast<int>(a.k);
   TORCH_CHECK(a.k == b.k, "inner dimensions differ: [", a.rows, ", ", a.k, "] x [", b.rows, ", ", b.k, "]^T");
+  TORCH_CHECK(a.bf16 == b.bf16, "gemm: operands of two types");
+  TORCH_CHECK(!(out_bf16 && accumulate), "gemm: nothing accumulates onto a bf16 result");
+  TORCH_CHECK(a.bf16 || !out_bf16, "gemm: fp32 operands have an fp32 result");
   TORCH_CHECK(act <= FB_ACT_SIGMOID, "gemm: no epilogue evaluates activation ", act);
   if (M == 0 || N == 0) return;
   const bool ok = tma_ok(a) && tma_ok(b);
   const int a_mn = a.s_k == 1 ? 0 : 1, b_mn = b.s_k == 1 ? 0 : 1;
   const ll lda = a_mn ? a.s_k : a.s_row, ldb = b_mn ? b.s_k : b.s_row;
   if (a.bf16 && ok) {
-    if (g_max_ctas.load(std::memory_order_relaxed) == 0 && !(out_bf16 && accumulate)) {
+    if (g_max_ctas.load(std::memory_order_relaxed) == 0) {
       if (splits && fb_gemm_bf16_splitk_use(M, N, K)) {
         FB_CALL(fb_gemm_bf16_splitk, a.p, b.p, out, act_grad, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_bf16, act,
                 accumulate, 0, status(), cur_stream());
@@ -150,7 +153,7 @@ void gemm(const Op& a, const Op& b, const float* bias, int act, void* out, ll ld
     return;
   }
   TORCH_CHECK(act_grad == nullptr, "activation derivatives need operands that a TMA map describes");
-  if (!a.bf16 && tf32 && ok) {
+  if (tf32 && ok) {
     int rc = -3;
     if (M >= 512 && N >= 256)
       launch("fb_gemm_tf32", [&] {
@@ -163,7 +166,7 @@ void gemm(const Op& a, const Op& b, const float* bias, int act, void* out, ll ld
               bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, act, accumulate, g_max_ctas, status(), cur_stream());
     return;
   }
-  if (a.bf16 && b.bf16 && !(out_bf16 && accumulate)) {  // operands that a TMA map cannot describe
+  if (a.bf16) {  // operands that a TMA map cannot describe
     const bool rows_tma = reinterpret_cast<uintptr_t>(out) % 16 == 0 && ldc * (out_bf16 ? 2 : 4) % 16 == 0;
     if (like != nullptr && copies_repay(a, b, rows_tma)) {
       Tensor ka, kb;
@@ -176,38 +179,14 @@ void gemm(const Op& a, const Op& b, const float* bias, int act, void* out, ll ld
             accumulate, status(), cur_stream());
     return;
   }
-  if (!a.bf16 && !out_bf16 && K > kSimtK) {
+  if (K > kSimtK) {
     FB_CALL(fb_gemm_f32_tensor, static_cast<const float*>(a.p), static_cast<const float*>(b.p), static_cast<float*>(out),
             bias, M, N, K, a.s_row, a.s_k, b.s_row, b.s_k, ldc, act, accumulate, 1.f, 1, 1, 0, 0, 0, 0, 0, 0, status(),
             cur_stream());
     return;
   }
-  if (!a.bf16 && !out_bf16) {
-    FB_CALL(fb_gemm_f32_simt, static_cast<const float*>(a.p), static_cast<const float*>(b.p), static_cast<float*>(out),
-            bias, M, N, K, a.s_row, a.s_k, b.s_k, b.s_row, ldc, act, accumulate, 1, 0, 0, 0, cur_stream());
-    return;
-  }
-  // bf16 operands whose row pitch is not a multiple of 16 bytes: exact fp32 kernel on fp32 copies
-  TORCH_CHECK(like != nullptr, "gemm: missing tensor options");
-  auto wide = [&](const Op& o) {
-    Tensor v = at::from_blob(const_cast<void*>(o.p), {o.rows, o.k}, {o.s_row, o.s_k},
-                             like->options().dtype(o.bf16 ? at::kBFloat16 : at::kFloat));
-    return f32c(v);
-  };
-  Tensor af = wide(a), bf = wide(b);
-  if (out_bf16) {
-    Tensor res = empty({M, N}, *like, at::kFloat);
-    FB_CALL(fb_gemm_f32_simt, af.data_ptr<float>(), bf.data_ptr<float>(), res.data_ptr<float>(), bias, M, N, K, K, 1, 1,
-            K, N, act, 0, 1, 0, 0, 0, cur_stream());
-    Tensor o = at::from_blob(out, {M, N}, {ldc, 1}, like->options().dtype(at::kBFloat16));
-    if (ldc == N)
-      FB_CALL(fb_cast, res.data_ptr(), out, res.numel(), FB_DT_F32, FB_DT_BF16, cur_stream());
-    else
-      o.copy_(res);
-  } else {
-    FB_CALL(fb_gemm_f32_simt, af.data_ptr<float>(), bf.data_ptr<float>(), static_cast<float*>(out), bias, M, N, K, K, 1,
-            1, K, ldc, act, accumulate, 1, 0, 0, 0, cur_stream());
-  }
+  FB_CALL(fb_gemm_f32_simt, static_cast<const float*>(a.p), static_cast<const float*>(b.p), static_cast<float*>(out), bias,
+          M, N, K, a.s_row, a.s_k, b.s_k, b.s_row, ldc, act, accumulate, 1, 0, 0, 0, cur_stream());
 }
 
 // --------------------------------------------------------------------------------------------------- sinks

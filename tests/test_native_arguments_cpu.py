@@ -71,3 +71,12 @@ def test_no_mean_over_nothing(shape):
     assert lib.fb_ce_fwd(None, None, None, None, None, *shape, 1.0, 0, None) != 0
     assert lib.fb_nll_fwd(None, None, None, None, *shape, 1.0, 0, None, None) != 0
     assert lib.fb_loss_mean_fwd(None, None, None, None, 0, 0, 1.0, None) != 0
+
+
+def test_products_that_no_kernel_has():
+    """Mixed operand types, fp32 operands with a bf16 result, accumulation onto a bf16 result, an unknown activation."""
+    f, h = torch.zeros(8, 8), torch.zeros(8, 8, dtype=torch.bfloat16)
+    for a, b, out, act, acc in ((f, h, f, 0, False), (h, f, f, 0, False), (f, f, h, 0, False), (h, h, h, 0, True),
+                                (f, f, f, 6, False)):
+        with pytest.raises(RuntimeError, match="gemm"):
+            _native().gemm_nt(a, b, None, act, out, acc, False)
