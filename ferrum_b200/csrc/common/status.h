@@ -17,6 +17,10 @@ enum StatusCode : int32_t {
   kStatusBadArgument = 4,
 };
 
+// Site ids of the bounded waits, one range per kernel: 1 - 4 tcgen05_gemm, 11 - 14 tcgen05_gemm_2cta, 21 - 22
+// f32_tensor_gemm, 23 - 25 splitk_gemm, 31 - 32 layernorm, 51 - 57 attention, 61 - 77 attention_bwd, 81 - 82 rnn_seq;
+// index checks count apart (their code is kStatusBoundsViolation).
+
 // Layout of the status block (int32 words).
 enum StatusWord : int {
   kWordCode = 0,   // first non-zero StatusCode recorded

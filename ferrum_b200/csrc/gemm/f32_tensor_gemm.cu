@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split_kernel(const __grid_co
     }
     if (ok && nkb > 0) read_block();
     if (!ok) {
-      if (lane == 0) report_status(p.status, kStatusGemmTimeout, 50, blockIdx.x, warp);
+      if (lane == 0) report_status(p.status, kStatusGemmTimeout, 21, blockIdx.x, warp);
     }
   } else if (lane == 0) {
     // ---------------------------------------------------------------- MMA issue
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split_kernel(const __grid_co
       const int s = kb % C::kStages, buf = kb & 1;
       if (!ptx::mbar_wait(&acc_empty[buf], ((kb >> 1) & 1) ^ 1, abort_flag, p.timeout_ns) ||
           !ptx::mbar_wait(&full_bar[s], (kb / C::kStages) & 1, abort_flag, p.timeout_ns)) {
-        report_status(p.status, kStatusGemmTimeout, 51, blockIdx.x, kb);
+        report_status(p.status, kStatusGemmTimeout, 22, blockIdx.x, kb);
         break;
       }
       ptx::tc_fence_after();

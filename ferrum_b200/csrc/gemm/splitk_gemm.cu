@@ -133,7 +133,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
       bool ok = true;
       for (int kb = kb_lo; kb < kb_hi; ++kb, ++issued) {
         if (!ptx::mbar_wait(&empty_bar[s], phase, abort_flag, p.timeout_ns)) {
-          report_status(p.status, kStatusGemmTimeout, 60, blockIdx.x, kb);
+          report_status(p.status, kStatusGemmTimeout, 23, blockIdx.x, kb);
           ok = false;
           break;
         }
@@ -177,7 +177,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
       bool ok = true;
       for (int i = 0; i < kb_hi - kb_lo; ++i) {
         if (!ptx::mbar_wait(&full_bar[s], phase, abort_flag, p.timeout_ns)) {
-          report_status(p.status, kStatusGemmTimeout, 61, blockIdx.x, i);
+          report_status(p.status, kStatusGemmTimeout, 24, blockIdx.x, i);
           ok = false;
           break;
         }
@@ -205,7 +205,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
     if (have) {  // every MMA has completed, hence every copy too: the stages are free
       const bool ready = ptx::mbar_wait(acc_full, 0, abort_flag, p.timeout_ns);
       if (!__all_sync(0xffffffffu, ready)) {
-        if (lane == 0) report_status(p.status, kStatusGemmTimeout, 62, blockIdx.x, warp);
+        if (lane == 0) report_status(p.status, kStatusGemmTimeout, 25, blockIdx.x, warp);
         have = false;
       }
       ptx::tc_fence_after();

@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(kT, 1) seq_fwd_kernel(const SeqArgs a) {
     if (t > 0) {
       // a wait that gives up (reported) goes on with what is there, so that every thread keeps meeting the same barriers
       if (!ptx::mbar_wait(&arrived[buf], ((t - 1) >> 1) & 1, &abort_flag, a.timeout_ns))
-        report_status(a.status, kStatusGemmTimeout, 60, blockIdx.x, t);
+        report_status(a.status, kStatusGemmTimeout, 81, blockIdx.x, t);
       if (threadIdx.x == 0) ptx::mbar_arrive_expect_tx(&arrived[buf], bytes);  // for the step after next
     }
     if constexpr (kReg)
@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(kT, 1) seq_bwd_kernel(const SeqArgs a) {
     }
     in = fetch(t - 1);
     if (!ptx::mbar_wait(&arrived[buf], ((a.T - 1 - t) >> 1) & 1, &abort_flag, a.timeout_ns))
-      report_status(a.status, kStatusGemmTimeout, 61, blockIdx.x, t);
+      report_status(a.status, kStatusGemmTimeout, 82, blockIdx.x, t);
     if (threadIdx.x == 0) ptx::mbar_arrive_expect_tx(&arrived[buf], bytes);  // for the step after next
     if constexpr (kReg)
       matvec_reg<BS>(wreg, lane, cur, part);
