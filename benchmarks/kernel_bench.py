@@ -88,12 +88,12 @@ def _cases(small: bool):
     Cs = 1000
     lg = torch.randn(R, Cs, device=dev).to(bf)
     labels = torch.randint(0, Cs, (R,), device=dev)
-    rl = torch.empty(R, device=dev)
+    loss, ws = torch.empty((), device=dev), torch.empty(2048, device=dev)
     dl = torch.empty_like(lg)
     case("softmax_fwd_bf16_1000", lambda: F.softmax(lg, -1), R * Cs * 4, "K6")
     case("cross_entropy_fused_bf16_1000",
-         lambda: lib.fb_ce_fwd_bwd(lg.data_ptr(), labels.data_ptr(), rl.data_ptr(), dl.data_ptr(), R, Cs, 1.0 / R, 3, 3,
-                                   st()), R * Cs * 4, "K6b loss + dlogits")
+         lambda: lib.fb_ce_fwd(lg.data_ptr(), labels.data_ptr(), dl.data_ptr(), loss.data_ptr(), ws.data_ptr(), R, Cs,
+                               1.0 / R, 3, st()), R * Cs * 4, "K6b mean loss + dlogits")
     p32 = torch.rand(R, C, device=dev) * 0.9 + 0.05
     t32 = torch.rand(R, C, device=dev)
     case("mse_loss_fwd_f32", lambda: F.elementwise_loss(p32, t32, "mse"), n * 8, "K11")

@@ -156,11 +156,9 @@ _CUDA_SIGS = {
     # softmax / losses
     "fb_softmax_fwd": (I, [P, P, LL, I, I, I, P]),
     "fb_softmax_bwd": (I, [P, P, P, LL, I, I, I, P]),
-    "fb_ce_fwd_bwd": (I, [P, P, P, P, LL, I, F, I, I, P]),
     "fb_ce_fwd": (I, [P, P, P, P, P, LL, I, F, I, P]),
     "fb_nll_fwd": (I, [P, P, P, P, LL, I, F, I, P, P]),
     "fb_loss_mean_fwd": (I, [P, P, P, P, LL, I, F, P]),
-    "fb_loss_fwd": (I, [P, P, P, LL, I, F, P]),
     "fb_loss_bwd": (I, [P, P, P, P, LL, I, F, P]),
     # dropout / embedding / gather
     "fb_dropout_fwd": (I, [P, P, P, LL, F, U64, U64, I, P]),

@@ -159,10 +159,6 @@ int fb_batchnorm_bwd(const float* dy, const float* x, const float* gamma, const 
 int fb_softmax_fwd(const void* x, void* y, long long rows, int cols, int log_mode, int dtype, cudaStream_t stream);
 int fb_softmax_bwd(const void* dy, const void* y, void* dx, long long rows, int cols, int log_mode, int dtype,
                    cudaStream_t stream);
-// Fused log-softmax + NLL over integer labels.  Writes per-row loss, and when
-// dlogits != NULL the gradient (softmax - onehot) * grad_scale in `dlogits_dtype`.
-int fb_ce_fwd_bwd(const void* logits, const long long* labels, float* row_loss, void* dlogits, long long rows,
-                  int cols, float grad_scale, int dtype, int dlogits_dtype, cudaStream_t stream);
 // Mean losses (kernels/mean_loss.cu): the scalar scale * sum lands in `loss`; workspace = fb_mean_loss_workspace(n)
 // floats.  dlogits (optional, of the logits' type): (softmax - onehot) * scale.  gout: the incoming scalar gradient, read
 // on the device.
@@ -176,9 +172,7 @@ int fb_nll_bwd(const long long* target, const float* gout, void* dlog_probs, lon
                int dtype, cudaStream_t stream);
 int fb_loss_mean_fwd(const float* pred, const float* target, float* loss, float* workspace, long long n, int kind,
                      float scale, cudaStream_t stream);
-// Elementwise losses: sum of per-element loss into out[0] (pre-zeroed), scaled by `scale`.
-int fb_loss_fwd(const float* pred, const float* target, float* out, long long n, int kind, float scale,
-                cudaStream_t stream);
+// Gradient of the mean elementwise losses.
 int fb_loss_bwd(const float* pred, const float* target, const float* gout, float* dpred, long long n, int kind,
                 float scale, cudaStream_t stream);
 

@@ -97,36 +97,23 @@ __global__ void __launch_bounds__(kThreads) add_partials_kernel(const float* __r
   }
 }
 
-template <typename T>
-struct Vec {
-  static constexpr int n = 16 / sizeof(T);
-  __device__ static void load(const T* p, float (&f)[n]) {
-    const uint4 raw = *reinterpret_cast<const uint4*>(p);
-    if constexpr (sizeof(T) == 2) {
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+__device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&f)[8]) {
+  const uint4 raw = *reinterpret_cast<const uint4*>(p);
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 t = __bfloat1622float2(h[e]);
-        f[2 * e] = t.x;
-        f[2 * e + 1] = t.y;
-      }
-    } else {
-      f[0] = __uint_as_float(raw.x); f[1] = __uint_as_float(raw.y);
-      f[2] = __uint_as_float(raw.z); f[3] = __uint_as_float(raw.w);
-    }
+  for (int e = 0; e < 4; ++e) {
+    const float2 t = __bfloat1622float2(h[e]);
+    f[2 * e] = t.x;
+    f[2 * e + 1] = t.y;
   }
-  __device__ static void store(T* p, const float (&f)[n]) {
-    if constexpr (sizeof(T) == 2) {
-      uint4 raw;
-      __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&raw);
+}
+__device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
+  uint4 raw;
+  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&raw);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) h[e] = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
-      *reinterpret_cast<uint4*>(p) = raw;
-    } else {
-      *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]);
-    }
-  }
-};
+  for (int e = 0; e < 4; ++e) h[e] = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
+  *reinterpret_cast<uint4*>(p) = raw;
+}
 
 // Rows of 264 .. 4096 bf16 logits (multiples of 8, 16-byte aligned): a warp owns a row and keeps it in registers (K
 // vectors of 8 per lane), so the row is read once and both reductions are warp shuffles.
@@ -148,7 +135,7 @@ ce_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const long long* __restr
     for (int k = 0; k < K; ++k) {
       const int vi = lane + 32 * k;
       if (vi < nvec) {
-        Vec<__nv_bfloat16>::load(xr + vi * 8, v[k]);
+        load8(xr + vi * 8, v[k]);
 #pragma unroll
         for (int e = 0; e < 8; ++e) m = fmaxf(m, v[k][e]);
       } else {
@@ -185,7 +172,7 @@ ce_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const long long* __restr
           d[e] = v[k][e] * inv;
           if (valid && vi * 8 + e == lab) d[e] -= scale;
         }
-        Vec<__nv_bfloat16>::store(dx + row * cols + vi * 8, d);
+        store8(dx + row * cols + vi * 8, d);
       }
     }
   }

@@ -1,6 +1,5 @@
-// Row softmax / log-softmax (forward, backward), the fused log-softmax + NLL /
-// cross-entropy kernel that also emits the logit gradient, and the fused
-// elementwise losses (mse, bce, l1, smooth-l1) with their backward.
+// Row softmax / log-softmax (forward, backward) and the backward of the elementwise losses (mse, bce, l1,
+// smooth-l1); the losses themselves are in mean_loss.cu.
 //
 // Reference:
 //   ferrum-cuda/src/kernels.rs:501-621  softmax / log_softmax: per row over the last
@@ -15,7 +14,6 @@
 #include <cuda_runtime.h>
 #include <float.h>
 
-#include "../common/status.h"
 #include "../include/ferrum_kernels.h"
 
 namespace fb {
@@ -237,136 +235,7 @@ softmax_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ y, T* __restr
   }
 }
 
-template <typename T, typename G, int TPR>
-__global__ void __launch_bounds__(256)
-ce_kernel(const T* __restrict__ logits, const long long* __restrict__ labels, float* __restrict__ row_loss,
-          G* __restrict__ dlogits, long long rows, int cols, float grad_scale, int32_t* bstatus) {
-  __shared__ float smem[8];
-  constexpr int kRPB = 256 / TPR;
-  const int sub = threadIdx.x / TPR, t = threadIdx.x % TPR;
-  for (long long row0 = static_cast<long long>(blockIdx.x) * kRPB; row0 < rows;
-       row0 += static_cast<long long>(gridDim.x) * kRPB) {
-    const long long row = row0 + sub;
-    const bool live = row < rows;
-    const T* xr = logits + (live ? row : 0) * cols;
-    float m = -FLT_MAX;
-    if (live)
-      for (int c = t; c < cols; c += TPR) m = fmaxf(m, ldf(xr + c));
-    m = group_reduce<TPR, true>(m, smem);
-    float s = 0.f;
-    if (live)
-      for (int c = t; c < cols; c += TPR) s += expf(ldf(xr + c) - m);
-    s = group_reduce<TPR, false>(s, smem);
-    if (live) {
-      long long lab = labels[row];
-      const bool valid = lab >= 0 && lab < cols;  // out-of-range labels contribute nothing
-      if (!valid && t == 0) (void)FB_INDEX_OK(bstatus, 41, lab, cols);  // the debug build also reports them
-      if (t == 0 && row_loss) row_loss[row] = valid ? (m + logf(s) - ldf(xr + lab)) : 0.f;
-      if (dlogits) {
-        const float inv = 1.f / s;
-        G* gr = dlogits + row * cols;
-        for (int c = t; c < cols; c += TPR) {
-          float p = expf(ldf(xr + c) - m) * inv;
-          if (c == lab) p -= 1.f;
-          stf(gr + c, valid ? p * grad_scale : 0.f);
-        }
-      }
-    }
-  }
-}
-
-
-// bf16 rows of 264..4096 columns (multiples of 8, 16-byte aligned): a warp owns a row, every lane keeps its
-// elements in registers (K vectors of 8), so the row is read once, exp is evaluated once per element and the
-// three reductions are warp shuffles without a block barrier.
-template <int K>
-__global__ void __launch_bounds__(256, K <= 4 ? 4 : (K <= 8 ? 2 : 1))
-ce_warp_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __restrict__ labels,
-               float* __restrict__ row_loss, __nv_bfloat16* __restrict__ dlogits, long long rows, int cols,
-               float grad_scale, int32_t* bstatus) {
-  const int lane = threadIdx.x & 31;
-  const int nvec = cols >> 3;
-  const long long warp_id = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const long long nwarps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
-  for (long long row = warp_id; row < rows; row += nwarps) {
-    const __nv_bfloat16* xr = logits + row * cols;
-    float v[K][8];
-    float m = -FLT_MAX;
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int vi = lane + 32 * k;
-      if (vi < nvec) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(xr + vi * 8);
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = __bfloat1622float2(h[e]);
-          v[k][2 * e] = f.x;
-          v[k][2 * e + 1] = f.y;
-          m = fmaxf(m, fmaxf(f.x, f.y));
-        }
-      } else {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) v[k][e] = -FLT_MAX;
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    float s = 0.f;
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        v[k][e] = __expf(v[k][e] - m);  // padded lanes: exp(-huge) = 0
-        s += v[k][e];
-      }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    const long long lab = labels[row];
-    const bool valid = lab >= 0 && lab < cols;
-    if (!valid && lane == 0) (void)FB_INDEX_OK(bstatus, 41, lab, cols);
-    if (lane == 0 && row_loss) row_loss[row] = valid ? (m + logf(s) - __bfloat162float(xr[lab])) : 0.f;
-    if (dlogits) {
-      const float inv = valid ? grad_scale / s : 0.f;
-      __nv_bfloat16* gr = dlogits + row * cols;
-#pragma unroll
-      for (int k = 0; k < K; ++k) {
-        const int vi = lane + 32 * k;
-        if (vi < nvec) {
-          uint4 out;
-          __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&out);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            float a = v[k][2 * e] * inv, b = v[k][2 * e + 1] * inv;
-            if (valid && vi * 8 + 2 * e == lab) a -= grad_scale;
-            if (valid && vi * 8 + 2 * e + 1 == lab) b -= grad_scale;
-            h[e] = __floats2bfloat162_rn(a, b);
-          }
-          *reinterpret_cast<uint4*>(gr + vi * 8) = out;
-        }
-      }
-    }
-  }
-}
-
 // ------------------------------------------------------- elementwise losses
-__device__ __forceinline__ float loss_elem(float p, float t, int kind) {
-  const float d = p - t;
-  switch (kind) {
-    case FB_LOSS_MSE: return d * d;
-    case FB_LOSS_BCE: {
-      const float eps = 1e-7f;
-      const float pc = p + eps;
-      const float q = (1.f + eps) - pc;
-      return -(t * logf(pc) + (1.f - t) * logf(q));
-    }
-    case FB_LOSS_L1: return fabsf(d);
-    default: {
-      const float a = fabsf(d);
-      return a < 1.f ? 0.5f * d * d : a - 0.5f;
-    }
-  }
-}
 __device__ __forceinline__ float loss_grad(float p, float t, int kind) {
   const float d = p - t;
   switch (kind) {
@@ -383,17 +252,6 @@ __device__ __forceinline__ float loss_grad(float p, float t, int kind) {
       return a < 1.f ? d : (d > 0.f ? 1.f : -1.f);
     }
   }
-}
-
-__global__ void loss_fwd_kernel(const float* __restrict__ p, const float* __restrict__ t, float* __restrict__ out,
-                                long long n, int kind, float scale) {
-  __shared__ float smem[8];
-  float acc = 0.f;
-  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
-  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
-    acc += loss_elem(p[i], t[i], kind);
-  acc = group_reduce<256, false>(acc, smem);
-  if (threadIdx.x == 0) atomicAdd(out, acc * scale);
 }
 
 __global__ void loss_bwd_kernel(const float* __restrict__ p, const float* __restrict__ t,
@@ -462,39 +320,6 @@ int softmax_bwd_t(const void* dy, const void* y, void* dx, long long rows, int c
         static_cast<const T*>(dy), static_cast<const T*>(y), static_cast<T*>(dx), rows, cols, log_mode);
   return static_cast<int>(cudaGetLastError());
 }
-// bf16 logits with bf16 gradient, vectorisable rows: the warp-per-row kernel.
-bool ce_warp_launch(const void* logits, const long long* labels, float* row_loss, void* dlogits, long long rows,
-                    int cols, float gs, cudaStream_t st) {
-  if (cols % 8 != 0 || cols < 264 || cols > 4096) return false;
-  if (((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(dlogits)) & 15) != 0) return false;
-  const __nv_bfloat16* x = static_cast<const __nv_bfloat16*>(logits);
-  __nv_bfloat16* g = static_cast<__nv_bfloat16*>(dlogits);
-  const int grid = row_grid(rows, 8);
-  const int k = (cols / 8 + 31) / 32;
-  if (k <= 4)
-    ce_warp_kernel<4><<<grid, 256, 0, st>>>(x, labels, row_loss, g, rows, cols, gs, bounds_status_ref());
-  else if (k <= 8)
-    ce_warp_kernel<8><<<grid, 256, 0, st>>>(x, labels, row_loss, g, rows, cols, gs, bounds_status_ref());
-  else
-    ce_warp_kernel<16><<<grid, 256, 0, st>>>(x, labels, row_loss, g, rows, cols, gs, bounds_status_ref());
-  return true;
-}
-
-template <typename T, typename G>
-int ce_t(const void* logits, const long long* labels, float* row_loss, void* dlogits, long long rows, int cols,
-         float gs, cudaStream_t st) {
-  if (sizeof(T) == 2 && sizeof(G) == 2 && ce_warp_launch(logits, labels, row_loss, dlogits, rows, cols, gs, st))
-    return static_cast<int>(cudaGetLastError());
-  if (cols <= 512)
-    ce_kernel<T, G, 32><<<row_grid(rows, 8), 256, 0, st>>>(static_cast<const T*>(logits), labels, row_loss,
-                                                          static_cast<G*>(dlogits), rows, cols, gs,
-                                                          bounds_status_ref());
-  else
-    ce_kernel<T, G, 256><<<row_grid(rows, 1), 256, 0, st>>>(static_cast<const T*>(logits), labels, row_loss,
-                                                           static_cast<G*>(dlogits), rows, cols, gs,
-                                                          bounds_status_ref());
-  return static_cast<int>(cudaGetLastError());
-}
 
 }  // namespace
 }  // namespace fb
@@ -514,29 +339,6 @@ extern "C" int fb_softmax_bwd(const void* dy, const void* y, void* dx, long long
   if (dtype == FB_DT_F32) return softmax_bwd_t<float>(dy, y, dx, rows, cols, log_mode, stream);
   if (dtype == FB_DT_BF16) return softmax_bwd_t<__nv_bfloat16>(dy, y, dx, rows, cols, log_mode, stream);
   return -1;
-}
-extern "C" int fb_ce_fwd_bwd(const void* logits, const long long* labels, float* row_loss, void* dlogits,
-                             long long rows, int cols, float grad_scale, int dtype, int dlogits_dtype,
-                             cudaStream_t stream) {
-  if (rows <= 0 || cols <= 0) return 0;
-  if (dtype == FB_DT_F32 && dlogits_dtype == FB_DT_F32)
-    return ce_t<float, float>(logits, labels, row_loss, dlogits, rows, cols, grad_scale, stream);
-  if (dtype == FB_DT_F32 && dlogits_dtype == FB_DT_BF16)
-    return ce_t<float, __nv_bfloat16>(logits, labels, row_loss, dlogits, rows, cols, grad_scale, stream);
-  if (dtype == FB_DT_BF16 && dlogits_dtype == FB_DT_BF16)
-    return ce_t<__nv_bfloat16, __nv_bfloat16>(logits, labels, row_loss, dlogits, rows, cols, grad_scale, stream);
-  if (dtype == FB_DT_BF16 && dlogits_dtype == FB_DT_F32)
-    return ce_t<__nv_bfloat16, float>(logits, labels, row_loss, dlogits, rows, cols, grad_scale, stream);
-  return -1;
-}
-extern "C" int fb_loss_fwd(const float* pred, const float* target, float* out, long long n, int kind, float scale,
-                           cudaStream_t stream) {
-  if (n <= 0) return 0;
-  long long nb = (n + 255) / 256;
-  const long long cap = static_cast<long long>(sm_count()) * 4;
-  if (nb > cap) nb = cap;
-  loss_fwd_kernel<<<static_cast<int>(nb), 256, 0, stream>>>(pred, target, out, n, kind, scale);
-  return static_cast<int>(cudaGetLastError());
 }
 extern "C" int fb_loss_bwd(const float* pred, const float* target, const float* gout, float* dpred, long long n,
                            int kind, float scale, cudaStream_t stream) {
