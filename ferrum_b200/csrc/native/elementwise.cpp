@@ -181,13 +181,18 @@ struct NllNode : Node {
   }
 };
 
+// Whether the op takes these arguments: one target per row, on the device of the log-probabilities.
+bool nll_takes(const Tensor& log_probs, const Tensor& target) {
+  return log_probs.is_cuda() && (is_f32(log_probs) || is_bf16(log_probs)) && log_probs.numel() > 0 &&
+         target.numel() == rows_of(log_probs) && target.device() == log_probs.device();
+}
 Tensor nll(const Tensor& log_probs, const Tensor& target) {
   NoAutograd below;
   const int64_t cols = log_probs.size(-1), rows = rows_of(log_probs);
   TORCH_CHECK_VALUE(rows > 0 && target.numel() == rows, "nll: one target per row expected, got ", target.sizes(), " for ",
                     log_probs.sizes());
   check_on(log_probs, target, "the target");
-  Tensor x = contig(log_probs), t = contig(target);
+  Tensor x = contig(log_probs), t = contig(target.scalar_type() == at::kLong ? target : target.to(at::kLong));
   Tensor loss = empty({}, x, at::kFloat), ws = empty({fb_mean_loss_workspace(rows)}, x, at::kFloat);
   FB_CALL(fb_nll_fwd, x.data_ptr(), reinterpret_cast<const ll*>(t.data_ptr<int64_t>()), loss.data_ptr<float>(),
           ws.data_ptr<float>(), rows, static_cast<int>(cols), -1.f / static_cast<float>(rows), dt(x), status(), cur_stream());
@@ -256,6 +261,7 @@ void bind_elementwise(py::module_& m) {
   m.def("softmax", &softmax);
   m.def("cross_entropy", &cross_entropy);
   m.def("nll", &nll);
+  m.def("nll_takes", &nll_takes);
   m.def("elementwise_loss", &elementwise_loss);
 }
 

@@ -14,6 +14,7 @@ import functools
 
 import torch
 
+from .. import _lib
 from ..core import ShapeMismatch, Tensor, _unwrap
 from ..ops import functional as F
 
@@ -47,10 +48,9 @@ def _ce_onehot(log_probs, targets):
 
 
 def _nll_index(log_probs, targets):
-    C = log_probs.shape[-1]
-    if (F._native(log_probs) and targets.device == log_probs.device and log_probs.numel() > 0
-            and targets.numel() * C == log_probs.numel()):
+    if F._native(log_probs) and _lib.native().nll_takes(log_probs, targets):
         return F.nll_index(log_probs, targets)
+    C = log_probs.shape[-1]
     lp2 = log_probs.reshape(-1, C)
     onehot = torch.zeros(lp2.shape, device=lp2.device, dtype=lp2.dtype)
     onehot.scatter_(1, targets.reshape(-1, 1).to(torch.int64), 1.0)

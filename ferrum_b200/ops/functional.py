@@ -808,7 +808,7 @@ def cross_entropy_logits(logits: torch.Tensor, labels: torch.Tensor) -> torch.Te
 
 def nll_index(log_probs: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
     """Mean over the rows of ``-log_probs[i, targets[i]]`` for integer ``targets`` on the GPU."""
-    return _lib.native().nll(log_probs, targets.reshape(-1).to(torch.int64))
+    return _lib.native().nll(log_probs, targets)
 
 
 def elementwise_loss(pred: torch.Tensor, target: torch.Tensor, kind: str) -> torch.Tensor:
