@@ -130,9 +130,9 @@ extern std::atomic<int> g_max_ctas;
 bool tma_ok(const Op& a);
 // out[M, N] (row pitch ldc) = act(a b^T + bias), += out when `accumulate`; act_grad: see fb_gemm_bf16.  `splits`: bf16
 // products of few output tiles may divide K over a cluster.  Set for weight gradients alone: forward results and input
-// gradients keep one order of summation, so that a row's result depends neither on the rows beside it nor on whether
-// gradients are recorded (carried through eight bf16 layers, another order moved the logits by 0.9 %, as far from the
-// exact ones as before).
+// gradients of aligned bf16 operands keep one order of summation, so that a row's result depends neither on the rows
+// beside it nor on whether gradients are recorded (carried through eight bf16 layers, another order moved the logits by
+// 0.9 %, as far from the exact ones as before).
 void gemm(const Op& a, const Op& b, const float* bias, int act, void* out, ll ldc, bool out_bf16,
           bool accumulate = false, void* act_grad = nullptr, const Tensor* like = nullptr, bool tf32 = false, bool splits = false);
 

@@ -1,5 +1,6 @@
-"""A bf16 forward pass has one order of summation: neither the recording of gradients, nor the rows that share a batch,
-nor the kernel that a number of rows selects changes a bit, at sizes where weight gradients divide their reduction."""
+"""A bf16 forward pass over aligned rows has one order of summation: neither the recording of gradients, nor the rows that
+share a batch, nor the kernel that a number of rows selects changes a bit, at sizes where weight gradients divide their
+reduction."""
 import pytest
 import torch
 
