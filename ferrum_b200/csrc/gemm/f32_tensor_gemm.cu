@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split_kernel(const __grid_co
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
   cg::cluster_group cluster = cg::this_cluster();
   const int splits = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
 
@@ -416,9 +416,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split_kernel(const __grid_co
     if (!ok) {
       if (lane == 0) report_status(p.status, kStatusGemmTimeout, 21, blockIdx.x, warp);
     }
-  } else if (lane == 0) {
+  } else if (ptx::elect_one()) {
     // ---------------------------------------------------------------- MMA issue
     const uint32_t idesc = ptx::make_idesc(1u, kBM, BN, 0, 0);
+    const uint64_t first = C::desc(ptx::smem_u32(smem));
     for (int kb = 0; kb < nkb; ++kb) {
       const int s = kb % C::kStages, buf = kb & 1;
       if (!ptx::mbar_wait(&acc_empty[buf], ((kb >> 1) & 1) ^ 1, abort_flag, p.timeout_ns) ||
@@ -427,7 +428,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split_kernel(const __grid_co
         break;
       }
       ptx::tc_fence_after();
-      const uint32_t sa = ptx::smem_u32(smem + s * C::kStage), sb = sa + kPlanes * C::kPlaneA;
+      const uint64_t da = ptx::desc_advance(first, s * C::kStage), db = ptx::desc_advance(da, kPlanes * C::kPlaneA);
       const uint32_t d = tmem + buf * BN;
       constexpr int ia[6] = {2, 0, 1, 1, 0, 0}, ib[6] = {0, 2, 1, 0, 1, 0};  // small products first
       constexpr int kFirst = 6 - El<T>::kProducts;
@@ -435,9 +436,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split_kernel(const __grid_co
       for (int q = kFirst; q < 6; ++q) {
 #pragma unroll
         for (int k = 0; k < C::kBK / 16; ++k) {
-          const uint64_t ad = C::desc(sa + ia[q] * C::kPlaneA + k * 32);
-          const uint64_t bd = C::desc(sb + ib[q] * C::kPlaneB + k * 32);
-          ptx::umma_f16(d, ad, bd, idesc, (q != kFirst || k != 0) ? 1u : 0u);
+          ptx::umma_f16(d, ptx::desc_advance(da, ia[q] * C::kPlaneA + k * 32),
+                        ptx::desc_advance(db, ib[q] * C::kPlaneB + k * 32), idesc, (q != kFirst || k != 0) ? 1u : 0u);
         }
       }
       ptx::umma_commit(&empty_bar[s]);

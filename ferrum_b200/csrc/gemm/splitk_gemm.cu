@@ -99,7 +99,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
   cg::cluster_group cluster = cg::this_cluster();
   const int splits = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
   const int tile_id = static_cast<int>(blockIdx.x) / splits;
@@ -127,7 +127,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       int issued = 0, s = 0;
       uint32_t phase = 1;
       bool ok = true;
@@ -168,10 +168,12 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && kb_hi > kb_lo) {
+    if (kb_hi > kb_lo && ptx::elect_one()) {
       const uint32_t idesc = ptx::make_idesc(1u, kRowsP, BN, p.p_mn, p.q_mn);
       const uint32_t p_lbo = p.p_mn ? kChunk : 16, q_lbo = p.q_mn ? kChunk : 16;
       const uint32_t p_step = p.p_mn ? 16 * 128 : 32, q_step = p.q_mn ? 16 * 128 : 32;
+      const uint64_t p_first = ptx::make_smem_desc_sw128(ptx::smem_u32(smem), p_lbo, 1024);
+      const uint64_t q_first = ptx::make_smem_desc_sw128(ptx::smem_u32(smem) + C::kP, q_lbo, 1024);
       int s = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -182,11 +184,11 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
           break;
         }
         ptx::tc_fence_after();
-        const uint32_t sp = ptx::smem_u32(smem + s * p.stage_bytes), sq = sp + C::kP;
+        const uint64_t dp = ptx::desc_advance(p_first, s * p.stage_bytes), dq = ptx::desc_advance(q_first, s * p.stage_bytes);
 #pragma unroll
         for (int k = 0; k < kBK / 16; ++k)
-          ptx::umma_f16(tmem, ptx::make_smem_desc_sw128(sp + k * p_step, p_lbo, 1024),
-                        ptx::make_smem_desc_sw128(sq + k * q_step, q_lbo, 1024), idesc, (i | k) != 0 ? 1u : 0u);
+          ptx::umma_f16(tmem, ptx::desc_advance(dp, k * p_step), ptx::desc_advance(dq, k * q_step), idesc,
+                        (i | k) != 0 ? 1u : 0u);
         ptx::umma_commit(&empty_bar[s]);
         if (++s == p.stages) {
           s = 0;

@@ -84,18 +84,20 @@ __device__ __forceinline__ float ex2f(float x) {
 // 128 x 128 x D product of two K-major tiles (rows x D): the score shape.
 template <int D>
 __device__ __forceinline__ void mma_scores(uint32_t tmem, uint32_t a, uint32_t b, uint32_t idesc) {
+  const uint64_t da = ptx::make_smem_desc_sw128(a, 16, 1024), db = ptx::make_smem_desc_sw128(b, 16, 1024);
 #pragma unroll
   for (int k = 0; k < D / 16; ++k)
-    ptx::umma_f16(tmem, ptx::make_smem_desc_sw128(a + (k >> 2) * kBlk + (k & 3) * 32, 16, 1024),
-                  ptx::make_smem_desc_sw128(b + (k >> 2) * kBlk + (k & 3) * 32, 16, 1024), idesc, k != 0 ? 1u : 0u);
+    ptx::umma_f16(tmem, ptx::desc_advance(da, (k >> 2) * kBlk + (k & 3) * 32),
+                  ptx::desc_advance(db, (k >> 2) * kBlk + (k & 3) * 32), idesc, k != 0 ? 1u : 0u);
 }
 // 128 x D x 128 product: A = a 128 x 128 matrix in two K-major k-blocks, B = a 128 x D tile whose D columns are
 // contiguous (MN-major; its 64-column blocks lie kBlk apart): the P V shape of the forward kernel.
 __device__ __forceinline__ void mma_pv(uint32_t tmem, uint32_t a, uint32_t b, uint32_t idesc, bool accumulate) {
+  const uint64_t da = ptx::make_smem_desc_sw128(a, 16, 1024), db = ptx::make_smem_desc_sw128(b, kBlk, 1024);
 #pragma unroll
   for (int k = 0; k < kT / 16; ++k)
-    ptx::umma_f16(tmem, ptx::make_smem_desc_sw128(a + (k >> 2) * kBlk + (k & 3) * 32, 16, 1024),
-                  ptx::make_smem_desc_sw128(b + k * 2048, kBlk, 1024), idesc, (accumulate || k != 0) ? 1u : 0u);
+    ptx::umma_f16(tmem, ptx::desc_advance(da, (k >> 2) * kBlk + (k & 3) * 32), ptx::desc_advance(db, k * 2048), idesc,
+                  (accumulate || k != 0) ? 1u : 0u);
 }
 
 // 16 columns (8 bf16 pairs) of one row, starting at column col (a multiple of 16): two 16-byte chunks of the row's
@@ -156,7 +158,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(dq_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
   const int q0 = blockIdx.x * kT;
   const int h = blockIdx.y % p.H, b = blockIdx.y / p.H;
   const int off = p.Skv - p.Sq;
@@ -191,7 +193,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   const uint32_t t_s = tmem_base, t_dp = tmem_base + 128, t_dq = tmem_base + 256;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       ptx::mbar_arrive_expect_tx(q_full, 2 * kTile);
       load_tile<D>(sq, &map_q, q_full, q0, h, b);
       load_tile<D>(sdo, &map_do, q_full, q0, h, b);
@@ -208,7 +210,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       const uint32_t idesc_s = ptx::make_idesc(1u, kT, kT, 0, 0);
       const uint32_t idesc_o = ptx::make_idesc(1u, kT, D, 0, 1);
       const uint32_t sq_a = ptx::smem_u32(sq), sdo_a = ptx::smem_u32(sdo), sds_a = ptx::smem_u32(sds);
@@ -374,7 +376,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
   const int k0 = blockIdx.x * kT;
   const int h = blockIdx.y % p.H, b = blockIdx.y / p.H;
   const int off = p.Skv - p.Sq;
@@ -411,7 +413,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   const uint32_t t_s = tmem_base, t_dp = tmem_base + 128, t_dv = tmem_base + 256, t_dk = tmem_base + 256 + D;
 
   if (warp == 0) {
-    if (lane == 0 && n_iter > 0) {
+    if (n_iter > 0 && ptx::elect_one()) {
       ptx::mbar_arrive_expect_tx(kv_full, 2 * kTile);
       load_tile<D>(sk, &map_k, kv_full, k0, h, b);
       load_tile<D>(sv, &map_v, kv_full, k0, h, b);
@@ -428,7 +430,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && n_iter > 0) {
+    if (n_iter > 0 && ptx::elect_one()) {
       const uint32_t idesc_s = ptx::make_idesc(1u, kT, kT, 0, 0);
       const uint32_t idesc_o = ptx::make_idesc(1u, kT, D, 0, 1);
       const uint32_t sk_a = ptx::smem_u32(sk), sv_a = ptx::smem_u32(sv);
