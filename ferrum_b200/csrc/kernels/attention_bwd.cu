@@ -6,12 +6,15 @@
 // Two kernels, both shaped like the forward kernel (same operand layouts, same roles), so that neither needs an
 // atomic or a cross-CTA reduction:
 //
-// Roles of a CTA (320 threads): warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 the elementwise work — two
-// warps per tensor-memory lane quarter, each taking 64 of a tile's 128 columns, because that work (two
-// tensor-memory reads, an exponential and half a dozen multiply-adds per score) and not the MMAs bounds a tile.
+// Roles of a CTA (320 threads): warp 0 TMA producer, warp 1 MMA issuer, warps 2-5 and 6-9 two groups for the elementwise
+// work (two tensor-memory reads, an exponential and half a dozen multiply-adds per score).  The stationary tile has 128
+// rows, the other side is walked 64 at a time: a tile's scores and dP take 128 columns of tensor memory, so there are two
+// of them, one per group, and the products of one tile run beside the elementwise work of the other.  With tiles of 128 x
+// 128 the scores filled tensor memory and every tile was a serial chain of product, elementwise work and product.  8 x 16
+// heads of 64, 1024 rows: dQ 116 -> 99 us, dK / dV 170 -> 140; the sums and their order are the same.
 //
 //   attn_bwd_dq_kernel    a CTA owns 128 query rows and walks the key / value tiles:
-//                           S = Q K_j^T, dP = dO V_j^T            (tensor memory, 2 x 128 columns)
+//                           S = Q K_j^T, dP = dO V_j^T            (tensor memory, 2 x 64 columns per group)
 //                           dS = P * (dP - delta) * scale          (thread = query row; bf16 into shared memory)
 //                           dQ += dS K_j                           (accumulates in tensor memory over all tiles)
 //   attn_bwd_dkv_kernel   a CTA owns 128 keys and walks the query tiles, everything transposed:
@@ -28,6 +31,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <utility>
 
 #include "../common/ptx.cuh"
 #include "../common/status.h"
@@ -36,29 +40,37 @@
 namespace fb {
 namespace {
 
-constexpr int kT = 128;                     // rows of a query tile = rows of a key tile
+constexpr int kT = 128;                     // rows of the stationary tile
+constexpr int kW = 64;                      // rows of a tile of the side that is walked
 constexpr int kBlk = kT * 128;              // 16 KB: 128 rows of 64 bf16 = one 128-byte-swizzled block
-constexpr int kPBytes = 2 * kBlk;           // a 128 x 128 bf16 matrix: two k-blocks of 128 rows x 128 bytes
-constexpr int kBwdThreads = 320;            // TMA warp, MMA warp, eight softmax warps
-constexpr int kSoftmaxWarps = 8;            // two per tensor-memory lane quarter, 64 of the tile's 128 columns each
-constexpr int kTmemBwd = 512;
-// D = head dimension (64 or 128).  An operand tile (128 rows x D) is D / 64 blocks side by side.  With D = 64 the
-// tiles that change per iteration sit in a two-stage ring; with D = 128 shared memory (160 KB / 206 KB) and tensor
-// memory (dK/dV: all 512 columns) leave room for one stage only.
+constexpr int kBlkW = kW * 128;             // the same of 64 rows
+constexpr int kBwdThreads = 320;            // TMA warp, MMA warp, two groups of four softmax warps
+constexpr int kTmemBwd = 512;               // scores and dP of the groups: columns 0 .. 255; accumulators from 256 on
+// D = head dimension (64 or 128).  An operand tile is D / 64 blocks side by side.
 template <int D>
 struct BwdCfg {
   static constexpr int kNB = D / 64;
-  static constexpr int kTile = kNB * kBlk;
-  static constexpr int kStages = D == 64 ? 2 : 1;
-  static constexpr int kSmemDq = 2 * kTile + 2 * kStages * kTile + kPBytes + 1024 + 256;  // Q dO | K | V | dS
-  static constexpr int kSmemDkv = 2 * kTile + 2 * kStages * kTile + 2 * kPBytes + 8192 + 1024 + 256;  // K V | Q | dO | P^T dS^T | lse, delta
+  static constexpr int kTile = kNB * kBlk, kTileW = kNB * kBlkW;
+  static constexpr int kStages = D == 64 ? 4 : 3;  // three: a tile's scores are issued two tiles ahead of its release
+  static constexpr int kSmemDq = 2 * kTile + 2 * kStages * kTileW + 2 * kBlk + 1024 + 256;          // Q dO | K V | dS
+  static constexpr int kSmemDkv = 2 * kTile + 2 * kStages * kTileW + 4 * kBlk + 1024 + 1024 + 256;  // K V | Q dO | P^T dS^T | lse, delta
 };
 
-// One operand tile: D / 64 boxes of 64 columns x 128 rows.
+// One operand tile: D / 64 boxes of 64 columns, `bytes` each.
 template <int D>
-__device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int row0, int h, int b) {
+__device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int row0, int h, int b,
+                                          int bytes) {
 #pragma unroll
-  for (int nb = 0; nb < D / 64; ++nb) ptx::tma_load_4d(dst + nb * kBlk, map, bar, nb * 64, row0, h, b);
+  for (int nb = 0; nb < D / 64; ++nb) ptx::tma_load_4d(dst + nb * bytes, map, bar, nb * 64, row0, h, b);
+}
+// Given up: no copy may outlive the CTA (bounded).  `issued` tiles went through the ring.
+__device__ __forceinline__ void drain(uint64_t* fixed, uint64_t* full, int issued, int stages, unsigned long long timeout_ns) {
+  const uint64_t t0 = ptx::globaltimer();
+  while (!ptx::mbar_try_wait(fixed, 0) && ptx::globaltimer() - t0 <= timeout_ns) {
+  }
+  for (int st = 0; st < stages && st < issued; ++st)
+    while (!ptx::mbar_try_wait(&full[st], ((issued - 1 - st) / stages) & 1) && ptx::globaltimer() - t0 <= timeout_ns) {
+    }
 }
 constexpr float kLog2e = 1.4426950408889634f;
 
@@ -81,32 +93,55 @@ __device__ __forceinline__ float ex2f(float x) {
   return y;
 }
 
-// 128 x 128 x D product of two K-major tiles (rows x D): the score shape.
+// 128 x 64 x D product of two K-major tiles (rows x D): the score shape.
 template <int D>
 __device__ __forceinline__ void mma_scores(uint32_t tmem, uint32_t a, uint32_t b, uint32_t idesc) {
   const uint64_t da = ptx::make_smem_desc_sw128(a, 16, 1024), db = ptx::make_smem_desc_sw128(b, 16, 1024);
 #pragma unroll
   for (int k = 0; k < D / 16; ++k)
     ptx::umma_f16(tmem, ptx::desc_advance(da, (k >> 2) * kBlk + (k & 3) * 32),
-                  ptx::desc_advance(db, (k >> 2) * kBlk + (k & 3) * 32), idesc, k != 0 ? 1u : 0u);
+                  ptx::desc_advance(db, (k >> 2) * kBlkW + (k & 3) * 32), idesc, k != 0 ? 1u : 0u);
 }
-// 128 x D x 128 product: A = a 128 x 128 matrix in two K-major k-blocks, B = a 128 x D tile whose D columns are
-// contiguous (MN-major; its 64-column blocks lie kBlk apart): the P V shape of the forward kernel.
+// 128 x D x 64 product: A = a 128 x 64 matrix, K-major, B = a 64 x D tile whose D columns are contiguous (MN-major; its
+// 64-column blocks lie kBlkW apart): the P V shape of the forward kernel.
 __device__ __forceinline__ void mma_pv(uint32_t tmem, uint32_t a, uint32_t b, uint32_t idesc, bool accumulate) {
-  const uint64_t da = ptx::make_smem_desc_sw128(a, 16, 1024), db = ptx::make_smem_desc_sw128(b, kBlk, 1024);
+  const uint64_t da = ptx::make_smem_desc_sw128(a, 16, 1024), db = ptx::make_smem_desc_sw128(b, kBlkW, 1024);
 #pragma unroll
-  for (int k = 0; k < kT / 16; ++k)
-    ptx::umma_f16(tmem, ptx::desc_advance(da, (k >> 2) * kBlk + (k & 3) * 32), ptx::desc_advance(db, k * 2048), idesc,
+  for (int k = 0; k < kW / 16; ++k)
+    ptx::umma_f16(tmem, ptx::desc_advance(da, k * 32), ptx::desc_advance(db, k * 2048), idesc,
                   (accumulate || k != 0) ? 1u : 0u);
 }
 
-// 16 columns (8 bf16 pairs) of one row, starting at column col (a multiple of 16): two 16-byte chunks of the row's
-// 128-byte line in k-block (col >> 6), swizzled.
+// 16 columns (8 bf16 pairs) of one row of a 128 x 64 matrix, starting at column col (a multiple of 16): two 16-byte chunks
+// of the row's 128-byte line, swizzled.
 __device__ __forceinline__ void store_cols16(uint8_t* mat, int row, int col, const uint32_t (&w)[8]) {
-  uint8_t* blk = mat + (col >> 6) * kBlk + row * 128;
-  const int chunk = (col & 63) >> 3;
-  *reinterpret_cast<uint4*>(blk + (((chunk) ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-  *reinterpret_cast<uint4*>(blk + (((chunk + 1) ^ (row & 7)) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
+  uint8_t* line = mat + row * 128;
+  const int chunk = col >> 3;
+  *reinterpret_cast<uint4*>(line + (((chunk) ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+  *reinterpret_cast<uint4*>(line + (((chunk + 1) ^ (row & 7)) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
+}
+// The 64 columns of a tile in four batches of 16: the tensor-memory loads of batch k + 1 are in flight while batch k is
+// computed (tcgen05.wait::ld waits for every load issued before it, so the wait for a batch comes after the arithmetic of
+// the previous one).
+template <class Batch>
+__device__ __forceinline__ void walk_columns(uint32_t t_s, uint32_t t_dp, Batch batch) {
+  uint32_t sa[16], pa[16], sb[16], pb[16];
+  ptx::tmem_ld_32x32b_x16(t_s, sa);
+  ptx::tmem_ld_32x32b_x16(t_dp, pa);
+  ptx::tmem_wait_ld();
+  ptx::tmem_ld_32x32b_x16(t_s + 16, sb);
+  ptx::tmem_ld_32x32b_x16(t_dp + 16, pb);
+  batch(0, sa, pa);
+  ptx::tmem_wait_ld();
+  ptx::tmem_ld_32x32b_x16(t_s + 32, sa);
+  ptx::tmem_ld_32x32b_x16(t_dp + 32, pa);
+  batch(16, sb, pb);
+  ptx::tmem_wait_ld();
+  ptx::tmem_ld_32x32b_x16(t_s + 48, sb);
+  ptx::tmem_ld_32x32b_x16(t_dp + 48, pb);
+  batch(32, sa, pa);
+  ptx::tmem_wait_ld();
+  batch(48, sb, pb);
 }
 
 // Chunks c_lo .. c_hi - 1 (32 columns each) of an accumulator row from tensor memory to bf16 in global memory.  The tensor-memory loads are
@@ -141,40 +176,42 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                    const BwdArgs p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  constexpr int kTile = BwdCfg<D>::kTile, kStages = BwdCfg<D>::kStages;
+  constexpr int kTile = BwdCfg<D>::kTile, kTileW = BwdCfg<D>::kTileW, kStages = BwdCfg<D>::kStages;
   uint8_t* sq = smem;
   uint8_t* sdo = sq + kTile;
-  uint8_t* sk = sdo + kTile;             // kStages stages
-  uint8_t* sv = sk + kStages * kTile;    // kStages stages
-  uint8_t* sds = sv + kStages * kTile;   // dS: 128 x 128 bf16
-  uint8_t* bar_base = sds + kPBytes;
-  uint64_t* q_full = reinterpret_cast<uint64_t*>(bar_base);
-  uint64_t* kv_full = q_full + 1;    // [2]
-  uint64_t* kv_empty = kv_full + 2;  // [2]
-  uint64_t* sp_full = kv_empty + 2;  // S and dP of a tile are complete
-  uint64_t* ds_full = sp_full + 1;   // dS written (and S, dP read) by the four softmax warps
-  uint64_t* ds_empty = ds_full + 1;  // the dQ MMAs have read dS
-  uint64_t* dq_full = ds_empty + 1;
+  uint8_t* sk = sdo + kTile;              // kStages tiles
+  uint8_t* sv = sk + kStages * kTileW;    // kStages tiles
+  uint8_t* sds = sv + kStages * kTileW;   // dS of the groups: 128 x 64 bf16 each
+  uint64_t* q_full = reinterpret_cast<uint64_t*>(sds + 2 * kBlk);
+  uint64_t* kv_full = q_full + 1;           // [kStages]
+  uint64_t* kv_empty = kv_full + kStages;   // [kStages]
+  uint64_t* sp_full = kv_empty + kStages;   // [2] S and dP of a group's tile are complete
+  uint64_t* ds_full = sp_full + 2;          // [2] dS written (and S, dP read) by the group's four warps
+  uint64_t* ds_empty = ds_full + 2;         // [2] the dQ MMAs have read dS
+  uint64_t* dq_full = ds_empty + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(dq_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
-  const int q0 = blockIdx.x * kT;
+  // under a causal mask the query tiles with the most keys first
+  const int q0 = static_cast<int>(p.causal ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * kT;
   const int h = blockIdx.y % p.H, b = blockIdx.y / p.H;
   const int off = p.Skv - p.Sq;
   const int kv_end = p.causal ? min(p.Skv, q0 + kT + off) : p.Skv;
-  const int n_tiles = (kv_end + kT - 1) / kT;
+  const int n_tiles = (kv_end + kW - 1) / kW;
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     ptx::mbar_init(q_full, 1);
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < kStages; ++s) {
       ptx::mbar_init(&kv_full[s], 1);
       ptx::mbar_init(&kv_empty[s], 1);
     }
-    ptx::mbar_init(sp_full, 1);
-    ptx::mbar_init(ds_full, kSoftmaxWarps);
-    ptx::mbar_init(ds_empty, 1);
+    for (int g = 0; g < 2; ++g) {
+      ptx::mbar_init(&sp_full[g], 1);
+      ptx::mbar_init(&ds_full[g], 4);
+      ptx::mbar_init(&ds_empty[g], 1);
+    }
     ptx::mbar_init(dq_full, 1);
     ptx::fence_mbar_init();
     ptx::prefetch_tensormap(&map_q);
@@ -190,87 +227,90 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t t_s = tmem_base, t_dp = tmem_base + 128, t_dq = tmem_base + 256;
+  const uint32_t t_dq = tmem_base + 256;
 
   if (warp == 0) {
     if (ptx::elect_one()) {
       ptx::mbar_arrive_expect_tx(q_full, 2 * kTile);
-      load_tile<D>(sq, &map_q, q_full, q0, h, b);
-      load_tile<D>(sdo, &map_do, q_full, q0, h, b);
-      for (int j = 0; j < n_tiles; ++j) {
+      load_tile<D>(sq, &map_q, q_full, q0, h, b, kBlk);
+      load_tile<D>(sdo, &map_do, q_full, q0, h, b, kBlk);
+      int j = 0;
+      for (; j < n_tiles; ++j) {
         const int st = j % kStages;
-        const uint32_t round = static_cast<uint32_t>(j / kStages) & 1u;
-        if (!ptx::mbar_wait(&kv_empty[st], round ^ 1u, abort_flag, p.timeout_ns)) {
+        if (!ptx::mbar_wait(&kv_empty[st], ((j / kStages) & 1) ^ 1, abort_flag, p.timeout_ns)) {
           report_status(p.status, kStatusGemmTimeout, 61, blockIdx.x, j);
           break;
         }
-        ptx::mbar_arrive_expect_tx(&kv_full[st], 2 * kTile);
-        load_tile<D>(sk + st * kTile, &map_k, &kv_full[st], j * kT, h, b);
-        load_tile<D>(sv + st * kTile, &map_v, &kv_full[st], j * kT, h, b);
+        ptx::mbar_arrive_expect_tx(&kv_full[st], 2 * kTileW);
+        load_tile<D>(sk + st * kTileW, &map_k, &kv_full[st], j * kW, h, b, kBlkW);
+        load_tile<D>(sv + st * kTileW, &map_v, &kv_full[st], j * kW, h, b, kBlkW);
       }
+      if (j < n_tiles || *abort_flag) drain(q_full, kv_full, j, kStages, p.timeout_ns);
     }
   } else if (warp == 1) {
     if (ptx::elect_one()) {
-      const uint32_t idesc_s = ptx::make_idesc(1u, kT, kT, 0, 0);
+      const uint32_t idesc_s = ptx::make_idesc(1u, kT, kW, 0, 0);
       const uint32_t idesc_o = ptx::make_idesc(1u, kT, D, 0, 1);
       const uint32_t sq_a = ptx::smem_u32(sq), sdo_a = ptx::smem_u32(sdo), sds_a = ptx::smem_u32(sds);
-      bool ok = ptx::mbar_wait(q_full, 0, abort_flag, p.timeout_ns);
-      if (!ok) report_status(p.status, kStatusGemmTimeout, 62, blockIdx.x, 0);
-      for (int j = 0; ok && j < n_tiles; ++j) {
-        const int st = j % kStages;
-        const uint32_t sk_a = ptx::smem_u32(sk + st * kTile), sv_a = ptx::smem_u32(sv + st * kTile);
-        if (!ptx::mbar_wait(&kv_full[st], static_cast<uint32_t>(j / kStages) & 1u, abort_flag, p.timeout_ns)) {
+      const uint32_t sk_a = ptx::smem_u32(sk), sv_a = ptx::smem_u32(sv);
+      auto issue_s = [&](int j) {  // S and dP of tile j
+        const int st = j % kStages, g = j & 1;
+        if (!ptx::mbar_wait(&kv_full[st], (j / kStages) & 1, abort_flag, p.timeout_ns)) {
           report_status(p.status, kStatusGemmTimeout, 63, blockIdx.x, j);
-          break;
+          return false;
         }
         ptx::tc_fence_after();
-        // (S and dP of the previous tile were read before its ds_full, which the previous iteration waited for)
-        mma_scores<D>(t_s, sq_a, sk_a, idesc_s);
-        mma_scores<D>(t_dp, sdo_a, sv_a, idesc_s);
-        ptx::umma_commit(sp_full);
-        if (!ptx::mbar_wait(ds_full, j & 1, abort_flag, p.timeout_ns)) {
+        mma_scores<D>(tmem_base + g * 2 * kW, sq_a, sk_a + st * kTileW, idesc_s);
+        mma_scores<D>(tmem_base + g * 2 * kW + kW, sdo_a, sv_a + st * kTileW, idesc_s);
+        ptx::umma_commit(&sp_full[g]);
+        return true;
+      };
+      bool ok = ptx::mbar_wait(q_full, 0, abort_flag, p.timeout_ns);
+      if (!ok) report_status(p.status, kStatusGemmTimeout, 62, blockIdx.x, 0);
+      for (int j = 0; ok && j < 2 && j < n_tiles; ++j) ok = issue_s(j);
+      for (int j = 0; ok && j < n_tiles; ++j) {
+        const int st = j % kStages, g = j & 1;
+        // dS of tile j is written, its S and dP have been read
+        if (!ptx::mbar_wait(&ds_full[g], (j >> 1) & 1, abort_flag, p.timeout_ns)) {
           report_status(p.status, kStatusGemmTimeout, 64, blockIdx.x, j);
           break;
         }
         ptx::tc_fence_after();
-        mma_pv(t_dq, sds_a, sk_a, idesc_o, j != 0);
+        if (j + 2 < n_tiles) {
+          ok = issue_s(j + 2);
+          if (!ok) break;
+        }
+        mma_pv(t_dq, sds_a + g * kBlk, sk_a + st * kTileW, idesc_o, j != 0);
         ptx::umma_commit(&kv_empty[st]);
-        ptx::umma_commit(ds_empty);
+        ptx::umma_commit(&ds_empty[g]);
         if (j + 1 == n_tiles) ptx::umma_commit(dq_full);
       }
     }
   } else {
-    const int quarter = warp & 3;
-    const int half = (warp - 2) >> 2;      // which 64 columns of a tile this warp handles
+    const int quarter = warp & 3, g = (warp - 2) >> 2;
     const int row = quarter * 32 + lane;
     const int qrow = q0 + row;
     const uint32_t t_row = (static_cast<uint32_t>(quarter * 32) << 16);
+    const uint32_t t_s = tmem_base + t_row + g * 2 * kW;
+    uint8_t* my_ds = sds + g * kBlk;
     const long long stat = (static_cast<long long>(b) * p.H + h) * p.Sq + qrow;
     // a row past the end contributes nothing: +inf makes every probability zero
     const float lse2 = qrow < p.Sq ? p.lse[stat] * kLog2e : INFINITY;
     const float delta = qrow < p.Sq ? p.delta[stat] : 0.f;
     bool ok = true;
-    for (int j = 0; j < n_tiles; ++j) {
-      const bool ready = ptx::mbar_wait(sp_full, j & 1, abort_flag, p.timeout_ns);
+    for (int j = g; j < n_tiles; j += 2) {
+      const int turn = j >> 1;
+      // S and dP are there; the dQ MMAs of the group's tile before have read dS
+      bool ready = ptx::mbar_wait(&sp_full[g], turn & 1, abort_flag, p.timeout_ns);
+      if (ready && turn > 0) ready = ptx::mbar_wait(&ds_empty[g], (turn - 1) & 1, abort_flag, p.timeout_ns);
       if (!__all_sync(0xffffffffu, ready)) {
         if (lane == 0) report_status(p.status, kStatusGemmTimeout, 65, blockIdx.x, j);
         ok = false;
         break;
       }
       ptx::tc_fence_after();
-      if (j > 0) {  // the dQ MMAs of the previous tile have read dS
-        const bool freed = ptx::mbar_wait(ds_empty, (j - 1) & 1, abort_flag, p.timeout_ns);
-        if (!__all_sync(0xffffffffu, freed)) {
-          if (lane == 0) report_status(p.status, kStatusGemmTimeout, 66, blockIdx.x, j);
-          ok = false;
-          break;
-        }
-      }
-      int valid = min(kT, p.Skv - j * kT);
-      if (p.causal) valid = max(0, min(valid, qrow + off + 1 - j * kT));
-      // The warp's 64 columns in four batches of 16: the tensor-memory loads of batch k + 1 are in flight while
-      // batch k is computed (tcgen05.wait::ld waits for every load issued before it, so the wait for a batch comes
-      // after the arithmetic of the previous one).
+      int valid = min(kW, p.Skv - j * kW);
+      if (p.causal) valid = max(0, min(valid, qrow + off + 1 - j * kW));
       {
         const float2 sl2 = make_float2(p.scale_log2, p.scale_log2), nl2 = make_float2(-lse2, -lse2);
         const float2 sc2 = make_float2(p.scale, p.scale), nd2 = make_float2(-delta * p.scale, -delta * p.scale);
@@ -299,45 +339,23 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
               w[i >> 1] = *reinterpret_cast<const uint32_t*>(&pk);
             }
           }
-          store_cols16(sds, row, col, w);
+          store_cols16(my_ds, row, col, w);
         };
-        const int c0 = half * 64;
-        uint32_t sa[16], pa[16], sb[16], pb[16];
-        ptx::tmem_ld_32x32b_x16(t_s + t_row + c0, sa);
-        ptx::tmem_ld_32x32b_x16(t_dp + t_row + c0, pa);
-        ptx::tmem_wait_ld();
-        ptx::tmem_ld_32x32b_x16(t_s + t_row + c0 + 16, sb);
-        ptx::tmem_ld_32x32b_x16(t_dp + t_row + c0 + 16, pb);
-        batch(c0, sa, pa);
-        ptx::tmem_wait_ld();
-        ptx::tmem_ld_32x32b_x16(t_s + t_row + c0 + 32, sa);
-        ptx::tmem_ld_32x32b_x16(t_dp + t_row + c0 + 32, pa);
-        batch(c0 + 16, sb, pb);
-        ptx::tmem_wait_ld();
-        ptx::tmem_ld_32x32b_x16(t_s + t_row + c0 + 48, sb);
-        ptx::tmem_ld_32x32b_x16(t_dp + t_row + c0 + 48, pb);
-        batch(c0 + 32, sa, pa);
-        ptx::tmem_wait_ld();
-        batch(c0 + 48, sb, pb);
+        walk_columns(t_s, t_s + kW, batch);
       }
       ptx::tc_fence_before();
       ptx::fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(ds_full);
+      if (lane == 0) ptx::mbar_arrive(&ds_full[g]);
     }
     if (ok) {
-      const bool done = n_tiles > 0 ? ptx::mbar_wait(dq_full, 0, abort_flag, p.timeout_ns) : true;
+      const bool done = ptx::mbar_wait(dq_full, 0, abort_flag, p.timeout_ns);
       if (!__all_sync(0xffffffffu, done)) {
         if (lane == 0) report_status(p.status, kStatusGemmTimeout, 67, blockIdx.x, 0);
       } else {
         ptx::tc_fence_after();
         __nv_bfloat16* dst = p.dq + ((static_cast<long long>(b) * p.Sq + qrow) * p.H + h) * D;
-        if (n_tiles > 0) {  // uniform over the CTA; each warp of a quarter stores half of the D columns
-          store_row_bf16(dst, t_dq + t_row, qrow < p.Sq, half * (D / 64), (half + 1) * (D / 64));
-        } else if (qrow < p.Sq && half == 0) {
-#pragma unroll
-          for (int q = 0; q < D / 8; ++q) reinterpret_cast<uint4*>(dst)[q] = make_uint4(0u, 0u, 0u, 0u);
-        }
+        store_row_bf16(dst, t_dq + t_row, qrow < p.Sq, g * (D / 64), (g + 1) * (D / 64));  // a group each half of the columns
       }
     }
   }
@@ -357,22 +375,21 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     const BwdArgs p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  constexpr int kTile = BwdCfg<D>::kTile, kStages = BwdCfg<D>::kStages;
+  constexpr int kTile = BwdCfg<D>::kTile, kTileW = BwdCfg<D>::kTileW, kStages = BwdCfg<D>::kStages;
   uint8_t* sk = smem;
   uint8_t* sv = sk + kTile;
-  uint8_t* sq = sv + kTile;              // kStages stages
-  uint8_t* sdo = sq + kStages * kTile;   // kStages stages
-  uint8_t* spt = sdo + kStages * kTile;  // P^T: 128 keys x 128 queries bf16
-  uint8_t* sdst = spt + kPBytes;   // dS^T
-  float* s_stat = reinterpret_cast<float*>(sdst + kPBytes);  // per softmax warp: [lse2 | delta][128]
-  uint8_t* bar_base = reinterpret_cast<uint8_t*>(s_stat) + 8192;
-  uint64_t* kv_full = reinterpret_cast<uint64_t*>(bar_base);
-  uint64_t* qd_full = kv_full + 1;    // [2]
-  uint64_t* qd_empty = qd_full + 2;   // [2]
-  uint64_t* sp_full = qd_empty + 2;
-  uint64_t* pt_full = sp_full + 1;
-  uint64_t* pt_empty = pt_full + 1;
-  uint64_t* acc_full = pt_empty + 1;
+  uint8_t* sq = sv + kTile;               // kStages tiles
+  uint8_t* sdo = sq + kStages * kTileW;   // kStages tiles
+  uint8_t* spt = sdo + kStages * kTileW;  // P^T of the groups: 128 keys x 64 queries bf16 each
+  uint8_t* sdst = spt + 2 * kBlk;         // dS^T
+  float* s_stat = reinterpret_cast<float*>(sdst + 2 * kBlk);  // per group: lse and delta of its tile's 64 queries
+  uint64_t* kv_full = reinterpret_cast<uint64_t*>(s_stat + 4 * kW);
+  uint64_t* qd_full = kv_full + 1;          // [kStages]
+  uint64_t* qd_empty = qd_full + kStages;   // [kStages]
+  uint64_t* sp_full = qd_empty + kStages;   // [2] S^T and dP^T of a group's tile are complete
+  uint64_t* pt_full = sp_full + 2;          // [2] P^T and dS^T written by the group's four warps
+  uint64_t* pt_empty = pt_full + 2;         // [2] the MMAs have read them
+  uint64_t* acc_full = pt_empty + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -380,21 +397,23 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   const int k0 = blockIdx.x * kT;
   const int h = blockIdx.y % p.H, b = blockIdx.y / p.H;
   const int off = p.Skv - p.Sq;
-  const int n_qtiles = (p.Sq + kT - 1) / kT;
+  const int n_qtiles = (p.Sq + kW - 1) / kW;
   // causal: query q sees key k when k <= q + off, so the first query that sees this tile's first key is k0 - off
-  const int i_begin = p.causal ? max(0, k0 - off) / kT : 0;
+  const int i_begin = p.causal ? max(0, k0 - off) / kW : 0;
   const int n_iter = max(0, n_qtiles - i_begin);
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     ptx::mbar_init(kv_full, 1);
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < kStages; ++s) {
       ptx::mbar_init(&qd_full[s], 1);
       ptx::mbar_init(&qd_empty[s], 1);
     }
-    ptx::mbar_init(sp_full, 1);
-    ptx::mbar_init(pt_full, kSoftmaxWarps);
-    ptx::mbar_init(pt_empty, 1);
+    for (int g = 0; g < 2; ++g) {
+      ptx::mbar_init(&sp_full[g], 1);
+      ptx::mbar_init(&pt_full[g], 4);
+      ptx::mbar_init(&pt_empty[g], 1);
+    }
     ptx::mbar_init(acc_full, 1);
     ptx::fence_mbar_init();
     ptx::prefetch_tensormap(&map_q);
@@ -410,96 +429,103 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t t_s = tmem_base, t_dp = tmem_base + 128, t_dv = tmem_base + 256, t_dk = tmem_base + 256 + D;
+  const uint32_t t_dv = tmem_base + 256, t_dk = tmem_base + 256 + D;
 
   if (warp == 0) {
     if (n_iter > 0 && ptx::elect_one()) {
       ptx::mbar_arrive_expect_tx(kv_full, 2 * kTile);
-      load_tile<D>(sk, &map_k, kv_full, k0, h, b);
-      load_tile<D>(sv, &map_v, kv_full, k0, h, b);
-      for (int it = 0; it < n_iter; ++it) {
+      load_tile<D>(sk, &map_k, kv_full, k0, h, b, kBlk);
+      load_tile<D>(sv, &map_v, kv_full, k0, h, b, kBlk);
+      int it = 0;
+      for (; it < n_iter; ++it) {
         const int st = it % kStages, i = i_begin + it;
-        const uint32_t round = static_cast<uint32_t>(it / kStages) & 1u;
-        if (!ptx::mbar_wait(&qd_empty[st], round ^ 1u, abort_flag, p.timeout_ns)) {
+        if (!ptx::mbar_wait(&qd_empty[st], ((it / kStages) & 1) ^ 1, abort_flag, p.timeout_ns)) {
           report_status(p.status, kStatusGemmTimeout, 71, blockIdx.x, it);
           break;
         }
-        ptx::mbar_arrive_expect_tx(&qd_full[st], 2 * kTile);
-        load_tile<D>(sq + st * kTile, &map_q, &qd_full[st], i * kT, h, b);
-        load_tile<D>(sdo + st * kTile, &map_do, &qd_full[st], i * kT, h, b);
+        ptx::mbar_arrive_expect_tx(&qd_full[st], 2 * kTileW);
+        load_tile<D>(sq + st * kTileW, &map_q, &qd_full[st], i * kW, h, b, kBlkW);
+        load_tile<D>(sdo + st * kTileW, &map_do, &qd_full[st], i * kW, h, b, kBlkW);
       }
+      if (it < n_iter || *abort_flag) drain(kv_full, qd_full, it, kStages, p.timeout_ns);
     }
   } else if (warp == 1) {
     if (n_iter > 0 && ptx::elect_one()) {
-      const uint32_t idesc_s = ptx::make_idesc(1u, kT, kT, 0, 0);
+      const uint32_t idesc_s = ptx::make_idesc(1u, kT, kW, 0, 0);
       const uint32_t idesc_o = ptx::make_idesc(1u, kT, D, 0, 1);
-      const uint32_t sk_a = ptx::smem_u32(sk), sv_a = ptx::smem_u32(sv);
+      const uint32_t sk_a = ptx::smem_u32(sk), sv_a = ptx::smem_u32(sv), sq_a = ptx::smem_u32(sq), sdo_a = ptx::smem_u32(sdo);
       const uint32_t spt_a = ptx::smem_u32(spt), sdst_a = ptx::smem_u32(sdst);
-      bool ok = ptx::mbar_wait(kv_full, 0, abort_flag, p.timeout_ns);
-      if (!ok) report_status(p.status, kStatusGemmTimeout, 72, blockIdx.x, 0);
-      for (int it = 0; ok && it < n_iter; ++it) {
-        const int st = it % kStages;
-        const uint32_t sq_a = ptx::smem_u32(sq + st * kTile), sdo_a = ptx::smem_u32(sdo + st * kTile);
-        if (!ptx::mbar_wait(&qd_full[st], static_cast<uint32_t>(it / kStages) & 1u, abort_flag, p.timeout_ns)) {
+      auto issue_s = [&](int it) {
+        const int st = it % kStages, g = it & 1;
+        if (!ptx::mbar_wait(&qd_full[st], (it / kStages) & 1, abort_flag, p.timeout_ns)) {
           report_status(p.status, kStatusGemmTimeout, 73, blockIdx.x, it);
-          break;
+          return false;
         }
         ptx::tc_fence_after();
-        mma_scores<D>(t_s, sk_a, sq_a, idesc_s);     // S^T  = K Q_i^T
-        mma_scores<D>(t_dp, sv_a, sdo_a, idesc_s);   // dP^T = V dO_i^T
-        ptx::umma_commit(sp_full);
-        if (!ptx::mbar_wait(pt_full, it & 1, abort_flag, p.timeout_ns)) {
+        mma_scores<D>(tmem_base + g * 2 * kW, sk_a, sq_a + st * kTileW, idesc_s);        // S^T  = K Q_i^T
+        mma_scores<D>(tmem_base + g * 2 * kW + kW, sv_a, sdo_a + st * kTileW, idesc_s);  // dP^T = V dO_i^T
+        ptx::umma_commit(&sp_full[g]);
+        return true;
+      };
+      bool ok = ptx::mbar_wait(kv_full, 0, abort_flag, p.timeout_ns);
+      if (!ok) report_status(p.status, kStatusGemmTimeout, 72, blockIdx.x, 0);
+      for (int it = 0; ok && it < 2 && it < n_iter; ++it) ok = issue_s(it);
+      for (int it = 0; ok && it < n_iter; ++it) {
+        const int st = it % kStages, g = it & 1;
+        if (!ptx::mbar_wait(&pt_full[g], (it >> 1) & 1, abort_flag, p.timeout_ns)) {
           report_status(p.status, kStatusGemmTimeout, 74, blockIdx.x, it);
           break;
         }
         ptx::tc_fence_after();
-        mma_pv(t_dv, spt_a, sdo_a, idesc_o, it != 0);   // dV += P^T dO_i
-        mma_pv(t_dk, sdst_a, sq_a, idesc_o, it != 0);   // dK += dS^T Q_i
+        if (it + 2 < n_iter) {
+          ok = issue_s(it + 2);
+          if (!ok) break;
+        }
+        mma_pv(t_dv, spt_a + g * kBlk, sdo_a + st * kTileW, idesc_o, it != 0);   // dV += P^T dO_i
+        mma_pv(t_dk, sdst_a + g * kBlk, sq_a + st * kTileW, idesc_o, it != 0);   // dK += dS^T Q_i
         ptx::umma_commit(&qd_empty[st]);
-        ptx::umma_commit(pt_empty);
+        ptx::umma_commit(&pt_empty[g]);
         if (it + 1 == n_iter) ptx::umma_commit(acc_full);
       }
     }
   } else {
-    const int quarter = warp & 3;
-    const int half = (warp - 2) >> 2;      // which 64 query columns of a tile this warp handles
+    const int quarter = warp & 3, g = (warp - 2) >> 2;
     const int row = quarter * 32 + lane;   // key row of this thread
     const int krow = k0 + row;
     const uint32_t t_row = (static_cast<uint32_t>(quarter * 32) << 16);
+    const uint32_t t_s = tmem_base + t_row + g * 2 * kW;
+    uint8_t *my_pt = spt + g * kBlk, *my_dst = sdst + g * kBlk;
+    float* slot = s_stat + g * 2 * kW;
     const long long stat_base = (static_cast<long long>(b) * p.H + h) * p.Sq;
     bool ok = true;
-    for (int it = 0; it < n_iter; ++it) {
-      const int i = i_begin + it;
-      // Every warp keeps its own copy of the tile's 128 (lse, delta) pairs, so that no barrier between warps is
-      // needed (a warp that gave up on a wait must not leave the others stuck at one).
-      float* slot = s_stat + (warp - 2) * 256;
-      __syncwarp();  // the previous iteration's reads are done
+    for (int it = g; it < n_iter; it += 2) {
+      const int i = i_begin + it, turn = it >> 1;
+      float nl[2], nd[2];
 #pragma unroll
-      for (int x = 2 * half; x < 2 * half + 2; ++x) {  // only the columns this warp handles
-        const int ql = x * 32 + lane, q = i * kT + ql;
+      for (int x = 0; x < 2; ++x) {
+        const int q = i * kW + x * 32 + lane;
         // negated, so that one fused multiply-add forms the exponent; -inf: a query past the end sees nothing
-        slot[ql] = q < p.Sq ? -p.lse[stat_base + q] * kLog2e : -INFINITY;
-        slot[128 + ql] = q < p.Sq ? -p.delta[stat_base + q] * p.scale : 0.f;
+        nl[x] = q < p.Sq ? -p.lse[stat_base + q] * kLog2e : -INFINITY;
+        nd[x] = q < p.Sq ? -p.delta[stat_base + q] * p.scale : 0.f;
       }
-      __syncwarp();
-      const bool ready = ptx::mbar_wait(sp_full, it & 1, abort_flag, p.timeout_ns);
+      bool ready = ptx::mbar_wait(&sp_full[g], turn & 1, abort_flag, p.timeout_ns);
+      if (ready && turn > 0) ready = ptx::mbar_wait(&pt_empty[g], (turn - 1) & 1, abort_flag, p.timeout_ns);
       if (!__all_sync(0xffffffffu, ready)) {
         if (lane == 0) report_status(p.status, kStatusGemmTimeout, 75, blockIdx.x, it);
         ok = false;
         break;
       }
       ptx::tc_fence_after();
-      if (it > 0) {
-        const bool freed = ptx::mbar_wait(pt_empty, (it - 1) & 1, abort_flag, p.timeout_ns);
-        if (!__all_sync(0xffffffffu, freed)) {
-          if (lane == 0) report_status(p.status, kStatusGemmTimeout, 76, blockIdx.x, it);
-          ok = false;
-          break;
-        }
+      // All four warps write the same values.  The scores of this tile were issued after every one of them was done with
+      // the tile before, so nobody reads the slot any more.
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        slot[x * 32 + lane] = nl[x];
+        slot[kW + x * 32 + lane] = nd[x];
       }
+      __syncwarp();
       // queries of this tile that may see this key: all of them, or (causal) those with q + off >= key
-      const int q_first = p.causal ? max(0, krow - off - i * kT) : 0;  // first local query column that sees the key
-      // Four batches of 16 query columns, tensor-memory loads of the next batch in flight during the arithmetic.
+      const int q_first = p.causal ? max(0, krow - off - i * kW) : 0;  // first local query column that sees the key
       // Keys past the end need no mask (their rows of dK / dV are never stored and no other row depends on them);
       // only the causal diagonal does.
       {
@@ -510,7 +536,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 #pragma unroll
             for (int x = 0; x < 16; x += 4) {
               const float4 nl = *reinterpret_cast<const float4*>(slot + col + x);
-              const float4 nd = *reinterpret_cast<const float4*>(slot + 128 + col + x);
+              const float4 nd = *reinterpret_cast<const float4*>(slot + kW + col + x);
               const float2 e0 = __ffma2_rn(make_float2(__uint_as_float(rs[x]), __uint_as_float(rs[x + 1])), sl2,
                                            make_float2(nl.x, nl.y));
               const float2 e1 = __ffma2_rn(make_float2(__uint_as_float(rs[x + 2]), __uint_as_float(rs[x + 3])), sl2,
@@ -535,45 +561,28 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
               const int qa = col + x;
               if (qa >= q_first) {
                 p0 = ex2f(fmaf(__uint_as_float(rs[x]), p.scale_log2, slot[qa]));
-                d0 = p0 * fmaf(__uint_as_float(rp[x]), p.scale, slot[128 + qa]);
+                d0 = p0 * fmaf(__uint_as_float(rp[x]), p.scale, slot[kW + qa]);
               }
               if (qa + 1 >= q_first) {
                 p1 = ex2f(fmaf(__uint_as_float(rs[x + 1]), p.scale_log2, slot[qa + 1]));
-                d1 = p1 * fmaf(__uint_as_float(rp[x + 1]), p.scale, slot[128 + qa + 1]);
+                d1 = p1 * fmaf(__uint_as_float(rp[x + 1]), p.scale, slot[kW + qa + 1]);
               }
               const __nv_bfloat162 a = __floats2bfloat162_rn(p0, p1), d = __floats2bfloat162_rn(d0, d1);
               wp[x >> 1] = *reinterpret_cast<const uint32_t*>(&a);
               wd[x >> 1] = *reinterpret_cast<const uint32_t*>(&d);
             }
           }
-          store_cols16(spt, row, col, wp);
-          store_cols16(sdst, row, col, wd);
+          store_cols16(my_pt, row, col, wp);
+          store_cols16(my_dst, row, col, wd);
         };
-        const int c0 = half * 64;
-        uint32_t sa[16], pa[16], sb[16], pb[16];
-        ptx::tmem_ld_32x32b_x16(t_s + t_row + c0, sa);
-        ptx::tmem_ld_32x32b_x16(t_dp + t_row + c0, pa);
-        ptx::tmem_wait_ld();
-        ptx::tmem_ld_32x32b_x16(t_s + t_row + c0 + 16, sb);
-        ptx::tmem_ld_32x32b_x16(t_dp + t_row + c0 + 16, pb);
-        batch(c0, sa, pa);
-        ptx::tmem_wait_ld();
-        ptx::tmem_ld_32x32b_x16(t_s + t_row + c0 + 32, sa);
-        ptx::tmem_ld_32x32b_x16(t_dp + t_row + c0 + 32, pa);
-        batch(c0 + 16, sb, pb);
-        ptx::tmem_wait_ld();
-        ptx::tmem_ld_32x32b_x16(t_s + t_row + c0 + 48, sb);
-        ptx::tmem_ld_32x32b_x16(t_dp + t_row + c0 + 48, pb);
-        batch(c0 + 32, sa, pa);
-        ptx::tmem_wait_ld();
-        batch(c0 + 48, sb, pb);
+        walk_columns(t_s, t_s + kW, batch);
       }
       ptx::tc_fence_before();
       ptx::fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(pt_full);
+      if (lane == 0) ptx::mbar_arrive(&pt_full[g]);
     }
-    if (n_iter == 0 && krow < p.Skv && half == 0) {  // no query sees these keys
+    if (n_iter == 0 && krow < p.Skv && g == 0) {  // no query sees these keys
       __nv_bfloat16* dv = p.dv + ((static_cast<long long>(b) * p.Skv + krow) * p.H + h) * D;
       __nv_bfloat16* dk = p.dk + ((static_cast<long long>(b) * p.Skv + krow) * p.H + h) * D;
 #pragma unroll
@@ -588,8 +597,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         if (lane == 0) report_status(p.status, kStatusGemmTimeout, 77, blockIdx.x, 0);
       } else {
         ptx::tc_fence_after();
-        // the two warps of a lane quarter share the work: one stores the dV rows, the other the dK rows
-        if (half == 0)
+        // one group stores the dV rows, the other the dK rows
+        if (g == 0)
           store_row_bf16(p.dv + ((static_cast<long long>(b) * p.Skv + krow) * p.H + h) * D, t_dv + t_row,
                          krow < p.Skv, 0, D / 32);
         else
@@ -606,24 +615,28 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   }
 }
 
-// delta[b, h, s] = sum_d dO[b, s, h, d] * O[b, s, h, d]  (both [B, S, H, D] contiguous bf16); warp per row.
+// delta[b, h, s] = sum_d dO[b, s, h, d] * O[b, s, h, d]  (both [B, S, H, D] contiguous bf16); D / 8 lanes per row, 16 bytes
+// of either operand each.  Bound by HBM (8 x 16 heads of 64, 1024 rows: a warp per row took 20.8 us).
 template <int D>
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                                  float* __restrict__ delta, int B, int H, int S) {
-  const long long row = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;  // over B * S * H
-  const int lane = threadIdx.x & 31;
-  const long long rows = static_cast<long long>(B) * S * H;
-  if (row >= rows) return;
+__global__ void __launch_bounds__(256)
+attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, float* __restrict__ delta,
+                  int B, int H, int S) {
+  constexpr int kLanes = D / 8;
+  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x, row = i / kLanes;  // over B * S * H
+  const bool in = row < static_cast<long long>(B) * S * H;
   float acc = 0.f;
+  if (in) {
+    const uint4 a = __ldg(reinterpret_cast<const uint4*>(o) + i), g = __ldg(reinterpret_cast<const uint4*>(d_o) + i);
+    const __nv_bfloat162 *av = reinterpret_cast<const __nv_bfloat162*>(&a), *gv = reinterpret_cast<const __nv_bfloat162*>(&g);
 #pragma unroll
-  for (int i = 0; i < D / 64; ++i) {
-    const __nv_bfloat162 a = reinterpret_cast<const __nv_bfloat162*>(o + row * D)[lane + 32 * i];
-    const __nv_bfloat162 g = reinterpret_cast<const __nv_bfloat162*>(d_o + row * D)[lane + 32 * i];
-    acc += __bfloat162float(a.x) * __bfloat162float(g.x) + __bfloat162float(a.y) * __bfloat162float(g.y);
+    for (int k = 0; k < 4; ++k) {
+      const float2 x = __bfloat1622float2(av[k]), y = __bfloat1622float2(gv[k]);
+      acc += x.x * y.x + x.y * y.y;
+    }
   }
 #pragma unroll
-  for (int s = 16; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-  if (lane == 0) {
+  for (int s = kLanes / 2; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+  if (in && threadIdx.x % kLanes == 0) {
     const int hh = static_cast<int>(row % H);
     const long long bs = row / H;
     const int ss = static_cast<int>(bs % S);
@@ -657,11 +670,11 @@ EncodeTiledFnB encode_fn_b() {
   return fn;
 }
 
-// [B, H, S, D] bf16 view with element strides (sb, sh, ss): 4-D map, 64 x 128 x 1 x 1 box, rows past S read zeros.
+// [B, H, S, D] bf16 view with element strides (sb, sh, ss): 4-D map, 64 x `rows` x 1 x 1 box, rows past S read zeros.
 int g_map_error = 0;  // why the last map_bhsd failed: -1 no driver entry point, -2 / -3 alignment, > 0 the driver's code
 
-bool map_bhsd(CUtensorMap* map, const void* ptr, int B, int H, int S, int kD, long long sb, long long sh,
-              long long ss) {
+bool map_bhsd(CUtensorMap* map, const void* ptr, int B, int H, int S, int kD, long long sb, long long sh, long long ss,
+              int rows) {
   EncodeTiledFnB enc = encode_fn_b();
   g_map_error = -1;
   if (enc == nullptr) return false;
@@ -675,7 +688,7 @@ bool map_bhsd(CUtensorMap* map, const void* ptr, int B, int H, int S, int kD, lo
                         static_cast<cuuint64_t>(B)};
   cuuint64_t strides[3] = {static_cast<cuuint64_t>(ss) * 2, static_cast<cuuint64_t>(sh_ok) * 2,
                            static_cast<cuuint64_t>(sb_ok) * 2};
-  cuuint32_t box[4] = {64, 128, 1, 1};
+  cuuint32_t box[4] = {64, static_cast<cuuint32_t>(rows), 1, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   g_map_error = static_cast<int>(enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(ptr), dims, strides,
                                        box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -692,8 +705,7 @@ extern "C" int fb_attention_bwd_map_error() { return fb::g_map_error; }
 namespace fb {
 namespace {
 template <int D>
-int launch_bwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo,
-               const void* out, const void* d_out, const BwdArgs& a, cudaStream_t stream) {
+int launch_bwd(const CUtensorMap (&fixed)[4], const CUtensorMap (&walked)[4], const void* out, const void* d_out, const BwdArgs& a, cudaStream_t stream) {
   static bool attr_set = false;
   if (!attr_set) {
     if (cudaFuncSetAttribute(attn_bwd_dq_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -704,13 +716,13 @@ int launch_bwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& 
     attr_set = true;
   }
   const long long rows = static_cast<long long>(a.B) * a.Sq * a.H;
-  attn_delta_kernel<D><<<static_cast<unsigned>((rows * 32 + 255) / 256), 256, 0, stream>>>(
+  attn_delta_kernel<D><<<static_cast<unsigned>((rows * (D / 8) + 255) / 256), 256, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out),
       const_cast<float*>(a.delta), a.B, a.H, a.Sq);
   attn_bwd_dq_kernel<D><<<dim3((a.Sq + kT - 1) / kT, a.B * a.H), kBwdThreads, BwdCfg<D>::kSmemDq, stream>>>(
-      mq, mk, mv, mdo, a);
+      fixed[0], walked[1], walked[2], fixed[3], a);
   attn_bwd_dkv_kernel<D><<<dim3((a.Skv + kT - 1) / kT, a.B * a.H), kBwdThreads, BwdCfg<D>::kSmemDkv, stream>>>(
-      mq, mk, mv, mdo, a);
+      walked[0], fixed[1], fixed[2], walked[3], a);
   return static_cast<int>(cudaGetLastError());
 }
 }  // namespace
@@ -732,12 +744,15 @@ extern "C" int fb_attention_bwd(const void* q, const void* k, const void* v, con
   if ((reinterpret_cast<uintptr_t>(dq) | reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv) |
        reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(d_out)) & 15)
     return -1;
-  CUtensorMap mq, mk, mv, mdo;
+  // q, k, v, d_out as the stationary side of a kernel (tiles of 128 rows) and as the side that is walked (64)
+  CUtensorMap fixed[4], walked[4];
   const long long o_sb = static_cast<long long>(Sq) * H * D, o_sh = D, o_ss = static_cast<long long>(H) * D;
-  if (!map_bhsd(&mq, q, B, H, Sq, D, q_sb, q_sh, q_ss)) return -2;
-  if (!map_bhsd(&mk, k, B, H, Skv, D, k_sb, k_sh, k_ss)) return -3;
-  if (!map_bhsd(&mv, v, B, H, Skv, D, v_sb, v_sh, v_ss)) return -4;
-  if (!map_bhsd(&mdo, d_out, B, H, Sq, D, o_sb, o_sh, o_ss)) return -5;
+  for (auto [maps, rows] : {std::make_pair(fixed, kT), std::make_pair(walked, kW)}) {
+    if (!map_bhsd(&maps[0], q, B, H, Sq, D, q_sb, q_sh, q_ss, rows)) return -2;
+    if (!map_bhsd(&maps[1], k, B, H, Skv, D, k_sb, k_sh, k_ss, rows)) return -3;
+    if (!map_bhsd(&maps[2], v, B, H, Skv, D, v_sb, v_sh, v_ss, rows)) return -4;
+    if (!map_bhsd(&maps[3], d_out, B, H, Sq, D, o_sb, o_sh, o_ss, rows)) return -5;
+  }
   BwdArgs a;
   a.dq = static_cast<__nv_bfloat16*>(dq);
   a.dk = static_cast<__nv_bfloat16*>(dk);
@@ -753,6 +768,6 @@ extern "C" int fb_attention_bwd(const void* q, const void* k, const void* v, con
   a.causal = causal ? 1 : 0;
   a.status = status;
   a.timeout_ns = 2000000000ull;
-  return D == 64 ? launch_bwd<64>(mq, mk, mv, mdo, out, d_out, a, stream)
-                 : launch_bwd<128>(mq, mk, mv, mdo, out, d_out, a, stream);
+  return D == 64 ? launch_bwd<64>(fixed, walked, out, d_out, a, stream)
+                 : launch_bwd<128>(fixed, walked, out, d_out, a, stream);
 }
