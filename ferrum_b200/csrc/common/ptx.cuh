@@ -75,16 +75,23 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // Bounded wait on an mbarrier phase.  `abort_flag` lives in shared memory and
 // is shared by all roles of the CTA: once any wait gives up, every other wait
 // in the CTA returns false at its next poll, so the CTA drains quickly.
+// The clock is first read after 64 polls: a read of %globaltimer takes some 450
+// cycles, and a wait that starts with one makes that the shortest time in which
+// a k-block can pass through a pipeline (495 cycles for two loads and four
+// products of 128 x 16 x 16, whatever the number of stages).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           uint64_t timeout_ns) {
   if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = globaltimer();
+  uint64_t t0 = 0;
   uint32_t it = 0;
   for (;;) {
     if (mbar_try_wait(bar, parity)) return true;
     if (((++it) & 63u) == 0u) {
       if (*abort_flag) return false;
-      if (globaltimer() - t0 > timeout_ns) {
+      const uint64_t now = globaltimer();
+      if (t0 == 0) {
+        t0 = now;
+      } else if (now - t0 > timeout_ns) {
         *abort_flag = 1;
         return false;
       }
