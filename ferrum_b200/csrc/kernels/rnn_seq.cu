@@ -10,11 +10,14 @@
 // enough because nobody can run a step ahead of the slowest.  Arithmetic is fp32 multiply-adds as in the step-by-step
 // kernels.
 //
-// A step is bound by latency: the product (700 cycles at LSTM 256 on 8 CTAs), two block barriers, the gates and the
-// way to the other CTAs; everything a step needs from global memory is fetched one step ahead.
+// A step is bound by latency: the product, two block barriers, the gates and the way to the other CTAs; everything a step
+// needs from global memory is fetched one step ahead.  How many clusters of eight are on the chip at once is asked of the
+// driver (it is fewer than SMs / 8, a cluster lies within one part of the chip): LSTM 256, batch 32, 64 steps ran as 16
+// clusters of which not all fitted, 270 us forward and 301 backward for two waves of 150 and 180.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 
 #include "../common/ptx.cuh"
@@ -44,10 +47,34 @@ struct SeqArgs {
   unsigned long long timeout_ns;
 };
 
-// part[ks][rows4][BS] += over k = ks, ks + KS, ... of w[k][4 rows] * v[k][BS]; then out[r][b] = sum over ks.
-// Threads are (row quad, k slice); lanes of a warp read consecutive k (or the quads of one k): conflict-free.
+// How a CTA's threads share the product of its `rows4` rows (a multiple of 4) with a vector v[k][BS] of K entries: a thread
+// takes four rows and a slice of k, the `ks_n` partial sums of an output meet in part[ks][b][row].
+struct Tile {
+  int quads, ks_n;        // row quads, slices
+  int vec4;               // weights in registers: 16-byte pieces of the vector per slice
+  int threads, pitch;     // threads that add an output's slices (a power of two within a warp), floats per slice of part
+  __host__ __device__ int vec(int K, int bs, bool reg) const { return reg ? ks_n * vec4 * 4 : (K + 3) / 4 * 4 * bs; }
+};
+__host__ __device__ inline Tile tile_of(int rows4, int K, int bs, bool reg) {
+  Tile t;
+  t.quads = rows4 / 4;
+  t.ks_n = kT / t.quads;
+  const int pieces = (K * bs + 3) / 4;
+  if (reg && t.ks_n > pieces) t.ks_n = pieces;
+  t.vec4 = (pieces + t.ks_n - 1) / t.ks_n;
+  const int n = rows4 * bs;
+  t.threads = 1;
+  while (t.threads < 32 && t.threads * 2 * n <= kT) t.threads *= 2;
+  // the threads of an output read different slices: shifted so that a warp's reads fall into different banks (not where
+  // the weights want the shared memory)
+  t.pitch = n + (!reg || t.threads == 1 ? 0 : t.threads >= 8 ? 4 : 32 / t.threads);
+  return t;
+}
+
+// Weights from shared memory or, past k_res, from L2.  Threads are (k slice, row quad); lanes of a warp read the quads of
+// one k: conflict-free.
 template <int BS, class Stream>
-__device__ __forceinline__ void matvec(const float* wsm, int k_res, int K, int rows4, const float* v, float* part,
+__device__ __forceinline__ void matvec(const float* wsm, int k_res, int K, int rows4, int pitch, const float* v, float* part,
                                        Stream stream_w) {
   const int rq_n = rows4 >> 2, ks_n = kT / rq_n;
   const int ks = threadIdx.x / rq_n, rq = threadIdx.x - ks * rq_n;
@@ -83,107 +110,156 @@ __device__ __forceinline__ void matvec(const float* wsm, int k_res, int K, int r
       for (int i = 0; i < 4; ++i) acc[i][b] = fmaf(w[i], x, acc[i][b]);
     }
   }
-  float* p = part + (ks * rows4 + rq * 4) * BS;
+  float* p = part + ks * pitch + rq * 4;
+#pragma unroll
+  for (int b = 0; b < BS; ++b)
+    *reinterpret_cast<float4*>(p + b * rows4) = make_float4(acc[0][b], acc[1][b], acc[2][b], acc[3][b]);
+}
+
+// The same product with the weights in registers: four rows and up to kKpt k per thread.  What a step then moves is the
+// vector, and a 16-byte read takes four cycles of the shared memory's 128 bytes per cycle even where all lanes read the
+// same address: with two rows and 32 k per thread that was 1470 cycles at LSTM 256 on 8 CTAs, two batch rows.  Slice ks
+// takes the 16-byte pieces ks, ks + ks_n, ...: neighbouring slices in a warp read neighbouring pieces.
+constexpr int kKpt = 16;
+template <int BS>
+__device__ __forceinline__ void matvec_reg(const float (&w)[4][kKpt], const Tile& t, int rows4, int ks, int rq, const float* v,
+                                           float* part) {
+  if (ks >= t.ks_n) return;
+  constexpr int kPer = 4 / BS;  // k of a piece
+  float acc[4][BS];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int b = 0; b < BS; ++b) p[i * BS + b] = acc[i][b];
+    for (int b = 0; b < BS; ++b) acc[i][b] = 0.f;
+  const float4* x = reinterpret_cast<const float4*>(v) + ks;
+  auto piece = [&](int j) {
+    const float4 f = x[j * t.ks_n];
+    const float e[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+    for (int k = 0; k < kPer; ++k)
+#pragma unroll
+      for (int b = 0; b < BS; ++b)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i][b] = fmaf(w[i][j * kPer + k], e[k * BS + b], acc[i][b]);
+  };
+  if (t.vec4 == kKpt / kPer) {
+#pragma unroll
+    for (int j = 0; j < kKpt / kPer; ++j) piece(j);
+  } else {
+#pragma unroll
+    for (int j = 0; j < kKpt / kPer; ++j)
+      if (j < t.vec4) piece(j);
+  }
+  float* p = part + ks * t.pitch + rq * 4;
+#pragma unroll
+  for (int b = 0; b < BS; ++b)
+    *reinterpret_cast<float4*>(p + b * rows4) = make_float4(acc[0][b], acc[1][b], acc[2][b], acc[3][b]);
 }
-
-// The same product with the weights in registers: a thread owns two rows and kKpt consecutive k, so a step reads only
-// the vector (one broadcast per k) from shared memory.  LSTM 256 on 8 CTAs: 2800 -> 700 cycles per step.
-constexpr int kKpt = 32;
-struct RegTile {
-  int pairs, ks_n, kpt;  // row pairs, k slices, k per slice (<= kKpt)
-};
-__host__ __device__ inline RegTile reg_tile(int rows4, int K) {
-  RegTile r;
-  r.pairs = rows4 / 2;
-  r.ks_n = kT / r.pairs;
-  if (r.ks_n > K / 4) r.ks_n = K / 4 > 0 ? K / 4 : 1;
-  r.kpt = ((K + r.ks_n - 1) / r.ks_n + 3) / 4 * 4;
-  return r;
-}
-struct RegLane {
-  int n, v_at, part_at;  // k of this thread's slice (<= 0: idle), its offsets in the vector and in `part`
-};
-template <int BS>
-__device__ __forceinline__ RegLane reg_lane(const RegTile rt, int K, int rows4) {
-  const int ks = threadIdx.x / rt.pairs, rp = threadIdx.x - ks * rt.pairs;
-  return RegLane{ks < rt.ks_n ? max(0, min(rt.kpt, K - ks * rt.kpt)) : -1, ks * rt.kpt * BS, (ks * rows4 + rp * 2) * BS};
-}
-template <int BS>
-__device__ __forceinline__ void matvec_reg(const float (&w)[2][kKpt], const RegLane l, const float* v, float* part) {
-  if (l.n < 0) return;
-  float acc[2][BS];
+// This thread's weights: at(row) is the address of the row's first one or NULL, `step` the distance from k to k + 1.
+template <int BS, class At>
+__device__ __forceinline__ void load_weights(float (&w)[4][kKpt], const Tile& t, int K, int ks, int rq, long long step, At at) {
+  constexpr int kPer = 4 / BS;
 #pragma unroll
-  for (int b = 0; b < BS; ++b) acc[0][b] = acc[1][b] = 0.f;
-  const float* x = v + l.v_at;
+  for (int i = 0; i < 4; ++i) {
+    const float* p = ks < t.ks_n ? at(rq * 4 + i) : nullptr;
 #pragma unroll
-  for (int k0 = 0; k0 < kKpt; k0 += 4) {
-    if (k0 < l.n) {  // the vector is padded with zeros to a multiple of four
-      float xv[4 * BS];
-#pragma unroll
-      for (int i = 0; i < BS; ++i) {
-        const float4 f = *reinterpret_cast<const float4*>(x + k0 * BS + 4 * i);
-        xv[4 * i] = f.x; xv[4 * i + 1] = f.y; xv[4 * i + 2] = f.z; xv[4 * i + 3] = f.w;
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-#pragma unroll
-        for (int b = 0; b < BS; ++b) {
-          acc[0][b] = fmaf(w[0][k0 + k], xv[k * BS + b], acc[0][b]);
-          acc[1][b] = fmaf(w[1][k0 + k], xv[k * BS + b], acc[1][b]);
-        }
+    for (int j = 0; j < kKpt; ++j) {
+      const int k = (ks + j / kPer * t.ks_n) * kPer + j % kPer;
+      w[i][j] = p != nullptr && j / kPer < t.vec4 && k < K ? __ldg(p + k * step) : 0.f;
     }
   }
-  float* p = part + l.part_at;
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int b = 0; b < BS; ++b) p[i * BS + b] = acc[i][b];
 }
 
-// Sums the k slices of n = rows4 * BS outputs with all threads: `threads` of them (a power of two within a warp) share
-// an output; `out` is the thread's first output and `leader` tells who hands the sum on.
+// Sums the k slices of n = rows4 * BS outputs with all threads: `out` is the thread's first output, `passes` how many it
+// has, `step` outputs apart, and `leader` tells who hands the sum on.
 struct Fold {
-  int threads, part, out, step;
+  int part, out, step, passes;
   bool leader;
 };
-__device__ __forceinline__ Fold fold_of(int n) {
+__device__ __forceinline__ Fold fold_of(const Tile& t, int n) {
   Fold f;
-  f.threads = 1;
-  while (f.threads < 32 && f.threads * 2 * n <= kT) f.threads *= 2;
-  f.part = threadIdx.x & (f.threads - 1);
-  f.out = threadIdx.x / f.threads;
-  f.step = kT / f.threads;
+  f.part = threadIdx.x & (t.threads - 1);
+  f.out = threadIdx.x / t.threads;
+  f.step = kT / t.threads;
+  f.passes = (n + f.step - 1) / f.step;
   f.leader = f.part == 0;
   return f;
 }
-__device__ __forceinline__ float fold_sum(const Fold& f, const float* part, int o, int n, int ks_n) {
+__device__ __forceinline__ float fold_sum(const Fold& f, const Tile& t, const float* part, int o, int n) {
   float s = 0.f;
   if (o < n) {
+    const float* p = part + f.part * t.pitch + o;
+    const int step = t.threads * t.pitch;
 #pragma unroll 8
-    for (int ks = f.part; ks < ks_n; ks += f.threads) s += part[ks * n + o];
+    for (int ks = f.part; ks < t.ks_n; ks += t.threads, p += step) s += *p;
   }
-  for (int d = f.threads >> 1; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+  for (int d = t.threads >> 1; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
   return s;
 }
 
-// A value for the same place in the shared memory of every CTA of the cluster; the receivers' mbarriers count the bytes.
-__device__ __forceinline__ void send(uint32_t local_addr, uint32_t local_bar, int rank, float v) {
-  uint32_t dst, bar;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(local_addr), "r"(rank));
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(local_bar), "r"(rank));
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst),
-               "r"(__float_as_uint(v)), "r"(bar)
-               : "memory");
+// Values for the same place in the shared memory of every CTA of the cluster; the receivers' mbarriers count the bytes.  A
+// thread holds element threadIdx.x of the CTA's `count`, consecutive floats of a vector.  Four travel in a message,
+// collected from the warp's lanes, which take the (quad, CTA) pairs in turn; where quads do not lie on 16-byte
+// boundaries every thread sends its own value to everybody.
+struct Outbox {
+  uint32_t first, bar;              // element 0 and the barrier, here
+  uint32_t to[2], to_bar[2];        // quads: where this lane's one or two messages go (0: nowhere)
+  int count, ncl;
+  bool quads, mine;                 // `mine`: this warp sends
+};
+__device__ __forceinline__ uint32_t at_rank(uint32_t local, int rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
+  return a;
+}
+template <int BS>
+__device__ __forceinline__ Outbox outbox(float* vec, uint64_t* bar, int u0, int Hs, int H, int ncl) {
+  Outbox o;
+  o.first = ptx::smem_u32(vec) + u0 * BS * 4;
+  o.bar = ptx::smem_u32(bar);
+  o.count = max(0, min(Hs, H - u0)) * BS;
+  o.ncl = ncl;
+  o.quads = Hs * BS % 4 == 0 && H * BS % 4 == 0;
+  const int lane = threadIdx.x & 31, e0 = threadIdx.x - lane, q = (lane & 7) * 4;
+  o.mine = e0 < o.count;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {  // eight quads to up to eight CTAs: one or two rounds of 32 lanes
+    const int r = i * 4 + (lane >> 3);
+    const bool any = o.quads && r < ncl && e0 + q < o.count;
+    o.to[i] = any ? at_rank(o.first + (e0 + q) * 4, r) : 0;
+    o.to_bar[i] = any ? at_rank(o.bar, r) : 0;
+  }
+  return o;
+}
+// Called by the warps that send, whole.  `offset`: bytes from the vector to the one that is written, `bar`: 0 or 1.
+__device__ __forceinline__ void send_all(const Outbox& o, uint32_t offset, int bar, float v) {
+  if (!o.quads) {
+    const int e = threadIdx.x;
+    if (e < o.count)
+      for (int r = 0; r < o.ncl; ++r)
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(
+                         at_rank(o.first + offset + e * 4, r)),
+                     "r"(__float_as_uint(v)), "r"(at_rank(o.bar + bar * 8, r))
+                     : "memory");
+    return;
+  }
+  const int q = (threadIdx.x & 7) * 4;
+  const float a = __shfl_sync(0xffffffffu, v, q), b = __shfl_sync(0xffffffffu, v, q + 1);
+  const float c = __shfl_sync(0xffffffffu, v, q + 2), d = __shfl_sync(0xffffffffu, v, q + 3);
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    if (o.to[i] != 0)
+      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(
+                       o.to[i] + offset),
+                   "r"(__float_as_uint(a)), "r"(__float_as_uint(b)), "r"(__float_as_uint(c)), "r"(__float_as_uint(d)),
+                   "r"(o.to_bar[i] + bar * 8)
+                   : "memory");
 }
 
 // G = 4: LSTM (input, forget, cell, output); G = 3: GRU (reset, update, new).
 template <int G, int BS, bool kReg>
 __global__ void __launch_bounds__(kT, 1) seq_fwd_kernel(const SeqArgs a) {
-  extern __shared__ float sm[];
+  extern __shared__ __align__(16) float sm[];
   cg::cluster_group cluster = cg::this_cluster();
   const int ncl = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
   const int H = a.H, Hs = a.hs_units, R4 = a.rows4, u0 = rank * Hs, b0 = static_cast<int>(blockIdx.x / ncl) * BS;
@@ -191,13 +267,12 @@ __global__ void __launch_bounds__(kT, 1) seq_fwd_kernel(const SeqArgs a) {
   __shared__ uint64_t arrived[2];           // hidden values of a step complete, one barrier per buffer
   __shared__ int abort_flag;
   float* wsm = sm;                          // [k_res][R4]
-  float* hbuf = wsm + a.k_res * R4;         // [2][H][BS]
-  const int Hp = (H + 3) / 4 * 4;
-  float* part = hbuf + 2 * Hp * BS;         // [4 * kT][BS]
-  float* pre = part + 4 * kT * BS;          // [R4][BS]: gate values (GRU's new gate: the hidden projection)
-  const RegTile rt = reg_tile(R4, H);
-  const RegLane lane = reg_lane<BS>(rt, H, R4);
-  const int ks_n = kReg ? rt.ks_n : kT / (R4 >> 2);
+  const Tile tile = tile_of(R4, H, BS, kReg);
+  const int n_out = R4 * BS, vec = tile.vec(H, BS, kReg);
+  float* hbuf = wsm + a.k_res * R4;         // [2][H][BS], padded
+  float* part = hbuf + 2 * vec;             // [slice][b][R4]
+  float* pre = part + tile.ks_n * tile.pitch;  // [b][R4]: gate values (GRU's new gate: the hidden projection)
+  const int ks = threadIdx.x / tile.quads, rq = threadIdx.x - ks * tile.quads;
 
   auto weight = [&](int k, int r) {         // a.w = transposed matrix [H][G H]
     const int gate = r / Hs, u = u0 + r - gate * Hs;
@@ -207,36 +282,30 @@ __global__ void __launch_bounds__(kT, 1) seq_fwd_kernel(const SeqArgs a) {
     const int k = i / R4;
     wsm[i] = weight(k, i - k * R4);
   }
-  float wreg[2][kKpt];
-  if constexpr (kReg) {
-    const int ks = threadIdx.x / rt.pairs, rp = threadIdx.x - ks * rt.pairs;
-#pragma unroll
-    for (int k = 0; k < kKpt; ++k) {
-      const int kk = ks * rt.kpt + k;
-      const bool in = ks < rt.ks_n && k < rt.kpt && kk < H;
-      wreg[0][k] = in ? weight(kk, rp * 2) : 0.f;
-      wreg[1][k] = in ? weight(kk, rp * 2 + 1) : 0.f;
-    }
-  }
-  for (int i = threadIdx.x; i < 2 * Hp * BS; i += kT) {
+  float wreg[4][kKpt];
+  if constexpr (kReg)
+    load_weights<BS>(wreg, tile, H, ks, rq, GH, [&](int r) {
+      const int gate = r / Hs, u = u0 + r - gate * Hs;
+      return gate < G && u < H ? a.w + gate * H + u : nullptr;
+    });
+  for (int i = threadIdx.x; i < 2 * vec; i += kT) {
     const int k = i / BS, b = i - k * BS;
     hbuf[i] = (a.h0 != nullptr && b < nb && k < H) ? a.h0[static_cast<long long>(b0 + b) * H + k] : 0.f;
   }
   // thread <-> (unit, batch row) of the pointwise part
-  const int pu = threadIdx.x % Hs, pb = threadIdx.x / Hs;
-  const bool mine = pb < nb && u0 + pu < H;
+  const int pu = threadIdx.x / BS, pb = threadIdx.x % BS;
+  const bool mine = pb < nb && pu < Hs && u0 + pu < H;
   const int unit = u0 + pu;
   const long long row = b0 + pb;
   float c = 0.f;
   if (G == 4 && mine && a.c0 != nullptr) c = a.c0[row * H + unit];
   // the gates' inputs of a step: fetched one step ahead into two alternating buffers.  What a thread folds, adds and
-  // fetches is the same at every step: output `o` = (row r, batch row b), worked out once where one pass covers all.
-  float* xbuf = pre + R4 * BS;              // [2][R4 * BS]
-  const int n_out = R4 * BS;
-  const Fold fd = fold_of(n_out);
+  // fetches is the same at every step: output `o` = (batch row b, row r), worked out once where one pass covers all.
+  float* xbuf = pre + n_out;                // [2][b][R4]
+  const Fold fd = fold_of(tile, n_out);
   auto place = [&](int o, int& gate, int& u, int& b) {
-    const int r = o / BS;
-    b = o - r * BS;
+    b = o / R4;
+    const int r = o - b * R4;
     gate = r / Hs;
     u = u0 + r - gate * Hs;
     return o < n_out && b < nb && gate < G && u < H;
@@ -255,7 +324,7 @@ __global__ void __launch_bounds__(kT, 1) seq_fwd_kernel(const SeqArgs a) {
       if (place(o, gate, u, b)) cp_async4(dst + o, a.xi + t * x_step + static_cast<long long>(b0 + b) * GH + gate * H + u);
     }
   };
-  const uint32_t bytes = static_cast<uint32_t>(H * nb * 4);  // what a CTA receives per step, its own part included
+  const uint32_t bytes = static_cast<uint32_t>(H * BS * 4);  // what a CTA receives per step, its own part included
   if (threadIdx.x == 0) {
     abort_flag = 0;
     ptx::mbar_init(&arrived[0], 1);
@@ -267,12 +336,12 @@ __global__ void __launch_bounds__(kT, 1) seq_fwd_kernel(const SeqArgs a) {
   fetch_x(0);
   const long long e_step = static_cast<long long>(a.B) * H;
   const long long e_mine = row * H + unit, e4_mine = row * 4 * H + unit;
-  const uint32_t send_at = ptx::smem_u32(hbuf) + (unit * BS + pb) * 4;
+  const Outbox box = outbox<BS>(hbuf, arrived, u0, Hs, H, ncl);
   cluster.sync();
 
   for (int t = 0; t < a.T; ++t) {
     const int buf = t & 1;
-    const float* cur = hbuf + buf * Hp * BS;
+    const float* cur = hbuf + buf * vec;
     const float* x = xbuf + buf * n_out;
     if (t > 0) {
       // a wait that gives up (reported) goes on with what is there, so that every thread keeps meeting the same barriers
@@ -281,17 +350,17 @@ __global__ void __launch_bounds__(kT, 1) seq_fwd_kernel(const SeqArgs a) {
       if (threadIdx.x == 0) ptx::mbar_arrive_expect_tx(&arrived[buf], bytes);  // for the step after next
     }
     if constexpr (kReg)
-      matvec_reg<BS>(wreg, lane, cur, part);
+      matvec_reg<BS>(wreg, tile, R4, ks, rq, cur, part);
     else
-      matvec<BS>(wsm, a.k_res, H, R4, cur, part, [&](int k, int r, float (&w)[4]) {
+      matvec<BS>(wsm, a.k_res, H, R4, tile.pitch, cur, part, [&](int k, int r, float (&w)[4]) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) w[i] = weight(k, r + i);
       });
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     // gate activations in the threads that add the slices: the serial part below is the cell update alone
-    for (int o = fd.out; o < (n_out + fd.step - 1) / fd.step * fd.step; o += fd.step) {
-      float s = fold_sum(fd, part, o, n_out, ks_n);
+    for (int pass = 0, o = fd.out; pass < fd.passes; ++pass, o += fd.step) {
+      float s = fold_sum(fd, tile, part, o, n_out);
       if (!fd.leader || o >= n_out) continue;
       int gate = gate0, u = uu0, b = bb0;
       bool ok = valid0;
@@ -310,21 +379,18 @@ __global__ void __launch_bounds__(kT, 1) seq_fwd_kernel(const SeqArgs a) {
     float h = 0.f, p[G];
     if (mine) {
 #pragma unroll
-      for (int q = 0; q < G; ++q) p[q] = pre[(q * Hs + pu) * BS + pb];
+      for (int q = 0; q < G; ++q) p[q] = pre[pb * R4 + q * Hs + pu];
       if constexpr (G == 4) {
         c = p[1] * c + p[0] * p[2];
         h = p[3] * tanhf(c);
       } else {
-        const float n = tanhf(x[(2 * Hs + pu) * BS + pb] + p[0] * p[2]);
+        const float n = tanhf(x[pb * R4 + 2 * Hs + pu] + p[0] * p[2]);
         h = (1.f - p[1]) * n + p[1] * cur[unit * BS + pb];
         if (a.saved != nullptr) a.saved[e4_mine + 4 * t * e_step + 2 * H] = n;
       }
-      if (t + 1 < a.T) {
-        const int nxt = buf ^ 1;
-        for (int r = 0; r < ncl; ++r)
-          send(send_at + nxt * Hp * BS * 4, ptx::smem_u32(&arrived[nxt]), r, h);
-      }
-      // what the others do not wait for
+    }
+    if (box.mine && t + 1 < a.T) send_all(box, (buf ^ 1) * vec * 4, buf ^ 1, h);
+    if (mine) {  // what the others do not wait for
       a.hs[e_mine + t * e_step] = h;
       if (a.hs_kept != nullptr) a.hs_kept[e_mine + t * e_step] = h;
       if (G == 4 && a.cs != nullptr) a.cs[e_mine + t * e_step] = c;
@@ -344,7 +410,7 @@ __global__ void __launch_bounds__(kT, 1) seq_fwd_kernel(const SeqArgs a) {
 
 template <int G, int BS, bool kReg>
 __global__ void __launch_bounds__(kT, 1) seq_bwd_kernel(const SeqArgs a) {
-  extern __shared__ float sm[];
+  extern __shared__ __align__(16) float sm[];
   cg::cluster_group cluster = cg::this_cluster();
   const int ncl = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
   const int H = a.H, Hs = a.hs_units, R4 = a.rows4, u0 = rank * Hs, b0 = static_cast<int>(blockIdx.x / ncl) * BS;
@@ -352,13 +418,12 @@ __global__ void __launch_bounds__(kT, 1) seq_bwd_kernel(const SeqArgs a) {
   __shared__ uint64_t arrived[2];           // gate gradients of a step complete, one barrier per buffer
   __shared__ int abort_flag;
   float* wsm = sm;                          // [k_res][R4]: rows of the recurrent matrix, this CTA's columns
-  float* dbuf = wsm + a.k_res * R4;         // [2][K][BS]: gate gradients of the step, all units
-  const int Kp = (K + 3) / 4 * 4;
-  float* part = dbuf + 2 * Kp * BS;         // [4 * kT][BS]
-  float* dh = part + 4 * kT * BS;           // [R4][BS]: gradient that arrives from the next step
-  const RegTile rt = reg_tile(R4, K);
-  const RegLane lane = reg_lane<BS>(rt, K, R4);
-  const int ks_n = kReg ? rt.ks_n : kT / (R4 >> 2);
+  const Tile tile = tile_of(R4, K, BS, kReg);
+  const int n_out = R4 * BS, vec = tile.vec(K, BS, kReg);
+  float* dbuf = wsm + a.k_res * R4;         // [2][K][BS], padded: gate gradients of the step, all units
+  float* part = dbuf + 2 * vec;             // [slice][b][R4]
+  float* dh = part + tile.ks_n * tile.pitch;  // [b][R4]: gradient that arrives from the next step
+  const int ks = threadIdx.x / tile.quads, rq = threadIdx.x - ks * tile.quads;
 
   auto weight = [&](int k, int r) {         // a.w = [G H][H]
     return r < Hs && u0 + r < H ? __ldg(a.w + static_cast<long long>(k) * H + u0 + r) : 0.f;
@@ -367,28 +432,19 @@ __global__ void __launch_bounds__(kT, 1) seq_bwd_kernel(const SeqArgs a) {
     const int k = i / R4;
     wsm[i] = weight(k, i - k * R4);
   }
-  float wreg[2][kKpt];
-  if constexpr (kReg) {
-    const int ks = threadIdx.x / rt.pairs, rp = threadIdx.x - ks * rt.pairs;
-#pragma unroll
-    for (int k = 0; k < kKpt; ++k) {
-      const int kk = ks * rt.kpt + k;
-      const bool in = ks < rt.ks_n && k < rt.kpt && kk < K;
-      wreg[0][k] = in ? weight(kk, rp * 2) : 0.f;
-      wreg[1][k] = in ? weight(kk, rp * 2 + 1) : 0.f;
-    }
-  }
-  for (int i = threadIdx.x; i < 2 * Kp * BS; i += kT) dbuf[i] = 0.f;
-  for (int i = threadIdx.x; i < R4 * BS; i += kT) dh[i] = 0.f;
+  float wreg[4][kKpt];
+  if constexpr (kReg)
+    load_weights<BS>(wreg, tile, K, ks, rq, H, [&](int r) { return r < Hs && u0 + r < H ? a.w + u0 + r : nullptr; });
+  for (int i = threadIdx.x; i < 2 * vec; i += kT) dbuf[i] = 0.f;
+  for (int i = threadIdx.x; i < n_out; i += kT) dh[i] = 0.f;
 
-  const int pu = threadIdx.x % Hs, pb = threadIdx.x / Hs;
-  const bool mine = pb < nb && u0 + pu < H;
+  const int pu = threadIdx.x / BS, pb = threadIdx.x % BS;
+  const bool mine = pb < nb && pu < Hs && u0 + pu < H;
   const int unit = u0 + pu;
   const long long row = b0 + pb;
-  const int n_out = R4 * BS;
-  const Fold fd = fold_of(n_out);
+  const Fold fd = fold_of(tile, n_out);
   const long long e_step = static_cast<long long>(a.B) * K, e_mine = row * K + unit;
-  const uint32_t send_at = ptx::smem_u32(dbuf) + (unit * BS + pb) * 4;
+  const Outbox box = outbox<BS>(dbuf, arrived, u0, Hs, H, ncl);
   float carry = 0.f;                        // LSTM: dc; GRU: dh * z of the step after
   if (G == 4 && mine && a.d_c_last != nullptr) carry = a.d_c_last[row * H + unit];
   // what the pointwise part of step t reads from global memory
@@ -410,7 +466,7 @@ __global__ void __launch_bounds__(kT, 1) seq_bwd_kernel(const SeqArgs a) {
     if (a.d_hs != nullptr) v.d = __ldg(a.d_hs + e);
     return v;
   };
-  const uint32_t bytes = static_cast<uint32_t>(K * nb * 4);  // what a CTA receives per step, its own part included
+  const uint32_t bytes = static_cast<uint32_t>(K * BS * 4);  // what a CTA receives per step, its own part included
   if (threadIdx.x == 0) {
     abort_flag = 0;
     ptx::mbar_init(&arrived[0], 1);
@@ -424,10 +480,12 @@ __global__ void __launch_bounds__(kT, 1) seq_bwd_kernel(const SeqArgs a) {
 
   for (int t = a.T - 1; t >= 0; --t) {
     const int buf = t & 1;
-    float* cur = dbuf + buf * Kp * BS;
+    float* cur = dbuf + buf * vec;
     float dx[G], dq[G];
+#pragma unroll
+    for (int q = 0; q < G; ++q) dq[q] = 0.f;
     if (mine) {
-      const float g = in.d + dh[pu * BS + pb] + (G == 3 ? carry : 0.f);
+      const float g = in.d + dh[pb * R4 + pu] + (G == 3 ? carry : 0.f);
       if constexpr (G == 4) {
         const float i = in.s[0], f = in.s[1], cc = in.s[2], o = in.s[3];
         const float tc = tanhf(in.c);
@@ -450,12 +508,12 @@ __global__ void __launch_bounds__(kT, 1) seq_bwd_kernel(const SeqArgs a) {
         dq[2] = dn * r;
         carry = g * z;
       }
-      for (int r = 0; r < ncl; ++r) {
+    }
+    if (box.mine) {
 #pragma unroll
-        for (int q = 0; q < G; ++q)
-          send(send_at + (buf * Kp + q * H) * BS * 4, ptx::smem_u32(&arrived[buf]), r, dq[q]);
-      }
-      // what the others do not wait for
+      for (int q = 0; q < G; ++q) send_all(box, (buf * vec + q * H * BS) * 4, buf, dq[q]);
+    }
+    if (mine) {  // what the others do not wait for
       const long long e = e_mine + t * e_step;
 #pragma unroll
       for (int q = 0; q < G; ++q) {
@@ -468,21 +526,21 @@ __global__ void __launch_bounds__(kT, 1) seq_bwd_kernel(const SeqArgs a) {
       report_status(a.status, kStatusGemmTimeout, 82, blockIdx.x, t);
     if (threadIdx.x == 0) ptx::mbar_arrive_expect_tx(&arrived[buf], bytes);  // for the step after next
     if constexpr (kReg)
-      matvec_reg<BS>(wreg, lane, cur, part);
+      matvec_reg<BS>(wreg, tile, R4, ks, rq, cur, part);
     else
-      matvec<BS>(wsm, a.k_res, K, R4, cur, part, [&](int k, int r, float (&w)[4]) {
+      matvec<BS>(wsm, a.k_res, K, R4, tile.pitch, cur, part, [&](int k, int r, float (&w)[4]) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) w[i] = weight(k, r + i);
       });
     __syncthreads();
-    for (int o = fd.out; o < (n_out + fd.step - 1) / fd.step * fd.step; o += fd.step) {
-      const float s = fold_sum(fd, part, o, n_out, ks_n);
+    for (int pass = 0, o = fd.out; pass < fd.passes; ++pass, o += fd.step) {
+      const float s = fold_sum(fd, tile, part, o, n_out);
       if (fd.leader && o < n_out) dh[o] = s;
     }
     __syncthreads();
   }
   if (mine) {
-    if (a.dh0 != nullptr) a.dh0[row * H + unit] = dh[pu * BS + pb] + (G == 3 ? carry : 0.f);
+    if (a.dh0 != nullptr) a.dh0[row * H + unit] = dh[pb * R4 + pu] + (G == 3 ? carry : 0.f);
     if (G == 4 && a.dc0 != nullptr) a.dc0[row * H + unit] = carry;
   }
   cluster.sync();  // the other CTAs may still write into this one's shared memory
@@ -498,27 +556,20 @@ int smem_limit() {
   return v;
 }
 
-int sm_count() {
-  static const int n = [] {
-    int dev = 0, v = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    return v;
-  }();
-  return n;
-}
-
 struct Plan {
   int ncl, bs, hs_units, rows4, k_res;
   bool reg;  // weights in registers
   size_t smem;
 };
+// Clusters of `ncl` CTAs, one CTA per SM, that are on the chip at once.
+int cluster_slots(int ncl);
+
 // Cluster size: one CTA per 32 hidden units up to eight (a CTA's share of the weights is then what a step has to
 // stream from shared memory).  Batch slice: as small as keeps every cluster on the chip at once.
 bool plan(int G, int B, int H, bool backward, Plan* p) {
   if (H < 1 || H > 1024) return false;
   p->ncl = H >= 256 ? 8 : (H >= 128 ? 4 : (H >= 64 ? 2 : 1));
-  const int slots = sm_count() / p->ncl;
+  const int slots = cluster_slots(p->ncl);
   p->bs = B <= slots ? 1 : (B <= 2 * slots ? 2 : (B <= 4 * slots ? 4 : 8));
   p->hs_units = (H + p->ncl - 1) / p->ncl;
   const int rows = backward ? p->hs_units : G * p->hs_units, K = backward ? G * H : H;
@@ -526,9 +577,12 @@ bool plan(int G, int B, int H, bool backward, Plan* p) {
   if (p->rows4 / 4 > kT) return false;
   const size_t limit = static_cast<size_t>(smem_limit()) - 1024;
   for (; p->bs >= 1; p->bs >>= 1) {  // a smaller slice leaves more shared memory to the weights
-    const size_t fixed = (2 * static_cast<size_t>((K + 3) / 4 * 4) + 4 * kT + 3 * p->rows4) * p->bs * 4;
+    p->reg = p->bs <= 4 && tile_of(p->rows4, K, p->bs, true).vec4 * (4 / p->bs) <= kKpt;
+    const Tile t = tile_of(p->rows4, K, p->bs, p->reg);
+    // two vectors, the partial sums, and the gates with their two input buffers
+    const size_t fixed = (2 * static_cast<size_t>(t.vec(K, p->bs, p->reg)) + static_cast<size_t>(t.ks_n) * t.pitch +
+                          3 * static_cast<size_t>(p->rows4) * p->bs) * 4;
     if (p->hs_units * p->bs > kT || fixed > limit) continue;
-    p->reg = p->bs <= 4 && reg_tile(p->rows4, K).kpt <= kKpt;
     if (p->reg) {
       p->k_res = 0;
       p->smem = fixed;
@@ -544,6 +598,28 @@ bool plan(int G, int B, int H, bool backward, Plan* p) {
     return true;
   }
   return false;
+}
+
+int cluster_slots(int ncl) {
+  static std::atomic<int> known[9];
+  int n = known[ncl].load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ncl);
+  cfg.blockDim = dim3(kT);
+  cfg.dynamicSmemBytes = 0;  // 512 threads of more than 64 registers: one CTA per SM whatever its shared memory
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ncl;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, seq_fwd_kernel<4, 2, true>, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    return 1;
+  }
+  known[ncl].store(n, std::memory_order_relaxed);
+  return n;
 }
 
 template <int G, int BS, bool kReg>
