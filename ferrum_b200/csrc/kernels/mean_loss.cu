@@ -24,6 +24,7 @@ namespace cg = cooperative_groups;
 constexpr int kThreads = 256;
 constexpr int kCluster = 8;
 constexpr long long kClusterElems = 256 * 1024;
+constexpr int kClusterTrips = 3;
 constexpr int kMaxPartials = 1184;  // 8 blocks per SM on 148 SMs
 
 __device__ __forceinline__ float to_f(float v) { return v; }
@@ -297,9 +298,9 @@ int wide_grid(long long blocks) {
 
 // Launches the one-cluster form of a kernel for small inputs, else the wide form followed by the final addition.
 template <typename... P, typename... A>
-int run_mean(void (*clustered)(P...), void (*wide)(P...), long long elems, long long blocks, float* loss,
-             float* partial, float scale, cudaStream_t st, A... args) {
-  if (elems <= kClusterElems) {
+int run_mean(void (*clustered)(P...), void (*wide)(P...), bool small, long long blocks, float* loss, float* partial,
+             float scale, cudaStream_t st, A... args) {
+  if (small) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kCluster);
     cfg.blockDim = dim3(kThreads);
@@ -325,6 +326,11 @@ bool vec_ok(const void* a, const void* b, int cols, size_t elem) {
 // Rows that the register-resident warp kernel takes.
 bool warp_row(const void* x, const void* dx, int cols) { return cols >= 264 && cols <= 4096 && vec_ok(x, dx, cols, 2); }
 
+// A row of a cross-entropy is a chain of loads, reductions and exponentials, 1.2 us of a warp: the cluster's eight blocks
+// take at most three rounds of them, beyond that the whole chip and a second launch are faster (777 x 37 bf16: 19.1 us on
+// eight SMs, 512 x 512 15.2).
+bool few_rows(long long elems, long long blocks) { return elems <= kClusterElems && blocks <= kClusterTrips * kCluster; }
+
 template <typename T>
 int ce_fwd(const void* x, const long long* labels, void* dlogits, float* loss, float* partial, long long rows, int cols,
            float scale, cudaStream_t st) {
@@ -333,8 +339,8 @@ int ce_fwd(const void* x, const long long* labels, void* dlogits, float* loss, f
     if (warp_row(x, dx, cols)) {
       const int k = (cols / 8 + 31) / 32;
 #define FB_CE_WARP(K)                                                                                                  \
-  return run_mean(ce_fwd_warp_kernel<K, true>, ce_fwd_warp_kernel<K, false>, rows * cols, (rows + 7) / 8, loss, partial, \
-                  scale, st, static_cast<const __nv_bfloat16*>(x), labels, dx, loss, partial, rows, cols, scale,      \
+  return run_mean(ce_fwd_warp_kernel<K, true>, ce_fwd_warp_kernel<K, false>, few_rows(rows * cols, (rows + 7) / 8),     \
+                  (rows + 7) / 8, loss, partial, scale, st, static_cast<const __nv_bfloat16*>(x), labels, dx, loss, partial, rows, cols, scale,      \
                   bounds_status_ref())
       if (k <= 4) FB_CE_WARP(4);
       if (k <= 8) FB_CE_WARP(8);
@@ -343,11 +349,12 @@ int ce_fwd(const void* x, const long long* labels, void* dlogits, float* loss, f
     }
   }
   if (cols <= 512)
-    return run_mean(ce_fwd_kernel<T, 32, true>, ce_fwd_kernel<T, 32, false>, rows * cols, (rows + 7) / 8, loss, partial,
-                    scale, st, static_cast<const T*>(x), labels, dx, loss, partial, rows, cols, scale,
-                    bounds_status_ref());
-  return run_mean(ce_fwd_kernel<T, 256, true>, ce_fwd_kernel<T, 256, false>, rows * cols, rows, loss, partial, scale, st,
-                  static_cast<const T*>(x), labels, dx, loss, partial, rows, cols, scale, bounds_status_ref());
+    return run_mean(ce_fwd_kernel<T, 32, true>, ce_fwd_kernel<T, 32, false>, few_rows(rows * cols, (rows + 7) / 8),
+                    (rows + 7) / 8, loss, partial, scale, st, static_cast<const T*>(x), labels, dx, loss, partial, rows,
+                    cols, scale, bounds_status_ref());
+  return run_mean(ce_fwd_kernel<T, 256, true>, ce_fwd_kernel<T, 256, false>, few_rows(rows * cols, rows), rows, loss,
+                  partial, scale, st, static_cast<const T*>(x), labels, dx, loss, partial, rows, cols, scale,
+                  bounds_status_ref());
 }
 
 }  // namespace
@@ -371,11 +378,11 @@ extern "C" int fb_nll_fwd(const void* log_probs, const long long* target, float*
   if (rows <= 0 || cols <= 0) return -1;  // no mean over nothing: `loss` stays unwritten
   const long long blocks = (rows + kThreads - 1) / kThreads;
   if (dtype == FB_DT_F32)
-    return run_mean(nll_fwd_kernel<float, true>, nll_fwd_kernel<float, false>, rows, blocks, loss, workspace, scale,
-                    stream, static_cast<const float*>(log_probs), target, loss, workspace, rows, cols, scale, status);
+    return run_mean(nll_fwd_kernel<float, true>, nll_fwd_kernel<float, false>, rows <= kClusterElems, blocks, loss, workspace,
+                    scale, stream, static_cast<const float*>(log_probs), target, loss, workspace, rows, cols, scale, status);
   if (dtype == FB_DT_BF16)
-    return run_mean(nll_fwd_kernel<__nv_bfloat16, true>, nll_fwd_kernel<__nv_bfloat16, false>, rows, blocks, loss,
-                    workspace, scale, stream, static_cast<const __nv_bfloat16*>(log_probs), target, loss, workspace,
+    return run_mean(nll_fwd_kernel<__nv_bfloat16, true>, nll_fwd_kernel<__nv_bfloat16, false>, rows <= kClusterElems, blocks,
+                    loss, workspace, scale, stream, static_cast<const __nv_bfloat16*>(log_probs), target, loss, workspace,
                     rows, cols, scale, status);
   return -1;
 }
@@ -401,6 +408,6 @@ extern "C" int fb_nll_bwd(const long long* target, const float* gout, void* dlog
 extern "C" int fb_loss_mean_fwd(const float* pred, const float* target, float* loss, float* workspace, long long n,
                                 int kind, float scale, cudaStream_t stream) {
   if (n <= 0) return -1;
-  return run_mean(elem_loss_kernel<true>, elem_loss_kernel<false>, n, (n + 4 * kThreads - 1) / (4 * kThreads), loss,
-                  workspace, scale, stream, pred, target, loss, workspace, n, kind, scale);
+  return run_mean(elem_loss_kernel<true>, elem_loss_kernel<false>, n <= kClusterElems,
+                  (n + 4 * kThreads - 1) / (4 * kThreads), loss, workspace, scale, stream, pred, target, loss, workspace, n, kind, scale);
 }
