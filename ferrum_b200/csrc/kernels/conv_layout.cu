@@ -2,18 +2,22 @@
 // keeps activations as NCHW fp32 (ferrum-nn/src/conv.rs:209-330); the tensor-core kernels read NHWC bf16 through
 // 4-D TMA boxes, with the channel count padded to a multiple of 8 so that every pixel starts on a 16-byte boundary.
 //
-//   fb_nchw_to_nhwc_bf16   [B, C, P] fp32 -> [B, P, Cp] bf16   (P = H * W; channels C .. Cp - 1 are written as zero)
-//   fb_nhwc_to_nchw_f32    [B, P, ld] fp32 (first C of ld channels) -> [B, C, P] fp32
+// A convolution of any stride is one of stride 1 over a space-to-depth arrangement of its input:
+//   z[b, I, J, (rh * ew + rw) * C + c] = x[b, c, I * sh + rh - ph, J * sw + rw - pw],  rh < eh = min(sh, kh), rw < ew,
+// zero outside the image, with ceil(kh / sh) x ceil(kw / sw) filters.  Rows and columns that the stride skips altogether
+// (kernel < stride: the 1 x 1 shortcut of a residual block) are not in z.  Stride 1 is the case sh = sw = 1, ph = pw = 0:
+// a plain NCHW -> NHWC conversion, the padding being the TMA unit's zero fill.
 //
-//   fb_nchw_to_s2d_nhwc_bf16  strided convolutions: [B, C, H, W] fp32 -> space-to-depth NHWC bf16
-//                             z[b, I, J, (rh * sw + rw) * C + c] = x[b, c, I * sh + rh - ph, J * sw + rw - pw]
-//                             (zero outside the image), which turns a stride-(sh, sw) convolution with a kh x kw
-//                             filter into a stride-1 one with a ceil(kh / sh) x ceil(kw / sw) filter over sh * sw * C
-//                             channels, i.e. into the implicit-GEMM kernel's case
-//   fb_s2d_nhwc_to_nchw_f32   the inverse, for the data gradient: [B, Hz, Wz, ld] fp32 -> [B, C, H, W] fp32
+//   fb_conv_pack_input    x -> z, optionally with the gradient of a ReLU in front (x counts where mask > 0)
+//   fb_conv_pack_filters  [O, C, kh, kw] fp32 -> the bf16 filters of the forward product or of the data gradient
+//   fb_conv_fold_wgrad    the splits of fb_conv_wgrad -> their sum as [O, C, kh, kw]
+//   fb_s2d_nhwc_to_nchw_f32  the data gradient of z -> that of x
+//   fb_nhwc_to_nchw_f32      a result [B, P, ld] -> [B, C, P], plus a residual, behind a ReLU
 //
-// All are 32 x 32 tile transposes through shared memory: coalesced reads along P (NCHW) or C (NHWC), coalesced
-// writes along the other.
+// All are bound by HBM.  The input conversion goes through shared memory in blocks of 64 channels x 64 pixels of bf16
+// pairs: 128-byte reads along the pixels, 16-byte writes along the channels.  (Results stored as NCHW from the GEMM's
+// accumulator rows, a 4-byte store per channel and pixel, were slower than the transposing kernel: 243 us of GEMMs in a
+// residual block's training step against 176 + 67.)
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -22,86 +26,130 @@
 namespace fb {
 namespace {
 
-__global__ void __launch_bounds__(256)
-nchw_to_nhwc_bf16_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, int C, long long P, int Cp) {
-  __shared__ float tile[32][33];
-  const long long b = blockIdx.z;
-  const long long p0 = static_cast<long long>(blockIdx.x) * 32;
-  const int c0 = blockIdx.y * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
-  const float* xb = x + b * C * P;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int c = c0 + ty + 8 * i;
-    const long long p = p0 + tx;
-    tile[ty + 8 * i][tx] = (c < C && p < P) ? xb[c * P + p] : 0.f;
-  }
-  __syncthreads();
-  __nv_bfloat16* yb = y + b * P * Cp;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const long long p = p0 + ty + 8 * i;
-    const int c = c0 + tx;
-    if (p < P && c < Cp) yb[p * Cp + c] = __float2bfloat16_rn(tile[tx][ty + 8 * i]);
-  }
-}
-
-__global__ void __launch_bounds__(256)
-nhwc_to_nchw_f32_kernel(const float* __restrict__ x, float* __restrict__ y, int C, long long P, long long ld) {
-  __shared__ float tile[32][33];
-  const long long b = blockIdx.z;
-  const long long p0 = static_cast<long long>(blockIdx.x) * 32;
-  const int c0 = blockIdx.y * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const float* xb = x + b * P * ld;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const long long p = p0 + ty + 8 * i;
-    const int c = c0 + tx;
-    tile[ty + 8 * i][tx] = (p < P && c < C) ? xb[p * ld + c] : 0.f;
-  }
-  __syncthreads();
-  float* yb = y + b * C * P;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int c = c0 + ty + 8 * i;
-    const long long p = p0 + tx;
-    if (c < C && p < P) yb[c * P + p] = tile[tx][ty + 8 * i];
-  }
-}
-
-// Space-to-depth geometry shared by the two strided-convolution layout kernels.
+// A convolution as the layouts see it; q counts the columns of z times ew, r its rows times eh.
 struct S2d {
-  int C, H, W, sh, sw, ph, pw, Hz, Wz;
-  long long ld;  // channels per pixel of the NHWC side (>= sh * sw * C)
+  int C, H, W, sh, sw, eh, ew, ph, pw, Hz, Wz;
+  long long ld;  // channels per pixel of the NHWC side (>= eh * ew * C)
 };
 
-// Block = image row (b, i) x 32 columns x 32 channels of the NCHW side.
+constexpr int kTileC = 64, kTileQ = 64;
+
+template <bool kVec>
 __global__ void __launch_bounds__(256)
-nchw_to_s2d_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ z, const S2d g) {
-  __shared__ float tile[32][33];
-  const long long bi = blockIdx.x;
-  const long long b = bi / g.H;
-  const int i = static_cast<int>(bi - b * g.H);
-  const int I = (i + g.ph) / g.sh, rh = (i + g.ph) % g.sh;
-  if (I >= g.Hz) return;  // a row no window reaches (uniform over the block)
-  const int j0 = blockIdx.y * 32, c0 = blockIdx.z * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const float* xr = x + (b * g.C * g.H + i) * static_cast<long long>(g.W);
+pack_input_kernel(const float* __restrict__ x, const float* __restrict__ mask, __nv_bfloat16* __restrict__ z, const S2d g,
+                  int q_tiles) {
+  __shared__ uint32_t tile[kTileC / 2][kTileQ + 1];
+  const int q0 = static_cast<int>(blockIdx.x % q_tiles) * kTileQ;
+  const long long br = blockIdx.x / q_tiles;
+  const int rows = g.Hz * g.eh;
+  const long long b = br / rows;
+  const int r = static_cast<int>(br - b * rows), I = r / g.eh, rh = r - I * g.eh, i = I * g.sh + rh - g.ph;
+  const int c0 = blockIdx.y * kTileC, nc = min(kTileC, g.C - c0);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool row_in = i >= 0 && i < g.H;
+  const long long plane = static_cast<long long>(g.H) * g.W;
+  const long long base = (b * g.C + c0) * plane + static_cast<long long>(i) * g.W;
+  const int n_q = g.Wz * g.ew;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int c = c0 + ty + 8 * k, j = j0 + tx;
-    tile[ty + 8 * k][tx] = (c < g.C && j < g.W) ? xr[static_cast<long long>(c) * g.H * g.W + j] : 0.f;
+  for (int h = 0; h < 2; ++h) {
+    const int q = q0 + h * 32 + lane;
+    int j = q;
+    if (g.sw != 1 || g.ew != 1) {
+      const int J = q / g.ew;
+      j = J * g.sw + q - J * g.ew;
+    }
+    j -= g.pw;
+    const bool in = row_in && q < n_q && j >= 0 && j < g.W;
+    float v[2][kTileC / 16];
+#pragma unroll
+    for (int k = 0; k < kTileC / 16; ++k) {
+      const int c = (warp + 8 * k) * 2;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        v[e][k] = 0.f;
+        if (in && c + e < nc) v[e][k] = __ldg(x + base + (c + e) * plane + j);
+      }
+    }
+    if (mask != nullptr) {
+#pragma unroll
+      for (int k = 0; k < kTileC / 16; ++k) {
+        const int c = (warp + 8 * k) * 2;
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          if (in && c + e < nc && !(__ldg(mask + base + (c + e) * plane + j) > 0.f)) v[e][k] = 0.f;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kTileC / 16; ++k) {
+      const __nv_bfloat162 p = __floats2bfloat162_rn(v[0][k], v[1][k]);
+      tile[warp + 8 * k][h * 32 + lane] = *reinterpret_cast<const uint32_t*>(&p);
+    }
   }
   __syncthreads();
+  const int oct = threadIdx.x & 7;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int j = j0 + ty + 8 * k, c = c0 + tx;
-    if (j >= g.W || c >= g.C) continue;
-    const int J = (j + g.pw) / g.sw, rw = (j + g.pw) % g.sw;
-    if (J >= g.Wz) continue;
-    z[((b * g.Hz + I) * g.Wz + J) * g.ld + static_cast<long long>(rh * g.sw + rw) * g.C + c] =
-        __float2bfloat16_rn(tile[tx][ty + 8 * k]);
+  for (int k = 0; k < 2; ++k) {
+    const int ql = k * 32 + (threadIdx.x >> 3), q = q0 + ql;
+    if (q >= n_q) continue;
+    const int J = q / g.ew, rw = q - J * g.ew;
+    __nv_bfloat16* pixel = z + ((b * g.Hz + I) * g.Wz + J) * g.ld;
+    __nv_bfloat16* dst = pixel + static_cast<long long>(rh * g.ew + rw) * g.C + c0 + oct * 8;
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) w[e] = tile[oct * 4 + e][ql];
+    if (kVec) {  // whole octets of channels on 16-byte boundaries
+      if (oct * 8 < nc) *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (oct * 8 + e < nc)
+          dst[e] = __ushort_as_bfloat16(static_cast<unsigned short>(e & 1 ? w[e >> 1] >> 16 : w[e >> 1] & 0xffff));
+      if (oct == 0 && c0 == 0 && rh == g.eh - 1 && rw == g.ew - 1)  // the padding channels
+        for (long long c = static_cast<long long>(g.eh) * g.ew * g.C; c < g.ld; ++c) pixel[c] = __float2bfloat16_rn(0.f);
+    }
+  }
+}
+
+// Filter tap of channel ch of z under tap (I, J) of the stride-1 convolution; -1: there is none (a zero).
+struct Filter {
+  int O, C, kh, kw, sh, sw, eh, ew, k2h, k2w, pitch;  // pitch: elements per tap of a packed row
+};
+__device__ __forceinline__ int filter_at(const Filter& f, int I, int J, int ch, int& c) {
+  const int rc = ch / f.C, rh = rc / f.ew, rw = rc - rh * f.ew;
+  c = ch - rc * f.C;
+  const int ki = I * f.sh + rh, kj = J * f.sw + rw;
+  return rh < f.eh && ki < f.kh && kj < f.kw ? ki * f.kw + kj : -1;
+}
+
+// kDgrad = false: out[o][I, J][ch] (pitch >= eh ew C); true: out[ch][I, J flipped][o] (pitch >= O).
+template <bool kDgrad>
+__global__ void __launch_bounds__(256)
+pack_filters_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ out, const Filter f, int total) {
+  for (int at = blockIdx.x * 256 + threadIdx.x; at < total; at += gridDim.x * 256) {
+    const int k = at % f.pitch, rt = at / f.pitch, taps = f.k2h * f.k2w, row = rt / taps;
+    int tap = rt - row * taps;
+    if (kDgrad) tap = taps - 1 - tap;
+    const int I = tap / f.k2w, J = tap - I * f.k2w, ch = kDgrad ? row : k, o = kDgrad ? k : row;
+    int c;
+    const int t = filter_at(f, I, J, ch, c);
+    const bool in = t >= 0 && o < f.O;
+    out[at] = __float2bfloat16_rn(in ? __ldg(w + (static_cast<long long>(o) * f.C + c) * f.kh * f.kw + t) : 0.f);
+  }
+}
+
+// dw[o, c, ki, kj] = sum over the splits of part[split][o][I, J][ch], in their order.
+__global__ void __launch_bounds__(256)
+fold_wgrad_kernel(const float* __restrict__ part, float* __restrict__ dw, const Filter f, int splits, int total) {
+  for (int at = blockIdx.x * 256 + threadIdx.x; at < total; at += gridDim.x * 256) {
+    const int ch = at % f.pitch, rt = at / f.pitch, taps = f.k2h * f.k2w, o = rt / taps, tap = rt - o * taps;
+    const int I = tap / f.k2w, J = tap - I * f.k2w;
+    int c;
+    const int t = filter_at(f, I, J, ch, c);
+    if (t < 0) continue;
+    float s = 0.f;
+#pragma unroll 8
+    for (int i = 0; i < splits; ++i) s += __ldg(part + static_cast<long long>(i) * total + at);
+    dw[(static_cast<long long>(o) * f.C + c) * f.kh * f.kw + t] = s;
   }
 }
 
@@ -118,9 +166,10 @@ s2d_to_nchw_kernel(const float* __restrict__ z, float* __restrict__ x, const S2d
   for (int k = 0; k < 4; ++k) {
     const int j = j0 + ty + 8 * k, c = c0 + tx;
     float v = 0.f;
-    if (I < g.Hz && j < g.W && c < g.C) {
+    if (I < g.Hz && rh < g.eh && j < g.W && c < g.C) {
       const int J = (j + g.pw) / g.sw, rw = (j + g.pw) % g.sw;
-      if (J < g.Wz) v = z[((b * g.Hz + I) * g.Wz + J) * g.ld + static_cast<long long>(rh * g.sw + rw) * g.C + c];
+      if (J < g.Wz && rw < g.ew)
+        v = z[((b * g.Hz + I) * g.Wz + J) * g.ld + static_cast<long long>(rh * g.ew + rw) * g.C + c];
     }
     tile[ty + 8 * k][tx] = v;
   }
@@ -133,49 +182,150 @@ s2d_to_nchw_kernel(const float* __restrict__ z, float* __restrict__ x, const S2d
   }
 }
 
+// y[b, c, p] = act(x[b, p, c] + add[b, c, p]): blocks of 64 pixels x 64 channels.  The addition of a residual and a ReLU
+// cost their reads beside the transposition, no pass of their own.
+__global__ void __launch_bounds__(256)
+nhwc_to_nchw_f32_kernel(const float* __restrict__ x, const float* __restrict__ add, float* __restrict__ y, int C, long long P,
+                        long long ld, int relu, int p_tiles) {
+  __shared__ float tile[64][65];
+  const long long b = blockIdx.x / p_tiles, p0 = static_cast<long long>(blockIdx.x % p_tiles) * 64;
+  const int c0 = blockIdx.y * 64;
+  const bool vec = ld % 4 == 0 && C % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  const float* xb = x + b * P * ld;
+  if (vec) {
+    const int c = (threadIdx.x & 15) * 4, pr = threadIdx.x >> 4;
+    float4 v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const long long p = p0 + pr + 16 * k;
+      v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (p < P && c0 + c < C) v[k] = __ldg(reinterpret_cast<const float4*>(xb + p * ld + c0 + c));
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      tile[c][pr + 16 * k] = v[k].x;
+      tile[c + 1][pr + 16 * k] = v[k].y;
+      tile[c + 2][pr + 16 * k] = v[k].z;
+      tile[c + 3][pr + 16 * k] = v[k].w;
+    }
+  } else {
+    const int c = threadIdx.x & 63, pr = threadIdx.x >> 6;
+    for (int k = 0; k < 16; ++k) {
+      const long long p = p0 + pr + 4 * k;
+      tile[c][pr + 4 * k] = p < P && c0 + c < C ? xb[p * ld + c0 + c] : 0.f;
+    }
+  }
+  __syncthreads();
+  const int px = threadIdx.x & 63, cr = threadIdx.x >> 6;
+  const long long p = p0 + px;
+  if (p >= P) return;
+  const long long at = (b * C + c0) * P + p;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float r[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int c = cr + 4 * (h * 8 + k);
+      r[k] = add != nullptr && c0 + c < C ? __ldg(add + at + c * P) : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int c = cr + 4 * (h * 8 + k);
+      if (c0 + c >= C) continue;
+      float v = tile[c][px];
+      if (add != nullptr) v += r[k];
+      if (relu) v = fmaxf(v, 0.f);
+      y[at + c * P] = v;
+    }
+  }
+}
+
 bool s2d_ok(int B, const S2d& g) {
-  return B > 0 && g.C > 0 && g.H > 0 && g.W > 0 && g.sh > 0 && g.sw > 0 && g.ph >= 0 && g.pw >= 0 && g.Hz > 0 &&
-         g.Wz > 0 && g.ld >= static_cast<long long>(g.sh) * g.sw * g.C && static_cast<long long>(B) * g.H < 0x7fffffffll &&
+  return B > 0 && g.C > 0 && g.H > 0 && g.W > 0 && g.sh > 0 && g.sw > 0 && g.eh > 0 && g.eh <= g.sh && g.ew > 0 &&
+         g.ew <= g.sw && g.ph >= 0 && g.pw >= 0 && g.Hz > 0 && g.Wz > 0 &&
+         g.ld >= static_cast<long long>(g.eh) * g.ew * g.C && static_cast<long long>(B) * g.H < 0x7fffffffll &&
          (g.W + 31) / 32 <= 65535 && (g.C + 31) / 32 <= 65535;
+}
+
+// Elements of a filter matrix of `rows` rows, 0 where the kernels' 32-bit indices would not do.
+int filter_total(const Filter& f, int rows) {
+  if (f.O <= 0 || f.C <= 0 || f.kh <= 0 || f.kw <= 0 || f.sh <= 0 || f.sw <= 0 || f.eh <= 0 || f.ew <= 0) return 0;
+  const long long n = static_cast<long long>(rows) * f.k2h * f.k2w * f.pitch;
+  return n > 0 && n < 0x7f000000ll ? static_cast<int>(n) : 0;
 }
 
 }  // namespace
 }  // namespace fb
 
-// z (bf16, [B, Hz, Wz, ld]) is zeroed first: pixels outside the image and channels sh * sw * C .. ld - 1 stay zero.
-extern "C" int fb_nchw_to_s2d_nhwc_bf16(const float* x, void* z, int B, int C, int H, int W, int sh, int sw, int ph,
-                                        int pw, int Hz, int Wz, long long ld, cudaStream_t stream) {
-  const fb::S2d g{C, H, W, sh, sw, ph, pw, Hz, Wz, ld};
+// x [B, C, H, W] fp32 -> z [B, Hz, Wz, ld] bf16, every element of it written.  mask (optional): x is the gradient behind
+// a ReLU whose result was mask.
+extern "C" int fb_conv_pack_input(const float* x, const float* mask, void* z, int B, int C, int H, int W, int sh, int sw,
+                                  int eh, int ew, int ph, int pw, int Hz, int Wz, long long ld, cudaStream_t stream) {
+  fb::S2d g{C, H, W, sh, sw, eh, ew, ph, pw, Hz, Wz, ld};
   if (!fb::s2d_ok(B, g)) return -1;
-  cudaError_t e = cudaMemsetAsync(z, 0, static_cast<size_t>(B) * Hz * Wz * ld * 2, stream);
-  if (e != cudaSuccess) return static_cast<int>(e);
-  dim3 grid(static_cast<unsigned>(B) * H, static_cast<unsigned>((W + 31) / 32), static_cast<unsigned>((C + 31) / 32));
-  fb::nchw_to_s2d_kernel<<<grid, 256, 0, stream>>>(x, static_cast<__nv_bfloat16*>(z), g);
+  const bool plain = sh == 1 && sw == 1 && ph == 0 && pw == 0 && Hz == H && Wz == W;
+  if (plain && static_cast<long long>(H) * W < 0x7fffffffll - 64) {  // rows are contiguous: one long row per image
+    g.W = g.Wz = H * W;
+    g.H = g.Hz = 1;
+  }
+  const long long q_tiles = (static_cast<long long>(g.Wz) * ew + fb::kTileQ - 1) / fb::kTileQ;
+  const long long blocks = q_tiles * B * g.Hz * eh;
+  if (blocks > 0x7fffffffll) return -1;
+  const dim3 grid(static_cast<unsigned>(blocks), static_cast<unsigned>((C + fb::kTileC - 1) / fb::kTileC));
+  const bool vec = C % 8 == 0 && ld == static_cast<long long>(eh) * ew * C && reinterpret_cast<uintptr_t>(z) % 16 == 0;
+  if (vec)
+    fb::pack_input_kernel<true><<<grid, 256, 0, stream>>>(x, mask, static_cast<__nv_bfloat16*>(z), g,
+                                                          static_cast<int>(q_tiles));
+  else
+    fb::pack_input_kernel<false><<<grid, 256, 0, stream>>>(x, mask, static_cast<__nv_bfloat16*>(z), g,
+                                                           static_cast<int>(q_tiles));
   return static_cast<int>(cudaGetLastError());
 }
 
-// x[b, c, i, j] = z[b, (i + ph) / sh, (j + pw) / sw, (((i + ph) % sh) * sw + (j + pw) % sw) * C + c], zero where no
+// dgrad = 0: out [O, k2h * k2w, pitch], dgrad = 1: out [eh * ew * C, k2h * k2w, pitch] with the taps in reverse order.
+extern "C" int fb_conv_pack_filters(const float* w, void* out, int O, int C, int kh, int kw, int sh, int sw, int eh,
+                                    int ew, int pitch, int dgrad, cudaStream_t stream) {
+  if (sh <= 0 || sw <= 0) return -1;
+  const fb::Filter f{O, C, kh, kw, sh, sw, eh, ew, (kh + sh - 1) / sh, (kw + sw - 1) / sw, pitch};
+  const int rows = dgrad ? eh * ew * C : O, total = fb::filter_total(f, rows);
+  if (total == 0 || pitch < (dgrad ? O : eh * ew * C)) return -1;
+  const int blocks = (total + 255) / 256, grid = blocks < 1184 ? blocks : 1184;
+  if (dgrad)
+    fb::pack_filters_kernel<true><<<grid, 256, 0, stream>>>(w, static_cast<__nv_bfloat16*>(out), f, total);
+  else
+    fb::pack_filters_kernel<false><<<grid, 256, 0, stream>>>(w, static_cast<__nv_bfloat16*>(out), f, total);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// part [splits, O, k2h * k2w, pitch] -> dw [O, C, kh, kw].
+extern "C" int fb_conv_fold_wgrad(const float* part, float* dw, int splits, int O, int C, int kh, int kw, int sh, int sw,
+                                  int eh, int ew, int pitch, cudaStream_t stream) {
+  if (sh <= 0 || sw <= 0) return -1;
+  const fb::Filter f{O, C, kh, kw, sh, sw, eh, ew, (kh + sh - 1) / sh, (kw + sw - 1) / sw, pitch};
+  const int total = fb::filter_total(f, O);
+  if (total == 0 || splits <= 0 || pitch < eh * ew * C) return -1;
+  const int blocks = (total + 255) / 256, grid = blocks < 1184 ? blocks : 1184;
+  fb::fold_wgrad_kernel<<<grid, 256, 0, stream>>>(part, dw, f, splits, total);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// x[b, c, i, j] = z[b, (i + ph) / sh, (j + pw) / sw, (((i + ph) % sh) * ew + (j + pw) % sw) * C + c], zero where no
 // window reaches.
-extern "C" int fb_s2d_nhwc_to_nchw_f32(const float* z, float* x, int B, int C, int H, int W, int sh, int sw, int ph,
-                                       int pw, int Hz, int Wz, long long ld, cudaStream_t stream) {
-  const fb::S2d g{C, H, W, sh, sw, ph, pw, Hz, Wz, ld};
+extern "C" int fb_s2d_nhwc_to_nchw_f32(const float* z, float* x, int B, int C, int H, int W, int sh, int sw, int eh,
+                                       int ew, int ph, int pw, int Hz, int Wz, long long ld, cudaStream_t stream) {
+  const fb::S2d g{C, H, W, sh, sw, eh, ew, ph, pw, Hz, Wz, ld};
   if (!fb::s2d_ok(B, g)) return -1;
   dim3 grid(static_cast<unsigned>(B) * H, static_cast<unsigned>((W + 31) / 32), static_cast<unsigned>((C + 31) / 32));
   fb::s2d_to_nchw_kernel<<<grid, 256, 0, stream>>>(z, x, g);
   return static_cast<int>(cudaGetLastError());
 }
 
-extern "C" int fb_nchw_to_nhwc_bf16(const float* x, void* y, int B, int C, long long P, int Cp, cudaStream_t stream) {
-  if (B <= 0 || C <= 0 || P <= 0 || Cp < C || B > 65535 || (Cp + 31) / 32 > 65535) return -1;
-  dim3 grid(static_cast<unsigned>((P + 31) / 32), static_cast<unsigned>((Cp + 31) / 32), static_cast<unsigned>(B));
-  fb::nchw_to_nhwc_bf16_kernel<<<grid, 256, 0, stream>>>(x, static_cast<__nv_bfloat16*>(y), C, P, Cp);
-  return static_cast<int>(cudaGetLastError());
-}
-
-extern "C" int fb_nhwc_to_nchw_f32(const float* x, float* y, int B, int C, long long P, long long ld,
-                                   cudaStream_t stream) {
-  if (B <= 0 || C <= 0 || P <= 0 || ld < C || B > 65535 || (C + 31) / 32 > 65535) return -1;
-  dim3 grid(static_cast<unsigned>((P + 31) / 32), static_cast<unsigned>((C + 31) / 32), static_cast<unsigned>(B));
-  fb::nhwc_to_nchw_f32_kernel<<<grid, 256, 0, stream>>>(x, y, C, P, ld);
+// y [B, C, P] = x [B, P, ld] (first C channels), plus add [B, C, P] (optional), behind a ReLU with relu = 1.
+extern "C" int fb_nhwc_to_nchw_f32(const float* x, const float* add, float* y, int B, int C, long long P, long long ld,
+                                   int relu, cudaStream_t stream) {
+  const long long tiles = (P + 63) / 64;
+  if (B <= 0 || C <= 0 || P <= 0 || ld < C || tiles * B > 0x7fffffffll || (C + 63) / 64 > 65535) return -1;
+  const dim3 grid(static_cast<unsigned>(tiles * B), static_cast<unsigned>((C + 63) / 64));
+  fb::nhwc_to_nchw_f32_kernel<<<grid, 256, 0, stream>>>(x, add, y, C, P, ld, relu, static_cast<int>(tiles));
   return static_cast<int>(cudaGetLastError());
 }

@@ -256,5 +256,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   bind_linear(m);
   bind_elementwise(m);
   bind_layers(m);
+  bind_conv(m);
   bind_optim(m);
 }

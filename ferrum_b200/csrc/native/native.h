@@ -151,6 +151,7 @@ void sink_ready(Sink& s);
 void bind_linear(py::module_& m);
 void bind_elementwise(py::module_& m);
 void bind_layers(py::module_& m);
+void bind_conv(py::module_& m);
 void bind_optim(py::module_& m);
 
 }  // namespace fbn

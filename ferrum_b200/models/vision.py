@@ -7,7 +7,7 @@ from __future__ import annotations
 import torch
 
 from .. import nn
-from ..nn.conv import AdaptiveAvgPool2d, Conv2d, MaxPool2d
+from ..nn.conv import AdaptiveAvgPool2d, Conv2d, MaxPool2d, conv_fused
 from ..ops import functional as F
 
 
@@ -26,8 +26,8 @@ class BasicBlock(nn.Module):
     @nn.tensor_io
     def forward(self, x):
         identity = self.downsample(x) if self.downsample is not None else x
-        y = self.conv2(F.unary(self.conv1(x), "relu"))
-        return F.unary(F.binary(y, identity, "add"), "relu")
+        y = conv_fused(self.conv1, x, act="relu")
+        return F.unary(conv_fused(self.conv2, y, add=identity), "relu")
 
 
 class ResNet(nn.Module):

@@ -1,9 +1,9 @@
 """Convolutions and pooling (ferrum-nn/src/conv.rs:9-497; forward-only host loops there).
 
 Under bf16 autocast an ungrouped convolution runs as an implicit GEMM on the tensor cores in all three directions
-(``ops.functional._ConvIgemmFn``: NHWC bf16 activations read through 4-D TMA boxes shifted by the filter tap, no
-window matrix in memory; strided convolutions reach the same kernels through a space-to-depth layout,
-``_ConvS2dFn``; stride together with dilation takes the explicit path).  Otherwise convolution is lowered to GEMM explicitly: an im2col kernel writes the input windows as a K-major matrix (one row per output
+(``ops.functional.conv2d_igemm``: NHWC bf16 activations read through 4-D TMA boxes shifted by the filter tap, no
+window matrix in memory; strided convolutions reach the same kernels through a space-to-depth layout; stride together
+with dilation takes the explicit path).  Otherwise convolution is lowered to GEMM explicitly: an im2col kernel writes the input windows as a K-major matrix (one row per output
 position) and the product with the flattened filters runs on this package's GEMM kernels (tcgen05 under bf16
 autocast, fp32 SIMT otherwise); the backward is the dgrad / wgrad GEMMs plus a gather-form col2im kernel.  Groups,
 dilation, stride and padding follow the reference; weights ~ U(+-1/sqrt(fan_in)).  Max / average pooling are
@@ -91,6 +91,31 @@ class Conv2d(Module):
         if x.dim() != 4:
             raise ShapeMismatch("Conv2d.forward", "[B, C, H, W]", list(x.shape))
         return conv2d(x, self.weight, self.bias, self._stride, self._padding, self.dilation, self.groups)
+
+
+def _bare(m) -> bool:
+    """True when calling ``m`` runs ``Conv2d.forward`` and nothing else: no subclass, no hooks."""
+    g = torch.nn.modules.module
+    return (type(m) is Conv2d and "forward" not in m.__dict__
+            and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+                     or g._global_forward_hooks or g._global_forward_pre_hooks or g._global_backward_hooks
+                     or g._global_backward_pre_hooks))
+
+
+def conv_fused(conv, x, add=None, act=None):
+    """``act(conv(x))`` (``act``: "relu") or ``conv(x) + add``, in the convolution's last kernel where that runs as an
+    implicit GEMM, else as ops of their own."""
+    w = conv.weight
+    if (_bare(conv) and x.dim() == 4 and x.shape[1] == w.shape[1] * conv.groups
+            and F.conv_igemm_ok(x, conv._stride, conv.dilation, conv._padding, conv.kernel_size, conv.groups)):
+        size = (x.shape[0], w.shape[0]) + _out_hw(x, conv.kernel_size, conv._stride, conv._padding, conv.dilation)
+        if add is None or (tuple(add.shape) == size and add.device == x.device
+                           and add.dtype in (torch.float32, torch.bfloat16)):
+            return F.conv2d_igemm(x, w, conv.bias, conv._padding, conv.dilation, conv._stride, add, act)
+    y = conv(x)
+    if add is not None:
+        y = F.binary(y, add, "add")
+    return y if act is None else F.unary(y, act)
 
 
 class Conv1d(Module):

@@ -1061,88 +1061,12 @@ def _pad8(n: int) -> int:
     return (n + 7) // 8 * 8
 
 
-def _to_nhwc_bf16(x: torch.Tensor) -> torch.Tensor:
-    """[B, C, H, W] fp32 -> [B, H, W, Cp] bf16 with the channels padded by zeros to a multiple of 8."""
-    x = _f32(x).contiguous()
-    B, C, H, W = x.shape
-    y = torch.empty((B, H, W, _pad8(C)), device=x.device, dtype=torch.bfloat16)
-    _lib.check(_lib.cuda().fb_nchw_to_nhwc_bf16(x.data_ptr(), y.data_ptr(), B, C, H * W, y.shape[3], _stream()),
-               "fb_nchw_to_nhwc_bf16")
-    return y
-
-
-def _to_nchw_f32(y: torch.Tensor, C: int) -> torch.Tensor:
-    """[B, H, W, ld] fp32 (first C channels) -> [B, C, H, W] fp32."""
-    B, H, W, ld = y.shape
-    out = torch.empty((B, C, H, W), device=y.device, dtype=torch.float32)
-    _lib.check(_lib.cuda().fb_nhwc_to_nchw_f32(y.data_ptr(), out.data_ptr(), B, C, H * W, ld, _stream()),
-               "fb_nhwc_to_nchw_f32")
-    return out
-
-
-def _conv_igemm(xh: torch.Tensor, wk: torch.Tensor, bias, O: int, kernel, padding, dilation) -> torch.Tensor:
-    """NHWC bf16 ``xh`` [B, H, W, Cp] * ``wk`` [O, kh * kw * Cp] -> NHWC fp32 [B, Ho, Wo, O] on the tensor cores."""
-    B, H, W, Cp = xh.shape
-    (kh, kw), (ph, pw), (dh, dw) = kernel, padding, dilation
-    Ho, Wo = H + 2 * ph - dh * (kh - 1), W + 2 * pw - dw * (kw - 1)
-    y = torch.empty((B, Ho, Wo, O), device=xh.device, dtype=torch.float32)
-    _lib.check(_lib.cuda().fb_conv_igemm(xh.data_ptr(), wk.data_ptr(), y.data_ptr(), _ptr(bias), B, H, W, Cp, O, kh,
-                                         kw, ph, pw, dh, dw, O, 0, _rt.status_ptr(), _stream()), "fb_conv_igemm")
-    return y
-
-
-class _ConvIgemmFn(Function):
-    """Stride-1, ungrouped 2-D convolution without a window matrix (csrc/gemm/tcgen05_gemm.cu, conv forms): all three
-    products — forward, data gradient, weight gradient — read NHWC bf16 activations through 4-D TMA boxes shifted by
-    the filter tap (zero fill = padding) and run on tcgen05.  Counterpart of the reference's direct loops
-    (ferrum-nn/src/conv.rs:209-330)."""
-
-    @staticmethod
-    def forward(ctx, x, weight, bias, padding, dilation):
-        B, C, H, W = x.shape
-        O, _, kh, kw = weight.shape
-        xh = _to_nhwc_bf16(x)                                              # [B, H, W, Cp]
-        wk = _to_nhwc_bf16(weight.detach()).reshape(O, -1)                 # [O, kh * kw * Cp]
-        b = _f32(bias.detach()).contiguous() if bias is not None else None
-        y = _conv_igemm(xh, wk, b, O, (kh, kw), padding, dilation)
-        ctx.save_for_backward(xh, weight)
-        ctx.geom = (C, tuple(padding), tuple(dilation), bias is not None)
-        return _to_nchw_f32(y, O)
-
-    @staticmethod
-    def backward(ctx, g):
-        xh, weight = ctx.saved_tensors
-        C, (ph, pw), (dh, dw), has_bias = ctx.geom
-        B, H, W, Cp = xh.shape
-        O, _, kh, kw = weight.shape
-        gh = _to_nhwc_bf16(g)                                              # [B, Ho, Wo, Op]
-        Op = gh.shape[3]
-        dx = dwt = db = None
-        if ctx.needs_input_grad[0]:
-            # dx = dy convolved with the filters flipped in both directions and input / output channels exchanged
-            wt = _to_nhwc_bf16(weight.detach().transpose(0, 1).flip(2, 3)).reshape(C, -1)   # [C, kh * kw * Op]
-            dxh = _conv_igemm(gh, wt, None, C, (kh, kw), (dh * (kh - 1) - ph, dw * (kw - 1) - pw), (dh, dw))
-            dx = _to_nchw_f32(dxh, C)
-        if ctx.needs_input_grad[1]:
-            lib = _lib.cuda()
-            Ho, Wo = gh.shape[1], gh.shape[2]
-            splits = lib.fb_conv_wgrad_splits(B, Ho, Wo, O, Cp, kh * kw)
-            part = torch.empty((splits, O, kh * kw * Cp), device=g.device, dtype=torch.float32)
-            _lib.check(lib.fb_conv_wgrad(gh.data_ptr(), xh.data_ptr(), part.data_ptr(), B, H, W, Cp, O, Op, kh, kw, ph,
-                                         pw, dh, dw, _rt.status_ptr(), _stream()), "fb_conv_wgrad")
-            full = raw_reduce(part, "sum", 0) if splits > 1 else part[0]
-            dwt = full.reshape(O, kh, kw, Cp)[..., :C].permute(0, 3, 1, 2).contiguous()
-        if has_bias and ctx.needs_input_grad[2]:
-            db = raw_colsum(gh.reshape(-1, Op))[:O]
-        return dx, dwt, db, None, None
-
-
-class _ConvS2dFn(Function):
-    """Strided, undilated, ungrouped 2-D convolution on the implicit-GEMM kernels: the input goes through a
-    space-to-depth layout change (``z[b, I, J, (rh, rw, c)] = x[b, c, I * sh + rh - ph, J * sw + rw - pw]``), after
-    which the stride-(sh, sw) convolution with a kh x kw filter IS a stride-1 convolution with a
-    ceil(kh / sh) x ceil(kw / sw) filter over sh * sw * C channels (filter taps that do not exist are zero).  A
-    patch embedding (kernel = stride) becomes one plain GEMM."""
+class _ConvS2dFn:
+    """The space-to-depth form of a strided convolution in plain torch: with
+    ``z[b, I, J, (rh, rw, c)] = x[b, c, I * sh + rh - ph, J * sw + rw - pw]`` the stride-(sh, sw) convolution with a
+    kh x kw filter IS a stride-1 convolution with a ceil(kh / sh) x ceil(kw / sw) filter over sh * sw * C channels (filter
+    taps that do not exist are zero).  What csrc/kernels/conv_layout.cu does on the GPU; there, rows and columns that the
+    stride skips altogether are left out."""
 
     @staticmethod
     def _geometry(x_shape, w_shape, stride, padding):
@@ -1165,54 +1089,6 @@ class _ConvS2dFn(Function):
         out[..., :sh * sw * C] = w
         return out
 
-    @staticmethod
-    def forward(ctx, x, weight, bias, stride, padding):
-        x = _f32(x).contiguous()
-        B, C, H, W = x.shape
-        O = weight.shape[0]
-        (sh, sw), (ph, pw) = stride, padding
-        Ho, Wo, k2h, k2w, Hz, Wz, Cz = _ConvS2dFn._geometry(x.shape, weight.shape, stride, padding)
-        z = torch.empty((B, Hz, Wz, Cz), device=x.device, dtype=torch.bfloat16)
-        _lib.check(_lib.cuda().fb_nchw_to_s2d_nhwc_bf16(x.data_ptr(), z.data_ptr(), B, C, H, W, sh, sw, ph, pw, Hz, Wz,
-                                                        Cz, _stream()), "fb_nchw_to_s2d_nhwc_bf16")
-        w2 = _ConvS2dFn._filters(weight, stride, k2h, k2w, Cz)
-        b = _f32(bias.detach()).contiguous() if bias is not None else None
-        y = _conv_igemm(z, w2.reshape(O, -1).to(torch.bfloat16), b, O, (k2h, k2w), (0, 0), (1, 1))
-        ctx.save_for_backward(z, weight)
-        ctx.geom = (x.shape, tuple(stride), tuple(padding), bias is not None)
-        return _to_nchw_f32(y, O)
-
-    @staticmethod
-    def backward(ctx, g):
-        z, weight = ctx.saved_tensors
-        x_shape, (sh, sw), (ph, pw), has_bias = ctx.geom
-        B, C, H, W = x_shape
-        O, _, kh, kw = weight.shape
-        Ho, Wo, k2h, k2w, Hz, Wz, Cz = _ConvS2dFn._geometry(x_shape, weight.shape, (sh, sw), (ph, pw))
-        gh = _to_nhwc_bf16(g)                                              # [B, Ho, Wo, Op]
-        Op = gh.shape[3]
-        lib = _lib.cuda()
-        dx = dwt = db = None
-        if ctx.needs_input_grad[0]:
-            w2 = _ConvS2dFn._filters(weight, (sh, sw), k2h, k2w, Cz)       # [O, k2h, k2w, Cz]
-            wt = torch.zeros((Cz, k2h, k2w, Op), device=g.device, dtype=torch.float32)
-            wt[..., :O] = w2.permute(3, 1, 2, 0).flip(1, 2)
-            dz = _conv_igemm(gh, wt.reshape(Cz, -1).to(torch.bfloat16), None, Cz, (k2h, k2w), (k2h - 1, k2w - 1), (1, 1))
-            dx = torch.empty(x_shape, device=g.device, dtype=torch.float32)
-            _lib.check(lib.fb_s2d_nhwc_to_nchw_f32(dz.data_ptr(), dx.data_ptr(), B, C, H, W, sh, sw, ph, pw, Hz, Wz, Cz,
-                                                   _stream()), "fb_s2d_nhwc_to_nchw_f32")
-        if ctx.needs_input_grad[1]:
-            splits = lib.fb_conv_wgrad_splits(B, Ho, Wo, O, Cz, k2h * k2w)
-            part = torch.empty((splits, O, k2h * k2w * Cz), device=g.device, dtype=torch.float32)
-            _lib.check(lib.fb_conv_wgrad(gh.data_ptr(), z.data_ptr(), part.data_ptr(), B, Hz, Wz, Cz, O, Op, k2h, k2w, 0, 0,
-                                         1, 1, _rt.status_ptr(), _stream()), "fb_conv_wgrad")
-            full = raw_reduce(part, "sum", 0) if splits > 1 else part[0]
-            d2 = full.reshape(O, k2h, k2w, Cz)[..., :sh * sw * C].reshape(O, k2h, k2w, sh, sw, C)
-            dwt = d2.permute(0, 5, 1, 3, 2, 4).reshape(O, C, k2h * sh, k2w * sw)[:, :, :kh, :kw].contiguous()
-        if has_bias and ctx.needs_input_grad[2]:
-            db = raw_colsum(gh.reshape(-1, Op))[:O]
-        return dx, dwt, db, None, None
-
 
 def conv_igemm_ok(x: torch.Tensor, stride, dilation, padding, kernel, groups: int) -> bool:
     """True when ``conv2d`` can take the implicit-GEMM path: CUDA, bf16 autocast on, one group, and either stride 1
@@ -1225,10 +1101,12 @@ def conv_igemm_ok(x: torch.Tensor, stride, dilation, padding, kernel, groups: in
     return tuple(dilation) == (1, 1) and padding[0] >= 0 and padding[1] >= 0
 
 
-def conv2d_igemm(x, weight, bias, padding=(0, 0), dilation=(1, 1), stride=(1, 1)):
-    if tuple(stride) != (1, 1):
-        return _ConvS2dFn.apply(x, weight, bias, tuple(stride), tuple(padding))
-    return _ConvIgemmFn.apply(x, weight, bias, tuple(padding), tuple(dilation))
+def conv2d_igemm(x, weight, bias, padding=(0, 0), dilation=(1, 1), stride=(1, 1), add=None, act=None):
+    """``act(conv(x))`` or ``conv(x) + add`` as one node (csrc/native/conv.cpp) where :func:`conv_igemm_ok` says so.  All
+    three products read NHWC bf16 activations through 4-D TMA boxes shifted by the filter tap (no window matrix); strides
+    are gone after a space-to-depth layout.  ``act``: None or "relu".  Counterpart of the reference's direct loops
+    (ferrum-nn/src/conv.rs:209-330)."""
+    return _lib.native().conv2d(x, weight, bias, add, stride, padding, dilation, _gemm.ACT[act])
 
 
 def im2col(x, kernel, stride=(1, 1), padding=(0, 0), dilation=(1, 1)):

@@ -1,0 +1,83 @@
+"""Convolutions as implicit GEMMs with what is fused around them: a ReLU, an added tensor, strides larger than the kernel,
+channel counts that are no multiple of 8.  Against an fp64 convolution of the bf16-rounded operands.
+
+Bound: products of bf16 numbers are exact in fp32 and at most a few thousand are added (1e-5 of the norm); gradients pass
+through one more bf16 rounding of the incoming gradient, which the reference makes, too."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _r16(t):
+    return t.bfloat16().double()
+
+
+def _close(got, want):
+    assert (got.double() - want).norm() <= 2e-5 * want.norm() + 1e-6
+
+
+@pytest.mark.parametrize("fused", [None, "relu", "add"])
+@pytest.mark.parametrize("B,C,O,H,W,k,stride,pad,dil", [
+    (2, 8, 16, 9, 11, (3, 3), (1, 1), (1, 1), (1, 1)), (1, 3, 5, 17, 19, (3, 3), (2, 2), (1, 1), (1, 1)),
+    (3, 64, 130, 28, 28, (1, 1), (2, 2), (0, 0), (1, 1)), (2, 65, 64, 14, 13, (2, 1), (3, 2), (1, 0), (1, 1)),
+    (1, 128, 72, 7, 70, (3, 3), (1, 1), (2, 2), (2, 2)), (2, 12, 24, 33, 31, (5, 3), (2, 3), (2, 1), (1, 1)),
+    (1, 24, 8, 32, 32, (4, 4), (4, 4), (0, 0), (1, 1)), (1, 1, 1, 1, 1, (1, 1), (1, 1), (0, 0), (1, 1))])
+def test_forward_and_backward(B, C, O, H, W, k, stride, pad, dil, fused):
+    import ferrum_b200 as fb
+    from ferrum_b200.ops import functional as F
+    from ferrum_b200.utils.runtime import check_status
+
+    g = torch.Generator(device="cuda").manual_seed(C + O + H)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x, w, b = rand(B, C, H, W).requires_grad_(True), (rand(O, C, *k) * 0.1).requires_grad_(True), rand(O).requires_grad_(True)
+    xd, wd, bd = _r16(x.detach()).requires_grad_(True), _r16(w.detach()).requires_grad_(True), b.detach().double().requires_grad_(True)
+    zd = torch.nn.functional.conv2d(xd, wd, bd, stride, pad, dil)
+    add = rand(*zd.shape).requires_grad_(True) if fused == "add" else None
+    with fb.autocast():
+        assert F.conv_igemm_ok(x, stride, dil, pad, k, 1)
+        y = F.conv2d_igemm(x, w, b, pad, dil, stride, add, "relu" if fused == "relu" else None)
+    gy = rand(*zd.shape)
+    if fused == "relu":
+        kept = y.detach() > 0  # next to zero either side is right
+        yd, gd = zd * kept, gy * kept
+        assert zd.detach()[kept != (zd > 0)].abs().sum() < 1e-3
+    else:
+        yd, gd = zd + (add.detach().double() if add is not None else 0), gy
+    _close(y.detach(), yd.detach())
+    y.backward(gy)
+    zd.backward(_r16(gd))
+    check_status()
+    for got, want in ((x.grad, xd.grad), (w.grad, wd.grad)):
+        _close(got, want)
+    # the bias gradient is a sum of the bf16-rounded gradient
+    _close(b.grad, bd.grad)
+    if add is not None:
+        assert torch.equal(add.grad, gy)
+
+
+def test_block_with_hooks():
+    """The residual block fuses only convolutions that nobody looks at."""
+    import ferrum_b200 as fb
+    from ferrum_b200.models import BasicBlock
+
+    torch.manual_seed(0)
+    block = BasicBlock(8, 16, 2, device=fb.Device.Cuda(0))
+    x = torch.randn(2, 8, 14, 14, device="cuda")
+    with fb.autocast():
+        block(x).sum().backward()
+    grads = [p.grad.clone() for p in block.torch_parameters()]
+    seen = []
+    hooks = [c.register_forward_hook(lambda m, i, o: seen.append(tuple(o.shape))) for c in (block.conv1, block.conv2)]
+    for p in block.torch_parameters():
+        p.grad = None
+    with fb.autocast():
+        got = block(x)
+        loss = got.sum()
+    got.detach().mul_(0.0)  # the output is the caller's
+    loss.backward()
+    assert seen == [(2, 16, 7, 7)] * 2
+    for p, g in zip(block.torch_parameters(), grads):
+        assert torch.equal(p.grad, g)
+    for h in hooks:
+        h.remove()
