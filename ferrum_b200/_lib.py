@@ -141,6 +141,7 @@ _CUDA_SIGS = {
     "fb_unary_bwd": (I, [P, P, P, LL, I, F, F, I, P]),
     "fb_binary_fwd": (I, [P, P, P, I, I, POINTER(LL), POINTER(LL), POINTER(LL), P]),
     "fb_cast": (I, [P, P, LL, I, I, P]),
+    "fb_repack_rows": (I, [P, P, LL, I, LL, P, P, LL, I, LL, P]),
     "fb_transpose_2d": (I, [P, P, I, I, I, P]),
     # reductions
     "fb_reduce_scratch_elems": (LL, [LL, LL, LL]),

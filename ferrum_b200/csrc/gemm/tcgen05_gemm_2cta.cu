@@ -25,7 +25,7 @@
 // result is accumulated into an existing fp32 matrix).  Global memory therefore sees whole 128-byte lines instead of
 // 16-byte pieces of 32 different rows, and the warp is free for the next slab while the copy drains; each warp
 // double-buffers its slab (bulk groups, wait_group.read before a buffer is rewritten).  Results whose base or row
-// pitch is not 16-byte aligned leave through plain register stores.
+// pitch is not 16-byte aligned leave through plain stores, a row of 32 columns per instruction.
 // Every wait is bounded; the two cluster barriers (after set-up, before exit) are
 // reached on every path, including the abort path.
 #include <cuda.h>
@@ -76,7 +76,7 @@ struct Args2 {
   int out_bf16;
   int act;
   int beta;
-  int out_mode;  // kOutTma: slabs leave through the TMA unit; kOutRegs: register stores (unaligned results); kOutPush
+  int out_mode;  // kOutTma: slabs leave through the TMA unit; kOutRegs: plain stores (unaligned results); kOutPush
   int group_m;   // pair-tiles (256 rows) per rasterisation group
   int32_t* status;
   unsigned long long timeout_ns;
@@ -301,8 +301,6 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     const int quarter = warp & 3;          // TMEM lanes a warp may read: 32 * (warp % 4) ...
     int acc = 0;
     uint32_t acc_phase = 0;
-    const bool vec_ok = ((p.ldc * (p.out_bf16 ? 2 : 4)) % 16 == 0) &&
-                        ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0);
     uint8_t* my_slabs = slab_base + (warp - 2) * (2 * kSlabBytes);
     const uint32_t slab_u32 = ptx::smem_u32(my_slabs);
     const uint32_t row_off = static_cast<uint32_t>(lane) * kRowBytes;  // this lane's row inside a slab
@@ -314,7 +312,6 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       int m_blk, n_blk;
       tile_coords2(t, num_m, num_n, p.group_m, m_blk, n_blk);
       const int row_base = m_blk * 2 * kBM + static_cast<int>(rank) * kBM + quarter * 32;  // first of this warp's rows
-      const int row = row_base + lane;
       const int n0 = n_blk * kBN;
       const bool ready = ptx::mbar_wait(&tmem_full[acc], acc_phase, abort_flag, p.timeout_ns);
       const unsigned long long e0 = p.prof ? ptx::globaltimer() : 0;
@@ -444,66 +441,48 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
           }
           continue;
         }
-        // ---- register stores (results the TMA unit cannot address)
-        if (row < p.M && col0 < p.N) {
-          const bool full = (col0 + 32 <= p.N) && vec_ok;
-          if (dual) {
-            // value and derivative of the activation, both stored as bf16
-            __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<long long>(row) * p.ldc + col0;
-            __nv_bfloat16* o2 = reinterpret_cast<__nv_bfloat16*>(p.out2) + static_cast<long long>(row) * p.ldc + col0;
-            float dv[32];
-            act_both_chunk(v, dv, p.act);
-            if (full) {
+        // ---- results the TMA unit cannot address: the 32 x 32 block is turned through the warp's slabs, so that a
+        // store instruction writes 32 neighbouring columns of one row
+        float dv[32];
+        if (dual) act_both_chunk(v, dv, p.act);
+        else if (p.act != FB_ACT_NONE) act_chunk(v, p.act);
+        const auto store_rows = [&](const float (&x)[32], void* out) {
+          __syncwarp();
+          if (p.out_bf16) {
 #pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                reinterpret_cast<uint4*>(o)[q] =
-                    make_uint4(pack_bf16(v[q * 8], v[q * 8 + 1]), pack_bf16(v[q * 8 + 2], v[q * 8 + 3]),
-                               pack_bf16(v[q * 8 + 4], v[q * 8 + 5]), pack_bf16(v[q * 8 + 6], v[q * 8 + 7]));
-                reinterpret_cast<uint4*>(o2)[q] =
-                    make_uint4(pack_bf16(dv[q * 8], dv[q * 8 + 1]), pack_bf16(dv[q * 8 + 2], dv[q * 8 + 3]),
-                               pack_bf16(dv[q * 8 + 4], dv[q * 8 + 5]), pack_bf16(dv[q * 8 + 6], dv[q * 8 + 7]));
-              }
-            } else {
-              for (int i = 0; i < 32; ++i)
-                if (col0 + i < p.N) {
-                  o[i] = __float2bfloat16_rn(v[i]);
-                  o2[i] = __float2bfloat16_rn(dv[i]);
-                }
-            }
+            for (int q = 0; q < 4; ++q)
+              ptx::st_shared_v4(slab_u32 + row_off + ((static_cast<uint32_t>(q) ^ sw) << 4),
+                                pack_bf16(x[q * 8], x[q * 8 + 1]), pack_bf16(x[q * 8 + 2], x[q * 8 + 3]),
+                                pack_bf16(x[q * 8 + 4], x[q * 8 + 5]), pack_bf16(x[q * 8 + 6], x[q * 8 + 7]));
           } else {
-            if (p.act != FB_ACT_NONE) act_chunk(v, p.act);
-            if (p.out_bf16) {
-              __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<long long>(row) * p.ldc + col0;
-              if (full) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q)
-                  reinterpret_cast<uint4*>(o)[q] =
-                      make_uint4(pack_bf16(v[q * 8], v[q * 8 + 1]), pack_bf16(v[q * 8 + 2], v[q * 8 + 3]),
-                                 pack_bf16(v[q * 8 + 4], v[q * 8 + 5]), pack_bf16(v[q * 8 + 6], v[q * 8 + 7]));
-              } else {
-                for (int i = 0; i < 32; ++i)
-                  if (col0 + i < p.N) o[i] = __float2bfloat16_rn(v[i]);
-              }
-            } else {
-              float* o = reinterpret_cast<float*>(p.out) + static_cast<long long>(row) * p.ldc + col0;
-              if (full) {
-                float4* o4 = reinterpret_cast<float4*>(o);
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                  float4 x = make_float4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
-                  if (p.beta) {
-                    const float4 old = o4[q];
-                    x.x += old.x; x.y += old.y; x.z += old.z; x.w += old.w;
-                  }
-                  o4[q] = x;
-                }
-              } else {
-                for (int i = 0; i < 32; ++i)
-                  if (col0 + i < p.N) o[i] = p.beta ? o[i] + v[i] : v[i];
-              }
+            for (int q = 0; q < 8; ++q)
+              ptx::st_shared_v4(slab_u32 + row_off + ((static_cast<uint32_t>(q) ^ sw) << 4), __float_as_uint(x[q * 4]),
+                                __float_as_uint(x[q * 4 + 1]), __float_as_uint(x[q * 4 + 2]),
+                                __float_as_uint(x[q * 4 + 3]));
+          }
+          __syncwarp();
+          const int col = col0 + lane, rows = min(32, p.M - row_base);
+          if (col >= p.N) return;
+          const long long at = static_cast<long long>(row_base) * p.ldc + col;
+          if (p.out_bf16) {
+            __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out) + at;
+#pragma unroll 8
+            for (int rr = 0; rr < rows; ++rr)
+              o[rr * p.ldc] = *reinterpret_cast<const __nv_bfloat16*>(my_slabs + rr * kRowBytes +
+                                                                      (((lane >> 3) ^ (rr & 7)) << 4) + (lane & 7) * 2);
+          } else {
+            float* o = static_cast<float*>(out) + at;
+#pragma unroll 8
+            for (int rr = 0; rr < rows; ++rr) {
+              const float y = *reinterpret_cast<const float*>(my_slabs + rr * kRowBytes + (((lane >> 2) ^ (rr & 7)) << 4) +
+                                                              (lane & 3) * 4);
+              o[rr * p.ldc] = p.beta ? o[rr * p.ldc] + y : y;
             }
           }
-        }
+        };
+        store_rows(v, p.out);
+        if (dual) store_rows(dv, p.out2);
       }
       ptx::tc_fence_before();
       __syncwarp();
@@ -630,7 +609,7 @@ int launch2(const void* a, const void* b, Args2& args, long long lda, long long 
 
 // Arguments every entry point fills the same way.
 void fill_common(Args2& args, int32_t* status) {
-  args.out_mode = kOutTma;  // launch2 falls back to register stores where no map can be built
+  args.out_mode = kOutTma;  // launch2 falls back to plain stores where no map can be built
   args.group_m = g_group_m;
   args.push_world = 0;
   args.push_rank = 0;

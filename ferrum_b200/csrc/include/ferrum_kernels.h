@@ -121,6 +121,8 @@ int fb_unary_bwd(const void* dy, const void* saved, void* dx, long long n, int o
 int fb_binary_fwd(const float* a, const float* b, float* out, int op, int ndim, const long long* shape,
                   const long long* stride_a, const long long* stride_b, cudaStream_t stream);
 int fb_cast(const void* src, void* dst, long long n, int src_dtype, int dst_dtype, cudaStream_t stream);
+int fb_repack_rows(const void* src0, void* dst0, long long rows0, int cols0, long long pitch0, const void* src1, void* dst1,
+                   long long rows1, int cols1, long long pitch1, cudaStream_t stream);
 int fb_transpose_2d(const void* src, void* dst, int rows, int cols, int elem_size, cudaStream_t stream);
 
 // ---- reductions: input viewed as [outer, R, inner] --------------------------

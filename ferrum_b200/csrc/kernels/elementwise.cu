@@ -430,6 +430,52 @@ transpose16_pairs_kernel(const uint16_t* __restrict__ s, uint16_t* __restrict__ 
   }
 }
 
+// Rows of 2-byte elements at any pitch and address -> rows at a pitch that is a multiple of 8 elements, so that a TMA map
+// can describe them; one or two matrices in a launch.  A thread writes one 16-byte piece from the one or two aligned
+// words that cover it in the source (element by element where those reach past the matrix); the padding is zero.  Bound
+// by HBM.
+struct Repack {
+  const uint16_t* src;
+  uint16_t* dst;
+  long long src_pitch, pieces;
+  uintptr_t lo, hi;  // the matrix's first byte and the one behind its last
+  int cols, row_pieces;
+};
+__global__ void __launch_bounds__(256) repack_rows_kernel(const Repack a, const Repack b) {
+  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < a.pieces + b.pieces; i += stride) {
+    const bool second = i >= a.pieces;
+    const Repack& m = second ? b : a;
+    const long long at = second ? i - a.pieces : i, r = at / m.row_pieces;
+    const int c = static_cast<int>(at - r * m.row_pieces) * 8;
+    const uint16_t* p = m.src + r * m.src_pitch + c;
+    const uintptr_t from = reinterpret_cast<uintptr_t>(p), word = from & ~uintptr_t(15);
+    const uint32_t off = static_cast<uint32_t>(from & 15);
+    uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0}, out[4];
+    if (c + 8 <= m.cols && word >= m.lo && word + (off ? 32 : 16) <= m.hi) {
+      const uint4 x = __ldg(reinterpret_cast<const uint4*>(word));
+      w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w;
+      if (off) {
+        const uint4 y = __ldg(reinterpret_cast<const uint4*>(word) + 1);
+        w[4] = y.x; w[5] = y.y; w[6] = y.z; w[7] = y.w;
+      }
+      uint32_t t[6], s[5];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) t[k] = off & 8 ? w[k + 2] : w[k];
+#pragma unroll
+      for (int k = 0; k < 5; ++k) s[k] = off & 4 ? t[k + 1] : t[k];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) out[k] = __funnelshift_r(s[k], s[k + 1], (off & 2) * 8);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) w[k] = c + k < m.cols ? __ldg(p + k) : 0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) out[k] = w[2 * k] | w[2 * k + 1] << 16;
+    }
+    reinterpret_cast<uint4*>(m.dst)[at] = make_uint4(out[0], out[1], out[2], out[3]);
+  }
+}
+
 // y = x * (*scalar): the incoming gradient of a scalar loss applied to a stored gradient, without a host read.
 template <typename T>
 __global__ void scale_by_scalar_kernel(const T* __restrict__ x, const float* __restrict__ scalar, T* __restrict__ y,
@@ -633,5 +679,27 @@ extern "C" int fb_scale_by_device_scalar(const void* x, const float* scalar, voi
         static_cast<const __nv_bfloat16*>(x), scalar, static_cast<__nv_bfloat16*>(y), n);
   else
     return -1;
+  return static_cast<int>(cudaGetLastError());
+}
+
+// dst[r][c] = src[r * pitch + c], rows x cols of 2-byte elements, dst at a pitch of cols rounded up to 8 (16-byte aligned
+// address); src1 NULL: one matrix.
+extern "C" int fb_repack_rows(const void* src0, void* dst0, long long rows0, int cols0, long long pitch0, const void* src1,
+                              void* dst1, long long rows1, int cols1, long long pitch1, cudaStream_t stream) {
+  const auto make = [](const void* src, void* dst, long long rows, int cols, long long pitch) {
+    const uintptr_t lo = reinterpret_cast<uintptr_t>(src);
+    const int row_pieces = (cols + 7) / 8;
+    return Repack{static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), pitch, rows * row_pieces, lo,
+                  lo + ((rows - 1) * pitch + cols) * 2, cols, row_pieces};
+  };
+  const auto bad = [](const void* src, const void* dst, long long rows, int cols, long long pitch) {
+    return src == nullptr || rows <= 0 || cols <= 0 || cols > 0x7ffffff0 || pitch < cols ||
+           reinterpret_cast<uintptr_t>(dst) % 16 != 0 || reinterpret_cast<uintptr_t>(src) % 2 != 0;
+  };
+  if (bad(src0, dst0, rows0, cols0, pitch0)) return -1;
+  if (src1 != nullptr && bad(src1, dst1, rows1, cols1, pitch1)) return -1;
+  const Repack a = make(src0, dst0, rows0, cols0, pitch0);
+  const Repack b = src1 != nullptr ? make(src1, dst1, rows1, cols1, pitch1) : Repack{nullptr, nullptr, 0, 0, 0, 0, 8, 1};
+  repack_rows_kernel<<<grid_for(a.pieces + b.pieces, 256), 256, 0, stream>>>(a, b);
   return static_cast<int>(cudaGetLastError());
 }

@@ -79,16 +79,34 @@ bool tma_ok(const Op& a) {
   return false;
 }
 
-// A bf16 operand that no TMA map describes, laid out again with its reduction (a multiple of 8) contiguous.
-static Op aligned_copy(const Op& o, const at::TensorOptions& opt, Tensor& keep) {
-  if (o.s_row == 1 && o.s_k == o.rows) {  // a contiguous matrix seen transposed: the operands of a weight gradient
-    keep = at::empty({o.rows, o.k}, opt);
-    FB_CALL(fb_transpose_2d, o.p, keep.data_ptr(), static_cast<int>(o.k), static_cast<int>(o.rows), 2, cur_stream());
-  } else {
-    keep = at::from_blob(const_cast<void*>(o.p), {o.rows, o.k}, {o.s_row, o.s_k}, opt)
-               .clone(at::MemoryFormat::Contiguous);
+// bf16 operands that no TMA map describes, copied to a row pitch (or column pitch, whichever direction is contiguous)
+// that one does describe; both in one launch.
+static void aligned_copies(Op& a, Op& b, const at::TensorOptions& opt, Tensor& keep_a, Tensor& keep_b) {
+  struct Copy {
+    const void* src = nullptr;
+    void* dst = nullptr;
+    ll rows = 0, pitch = 0;
+    int cols = 0;
+  } c[2];
+  int n = 0;
+  for (int i = 0; i < 2; ++i) {
+    Op& o = i ? b : a;
+    if (tma_ok(o)) continue;
+    Tensor& keep = i ? keep_b : keep_a;
+    const bool mn = o.s_k != 1 && o.s_row == 1;
+    const ll rows = mn ? o.k : o.rows, cols = mn ? o.rows : o.k, pitch = mn ? o.s_k : o.s_row, to = (cols + 7) / 8 * 8;
+    keep = at::empty({rows, to}, opt);
+    if ((mn || o.s_k == 1) && pitch >= cols) {
+      c[n++] = Copy{o.p, keep.data_ptr(), rows, pitch, static_cast<int>(cols)};
+    } else {  // neither direction is contiguous, or rows share elements
+      keep.narrow(1, 0, cols).copy_(
+          at::from_blob(const_cast<void*>(o.p), {rows, cols}, {mn ? o.s_k : o.s_row, mn ? o.s_row : o.s_k}, opt));
+    }
+    o = Op{keep.data_ptr(), o.rows, o.k, mn ? 1 : to, mn ? to : 1, true};
   }
-  return op2d(keep);
+  if (n > 0)
+    FB_CALL(fb_repack_rows, c[0].src, c[0].dst, c[0].rows, c[0].cols, c[0].pitch, c[1].src, c[1].dst, c[1].rows, c[1].cols,
+            c[1].pitch, cur_stream());
 }
 // Where the copies repay.  The kernel that reads such operands in place does 70 products (multiply-adds) per ns, the
 // aligned kernels many times that; a copy takes 6 us and 1.6 TB/s, and 5 us are left to be sure.  Behind a single
@@ -111,6 +129,11 @@ static bool copies_repay(const Op& a, const Op& b, bool rows_tma) {
   us += static_cast<double>(a.rows) * b.rows * 3e-6;
   return us > cost - 2.;
 }
+
+// Products with a bf16 result (layers and gradients of activations) of more than this many output rows, columns and
+// k: the aligned kernels' fp32 accumulation in tensor memory is theirs for aligned operands, too.  Products with an fp32
+// result keep the in-place kernel, whose split accumulation is the more exact one, up to the line above.
+static bool repack_repays(const Op& a, const Op& b) { return a.rows >= 256 && b.rows >= 128 && a.k >= 128; }
 
 // fp32 products with a reduction this short do not repay the tensor-core kernel's set-up (7 us against 2 - 3).
 constexpr int kSimtK = 32;
@@ -168,11 +191,11 @@ void gemm(const Op& a, const Op& b, const float* bias, int act, void* out, ll ld
   }
   if (a.bf16) {  // operands that a TMA map cannot describe
     const bool rows_tma = reinterpret_cast<uintptr_t>(out) % 16 == 0 && ldc * (out_bf16 ? 2 : 4) % 16 == 0;
-    if (like != nullptr && copies_repay(a, b, rows_tma)) {
+    if (like != nullptr && (copies_repay(a, b, rows_tma) || (out_bf16 && repack_repays(a, b)))) {
       Tensor ka, kb;
-      const auto opt = like->options().dtype(at::kBFloat16).requires_grad(false);
-      gemm(tma_ok(a) ? a : aligned_copy(a, opt, ka), tma_ok(b) ? b : aligned_copy(b, opt, kb), bias, act, out, ldc,
-           out_bf16, accumulate, nullptr, like, tf32, splits);
+      Op pa = a, pb = b;
+      aligned_copies(pa, pb, like->options().dtype(at::kBFloat16).requires_grad(false), ka, kb);
+      gemm(pa, pb, bias, act, out, ldc, out_bf16, accumulate, nullptr, like, tf32, splits);
       return;
     }
     FB_CALL(fb_gemm_bf16_any, a.p, b.p, out, bias, M, N, K, a.s_row, a.s_k, b.s_row, b.s_k, ldc, out_bf16, act,
