@@ -153,6 +153,8 @@ _CUDA_SIGS = {
     "fb_layernorm_set_status": (None, [P]),
     "fb_layernorm_bwd": (I, [P, P, P, P, P, P, P, P, P, LL, I, I, I, I, I, P]),
     "fb_layernorm_bwd_blocks": (I, [LL, I]),
+    "fb_add_layernorm_fwd": (I, [P] * 8 + [LL, I, F, I, P]),
+    "fb_add_layernorm_bwd": (I, [P] * 9 + [LL, I, I, P]),
     "fb_batchnorm_fwd": (I, [P, P, P, P, P, P, P, P, LL, I, F, F, I, P]),
     "fb_batchnorm_bwd": (I, [P, P, P, P, P, P, P, P, LL, I, P]),
     # softmax / losses

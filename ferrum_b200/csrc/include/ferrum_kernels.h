@@ -150,6 +150,11 @@ int fb_layernorm_bwd(const void* dy, const void* x, const void* act_grad, const 
                      const float* rstd, void* dx, float* partial, float* stats, long long rows, int cols,
                      int pre_act, int dtype, int nblk, int want_colsum, cudaStream_t stream);
 int fb_layernorm_bwd_blocks(long long rows, int cols);
+int fb_add_layernorm_fwd(const float* x, const void* r, const float* gamma, const float* beta, float* sum, float* y,
+                         float* mean, float* rstd, long long rows, int cols, float eps, int r_dtype, cudaStream_t stream);
+int fb_add_layernorm_bwd(const float* dy, const float* sum, const float* gamma, const float* mean, const float* rstd,
+                         float* dx, void* dx_low, float* partial, float* stats, long long rows, int cols, int nblk,
+                         cudaStream_t stream);
 int fb_batchnorm_fwd(const float* x, const float* gamma, const float* beta, float* y, float* save_mean,
                      float* save_rstd, float* running_mean, float* running_var, long long rows, int cols,
                      float eps, float momentum, int training, cudaStream_t stream);

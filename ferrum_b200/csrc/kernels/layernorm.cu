@@ -216,6 +216,108 @@ ln_fwd_kernel(const T* __restrict__ x, const float* __restrict__ gamma, const fl
   }
 }
 
+// Forward of norm(x + r): the residual connection in front of a normalisation, fp32 x and a sub-layer's result r of
+// either type.  Bound by HBM: x and r are read once and the sum (what the backward pass needs; NULL: not kept) and y
+// written, where an addition of its own writes the sum and this kernel's like reads it again.
+template <typename R, int TPR, int K>
+__global__ void __launch_bounds__(256)
+ln_add_fwd_kernel(const float* __restrict__ x, const R* __restrict__ r, const float* __restrict__ gamma,
+                  const float* __restrict__ beta, float* __restrict__ sum, float* __restrict__ y,
+                  float* __restrict__ mean_out, float* __restrict__ rstd_out, long long rows, int cols, float eps) {
+  __shared__ float smem[8][8];
+  constexpr int kRowsPerBlock = 256 / TPR;
+  const int sub = threadIdx.x / TPR;
+  const int t = threadIdx.x % TPR;
+  const int nvec = cols >> 3;
+  const float inv_n = 1.f / static_cast<float>(cols);
+  const long long row_stride = static_cast<long long>(gridDim.x) * kRowsPerBlock;
+  V8<float>::Raw raw[K], nxt[K];
+  typename V8<R>::Raw res[K], res_nxt[K];
+  {
+    const long long r0 = static_cast<long long>(blockIdx.x) * kRowsPerBlock + sub;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int vi = t + k * TPR;
+      if (r0 < rows && vi < nvec) {
+        raw[k] = V8<float>::ld(x + r0 * cols + vi * 8);
+        res[k] = V8<R>::ld(r + r0 * cols + vi * 8);
+      }
+    }
+  }
+  for (long long row0 = static_cast<long long>(blockIdx.x) * kRowsPerBlock; row0 < rows; row0 += row_stride) {
+    const long long row = row0 + sub;
+    const bool live = row < rows;
+    {  // the next row's loads are in flight while this one is reduced and written
+      const long long rn = row + row_stride;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const int vi = t + k * TPR;
+        if (rn < rows && vi < nvec) {
+          nxt[k] = V8<float>::ld(x + rn * cols + vi * 8);
+          res_nxt[k] = V8<R>::ld(r + rn * cols + vi * 8);
+        }
+      }
+    }
+    float v[K][8];
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int vi = t + k * TPR;
+      if (live && vi < nvec) {
+        float w[8];
+        V8<float>::unpack(raw[k], v[k]);
+        V8<R>::unpack(res[k], w);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          v[k][i] += w[i];
+          s += v[k][i];
+        }
+        if (sum != nullptr) V8<float>::st(sum + row * cols + vi * 8, v[k]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[k][i] = 0.f;
+      }
+    }
+    const float mu = row_sum<TPR>(s, smem) * inv_n;
+    float q = 0.f;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int vi = t + k * TPR;
+      if (live && vi < nvec) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float d = v[k][i] - mu;
+          q += d * d;
+        }
+      }
+    }
+    const float var = row_sum<TPR>(q, smem) * inv_n;
+    const float rs = rsqrtf(var + eps);
+    if (live && t == 0) {
+      mean_out[row] = mu;
+      rstd_out[row] = rs;
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int vi = t + k * TPR;
+      if (live && vi < nvec) {
+        float g[8], b[8], o[8];
+        if (gamma) ld8f(gamma + vi * 8, g);
+        if (beta) ld8f(beta + vi * 8, b);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          o[i] = (v[k][i] - mu) * rs * (gamma ? g[i] : 1.f) + (beta ? b[i] : 0.f);
+        V8<float>::st(y + row * cols + vi * 8, o);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      raw[k] = nxt[k];
+      res[k] = res_nxt[k];
+    }
+  }
+}
+
 __device__ __forceinline__ void ld_pairs_f32(const float* p, float2 (&o)[4]);
 
 // Forward, one WARP per row (bf16, 1024..4096 columns): a lane keeps its K 16-byte vectors packed in registers,
@@ -325,13 +427,13 @@ ln_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
 
 // Backward.  x and dy stay packed in registers between the statistics pass and the output pass; the
 // three column partials (dy*xhat, dy, dx) accumulate in registers over all rows the block visits and are
-// written once to partial[blockIdx][3][cols].
+// written once to partial[blockIdx][3][cols].  dx_low (optional): dx once more in bf16, the gradient of a residual's branch.
 template <typename T, int TPR, int K>
 __global__ void __launch_bounds__(256, 2)
 ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ act_grad,
               const float* __restrict__ gamma, const float* __restrict__ mean, const float* __restrict__ rstd,
-              T* __restrict__ dx, float* __restrict__ partial, long long rows, int cols, int pre_act,
-              int want_colsum) {
+              T* __restrict__ dx, __nv_bfloat16* __restrict__ dx_low, float* __restrict__ partial, long long rows,
+              int cols, int pre_act, int want_colsum) {
   __shared__ float smem[8][8];
   constexpr int kRowsPerBlock = 256 / TPR;
   constexpr bool kFast = V8<T>::kFastMath;
@@ -424,6 +526,7 @@ ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __rest
           for (int i = 0; i < 8; ++i) acc_c[k][i] += o[i];
         }
         V8<T>::st(dx + row * cols + vi * 8, o);
+        if (dx_low != nullptr) V8<__nv_bfloat16>::st(dx_low + row * cols + vi * 8, o);
       }
     }
 #pragma unroll
@@ -1239,6 +1342,25 @@ int fwd_t(const void* x, const float* gamma, const float* beta, void* y, float* 
   return static_cast<int>(cudaGetLastError());
 }
 
+template <typename R>
+int add_fwd_t(const float* x, const R* r, const float* gamma, const float* beta, float* sum, float* y, float* mean,
+              float* rstd, long long rows, int cols, float eps, cudaStream_t st) {
+  Geo g;
+  if (!geometry(cols, &g) || !aligned16(x, r, gamma, beta) || !aligned16(sum, y, nullptr, nullptr)) return -2;
+  const long long nb = (rows + 256 / g.tpr - 1) / (256 / g.tpr);
+  const int grid = static_cast<int>(nb < sm_count() * 8LL ? nb : sm_count() * 8LL);
+#define FB_LN_ADD(TPR, K) \
+  ln_add_fwd_kernel<R, TPR, K><<<grid, 256, 0, st>>>(x, r, gamma, beta, sum, y, mean, rstd, rows, cols, eps)
+  if (g.tpr == 32 && g.k == 1) FB_LN_ADD(32, 1);
+  else if (g.tpr == 32) FB_LN_ADD(32, 2);
+  else if (g.tpr == 128 && g.k == 1) FB_LN_ADD(128, 1);
+  else if (g.tpr == 128) FB_LN_ADD(128, 2);
+  else if (g.k == 2) FB_LN_ADD(256, 2);
+  else FB_LN_ADD(256, 4);
+#undef FB_LN_ADD
+  return static_cast<int>(cudaGetLastError());
+}
+
 template <typename T>
 bool launch_wide(const T*, const T*, const T*, const float*, const float*, const float*, T*, float*, long long, int,
                  int, int, cudaStream_t) {
@@ -1269,21 +1391,22 @@ bool launch_wide<__nv_bfloat16>(const __nv_bfloat16* dy, const __nv_bfloat16* x,
 
 template <typename T>
 int bwd_t(const void* dy, const void* x, const void* act_grad, const float* gamma, const float* mean,
-          const float* rstd, void* dx, float* partial, float* stats, long long rows, int cols, int pre_act, int nblk,
-          int want_colsum, cudaStream_t st) {
+          const float* rstd, void* dx, __nv_bfloat16* dx_low, float* partial, float* stats, long long rows, int cols,
+          int pre_act, int nblk, int want_colsum, cudaStream_t st) {
   const T* dyp = static_cast<const T*>(dy);
   const T* xp = static_cast<const T*>(x);
   const T* agp = static_cast<const T*>(act_grad);
   T* dxp = static_cast<T*>(dx);
   Geo g;
   const bool fast = nblk > 0 && partial != nullptr && geometry(cols, &g) && aligned16(dy, x, dx, gamma) &&
-                    aligned16(partial, stats, act_grad, nullptr);
+                    aligned16(partial, stats, act_grad, dx_low);
+  if (dx_low != nullptr && !fast) return -2;
   Geo any;
   if (fast || (nblk > 0 && partial != nullptr && geometry_any(cols, &any))) {
     int used = nblk;
     const int nvec = cols / 8;
     const int wide_blocks = nblk / 2 < sm_count() ? nblk / 2 : sm_count();  // two rows of partial[] per block
-    if (fast && ring_enabled() && pre_act == FB_ACT_NONE && cols * 2 >= 2048 && nvec <= 2 * kGroupThreads &&
+    if (fast && dx_low == nullptr && ring_enabled() && pre_act == FB_ACT_NONE && cols * 2 >= 2048 && nvec <= 2 * kGroupThreads &&
         wide_blocks >= 1 &&
         launch_wide<T>(dyp, xp, agp, gamma, mean, rstd, dxp, partial, rows, cols, wide_blocks, want_colsum, st)) {
       used = 2 * wide_blocks;
@@ -1295,8 +1418,8 @@ int bwd_t(const void* dy, const void* x, const void* act_grad, const float* gamm
 #undef FB_LN_BWD
     } else {
 #define FB_LN_BWD(TPR, K) \
-  ln_bwd_kernel<T, TPR, K><<<nblk, 256, 0, st>>>(dyp, xp, agp, gamma, mean, rstd, dxp, partial, rows, cols, pre_act, \
-                                                 want_colsum)
+  ln_bwd_kernel<T, TPR, K><<<nblk, 256, 0, st>>>(dyp, xp, agp, gamma, mean, rstd, dxp, dx_low, partial, rows, cols, \
+                                                 pre_act, want_colsum)
     if (g.tpr == 32 && g.k == 1) FB_LN_BWD(32, 1);
     else if (g.tpr == 32) FB_LN_BWD(32, 2);
     else if (g.tpr == 128 && g.k == 1) FB_LN_BWD(128, 1);
@@ -1362,10 +1485,35 @@ extern "C" int fb_layernorm_bwd(const void* dy, const void* x, const void* act_g
   if (stats == nullptr) return -1;
   if (act_grad != nullptr && pre_act != FB_ACT_NONE) return -1;
   if (dtype == FB_DT_F32)
-    return bwd_t<float>(dy, x, act_grad, gamma, mean, rstd, dx, partial, stats, rows, cols, pre_act, nblk,
+    return bwd_t<float>(dy, x, act_grad, gamma, mean, rstd, dx, nullptr, partial, stats, rows, cols, pre_act, nblk,
                         want_colsum, stream);
   if (dtype == FB_DT_BF16)
-    return bwd_t<__nv_bfloat16>(dy, x, act_grad, gamma, mean, rstd, dx, partial, stats, rows, cols, pre_act, nblk,
+    return bwd_t<__nv_bfloat16>(dy, x, act_grad, gamma, mean, rstd, dx, nullptr, partial, stats, rows, cols, pre_act, nblk,
                                 want_colsum, stream);
   return -1;
+}
+
+// norm(x + r) of fp32 x and r of r_dtype; sum (optional) = x + r.  -2, and nothing is launched: widths or addresses that
+// are not made of whole 16-byte pieces, more than 8192 columns.
+extern "C" int fb_add_layernorm_fwd(const float* x, const void* r, const float* gamma, const float* beta, float* sum,
+                                    float* y, float* mean, float* rstd, long long rows, int cols, float eps, int r_dtype,
+                                    cudaStream_t stream) {
+  if (rows <= 0 || cols <= 0) return 0;
+  if (mean == nullptr || rstd == nullptr) return -1;
+  if (r_dtype == FB_DT_F32)
+    return add_fwd_t<float>(x, static_cast<const float*>(r), gamma, beta, sum, y, mean, rstd, rows, cols, eps, stream);
+  if (r_dtype == FB_DT_BF16)
+    return add_fwd_t<__nv_bfloat16>(x, static_cast<const __nv_bfloat16*>(r), gamma, beta, sum, y, mean, rstd, rows, cols,
+                                    eps, stream);
+  return -1;
+}
+
+// fb_layernorm_bwd of fp32 rows, whose dx also goes to dx_low (optional) in bf16.
+extern "C" int fb_add_layernorm_bwd(const float* dy, const float* sum, const float* gamma, const float* mean,
+                                    const float* rstd, float* dx, void* dx_low, float* partial, float* stats,
+                                    long long rows, int cols, int nblk, cudaStream_t stream) {
+  if (rows <= 0 || cols <= 0) return 0;
+  if (stats == nullptr) return -1;
+  return bwd_t<float>(dy, sum, nullptr, gamma, mean, rstd, dx, static_cast<__nv_bfloat16*>(dx_low), partial, stats, rows,
+                      cols, FB_ACT_NONE, nblk, 0, stream);
 }

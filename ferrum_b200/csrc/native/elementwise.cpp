@@ -66,6 +66,7 @@ struct AddNode : Node {
   }
 };
 
+}  // namespace
 Tensor add(const Tensor& a, const Tensor& b) {
   NoAutograd below;
   Tensor ac = f32c(a), bc = f32c(b), y = empty(a.sizes(), a, at::kFloat);
@@ -81,6 +82,7 @@ Tensor add(const Tensor& a, const Tensor& b) {
   }
   return y;
 }
+namespace {
 
 // ------------------------------------------------------------------------------------------------- softmax
 struct SoftmaxNode : Node {

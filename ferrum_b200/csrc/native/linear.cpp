@@ -200,6 +200,89 @@ Tensor layer_norm(const Tensor& x, const c10::optional<Tensor>& gamma_, const c1
   return y;
 }
 
+// ---------------------------------------------------------------- LayerNorm(x + r) as one node
+// The residual connection of fp32 activations: the addition goes along with the normalisation, and the backward kernel
+// writes the gradient of a bf16 branch beside the fp32 one.
+struct AddNormNode : Node {
+  SavedVariable sum_, g_, mean_, rstd_;
+  bool has_beta = false, has_gamma = false;
+  at::ScalarType r_dtype = at::kFloat;
+  std::string name() const override { return "FerrumAddLayerNormBackward"; }
+  void release_variables() override {
+    for (SavedVariable* s : {&sum_, &g_, &mean_, &rstd_}) s->reset_data();
+  }
+  variable_list apply(variable_list&& grads) override {
+    variable_list out(4);  // x, r, gamma, beta
+    if (!grads[0].defined()) return out;
+    Tensor sum = sum_.unpack(), g = g_.unpack(), mean = mean_.unpack(), rstd = rstd_.unpack();
+    NoAutograd below;
+    sum = contig(sum);
+    Tensor s2 = as2d(sum), gy = f32c(grads[0]), dx = empty(sum.sizes(), sum, at::kFloat), low;
+    if (r_dtype == at::kBFloat16 && task_should_compute_output(1)) low = empty(sum.sizes(), sum, at::kBFloat16);
+    const int64_t rows = s2.size(0), cols = s2.size(1);
+    Tensor stats;
+    if (low.defined() && reinterpret_cast<uintptr_t>(gy.data_ptr()) % 16 == 0 &&
+        reinterpret_cast<uintptr_t>(sum.data_ptr()) % 16 == 0 && (!g.defined() || reinterpret_cast<uintptr_t>(g.data_ptr()) % 16 == 0)) {
+      const int nblk = fb_layernorm_bwd_blocks(rows, static_cast<int>(cols));
+      Tensor partial = empty({std::max(nblk, 1), 3, cols}, sum, at::kFloat);
+      stats = empty({3, cols}, sum, at::kFloat);
+      fb_rt_memset(stats.data_ptr(), 0, stats.numel() * 4, cur_stream());
+      FB_CALL(fb_add_layernorm_bwd, gy.data_ptr<float>(), sum.data_ptr<float>(), fptr(g), mean.data_ptr<float>(),
+              rstd.data_ptr<float>(), dx.data_ptr<float>(), low.data_ptr(), partial.data_ptr<float>(),
+              stats.data_ptr<float>(), rows, static_cast<int>(cols), nblk, cur_stream());
+      out[1] = low;
+    } else {
+      stats = norm_bwd(as2d(gy), s2, Tensor(), g, NormStats{mean, rstd}, dx, kNone, false);
+      if (task_should_compute_output(1)) out[1] = cast(dx, r_dtype);
+    }
+    out[0] = dx;
+    if (has_gamma) out[2] = stats[0];
+    if (has_beta) out[3] = stats[1];
+    return out;
+  }
+};
+
+Tensor add_layer_norm(const Tensor& x, const Tensor& r, const c10::optional<Tensor>& gamma_,
+                      const c10::optional<Tensor>& beta_, double eps) {
+  const Tensor gamma = gamma_.value_or(Tensor()), beta = beta_.value_or(Tensor());
+  const int64_t cols = x.dim() > 0 ? x.size(-1) : 0;
+  const auto f32 = [&](const Tensor& t) { return !t.defined() || (t.scalar_type() == at::kFloat && t.is_cuda() && t.numel() == cols); };
+  const bool whole = x.scalar_type() == at::kFloat && (r.scalar_type() == at::kFloat || is_bf16(r)) &&
+                     x.sizes() == r.sizes() && x.device() == r.device() && x.numel() > 0 && cols % 8 == 0 && cols <= 8192 &&
+                     f32(gamma) && f32(beta);
+  Tensor y;
+  if (whole) {
+    NoAutograd below;
+    Tensor xc = contig(x), rc = contig(r), g = gamma.defined() ? contig(gamma) : gamma, b = beta.defined() ? contig(beta) : beta;
+    uintptr_t at = reinterpret_cast<uintptr_t>(xc.data_ptr()) | reinterpret_cast<uintptr_t>(rc.data_ptr());
+    for (const Tensor& t : {g, b})
+      if (t.defined()) at |= reinterpret_cast<uintptr_t>(t.data_ptr());
+    if (at % 16 == 0) {
+      const bool grad = wants_grad({&x, &r, &gamma, &beta});
+      const int64_t rows = xc.numel() / cols;
+      Tensor sum = grad ? empty(xc.sizes(), xc, at::kFloat) : Tensor();
+      NormStats st{empty({rows}, xc, at::kFloat), empty({rows}, xc, at::kFloat)};
+      y = empty(xc.sizes(), xc, at::kFloat);
+      FB_CALL(fb_add_layernorm_fwd, xc.data_ptr<float>(), rc.data_ptr(), fptr(g), fptr(b), static_cast<float*>(ptr(sum)), y.data_ptr<float>(),
+              st.mean.data_ptr<float>(), st.rstd.data_ptr<float>(), rows, static_cast<int>(cols), static_cast<float>(eps),
+              dt(rc), cur_stream());
+      if (grad) {
+        auto n = make_node<AddNormNode>(x, r, gamma, beta);
+        n->has_gamma = gamma.defined();
+        n->has_beta = beta.defined();
+        n->r_dtype = r.scalar_type();
+        n->sum_ = below.keep(sum);
+        n->g_ = below.keep(g);
+        n->mean_ = below.keep(st.mean);
+        n->rstd_ = below.keep(st.rstd);
+        torch::autograd::set_history(y, n);
+      }
+      return y;
+    }
+  }
+  return layer_norm(fbn::add(x, r), gamma_, beta_, eps, kNone);
+}
+
 // ---------------------------------------------------------------- LayerNorm(act(x W^T + b)) as one node
 // Tensor-core path: the GEMM epilogue writes act(z) and, where a backward pass follows, act'(z); the normalisation
 // reads act(z).  Backward: one streaming kernel turns dy into dz and yields d_gamma, d_beta and the bias gradient,
@@ -375,6 +458,7 @@ Tensor bmm(const Tensor& a, const Tensor& b, double alpha, bool heads_inner, boo
 void bind_linear(py::module_& m) {
   m.def("linear", &linear);
   m.def("layer_norm", &layer_norm);
+  m.def("add_layer_norm", &add_layer_norm);
   m.def("linear_act_norm", &linear_act_norm);
   m.def("bmm", &bmm);
   m.def("gemm_nt",  // out = act(a b^T + bias) without a graph; see ops/functional.py

@@ -114,6 +114,7 @@ struct NoAutograd {
   }
 };
 
+Tensor add(const Tensor& a, const Tensor& b);
 Tensor unary(const Tensor& x, int op, double alpha, double beta);
 
 // ---------------------------------------------------------------------------------------------------- GEMM

@@ -89,6 +89,18 @@ class MultiHeadAttention(Module):
         return self.forward_attn(x, x, x)
 
 
+def _add_norm(norm, x, r):
+    """``norm(x + r)``; one node for a plain LayerNorm over the last dimension that nobody looks into."""
+    g = torch.nn.modules.module
+    if (type(norm) is LayerNorm and "forward" not in norm.__dict__ and norm.weight is not None
+            and norm.normalized_shape == tuple(x.shape[-1:])
+            and not (norm._forward_hooks or norm._forward_pre_hooks or norm._backward_hooks or norm._backward_pre_hooks
+                     or g._global_forward_hooks or g._global_forward_pre_hooks or g._global_backward_hooks
+                     or g._global_backward_pre_hooks)):
+        return F.add_layer_norm(x, r, norm.weight, norm.bias, norm.eps)
+    return norm(F.binary(x, r, "add"))
+
+
 class TransformerEncoderLayer(Module):
     def __init__(self, d_model: int, nhead: int, dim_feedforward: int, device=None):
         super().__init__()
@@ -104,9 +116,9 @@ class TransformerEncoderLayer(Module):
 
     @tensor_io
     def forward(self, x):
-        x = self.norm1(F.binary(x, self.self_attn(x), "add"))
+        x = _add_norm(self.norm1, x, self.self_attn(x))
         ff = self.linear2(self.linear1._forward_act(x, "relu") if x.is_cuda else F.unary(self.linear1(x), "relu"))
-        return self.norm2(F.binary(x, ff, "add"))
+        return _add_norm(self.norm2, x, ff)
 
 
 class PositionalEncoding(Module):

@@ -690,6 +690,13 @@ def layer_norm(x: torch.Tensor, gamma=None, beta=None, eps: float = 1e-5, pre_ac
     return y
 
 
+def add_layer_norm(x, r, gamma=None, beta=None, eps: float = 1e-5):
+    """``layer_norm(x + r)`` over the last dimension as one node (tensors of one size)."""
+    if _native(x) and _native(r) and x.shape == r.shape:
+        return _lib.native().add_layer_norm(x, r, gamma, beta, eps)
+    return layer_norm(binary(x, r, "add"), gamma, beta, eps)
+
+
 def linear_act_layernorm(x, weight, bias, gamma, beta, eps: float = 1e-5, act: str = "gelu", w_low=None,
                          sink: GradSink | None = None):
     """``LayerNorm(act(x @ weight^T + bias)) * gamma + beta`` as one fused block (CUDA); composed ops on CPU."""

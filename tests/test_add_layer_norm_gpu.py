@@ -1,0 +1,32 @@
+"""LayerNorm(x + r) as one node against the addition and the normalisation as nodes of their own: the same arithmetic, so
+the same bits forward; gradients too, the parameters' from partial sums in another order (2^-20 of their norm)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("r_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (7, 256), (300, 264), (33, 1024), (513, 1032), (5, 4096), (9, 8192),
+                                       (3, 8200), (4, 1001)])
+def test_against_two_nodes(rows, cols, r_dtype):
+    from ferrum_b200.ops import functional as F
+    from ferrum_b200.utils.runtime import check_status
+
+    got = []
+    for fused in (True, False):
+        g = torch.Generator(device="cuda").manual_seed(rows + cols)
+        rand = lambda *s: torch.randn(*s, device="cuda", generator=g)
+        x, r = rand(2, rows, cols).requires_grad_(True), rand(2, rows, cols).to(r_dtype).requires_grad_(True)
+        w, b = rand(cols).requires_grad_(True), rand(cols).requires_grad_(True)
+        y = F.add_layer_norm(x, r, w, b) if fused else F.layer_norm(F.binary(x, r, "add"), w, b)
+        with torch.no_grad():
+            z = F.add_layer_norm(x, r, w, b)
+        y.backward(rand(2, rows, cols))
+        check_status()
+        assert torch.equal(y.detach(), z)
+        got.append((y.detach(), x.grad, r.grad, w.grad, b.grad))
+    assert all(a.dtype == c.dtype and a.shape == c.shape for a, c in zip(*got))
+    assert all(torch.equal(a, c) for a, c in zip(got[0][:3], got[1][:3]))
+    for a, c in zip(got[0][3:], got[1][3:]):
+        assert (a - c).norm() <= 2.0 ** -20 * c.norm()
