@@ -113,7 +113,7 @@ def _cases(small: bool):
     sidx, perm = torch.sort(idx.reshape(-1), stable=True)
     dw = torch.zeros(V, D, device=dev)
     case("embedding_scatter_add_bwd",
-         lambda: lib.fb_embedding_bwd_sorted(gout.data_ptr(), sidx.data_ptr(), perm.data_ptr(), dw.data_ptr(),
+         lambda: lib.fb_embedding_bwd_sorted(gout.data_ptr(), sidx.data_ptr(), 8, perm.data_ptr(), dw.data_ptr(),
                                              Bt * S, D, S, 1.0 / S, -1, V, 3, st()), Bt * S * D * 2, "K10 bwd")
     gi = torch.randint(0, R, (R,), device=dev)
     case("gather_rows_f32", lambda: F.gather_rows(x32, gi), n * 8, "K18 collate")

@@ -170,7 +170,8 @@ _CUDA_SIGS = {
     "fb_dropout_bwd": (I, [P, P, P, LL, F, I, P]),
     "fb_embedding_fwd": (I, [P, P, P, LL, I, LL, LL, I, P, P]),
     "fb_embedding_meanpool_fwd": (I, [P, P, P, LL, I, I, LL, I, P]),
-    "fb_embedding_bwd_sorted": (I, [P, P, P, P, LL, I, I, F, LL, LL, I, P]),
+    "fb_embedding_bwd_sorted": (I, [P, P, I, P, P, LL, I, I, F, LL, LL, I, P]),
+    "fb_embedding_keys": (I, [P, P, LL, LL, P]),
     "fb_gather_rows": (I, [P, P, P, LL, LL, LL, P, P]),
     "fb_attention_fwd": (I, [P, P, P, P, P, I, I, I, I, I, LL, LL, LL, LL, LL, LL, LL, LL, LL, F, I, P, P]),
     "fb_attention_bwd": (I, [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, LL, LL, LL, LL, LL, LL, LL, LL, LL, F, I, P, P]),

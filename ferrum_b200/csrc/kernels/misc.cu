@@ -243,14 +243,25 @@ __global__ void embedding_meanpool_kernel(const float* __restrict__ w, const lon
   }
 }
 
+// Row numbers as 32-bit sort keys: half the bytes and half the passes of a radix sort of the 64-bit indices.  Indices
+// outside the table (reported by the forward pass) become `vocab`, which the scatter drops.
+__global__ void embedding_keys_kernel(const long long* __restrict__ idx, int32_t* __restrict__ keys, long long n,
+                                      long long vocab) {
+  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
+    const long long id = __ldg(idx + i);
+    keys[i] = static_cast<int32_t>(id < 0 || id > vocab ? vocab : id);
+  }
+}
+
 // Scatter-add over a SORTED index list: a block walks a chunk of 32 consecutive positions, sums runs of equal
 // indices in registers and flushes each run once, so heavily repeated tokens cost one flush per chunk instead of
 // one per occurrence.  perm[i] is the original position.  The chunk's ids and source rows are staged in shared
 // memory once (one 64-bit division per position instead of one per thread and position); with dim % 4 == 0 a
 // thread owns four adjacent columns: 8- or 16-byte loads of dout and one vector atomic (red.global.add.v4.f32)
 // per run.
-template <typename G>
-__global__ void embedding_bwd_sorted_kernel(const G* __restrict__ dout, const long long* __restrict__ sorted_idx,
+template <typename G, typename Key>
+__global__ void embedding_bwd_sorted_kernel(const G* __restrict__ dout, const Key* __restrict__ sorted_idx,
                                             const long long* __restrict__ perm, float* __restrict__ dw,
                                             long long n_idx, int dim, int group, float scale,
                                             long long padding_idx, long long vocab, int32_t* bstatus) {
@@ -662,24 +673,34 @@ extern "C" int fb_embedding_meanpool_fwd(const float* weight, const long long* i
   return static_cast<int>(cudaGetLastError());
 }
 
-extern "C" int fb_embedding_bwd_sorted(const void* dout, const long long* sorted_idx, const long long* perm,
+// keys[i] = idx[i], or vocab (< 2^31 - 1) where that is no row of the table.
+extern "C" int fb_embedding_keys(const long long* idx, int32_t* keys, long long n, long long vocab, cudaStream_t stream) {
+  if (n <= 0) return 0;
+  if (vocab <= 0 || vocab >= 0x7fffffffLL) return -1;
+  const long long want = (n + 255) / 256, cap = sm_count() * 8LL;
+  embedding_keys_kernel<<<static_cast<int>(want < cap ? want : cap), 256, 0, stream>>>(idx, keys, n, vocab);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// sorted_idx: 32-bit (key_bytes = 4) or 64-bit (8) row numbers.
+extern "C" int fb_embedding_bwd_sorted(const void* dout, const void* sorted_idx, int key_bytes, const long long* perm,
                                        float* dweight, long long n_idx, int dim, int group, float scale,
                                        long long padding_idx, long long vocab, int dtype, cudaStream_t stream) {
   if (n_idx <= 0 || dim <= 0) return 0;
-  if (group < 1) return -1;
+  if (group < 1 || (key_bytes != 4 && key_bytes != 8)) return -1;
   const long long nb = (n_idx + 31) / 32;
   if (nb > 2147483647LL) return -1;
   const int threads = dim >= 256 ? 256 : (dim >= 128 ? 128 : 64);
-  if (dtype == FB_DT_F32)
-    embedding_bwd_sorted_kernel<float><<<static_cast<unsigned>(nb), threads, 0, stream>>>(
-        static_cast<const float*>(dout), sorted_idx, perm, dweight, n_idx, dim, group, scale, padding_idx, vocab,
-        bounds_status_ref());
-  else if (dtype == FB_DT_BF16)
-    embedding_bwd_sorted_kernel<__nv_bfloat16><<<static_cast<unsigned>(nb), threads, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(dout), sorted_idx, perm, dweight, n_idx, dim, group, scale, padding_idx,
-        vocab, bounds_status_ref());
-  else
-    return -1;
+#define FB_EMBEDDING_BWD(G, KEY)                                                                                   \
+  embedding_bwd_sorted_kernel<G, KEY><<<static_cast<unsigned>(nb), threads, 0, stream>>>(                           \
+      static_cast<const G*>(dout), static_cast<const KEY*>(sorted_idx), perm, dweight, n_idx, dim, group, scale,    \
+      padding_idx, vocab, bounds_status_ref())
+  if (dtype == FB_DT_F32 && key_bytes == 4) FB_EMBEDDING_BWD(float, int32_t);
+  else if (dtype == FB_DT_F32) FB_EMBEDDING_BWD(float, long long);
+  else if (dtype == FB_DT_BF16 && key_bytes == 4) FB_EMBEDDING_BWD(__nv_bfloat16, int32_t);
+  else if (dtype == FB_DT_BF16) FB_EMBEDDING_BWD(__nv_bfloat16, long long);
+  else return -1;
+#undef FB_EMBEDDING_BWD
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -18,7 +18,13 @@ struct EmbeddingNode : Node {
     {
       NoAutograd below;
       g2 = contig(grads[0]).reshape({-1, dim});
-      std::tie(sorted, perm) = at::sort(idx.reshape({-1}), /*stable=*/true, /*dim=*/0, /*descending=*/false);
+      Tensor keys = idx.reshape({-1});
+      if (vocab < 0x7fffffff) {  // 512k indices: sorted in 66 us instead of 106
+        keys = empty({idx.numel()}, idx, at::kInt);
+        FB_CALL(fb_embedding_keys, reinterpret_cast<const ll*>(contig(idx).data_ptr<int64_t>()), keys.data_ptr<int32_t>(),
+                idx.numel(), vocab, cur_stream());
+      }
+      std::tie(sorted, perm) = at::sort(keys, /*stable=*/true, /*dim=*/0, /*descending=*/false);
     }
     if (sink) {  // accumulate straight into the data-parallel gradient arena
       py::gil_scoped_acquire gil;
@@ -28,7 +34,7 @@ struct EmbeddingNode : Node {
     } else {
       dw = at::zeros({vocab, dim}, g2.options().dtype(at::kFloat));
     }
-    FB_CALL(fb_embedding_bwd_sorted, g2.data_ptr(), reinterpret_cast<const ll*>(sorted.data_ptr<int64_t>()),
+    FB_CALL(fb_embedding_bwd_sorted, g2.data_ptr(), sorted.data_ptr(), static_cast<int>(sorted.element_size()),
             reinterpret_cast<const ll*>(perm.data_ptr<int64_t>()), dw.data_ptr<float>(), sorted.numel(),
             static_cast<int>(dim), static_cast<int>(group), 1.f / static_cast<float>(group), padding, vocab, dt(g2),
             cur_stream());
