@@ -34,13 +34,13 @@ namespace cg = cooperative_groups;
 constexpr int kRowsP = 128;   // rows of the operand on the 128-row side of the MMA
 constexpr int kBK = 64;       // one 128-byte swizzle row of bf16
 constexpr int kThreads = 192;
-constexpr int kMaxStages = 12;
+constexpr int kMaxStages = 32;
 constexpr int kSmemAlone = 200 * 1024, kSmemShared = 98 * 1024;  // stages of a CTA that has its SM alone, or half of it
 constexpr int kChunk = 64 * 128;  // 64 rows of 128 bytes: one block of an MN-major operand
 
 template <int BN>
 struct Cfg {
-  static constexpr int kP = kRowsP * 128;
+  static constexpr int kP = kRowsP * 128;  // what the MMA reads; Args::p_bytes of it are loaded
   static constexpr int kQ = (BN < 64 ? 64 : BN) * 128;  // an MN-major operand arrives in blocks of 64 columns
   static constexpr int kTile = (kRowsP + 4) * (BN + 4) * 4;
   static constexpr int kTmemCols = BN < 32 ? 32 : BN;
@@ -55,7 +55,7 @@ struct Args {
   int p_mn, q_mn;  // operand stored with its rows contiguous
   int out_bf16, act, beta;
   int kb_total, kb_per_split, tiles_p;
-  int stages, stage_bytes, body_bytes;
+  int stages, stage_bytes, body_bytes, p_bytes;
   int32_t* status;
   unsigned long long timeout_ns;
 };
@@ -138,7 +138,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
           break;
         }
         uint8_t* sp = smem + s * p.stage_bytes;
-        uint8_t* sq = sp + C::kP;
+        uint8_t* sq = sp + p.p_bytes;
         ptx::mbar_arrive_expect_tx(&full_bar[s], p.stage_bytes);
         const int k0 = kb * kBK;
         if (p.p_mn) {
@@ -173,7 +173,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
       const uint32_t p_lbo = p.p_mn ? kChunk : 16, q_lbo = p.q_mn ? kChunk : 16;
       const uint32_t p_step = p.p_mn ? 16 * 128 : 32, q_step = p.q_mn ? 16 * 128 : 32;
       const uint64_t p_first = ptx::make_smem_desc_sw128(ptx::smem_u32(smem), p_lbo, 1024);
-      const uint64_t q_first = ptx::make_smem_desc_sw128(ptx::smem_u32(smem) + C::kP, q_lbo, 1024);
+      const uint64_t q_first = ptx::make_smem_desc_sw128(ptx::smem_u32(smem) + p.p_bytes, q_lbo, 1024);
       int s = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -364,9 +364,10 @@ int choose_splits(long long tiles, int kb_total) {
 }
 
 template <int BN, bool kSwap>
-int launch(const CUtensorMap& mp, const CUtensorMap& mq, Args& g, int rows_p, int rows_q, bool split, cudaStream_t st) {
+int launch(const CUtensorMap& mp, const CUtensorMap& mq, Args& g, int rows_p, int rows_q, int box_p, bool split,
+           cudaStream_t st) {
   using C = Cfg<BN>;
-  constexpr int kExtra = 1024 + 256;  // alignment, barriers
+  constexpr int kExtra = 1024 + 768;  // alignment, barriers
   static const cudaError_t configured = cudaFuncSetAttribute(
       gemm_splitk_kernel<BN, kSwap>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAlone + kExtra);
   if (configured != cudaSuccess) return static_cast<int>(configured);
@@ -375,11 +376,13 @@ int launch(const CUtensorMap& mp, const CUtensorMap& mq, Args& g, int rows_p, in
   if (tiles > (1 << 27)) return -1;
   const int splits = split ? choose_splits(tiles, g.kb_total) : 1;
   g.kb_per_split = (g.kb_total + splits - 1) / splits;
-  g.stage_bytes = C::kP + (g.q_mn ? C::kQ : BN * 128);
-  const int room = (tiles * splits <= sm_count() ? kSmemAlone : kSmemShared) / g.stage_bytes;
+  g.p_bytes = box_p * 128;
+  g.stage_bytes = g.p_bytes + (g.q_mn ? C::kQ : BN * 128);
+  const int tail = C::kP - g.p_bytes;  // the MMA's reads of rows that were not loaded stay inside the allocation
+  const int room = ((tiles * splits <= sm_count() ? kSmemAlone : kSmemShared) - tail) / g.stage_bytes;
   g.stages = room < kMaxStages ? room : kMaxStages;
   if (g.stages > g.kb_per_split) g.stages = g.kb_per_split;
-  g.body_bytes = g.stages * g.stage_bytes;
+  g.body_bytes = (g.stages * g.stage_bytes + tail + 1023) / 1024 * 1024;
   if (g.body_bytes < C::kTile) g.body_bytes = (C::kTile + 1023) / 1024 * 1024;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(tiles * splits));
@@ -421,11 +424,14 @@ int run(bool split, const void* a, const void* b, void* out, void* out2, const f
   if (M <= 0 || N <= 0 || K <= 0) return -1;
   if ((out2 != nullptr && !out_bf16) || (out_bf16 && beta)) return -1;
   if (tile == 0) tile = choose_tile(M, N);
-  if (tile != 16 && tile != 32 && tile != 64 && tile != 192 && tile != 256) return -1;
+  if (tile != 16 && tile != 32 && tile != 64 && tile != 160 && tile != 192 && tile != 256) return -1;
   const bool swap = tile <= 64;
   const int bn = swap ? tile : tile - 128;
+  // Few rows of A on the 128-row side: only they are loaded (what else the MMA reads there goes into rows of the
+  // accumulator that nobody stores).
+  const int box_p = swap || a_mn_major || M > 64 ? kRowsP : M <= 16 ? 16 : M <= 32 ? 32 : 64;
   CUtensorMap ma, mb;
-  if (!make_map(&ma, a, M, K, lda, a_mn_major != 0, swap ? bn : kRowsP) ||
+  if (!make_map(&ma, a, M, K, lda, a_mn_major != 0, swap ? bn : box_p) ||
       !make_map(&mb, b, N, K, ldb, b_mn_major != 0, swap ? kRowsP : bn))
     return -2;
   Args g;
@@ -444,11 +450,12 @@ int run(bool split, const void* a, const void* b, void* out, void* out2, const f
   g.status = status;
   g.timeout_ns = 2000000000ull;
   switch (tile) {
-    case 16: return launch<16, true>(mb, ma, g, N, M, split, stream);
-    case 32: return launch<32, true>(mb, ma, g, N, M, split, stream);
-    case 64: return launch<64, true>(mb, ma, g, N, M, split, stream);
-    case 192: return launch<64, false>(ma, mb, g, M, N, split, stream);
-    default: return launch<128, false>(ma, mb, g, M, N, split, stream);
+    case 16: return launch<16, true>(mb, ma, g, N, M, box_p, split, stream);
+    case 32: return launch<32, true>(mb, ma, g, N, M, box_p, split, stream);
+    case 64: return launch<64, true>(mb, ma, g, N, M, box_p, split, stream);
+    case 160: return launch<32, false>(ma, mb, g, M, N, box_p, split, stream);
+    case 192: return launch<64, false>(ma, mb, g, M, N, box_p, split, stream);
+    default: return launch<128, false>(ma, mb, g, M, N, box_p, split, stream);
   }
 }
 
@@ -473,6 +480,10 @@ extern "C" int fb_gemm_bf16_narrow_use(int M, int N, int K) {
 extern "C" int fb_gemm_bf16_narrow(const void* a, const void* b, void* out, void* out2, const float* bias, int M, int N,
                                    int K, long long lda, long long ldb, long long ldc, int a_mn_major, int b_mn_major,
                                    int out_bf16, int act, int beta, int tile, int32_t* status, cudaStream_t stream) {
+  // The narrowest tile that one wave holds: a CTA's loop is bound by its own copies and MMAs, and the rows of A that every
+  // CTA reads again are few.  (An MN-major B arrives in blocks of 64 columns.)
+  if (tile == 0 && !b_mn_major && fb::tiles_of(N, 32) <= fb::sm_count()) tile = 160;
+  if (tile == 0 && !b_mn_major && fb::tiles_of(N, 64) <= fb::sm_count()) tile = 192;
   if (tile == 0) tile = M <= 32 ? fb::choose_tile(M, N) : 192;
   return fb::run(false, a, b, out, out2, bias, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, out_bf16, act, beta, tile,
                  status, stream);
