@@ -103,6 +103,19 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 __device__ __forceinline__ void prefetch_tensormap(const void* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
+// A kernel launched as a programmatic dependent starts beside the tail of the one before it in the stream: nothing of
+// what that one (or any before it) reads or writes may be touched before grid_wait, which returns when all of it has
+// completed and is visible; without the launch attribute it returns at once.  grid_launch_dependents lets such a
+// successor start once every CTA of this grid has said so.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Brings a box into L2; x (elements) on a 16-byte boundary like any TMA copy.  Reads nothing into the SM, so it may run
+// ahead of grid_wait: what is written later is written in L2.
+__device__ __forceinline__ void tma_prefetch_2d(const void* map, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x),
+               "r"(y)
+               : "memory");
+}
 // Untiled bulk copy global -> shared (no tensor map): both addresses 16-byte aligned, size a multiple of 16.
 __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(

@@ -56,6 +56,7 @@ struct Args {
   int out_bf16, act, beta;
   int kb_total, kb_per_split, tiles_p;
   int stages, stage_bytes, body_bytes, p_bytes;
+  int prefetch;  // bring this CTA's rows of B into L2 before the kernel ahead has completed
   int32_t* status;
   unsigned long long timeout_ns;
 };
@@ -125,6 +126,10 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  ptx::grid_launch_dependents();
+  if (p.prefetch && warp == 2 && ptx::elect_one())
+    for (int kb = kb_lo; kb < kb_hi; ++kb) ptx::tma_prefetch_2d(kSwap ? &map_p : &map_q, kb * kBK, kSwap ? p0 : q0);
+  ptx::grid_wait();
 
   if (warp == 0) {
     if (ptx::elect_one()) {
@@ -379,7 +384,9 @@ int launch(const CUtensorMap& mp, const CUtensorMap& mq, Args& g, int rows_p, in
   g.p_bytes = box_p * 128;
   g.stage_bytes = g.p_bytes + (g.q_mn ? C::kQ : BN * 128);
   const int tail = C::kP - g.p_bytes;  // the MMA's reads of rows that were not loaded stay inside the allocation
-  const int room = ((tiles * splits <= sm_count() ? kSmemAlone : kSmemShared) - tail) / g.stage_bytes;
+  // Half an SM for narrow tiles, too: the next one's CTAs start beside this one's.
+  const int room = ((split && tiles * splits <= sm_count() ? kSmemAlone : kSmemShared) - tail) / g.stage_bytes;
+  g.prefetch = !split && (kSwap ? !g.p_mn : !g.q_mn);
   g.stages = room < kMaxStages ? room : kMaxStages;
   if (g.stages > g.kb_per_split) g.stages = g.kb_per_split;
   g.body_bytes = (g.stages * g.stage_bytes + tail + 1023) / 1024 * 1024;
@@ -389,12 +396,14 @@ int launch(const CUtensorMap& mp, const CUtensorMap& mq, Args& g, int rows_p, in
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = g.body_bytes + kExtra;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = splits;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = split ? 1 : 2;
   return static_cast<int>(cudaLaunchKernelEx(&cfg, gemm_splitk_kernel<BN, kSwap>, mp, mq, g));
 }
 

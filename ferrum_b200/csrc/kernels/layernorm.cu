@@ -332,6 +332,10 @@ __global__ void __launch_bounds__(256, 2)
 ln_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
                    __nv_bfloat16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out,
                    long long rows, int cols, float eps) {
+  if constexpr (W > 1) {
+    ptx::grid_launch_dependents();
+    ptx::grid_wait();
+  }
   const int lane = threadIdx.x & 31;
   const int nvec = cols >> 3;
   const float inv_n = 1.f / static_cast<float>(cols);
@@ -1256,13 +1260,18 @@ bool launch_fwd_warp<__nv_bfloat16>(const __nv_bfloat16* xp, const float* gamma,
   // A block per row while two blocks per SM hold them all: 16 x 4096 6.9 -> 3.5 us, 296 x 2048 4.4 -> 3.2, 296 x 1024
   // 3.0 -> 2.3; at 592 rows the warps are as fast (4096 columns: 7.1 against 7.2 us), at 1184 almost twice as fast.
   if (rows <= 2LL * sm_count()) {
-    const int few = static_cast<int>(rows);
-    if (k <= 4)
-      ln_fwd_warp_kernel<4, 4><<<few, 128, 0, st>>>(xp, gamma, beta, yp, mean, rstd, rows, cols, eps);
-    else if (k <= 8)
-      ln_fwd_warp_kernel<8, 8><<<few, 256, 0, st>>>(xp, gamma, beta, yp, mean, rstd, rows, cols, eps);
-    else
-      ln_fwd_warp_kernel<16, 8><<<few, 256, 0, st>>>(xp, gamma, beta, yp, mean, rstd, rows, cols, eps);
+    // It starts beside the tail of the kernel ahead (see ptx::grid_wait).
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(rows));
+    cfg.blockDim = dim3(k <= 4 ? 128 : 256);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const auto kernel = k <= 4 ? ln_fwd_warp_kernel<4, 4> : k <= 8 ? ln_fwd_warp_kernel<8, 8> : ln_fwd_warp_kernel<16, 8>;
+    cudaLaunchKernelEx(&cfg, kernel, xp, gamma, beta, yp, mean, rstd, rows, cols, eps);
     return true;
   }
   const long long want = (rows + 7) / 8;  // eight warps per block
