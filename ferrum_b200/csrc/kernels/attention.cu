@@ -15,10 +15,12 @@
 //
 // What bounds it: the exponentials (16 per clock and SM: 2048 clocks per pair of tiles, as long as the MMAs of D = 128)
 // and the instructions around them.  Hence the two query tiles: one group's exponentials run beside the other's
-// reductions, and a group never waits for its own products: S_j+1 is issued as soon as S_j has been read, and O_j is
-// picked up one tile later, when the next maximum is known.  One query tile per CTA, where every tile paid both round
-// trips to the tensor core, against this, the same bits: 16 heads of 128, 8192 rows, causal: 639 -> 335 us
-// (820 TFLOP/s); 8 x 16 heads of 64, 1024 rows: 97 -> 87 us; 4 x 16 heads of 64, 8192 rows, causal: 1404 -> 955 us.
+// reductions, and a group never waits for its own products: S_j+1 is issued as soon as S_j has left tensor memory
+// (P_j is still being packed then), and O_j is picked up one tile later, where one multiply-add brings the sums to the
+// new maximum and adds it.  One query tile per CTA, where every tile paid both round trips to the tensor core: 16 heads
+// of 128, 8192 rows, causal: 639 us; two, with S_j+1 behind P_j and the MMA descriptors in ordinary registers (which
+// made their issue the bound): 340; now 285 (960 TFLOP/s).  8 x 16 heads of 64, 1024 rows: 97, 87 and 81 us; 4 x 16
+// heads of 64, 8192 rows, causal: 1404, 970 and 902 us.
 //
 // Every mbarrier wait is bounded (status block + abort flag shared by the CTA's roles); nothing traps.
 // Output: [B, S, H, D] contiguous bf16 (so the output projection sees [B, S, H*D]) and, optionally, the
@@ -81,22 +83,12 @@ __device__ __forceinline__ float2 fma2(float2 x, float2 y, float2 z) {
       : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y), "f"(z.x), "f"(z.y));
   return r;
 }
-__device__ __forceinline__ float2 add2(float2 x, float2 y) {
-  float2 r;
-  asm("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nadd.rn.f32x2 d, a, b;\nmov.b64 {%0, %1}, d;\n}"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
-  return r;
-}
-__device__ __forceinline__ float2 mul2(float2 x, float2 y) {
-  float2 r;
-  asm("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmul.rn.f32x2 d, a, b;\nmov.b64 {%0, %1}, d;\n}"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
-  return r;
-}
 __device__ __forceinline__ void tmem_ld(uint32_t addr, uint32_t (&r)[16]) { ptx::tmem_ld_32x32b_x16(addr, r); }
 __device__ __forceinline__ void tmem_ld(uint32_t addr, uint32_t (&r)[32]) { ptx::tmem_ld_32x32b_x32(addr, r); }
+// A store that may move across the waits for tensor memory (the fence in front of the arrival keeps it before that).
+__device__ __forceinline__ void st_shared(uint32_t at, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(a), "r"(b), "r"(c), "r"(d));
+}
 // Waits for the loads in flight; the registers pass through, so that no use of them can move above the wait.
 template <int N>
 __device__ __forceinline__ void tmem_ready(uint32_t (&r)[N]) {
@@ -129,42 +121,53 @@ __device__ __forceinline__ float row_max(uint32_t t_s, int valid) {
 }
 
 // p = 2^(s * scale - m): adds the row sum to l, 32 columns at a time, and writes bf16 P into shared memory (K-major,
-// 128-byte swizzle).
-template <int CH, bool kMask>
+// 128-byte swizzle).  One warp of a group per scheduler: a chunk's exponentials are started before the chunk ahead is
+// added up, packed and stored, so that the unit that evaluates them does not wait for that.  `s_read` runs when the last
+// scores have left tensor memory.
+template <int CH, bool kMask, typename F>
 __device__ __forceinline__ void row_exp(uint32_t t_s, int valid, float scale, float neg_m, uint8_t* sp, int row,
-                                        float& l) {
+                                        float& l, F&& s_read) {
   constexpr int kN = kBKV / CH;
   uint32_t r[2][CH];
+  float2 e[2][CH / 2];
   float part = 0.f;
   const float2 sc = make_float2(scale, scale), nm = make_float2(neg_m, neg_m);
   tmem_ld(t_s, r[0]);
 #pragma unroll
-  for (int c = 0; c < kN; ++c) {
-    tmem_ready(r[c & 1]);
-    if (c + 1 < kN) tmem_ld(t_s + (c + 1) * CH, r[(c + 1) & 1]);
+  for (int c = 0; c <= kN; ++c) {
+    if (c < kN) {
+      tmem_ready(r[c & 1]);
+      if (c + 1 < kN) tmem_ld(t_s + (c + 1) * CH, r[(c + 1) & 1]);
+      else s_read();
+#pragma unroll
+      for (int i = 0; i < CH; i += 2) {
+        const float2 x = fma2(make_float2(__uint_as_float(r[c & 1][i]), __uint_as_float(r[c & 1][i + 1])), sc, nm);
+        e[c & 1][i / 2] = make_float2(ex2(x.x), ex2(x.y));
+      }
+    }
+    if (c == 0) continue;
+    const int d = c - 1;
     uint32_t packed[CH / 2];
 #pragma unroll
     for (int i = 0; i < CH; i += 2) {
-      const float2 x = fma2(make_float2(__uint_as_float(r[c & 1][i]), __uint_as_float(r[c & 1][i + 1])), sc, nm);
-      float2 e = make_float2(ex2(x.x), ex2(x.y));
+      float2 v = e[d & 1][i / 2];
       if (kMask) {
-        if (c * CH + i >= valid) e.x = 0.f;
-        if (c * CH + i + 1 >= valid) e.y = 0.f;
+        if (d * CH + i >= valid) v.x = 0.f;
+        if (d * CH + i + 1 >= valid) v.y = 0.f;
       }
-      part += e.x + e.y;
-      const __nv_bfloat162 pk = __floats2bfloat162_rn(e.x, e.y);
+      part += v.x + v.y;
+      const __nv_bfloat162 pk = __floats2bfloat162_rn(v.x, v.y);
       packed[i >> 1] = *reinterpret_cast<const uint32_t*>(&pk);
     }
-    if ((c + 1) * CH % 32 == 0) {
+    if ((d + 1) * CH % 32 == 0) {
       l += part;
       part = 0.f;
     }
-    uint8_t* blk = sp + (c * CH / 64) * kBlk + row * 128;
+    const uint32_t blk = ptx::smem_u32(sp) + (d * CH / 64) * kBlk + row * 128;
 #pragma unroll
     for (int q = 0; q < CH / 8; ++q) {
-      const int chunk = (c * CH % 64) / 8 + q;
-      *reinterpret_cast<uint4*>(blk + ((chunk ^ (row & 7)) << 4)) =
-          make_uint4(packed[q * 4], packed[q * 4 + 1], packed[q * 4 + 2], packed[q * 4 + 3]);
+      const int chunk = (d * CH % 64) / 8 + q;
+      st_shared(blk + ((chunk ^ (row & 7)) << 4), packed[q * 4], packed[q * 4 + 1], packed[q * 4 + 2], packed[q * 4 + 3]);
     }
   }
 }
@@ -184,12 +187,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   uint64_t* full = q_full + 1;       // [kRing]
   uint64_t* empty = full + kRing;    // [kRing]
   uint64_t* s_full = empty + kRing;  // [2]
-  uint64_t* p_full = s_full + 2;     // [2]
+  uint64_t* s_free = s_full + 2;     // [2]
+  uint64_t* p_full = s_free + 2;     // [2]
   uint64_t* o_full = p_full + 2;     // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
   // CTAs in the order of `head_group` heads at a time (their keys and values stay in L2), the query blocks with the
   // most keys first: under a causal mask the short ones fill the end of the last wave.
   const int t = static_cast<int>(blockIdx.x), per_group = p.head_group * p.q_blocks;
@@ -217,7 +221,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     }
     for (int g = 0; g < 2; ++g) {
       ptx::mbar_init(&s_full[g], 1);
-      ptx::mbar_init(&p_full[g], 4);  // one arrival per softmax warp
+      ptx::mbar_init(&s_free[g], 4);  // one arrival per softmax warp
+      ptx::mbar_init(&p_full[g], 4);
       ptx::mbar_init(&o_full[g], 1);
     }
     ptx::fence_mbar_init();
@@ -266,30 +271,32 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                  ptx::globaltimer() - t0 <= p.timeout_ns) {
           }
       }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && ptx::elect_one()) {
       // ---------------------------------------------------------------- MMA issuer
       const uint32_t idesc_s = ptx::make_idesc(1u, kBQ, kBKV, 0, 0);   // Q, K both K-major
       const uint32_t idesc_o = ptx::make_idesc(1u, kBQ, D, 0, 1);      // P K-major, V with d contiguous (MN-major)
+      const uint64_t q_first = ptx::make_smem_desc_sw128(ptx::smem_u32(sq), 16, 1024);
+      const uint64_t ring_first = ptx::make_smem_desc_sw128(ptx::smem_u32(ring), 16, 1024);
+      const uint64_t v_first = ptx::make_smem_desc_sw128(ptx::smem_u32(ring), kBlk, 1024);
+      const uint64_t p_first = ptx::make_smem_desc_sw128(ptx::smem_u32(sp), 16, 1024);
       auto wait_item = [&](int i) { return ptx::mbar_wait(&full[i % kRing], (i / kRing) & 1, abort_flag, p.timeout_ns); };
       auto last_of = [&](int j) { return j < n[1] ? 1 : 0; };  // the group that uses tile j last
       auto issue_s = [&](int g, int j) {
-        const uint32_t a = ptx::smem_u32(sq + g * kTileBytes), k_at = ptx::smem_u32(ring + (2 * j % kRing) * kTileBytes);
+        const uint64_t a = ptx::desc_advance(q_first, g * kTileBytes), b = ptx::desc_advance(ring_first, (2 * j % kRing) * kTileBytes);
 #pragma unroll
         for (int k = 0; k < D / 16; ++k)
-          ptx::umma_f16(tmem_base + g * kBKV, ptx::make_smem_desc_sw128(a + (k >> 2) * kBlk + (k & 3) * 32, 16, 1024),
-                        ptx::make_smem_desc_sw128(k_at + (k >> 2) * kBlk + (k & 3) * 32, 16, 1024), idesc_s,
-                        k != 0 ? 1u : 0u);
+          ptx::umma_f16(tmem_base + g * kBKV, ptx::desc_advance(a, (k >> 2) * kBlk + (k & 3) * 32),
+                        ptx::desc_advance(b, (k >> 2) * kBlk + (k & 3) * 32), idesc_s, k != 0 ? 1u : 0u);
         ptx::umma_commit(&s_full[g]);
         if (g == last_of(j)) ptx::umma_commit(&empty[2 * j % kRing]);  // free once these MMAs have read it
       };
       auto issue_o = [&](int g, int j) {
-        const uint32_t a = ptx::smem_u32(sp + g * 2 * kBlk);
-        const uint32_t v_at = ptx::smem_u32(ring + ((2 * j + 1) % kRing) * kTileBytes);
+        const uint64_t a = ptx::desc_advance(p_first, g * 2 * kBlk), b = ptx::desc_advance(v_first, (2 * j + 1) % kRing * kTileBytes);
 #pragma unroll
         for (int k = 0; k < kBKV / 16; ++k)
           // V: 16 keys (rows of 128 bytes) per MMA; its 64-column blocks lie kBlk apart (the leading-dimension offset)
-          ptx::umma_f16(tmem_base + 2 * kBKV + g * D, ptx::make_smem_desc_sw128(a + (k >> 2) * kBlk + (k & 3) * 32, 16, 1024),
-                        ptx::make_smem_desc_sw128(v_at + k * 2048, kBlk, 1024), idesc_o, k != 0 ? 1u : 0u);
+          ptx::umma_f16(tmem_base + 2 * kBKV + g * D, ptx::desc_advance(a, (k >> 2) * kBlk + (k & 3) * 32),
+                        ptx::desc_advance(b, k * 2048), idesc_o, k != 0 ? 1u : 0u);
         ptx::umma_commit(&o_full[g]);
         if (g == last_of(j)) ptx::umma_commit(&empty[(2 * j + 1) % kRing]);
       };
@@ -303,16 +310,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       for (int j = 0; ok && j < n_max; ++j) {
         for (int g = 0; ok && g < 2; ++g) {
           if (j >= n[g]) continue;
-          // P_j is written, S_j has been read and O_(j-1) picked up
-          ok = ptx::mbar_wait(&p_full[g], j & 1, abort_flag, p.timeout_ns);
-          if (ok && j + 1 < n[g]) {
-            ok = wait_item(2 * (j + 1));
+          if (j + 1 < n[g]) {  // S_j has been read
+            ok = ptx::mbar_wait(&s_free[g], j & 1, abort_flag, p.timeout_ns) && wait_item(2 * (j + 1));
             if (ok) {
               ptx::tc_fence_after();
               issue_s(g, j + 1);
             }
           }
-          ok = ok && wait_item(2 * j + 1);
+          // P_j is written and O_(j-1) picked up
+          ok = ok && ptx::mbar_wait(&p_full[g], j & 1, abort_flag, p.timeout_ns) && wait_item(2 * j + 1);
           if (!ok) {
             report_status(p.status, kStatusGemmTimeout, 53, blockIdx.x, j);
             break;
@@ -344,7 +350,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       if (lane == 0) report_status(p.status, kStatusGemmTimeout, code, blockIdx.x, j);
       return false;
     };
-    auto add_o = [&]() {  // o += the product of the tile before
+    auto add_o = [&](float scale) {  // o = o * scale + the product of the tile before
+      const float2 sc = make_float2(scale, scale);
 #pragma unroll
       for (int c = 0; c < D / 32; ++c) {
         uint32_t r[32];
@@ -352,8 +359,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         tmem_ready(r);
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-          o[c * 16 + i] = add2(o[c * 16 + i], make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])));
+          o[c * 16 + i] = fma2(o[c * 16 + i], sc, make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])));
       }
+    };
+    float alpha = 0.f;  // what the sums of the tiles before the last one are still to be multiplied by
+    auto s_read = [&]() {
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&s_free[g]);
     };
     for (int j = 0; j < n_tiles; ++j) {
       ok = wait_all(&s_full[g], j & 1, 55, j);
@@ -365,30 +378,25 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       const bool whole = __all_sync(0xffffffffu, valid == kBKV);
       const float mx = whole ? row_max<kChunk, false>(t_s, valid) : row_max<kChunk, true>(t_s, valid);
       const float m_new = fmaxf(m, mx * p.scale_log2);
-      const float alpha = ex2(m - m_new);  // 0 for the first tile (m = -inf)
-      m = m_new;
-      l *= alpha;
       if (j > 0) {  // O_(j-1): its accumulators are free and its P has been read
         ok = wait_all(&o_full[g], (j - 1) & 1, 56, j);
         if (!ok) break;
-        add_o();
-        if (__any_sync(0xffffffffu, alpha != 1.f)) {
-          const float2 al = make_float2(alpha, alpha);
-#pragma unroll
-          for (int i = 0; i < D / 2; ++i) o[i] = mul2(o[i], al);
-        }
+        add_o(alpha);
       }
+      alpha = ex2(m - m_new);  // 0 for the first tile (m = -inf)
+      m = m_new;
+      l *= alpha;
       if (whole)
-        row_exp<kChunk, false>(t_s, valid, p.scale_log2, -m, my_p, row, l);
+        row_exp<kChunk, false>(t_s, valid, p.scale_log2, -m, my_p, row, l, s_read);
       else
-        row_exp<kChunk, true>(t_s, valid, p.scale_log2, -m, my_p, row, l);
+        row_exp<kChunk, true>(t_s, valid, p.scale_log2, -m, my_p, row, l, s_read);
       ptx::tc_fence_before();          // the reads of S and O are ordered before the MMAs that overwrite them
       ptx::fence_proxy_async_smem();   // P becomes visible to the tensor core's (async-proxy) reads
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&p_full[g]);
     }
     if (ok) ok = wait_all(&o_full[g], (n_tiles - 1) & 1, 57, n_tiles);
-    if (ok) add_o();
+    if (ok) add_o(alpha);
     if (ok && q_row < p.Sq) {
       const float inv = 1.f / l;
       __nv_bfloat16* dst = p.out + ((static_cast<long long>(b) * p.Sq + q_row) * p.H + h) * D;
