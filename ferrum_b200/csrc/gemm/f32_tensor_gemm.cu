@@ -28,7 +28,10 @@
 // multiple of 8, large operands are laid out again and take the aligned kernels (native/core.cpp, copies_repay).
 //
 // The issue of a k-block's MMAs takes as long as the MMAs themselves (the queue is short), so it has a warp of its own;
-// a loader warp that issued them held up the next stage (5200 instead of 2300 cycles per k-block).
+// a loader warp that issued them held up the next stage (5200 instead of 2300 cycles per k-block).  The splits' partial
+// sums are all asked for before the first is added and the values stay in registers (as an indexed array they went
+// through local memory: 2400 cycles per 4 x 544 results, now a quarter): 1024^3 23.9 -> 21.9 us, 4096 x 4096 x 1024
+// 261 -> 237, 128 x 256 x 784 9.4 -> 8.8.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -131,6 +134,13 @@ __device__ __forceinline__ float act_f(float x, int act) {
     case FB_ACT_SIGMOID: return 1.f / (1.f + expf(-x));
     default: return x;
   }
+}
+
+template <typename T>
+__device__ __noinline__ float dot_again(const T* a, long long sa, const T* b, long long sb, int K) {
+  float s = 0.f;
+  for (int k = 0; k < K; ++k) s = fmaf(a[k * sa], b[k * sb], s);
+  return s;
 }
 
 // Where piece `c` of an operand tile (row, 8 consecutive k) lies: neighbouring lanes follow the contiguous direction.
@@ -464,30 +474,38 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split_kernel(const __grid_co
     const int row = rank * rows_per + i / kVec, c = (i % kVec) * 4;
     const int m = m0 + row, n = n0 + c;
     if (m >= p.M || n >= p.N) continue;
+    float4 part[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+      if (r < splits) part[r] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(tile, r) + row * C::kPitch + c);
     float f[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int r = 0; r < splits; ++r) {
-      const float4 t = *reinterpret_cast<const float4*>(cluster.map_shared_rank(tile, r) + row * C::kPitch + c);
-      f[0] += t.x; f[1] += t.y; f[2] += t.z; f[3] += t.w;
-    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+      if (r < splits) {
+        f[0] += part[r].x; f[1] += part[r].y; f[2] += part[r].z; f[3] += part[r].w;
+      }
     if constexpr (kPlanes > 1) {
+#pragma unroll
       for (int j = 0; j < 4; ++j) {
         const bool finite = fabsf(f[j]) <= FLT_MAX;
         f[j] *= kDown;
-        if (finite || n + j >= p.N) continue;
         // not finite: an operand that does not survive the split, or a result that is not finite in fp32 either
-        float s = 0.f;
-        for (int k = 0; k < p.K; ++k)
-          s = fmaf(a[m * p.a.s_row + k * p.a.s_k], b[(n + j) * p.b.s_row + k * p.b.s_k], s);
-        f[j] = s;
+        if (!finite && n + j < p.N)
+          f[j] = dot_again(a + m * p.a.s_row, p.a.s_k, b + (n + j) * p.b.s_row, p.b.s_k, p.K);
       }
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (n + j < p.N) {
-        float x = f[j] * p.alpha;
-        if (p.bias != nullptr) x += __ldg(p.bias + n + j);
-        f[j] = act_f(x, p.act);
+    for (int j = 0; j < 4; ++j) {
+      f[j] *= p.alpha;
+      if (p.bias != nullptr && n + j < p.N) f[j] += __ldg(p.bias + n + j);
+    }
+    if (p.act != FB_ACT_NONE) {
+#pragma unroll 1
+      for (int j = 0; j < 4; ++j) {  // one copy of the code; the four values change places instead of being indexed
+        const float y = act_f(f[0], p.act);
+        f[0] = f[1]; f[1] = f[2]; f[2] = f[3]; f[3] = y;
       }
+    }
     const long long at = out_at + m * p.ldc + n;
     if (p.out_bf16) {
       __nv_bfloat16* o = static_cast<__nv_bfloat16*>(p.out) + at;
