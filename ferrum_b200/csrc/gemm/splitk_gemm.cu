@@ -55,7 +55,7 @@ struct Args {
   int p_mn, q_mn;  // operand stored with its rows contiguous
   int out_bf16, act, beta;
   int kb_total, kb_per_split, tiles_p;
-  int stages, stage_bytes, body_bytes, p_bytes;
+  int stages, block_bytes, body_bytes, p_bytes;  // block: a k-block of both operands
   int prefetch;  // bring this CTA's rows of B into L2 before the kernel ahead has completed
   int32_t* status;
   unsigned long long timeout_ns;
@@ -86,8 +86,9 @@ __device__ __forceinline__ void store_bf16(void* out, long long at, const float 
   }
 }
 
-// kSwap: P = B (rows are output columns), Q = A.
-template <int BN, bool kSwap>
+// kSwap: P = B (rows are output columns), Q = A.  kGroup: k-blocks per stage.  One thread issues the MMAs, and a wait,
+// a commit and a loop around every four of them take it longer (400 cycles) than the MMAs of a narrow tile (160).
+template <int BN, bool kSwap, int kGroup>
 __global__ void __launch_bounds__(kThreads, 2)
 gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q,
                    const __grid_constant__ Args p) {
@@ -136,27 +137,31 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
       int issued = 0, s = 0;
       uint32_t phase = 1;
       bool ok = true;
-      for (int kb = kb_lo; kb < kb_hi; ++kb, ++issued) {
+      for (int kb = kb_lo; kb < kb_hi; kb += kGroup, ++issued) {
         if (!ptx::mbar_wait(&empty_bar[s], phase, abort_flag, p.timeout_ns)) {
           report_status(p.status, kStatusGemmTimeout, 23, blockIdx.x, kb);
           ok = false;
           break;
         }
-        uint8_t* sp = smem + s * p.stage_bytes;
-        uint8_t* sq = sp + p.p_bytes;
-        ptx::mbar_arrive_expect_tx(&full_bar[s], p.stage_bytes);
-        const int k0 = kb * kBK;
-        if (p.p_mn) {
+        const int blocks = min(kGroup, kb_hi - kb);
+        ptx::mbar_arrive_expect_tx(&full_bar[s], blocks * p.block_bytes);
+        for (int i = 0; i < blocks; ++i) {
+          uint8_t* sp = smem + (s * kGroup + i) * p.block_bytes;
+          uint8_t* sq = sp + p.p_bytes;
+          const int k0 = (kb + i) * kBK;
+          if (p.p_mn) {
 #pragma unroll
-          for (int c = 0; c < kRowsP / 64; ++c) ptx::tma_load_2d(sp + c * kChunk, &map_p, &full_bar[s], p0 + c * 64, k0);
-        } else {
-          ptx::tma_load_2d(sp, &map_p, &full_bar[s], k0, p0);
-        }
-        if (p.q_mn) {
+            for (int c = 0; c < kRowsP / 64; ++c) ptx::tma_load_2d(sp + c * kChunk, &map_p, &full_bar[s], p0 + c * 64, k0);
+          } else {
+            ptx::tma_load_2d(sp, &map_p, &full_bar[s], k0, p0);
+          }
+          if (p.q_mn) {
 #pragma unroll
-          for (int c = 0; c < C::kQ / kChunk; ++c) ptx::tma_load_2d(sq + c * kChunk, &map_q, &full_bar[s], q0 + c * 64, k0);
-        } else {
-          ptx::tma_load_2d(sq, &map_q, &full_bar[s], k0, q0);
+            for (int c = 0; c < C::kQ / kChunk; ++c)
+              ptx::tma_load_2d(sq + c * kChunk, &map_q, &full_bar[s], q0 + c * 64, k0);
+          } else {
+            ptx::tma_load_2d(sq, &map_q, &full_bar[s], k0, q0);
+          }
         }
         if (++s == p.stages) {
           s = 0;
@@ -182,18 +187,27 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
       int s = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int i = 0; i < kb_hi - kb_lo; ++i) {
+      for (int kb = kb_lo; kb < kb_hi; kb += kGroup) {
         if (!ptx::mbar_wait(&full_bar[s], phase, abort_flag, p.timeout_ns)) {
-          report_status(p.status, kStatusGemmTimeout, 24, blockIdx.x, i);
+          report_status(p.status, kStatusGemmTimeout, 24, blockIdx.x, kb);
           ok = false;
           break;
         }
         ptx::tc_fence_after();
-        const uint64_t dp = ptx::desc_advance(p_first, s * p.stage_bytes), dq = ptx::desc_advance(q_first, s * p.stage_bytes);
+        const auto block = [&](int i) {
+          const int at = (s * kGroup + i) * p.block_bytes;
+          const uint64_t dp = ptx::desc_advance(p_first, at), dq = ptx::desc_advance(q_first, at);
 #pragma unroll
-        for (int k = 0; k < kBK / 16; ++k)
-          ptx::umma_f16(tmem, ptx::desc_advance(dp, k * p_step), ptx::desc_advance(dq, k * q_step), idesc,
-                        (i | k) != 0 ? 1u : 0u);
+          for (int k = 0; k < kBK / 16; ++k)
+            ptx::umma_f16(tmem, ptx::desc_advance(dp, k * p_step), ptx::desc_advance(dq, k * q_step), idesc,
+                          (kb - kb_lo) | i | k ? 1u : 0u);
+        };
+        if (kGroup == 1 || kb + kGroup <= kb_hi) {
+#pragma unroll
+          for (int i = 0; i < kGroup; ++i) block(i);
+        } else {
+          for (int i = 0; i < kb_hi - kb; ++i) block(i);
+        }
         ptx::umma_commit(&empty_bar[s]);
         if (++s == p.stages) {
           s = 0;
@@ -368,13 +382,13 @@ int choose_splits(long long tiles, int kb_total) {
   return splits;
 }
 
-template <int BN, bool kSwap>
+template <int BN, bool kSwap, int kGroup>
 int launch(const CUtensorMap& mp, const CUtensorMap& mq, Args& g, int rows_p, int rows_q, int box_p, bool split,
            cudaStream_t st) {
   using C = Cfg<BN>;
   constexpr int kExtra = 1024 + 768;  // alignment, barriers
   static const cudaError_t configured = cudaFuncSetAttribute(
-      gemm_splitk_kernel<BN, kSwap>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAlone + kExtra);
+      gemm_splitk_kernel<BN, kSwap, kGroup>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAlone + kExtra);
   if (configured != cudaSuccess) return static_cast<int>(configured);
   g.tiles_p = tiles_of(rows_p, kRowsP);
   const long long tiles = static_cast<long long>(g.tiles_p) * tiles_of(rows_q, BN);
@@ -382,14 +396,15 @@ int launch(const CUtensorMap& mp, const CUtensorMap& mq, Args& g, int rows_p, in
   const int splits = split ? choose_splits(tiles, g.kb_total) : 1;
   g.kb_per_split = (g.kb_total + splits - 1) / splits;
   g.p_bytes = box_p * 128;
-  g.stage_bytes = g.p_bytes + (g.q_mn ? C::kQ : BN * 128);
+  g.block_bytes = g.p_bytes + (g.q_mn ? C::kQ : BN * 128);
   const int tail = C::kP - g.p_bytes;  // the MMA's reads of rows that were not loaded stay inside the allocation
   // Half an SM for narrow tiles, too: the next one's CTAs start beside this one's.
-  const int room = ((split && tiles * splits <= sm_count() ? kSmemAlone : kSmemShared) - tail) / g.stage_bytes;
+  const int room = ((split && tiles * splits <= sm_count() ? kSmemAlone : kSmemShared) - tail) / g.block_bytes;
   g.prefetch = !split && (kSwap ? !g.p_mn : !g.q_mn);
-  g.stages = room < kMaxStages ? room : kMaxStages;
-  if (g.stages > g.kb_per_split) g.stages = g.kb_per_split;
-  g.body_bytes = (g.stages * g.stage_bytes + tail + 1023) / 1024 * 1024;
+  const int need = (g.kb_per_split + kGroup - 1) / kGroup;
+  g.stages = room / kGroup < kMaxStages ? room / kGroup : kMaxStages;
+  if (g.stages > need) g.stages = need;
+  g.body_bytes = (g.stages * kGroup * g.block_bytes + tail + 1023) / 1024 * 1024;
   if (g.body_bytes < C::kTile) g.body_bytes = (C::kTile + 1023) / 1024 * 1024;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(tiles * splits));
@@ -404,7 +419,7 @@ int launch(const CUtensorMap& mp, const CUtensorMap& mq, Args& g, int rows_p, in
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = split ? 1 : 2;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, gemm_splitk_kernel<BN, kSwap>, mp, mq, g));
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, gemm_splitk_kernel<BN, kSwap, kGroup>, mp, mq, g));
 }
 
 }  // namespace
@@ -458,13 +473,19 @@ int run(bool split, const void* a, const void* b, void* out, void* out2, const f
   g.kb_total = (K + kBK - 1) / kBK;
   g.status = status;
   g.timeout_ns = 2000000000ull;
+  // Stages of four k-blocks while 98 KB hold three of them (boxes of 16 rows of A).
+  const bool four = !split && !g.q_mn && box_p <= 16;
   switch (tile) {
-    case 16: return launch<16, true>(mb, ma, g, N, M, box_p, split, stream);
-    case 32: return launch<32, true>(mb, ma, g, N, M, box_p, split, stream);
-    case 64: return launch<64, true>(mb, ma, g, N, M, box_p, split, stream);
-    case 160: return launch<32, false>(ma, mb, g, M, N, box_p, split, stream);
-    case 192: return launch<64, false>(ma, mb, g, M, N, box_p, split, stream);
-    default: return launch<128, false>(ma, mb, g, M, N, box_p, split, stream);
+    case 16: return launch<16, true, 1>(mb, ma, g, N, M, box_p, split, stream);
+    case 32: return launch<32, true, 1>(mb, ma, g, N, M, box_p, split, stream);
+    case 64: return launch<64, true, 1>(mb, ma, g, N, M, box_p, split, stream);
+    case 160:
+      return four ? launch<32, false, 4>(ma, mb, g, M, N, box_p, split, stream)
+                  : launch<32, false, 2>(ma, mb, g, M, N, box_p, split, stream);
+    case 192:
+      return four ? launch<64, false, 2>(ma, mb, g, M, N, box_p, split, stream)
+                  : launch<64, false, 1>(ma, mb, g, M, N, box_p, split, stream);
+    default: return launch<128, false, 1>(ma, mb, g, M, N, box_p, split, stream);
   }
 }
 
@@ -479,9 +500,11 @@ extern "C" int fb_gemm_bf16_splitk(const void* a, const void* b, void* out, void
 }
 
 // Results of up to 64 rows whose sums may not change with the shape (forward passes, input gradients): narrow tiles and
-// one chain of MMAs over the whole reduction, the persistent kernels' bits.  They leave a 16 x 4096 product to 16 CTAs,
-// each of which reads 2 MB of weights alone; here it is 32 or 64.  Operands from HBM: 16 x 4096 x 4096 38.9 -> 29.6 us,
-// 16 x 1000 x 1024 20.5 -> 16.4, 64 x 4096 x 4096 39.0 -> 32.8; 16 x 128 x 512 12.3 -> 14.3, 128 x 512 x 512 18.4 both.
+// one chain of MMAs over the whole reduction, the persistent kernels' bits.  Operands from HBM, persistent kernels /
+// tiles of 128 columns of B (operands exchanged) / of 32, us: 16 x 4096 x 4096 29.7 / 22.7 / 17.1, 16 x 1024 x 4096
+// 29.0 / 20.0 / 13.8, 16 x 4096 x 1024 12.4 / 9.6 / 7.9, 64 x 1000 x 1024 12.8 / 11.0 / 8.4; 16 x 10000 x 1024, more
+// tiles of 32 than SMs: 13.0 / 11.3 / 14.9, with 64 columns 10.1.  16 x 128 x 512 was 12.3 on the persistent kernels and
+// 14.3 here, 128 x 512 x 512 18.4 on both.
 extern "C" int fb_gemm_bf16_narrow_use(int M, int N, int K) {
   return M > 0 && M <= 64 && N >= 512 && N <= fb::kRowsP * fb::sm_count() && K >= 512;
 }
