@@ -52,8 +52,10 @@ class MultiHeadAttention(Module):
                 or any(type(p) is not Linear or "forward" in p.__dict__ or p._forward_hooks or p._forward_pre_hooks
                        for p in (self.q_proj, self.k_proj, self.v_proj))):
             return query, key, value
-        low = {id(t): F.raw_cast(t, torch.bfloat16) if t.is_cuda and t.dtype == torch.float32 else t
-               for t in (query, key, value)}
+        low = {}
+        for t in (query, key, value):
+            if id(t) not in low:
+                low[id(t)] = F.raw_cast(t, torch.bfloat16) if t.is_cuda and t.dtype == torch.float32 else t
         return tuple(low[id(t)] for t in (query, key, value))
 
     @tensor_io
