@@ -130,10 +130,15 @@ static bool copies_repay(const Op& a, const Op& b, bool rows_tma) {
   return us > cost - 2.;
 }
 
-// Products with a bf16 result (layers and gradients of activations) of more than this many output rows, columns and
-// k: the aligned kernels' fp32 accumulation in tensor memory is theirs for aligned operands, too.  Products with an fp32
-// result keep the in-place kernel, whose split accumulation is the more exact one, up to the line above.
-static bool repack_repays(const Op& a, const Op& b) { return a.rows >= 256 && b.rows >= 128 && a.k >= 128; }
+// The same for products with a bf16 result (layers and gradients of activations) of any reduction, whose operands keep
+// their direction and go through one launch.  (Those with an fp32 result keep the in-place kernel up to the line above:
+// its split accumulation is the more exact one.)
+static bool repack_repays(const Op& a, const Op& b) {
+  double cost = 12.;
+  for (const Op* o : {&a, &b})
+    if (!tma_ok(*o)) cost += static_cast<double>(o->rows) * o->k * 4 / 4e6;
+  return static_cast<double>(a.rows) * b.rows * a.k / 7e7 > cost;
+}
 
 // fp32 products with a reduction this short do not repay the tensor-core kernel's set-up (7 us against 2 - 3).
 constexpr int kSimtK = 32;
