@@ -131,10 +131,14 @@ static bool copies_repay(const Op& a, const Op& b, bool rows_tma) {
 }
 
 // The same for products with a bf16 result (layers and gradients of activations) of any reduction, whose operands keep
-// their direction and go through one launch.  (Those with an fp32 result keep the in-place kernel up to the line above:
-// its split accumulation is the more exact one.)
+// their direction, go through one launch and then take the CTA pairs.  (Those with an fp32 result keep the in-place kernel
+// up to the line above: its split accumulation is the more exact one.)  In place against copy + product, us: 1024 x 1001 x
+// 1001 19.1 / 3.7 + 13.8, 2048 x 1001 x 1001 30.3 / 4.6 + 14.0, 777 x 2049 x 2049 49.2 / 6.3 + 20.4, 512 x 4095 x 4095
+// 84.9 / 16.6 + 32.0, 8191 x 4095 x 4095 1146 / 48 + 200; below 512 rows, without the pairs, 300 x 1001 x 4095 27.1 / 6.3 +
+// 55.2.
 static bool repack_repays(const Op& a, const Op& b) {
-  double cost = 12.;
+  if (a.rows < 512 || b.rows < 128) return false;
+  double cost = 14.;
   for (const Op* o : {&a, &b})
     if (!tma_ok(*o)) cost += static_cast<double>(o->rows) * o->k * 4 / 4e6;
   return static_cast<double>(a.rows) * b.rows * a.k / 7e7 > cost;

@@ -1,0 +1,36 @@
+"""LayerNorm over rows of any width, both directions, at the edges of the tiles, against fp64.
+
+Bounds: fp32 sums of up to 8193 terms, two passes: 2e-6 of the norm; bf16 results and gradients round once more (2^-8 of
+the norm covers an output rounding of 2^-9 and that of the GELU's fast evaluation)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,cols", [(1, 1), (3, 33), (130, 63), (7, 65), (900, 256), (5, 255), (64, 257), (700, 512),
+                                       (777, 1001), (1500, 1024), (9, 1023), (4, 1025), (6, 2047), (300, 2048), (5, 2049),
+                                       (3, 4095), (2, 4097), (3, 8191), (2, 8193)])
+@pytest.mark.parametrize("pre", [None, "gelu"])
+def test_against_fp64(rows, cols, dtype, pre):
+    from ferrum_b200.ops import functional as F
+    from ferrum_b200.utils.runtime import check_status
+
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x, gy = rand(rows, cols).to(dtype), rand(rows, cols).to(dtype)
+    w, b = rand(cols), rand(cols)
+    leaves = [t.clone().requires_grad_(True) for t in (x, w, b)]
+    exact = [t.double().requires_grad_(True) for t in (x, w, b)]
+    y = F.layer_norm(leaves[0], leaves[1], leaves[2], 1e-5, pre)
+    y.backward(gy)
+    z = torch.nn.functional.gelu(exact[0], approximate="tanh") if pre else exact[0]
+    want = torch.nn.functional.layer_norm(z, (cols,), exact[1], exact[2], 1e-5)
+    want.backward(gy.double())
+    check_status()
+    tol = 2e-6 if dtype is torch.float32 else 2.0 ** -8
+    assert (y.double() - want).norm() <= tol * want.norm() + 1e-6
+    # a row of one column has no gradient; next to none there, absolute
+    for got, ref in zip(leaves, exact):
+        assert (got.grad.double() - ref.grad).norm() <= 2 * tol * ref.grad.norm() + 1e-5 * rows ** 0.5
