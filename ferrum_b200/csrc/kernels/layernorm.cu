@@ -432,8 +432,11 @@ ln_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
 // Backward.  x and dy stay packed in registers between the statistics pass and the output pass; the
 // three column partials (dy*xhat, dy, dx) accumulate in registers over all rows the block visits and are
 // written once to partial[blockIdx][3][cols].  dx_low (optional): dx once more in bf16, the gradient of a residual's branch.
+// Bound by loads in flight, hence three blocks per SM where a thread holds one vector, and for few rows by the rows of a
+// block adding up, which they do in shared memory (one after the other through global memory each waited for the one
+// before).  fp32: 128 x 256 10.9 -> 4.4 us, 1024 x 1024 13.1 -> 8.8, 8192 x 1024 with dx_low 36.8 -> 31.7.
 template <typename T, int TPR, int K>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, K == 1 ? 3 : 2)
 ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ act_grad,
               const float* __restrict__ gamma, const float* __restrict__ mean, const float* __restrict__ rstd,
               T* __restrict__ dx, __nv_bfloat16* __restrict__ dx_low, float* __restrict__ partial, long long rows,
@@ -544,41 +547,38 @@ ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __rest
   float* pg = partial + static_cast<long long>(blockIdx.x) * 3 * cols;
   float* pb = pg + cols;
   float* pc = pb + cols;
-  if (kRowsPerBlock == 1) {
+  // Several row slots own the same columns: they add up in shared memory, one slot at a time, and the last one stores.
+  __shared__ float cols_sum[3][kRowsPerBlock > 1 ? K * TPR * 8 : 1];
+#pragma unroll 1
+  for (int slot = 0; slot < kRowsPerBlock; ++slot) {
+    if (kRowsPerBlock > 1) __syncthreads();
+    if (sub != slot) continue;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       const int vi = t + k * TPR;
-      if (vi < nvec) {
+      if (vi >= nvec) continue;
+      if (slot > 0) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          pg[vi * 8 + i] = acc_g[k][i];
-          pb[vi * 8 + i] = acc_b[k][i];
-          pc[vi * 8 + i] = acc_c[k][i];
+          const int at = (k * 8 + i) * TPR + t;
+          acc_g[k][i] = cols_sum[0][at] + acc_g[k][i];
+          acc_b[k][i] = cols_sum[1][at] + acc_b[k][i];
+          acc_c[k][i] = cols_sum[2][at] + acc_c[k][i];
         }
       }
-    }
-  } else {
-    // several row slots own the same columns: slot 0 stores, the others add, one slot at a time
-    for (int sidx = 0; sidx < kRowsPerBlock; ++sidx) {
-      __syncthreads();
-      if (sub == sidx) {
+      if (slot + 1 == kRowsPerBlock) {
+        V8<float>::st(pg + vi * 8, acc_g[k]);
+        V8<float>::st(pb + vi * 8, acc_b[k]);
+        V8<float>::st(pc + vi * 8, acc_c[k]);
+      } else {
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-          const int vi = t + k * TPR;
-          if (vi < nvec) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int c = vi * 8 + i;
-              if (sidx == 0) {
-                pg[c] = acc_g[k][i]; pb[c] = acc_b[k][i]; pc[c] = acc_c[k][i];
-              } else {
-                pg[c] += acc_g[k][i]; pb[c] += acc_b[k][i]; pc[c] += acc_c[k][i];
-              }
-            }
-          }
+        for (int i = 0; i < 8; ++i) {
+          const int at = (k * 8 + i) * TPR + t;
+          cols_sum[0][at] = acc_g[k][i];
+          cols_sum[1][at] = acc_b[k][i];
+          cols_sum[2][at] = acc_c[k][i];
         }
       }
-      __threadfence_block();
     }
   }
 }
@@ -1468,7 +1468,8 @@ extern "C" int fb_layernorm_bwd_blocks(long long rows, int cols) {
   if (!geometry(cols, &g) && !geometry_any(cols, &g)) return 0;
   const long long rpb = 256 / g.tpr;
   const long long nb = (rows + rpb - 1) / rpb;
-  const long long cap = static_cast<long long>(sm_count()) * 2;
+  // Three blocks per SM where a thread holds one vector of a row: loads in flight, not registers, are what is short.
+  const long long cap = static_cast<long long>(sm_count()) * (cols % 8 == 0 && g.k == 1 ? 3 : 2);
   return static_cast<int>(nb < cap ? nb : cap);
 }
 
