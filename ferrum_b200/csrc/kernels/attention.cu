@@ -16,11 +16,11 @@
 // What bounds it: the exponentials (16 per clock and SM: 2048 clocks per pair of tiles, as long as the MMAs of D = 128)
 // and the instructions around them.  Hence the two query tiles: one group's exponentials run beside the other's
 // reductions, and a group never waits for its own products: S_j+1 is issued as soon as S_j has left tensor memory
-// (P_j is still being packed then), and O_j is picked up one tile later, where one multiply-add brings the sums to the
-// new maximum and adds it.  One query tile per CTA, where every tile paid both round trips to the tensor core: 16 heads
-// of 128, 8192 rows, causal: 639 us; two, with S_j+1 behind P_j and the MMA descriptors in ordinary registers (which
-// made their issue the bound): 340; now 285 (960 TFLOP/s).  8 x 16 heads of 64, 1024 rows: 97, 87 and 81 us; 4 x 16
-// heads of 64, 8192 rows, causal: 1404, 970 and 902 us.
+// (P_j is still being packed then), and O_j is picked up one tile later, when the next maximum is known.  16 heads of
+// 128, 8192 rows, causal: 639 us with one query tile per CTA, where every tile paid both round trips to the tensor core;
+// 340 with two, S_j+1 behind P_j and the MMA descriptors in ordinary registers, which made their issue the bound; now 285
+// (960 TFLOP/s).  8 x 16 heads of 64, 1024 rows: 97, 87 and 81 us; 4 x 16 heads of 64, 8192 rows, causal: 1404, 970 and
+// 902.  The same bits.
 //
 // Every mbarrier wait is bounded (status block + abort flag shared by the CTA's roles); nothing traps.
 // Output: [B, S, H, D] contiguous bf16 (so the output projection sees [B, S, H*D]) and, optionally, the
@@ -81,6 +81,16 @@ __device__ __forceinline__ float2 fma2(float2 x, float2 y, float2 z) {
       "fma.rn.f32x2 d, a, b, c;\nmov.b64 {%0, %1}, d;\n}"
       : "=f"(r.x), "=f"(r.y)
       : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y), "f"(z.x), "f"(z.y));
+  return r;
+}
+// (x + y) * s, both rounded.  (As x * s + y it would be one operation less in the loop, but a packed product and sum are
+// contracted to a multiply-add, other bits.)
+__device__ __forceinline__ float2 add_scale2(float2 x, float2 y, float2 s) {
+  float2 r;
+  asm("{\n.reg .b64 a, b, c, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmov.b64 c, {%6, %7};\n"
+      "add.rn.f32x2 d, a, b;\nmul.rn.f32x2 d, d, c;\nmov.b64 {%0, %1}, d;\n}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y), "f"(s.x), "f"(s.y));
   return r;
 }
 __device__ __forceinline__ void tmem_ld(uint32_t addr, uint32_t (&r)[16]) { ptx::tmem_ld_32x32b_x16(addr, r); }
@@ -350,7 +360,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       if (lane == 0) report_status(p.status, kStatusGemmTimeout, code, blockIdx.x, j);
       return false;
     };
-    auto add_o = [&](float scale) {  // o = o * scale + the product of the tile before
+    auto add_o = [&](float scale) {  // o = (o + the product of the tile before) * scale
       const float2 sc = make_float2(scale, scale);
 #pragma unroll
       for (int c = 0; c < D / 32; ++c) {
@@ -359,10 +369,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         tmem_ready(r);
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-          o[c * 16 + i] = fma2(o[c * 16 + i], sc, make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])));
+          o[c * 16 + i] = add_scale2(o[c * 16 + i], make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), sc);
       }
     };
-    float alpha = 0.f;  // what the sums of the tiles before the last one are still to be multiplied by
     auto s_read = [&]() {
       ptx::tc_fence_before();
       __syncwarp();
@@ -378,14 +387,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       const bool whole = __all_sync(0xffffffffu, valid == kBKV);
       const float mx = whole ? row_max<kChunk, false>(t_s, valid) : row_max<kChunk, true>(t_s, valid);
       const float m_new = fmaxf(m, mx * p.scale_log2);
+      const float alpha = ex2(m - m_new);  // 0 for the first tile (m = -inf)
+      m = m_new;
       if (j > 0) {  // O_(j-1): its accumulators are free and its P has been read
         ok = wait_all(&o_full[g], (j - 1) & 1, 56, j);
         if (!ok) break;
         add_o(alpha);
       }
-      alpha = ex2(m - m_new);  // 0 for the first tile (m = -inf)
-      m = m_new;
-      l *= alpha;
+      l = __fmul_rn(l, alpha);
       if (whole)
         row_exp<kChunk, false>(t_s, valid, p.scale_log2, -m, my_p, row, l, s_read);
       else
@@ -396,7 +405,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       if (lane == 0) ptx::mbar_arrive(&p_full[g]);
     }
     if (ok) ok = wait_all(&o_full[g], (n_tiles - 1) & 1, 57, n_tiles);
-    if (ok) add_o(alpha);
+    if (ok) add_o(1.f);
     if (ok && q_row < p.Sq) {
       const float inv = 1.f / l;
       __nv_bfloat16* dst = p.out + ((static_cast<long long>(b) * p.Sq + q_row) * p.H + h) * D;
