@@ -328,7 +328,7 @@ bool warp_row(const void* x, const void* dx, int cols) { return cols >= 264 && c
 
 // A row of a cross-entropy is a chain of loads, reductions and exponentials, 1.2 us of a warp: the cluster's eight blocks
 // take at most three rounds of them, beyond that the whole chip and a second launch are faster (777 x 37 bf16: 19.1 us on
-// eight SMs, 512 x 512 15.2).
+// eight SMs, 3.0 and 1.8 for the partial sums on all).
 bool few_rows(long long elems, long long blocks) { return elems <= kClusterElems && blocks <= kClusterTrips * kCluster; }
 
 template <typename T>
