@@ -18,9 +18,9 @@
 // reductions, and a group never waits for its own products: S_j+1 is issued as soon as S_j has left tensor memory
 // (P_j is still being packed then), and O_j is picked up one tile later, when the next maximum is known.  16 heads of
 // 128, 8192 rows, causal: 639 us with one query tile per CTA, where every tile paid both round trips to the tensor core;
-// 340 with two, S_j+1 behind P_j and the MMA descriptors in ordinary registers, which made their issue the bound; now 285
-// (960 TFLOP/s).  8 x 16 heads of 64, 1024 rows: 97, 87 and 81 us; 4 x 16 heads of 64, 8192 rows, causal: 1404, 970 and
-// 902.  The same bits.
+// 340 with two, S_j+1 behind P_j and the MMA descriptors in ordinary registers, which made their issue the bound; now 288
+// (950 TFLOP/s).  8 x 16 heads of 64, 1024 rows: 97, 88 and 84 us; 4 x 16 heads of 64, 8192 rows, causal: 1404, 973 and
+// 923.  The same bits.
 //
 // Every mbarrier wait is bounded (status block + abort flag shared by the CTA's roles); nothing traps.
 // Output: [B, S, H, D] contiguous bf16 (so the output projection sees [B, S, H*D]) and, optionally, the
