@@ -39,7 +39,7 @@ def test_shared_input(train, how):
     want = run([x.detach().clone() for _ in range(3)])
     assert torch.equal(got[0], want[0])
     # sums by atomics may differ in order; the key bias' gradient is zero in exact arithmetic, all rounding
-    scale = max(float(b.norm()) for b in want[1:])
+    scale = max((float(b.norm()) for b in want[1:]), default=0.0)
     for a, b in zip(got[1:], want[1:]):
         assert (a - b).norm() <= 1e-5 * b.norm() + 1e-6 * scale
     if how == "grad" and train:
