@@ -461,6 +461,11 @@ void bind_linear(py::module_& m) {
   m.def("add_layer_norm", &add_layer_norm);
   m.def("linear_act_norm", &linear_act_norm);
   m.def("bmm", &bmm);
+  m.def("low_copy", [](const Tensor& x) {  // bf16 copy, without a graph, for several products; a dual tensor is refused
+    refuse_tangents({&x});
+    NoAutograd below;
+    return cast(x, at::kBFloat16);
+  });
   m.def("gemm_nt",  // out = act(a b^T + bias) without a graph; see ops/functional.py
         [](const Tensor& a, const Tensor& b, const c10::optional<Tensor>& bias, int act, const Tensor& out,
            bool accumulate, bool tf32) {

@@ -45,7 +45,8 @@ class MultiHeadAttention(Module):
         return t.reshape(B, S, self.num_heads, self.head_dim).transpose(1, 2)  # [B, H, S, D]
 
     def _inputs(self, query, key, value):
-        """The projections of one fp32 tensor that needs no gradient share its bf16 copy (a copy of 8192 x 2048: 18 us)."""
+        """The projections of one fp32 tensor that needs no gradient share its bf16 copy (a copy of 8192 x 2048: 18 us).
+        One with a tangent, which the copy would lose, is refused there as by the projections."""
         g = torch.nn.modules.module
         if (not config.low_precision_active() or g._global_forward_hooks or g._global_forward_pre_hooks
                 or any(type(p) is not Linear or "forward" in p.__dict__ or p._forward_hooks or p._forward_pre_hooks
@@ -55,7 +56,7 @@ class MultiHeadAttention(Module):
         for t in (query, key, value):
             if id(t) not in low:
                 share = t.is_cuda and t.dtype == torch.float32 and not (torch.is_grad_enabled() and t.requires_grad)
-                low[id(t)] = F.raw_cast(t, torch.bfloat16) if share else t
+                low[id(t)] = F.low_copy(t) if share else t
         return tuple(low[id(t)] for t in (query, key, value))
 
     @tensor_io

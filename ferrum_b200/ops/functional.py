@@ -73,6 +73,11 @@ def raw_cast(x: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     return x.to(dtype)
 
 
+def low_copy(x: torch.Tensor) -> torch.Tensor:
+    """bf16 copy of a CUDA tensor that needs no gradient, outside the graph; a dual tensor is refused."""
+    return _lib.native().low_copy(x)
+
+
 def raw_unary(x: torch.Tensor, op: str, alpha: float = 0.0, beta: float = 0.0) -> torch.Tensor:
     x = x.contiguous()
     y = torch.empty_like(x)

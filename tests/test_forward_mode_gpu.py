@@ -27,7 +27,27 @@ def _calls(d):
         "bmm": lambda: F.bmm_scaled(d.reshape(1, 1, 4, 8), q),
         "embedding": lambda: F.embedding(d, t),
         "rnn": lambda: F.rnn_sequence(4, d.reshape(4, 1, 8), torch.randn(8, 2, device="cuda"), None),
+        "add_layer_norm": lambda: F.add_layer_norm(d, torch.zeros_like(w[:4]), one, one),
+        "add_layer_norm_branch": lambda: F.add_layer_norm(torch.zeros_like(w[:4]), d, one, one),
+        "conv2d": lambda: F.conv2d_igemm(d.reshape(1, 1, 4, 8), torch.randn(2, 1, 3, 3, device="cuda"), None),
     }
+
+
+@pytest.mark.parametrize("grad", [True, False])
+@pytest.mark.parametrize("low", [True, False])
+def test_attention_refuses_dual_inputs(grad, low):
+    import ferrum_b200 as fb
+    from ferrum_b200 import nn
+
+    m = nn.MultiHeadAttention(128, 2, device=fb.Device.Cuda(0))
+    x = torch.randn(1, 5, 128, device="cuda")
+    with fwd.dual_level(), torch.set_grad_enabled(grad), fb.autocast(enabled=low):
+        d = fwd.make_dual(x, torch.ones_like(x))
+        for args in ((d, d, d), (d, x, x), (x, d, x), (x, x, d)):
+            with pytest.raises(NotImplementedError):
+                m.forward_attn(*args)
+                pytest.fail("a tangent was lost")
+        m.forward_attn(x, x, x)  # no tangent: nothing to refuse
 
 
 @pytest.mark.parametrize("grad", [True, False])
