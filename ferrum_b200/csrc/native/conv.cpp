@@ -115,7 +115,9 @@ Tensor conv2d(const Tensor& x, const Tensor& weight, const c10::optional<Tensor>
   TORCH_CHECK_VALUE(x.dim() == 4 && weight.dim() == 4 && x.size(1) == weight.size(1),
                     "conv2d: [B, C, H, W] and [O, C, kh, kw] expected, got ", x.sizes(), " and ", weight.sizes());
   TORCH_CHECK_VALUE(stride.size() == 2 && padding.size() == 2 && dilation.size() == 2, "conv2d: pairs expected");
-  TORCH_CHECK_VALUE(stride[0] > 0 && stride[1] > 0 && dilation[0] > 0 && dilation[1] > 0 && padding[0] >= 0 && padding[1] >= 0,
+  // Negative padding is a crop; the space-to-depth kernels have none.
+  TORCH_CHECK_VALUE(stride[0] > 0 && stride[1] > 0 && dilation[0] > 0 && dilation[1] > 0 &&
+                        ((padding[0] >= 0 && padding[1] >= 0) || (stride[0] == 1 && stride[1] == 1)),
                     "conv2d: strides ", stride, ", padding ", padding, ", dilation ", dilation);
   TORCH_CHECK_VALUE(act == FB_ACT_NONE || act == FB_ACT_RELU, "conv2d: no epilogue evaluates activation ", act);
   TORCH_CHECK_VALUE(act == FB_ACT_NONE || !add_.has_value(), "conv2d: an added tensor or an activation, not both");

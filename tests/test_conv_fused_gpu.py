@@ -81,3 +81,25 @@ def test_block_with_hooks():
         assert torch.equal(p.grad, g)
     for h in hooks:
         h.remove()
+
+
+@pytest.mark.parametrize("k,pad,dil", [((3, 3), (-1, -2), (1, 1)), ((1, 1), (-1, 0), (1, 1)), ((2, 3), (1, -3), (2, 1))])
+def test_negative_padding(k, pad, dil):
+    """A crop, as long as the stride is 1."""
+    import ferrum_b200 as fb
+    from ferrum_b200 import nn
+    from ferrum_b200.utils.runtime import check_status
+
+    torch.manual_seed(1)
+    conv = nn.Conv2d(8, 16, k, 1, pad, dil, device=fb.Device.Cuda(0))
+    x = torch.randn(2, 8, 13, 17, device="cuda", requires_grad=True)
+    with fb.autocast():
+        y = conv(x)
+    xd, wd, bd = (t.detach().double().requires_grad_(True) for t in (_r16(x.detach()), _r16(conv.weight.detach()), conv.bias))
+    want = torch.nn.functional.conv2d(torch.nn.functional.pad(xd, (pad[1], pad[1], pad[0], pad[0])), wd, bd, 1, 0, dil)
+    gy = torch.randn_like(y)
+    y.backward(gy)
+    want.backward(_r16(gy))
+    check_status()
+    for got, ref in ((y.detach(), want.detach()), (x.grad, xd.grad), (conv.weight.grad, wd.grad), (conv.bias.grad, bd.grad)):
+        _close(got, ref)
