@@ -243,8 +243,11 @@ nhwc_to_nchw_f32_kernel(const float* __restrict__ x, const float* __restrict__ a
 bool s2d_ok(int B, const S2d& g) {
   return B > 0 && g.C > 0 && g.H > 0 && g.W > 0 && g.sh > 0 && g.sw > 0 && g.eh > 0 && g.eh <= g.sh && g.ew > 0 &&
          g.ew <= g.sw && g.ph >= 0 && g.pw >= 0 && g.Hz > 0 && g.Wz > 0 &&
-         g.ld >= static_cast<long long>(g.eh) * g.ew * g.C && static_cast<long long>(B) * g.H < 0x7fffffffll &&
-         (g.W + 31) / 32 <= 65535 && (g.C + 31) / 32 <= 65535;
+         g.ld >= static_cast<long long>(g.eh) * g.ew * g.C && (g.C + 31) / 32 <= 65535;
+}
+// What the grid of s2d_to_nchw_kernel holds.
+bool s2d_grid_ok(int B, const S2d& g) {
+  return static_cast<long long>(B) * g.H < 0x7fffffffll && g.W <= 65535 * 32;
 }
 
 // Elements of a filter matrix of `rows` rows, 0 where the kernels' 32-bit indices would not do.
@@ -262,8 +265,8 @@ int filter_total(const Filter& f, int rows) {
 extern "C" int fb_conv_pack_input(const float* x, const float* mask, void* z, int B, int C, int H, int W, int sh, int sw,
                                   int eh, int ew, int ph, int pw, int Hz, int Wz, long long ld, cudaStream_t stream) {
   fb::S2d g{C, H, W, sh, sw, eh, ew, ph, pw, Hz, Wz, ld};
-  if (!fb::s2d_ok(B, g)) return -1;
-  const bool plain = sh == 1 && sw == 1 && ph == 0 && pw == 0 && Hz == H && Wz == W;
+  const bool plain = sh == 1 && sw == 1 && ph == 0 && pw == 0 && Hz == H && Wz == W;  // images and rows of any size
+  if (!fb::s2d_ok(B, g) || (!plain && !fb::s2d_grid_ok(B, g))) return -1;
   if (plain && static_cast<long long>(H) * W < 0x7fffffffll - 64) {  // rows are contiguous: one long row per image
     g.W = g.Wz = H * W;
     g.H = g.Hz = 1;
@@ -314,7 +317,7 @@ extern "C" int fb_conv_fold_wgrad(const float* part, float* dw, int splits, int 
 extern "C" int fb_s2d_nhwc_to_nchw_f32(const float* z, float* x, int B, int C, int H, int W, int sh, int sw, int eh,
                                        int ew, int ph, int pw, int Hz, int Wz, long long ld, cudaStream_t stream) {
   const fb::S2d g{C, H, W, sh, sw, eh, ew, ph, pw, Hz, Wz, ld};
-  if (!fb::s2d_ok(B, g)) return -1;
+  if (!fb::s2d_ok(B, g) || !fb::s2d_grid_ok(B, g)) return -1;
   dim3 grid(static_cast<unsigned>(B) * H, static_cast<unsigned>((W + 31) / 32), static_cast<unsigned>((C + 31) / 32));
   fb::s2d_to_nchw_kernel<<<grid, 256, 0, stream>>>(z, x, g);
   return static_cast<int>(cudaGetLastError());

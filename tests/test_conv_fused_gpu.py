@@ -103,3 +103,26 @@ def test_negative_padding(k, pad, dil):
     check_status()
     for got, ref in ((y.detach(), want.detach()), (x.grad, xd.grad), (conv.weight.grad, wd.grad), (conv.bias.grad, bd.grad)):
         _close(got, ref)
+
+
+def test_long_sequences():
+    """Conv1d over more than 2^21 samples (an image of one row)."""
+    import ferrum_b200 as fb
+    from ferrum_b200 import nn
+    from ferrum_b200.utils.runtime import check_status
+
+    torch.manual_seed(2)
+    conv = nn.Conv1d(1, 2, 5, 1, 2, device=fb.Device.Cuda(0))
+    x = torch.randn(1, 1, 2 ** 21 + 77, device="cuda", requires_grad=True)
+    with fb.autocast():
+        y = conv(x)
+    xd, wd, bd = (t.detach().double().requires_grad_(True) for t in (_r16(x.detach()), _r16(conv.weight.detach()), conv.bias))
+    want = torch.nn.functional.conv1d(xd, wd, bd, 1, 2)
+    gy = torch.randn_like(y)
+    y.backward(gy)
+    want.backward(_r16(gy))
+    check_status()
+    _close(y.detach(), want.detach()), _close(x.grad, xd.grad)
+    # 64 partial sums of 2^15 products (about 2^7.5), 16 of them added at a time, truncated by 2^-23 of the sum so far: at
+    # most 2^6 2^11 2^-23 2^7.5 = 2^1.5 in a gradient of about 2^10.5
+    assert (conv.weight.grad.double() - wd.grad).norm() <= 2.0 ** -9 * wd.grad.norm()
