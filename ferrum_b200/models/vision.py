@@ -7,7 +7,7 @@ from __future__ import annotations
 import torch
 
 from .. import nn
-from ..nn.conv import AdaptiveAvgPool2d, Conv2d, MaxPool2d, conv_fused
+from ..nn.conv import AdaptiveAvgPool2d, Conv2d, MaxPool2d, bare, conv_fused
 from ..ops import functional as F
 
 
@@ -26,7 +26,8 @@ class BasicBlock(nn.Module):
     @nn.tensor_io
     def forward(self, x):
         identity = self.downsample(x) if self.downsample is not None else x
-        y = conv_fused(self.conv1, x, act="relu")
+        # the fused node reads its result in the backward pass: not where a hook of conv2 may write to it
+        y = conv_fused(self.conv1, x, act="relu") if bare(self.conv2) else F.unary(self.conv1(x), "relu")
         return F.unary(conv_fused(self.conv2, y, add=identity), "relu")
 
 

@@ -93,7 +93,7 @@ class Conv2d(Module):
         return conv2d(x, self.weight, self.bias, self._stride, self._padding, self.dilation, self.groups)
 
 
-def _bare(m) -> bool:
+def bare(m) -> bool:
     """True when calling ``m`` runs ``Conv2d.forward`` and nothing else: no subclass, no hooks."""
     g = torch.nn.modules.module
     return (type(m) is Conv2d and "forward" not in m.__dict__
@@ -104,9 +104,10 @@ def _bare(m) -> bool:
 
 def conv_fused(conv, x, add=None, act=None):
     """``act(conv(x))`` (``act``: "relu") or ``conv(x) + add``, in the convolution's last kernel where that runs as an
-    implicit GEMM, else as ops of their own."""
+    implicit GEMM, else as ops of their own.  With ``act`` the result is kept for the backward pass and may not be
+    changed in place."""
     w = conv.weight
-    if (_bare(conv) and x.dim() == 4 and x.shape[1] == w.shape[1] * conv.groups
+    if (bare(conv) and x.dim() == 4 and x.shape[1] == w.shape[1] * conv.groups
             and F.conv_igemm_ok(x, conv._stride, conv.dilation, conv._padding, conv.kernel_size, conv.groups)):
         size = (x.shape[0], w.shape[0]) + _out_hw(x, conv.kernel_size, conv._stride, conv._padding, conv.dilation)
         if add is None or (tuple(add.shape) == size and add.device == x.device

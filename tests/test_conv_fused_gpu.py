@@ -126,3 +126,27 @@ def test_long_sequences():
     # 64 partial sums of 2^15 products (about 2^7.5), 16 of them added at a time, truncated by 2^-23 of the sum so far: at
     # most 2^6 2^11 2^-23 2^7.5 = 2^1.5 in a gradient of about 2^10.5
     assert (conv.weight.grad.double() - wd.grad).norm() <= 2.0 ** -9 * wd.grad.norm()
+
+
+def test_in_place_change_in_front_of_the_second_convolution():
+    """A hook of conv2 may change what the block's ReLU wrote."""
+    import ferrum_b200 as fb
+    from ferrum_b200.models import BasicBlock
+
+    torch.manual_seed(3)
+    block = BasicBlock(8, 16, 2, device=fb.Device.Cuda(0))
+    x = torch.randn(2, 8, 14, 14, device="cuda")
+
+    def grads(hook):
+        h = block.conv2.register_forward_pre_hook(hook)
+        for p in block.torch_parameters():
+            p.grad = None
+        with fb.autocast():
+            block(x).sum().backward()
+        h.remove()
+        return [p.grad.clone() for p in block.torch_parameters()]
+
+    got = grads(lambda m, a: (a[0].mul_(0.5),))
+    want = grads(lambda m, a: (a[0] * 0.5,))
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
