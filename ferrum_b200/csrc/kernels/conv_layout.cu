@@ -121,13 +121,15 @@ __device__ __forceinline__ int filter_at(const Filter& f, int I, int J, int ch, 
   return rh < f.eh && ki < f.kh && kj < f.kw ? ki * f.kw + kj : -1;
 }
 
-// kDgrad = false: out[o][I, J][ch] (pitch >= eh ew C); true: out[ch][I, J flipped][o] (pitch >= O).
-template <bool kDgrad>
+// kDgrad = false: out[o][I, J][ch] (pitch >= eh ew C); true: out[ch][I, J flipped][o] (pitch >= O).  Index: int, or 64
+// bits for filters beyond that.
+template <bool kDgrad, typename Index>
 __global__ void __launch_bounds__(256)
-pack_filters_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ out, const Filter f, int total) {
-  for (int at = blockIdx.x * 256 + threadIdx.x; at < total; at += gridDim.x * 256) {
-    const int k = at % f.pitch, rt = at / f.pitch, taps = f.k2h * f.k2w, row = rt / taps;
-    int tap = rt - row * taps;
+pack_filters_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ out, const Filter f, Index total) {
+  for (Index at = blockIdx.x * 256 + threadIdx.x; at < total; at += gridDim.x * 256) {
+    const Index rt = at / f.pitch;
+    const int k = static_cast<int>(at - rt * f.pitch), taps = f.k2h * f.k2w, row = static_cast<int>(rt / taps);
+    int tap = static_cast<int>(rt - static_cast<Index>(row) * taps);
     if (kDgrad) tap = taps - 1 - tap;
     const int I = tap / f.k2w, J = tap - I * f.k2w, ch = kDgrad ? row : k, o = kDgrad ? k : row;
     int c;
@@ -138,11 +140,13 @@ pack_filters_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ out
 }
 
 // dw[o, c, ki, kj] = sum over the splits of part[split][o][I, J][ch], in their order.
+template <typename Index>
 __global__ void __launch_bounds__(256)
-fold_wgrad_kernel(const float* __restrict__ part, float* __restrict__ dw, const Filter f, int splits, int total) {
-  for (int at = blockIdx.x * 256 + threadIdx.x; at < total; at += gridDim.x * 256) {
-    const int ch = at % f.pitch, rt = at / f.pitch, taps = f.k2h * f.k2w, o = rt / taps, tap = rt - o * taps;
-    const int I = tap / f.k2w, J = tap - I * f.k2w;
+fold_wgrad_kernel(const float* __restrict__ part, float* __restrict__ dw, const Filter f, int splits, Index total) {
+  for (Index at = blockIdx.x * 256 + threadIdx.x; at < total; at += gridDim.x * 256) {
+    const Index rt = at / f.pitch;
+    const int ch = static_cast<int>(at - rt * f.pitch), taps = f.k2h * f.k2w, o = static_cast<int>(rt / taps);
+    const int tap = static_cast<int>(rt - static_cast<Index>(o) * taps), I = tap / f.k2w, J = tap - I * f.k2w;
     int c;
     const int t = filter_at(f, I, J, ch, c);
     if (t < 0) continue;
@@ -250,11 +254,21 @@ bool s2d_grid_ok(int B, const S2d& g) {
   return static_cast<long long>(B) * g.H < 0x7fffffffll && g.W <= 65535 * 32;
 }
 
-// Elements of a filter matrix of `rows` rows, 0 where the kernels' 32-bit indices would not do.
-int filter_total(const Filter& f, int rows) {
+// Elements of a filter matrix of `rows` rows; 0: no such filter.
+long long filter_total(const Filter& f, int rows) {
   if (f.O <= 0 || f.C <= 0 || f.kh <= 0 || f.kw <= 0 || f.sh <= 0 || f.sw <= 0 || f.eh <= 0 || f.ew <= 0) return 0;
-  const long long n = static_cast<long long>(rows) * f.k2h * f.k2w * f.pitch;
-  return n > 0 && n < 0x7f000000ll ? static_cast<int>(n) : 0;
+  return static_cast<long long>(rows) * f.k2h * f.k2w * f.pitch;
+}
+// Launches `kernel` for each element, with 32-bit indices where they and a step of the grid beyond them fit.
+template <typename K32, typename K64, typename... A>
+int for_each_tap(K32 k32, K64 k64, long long total, cudaStream_t stream, A... args) {
+  const long long blocks = (total + 255) / 256;
+  const int grid = static_cast<int>(blocks < 1184 ? blocks : 1184);
+  if (total < 0x7f000000ll)
+    k32<<<grid, 256, 0, stream>>>(args..., static_cast<int>(total));
+  else
+    k64<<<grid, 256, 0, stream>>>(args..., total);
+  return static_cast<int>(cudaGetLastError());
 }
 
 }  // namespace
@@ -290,14 +304,14 @@ extern "C" int fb_conv_pack_filters(const float* w, void* out, int O, int C, int
                                     int ew, int pitch, int dgrad, cudaStream_t stream) {
   if (sh <= 0 || sw <= 0) return -1;
   const fb::Filter f{O, C, kh, kw, sh, sw, eh, ew, (kh + sh - 1) / sh, (kw + sw - 1) / sw, pitch};
-  const int rows = dgrad ? eh * ew * C : O, total = fb::filter_total(f, rows);
-  if (total == 0 || pitch < (dgrad ? O : eh * ew * C)) return -1;
-  const int blocks = (total + 255) / 256, grid = blocks < 1184 ? blocks : 1184;
-  if (dgrad)
-    fb::pack_filters_kernel<true><<<grid, 256, 0, stream>>>(w, static_cast<__nv_bfloat16*>(out), f, total);
-  else
-    fb::pack_filters_kernel<false><<<grid, 256, 0, stream>>>(w, static_cast<__nv_bfloat16*>(out), f, total);
-  return static_cast<int>(cudaGetLastError());
+  const int rows = dgrad ? eh * ew * C : O;
+  const long long total = fb::filter_total(f, rows);
+  if (total <= 0 || pitch < (dgrad ? O : eh * ew * C)) return -1;
+  __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
+  return dgrad ? fb::for_each_tap(fb::pack_filters_kernel<true, int>, fb::pack_filters_kernel<true, long long>, total,
+                                  stream, w, o, f)
+               : fb::for_each_tap(fb::pack_filters_kernel<false, int>, fb::pack_filters_kernel<false, long long>, total,
+                                  stream, w, o, f);
 }
 
 // part [splits, O, k2h * k2w, pitch] -> dw [O, C, kh, kw].
@@ -305,11 +319,9 @@ extern "C" int fb_conv_fold_wgrad(const float* part, float* dw, int splits, int 
                                   int eh, int ew, int pitch, cudaStream_t stream) {
   if (sh <= 0 || sw <= 0) return -1;
   const fb::Filter f{O, C, kh, kw, sh, sw, eh, ew, (kh + sh - 1) / sh, (kw + sw - 1) / sw, pitch};
-  const int total = fb::filter_total(f, O);
-  if (total == 0 || splits <= 0 || pitch < eh * ew * C) return -1;
-  const int blocks = (total + 255) / 256, grid = blocks < 1184 ? blocks : 1184;
-  fb::fold_wgrad_kernel<<<grid, 256, 0, stream>>>(part, dw, f, splits, total);
-  return static_cast<int>(cudaGetLastError());
+  const long long total = fb::filter_total(f, O);
+  if (total <= 0 || splits <= 0 || pitch < eh * ew * C) return -1;
+  return fb::for_each_tap(fb::fold_wgrad_kernel<int>, fb::fold_wgrad_kernel<long long>, total, stream, part, dw, f, splits);
 }
 
 // x[b, c, i, j] = z[b, (i + ph) / sh, (j + pw) / sw, (((i + ph) % sh) * ew + (j + pw) % sw) * C + c], zero where no

@@ -150,3 +150,22 @@ def test_in_place_change_in_front_of_the_second_convolution():
     want = grads(lambda m, a: (a[0] * 0.5,))
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+def test_filters_of_more_than_2_to_the_31():
+    """Packing and folding alone, one channel padded to eight."""
+    from ferrum_b200 import _lib
+
+    lib, st, O = _lib.cuda(), torch.cuda.current_stream().cuda_stream, 2 ** 28 + 5
+    w = torch.arange(O, device="cuda", dtype=torch.int32).remainder_(251).float()
+    out = torch.full((O, 8), 3.0, device="cuda", dtype=torch.bfloat16)
+    _lib.check(lib.fb_conv_pack_filters(w.data_ptr(), out.data_ptr(), O, 1, 1, 1, 1, 1, 1, 1, 8, 0, st), "fb_conv_pack_filters")
+    assert torch.equal(out[:, 0].float(), w) and not out[:, 1:].any()
+    del out
+    part = torch.full((1, O, 8), 3.0, device="cuda")
+    part[0, :, 0] = w
+    dw = torch.full((O,), 7.0, device="cuda")
+    _lib.check(lib.fb_conv_fold_wgrad(part.data_ptr(), dw.data_ptr(), 1, O, 1, 1, 1, 1, 1, 1, 1, 8, st), "fb_conv_fold_wgrad")
+    assert torch.equal(dw, w)
+    del part, dw
+    torch.cuda.empty_cache()
