@@ -15,8 +15,9 @@
 // partial[nblk][3][cols]; a second kernel folds the partials.  Register budgets are
 // kept small enough for two to four 256-thread blocks per SM: these kernels are
 // bandwidth-bound and need the bytes in flight.
-// Generic path (odd widths, very wide rows): scalar accesses, re-reads the row,
-// column sums by atomicAdd.
+// Rows of odd width or address: a row lives in registers there, too, element by
+// element (ln_*_any_kernel), or is re-read, with column sums by atomicAdd
+// (ln_*_generic), whichever is faster for its size; see any_fwd and any_bwd.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -968,7 +969,7 @@ ln_fold_kernel(const float* __restrict__ partial, float* __restrict__ stats, int
   }
 }
 
-// ---------------------------------------------------------------- rows of any width and alignment, up to 8192 columns
+// ---------------------------------------------------------------- rows of any width and alignment in registers
 // Widths that are no multiple of 8 (or bases off 16 bytes): TPR threads share a row, thread t owns columns t, t + TPR,
 // ...  (K of them, in registers), so every access of a warp is one contiguous run whatever the row's address.  A row is
 // read once; the column sums stay in registers over a block's rows, meet in shared memory and then in ln_fold_kernel.
@@ -1089,7 +1090,7 @@ ln_bwd_any_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __
   }
 }
 
-// ---------------------------------------------------------------- wider rows
+// ---------------------------------------------------------------- rows of any width, re-read
 template <typename T>
 __global__ void ln_fwd_generic(const T* __restrict__ x, const float* __restrict__ gamma,
                                const float* __restrict__ beta, T* __restrict__ y, float* __restrict__ mean_out,
@@ -1197,15 +1198,40 @@ bool geometry_any(int cols, Geo* g) {
   else *g = {256, 32};
   return true;
 }
-#define FB_LN_ANY(g, RUN)                            \
+#define FB_LN_ANY(g, RUN, WIDER)                     \
   do {                                               \
     if ((g).k == 2) RUN(32, 2);                      \
     else if ((g).tpr == 32) RUN(32, 8);              \
     else if ((g).tpr == 128) RUN(128, 8);            \
     else if ((g).k == 8) RUN(256, 8);                \
-    else if ((g).k == 16) RUN(256, 16);              \
-    else RUN(256, 32);                               \
+    else WIDER;                                      \
   } while (0)
+
+// Where rows of odd width or address are held in registers (any) rather than re-read (generic).  us, generic / any.
+// Forward: reading a row three times costs little while it stays in the cache and two blocks' reads overlap; registers
+// for 16 or 32 elements a thread leave fewer blocks per SM than the rows want.  fp32, 8192 rows: 257 columns 22.7 / 14.3,
+// 1025 26.8 / 23.4, 2049 37 / 52, 4095 70 / 77; 1301 columns: 592 rows 6.3 / 6.3, 1024 6.3 / 8.3, 2048 10.4 / 10.4; 3001:
+// 444 rows 8.3 / 6.3, 777 8.3 / 9.7; 7001: 150 rows 10.8 / 10.4, 300 11.5 / 12.6, 2048 29 / 43.  A GELU in front is
+// evaluated once instead of three times: 4095 columns, 8192 rows 130 / 84; 7001: 300 rows 16.5 / 15.8, 777 27 / 23, but
+// 4097: 300 rows 10.9 / 12.6, 777 16.5 / 18.6.
+bool any_fwd(long long rows, int cols, int pre_act) {
+  const long long sm = sm_count();
+  if (cols > 8192) return false;
+  if (pre_act == FB_ACT_GELU) return cols <= 4096 || rows <= sm || rows > 4 * sm;
+  if (cols <= 1024) return true;
+  if (cols <= 2048) return rows <= 4 * sm || rows > 8 * sm;
+  return rows <= (cols <= 4096 ? 3 : 1) * sm;
+}
+// Backward: for few rows the atomics are cheaper than a second launch; wide rows in registers leave one block per SM.
+// bf16, 129 columns: 300 rows 8.3 / 12.4, 777 13.3 / 12.4, 8192 92 / 17; 65: 1024 rows 10.8 / 12.4, 2048 18.5 / 12.4; 1001:
+// 300 rows 11.4 / 13.4, 444 13.4 / 13.5, 592 15.5 / 13.5, 8192 122 / 40; 1801, 8192 rows 134 / 120; 2047: 2048 rows 42 / 32,
+// 8192 137 / 163; 4097: 2048 rows 64 / 109.  fp32 rows up to 4096: 777 x 2049 25 / 22, 8192 x 2049 151 / 137, 8192 x 4095 194
+// / 158; behind a GELU 148 - 251 (the atomics' time varies) / 183 - 205 in that range; 2048 x 4097 70 / 139.
+bool any_bwd(long long rows, int cols, bool low) {
+  const long long sm = sm_count();
+  if (rows <= (cols <= 128 ? 8 : cols <= 256 ? 6 : 3) * sm) return false;
+  return cols <= (!low ? 4096 : rows <= 16 * sm ? 2048 : 1792);
+}
 bool aligned16(const void* a, const void* b, const void* c, const void* d) {
   return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) |
            reinterpret_cast<uintptr_t>(d)) & 15) == 0;
@@ -1337,12 +1363,12 @@ int fwd_t(const void* x, const float* gamma, const float* beta, void* y, float* 
     else if (g.k == 2) FB_LN_FWD(256, 2);
     else FB_LN_FWD(256, 4);
 #undef FB_LN_FWD
-  } else if (geometry_any(cols, &g)) {
+  } else if (any_fwd(rows, cols, pre_act) && geometry_any(cols, &g)) {
     const long long nb = (rows + 256 / g.tpr - 1) / (256 / g.tpr);
     const int grid = static_cast<int>(nb < sm_count() * 8LL ? nb : sm_count() * 8LL);
 #define FB_LN_FWD(TPR, K) \
   ln_fwd_any_kernel<T, TPR, K><<<grid, 256, 0, st>>>(xp, gamma, beta, yp, mean, rstd, rows, cols, eps, pre_act)
-    FB_LN_ANY(g, FB_LN_FWD);
+    FB_LN_ANY(g, FB_LN_FWD, if (g.k == 16) FB_LN_FWD(256, 16); else FB_LN_FWD(256, 32));
 #undef FB_LN_FWD
   } else {
     const int grid = static_cast<int>(rows < sm_count() * 8LL ? rows : sm_count() * 8LL);
@@ -1411,7 +1437,7 @@ int bwd_t(const void* dy, const void* x, const void* act_grad, const float* gamm
                     aligned16(partial, stats, act_grad, dx_low);
   if (dx_low != nullptr && !fast) return -2;
   Geo any;
-  if (fast || (nblk > 0 && partial != nullptr && geometry_any(cols, &any))) {
+  if (fast || (nblk > 0 && partial != nullptr && any_bwd(rows, cols, sizeof(T) == 2) && geometry_any(cols, &any))) {
     int used = nblk;
     const int nvec = cols / 8;
     const int wide_blocks = nblk / 2 < sm_count() ? nblk / 2 : sm_count();  // two rows of partial[] per block
@@ -1423,7 +1449,7 @@ int bwd_t(const void* dy, const void* x, const void* act_grad, const float* gamm
 #define FB_LN_BWD(TPR, K) \
   ln_bwd_any_kernel<T, TPR, K><<<nblk, 256, 0, st>>>(dyp, xp, agp, gamma, mean, rstd, dxp, partial, rows, cols, pre_act, \
                                                      want_colsum)
-      FB_LN_ANY(any, FB_LN_BWD);
+      FB_LN_ANY(any, FB_LN_BWD, if constexpr (sizeof(T) == 4) FB_LN_BWD(256, 16));
 #undef FB_LN_BWD
     } else {
 #define FB_LN_BWD(TPR, K) \
@@ -1461,11 +1487,11 @@ using namespace fb;
 // Status block (host-mapped, see common/status.h) that the bounded waits of the wide-row kernels report to.
 extern "C" void fb_layernorm_set_status(int32_t* status) { g_ln_status = status; }
 
-// Number of blocks (= rows of `partial`, each 3 * cols floats) the backward uses; 0 (more than 8192 columns) means that
-// the generic path runs and no partial buffer is needed.
+// Number of blocks (= rows of `partial`, each 3 * cols floats) the backward uses; 0 means that the generic path runs and
+// no partial buffer is needed.
 extern "C" int fb_layernorm_bwd_blocks(long long rows, int cols) {
   Geo g;
-  if (!geometry(cols, &g) && !geometry_any(cols, &g)) return 0;
+  if (!geometry(cols, &g) && !(any_bwd(rows, cols, false) && geometry_any(cols, &g))) return 0;
   const long long rpb = 256 / g.tpr;
   const long long nb = (rows + rpb - 1) / rpb;
   // Three blocks per SM where a thread holds one vector of a row: loads in flight, not registers, are what is short.

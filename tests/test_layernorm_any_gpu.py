@@ -11,7 +11,11 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rows,cols", [(1, 1), (3, 33), (130, 63), (7, 65), (900, 256), (5, 255), (64, 257), (700, 512),
                                        (777, 1001), (1500, 1024), (9, 1023), (4, 1025), (6, 2047), (300, 2048), (5, 2049),
-                                       (3, 4095), (2, 4097), (3, 8191), (2, 8193)])
+                                       (3, 4095), (2, 4097), (3, 8191), (2, 8193),
+                                       # where the rows that are held in registers end
+                                       (888, 129), (889, 129), (1184, 127), (1185, 127), (593, 1793), (2369, 1795),
+                                       (444, 2049), (445, 2049), (593, 4095), (444, 257), (445, 257), (593, 1025), (1185, 1025), (149, 4097),
+                                       (593, 4097)])
 @pytest.mark.parametrize("pre", [None, "gelu"])
 def test_against_fp64(rows, cols, dtype, pre):
     from ferrum_b200.ops import functional as F
