@@ -430,13 +430,20 @@ ln_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
   }
 }
 
+template <int N>
+__device__ __forceinline__ void st_piece(float* p, const float* v) {
+  if constexpr (N == 2) *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
+  else *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+
 // Backward.  x and dy stay packed in registers between the statistics pass and the output pass; the
 // three column partials (dy*xhat, dy, dx) accumulate in registers over all rows the block visits and are
-// written once to partial[blockIdx][3][cols].  dx_low (optional): dx once more in bf16, the gradient of a residual's branch.
+// written once to partial[blockIdx][3][cols].  kLow: dx once more in bf16, the gradient of a residual's branch (K = 4: if there
+// is a dx_low; that instance spills least).
 // Bound by loads in flight, hence three blocks per SM where a thread holds one vector, and for few rows by the rows of a
 // block adding up, which they do in shared memory (one after the other through global memory each waited for the one
 // before).  fp32: 128 x 256 10.9 -> 4.4 us, 1024 x 1024 13.1 -> 8.8, 8192 x 1024 with dx_low 36.8 -> 31.7.
-template <typename T, int TPR, int K>
+template <typename T, int TPR, int K, bool kLow>
 __global__ void __launch_bounds__(256, K == 1 ? 3 : 2)
 ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ act_grad,
               const float* __restrict__ gamma, const float* __restrict__ mean, const float* __restrict__ rstd,
@@ -534,7 +541,7 @@ ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __rest
           for (int i = 0; i < 8; ++i) acc_c[k][i] += o[i];
         }
         V8<T>::st(dx + row * cols + vi * 8, o);
-        if (dx_low != nullptr) V8<__nv_bfloat16>::st(dx_low + row * cols + vi * 8, o);
+        if (kLow && (K < 4 || dx_low != nullptr)) V8<__nv_bfloat16>::st(dx_low + row * cols + vi * 8, o);
       }
     }
 #pragma unroll
@@ -548,36 +555,53 @@ ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __rest
   float* pg = partial + static_cast<long long>(blockIdx.x) * 3 * cols;
   float* pb = pg + cols;
   float* pc = pb + cols;
-  // Several row slots own the same columns: they add up in shared memory, one slot at a time, and the last one stores.
-  __shared__ float cols_sum[3][kRowsPerBlock > 1 ? K * TPR * 8 : 1];
-#pragma unroll 1
-  for (int slot = 0; slot < kRowsPerBlock; ++slot) {
-    if (kRowsPerBlock > 1) __syncthreads();
-    if (sub != slot) continue;
+  if constexpr (kRowsPerBlock == 1) {
+    // K = 2 in pairs: 16-byte pieces cost the loop above 56 bytes of spills (fp32, 8192 x 3072 106 us instead of 99, though
+    // 300 x 4096 20.6 instead of 22.0); K = 4 spills either way (8192 x 8192 386 us, in pairs 431, element by element 520)
+    constexpr int kPiece = K == 2 ? 2 : 4;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       const int vi = t + k * TPR;
       if (vi >= nvec) continue;
-      if (slot > 0) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int at = (k * 8 + i) * TPR + t;
-          acc_g[k][i] = cols_sum[0][at] + acc_g[k][i];
-          acc_b[k][i] = cols_sum[1][at] + acc_b[k][i];
-          acc_c[k][i] = cols_sum[2][at] + acc_c[k][i];
-        }
+      for (int i = 0; i < 8; i += kPiece) {
+        st_piece<kPiece>(pg + vi * 8 + i, &acc_g[k][i]);
+        st_piece<kPiece>(pb + vi * 8 + i, &acc_b[k][i]);
+        st_piece<kPiece>(pc + vi * 8 + i, &acc_c[k][i]);
       }
-      if (slot + 1 == kRowsPerBlock) {
-        V8<float>::st(pg + vi * 8, acc_g[k]);
-        V8<float>::st(pb + vi * 8, acc_b[k]);
-        V8<float>::st(pc + vi * 8, acc_c[k]);
-      } else {
+    }
+  } else {
+    // Several row slots own the same columns: they add up in shared memory, one slot at a time, and the last one stores.
+    __shared__ float cols_sum[3][K * TPR * 8];
+#pragma unroll 1
+    for (int slot = 0; slot < kRowsPerBlock; ++slot) {
+      __syncthreads();
+      if (sub != slot) continue;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int at = (k * 8 + i) * TPR + t;
-          cols_sum[0][at] = acc_g[k][i];
-          cols_sum[1][at] = acc_b[k][i];
-          cols_sum[2][at] = acc_c[k][i];
+      for (int k = 0; k < K; ++k) {
+        const int vi = t + k * TPR;
+        if (vi >= nvec) continue;
+        if (slot > 0) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int at = (k * 8 + i) * TPR + t;
+            acc_g[k][i] = cols_sum[0][at] + acc_g[k][i];
+            acc_b[k][i] = cols_sum[1][at] + acc_b[k][i];
+            acc_c[k][i] = cols_sum[2][at] + acc_c[k][i];
+          }
+        }
+        if (slot + 1 == kRowsPerBlock) {
+          V8<float>::st(pg + vi * 8, acc_g[k]);
+          V8<float>::st(pb + vi * 8, acc_b[k]);
+          V8<float>::st(pc + vi * 8, acc_c[k]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int at = (k * 8 + i) * TPR + t;
+            cols_sum[0][at] = acc_g[k][i];
+            cols_sum[1][at] = acc_b[k][i];
+            cols_sum[2][at] = acc_c[k][i];
+          }
         }
       }
     }
@@ -931,7 +955,9 @@ ln_bwd_ring_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
 }
 
 // Fold partial[nblk][3*cols] into stats[3*cols] (accumulated into): block = 128 columns x a chunk of the
-// nblk rows, lanes own 4 adjacent columns, partials leave with one atomicAdd per column per block.
+// nblk rows, lanes own 4 adjacent columns, partials leave with one atomicAdd per column per block.  kVec: 16-byte loads
+// (ncols a multiple of 4, partial on a 16-byte address).
+template <bool kVec>
 __global__ void __launch_bounds__(256)
 ln_fold_kernel(const float* __restrict__ partial, float* __restrict__ stats, int nblk, int ncols,
                int rows_per_block) {
@@ -941,7 +967,7 @@ ln_fold_kernel(const float* __restrict__ partial, float* __restrict__ stats, int
   const int r_lo = blockIdx.y * rows_per_block;
   const int r_hi = min(nblk, r_lo + rows_per_block);
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-  if ((ncols & 3) != 0 || (reinterpret_cast<uintptr_t>(partial) & 15) != 0) {
+  if constexpr (!kVec) {
     for (int r = r_lo + warp; r < r_hi; r += 8) {
       const float* v = partial + static_cast<long long>(r) * ncols + c0;
       if (c0 < ncols) a.x += v[0];
@@ -1452,9 +1478,11 @@ int bwd_t(const void* dy, const void* x, const void* act_grad, const float* gamm
       FB_LN_ANY(any, FB_LN_BWD, if constexpr (sizeof(T) == 4) FB_LN_BWD(256, 16));
 #undef FB_LN_BWD
     } else {
-#define FB_LN_BWD(TPR, K) \
-  ln_bwd_kernel<T, TPR, K><<<nblk, 256, 0, st>>>(dyp, xp, agp, gamma, mean, rstd, dxp, dx_low, partial, rows, cols, \
-                                                 pre_act, want_colsum)
+      const auto run = [&](auto plain, auto low) {
+        (dx_low != nullptr ? low : plain)<<<nblk, 256, 0, st>>>(dyp, xp, agp, gamma, mean, rstd, dxp, dx_low, partial, rows,
+                                                                cols, pre_act, want_colsum);
+      };
+#define FB_LN_BWD(TPR, K) run(ln_bwd_kernel<T, TPR, K, K == 4>, ln_bwd_kernel<T, TPR, K, K == 4 || sizeof(T) == 4>)
     if (g.tpr == 32 && g.k == 1) FB_LN_BWD(32, 1);
     else if (g.tpr == 32) FB_LN_BWD(32, 2);
     else if (g.tpr == 128 && g.k == 1) FB_LN_BWD(128, 1);
@@ -1470,7 +1498,8 @@ int bwd_t(const void* dy, const void* x, const void* act_grad, const float* gamm
     if (row_blocks > max_rb) row_blocks = max_rb;
     if (row_blocks < 1) row_blocks = 1;
     const int rpb = (used + row_blocks - 1) / row_blocks;
-    ln_fold_kernel<<<dim3(col_blocks, row_blocks), 256, 0, st>>>(partial, stats, used, ncols, rpb);
+    const auto fold = ncols % 4 == 0 && aligned16(partial, nullptr, nullptr, nullptr) ? ln_fold_kernel<true> : ln_fold_kernel<false>;
+    fold<<<dim3(col_blocks, row_blocks), 256, 0, st>>>(partial, stats, used, ncols, rpb);
   } else {
     const int grid = static_cast<int>(rows < sm_count() * 4LL ? rows : sm_count() * 4LL);
     ln_bwd_generic<T><<<grid, 256, 0, st>>>(dyp, xp, agp, gamma, mean, rstd, dxp, stats, rows, cols, pre_act,
