@@ -199,6 +199,9 @@ int fb_gru_gates_bwd(const float* dh, const float* saved, const float* h_prev, f
 // gates H] transposed recurrent matrix, hs [T, B, H]; hs_kept (a second hs, so that the first is the caller's) / cs /
 // saved / c_last as the backward call reads them (NULL: not kept).  Backward: w [gates H, H]; dxi and, for GRU, dhh [T, B, gates H].  h0, c0 and the incoming gradients may be NULL.
 int fb_rnn_seq_supported(int gates, int B, int H);
+// The instance that runs: batch rows per cluster (1, 2, 4, 8), + 16: weights in registers, + 32: a full share of them in
+// every thread (the unrolled product); 0: not supported.
+int fb_rnn_seq_plan(int gates, int B, int H, int backward);
 int fb_rnn_seq_fwd(int gates, const float* xi, const float* w_t, const float* bias, const float* h0, const float* c0,
                    float* hs, float* hs_kept, float* cs, float* saved, float* c_last, int T, int B, int H,
                    int32_t* status, cudaStream_t stream);

@@ -671,6 +671,13 @@ extern "C" int fb_rnn_seq_supported(int gates, int B, int H) {
   return (gates == 3 || gates == 4) && B > 0 && plan(gates, B, H, false, &f) && plan(gates, B, H, true, &b);
 }
 
+extern "C" int fb_rnn_seq_plan(int gates, int B, int H, int backward) {
+  Plan p;
+  if ((gates != 3 && gates != 4) || B < 1 || !plan(gates, B, H, backward != 0, &p)) return 0;
+  const bool full = p.reg && tile_of(p.rows4, backward ? gates * H : H, p.bs, true).vec4 == kKpt / (4 / p.bs);
+  return p.bs + (p.reg ? 16 : 0) + (full ? 32 : 0);
+}
+
 extern "C" int fb_rnn_seq_fwd(int gates, const float* xi, const float* w_t, const float* bias, const float* h0,
                               const float* c0, float* hs, float* hs_kept, float* cs, float* saved, float* c_last, int T,
                               int B, int H, int32_t* status, cudaStream_t stream) {

@@ -187,6 +187,7 @@ void bind_layers(py::module_& m) {
   m.def("embedding", &embedding);
   m.def("rnn_seq", &rnn_seq);
   m.def("rnn_seq_supported", [](int gates, int batch, int hidden) { return fb_rnn_seq_supported(gates, batch, hidden) != 0; });
+  m.def("rnn_seq_plan", &fb_rnn_seq_plan);
 }
 
 }  // namespace fbn

@@ -51,6 +51,25 @@ def test_sequence(kind, T, B, I, H, L, state):
 
 
 @pytest.mark.parametrize("kind", ["LSTM", "GRU"])
+@pytest.mark.parametrize("H,bs", [(256, 1), (256, 2), (256, 4), (128, 4), (256, 8)])
+def test_batch_slices(kind, H, bs):
+    """Every number of batch rows per cluster, the last slice whole and not; how many clusters the chip holds decides which
+    batches that are."""
+    from ferrum_b200 import _lib
+
+    gates = 4 if kind == "LSTM" else 3
+    plans = {B: [_lib.native().rnn_seq_plan(gates, B, H, back) for back in (0, 1)] for B in range(1, 200)}
+    sizes = [B for B, p in plans.items() if p[0] % 16 == p[1] % 16 == bs]
+    assert sizes, plans
+    if bs <= 4:  # weights in registers; for LSTM 256 (four rows of 16 weights per thread in either direction) unrolled
+        assert all(p & 16 for B in sizes for p in plans[B])
+        assert all(p & 32 for B in sizes for p in plans[B]) or H != 256 or kind != "LSTM"
+    whole = max(B for B in sizes if B % bs == 0)
+    for B in {whole, whole - 1, sizes[0]} & set(sizes):
+        test_sequence(kind, 3, B, 5, H, 1, True)
+
+
+@pytest.mark.parametrize("kind", ["LSTM", "GRU"])
 @pytest.mark.parametrize("how", ["cell_cls", "one_cell", "other_type"])
 def test_cells_of_the_users_own(kind, how):
     """A cell class with its own step, in every layer or in one, and a layer of another type than fp32: step by step."""
