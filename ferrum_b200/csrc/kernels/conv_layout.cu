@@ -4,7 +4,8 @@
 //
 // A convolution of any stride is one of stride 1 over a space-to-depth arrangement of its input:
 //   z[b, I, J, (rh * ew + rw) * C + c] = x[b, c, I * sh + rh - ph, J * sw + rw - pw],  rh < eh = min(sh, kh), rw < ew,
-// zero outside the image, with ceil(kh / sh) x ceil(kw / sw) filters.  Rows and columns that the stride skips altogether
+// zero outside the image, with ceil(kh / sh) x ceil(kw / sw) filters (taps past kh x kw are zeros: an infinity in x makes
+// NaN of the windows that only they reach).  Rows and columns that the stride skips altogether
 // (kernel < stride: the 1 x 1 shortcut of a residual block) are not in z.  Stride 1 is the case sh = sw = 1, ph = pw = 0:
 // a plain NCHW -> NHWC conversion, the padding being the TMA unit's zero fill.
 //

@@ -1069,39 +1069,6 @@ class _Im2colFn(Function):
         return dx, None, None, None, None
 
 
-def _pad8(n: int) -> int:
-    return (n + 7) // 8 * 8
-
-
-class _ConvS2dFn:
-    """The space-to-depth form of a strided convolution in plain torch: with
-    ``z[b, I, J, (rh, rw, c)] = x[b, c, I * sh + rh - ph, J * sw + rw - pw]`` the stride-(sh, sw) convolution with a
-    kh x kw filter IS a stride-1 convolution with a ceil(kh / sh) x ceil(kw / sw) filter over sh * sw * C channels (filter
-    taps that do not exist are zero).  What csrc/kernels/conv_layout.cu does on the GPU; there, rows and columns that the
-    stride skips altogether are left out."""
-
-    @staticmethod
-    def _geometry(x_shape, w_shape, stride, padding):
-        B, C, H, W = x_shape
-        O, _, kh, kw = w_shape
-        (sh, sw), (ph, pw) = stride, padding
-        Ho, Wo = (H + 2 * ph - kh) // sh + 1, (W + 2 * pw - kw) // sw + 1
-        k2h, k2w = -(-kh // sh), -(-kw // sw)
-        return Ho, Wo, k2h, k2w, Ho + k2h - 1, Wo + k2w - 1, _pad8(sh * sw * C)
-
-    @staticmethod
-    def _filters(weight, stride, k2h, k2w, Cz):
-        """[O, C, kh, kw] -> [O, k2h, k2w, Cz] fp32 in the channel order (rh, rw, c) of the space-to-depth input."""
-        O, C, kh, kw = weight.shape
-        sh, sw = stride
-        w = torch.zeros((O, C, k2h * sh, k2w * sw), device=weight.device, dtype=torch.float32)
-        w[:, :, :kh, :kw] = weight.detach().float()
-        w = w.view(O, C, k2h, sh, k2w, sw).permute(0, 2, 4, 3, 5, 1).reshape(O, k2h, k2w, sh * sw * C)
-        out = torch.zeros((O, k2h, k2w, Cz), device=weight.device, dtype=torch.float32)
-        out[..., :sh * sw * C] = w
-        return out
-
-
 def conv_igemm_ok(x: torch.Tensor, stride, dilation, padding, kernel, groups: int) -> bool:
     """True when ``conv2d`` can take the implicit-GEMM path: CUDA, bf16 autocast on, one group, and either stride 1
     with a data gradient whose padding ``dilation * (kernel - 1) - padding`` is not negative, or any stride without

@@ -30,3 +30,21 @@ def test_against_two_nodes(rows, cols, r_dtype):
     assert all(torch.equal(a, c) for a, c in zip(got[0][:3], got[1][:3]))
     for a, c in zip(got[0][3:], got[1][3:]):
         assert (a - c).norm() <= 2.0 ** -20 * c.norm()
+
+
+@pytest.mark.parametrize("r_dtype", [torch.float32, torch.bfloat16])
+def test_values_that_are_not_finite(r_dtype):
+    from ferrum_b200.ops import functional as F
+
+    got = []
+    for fused in (True, False):
+        g = torch.Generator(device="cuda").manual_seed(5)
+        x, r, w = (torch.randn(*s, device="cuda", generator=g) for s in ((9, 264), (9, 264), (264,)))
+        x[1, 3], r[4, 7], x[6, 0], r[6, 0] = float("inf"), float("nan"), float("inf"), float("-inf")
+        x, r = x.requires_grad_(True), r.to(r_dtype).requires_grad_(True)
+        y = F.add_layer_norm(x, r, w, None) if fused else F.layer_norm(F.binary(x, r, "add"), w, None)
+        y.backward(torch.ones_like(y))
+        got.append((y.detach(), x.grad, r.grad))
+    for a, b in zip(*got):
+        assert torch.equal(torch.isnan(a).any(1).nonzero().flatten().cpu(), torch.tensor([1, 4, 6]))
+        assert torch.equal(torch.nan_to_num(a), torch.nan_to_num(b))

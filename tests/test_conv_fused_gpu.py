@@ -169,3 +169,82 @@ def test_filters_of_more_than_2_to_the_31():
     assert torch.equal(dw, w)
     del part, dw
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("C,stride", [(8, 1), (65, 1), (3, 2)])
+@pytest.mark.parametrize("fused", ["relu", "add"])
+def test_values_that_are_not_finite(C, stride, fused):
+    """The bits of the convolution and the fused op as two nodes, in both directions; a value spoils its own windows, which
+    strides round up to a multiple of themselves (with zeros as filter taps)."""
+    import ferrum_b200 as fb
+    from ferrum_b200.ops import functional as F
+
+    g = torch.Generator(device="cuda").manual_seed(C)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    base, w = rand(2, C, 9, 10), rand(6, C, 3, 3)
+    s = (stride, stride)
+    with fb.autocast(), torch.no_grad():
+        clean = F.conv2d_igemm(base, w, None, (1, 1), (1, 1), s)
+    add, gy = rand(*clean.shape), rand(*clean.shape)
+    for value in (float("inf"), float("nan")):
+        x = base.clone()
+        x[1, C - 1, 4, 5] = value
+        results = []
+        for one in (True, False):
+            leaves = [t.clone().requires_grad_(True) for t in (x, w, add)]
+            with fb.autocast():
+                if one:
+                    y = F.conv2d_igemm(leaves[0], leaves[1], None, (1, 1), (1, 1), s,
+                                       leaves[2] if fused == "add" else None, "relu" if fused == "relu" else None)
+                else:
+                    z = F.conv2d_igemm(leaves[0], leaves[1], None, (1, 1), (1, 1), s)
+                    y = F.unary(z, "relu") if fused == "relu" else F.binary(z, leaves[2], "add")
+            y.backward(gy)
+            results.append([y.detach()] + [t.grad for t in leaves if t.grad is not None])
+        for a, b in zip(*results):
+            assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(torch.nan_to_num(a), torch.nan_to_num(b))
+        with fb.autocast(), torch.no_grad():
+            y = F.conv2d_igemm(x, w, None, (1, 1), (1, 1), s)
+        k = -(-3 // stride) * stride
+        bad = torch.nn.functional.pad((~torch.isfinite(x)).float().amax(1, keepdim=True), (1, k - 2, 1, k - 2))
+        hit = torch.nn.functional.max_pool2d(bad, k, stride)[:, :, :y.shape[2], :y.shape[3]].bool().expand_as(y)
+        assert torch.equal(~torch.isfinite(y), hit) and torch.equal(y[~hit], clean[~hit])
+
+
+@pytest.mark.parametrize("shape", range(8))
+def test_layouts(shape):
+    """The layout kernels against the same arrangements in plain torch: exact but for the rounding to bf16, padding zero."""
+    from ferrum_b200 import _lib
+
+    from tests import _conv_s2d as s2d
+
+    B, C, O, H, W, k, s, p = s2d.SHAPES[shape]
+    lib, st = _lib.cuda(), torch.cuda.current_stream().cuda_stream
+    x, w = torch.randn(B, C, H, W, device="cuda"), torch.randn(O, C, *k, device="cuda")
+    Ho, Wo, k2h, k2w, Hz, Wz, eh, ew, Cz = s2d.geometry(x.shape, w.shape, s, p)
+    sizes, bf = (B, C, H, W, *s, eh, ew, *p, Hz, Wz), dict(device="cuda", dtype=torch.bfloat16)
+    mask = torch.randn_like(x)
+    for m in (None, mask):
+        z = torch.full((B, Hz, Wz, Cz), 3.0, **bf)
+        _lib.check(lib.fb_conv_pack_input(x.data_ptr(), None if m is None else m.data_ptr(), z.data_ptr(), *sizes, Cz, st), "x")
+        assert torch.equal(z, s2d.pack_input(x if m is None else torch.where(m > 0, x, 0.0), w.shape, s, p).bfloat16())
+    filters = s2d.pack_filters(w, s, Cz)
+    packed, Op = torch.full(filters.shape, 3.0, **bf), -(-O // 8) * 8
+    _lib.check(lib.fb_conv_pack_filters(w.data_ptr(), packed.data_ptr(), O, C, *k, *s, eh, ew, Cz, 0, st), "w")
+    assert torch.equal(packed, filters.bfloat16())
+    turned = torch.full((eh * ew * C, k2h * k2w, Op), 3.0, **bf)
+    _lib.check(lib.fb_conv_pack_filters(w.data_ptr(), turned.data_ptr(), O, C, *k, *s, eh, ew, Op, 1, st), "w turned")
+    assert torch.equal(turned[..., :O], filters[..., :eh * ew * C].flip(1).permute(2, 1, 0).bfloat16())
+    assert not turned[..., O:].any()
+    part = torch.randn(3, *filters.shape, device="cuda")
+    dw = torch.full_like(w, 7.0)
+    _lib.check(lib.fb_conv_fold_wgrad(part.data_ptr(), dw.data_ptr(), 3, O, C, *k, *s, eh, ew, Cz, st), "dw")
+    assert torch.equal(s2d.pack_filters(dw, s, Cz), torch.where(s2d.pack_filters(torch.ones_like(w), s, Cz) > 0,
+                                                                part[0] + part[1] + part[2], 0.0))
+    back = torch.full_like(x, 7.0)
+    dz = torch.randn(B, Hz, Wz, eh * ew * C, device="cuda")
+    _lib.check(lib.fb_s2d_nhwc_to_nchw_f32(dz.data_ptr(), back.data_ptr(), *sizes, eh * ew * C, st), "dx")
+    reach = s2d.pack_input(torch.ones_like(x), w.shape, s, p)[..., :eh * ew * C] > 0
+    assert torch.equal(s2d.pack_input(back, w.shape, s, p)[..., :eh * ew * C], torch.where(reach, dz, 0.0))
+    # every value of z arrives once, the pixels that no window reaches are zero
+    assert back.count_nonzero() == reach.sum()

@@ -23,13 +23,15 @@ def test_gradient(vocab, n, dim, padding):
         _lib.check(lib.fb_embedding_keys(ids.data_ptr(), keys.data_ptr(), n, vocab, st), "fb_embedding_keys")
         ok = (ids >= 0) & (ids < vocab)
         assert torch.equal(keys.long(), torch.where(ok, ids, vocab))
-        key, perm = torch.sort(keys, stable=True)
-        dw = torch.zeros(vocab, dim, device="cuda")
-        _lib.check(lib.fb_embedding_bwd_sorted(dout.data_ptr(), key.data_ptr(), 4, perm.data_ptr(), dw.data_ptr(), n, dim, 1,
-                                               1.0, padding, vocab, 0, st), "fb_embedding_bwd_sorted")
-        check_status()
-        ok &= ids != padding
+        ok_grad = ok & (ids != padding)
         want, size = (torch.zeros(vocab, dim, device="cuda", dtype=torch.float64) for _ in range(2))
-        want.index_add_(0, ids[ok], dout[ok].double())
-        size.index_add_(0, ids[ok], dout[ok].double().abs())
-        assert ((dw - want).abs() <= 2.0 ** -22 * size * 8).all()
+        want.index_add_(0, ids[ok_grad], dout[ok_grad].double())
+        size.index_add_(0, ids[ok_grad], dout[ok_grad].double().abs())
+        for unsorted in (keys, torch.where(ok, ids, vocab)):  # 64 bits: tables of 2^31 - 1 rows and more
+            key, perm = torch.sort(unsorted, stable=True)
+            dw = torch.zeros(vocab, dim, device="cuda")
+            _lib.check(lib.fb_embedding_bwd_sorted(dout.data_ptr(), key.data_ptr(), key.element_size(), perm.data_ptr(),
+                                                   dw.data_ptr(), n, dim, 1, 1.0, padding, vocab, 0, st),
+                       "fb_embedding_bwd_sorted")
+            check_status()
+            assert ((dw - want).abs() <= 2.0 ** -22 * size * 8).all()

@@ -6,8 +6,11 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("other", [True, False])
 @pytest.mark.parametrize("rows,width,deep", [(16, 4096, 6), (1, 1024, 5), (64, 2048, 4), (33, 1032, 3)])
-def test_chain(rows, width, deep):
+def test_chain(rows, width, deep, other):
+    """``other``: a kernel that is nobody's dependent between the layers; without it every one waits for the one ahead,
+    which itself may still be waiting."""
     from ferrum_b200.ops import functional as F
     from ferrum_b200.ops import gemm  # noqa: F401
     from ferrum_b200 import _lib
@@ -27,7 +30,8 @@ def test_chain(rows, width, deep):
             x = F.layer_norm(y, gamma, beta)
             if sync:
                 torch.cuda.synchronize()
-            w.mul_(1.0)  # the next product's weights may have been written just now
+            if other:
+                w.mul_(1.0)  # the next product's weights may have been written just now
         return x
 
     with torch.no_grad():

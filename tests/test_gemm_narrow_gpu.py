@@ -29,5 +29,11 @@ def test_bits(M, N, K, b_mn):
     want = run(lib.fb_gemm_bf16, 0)
     ref = a.double() @ (b.double() if b_mn else b.double().t()) + bias.double()
     assert (want.double() - ref).norm() <= 2.0 ** -8 * ref.norm()
-    for tile in [0, 160, 192, 256] + [t for t in (16, 32, 64) if M <= t]:
+    tiles = [0, 160, 192, 256] + [t for t in (16, 32, 64) if M <= t]
+    for tile in tiles:
         assert torch.equal(run(lib.fb_gemm_bf16_narrow, tile), want), tile
+    a[0, K - 1] = float("inf")  # a row's alone
+    spoiled = run(lib.fb_gemm_bf16, 0)
+    assert not torch.isfinite(spoiled[0]).any() and torch.equal(spoiled[1:], want[1:])
+    for tile in tiles:
+        assert torch.equal(run(lib.fb_gemm_bf16_narrow, tile).view(torch.int16), spoiled.view(torch.int16)), tile

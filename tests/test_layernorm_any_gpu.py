@@ -38,3 +38,28 @@ def test_against_fp64(rows, cols, dtype, pre):
     # a row of one column has no gradient; next to none there, absolute
     for got, ref in zip(leaves, exact):
         assert (got.grad.double() - ref.grad).norm() <= 2 * tol * ref.grad.norm() + 1e-5 * rows ** 0.5
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,cols", [(5, 33), (600, 257), (889, 129), (593, 1001), (20, 4097)])
+def test_values_that_are_not_finite(rows, cols, dtype):
+    """A row with an infinity or a NaN is NaN; the others keep their bits."""
+    from ferrum_b200.ops import functional as F
+
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    base, gy, w = rand(rows, cols).to(dtype), rand(rows, cols).to(dtype), rand(cols)
+
+    def run(x):
+        x = x.clone().requires_grad_(True)
+        y = F.layer_norm(x, w, None)
+        y.backward(gy)
+        return y.detach(), x.grad
+
+    clean = run(base)
+    others = torch.arange(rows, device="cuda") != rows // 2
+    for value in (float("inf"), float("nan")):
+        x = base.clone()
+        x[rows // 2, cols - 1] = value
+        for got, want in zip(run(x), clean):
+            assert torch.isnan(got[rows // 2]).all() and torch.equal(got[others], want[others])

@@ -172,27 +172,23 @@ def test_new_switches_are_inert_without_a_gpu():
 
 
 def test_space_to_depth_filters_reproduce_a_strided_convolution():
-    """The host-side half of the strided implicit-GEMM convolution, on the CPU: with the input rearranged as
-    z[b, I, J, (rh, rw, c)] = x_padded[b, c, I * sh + rh, J * sw + rw] and the filters rearranged by
-    ``_ConvS2dFn._filters``, a stride-1 convolution of z equals the strided convolution of x; the weight-gradient
-    mapping back is the exact inverse."""
+    """The arrangement that the layout kernels of the implicit-GEMM convolution are tested against: a stride-1 convolution
+    of the rearranged input with the rearranged filters is the strided convolution, the kernel larger or smaller than the
+    stride."""
     import torch.nn.functional as TF
 
-    from ferrum_b200.ops.functional import _ConvS2dFn, conv_igemm_ok
+    from ferrum_b200.ops.functional import conv_igemm_ok
+
+    from tests import _conv_s2d as s2d
 
     torch.manual_seed(0)
-    for (B, C, O, H, W, k, s, p) in [(2, 3, 5, 17, 19, (3, 3), (2, 2), (1, 1)), (1, 4, 6, 16, 16, (4, 4), (4, 4), (0, 0)),
-                                     (2, 5, 7, 15, 20, (5, 3), (2, 3), (2, 1)), (1, 3, 4, 14, 14, (7, 7), (2, 2), (3, 3))]:
+    for B, C, O, H, W, k, s, p in s2d.SHAPES:
         x, w = torch.randn(B, C, H, W), torch.randn(O, C, *k)
-        (sh, sw), (ph, pw) = s, p
-        Ho, Wo, k2h, k2w, Hz, Wz, Cz = _ConvS2dFn._geometry(x.shape, w.shape, s, p)
-        assert (Ho, Wo) == tuple(TF.conv2d(x, w, None, s, p).shape[2:]) and Cz % 8 == 0 and Cz >= sh * sw * C
-        xp = TF.pad(x, (pw, Wz * sw, ph, Hz * sh))[:, :, :Hz * sh, :Wz * sw]       # zero outside the image
-        z = xp.reshape(B, C, Hz, sh, Wz, sw).permute(0, 2, 4, 3, 5, 1).reshape(B, Hz, Wz, sh * sw * C)
-        w2 = _ConvS2dFn._filters(w, s, k2h, k2w, Cz)
-        assert w2.shape == (O, k2h, k2w, Cz) and not w2[..., sh * sw * C:].any()
-        y = TF.conv2d(z.permute(0, 3, 1, 2), w2[..., :sh * sw * C].permute(0, 3, 1, 2))
-        assert torch.allclose(y, TF.conv2d(x, w, None, s, p), atol=1e-4)
-        back = w2[..., :sh * sw * C].reshape(O, k2h, k2w, sh, sw, C).permute(0, 5, 1, 3, 2, 4)
-        assert torch.equal(back.reshape(O, C, k2h * sh, k2w * sw)[:, :, :k[0], :k[1]], w)
+        Ho, Wo, k2h, k2w, Hz, Wz, eh, ew, Cz = s2d.geometry(x.shape, w.shape, s, p)
+        want = TF.conv2d(x, w, None, s, p)
+        assert (Ho, Wo) == tuple(want.shape[2:])
+        z, w2 = s2d.pack_input(x, w.shape, s, p), s2d.pack_filters(w, s, Cz)
+        assert z.shape == (B, Hz, Wz, Cz) and w2.shape == (O, k2h * k2w, Cz)
+        y = TF.conv2d(z.permute(0, 3, 1, 2), w2.view(O, k2h, k2w, Cz).permute(0, 3, 1, 2))
+        assert torch.allclose(y, want, atol=1e-4)
         assert not conv_igemm_ok(x, s, (1, 1), p, k, 1)      # host tensors never take the tensor-core path

@@ -101,3 +101,29 @@ def test_cells_of_the_users_own(kind, how):
     got = model.forward_seq(x)[0]
     assert len(calls) == {"cell_cls": 10, "one_cell": 5, "other_type": 0}[how]
     assert (got - ref).norm() <= (2e-2 if how == "other_type" else 1e-6) * ref.norm()
+
+
+@pytest.mark.parametrize("kind", ["LSTM", "GRU"])
+@pytest.mark.parametrize("H,B", [(256, 40), (33, 5), (512, 3)])
+def test_values_that_are_not_finite(kind, H, B):
+    """A NaN stays in its batch row, though rows share a cluster's messages."""
+    import ferrum_b200 as fb
+    from ferrum_b200 import nn
+
+    torch.manual_seed(H)
+    m = getattr(nn, kind)(4, H, 1, device=fb.Device.Cuda(0))
+    base, gy = torch.randn(4, B, 4, device="cuda"), torch.randn(4, B, H, device="cuda")
+
+    def run(x):
+        x = x.clone().requires_grad_(True)
+        y = m.forward_seq(x)[0]
+        y.backward(gy)
+        return y.detach(), x.grad
+
+    clean = run(base)
+    x = base.clone()
+    x[1, B // 2] = float("nan")
+    others = torch.arange(B, device="cuda") != B // 2
+    (y, dx), (yc, dxc) = run(x), clean
+    assert torch.equal(y[:, others], yc[:, others]) and torch.equal(dx[:, others], dxc[:, others])
+    assert torch.equal(y[0], yc[0]) and torch.isnan(y[1:, B // 2]).all() and torch.isnan(dx[:, B // 2]).all()
