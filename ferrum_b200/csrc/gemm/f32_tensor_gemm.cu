@@ -24,8 +24,9 @@
 // same kernel with one plane and one product: no padded copies, no fp32 copies.  Rows at any 2-byte address are read
 // with aligned 16-byte loads and shifted into place; the loads and the shifts bound it, not the MMAs.  Against fp32
 // copies on the multiply-add kernel: 777 x 1001 x 1001 23 instead of 148 us, 8191 x 4095 x 4095 1.3 (both K-major) to
-// 1.8 ms (both row-major) instead of 12.4; relative error 9e-8 instead of 2.5e-7 at K = 1001.  Where the reduction is a
-// multiple of 8, large operands are laid out again and take the aligned kernels (native/core.cpp, copies_repay).
+// 1.8 ms (both row-major) instead of 12.4; relative error 9e-8 instead of 2.5e-7 at K = 1001.  Large operands are laid out
+// again and take the aligned kernels: with a bf16 result any, with an fp32 result those whose reduction is a multiple of 8
+// (native/core.cpp, repack_repays and copies_repay).
 //
 // The issue of a k-block's MMAs takes as long as the MMAs themselves (the queue is short), so it has a warp of its own;
 // a loader warp that issued them held up the next stage (5200 instead of 2300 cycles per k-block).  The splits' partial

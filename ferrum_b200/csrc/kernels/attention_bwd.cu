@@ -11,7 +11,7 @@
 // rows, the other side is walked 64 at a time: a tile's scores and dP take 128 columns of tensor memory, so there are two
 // of them, one per group, and the products of one tile run beside the elementwise work of the other.  With tiles of 128 x
 // 128 the scores filled tensor memory and every tile was a serial chain of product, elementwise work and product.  8 x 16
-// heads of 64, 1024 rows: dQ 116 -> 99 us, dK / dV 170 -> 140; the sums and their order are the same.
+// heads of 64, 1024 rows: dQ 116 -> 99 us, dK / dV 170 -> 140; the sums over the tiles and their order are the same.
 //
 //   attn_bwd_dq_kernel    a CTA owns 128 query rows and walks the key / value tiles:
 //                           S = Q K_j^T, dP = dO V_j^T            (tensor memory, 2 x 64 columns per group)
@@ -616,7 +616,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 }
 
 // delta[b, h, s] = sum_d dO[b, s, h, d] * O[b, s, h, d]  (both [B, S, H, D] contiguous bf16); D / 8 lanes per row, 16 bytes
-// of either operand each.  Bound by HBM (8 x 16 heads of 64, 1024 rows: a warp per row took 20.8 us).
+// of either operand each.  Bound by HBM (8 x 16 heads of 64, 1024 rows: a warp per row took 20.8 us; it added the row in another
+// order, which moves the gradients by roundings of dS to bf16).
 template <int D>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o, float* __restrict__ delta,

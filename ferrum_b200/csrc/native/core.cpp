@@ -108,34 +108,37 @@ static void aligned_copies(Op& a, Op& b, const at::TensorOptions& opt, Tensor& k
     FB_CALL(fb_repack_rows, c[0].src, c[0].dst, c[0].rows, c[0].cols, c[0].pitch, c[1].src, c[1].dst, c[1].rows, c[1].cols,
             c[1].pitch, cur_stream());
 }
-// Where the copies repay.  The kernel that reads such operands in place does 70 products (multiply-adds) per ns, the
-// aligned kernels many times that; a copy takes 6 us and 1.6 TB/s, and 5 us are left to be sure.  Behind a single
-// transpose, where the TMA unit can store the result's rows, the aligned kernels also start earlier and store 3 us per
-// million elements faster.  Weight gradients [N, K] of M rows, in place against copies and product: M 8192, 4095 x 4095
-// 1679 / 417 us; 1024, 2049 x 2049 88 / 65; 4096, 1001 x 1001 74 / 69; 1024, 1001 x 1001 31 / 36; 8192, 37 x 4095 74 /
-// 140; with bias gradient 64, 1001 x 2048 27 / 24; 512, 333 x 1024 27 / 30.
+// Where results of any type take the copies (fp32 ones, weight gradients, only here).  The kernel that reads such operands
+// in place adds its k-blocks in registers, rounded to nearest, the aligned kernels in one chain that truncates; an fp32
+// result shows it, and where the copies gain little the exact kernel stays.  The line charges it 70 products
+// (multiply-adds) per ns and a copy 6 us and 1.6 TB/s, though one launch of 4 us and 4 TB/s makes both copies; reductions
+// that are no multiple of 8 stay in place altogether.  Weight gradients [N, K] of M rows, in place / copies + product in us
+// (relative errors): M 777, 1001 x 1001 21.4 / 18.6 (9e-8 / 7e-7); 1024, 1001 x 1001 22.7 / 20.8 (9e-8 / 1e-6); 1024, 2049 x
+// 2049 74 / 33; 4096, 1001 x 1001 62 / 32; 8192, 37 x 4095 62 / 56; 8192, 4095 x 4095 1526 / 311 (2e-7 / 9e-6).  With a
+// single operand to copy and rows that the TMA unit can store the aligned kernels also save 3 us per million elements of
+// the result: 64, 1001 x 2048 12.4 / 12.3; 512, 333 x 1024 13.0 / 16.4; 512, 1001 x 4096 45 / 16; 4096, 1001 x 1024 62 / 27.
 static bool copies_repay(const Op& a, const Op& b, bool rows_tma) {
   if (a.k % 8 != 0) return false;
   double us = static_cast<double>(a.rows) * b.rows * a.k / 7e7, cost = 0.;
   int copies = 0;
-  bool transposes = true;
+  bool rows_first = true;  // the copied operands have their rows contiguous, as in a weight gradient
   for (const Op* o : {&a, &b})
     if (!tma_ok(*o)) {
       cost += 6. + static_cast<double>(o->rows) * o->k * 4 / 1.6e6;
-      transposes &= o->s_row == 1;
+      rows_first &= o->s_row == 1;
       ++copies;
     }
-  if (copies != 1 || !transposes || !rows_tma) return us > cost + 5.;
+  if (copies != 1 || !rows_first || !rows_tma) return us > cost + 5.;
   us += static_cast<double>(a.rows) * b.rows * 3e-6;
   return us > cost - 2.;
 }
 
-// The same for products with a bf16 result (layers and gradients of activations) of any reduction, whose operands keep
-// their direction, go through one launch and then take the CTA pairs.  (Those with an fp32 result keep the in-place kernel
-// up to the line above: its split accumulation is the more exact one.)  In place against copy + product, us: 1024 x 1001 x
-// 1001 19.1 / 3.7 + 13.8, 2048 x 1001 x 1001 30.3 / 4.6 + 14.0, 777 x 2049 x 2049 49.2 / 6.3 + 20.4, 512 x 4095 x 4095
-// 84.9 / 16.6 + 32.0, 8191 x 4095 x 4095 1146 / 48 + 200; below 512 rows, without the pairs, 300 x 1001 x 4095 27.1 / 6.3 +
-// 55.2.
+// The same for products with a bf16 result (layers and gradients of activations) of any reduction: the rounding of the
+// result (1.66e-3 of its norm either way; 1 in 500 to 2000 elements falls to the other neighbour) hides the difference,
+// 1e-7 against 1e-6 at K = 1001 and 4e-6 at K = 4095.  A row's bits may change when the rows beside it pass this line
+// (those of aligned operands never do).  In place against copy + product, us: 1024 x 1001 x 1001 19.1 / 3.7 + 13.8, 2048 x
+// 1001 x 1001 30.3 / 4.6 + 14.0, 777 x 2049 x 2049 49.2 / 6.3 + 20.4, 512 x 4095 x 4095 84.9 / 16.6 + 32.0, 8191 x 4095 x
+// 4095 1146 / 48 + 200; below 512 rows, without the pairs, 300 x 1001 x 4095 27.1 / 6.3 + 55.2.
 static bool repack_repays(const Op& a, const Op& b) {
   if (a.rows < 512 || b.rows < 128) return false;
   double cost = 14.;
