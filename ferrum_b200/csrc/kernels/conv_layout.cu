@@ -15,8 +15,12 @@
 //   fb_s2d_nhwc_to_nchw_f32  the data gradient of z -> that of x
 //   fb_nhwc_to_nchw_f32      a result [B, P, ld] -> [B, C, P], plus a residual, behind a ReLU
 //
-// All are bound by HBM.  The input conversion goes through shared memory in blocks of 64 channels x 64 pixels of bf16
-// pairs: 128-byte reads along the pixels, 16-byte writes along the channels.  (Results stored as NCHW from the GEMM's
+// All are bound by HBM if they do not spend too many instructions: a pixel a load and store they were bound by their issue
+// (ncu: 63 - 79 % of the slots, 23 - 39 % of the HBM rate), so rows of whole quads move four pixels at a time.  A residual
+// block's step (64 images, 64 -> 128 channels, 56 x 56, stride 2), us before and after: 64 x 56 x 56 images to s2d 19.6 -
+// 24 / 14.6, a gradient of 128 x 28 x 28 9.3 / 7.9, a result to NCHW 12.4 / 8.9.
+// The input conversion goes through shared memory in blocks of 64 channels x 64 pixels of bf16
+// pairs: 16-byte reads along the pixels, 16-byte writes along the channels.  (Results stored as NCHW from the GEMM's
 // accumulator rows, a 4-byte store per channel and pixel, were slower than the transposing kernel: 243 us of GEMMs in a
 // residual block's training step against 176 + 67.)
 #include <cuda_bf16.h>
@@ -35,7 +39,8 @@ struct S2d {
 
 constexpr int kTileC = 64, kTileQ = 64;
 
-template <bool kVec>
+// kQuads: four pixels a load (rows of whole quads on 16-byte boundaries, no columns skipped).
+template <bool kVec, bool kQuads>
 __global__ void __launch_bounds__(256)
 pack_input_kernel(const float* __restrict__ x, const float* __restrict__ mask, __nv_bfloat16* __restrict__ z, const S2d g,
                   int q_tiles) {
@@ -51,39 +56,84 @@ pack_input_kernel(const float* __restrict__ x, const float* __restrict__ mask, _
   const long long plane = static_cast<long long>(g.H) * g.W;
   const long long base = (b * g.C + c0) * plane + static_cast<long long>(i) * g.W;
   const int n_q = g.Wz * g.ew;
+  if constexpr (kQuads) {
+    const int j_lo = q0 - g.pw, quad = threadIdx.x & 15, pair0 = threadIdx.x >> 4;  // j_lo: column of the tile's first pixel
+    for (int j = (j_lo & ~3) + quad * 4; j < j_lo + kTileQ; j += 64) {
+      const bool in = row_in && j >= 0 && j < g.W;  // a quad is inside or outside as a whole
+      float4 v[2][2], m[2][2];
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int q = q0 + h * 32 + lane;
-    int j = q;
-    if (g.sw != 1 || g.ew != 1) {
-      const int J = q / g.ew;
-      j = J * g.sw + q - J * g.ew;
-    }
-    j -= g.pw;
-    const bool in = row_in && q < n_q && j >= 0 && j < g.W;
-    float v[2][kTileC / 16];
+      for (int k = 0; k < 2; ++k)
 #pragma unroll
-    for (int k = 0; k < kTileC / 16; ++k) {
-      const int c = (warp + 8 * k) * 2;
+        for (int e = 0; e < 2; ++e) {
+          const int c = (pair0 + 16 * k) * 2 + e;
+          v[k][e] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (in && c < nc) v[k][e] = __ldg(reinterpret_cast<const float4*>(x + base + c * plane + j));
+        }
+      if (mask != nullptr) {
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        v[e][k] = 0.f;
-        if (in && c + e < nc) v[e][k] = __ldg(x + base + (c + e) * plane + j);
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int c = (pair0 + 16 * k) * 2 + e;
+            m[k][e] = make_float4(1.f, 1.f, 1.f, 1.f);
+            if (in && c < nc) m[k][e] = __ldg(reinterpret_cast<const float4*>(mask + base + c * plane + j));
+          }
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            if (!(m[k][e].x > 0.f)) v[k][e].x = 0.f;
+            if (!(m[k][e].y > 0.f)) v[k][e].y = 0.f;
+            if (!(m[k][e].z > 0.f)) v[k][e].z = 0.f;
+            if (!(m[k][e].w > 0.f)) v[k][e].w = 0.f;
+          }
+      }
+      const int at = j - j_lo;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const float4 a = v[k][0], b2 = v[k][1];
+        const __nv_bfloat162 p[4] = {__floats2bfloat162_rn(a.x, b2.x), __floats2bfloat162_rn(a.y, b2.y),
+                                     __floats2bfloat162_rn(a.z, b2.z), __floats2bfloat162_rn(a.w, b2.w)};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (at + e >= 0 && at + e < kTileQ) tile[pair0 + 16 * k][at + e] = *reinterpret_cast<const uint32_t*>(&p[e]);
       }
     }
-    if (mask != nullptr) {
+  } else {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int q = q0 + h * 32 + lane;
+      int j = q;
+      if (g.sw != 1 || g.ew != 1) {
+        const int J = q / g.ew;
+        j = J * g.sw + q - J * g.ew;
+      }
+      j -= g.pw;
+      const bool in = row_in && q < n_q && j >= 0 && j < g.W;
+      float v[2][kTileC / 16];
 #pragma unroll
       for (int k = 0; k < kTileC / 16; ++k) {
         const int c = (warp + 8 * k) * 2;
 #pragma unroll
-        for (int e = 0; e < 2; ++e)
-          if (in && c + e < nc && !(__ldg(mask + base + (c + e) * plane + j) > 0.f)) v[e][k] = 0.f;
+        for (int e = 0; e < 2; ++e) {
+          v[e][k] = 0.f;
+          if (in && c + e < nc) v[e][k] = __ldg(x + base + (c + e) * plane + j);
+        }
       }
-    }
+      if (mask != nullptr) {
 #pragma unroll
-    for (int k = 0; k < kTileC / 16; ++k) {
-      const __nv_bfloat162 p = __floats2bfloat162_rn(v[0][k], v[1][k]);
-      tile[warp + 8 * k][h * 32 + lane] = *reinterpret_cast<const uint32_t*>(&p);
+        for (int k = 0; k < kTileC / 16; ++k) {
+          const int c = (warp + 8 * k) * 2;
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            if (in && c + e < nc && !(__ldg(mask + base + (c + e) * plane + j) > 0.f)) v[e][k] = 0.f;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < kTileC / 16; ++k) {
+        const __nv_bfloat162 p = __floats2bfloat162_rn(v[0][k], v[1][k]);
+        tile[warp + 8 * k][h * 32 + lane] = *reinterpret_cast<const uint32_t*>(&p);
+      }
     }
   }
   __syncthreads();
@@ -191,7 +241,7 @@ s2d_to_nchw_kernel(const float* __restrict__ z, float* __restrict__ x, const S2d
 // cost their reads beside the transposition, no pass of their own.
 __global__ void __launch_bounds__(256)
 nhwc_to_nchw_f32_kernel(const float* __restrict__ x, const float* __restrict__ add, float* __restrict__ y, int C, long long P,
-                        long long ld, int relu, int p_tiles) {
+                        long long ld, int relu, int p_tiles, bool quads) {
   __shared__ float tile[64][65];
   const long long b = blockIdx.x / p_tiles, p0 = static_cast<long long>(blockIdx.x % p_tiles) * 64;
   const int c0 = blockIdx.y * 64;
@@ -221,6 +271,28 @@ nhwc_to_nchw_f32_kernel(const float* __restrict__ x, const float* __restrict__ a
     }
   }
   __syncthreads();
+  if (quads) {  // channels of whole quads of pixels on 16-byte boundaries
+    const int pq = (threadIdx.x & 15) * 4, cq = threadIdx.x >> 4;
+    if (p0 + pq >= P) return;
+    const long long at = (b * C + c0) * P + p0 + pq;
+    float4 r[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int c = cq + 16 * k;
+      r[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (add != nullptr && c0 + c < C) r[k] = __ldg(reinterpret_cast<const float4*>(add + at + c * P));
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int c = cq + 16 * k;
+      if (c0 + c >= C) continue;
+      float4 v = make_float4(tile[c][pq], tile[c][pq + 1], tile[c][pq + 2], tile[c][pq + 3]);
+      if (add != nullptr) v = make_float4(v.x + r[k].x, v.y + r[k].y, v.z + r[k].z, v.w + r[k].w);
+      if (relu) v = make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
+      *reinterpret_cast<float4*>(y + at + c * P) = v;
+    }
+    return;
+  }
   const int px = threadIdx.x & 63, cr = threadIdx.x >> 6;
   const long long p = p0 + px;
   if (p >= P) return;
@@ -294,12 +366,11 @@ extern "C" int fb_conv_pack_input(const float* x, const float* mask, void* z, in
   // padding (a forward pass over 32 images of 65 x 30 x 30: 57.7 us channel by channel, 53.0 so).
   const bool vec = ld == static_cast<long long>(eh) * ew * ((C + 7) / 8 * 8) && (C % 8 == 0 || eh * ew == 1) &&
                    reinterpret_cast<uintptr_t>(z) % 16 == 0;
-  if (vec)
-    fb::pack_input_kernel<true><<<grid, 256, 0, stream>>>(x, mask, static_cast<__nv_bfloat16*>(z), g,
-                                                          static_cast<int>(q_tiles));
-  else
-    fb::pack_input_kernel<false><<<grid, 256, 0, stream>>>(x, mask, static_cast<__nv_bfloat16*>(z), g,
-                                                           static_cast<int>(q_tiles));
+  const bool quads = ew == sw && g.W % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 &&
+                     reinterpret_cast<uintptr_t>(mask) % 16 == 0;
+  const auto kernel = vec ? (quads ? fb::pack_input_kernel<true, true> : fb::pack_input_kernel<true, false>)
+                          : (quads ? fb::pack_input_kernel<false, true> : fb::pack_input_kernel<false, false>);
+  kernel<<<grid, 256, 0, stream>>>(x, mask, static_cast<__nv_bfloat16*>(z), g, static_cast<int>(q_tiles));
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -345,6 +416,7 @@ extern "C" int fb_nhwc_to_nchw_f32(const float* x, const float* add, float* y, i
   const long long tiles = (P + 63) / 64;
   if (B <= 0 || C <= 0 || P <= 0 || ld < C || tiles * B > 0x7fffffffll || (C + 63) / 64 > 65535) return -1;
   const dim3 grid(static_cast<unsigned>(tiles * B), static_cast<unsigned>((C + 63) / 64));
-  fb::nhwc_to_nchw_f32_kernel<<<grid, 256, 0, stream>>>(x, add, y, C, P, ld, relu, static_cast<int>(tiles));
+  const bool quads = P % 4 == 0 && reinterpret_cast<uintptr_t>(add) % 16 == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0;
+  fb::nhwc_to_nchw_f32_kernel<<<grid, 256, 0, stream>>>(x, add, y, C, P, ld, relu, static_cast<int>(tiles), quads);
   return static_cast<int>(cudaGetLastError());
 }

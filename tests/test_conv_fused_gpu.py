@@ -248,3 +248,33 @@ def test_layouts(shape):
     assert torch.equal(s2d.pack_input(back, w.shape, s, p)[..., :eh * ew * C], torch.where(reach, dz, 0.0))
     # every value of z arrives once, the pixels that no window reaches are zero
     assert back.count_nonzero() == reach.sum()
+
+
+@pytest.mark.parametrize("C,H,W,k,s,p", [(3, 2, 4, (3, 3), (2, 2), (1, 1)), (66, 3, 132, (3, 3), (2, 2), (1, 1)),
+                                         (64, 2, 64, (5, 5), (3, 3), (2, 2)), (16, 3, 128, (3, 3), (2, 2), (0, 3)),
+                                         (65, 6, 22, (3, 3), (1, 1), (1, 1)), (8, 5, 60, (4, 4), (4, 4), (3, 2))])
+@pytest.mark.parametrize("off", [0, 1])
+def test_layouts_by_quads_of_pixels(C, H, W, k, s, p, off):
+    """Rows of whole quads, on 16-byte boundaries or one element behind (read one by one); tiles with an odd first column."""
+    from ferrum_b200 import _lib
+
+    from tests import _conv_s2d as s2d
+
+    lib, st, B = _lib.cuda(), torch.cuda.current_stream().cuda_stream, 2
+    x, m = (torch.randn(B * C * H * W + 1, device="cuda")[off:][:B * C * H * W].view(B, C, H, W) for _ in range(2))
+    plain = s == (1, 1)
+    Ho, Wo, k2h, k2w, Hz, Wz, eh, ew, Cz = s2d.geometry(x.shape, (1, C, *k), s, p)
+    pw = (0, 0) if plain else p
+    for mask in (None, m):
+        z = torch.full((B, Hz, Wz, Cz), 3.0, device="cuda", dtype=torch.bfloat16)
+        _lib.check(lib.fb_conv_pack_input(x.data_ptr(), None if mask is None else m.data_ptr(), z.data_ptr(), B, C, H, W, *s,
+                                          eh, ew, *pw, Hz, Wz, Cz, st), "x")
+        assert torch.equal(z, s2d.pack_input(x if mask is None else torch.where(m > 0, x, 0.0), (1, C, *k), s, p).bfloat16())
+    for P in (H * W, H * W + 2):
+        src, add, y = torch.randn(B, P, C + 3, device="cuda"), *(torch.randn(B * C * P + 1, device="cuda") for _ in range(2))
+        add, y = (t[off:][:B * C * P].view(B, C, P) for t in (add, y))
+        for a, relu in ((None, 0), (add, 1)):
+            _lib.check(lib.fb_nhwc_to_nchw_f32(src.data_ptr(), None if a is None else a.data_ptr(), y.data_ptr(), B, C, P, C + 3,
+                                               relu, st), "y")
+            want = src[..., :C].transpose(1, 2) + (0 if a is None else a)
+            assert torch.equal(y, want.relu() if relu else want)
