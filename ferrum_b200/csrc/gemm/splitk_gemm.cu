@@ -13,6 +13,11 @@
 // operands change places: 128 rows of B against a tile of 16, 32 or 64 rows of A, so almost nothing is padding and B is
 // read once; the tile is turned round on its way to shared memory.
 //
+// Few rows of A on the 128-row side need no more than MMAs of 64 rows, whose reads of shared memory (what paces so narrow an
+// MMA) are half as many: 33 instead of 44 cycles each.  A programmatic dependent is let in when the last MMA has been issued,
+// not before: its CTAs, though they only wait, slowed the issue here from 54 to 81 cycles per MMA (16 x 4096 x 4096 in a
+// row 15.6 us, 12.6 so, 12.2 with 64 rows; eight layers of 4096 with their normalisations at 16 rows 183 -> 157).
+//
 // 192 threads: warp 0 TMA producer, warp 1 MMA issue, warps 2 - 5 read the accumulator; all of them write the output.
 #include <cooperative_groups.h>
 #include <cuda.h>
@@ -56,6 +61,7 @@ struct Args {
   int out_bf16, act, beta;
   int kb_total, kb_per_split, tiles_p;
   int stages, block_bytes, body_bytes, p_bytes;  // block: a k-block of both operands
+  int mma_rows;  // 128, or 64 where P has no more
   int prefetch;  // bring this CTA's rows of B into L2 before the kernel ahead has completed
   int32_t* status;
   unsigned long long timeout_ns;
@@ -127,7 +133,6 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  ptx::grid_launch_dependents();
   if (p.prefetch && warp == 2 && ptx::elect_one())
     for (int kb = kb_lo; kb < kb_hi; ++kb) ptx::tma_prefetch_2d(kSwap ? &map_p : &map_q, kb * kBK, kSwap ? p0 : q0);
   ptx::grid_wait();
@@ -179,7 +184,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
     }
   } else if (warp == 1) {
     if (kb_hi > kb_lo && ptx::elect_one()) {
-      const uint32_t idesc = ptx::make_idesc(1u, kRowsP, BN, p.p_mn, p.q_mn);
+      const uint32_t idesc = ptx::make_idesc(1u, p.mma_rows, BN, p.p_mn, p.q_mn);
       const uint32_t p_lbo = p.p_mn ? kChunk : 16, q_lbo = p.q_mn ? kChunk : 16;
       const uint32_t p_step = p.p_mn ? 16 * 128 : 32, q_step = p.q_mn ? 16 * 128 : 32;
       const uint64_t p_first = ptx::make_smem_desc_sw128(ptx::smem_u32(smem), p_lbo, 1024);
@@ -215,6 +220,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
         }
       }
       if (ok) ptx::umma_commit(acc_full);
+      ptx::grid_launch_dependents();
     }
   }
 
@@ -231,7 +237,9 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
       }
       ptx::tc_fence_after();
     }
-    const int row = (warp & 3) * 32 + lane;
+    // rows of the accumulator in tensor memory: 32 to a quarter of the lanes, or 16 (the lower half) of 64
+    const int row = (warp & 3) * (p.mma_rows / 4) + lane;
+    const bool held = lane < p.mma_rows / 4;
     const uint32_t taddr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
 #pragma unroll
     for (int j = 0; j < BN / 16; ++j) {
@@ -246,7 +254,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
       if constexpr (kSwap) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) tile[(j * 16 + i) * kPitch + row] = __uint_as_float(r[i]);
-      } else {
+      } else if (held) {
         float4* t4 = reinterpret_cast<float4*>(tile + row * kPitch + j * 16);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -397,7 +405,8 @@ int launch(const CUtensorMap& mp, const CUtensorMap& mq, Args& g, int rows_p, in
   g.kb_per_split = (g.kb_total + splits - 1) / splits;
   g.p_bytes = box_p * 128;
   g.block_bytes = g.p_bytes + (g.q_mn ? C::kQ : BN * 128);
-  const int tail = C::kP - g.p_bytes;  // the MMA's reads of rows that were not loaded stay inside the allocation
+  g.mma_rows = kSwap || rows_p > 64 ? kRowsP : 64;
+  const int tail = g.mma_rows * 128 > g.p_bytes ? g.mma_rows * 128 - g.p_bytes : 0;  // the MMA's reads of rows that were not loaded stay inside the allocation
   // Half an SM for narrow tiles, too: the next one's CTAs start beside this one's.
   const int room = ((split && tiles * splits <= sm_count() ? kSmemAlone : kSmemShared) - tail) / g.block_bytes;
   g.prefetch = !split && (kSwap ? !g.p_mn : !g.q_mn);
