@@ -8,10 +8,14 @@
 // normal numbers summed there alone: relative error 2.8e-5), so each k-block of 64 gets a fresh accumulator and the
 // k-blocks are added in registers, rounded to nearest: 1.7e-7, against 1.1e-6 of a chain of fp32 multiply-adds.
 //
-// What bounds it: six bf16 MMAs per fp32 product (271 TFLOP/s at the measured bf16 rate), and beside it the split:
-// about eight instructions per operand element in sixteen warps, in the shadow of the MMAs.  The split happens on the
-// way from global memory (registers) to shared memory (three bf16 planes, 128-byte swizzle, K-major), so any element
-// strides are accepted, nothing is staged in global memory and no second launch is needed.
+// What bounds it: the split, about eight instructions per operand element in sixteen warps and most of them in the integer
+// pipe (2700 cycles per k-block of a 128 x 128 tile, where the six bf16 MMAs per fp32 product take 1536: 271 TFLOP/s at the
+// measured bf16 rate).  It happens on the way from global memory (registers) to the tensor core, so any element strides are
+// accepted, nothing is staged in global memory and no second launch is needed.  The planes of A go to tensor memory, those of B
+// to shared memory (three bf16 planes, 128-byte swizzle): with both in shared memory the MMAs' reads and the split's stores
+// came to 2304 cycles of its bandwidth and a k-block to 3000.  A thread's elements of A are the ones that it may write to
+// tensor memory, in pieces that are still read 64 bytes a row (load_a).  B with contiguous rows keeps them in shared memory
+// (kVecRow): vector loads instead of eight single ones per piece, 1024^3 20.6 -> 18.9 us.
 //
 // One CTA per 128 x BN output tile and K split.  The splits of a tile are one thread-block cluster: the partial tiles
 // meet through distributed shared memory in a fixed order, so small outputs fill the chip without a workspace.
@@ -23,16 +27,16 @@
 // bf16 operands whose rows a TMA map cannot describe (a pitch that is no multiple of 16 bytes, an odd base) take the
 // same kernel with one plane and one product: no padded copies, no fp32 copies.  Rows at any 2-byte address are read
 // with aligned 16-byte loads and shifted into place; the loads and the shifts bound it, not the MMAs.  Against fp32
-// copies on the multiply-add kernel: 777 x 1001 x 1001 23 instead of 148 us, 8191 x 4095 x 4095 1.3 (both K-major) to
+// copies on the multiply-add kernel: 777 x 1001 x 1001 17 instead of 148 us, 8191 x 4095 x 4095 1.3 (both K-major) to
 // 1.8 ms (both row-major) instead of 12.4; relative error 9e-8 instead of 2.5e-7 at K = 1001.  Large operands are laid out
 // again and take the aligned kernels: with a bf16 result any, with an fp32 result those whose reduction is a multiple of 8
 // (native/core.cpp, repack_repays and copies_repay).
 //
 // The issue of a k-block's MMAs takes as long as the MMAs themselves (the queue is short), so it has a warp of its own;
-// a loader warp that issued them held up the next stage (5200 instead of 2300 cycles per k-block).  The splits' partial
-// sums are all asked for before the first is added and the values stay in registers (as an indexed array they went
-// through local memory: 2400 cycles per 4 x 544 results, now a quarter): 1024^3 23.9 -> 21.9 us, 4096 x 4096 x 1024
-// 261 -> 237, 128 x 256 x 784 9.4 -> 8.8.
+// a loader warp that issued them held up the next stage (5200 instead of 2300 cycles per k-block).  The first loads are
+// on their way before barriers and tensor memory are set up, tiles without splits meet without a cluster barrier, and the
+// partial sums are asked for several at a time.  us before all this and now: 1024 x 1024 x 64 8.8 / 6.2, 1024^3 21.1 / 19.2, 2048^3
+// 114 / 104, 591 x 1536 x 384 15.4 / 13.0, 128 x 256 x 784 8.8 / 7.6, 1 x 256 x 784 7.6 / 6.6.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -52,6 +56,7 @@ namespace cg = cooperative_groups;
 constexpr float kUp = 65536.f, kDown = 1.f / (kUp * kUp);  // of an operand before the split, of a sum after it
 
 constexpr int kBM = 128;
+constexpr int kBlock = 64 * 128;  // 64 rows (k) of 128 bytes: a block of an operand with its rows contiguous
 constexpr int kLoaders = 512;
 constexpr int kThreads = kLoaders + 32;  // 16 warps load, split, add up and write; one issues the MMAs
 
@@ -80,14 +85,16 @@ struct Cfg {
   static constexpr int kRow = kBK * 2;             // bytes of a row of a bf16 plane = its swizzle width
   static constexpr int kPieces = kBK / 8;          // 8-element pieces per row
   static constexpr int kPlaneA = kBM * kRow, kPlaneB = BN * kRow;
-  static constexpr int kStage = El<T>::kPlanes * (kPlaneA + kPlaneB);
-  static constexpr int kStages = El<T>::kPlanes == 1 ? 4 : BN == 64 ? 3 : 2;
+  static constexpr bool kATmem = El<T>::kPlanes > 1;   // the planes of A lie in tensor memory
+  static constexpr int kStage = El<T>::kPlanes * kPlaneB + (kATmem ? 0 : El<T>::kPlanes * kPlaneA);
+  static constexpr int kStages = kATmem && BN == 128 ? 2 : 4;
+  static constexpr int kPlaneCols = kBK / 2;           // columns of tensor memory of a plane of A
   static constexpr int kPitch = BN + 4;   // floats per row of the tile in shared memory: conflict-free 16-byte rows
   static constexpr int kTile = kBM * kPitch * 4;
   static constexpr int kBody = kStages * kStage > kTile ? kStages * kStage : kTile;
   static constexpr int kSmem = kBody + 1024 + 256;
-  static constexpr int kTmemCols = 2 * BN;
-  static constexpr int kPerThread = (kBM + BN) * kPieces / kLoaders;  // pieces of a stage per thread
+  static constexpr int kTmemCols = kATmem ? 512 : 2 * BN;  // two accumulators, then the stages of A
+  static constexpr int kPerThread = (kATmem ? BN : kBM + BN) * kPieces / kLoaders;  // pieces of a stage per thread
   static constexpr int kAcc = kBM * BN / kLoaders;                    // accumulators per thread: a quarter of a tile row
   // 16-byte chunk of a row, as the 128- / 64-byte swizzle of the matrix descriptors places it
   __device__ static uint32_t at(int row, int kc) {
@@ -106,8 +113,9 @@ struct Operand {
 };
 
 // How an operand lies in memory: K contiguous with 16-byte aligned rows (two vector loads per piece), K contiguous
-// with any alignment, or anything else (lanes follow the rows).
-enum Layout { kVecK = 0, kScalarK = 1, kRowFast = 2 };
+// with any alignment, anything else (lanes follow the rows), or (fp32, B) rows contiguous with 16-byte aligned steps of K: a
+// piece is then eight rows at one k, and the tile in shared memory has its rows contiguous, too.
+enum Layout { kVecK = 0, kScalarK = 1, kRowFast = 2, kVecRow = 3 };
 
 struct Args {
   Operand a, b;
@@ -150,6 +158,9 @@ __device__ __forceinline__ void piece(int c, int& row, int& kc) {
   if (L == kRowFast) {
     row = c % ROWS;
     kc = c / ROWS;
+  } else if (L == kVecRow) {  // eight rows from `row` at k = kc
+    row = c % (ROWS / 8) * 8;
+    kc = c / (ROWS / 8);
   } else {
     row = c / PIECES;
     kc = c % PIECES;
@@ -164,6 +175,22 @@ __device__ __forceinline__ void load_piece(const Operand& o, const float* base, 
   float(&v)[8] = out.v;
   int row, kc;
   piece<ROWS, L, PIECES>(c, row, kc);
+  if constexpr (L == kVecRow) {
+    const int r = row0 + row, k = k0 + kc;
+    const float* p = base + k * o.s_k + r;
+    if (k < K && r + 8 <= o.rows) {
+      const float4 x = __ldg(reinterpret_cast<const float4*>(p)), y = __ldg(reinterpret_cast<const float4*>(p) + 1);
+      v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+      v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        v[j] = 0.f;
+        if (k < K && r + j < o.rows) v[j] = __ldg(p + j);
+      }
+    }
+    return;
+  }
   const int r = min(row0 + row, o.rows - 1), k = k0 + kc * 8;
   if (k0 + PIECES * 8 <= K) {
     if constexpr (L == kVecK) {
@@ -267,19 +294,43 @@ __device__ __forceinline__ float2 wide_pair(uint32_t w) {
   return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
 }
 
+// Two values scaled and split: a word of each plane.
+__device__ __forceinline__ void split_pair(float x0, float x1, uint32_t& w0, uint32_t& w1, uint32_t& w2) {
+  const float2 x = scale2(make_float2(x0, x1), kUp);
+  w0 = bf16_pair(x);
+  const float2 r = sub2(x, wide_pair(w0));
+  w1 = bf16_pair(r);
+  w2 = bf16_pair(sub2(r, wide_pair(w1)));
+}
+
+// Splits a thread's share of A (load_a) into the planes at `at`: the lanes of its warp, the columns of its slice of K.
+template <int L, int PLANE>
+__device__ __forceinline__ void store_a(uint32_t at, const float (&v)[16]) {
+  uint32_t w0[8], w1[8], w2[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) split_pair(v[2 * j], v[2 * j + 1], w0[j], w1[j], w2[j]);
+  if constexpr (L == kRowFast) {
+    ptx::tmem_st_32x32b_x8(at, w0);
+    ptx::tmem_st_32x32b_x8(at + PLANE, w1);
+    ptx::tmem_st_32x32b_x8(at + 2 * PLANE, w2);
+  } else {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t to = at + (static_cast<uint32_t>(16 * h) << 16);
+      ptx::tmem_st_16x256b(to, w0[4 * h], w0[4 * h + 1], w0[4 * h + 2], w0[4 * h + 3]);
+      ptx::tmem_st_16x256b(to + PLANE, w1[4 * h], w1[4 * h + 1], w1[4 * h + 2], w1[4 * h + 3]);
+      ptx::tmem_st_16x256b(to + 2 * PLANE, w2[4 * h], w2[4 * h + 1], w2[4 * h + 2], w2[4 * h + 3]);
+    }
+  }
+}
+
 // Splits eight values and stores them into the three planes.
 template <int L>
 __device__ __forceinline__ void store_piece(uint32_t at, uint32_t plane_bytes, const El<float>::Piece& in) {
   const float(&v)[8] = in.v;
   uint32_t w0[4], w1[4], w2[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float2 x = scale2(make_float2(v[2 * j], v[2 * j + 1]), kUp);
-    w0[j] = bf16_pair(x);
-    const float2 r = sub2(x, wide_pair(w0[j]));
-    w1[j] = bf16_pair(r);
-    w2[j] = bf16_pair(sub2(r, wide_pair(w1[j])));
-  }
+  for (int j = 0; j < 4; ++j) split_pair(v[2 * j], v[2 * j + 1], w0[j], w1[j], w2[j]);
   ptx::st_shared_v4(at, w0[0], w0[1], w0[2], w0[3]);
   ptx::st_shared_v4(at + plane_bytes, w1[0], w1[1], w1[2], w1[3]);
   ptx::st_shared_v4(at + 2 * plane_bytes, w2[0], w2[1], w2[2], w2[3]);
@@ -300,6 +351,40 @@ __device__ __forceinline__ void store_piece(uint32_t at, uint32_t, const El<__nv
     const uint32_t sh = (v.off & 2) * 8;
     ptx::st_shared_v4(at, __funnelshift_r(s[0], s[1], sh), __funnelshift_r(s[1], s[2], sh),
                       __funnelshift_r(s[2], s[3], sh), __funnelshift_r(s[3], s[4], sh));
+  }
+}
+
+// A thread's share of a k-block of A on its way to tensor memory: 16 elements of 32 rows x 16 of K (the rows are the lanes
+// that its warp may write, the slice of K is its warp's).  K contiguous: four rows, four elements each, as tmem_st_16x256b
+// places them, so that four lanes read 64 bytes of a row; rows contiguous: one row each (tmem_st_32x32b_x8).
+template <int L>
+__device__ __forceinline__ void load_a(const Operand& o, const float* base, int row0, int k0, int K, float (&v)[16]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kw = k0 + (warp >> 2) * 16;
+  row0 += (warp & 3) * 32;
+  const bool whole = k0 + 64 <= K;
+  if constexpr (L == kRowFast) {
+    const float* p = base + min(row0 + lane, o.rows - 1) * o.s_row + kw * o.s_k;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      v[j] = 0.f;
+      if (whole || kw + j < K) v[j] = __ldg(p + j * o.s_k);
+    }
+  } else {
+    const int k = kw + (lane & 3) * 4;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float* p = base + min(row0 + i * 8 + (lane >> 2), o.rows - 1) * o.s_row + k;
+      if (L == kVecK && whole) {
+        const float4 x = __ldg(reinterpret_cast<const float4*>(p));
+        v[4 * i] = x.x; v[4 * i + 1] = x.y; v[4 * i + 2] = x.z; v[4 * i + 3] = x.w;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          v[4 * i + j] = 0.f;
+          if (whole || k + j < K) v[4 * i + j] = __ldg(p + j);
+        }
+      }
+    }
   }
 }
 
@@ -329,7 +414,26 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split_kernel(const __grid_co
   const int kb_lo = min(p.kb_total, rank * p.kb_per_split), kb_hi = min(p.kb_total, kb_lo + p.kb_per_split);
   const int nkb = kb_hi - kb_lo;
 
-  if (threadIdx.x == 0) {
+  // The first k-block's loads are on their way before barriers and tensor memory are set up.
+  constexpr int kPA = C::kATmem ? 0 : kBM * C::kPieces / kLoaders;  // pieces of A per thread; the rest are B's
+  typename El<T>::Piece v[C::kPerThread];
+  float va[C::kATmem ? 16 : 1];
+  auto fetch_a = [&](int kb) {
+    if constexpr (C::kATmem) load_a<LA>(p.a, a, m0, kb * C::kBK, p.K, va);
+  };
+  auto fetch = [&](int i, int kb) {
+    const int k0 = kb * C::kBK;
+    if (i < kPA)
+      load_piece<kBM, LA, C::kPieces>(p.a, a, m0, k0, p.K, i * kLoaders + threadIdx.x, v[i]);
+    else
+      load_piece<BN, LB, C::kPieces>(p.b, b, n0, k0, p.K, (i - kPA) * kLoaders + threadIdx.x, v[i]);
+  };
+  if (warp < kLoaders / 32 && nkb > 0) {
+    fetch_a(kb_lo);
+#pragma unroll
+    for (int i = 0; i < C::kPerThread; ++i) fetch(i, kb_lo);
+  }
+  if (threadIdx.x == kLoaders) {
     *abort_flag = 0;
     for (int s = 0; s < C::kStages; ++s) {
       ptx::mbar_init(&full_bar[s], kLoaders / 32);
@@ -341,7 +445,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split_kernel(const __grid_co
     }
     ptx::fence_mbar_init();
   }
-  if (warp == 0) {
+  if (warp == kLoaders / 32) {
+    __syncwarp();
     ptx::tmem_alloc(tmem_slot, C::kTmemCols);
     ptx::tmem_relinquish();
   }
@@ -353,19 +458,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split_kernel(const __grid_co
   float acc[C::kAcc];
   if (warp < kLoaders / 32) {
     // -------------------------------------------------------- load, split, add up
-    constexpr int kPA = kBM * C::kPieces / kLoaders;  // pieces of A per thread; the rest are B's
-    typename El<T>::Piece v[C::kPerThread];
-    auto fetch = [&](int i, int kb) {
-      const int k0 = kb * C::kBK;
-      if (i < kPA)
-        load_piece<kBM, LA, C::kPieces>(p.a, a, m0, k0, p.K, i * kLoaders + threadIdx.x, v[i]);
-      else
-        load_piece<BN, LB, C::kPieces>(p.b, b, n0, k0, p.K, (i - kPA) * kLoaders + threadIdx.x, v[i]);
-    };
-    if (nkb > 0) {
-#pragma unroll
-      for (int i = 0; i < C::kPerThread; ++i) fetch(i, kb_lo);
-    }
 #pragma unroll
     for (int i = 0; i < C::kAcc; ++i) acc[i] = 0.f;
     const uint32_t taddr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + (warp >> 2) * C::kAcc;
@@ -404,8 +496,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split_kernel(const __grid_co
         ok = false;
         break;
       }
-      const uint32_t sa = ptx::smem_u32(smem + s * C::kStage), sb = sa + kPlanes * C::kPlaneA;
+      const uint32_t sa = ptx::smem_u32(smem + s * C::kStage), sb = C::kATmem ? sa : sa + kPlanes * C::kPlaneA;
       const bool more = kb + 1 < nkb;
+      if constexpr (C::kATmem) {
+        ptx::tc_fence_after();
+        store_a<LA, C::kPlaneCols>(tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + 2 * BN +
+                                       s * kPlanes * C::kPlaneCols + (warp >> 2) * 8, va);
+        if (more) fetch_a(kb_lo + kb + 1);
+      }
 #pragma unroll
       for (int i = 0; i < C::kPerThread; ++i) {
         int row, kc;
@@ -414,11 +512,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split_kernel(const __grid_co
           store_piece<LA>(sa + C::at(row, kc), C::kPlaneA, v[i]);
         } else {
           piece<BN, LB, C::kPieces>((i - kPA) * kLoaders + threadIdx.x, row, kc);
-          store_piece<LB>(sb + C::at(row, kc), C::kPlaneB, v[i]);
+          // rows contiguous: blocks of 64 rows, 128 bytes per k
+          const int at = LB == kVecRow ? (row >> 6) * kBlock + C::at(kc, (row >> 3) & 7) : C::at(row, kc);
+          store_piece<LB>(sb + at, C::kPlaneB, v[i]);
         }
         if (more) fetch(i, kb_lo + kb + 1);
       }
       ptx::fence_proxy_async_smem();
+      if constexpr (C::kATmem) {
+        ptx::tmem_wait_st();
+        ptx::tc_fence_before();
+      }
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&full_bar[s]);
       if (kb > 0) read_block();  // the k-block before: added up while the MMAs of this one run
@@ -429,8 +533,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split_kernel(const __grid_co
     }
   } else if (ptx::elect_one()) {
     // ---------------------------------------------------------------- MMA issue
-    const uint32_t idesc = ptx::make_idesc(1u, kBM, BN, 0, 0);
-    const uint64_t first = C::desc(ptx::smem_u32(smem));
+    const uint32_t idesc = ptx::make_idesc(1u, kBM, BN, 0, LB == kVecRow ? 1 : 0);
+    const uint64_t first = LB == kVecRow ? ptx::make_smem_desc_sw128(ptx::smem_u32(smem), kBlock, 1024)
+                                         : C::desc(ptx::smem_u32(smem));
+    constexpr int kStepB = LB == kVecRow ? 16 * 128 : 32;  // 16 of K
     for (int kb = 0; kb < nkb; ++kb) {
       const int s = kb % C::kStages, buf = kb & 1;
       if (!ptx::mbar_wait(&acc_empty[buf], ((kb >> 1) & 1) ^ 1, abort_flag, p.timeout_ns) ||
@@ -439,7 +545,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split_kernel(const __grid_co
         break;
       }
       ptx::tc_fence_after();
-      const uint64_t da = ptx::desc_advance(first, s * C::kStage), db = ptx::desc_advance(da, kPlanes * C::kPlaneA);
+      const uint64_t da = ptx::desc_advance(first, s * C::kStage);
+      const uint64_t db = C::kATmem ? da : ptx::desc_advance(da, kPlanes * C::kPlaneA);
+      const uint32_t ta = tmem + 2 * BN + s * kPlanes * C::kPlaneCols;
       const uint32_t d = tmem + buf * BN;
       constexpr int ia[6] = {2, 0, 1, 1, 0, 0}, ib[6] = {0, 2, 1, 0, 1, 0};  // small products first
       constexpr int kFirst = 6 - El<T>::kProducts;
@@ -447,8 +555,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split_kernel(const __grid_co
       for (int q = kFirst; q < 6; ++q) {
 #pragma unroll
         for (int k = 0; k < C::kBK / 16; ++k) {
-          ptx::umma_f16(d, ptx::desc_advance(da, ia[q] * C::kPlaneA + k * 32),
-                        ptx::desc_advance(db, ib[q] * C::kPlaneB + k * 32), idesc, (q != kFirst || k != 0) ? 1u : 0u);
+          const uint64_t dbk = ptx::desc_advance(db, ib[q] * C::kPlaneB + k * kStepB);
+          const uint32_t sum = (q != kFirst || k != 0) ? 1u : 0u;
+          if constexpr (C::kATmem)
+            ptx::umma_f16_ta(d, ta + ia[q] * C::kPlaneCols + k * 8, dbk, idesc, sum);
+          else
+            ptx::umma_f16(d, ptx::desc_advance(da, ia[q] * C::kPlaneA + k * 32), dbk, idesc, sum);
         }
       }
       ptx::umma_commit(&empty_bar[s]);
@@ -457,84 +569,120 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_split_kernel(const __grid_co
   }
 
   // ------------------------------------------------------------------ partial tiles meet
-  __syncthreads();  // every MMA has completed (the loaders waited for the last one): the stages are free
+  // Every MMA of this CTA has completed (the loaders waited for the last one), so its stages hold the tile.
   float* tile = reinterpret_cast<float*>(smem);
+  const int rows_per = kBM / splits;  // what this CTA adds up and writes
   if (warp < kLoaders / 32) {
-    const int row = (warp & 3) * 32 + lane, c0 = (warp >> 2) * C::kAcc;
-    float4* t4 = reinterpret_cast<float4*>(tile + row * C::kPitch + c0);
+    float4* t4 = reinterpret_cast<float4*>(tile + ((warp & 3) * 32 + lane) * C::kPitch + (warp >> 2) * C::kAcc);
 #pragma unroll
     for (int i = 0; i < C::kAcc / 4; ++i)
       t4[i] = make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
   }
-  cluster.sync();
-  const int rows_per = kBM / splits;
-  const int esz = p.out_bf16 ? 2 : 4;
-  const bool vec = p.N % 4 == 0 && p.ldc % 4 == 0 && out_at % 4 == 0 && reinterpret_cast<uintptr_t>(p.out) % (4 * esz) == 0;
-  constexpr int kVec = BN / 4;
-  for (int i = threadIdx.x; i < rows_per * kVec; i += kThreads) {
-    const int row = rank * rows_per + i / kVec, c = (i % kVec) * 4;
-    const int m = m0 + row, n = n0 + c;
-    if (m >= p.M || n >= p.N) continue;
-    float4 part[8];
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
-      if (r < splits) part[r] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(tile, r) + row * C::kPitch + c);
-    float f[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
-      if (r < splits) {
-        f[0] += part[r].x; f[1] += part[r].y; f[2] += part[r].z; f[3] += part[r].w;
-      }
-    if constexpr (kPlanes > 1) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const bool finite = fabsf(f[j]) <= FLT_MAX;
-        f[j] *= kDown;
-        // not finite: an operand that does not survive the split, or a result that is not finite in fp32 either
-        if (!finite && n + j < p.N)
-          f[j] = dot_again(a + m * p.a.s_row, p.a.s_k, b + (n + j) * p.b.s_row, p.b.s_k, p.K);
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      f[j] *= p.alpha;
-      if (p.bias != nullptr && n + j < p.N) f[j] += __ldg(p.bias + n + j);
-    }
-    if (p.act != FB_ACT_NONE) {
-#pragma unroll 1
-      for (int j = 0; j < 4; ++j) {  // one copy of the code; the four values change places instead of being indexed
-        const float y = act_f(f[0], p.act);
-        f[0] = f[1]; f[1] = f[2]; f[2] = f[3]; f[3] = y;
-      }
-    }
-    const long long at = out_at + m * p.ldc + n;
-    if (p.out_bf16) {
-      __nv_bfloat16* o = static_cast<__nv_bfloat16*>(p.out) + at;
-      if (vec) {
-        *reinterpret_cast<uint2*>(o) = make_uint2(bf16_pair(make_float2(f[0], f[1])), bf16_pair(make_float2(f[2], f[3])));
-      } else {
-        for (int j = 0; j < 4 && n + j < p.N; ++j) o[j] = __float2bfloat16_rn(f[j]);
-      }
-      continue;
-    }
-    float* o = static_cast<float*>(p.out) + at;
-    if (vec) {
-      float4 x = make_float4(f[0], f[1], f[2], f[3]);
-      if (p.beta) {
-        const float4 old = *reinterpret_cast<float4*>(o);
-        x.x += old.x; x.y += old.y; x.z += old.z; x.w += old.w;
-      }
-      *reinterpret_cast<float4*>(o) = x;
-    } else {
-      for (int j = 0; j < 4 && n + j < p.N; ++j) o[j] = p.beta ? o[j] + f[j] : f[j];
-    }
-  }
   ptx::tc_fence_before();
-  cluster.sync();  // no CTA leaves while another one still reads its tile
-  if (warp == 0) {
+  if (splits > 1) cluster.sync();
+  else __syncthreads();
+  if (warp == kLoaders / 32) {
     ptx::tc_fence_after();
+    __syncwarp();
     ptx::tmem_dealloc(tmem, C::kTmemCols);
   }
+  const int esz = p.out_bf16 ? 2 : 4;
+  const bool vec = p.N % 4 == 0 && p.ldc % 4 == 0 && out_at % 4 == 0 && reinterpret_cast<uintptr_t>(p.out) % (4 * esz) == 0;
+  constexpr int kVec = BN / 4, kRowStep = kLoaders / kVec;
+  const int c = static_cast<int>(threadIdx.x) % kVec * 4, n = n0 + c;
+  const int row0 = rank * rows_per, rows = warp < kLoaders / 32 && n < p.N ? min(rows_per, p.M - m0 - row0) : 0;
+  float bias[4] = {0.f, 0.f, 0.f, 0.f};
+  if (p.bias != nullptr) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (n + j < p.N) bias[j] = __ldg(p.bias + n + j);
+  }
+  // Added up in the order of the splits, with several reads (of the other CTAs' tiles) on their way at a time: two rows of up
+  // to two splits, or one row of them all.
+  const int step = splits > 2 ? kRowStep : 2 * kRowStep;
+  for (int l0 = threadIdx.x / kVec; l0 < rows; l0 += step) {
+    const bool two = splits <= 2 && l0 + kRowStep < rows;
+    const int at0 = (row0 + l0) * C::kPitch + c;
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f), next = sum;
+    if (splits > 2) {
+      float4 part[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+        if (r < splits) part[r] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(tile, r) + at0);
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+        if (r < splits) {
+          sum.x += part[r].x; sum.y += part[r].y; sum.z += part[r].z; sum.w += part[r].w;
+        }
+    } else {
+#pragma unroll 2
+      for (int r = 0; r < splits; ++r) {
+        const float* from = cluster.map_shared_rank(tile, r) + at0;
+        const float4 x = *reinterpret_cast<const float4*>(from);
+        const float4 y = *reinterpret_cast<const float4*>(from + (two ? kRowStep * C::kPitch : 0));
+        sum.x += x.x; sum.y += x.y; sum.z += x.z; sum.w += x.w;
+        next.x += y.x; next.y += y.y; next.z += y.z; next.w += y.w;
+      }
+    }
+#pragma unroll 1
+    for (int u = 0; u <= static_cast<int>(two); ++u) {
+      const int m = m0 + row0 + l0 + u * kRowStep;
+      float f[4] = {sum.x, sum.y, sum.z, sum.w};
+      sum = next;
+      if constexpr (kPlanes > 1) {
+        bool finite = true;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          finite &= fabsf(f[j]) <= FLT_MAX;
+          f[j] *= kDown;
+        }
+        // not finite: an operand that does not survive the split, or a result that is not finite in fp32 either
+        if (!finite) {
+#pragma unroll 1
+          for (int j = 0; j < 4; ++j) {  // the four values change places instead of being indexed
+            float y = f[0];
+            if (!(fabsf(y) <= FLT_MAX) && n + j < p.N)
+              y = dot_again(a + m * p.a.s_row, p.a.s_k, b + (n + j) * p.b.s_row, p.b.s_k, p.K);
+            f[0] = f[1]; f[1] = f[2]; f[2] = f[3]; f[3] = y;
+          }
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        f[j] *= p.alpha;
+        if (p.bias != nullptr) f[j] += bias[j];
+      }
+      if (p.act != FB_ACT_NONE) {
+#pragma unroll 1
+        for (int j = 0; j < 4; ++j) {  // one copy of the code, as above
+          const float y = act_f(f[0], p.act);
+          f[0] = f[1]; f[1] = f[2]; f[2] = f[3]; f[3] = y;
+        }
+      }
+      const long long at = out_at + m * p.ldc + n;
+      if (p.out_bf16) {
+        __nv_bfloat16* o = static_cast<__nv_bfloat16*>(p.out) + at;
+        if (vec) {
+          *reinterpret_cast<uint2*>(o) = make_uint2(bf16_pair(make_float2(f[0], f[1])), bf16_pair(make_float2(f[2], f[3])));
+        } else {
+          for (int j = 0; j < 4 && n + j < p.N; ++j) o[j] = __float2bfloat16_rn(f[j]);
+        }
+        continue;
+      }
+      float* o = static_cast<float*>(p.out) + at;
+      if (vec) {
+        float4 x = make_float4(f[0], f[1], f[2], f[3]);
+        if (p.beta) {
+          const float4 old = *reinterpret_cast<float4*>(o);
+          x.x += old.x; x.y += old.y; x.z += old.z; x.w += old.w;
+        }
+        *reinterpret_cast<float4*>(o) = x;
+      } else {
+        for (int j = 0; j < 4 && n + j < p.N; ++j) o[j] = p.beta ? o[j] + f[j] : f[j];
+      }
+    }
+  }
+  if (splits > 1) cluster.sync();  // no CTA leaves while another one still reads its tile
 }
 
 int sm_count() {
@@ -576,6 +724,9 @@ template <typename T, int BN, int LA>
 int launch_b(int lb, const Args& args, int batch, int splits, cudaStream_t st) {
   if (lb == kVecK) return launch_one<T, BN, LA, kVecK>(args, batch, splits, st);
   if (lb == kScalarK) return launch_one<T, BN, LA, kScalarK>(args, batch, splits, st);
+  if constexpr (El<T>::kPlanes > 1) {
+    if (lb == kVecRow) return launch_one<T, BN, LA, kVecRow>(args, batch, splits, st);
+  }
   return launch_one<T, BN, LA, kRowFast>(args, batch, splits, st);
 }
 template <typename T, int BN>
@@ -636,7 +787,11 @@ int gemm_split(const T* a, const T* b, void* out, int out_bf16, const float* bia
   int splits = 1;
   while (splits < 8 && tiles * splits * 2 <= sm_count() && splits * 2 <= g.kb_total) splits *= 2;
   g.kb_per_split = (g.kb_total + splits - 1) / splits;
-  const int la = layout_of<T>(g.a), lb = layout_of<T>(g.b);
+  const int la = layout_of<T>(g.a);
+  int lb = layout_of<T>(g.b);
+  if (El<T>::kPlanes > 1 && lb == kRowFast && g.b.s_row == 1 && reinterpret_cast<uintptr_t>(g.b.p) % 16 == 0 &&
+      g.b.s_k % 4 == 0 && g.b.s_bo % 4 == 0 && g.b.s_bi % 4 == 0)
+    lb = kVecRow;
   return use_wide ? launch<T, 128>(la, lb, g, static_cast<int>(batch), splits, stream)
                   : launch<T, 64>(la, lb, g, static_cast<int>(batch), splits, stream);
 }

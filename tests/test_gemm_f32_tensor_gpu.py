@@ -95,3 +95,20 @@ def test_scaled_products_of_other_ranks(lead_a, lead_b):
     a, b = (torch.randn(*l, *s, device="cuda", generator=g) for l, s in ((lead_a, (5, 40)), (lead_b, (40, 7))))
     ref = 0.5 * (a.double() @ b.double())
     assert (F.bmm_scaled(a, b, 0.5).double() - ref).norm() <= 5e-7 * ref.norm()
+
+
+@pytest.mark.parametrize("la", ["k", "rows", "odd"])
+@pytest.mark.parametrize("M,N,K", [(5, 4, 33), (130, 12, 64), (31, 68, 100), (128, 132, 257), (96, 1028, 1030)])
+def test_rows_of_b_by_quads(la, M, N, K):
+    """B with its rows contiguous on 16-byte boundaries (read eight rows at a time) where the last eight are not whole, for each
+    way in which A reaches tensor memory; the operand ends where the last row of K does.  Bound as above."""
+    from ferrum_b200.ops.gemm import gemm_f32
+    from ferrum_b200.utils.runtime import check_status
+
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a, b = _operand(M, K, la, g), _operand(N, K, "rows", g)
+    ref = a.double() @ b.double().t()
+    out = gemm_f32(a, b)
+    check_status()
+    assert (out.double() - ref).norm() <= 5e-7 * ref.norm() + 1e-6
+    assert torch.equal(out, gemm_f32(a.contiguous(), b.contiguous()))  # the same sums, however the operands lie
