@@ -6,12 +6,12 @@
 // Two kernels, both shaped like the forward kernel (same operand layouts, same roles), so that neither needs an
 // atomic or a cross-CTA reduction:
 //
-// Roles of a CTA (320 threads): warp 0 TMA producer, warp 1 MMA issuer, warps 2-5 and 6-9 two groups for the elementwise
-// work (two tensor-memory reads, an exponential and half a dozen multiply-adds per score).  The stationary tile has 128
-// rows, the other side is walked 64 at a time: a tile's scores and dP take 128 columns of tensor memory, so there are two
-// of them, one per group, and the products of one tile run beside the elementwise work of the other.  With tiles of 128 x
-// 128 the scores filled tensor memory and every tile was a serial chain of product, elementwise work and product.  8 x 16
-// heads of 64, 1024 rows: dQ 116 -> 99 us, dK / dV 170 -> 140; the sums over the tiles and their order are the same.
+// Roles of a CTA: warp 0 TMA producer, warp 1 MMA issuer, then groups of four warps for the elementwise work (two
+// tensor-memory reads, an exponential and half a dozen multiply-adds per score).  The stationary tile has 128 rows, the other
+// side is walked 64 at a time: a tile's scores and dP take 128 columns of tensor memory, one group's, and the products of one
+// tile run beside the elementwise work of the others.  A group waits for its products longer than they take, so there are as
+// many groups as tensor memory holds beside the accumulators: three for a head dimension of 64, two for 128.  8 x 16 heads
+// of 64, 1024 rows, two and three groups: dQ 99 / 93 us, dK and dV 140 / 120; the sums over the tiles and their order are the same.
 //
 //   attn_bwd_dq_kernel    a CTA owns 128 query rows and walks the key / value tiles:
 //                           S = Q K_j^T, dP = dO V_j^T            (tensor memory, 2 x 64 columns per group)
@@ -44,16 +44,18 @@ constexpr int kT = 128;                     // rows of the stationary tile
 constexpr int kW = 64;                      // rows of a tile of the side that is walked
 constexpr int kBlk = kT * 128;              // 16 KB: 128 rows of 64 bf16 = one 128-byte-swizzled block
 constexpr int kBlkW = kW * 128;             // the same of 64 rows
-constexpr int kBwdThreads = 320;            // TMA warp, MMA warp, two groups of four softmax warps
-constexpr int kTmemBwd = 512;               // scores and dP of the groups: columns 0 .. 255; accumulators from 256 on
+constexpr int kTmemBwd = 512;               // scores and dP of the groups, 128 columns each; then the accumulators
 // D = head dimension (64 or 128).  An operand tile is D / 64 blocks side by side.
 template <int D>
 struct BwdCfg {
   static constexpr int kNB = D / 64;
   static constexpr int kTile = kNB * kBlk, kTileW = kNB * kBlkW;
-  static constexpr int kStages = D == 64 ? 4 : 3;  // three: a tile's scores are issued two tiles ahead of its release
-  static constexpr int kSmemDq = 2 * kTile + 2 * kStages * kTileW + 2 * kBlk + 1024 + 256;          // Q dO | K V | dS
-  static constexpr int kSmemDkv = 2 * kTile + 2 * kStages * kTileW + 4 * kBlk + 1024 + 1024 + 256;  // K V | Q dO | P^T dS^T | lse, delta
+  static constexpr int kG = D == 64 ? 3 : 2;       // groups of four softmax warps: as many as tensor memory has room for
+  static constexpr int kThreads = 64 + kG * 128;   // TMA warp, MMA warp, groups
+  static constexpr int kStages = D == 64 ? 5 : 3;  // a tile's scores are issued kG tiles ahead of its release
+  static constexpr int kSmemDq = 2 * kTile + 2 * kStages * kTileW + kG * kBlk + 1024 + 256;  // Q dO | K V | dS
+  // K V | Q dO | P^T dS^T | lse, delta
+  static constexpr int kSmemDkv = 2 * kTile + 2 * kStages * kTileW + 2 * kG * kBlk + kG * 2 * kW * 4 + 1024 + 256;
 };
 
 // One operand tile: D / 64 boxes of 64 columns, `bytes` each.
@@ -170,25 +172,25 @@ __device__ __forceinline__ void store_row_bf16(__nv_bfloat16* dst, uint32_t tmem
 
 // ------------------------------------------------------------------------------------------------ dQ
 template <int D>
-__global__ void __launch_bounds__(kBwdThreads, 1)
+__global__ void __launch_bounds__(BwdCfg<D>::kThreads, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                    const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
                    const BwdArgs p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  constexpr int kTile = BwdCfg<D>::kTile, kTileW = BwdCfg<D>::kTileW, kStages = BwdCfg<D>::kStages;
+  constexpr int kTile = BwdCfg<D>::kTile, kTileW = BwdCfg<D>::kTileW, kStages = BwdCfg<D>::kStages, kG = BwdCfg<D>::kG;
   uint8_t* sq = smem;
   uint8_t* sdo = sq + kTile;
   uint8_t* sk = sdo + kTile;              // kStages tiles
   uint8_t* sv = sk + kStages * kTileW;    // kStages tiles
   uint8_t* sds = sv + kStages * kTileW;   // dS of the groups: 128 x 64 bf16 each
-  uint64_t* q_full = reinterpret_cast<uint64_t*>(sds + 2 * kBlk);
+  uint64_t* q_full = reinterpret_cast<uint64_t*>(sds + kG * kBlk);
   uint64_t* kv_full = q_full + 1;           // [kStages]
   uint64_t* kv_empty = kv_full + kStages;   // [kStages]
-  uint64_t* sp_full = kv_empty + kStages;   // [2] S and dP of a group's tile are complete
-  uint64_t* ds_full = sp_full + 2;          // [2] dS written (and S, dP read) by the group's four warps
-  uint64_t* ds_empty = ds_full + 2;         // [2] the dQ MMAs have read dS
-  uint64_t* dq_full = ds_empty + 2;
+  uint64_t* sp_full = kv_empty + kStages;   // [kG] S and dP of a group's tile are complete
+  uint64_t* ds_full = sp_full + kG;         // [kG] dS written (and S, dP read) by the group's four warps
+  uint64_t* ds_empty = ds_full + kG;        // [kG] the dQ MMAs have read dS
+  uint64_t* dq_full = ds_empty + kG;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(dq_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -207,7 +209,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       ptx::mbar_init(&kv_full[s], 1);
       ptx::mbar_init(&kv_empty[s], 1);
     }
-    for (int g = 0; g < 2; ++g) {
+    for (int g = 0; g < kG; ++g) {
       ptx::mbar_init(&sp_full[g], 1);
       ptx::mbar_init(&ds_full[g], 4);
       ptx::mbar_init(&ds_empty[g], 1);
@@ -227,7 +229,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t t_dq = tmem_base + 256;
+  const uint32_t t_dq = tmem_base + kG * 2 * kW;
 
   if (warp == 0) {
     if (ptx::elect_one()) {
@@ -254,7 +256,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       const uint32_t sq_a = ptx::smem_u32(sq), sdo_a = ptx::smem_u32(sdo), sds_a = ptx::smem_u32(sds);
       const uint32_t sk_a = ptx::smem_u32(sk), sv_a = ptx::smem_u32(sv);
       auto issue_s = [&](int j) {  // S and dP of tile j
-        const int st = j % kStages, g = j & 1;
+        const int st = j % kStages, g = j % kG;
         if (!ptx::mbar_wait(&kv_full[st], (j / kStages) & 1, abort_flag, p.timeout_ns)) {
           report_status(p.status, kStatusGemmTimeout, 63, blockIdx.x, j);
           return false;
@@ -267,17 +269,17 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       };
       bool ok = ptx::mbar_wait(q_full, 0, abort_flag, p.timeout_ns);
       if (!ok) report_status(p.status, kStatusGemmTimeout, 62, blockIdx.x, 0);
-      for (int j = 0; ok && j < 2 && j < n_tiles; ++j) ok = issue_s(j);
+      for (int j = 0; ok && j < kG && j < n_tiles; ++j) ok = issue_s(j);
       for (int j = 0; ok && j < n_tiles; ++j) {
-        const int st = j % kStages, g = j & 1;
+        const int st = j % kStages, g = j % kG;
         // dS of tile j is written, its S and dP have been read
-        if (!ptx::mbar_wait(&ds_full[g], (j >> 1) & 1, abort_flag, p.timeout_ns)) {
+        if (!ptx::mbar_wait(&ds_full[g], (j / kG) & 1, abort_flag, p.timeout_ns)) {
           report_status(p.status, kStatusGemmTimeout, 64, blockIdx.x, j);
           break;
         }
         ptx::tc_fence_after();
-        if (j + 2 < n_tiles) {
-          ok = issue_s(j + 2);
+        if (j + kG < n_tiles) {
+          ok = issue_s(j + kG);
           if (!ok) break;
         }
         mma_pv(t_dq, sds_a + g * kBlk, sk_a + st * kTileW, idesc_o, j != 0);
@@ -298,8 +300,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     const float lse2 = qrow < p.Sq ? p.lse[stat] * kLog2e : INFINITY;
     const float delta = qrow < p.Sq ? p.delta[stat] : 0.f;
     bool ok = true;
-    for (int j = g; j < n_tiles; j += 2) {
-      const int turn = j >> 1;
+    for (int j = g; j < n_tiles; j += kG) {
+      const int turn = j / kG;
       // S and dP are there; the dQ MMAs of the group's tile before have read dS
       bool ready = ptx::mbar_wait(&sp_full[g], turn & 1, abort_flag, p.timeout_ns);
       if (ready && turn > 0) ready = ptx::mbar_wait(&ds_empty[g], (turn - 1) & 1, abort_flag, p.timeout_ns);
@@ -348,7 +350,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&ds_full[g]);
     }
-    if (ok) {
+    if (ok && g < 2) {
       const bool done = ptx::mbar_wait(dq_full, 0, abort_flag, p.timeout_ns);
       if (!__all_sync(0xffffffffu, done)) {
         if (lane == 0) report_status(p.status, kStatusGemmTimeout, 67, blockIdx.x, 0);
@@ -369,27 +371,27 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 
 // ------------------------------------------------------------------------------------------------ dK, dV
 template <int D>
-__global__ void __launch_bounds__(kBwdThreads, 1)
+__global__ void __launch_bounds__(BwdCfg<D>::kThreads, 1)
 attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
                     const BwdArgs p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  constexpr int kTile = BwdCfg<D>::kTile, kTileW = BwdCfg<D>::kTileW, kStages = BwdCfg<D>::kStages;
+  constexpr int kTile = BwdCfg<D>::kTile, kTileW = BwdCfg<D>::kTileW, kStages = BwdCfg<D>::kStages, kG = BwdCfg<D>::kG;
   uint8_t* sk = smem;
   uint8_t* sv = sk + kTile;
   uint8_t* sq = sv + kTile;               // kStages tiles
   uint8_t* sdo = sq + kStages * kTileW;   // kStages tiles
   uint8_t* spt = sdo + kStages * kTileW;  // P^T of the groups: 128 keys x 64 queries bf16 each
-  uint8_t* sdst = spt + 2 * kBlk;         // dS^T
-  float* s_stat = reinterpret_cast<float*>(sdst + 2 * kBlk);  // per group: lse and delta of its tile's 64 queries
-  uint64_t* kv_full = reinterpret_cast<uint64_t*>(s_stat + 4 * kW);
+  uint8_t* sdst = spt + kG * kBlk;        // dS^T
+  float* s_stat = reinterpret_cast<float*>(sdst + kG * kBlk);  // per group: lse and delta of its tile's 64 queries
+  uint64_t* kv_full = reinterpret_cast<uint64_t*>(s_stat + kG * 2 * kW);
   uint64_t* qd_full = kv_full + 1;          // [kStages]
   uint64_t* qd_empty = qd_full + kStages;   // [kStages]
-  uint64_t* sp_full = qd_empty + kStages;   // [2] S^T and dP^T of a group's tile are complete
-  uint64_t* pt_full = sp_full + 2;          // [2] P^T and dS^T written by the group's four warps
-  uint64_t* pt_empty = pt_full + 2;         // [2] the MMAs have read them
-  uint64_t* acc_full = pt_empty + 2;
+  uint64_t* sp_full = qd_empty + kStages;   // [kG] S^T and dP^T of a group's tile are complete
+  uint64_t* pt_full = sp_full + kG;         // [kG] P^T and dS^T written by the group's four warps
+  uint64_t* pt_empty = pt_full + kG;        // [kG] the MMAs have read them
+  uint64_t* acc_full = pt_empty + kG;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -409,7 +411,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       ptx::mbar_init(&qd_full[s], 1);
       ptx::mbar_init(&qd_empty[s], 1);
     }
-    for (int g = 0; g < 2; ++g) {
+    for (int g = 0; g < kG; ++g) {
       ptx::mbar_init(&sp_full[g], 1);
       ptx::mbar_init(&pt_full[g], 4);
       ptx::mbar_init(&pt_empty[g], 1);
@@ -429,7 +431,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t t_dv = tmem_base + 256, t_dk = tmem_base + 256 + D;
+  const uint32_t t_dv = tmem_base + kG * 2 * kW, t_dk = t_dv + D;
 
   if (warp == 0) {
     if (n_iter > 0 && ptx::elect_one()) {
@@ -456,7 +458,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       const uint32_t sk_a = ptx::smem_u32(sk), sv_a = ptx::smem_u32(sv), sq_a = ptx::smem_u32(sq), sdo_a = ptx::smem_u32(sdo);
       const uint32_t spt_a = ptx::smem_u32(spt), sdst_a = ptx::smem_u32(sdst);
       auto issue_s = [&](int it) {
-        const int st = it % kStages, g = it & 1;
+        const int st = it % kStages, g = it % kG;
         if (!ptx::mbar_wait(&qd_full[st], (it / kStages) & 1, abort_flag, p.timeout_ns)) {
           report_status(p.status, kStatusGemmTimeout, 73, blockIdx.x, it);
           return false;
@@ -469,16 +471,16 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       };
       bool ok = ptx::mbar_wait(kv_full, 0, abort_flag, p.timeout_ns);
       if (!ok) report_status(p.status, kStatusGemmTimeout, 72, blockIdx.x, 0);
-      for (int it = 0; ok && it < 2 && it < n_iter; ++it) ok = issue_s(it);
+      for (int it = 0; ok && it < kG && it < n_iter; ++it) ok = issue_s(it);
       for (int it = 0; ok && it < n_iter; ++it) {
-        const int st = it % kStages, g = it & 1;
-        if (!ptx::mbar_wait(&pt_full[g], (it >> 1) & 1, abort_flag, p.timeout_ns)) {
+        const int st = it % kStages, g = it % kG;
+        if (!ptx::mbar_wait(&pt_full[g], (it / kG) & 1, abort_flag, p.timeout_ns)) {
           report_status(p.status, kStatusGemmTimeout, 74, blockIdx.x, it);
           break;
         }
         ptx::tc_fence_after();
-        if (it + 2 < n_iter) {
-          ok = issue_s(it + 2);
+        if (it + kG < n_iter) {
+          ok = issue_s(it + kG);
           if (!ok) break;
         }
         mma_pv(t_dv, spt_a + g * kBlk, sdo_a + st * kTileW, idesc_o, it != 0);   // dV += P^T dO_i
@@ -498,8 +500,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     float* slot = s_stat + g * 2 * kW;
     const long long stat_base = (static_cast<long long>(b) * p.H + h) * p.Sq;
     bool ok = true;
-    for (int it = g; it < n_iter; it += 2) {
-      const int i = i_begin + it, turn = it >> 1;
+    for (int it = g; it < n_iter; it += kG) {
+      const int i = i_begin + it, turn = it / kG;
       float nl[2], nd[2];
 #pragma unroll
       for (int x = 0; x < 2; ++x) {
@@ -591,7 +593,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         reinterpret_cast<uint4*>(dk)[q] = make_uint4(0u, 0u, 0u, 0u);
       }
     }
-    if (n_iter > 0 && ok) {  // both uniform over the warp
+    if (n_iter > 0 && ok && g < 2) {  // all uniform over the warp
       const bool done = ptx::mbar_wait(acc_full, 0, abort_flag, p.timeout_ns);
       if (!__all_sync(0xffffffffu, done)) {
         if (lane == 0) report_status(p.status, kStatusGemmTimeout, 77, blockIdx.x, 0);
@@ -720,9 +722,9 @@ int launch_bwd(const CUtensorMap (&fixed)[4], const CUtensorMap (&walked)[4], co
   attn_delta_kernel<D><<<static_cast<unsigned>((rows * (D / 8) + 255) / 256), 256, 0, stream>>>(
       static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out),
       const_cast<float*>(a.delta), a.B, a.H, a.Sq);
-  attn_bwd_dq_kernel<D><<<dim3((a.Sq + kT - 1) / kT, a.B * a.H), kBwdThreads, BwdCfg<D>::kSmemDq, stream>>>(
+  attn_bwd_dq_kernel<D><<<dim3((a.Sq + kT - 1) / kT, a.B * a.H), BwdCfg<D>::kThreads, BwdCfg<D>::kSmemDq, stream>>>(
       fixed[0], walked[1], walked[2], fixed[3], a);
-  attn_bwd_dkv_kernel<D><<<dim3((a.Skv + kT - 1) / kT, a.B * a.H), kBwdThreads, BwdCfg<D>::kSmemDkv, stream>>>(
+  attn_bwd_dkv_kernel<D><<<dim3((a.Skv + kT - 1) / kT, a.B * a.H), BwdCfg<D>::kThreads, BwdCfg<D>::kSmemDkv, stream>>>(
       walked[0], fixed[1], fixed[2], walked[3], a);
   return static_cast<int>(cudaGetLastError());
 }

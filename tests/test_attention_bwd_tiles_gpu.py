@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("causal", [False, True])
 @pytest.mark.parametrize("D", [64, 128])
-@pytest.mark.parametrize("Sq,Skv", [(1, 1), (63, 64), (64, 65), (65, 127), (128, 128), (129, 192), (200, 257), (320, 385)])
+@pytest.mark.parametrize("Sq,Skv", [(1, 1), (63, 64), (64, 65), (65, 127), (128, 128), (129, 192), (200, 257), (320, 385), (449, 577)])
 def test_gradients(Sq, Skv, D, causal):
     from ferrum_b200.ops import functional as F
     from ferrum_b200.utils.runtime import check_status
