@@ -70,7 +70,7 @@ def _torch_flags() -> tuple[list[str], list[str]]:
     cflags = [*(f"-I{p}" for p in inc), f"-I{sysconfig.get_paths()['include']}",
               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DTORCH_EXTENSION_NAME=_native",
               "-fvisibility=hidden", "-Wno-deprecated-declarations"]
-    lflags = [f"-L{root / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+    lflags = [f"-L{root / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10_cuda", "-lc10"]
     return cflags, lflags
 
 

@@ -233,6 +233,11 @@ int fb_embedding_fwd(const float* weight, const long long* idx, void* out, long 
 int fb_embedding_meanpool_fwd(const float* weight, const long long* idx, void* out, long long batch, int seq,
                               int dim, long long vocab, int out_dtype, cudaStream_t stream);
 // dW[idx[i]] += scale * dout[i / group] ; `sorted_idx/perm` come from a radix sort of idx.
+int fb_embedding_pairs(const long long* idx, int32_t* keys, int32_t* rows, long long n, long long vocab, long long group,
+                       cudaStream_t stream);
+int fb_embedding_bwd_pairs(const void* dout, const int32_t* keys, const int32_t* rows, float* dweight, long long n_idx,
+                           int dim, int group, float scale, long long padding_idx, long long vocab, int dtype,
+                           cudaStream_t stream);
 int fb_embedding_keys(const long long* idx, int32_t* keys, long long n, long long vocab, cudaStream_t stream);
 int fb_embedding_bwd_sorted(const void* dout, const void* sorted_idx, int key_bytes, const long long* perm,
                             float* dweight, long long n_idx, int dim, int group, float scale, long long padding_idx,

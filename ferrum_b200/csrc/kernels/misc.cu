@@ -244,25 +244,28 @@ __global__ void embedding_meanpool_kernel(const float* __restrict__ w, const lon
 }
 
 // Row numbers as 32-bit sort keys: half the bytes and half the passes of a radix sort of the 64-bit indices.  Indices
-// outside the table (reported by the forward pass) become `vocab`, which the scatter drops.
-__global__ void embedding_keys_kernel(const long long* __restrict__ idx, int32_t* __restrict__ keys, long long n,
-                                      long long vocab) {
+// outside the table (reported by the forward pass) become `vocab`, which the scatter drops.  rows (optional): the row of
+// the gradient that position i adds, i / group.
+__global__ void embedding_keys_kernel(const long long* __restrict__ idx, int32_t* __restrict__ keys,
+                                      int32_t* __restrict__ rows, long long n, long long vocab, long long group) {
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
     const long long id = __ldg(idx + i);
     keys[i] = static_cast<int32_t>(id < 0 || id > vocab ? vocab : id);
+    if (rows != nullptr) rows[i] = static_cast<int32_t>(i / group);
   }
 }
 
-// Scatter-add over a SORTED index list: a block walks a chunk of 32 consecutive positions, sums runs of equal
+// Scatter-add over a SORTED index list: at[i] is the original position of the i-th index (64 bits) or the row of dout it
+// adds (32 bits).  A block walks a chunk of 32 consecutive positions, sums runs of equal
 // indices in registers and flushes each run once, so heavily repeated tokens cost one flush per chunk instead of
-// one per occurrence.  perm[i] is the original position.  The chunk's ids and source rows are staged in shared
+// one per occurrence.  The chunk's ids and source rows are staged in shared
 // memory once (one 64-bit division per position instead of one per thread and position); with dim % 4 == 0 a
 // thread owns four adjacent columns: 8- or 16-byte loads of dout and one vector atomic (red.global.add.v4.f32)
 // per run.
-template <typename G, typename Key>
+template <typename G, typename Key, typename At>
 __global__ void embedding_bwd_sorted_kernel(const G* __restrict__ dout, const Key* __restrict__ sorted_idx,
-                                            const long long* __restrict__ perm, float* __restrict__ dw,
+                                            const At* __restrict__ at, float* __restrict__ dw,
                                             long long n_idx, int dim, int group, float scale,
                                             long long padding_idx, long long vocab, int32_t* bstatus) {
   constexpr int kChunk = 32;
@@ -272,7 +275,7 @@ __global__ void embedding_bwd_sorted_kernel(const G* __restrict__ dout, const Ke
   const int cnt = static_cast<int>(min(n_idx, lo + kChunk) - lo);
   if (threadIdx.x < cnt) {
     long long id = sorted_idx[lo + threadIdx.x];
-    const long long row = perm[lo + threadIdx.x] / group;
+    const long long row = sizeof(At) == 4 ? static_cast<long long>(at[lo + threadIdx.x]) : at[lo + threadIdx.x] / group;
     // ids outside the table were reported by the forward pass; their gradient rows are dropped, never written.
     if (id >= vocab) id = -1;
     if (!FB_INDEX_OK(bstatus, 40, row, (n_idx + group - 1) / group)) id = -1;
@@ -673,35 +676,57 @@ extern "C" int fb_embedding_meanpool_fwd(const float* weight, const long long* i
   return static_cast<int>(cudaGetLastError());
 }
 
-// keys[i] = idx[i], or vocab (< 2^31 - 1) where that is no row of the table.
-extern "C" int fb_embedding_keys(const long long* idx, int32_t* keys, long long n, long long vocab, cudaStream_t stream) {
+// keys[i] = idx[i], or vocab (< 2^31 - 1) where that is no row of the table; rows[i] = i / group.
+extern "C" int fb_embedding_pairs(const long long* idx, int32_t* keys, int32_t* rows, long long n, long long vocab,
+                                  long long group, cudaStream_t stream) {
   if (n <= 0) return 0;
-  if (vocab <= 0 || vocab >= 0x7fffffffLL) return -1;
+  if (vocab <= 0 || vocab >= 0x7fffffffLL || group <= 0 || (n - 1) / group >= 0x7fffffffLL) return -1;
   const long long want = (n + 255) / 256, cap = sm_count() * 8LL;
-  embedding_keys_kernel<<<static_cast<int>(want < cap ? want : cap), 256, 0, stream>>>(idx, keys, n, vocab);
+  embedding_keys_kernel<<<static_cast<int>(want < cap ? want : cap), 256, 0, stream>>>(idx, keys, rows, n, vocab, group);
   return static_cast<int>(cudaGetLastError());
 }
+extern "C" int fb_embedding_keys(const long long* idx, int32_t* keys, long long n, long long vocab, cudaStream_t stream) {
+  if (n <= 0) return 0;
+  return fb_embedding_pairs(idx, keys, nullptr, n, vocab, n, stream);
+}
 
-// sorted_idx: 32-bit (key_bytes = 4) or 64-bit (8) row numbers.
+namespace {
+template <typename Key, typename At>
+int embedding_bwd(const void* dout, const void* sorted_idx, const void* at, float* dweight, long long n_idx, int dim, int group,
+                  float scale, long long padding_idx, long long vocab, int dtype, cudaStream_t stream) {
+  if (n_idx <= 0 || dim <= 0) return 0;
+  const long long nb = (n_idx + 31) / 32;
+  if (group < 1 || nb > 2147483647LL || (dtype != FB_DT_F32 && dtype != FB_DT_BF16)) return -1;
+  const int threads = dim >= 256 ? 256 : (dim >= 128 ? 128 : 64);
+  const auto run = [&](auto kernel, auto* d) {
+    kernel<<<static_cast<unsigned>(nb), threads, 0, stream>>>(d, static_cast<const Key*>(sorted_idx), static_cast<const At*>(at),
+                                                              dweight, n_idx, dim, group, scale, padding_idx, vocab,
+                                                              bounds_status_ref());
+    return static_cast<int>(cudaGetLastError());
+  };
+  return dtype == FB_DT_F32
+             ? run(embedding_bwd_sorted_kernel<float, Key, At>, static_cast<const float*>(dout))
+             : run(embedding_bwd_sorted_kernel<__nv_bfloat16, Key, At>, static_cast<const __nv_bfloat16*>(dout));
+}
+}  // namespace
+
+// sorted_idx: 32-bit (key_bytes = 4) or 64-bit (8) row numbers; perm: their original positions.
 extern "C" int fb_embedding_bwd_sorted(const void* dout, const void* sorted_idx, int key_bytes, const long long* perm,
                                        float* dweight, long long n_idx, int dim, int group, float scale,
                                        long long padding_idx, long long vocab, int dtype, cudaStream_t stream) {
-  if (n_idx <= 0 || dim <= 0) return 0;
-  if (group < 1 || (key_bytes != 4 && key_bytes != 8)) return -1;
-  const long long nb = (n_idx + 31) / 32;
-  if (nb > 2147483647LL) return -1;
-  const int threads = dim >= 256 ? 256 : (dim >= 128 ? 128 : 64);
-#define FB_EMBEDDING_BWD(G, KEY)                                                                                   \
-  embedding_bwd_sorted_kernel<G, KEY><<<static_cast<unsigned>(nb), threads, 0, stream>>>(                           \
-      static_cast<const G*>(dout), static_cast<const KEY*>(sorted_idx), perm, dweight, n_idx, dim, group, scale,    \
-      padding_idx, vocab, bounds_status_ref())
-  if (dtype == FB_DT_F32 && key_bytes == 4) FB_EMBEDDING_BWD(float, int32_t);
-  else if (dtype == FB_DT_F32) FB_EMBEDDING_BWD(float, long long);
-  else if (dtype == FB_DT_BF16 && key_bytes == 4) FB_EMBEDDING_BWD(__nv_bfloat16, int32_t);
-  else if (dtype == FB_DT_BF16) FB_EMBEDDING_BWD(__nv_bfloat16, long long);
-  else return -1;
-#undef FB_EMBEDDING_BWD
-  return static_cast<int>(cudaGetLastError());
+  if (key_bytes == 4)
+    return embedding_bwd<int32_t, long long>(dout, sorted_idx, perm, dweight, n_idx, dim, group, scale, padding_idx, vocab,
+                                             dtype, stream);
+  if (key_bytes == 8)
+    return embedding_bwd<long long, long long>(dout, sorted_idx, perm, dweight, n_idx, dim, group, scale, padding_idx, vocab,
+                                               dtype, stream);
+  return n_idx <= 0 || dim <= 0 ? 0 : -1;
+}
+// The same for pairs of fb_embedding_pairs, sorted by key: rows are rows of dout, `group` of the indices to each.
+extern "C" int fb_embedding_bwd_pairs(const void* dout, const int32_t* keys, const int32_t* rows, float* dweight,
+                                      long long n_idx, int dim, int group, float scale, long long padding_idx,
+                                      long long vocab, int dtype, cudaStream_t stream) {
+  return embedding_bwd<int32_t, int32_t>(dout, keys, rows, dweight, n_idx, dim, group, scale, padding_idx, vocab, dtype, stream);
 }
 
 extern "C" int fb_gather_rows(const void* src, const long long* idx, void* dst, long long n_idx,

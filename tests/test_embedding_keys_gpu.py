@@ -35,3 +35,43 @@ def test_gradient(vocab, n, dim, padding):
                        "fb_embedding_bwd_sorted")
             check_status()
             assert ((dw - want).abs() <= 2.0 ** -22 * size * 8).all()
+
+
+@pytest.mark.parametrize("vocab,batch,seq,dim", [(1, 3, 5, 4), (2, 1, 1, 8), (255, 7, 33, 12), (256, 64, 70, 8), (65536, 9, 31, 5)])
+def test_pairs(vocab, batch, seq, dim):
+    """Pairs sorted by no more bits than a row number has, index vocab (outside) included; mean of `seq` rows, padding."""
+    from ferrum_b200 import _lib
+    from ferrum_b200.ops import functional as F
+    from ferrum_b200.utils.runtime import check_status
+
+    g = torch.Generator(device="cuda").manual_seed(vocab)
+    n, idx = batch * seq, torch.randint(0, vocab, (batch, seq), device="cuda", generator=g)
+    idx.view(-1)[0] = vocab - 1
+    lib, st = _lib.cuda(), torch.cuda.current_stream().cuda_stream
+    odd = idx.clone().view(-1)
+    odd[-1] = vocab + 7
+    keys, rows = (torch.empty(n, dtype=torch.int32, device="cuda") for _ in range(2))
+    _lib.check(lib.fb_embedding_pairs(odd.data_ptr(), keys.data_ptr(), rows.data_ptr(), n, vocab, seq, st), "pairs")
+    assert torch.equal(keys.long(), odd.clamp(max=vocab)) and torch.equal(rows.long(), torch.arange(n, device="cuda") // seq)
+    key, perm = torch.sort(keys, stable=True)
+    dout, dw = torch.randn(batch, dim, device="cuda", generator=g), torch.zeros(vocab, dim, device="cuda")
+    _lib.check(lib.fb_embedding_bwd_pairs(dout.data_ptr(), key.data_ptr(), rows[perm].data_ptr(), dw.data_ptr(), n, dim, seq,
+                                          1.0 / seq, -1, vocab, 0, st), "bwd")
+    check_status()
+    per = dout.double().repeat_interleave(seq, 0) / seq
+    want, size = (torch.zeros(vocab, dim, device="cuda", dtype=torch.float64) for _ in range(2))
+    want.index_add_(0, odd[:-1], per[:-1])
+    size.index_add_(0, odd[:-1], per[:-1].abs())
+    assert ((dw - want).abs() <= 2.0 ** -22 * size * 8).all()
+    for pool, padding in ((True, None), (False, 0)):
+        w = torch.randn(vocab, dim, device="cuda", generator=g).requires_grad_(True)
+        y = F.embedding_mean_pool(w, idx) if pool else F.embedding(w, idx, padding_idx=padding)
+        gy = torch.randn(y.shape, device="cuda", generator=g)
+        y.backward(gy)
+        per = (gy.double() / seq).repeat_interleave(seq, 0) if pool else gy.double().reshape(n, dim)
+        want, size = (torch.zeros(vocab, dim, device="cuda", dtype=torch.float64) for _ in range(2))
+        keep = torch.ones(n, dtype=torch.bool, device="cuda") if padding is None else idx.view(-1) != padding
+        want.index_add_(0, idx.view(-1)[keep], per[keep])
+        size.index_add_(0, idx.view(-1)[keep], per[keep].abs())
+        check_status()
+        assert ((w.grad - want).abs() <= 2.0 ** -22 * size * 8).all()
