@@ -148,6 +148,7 @@ _CUDA_SIGS = {
     "fb_reduce": (I, [P, P, LL, LL, LL, I, P, LL, P]),
     "fb_arg_reduce": (I, [P, P, P, LL, LL, LL, I, P]),
     "fb_colsum": (I, [P, P, LL, LL, I, I, P]),
+    "fb_unary_bwd_colsum": (I, [P, P, P, P, LL, LL, I, I, P]),
     # norms
     "fb_layernorm_fwd": (I, [P, P, P, P, P, P, LL, I, F, I, I, P]),
     "fb_layernorm_set_status": (None, [P]),

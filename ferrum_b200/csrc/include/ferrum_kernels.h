@@ -134,6 +134,9 @@ int fb_reduce(const float* x, float* out, long long outer, long long R, long lon
 int fb_arg_reduce(const float* x, long long* idx, float* val, long long outer, long long R, long long inner,
                   int is_max, cudaStream_t stream);
 // Column sums of a [rows, cols] matrix (fp32 or bf16 in, fp32 out): bias gradients.
+// dx = dy * act'(y) of a ReLU, tanh or sigmoid, and its column sums; -3: these want fb_colsum.
+int fb_unary_bwd_colsum(const void* dy, const void* y, void* dx, float* sums, long long rows, long long cols, int op, int dtype,
+                        cudaStream_t stream);
 int fb_colsum(const void* x, float* out, long long rows, long long cols, int dtype, int accumulate,
               cudaStream_t stream);
 
@@ -143,7 +146,7 @@ void fb_layernorm_set_status(int32_t* status);
 // pre_act: FB_ACT_NONE or FB_ACT_GELU applied to x before normalising (fused block).
 int fb_layernorm_fwd(const void* x, const float* gamma, const float* beta, void* y, float* mean, float* rstd,
                      long long rows, int cols, float eps, int pre_act, int dtype, cudaStream_t stream);
-// stats = [3][cols]: d_gamma, d_beta, column sum of dx (accumulated into); partial = [nblk][3][cols] workspace.
+// stats = [3][cols]: d_gamma, d_beta, column sum of dx (added to, or written where want_colsum has the bit 2); partial = [nblk][3][cols] workspace.
 // act_grad (optional, dtype of x; excludes pre_act): x holds act(z) and act_grad holds act'(z) as written by
 // the producing GEMM's epilogue; dx is then the gradient of z.
 int fb_layernorm_bwd(const void* dy, const void* x, const void* act_grad, const float* gamma, const float* mean,

@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include "../include/ferrum_kernels.h"
+#include "column_sums.cuh"
 
 namespace fb {
 namespace {
@@ -184,6 +185,46 @@ __global__ void unary_bwd_f32(const float* __restrict__ dy, const float* __restr
     for (long long i = tid; i < n; i += stride) dx[i] = unary_grad(dy[i], sp[i], OP, a, b);
   }
 }
+
+// The gradient in front of an activation and its column sums (the gradient of a bias) in one pass: dx = dy * act'(y), the
+// sums those of the stored values.
+template <typename T, int OP>
+struct GradRows {
+  static constexpr int kV = 16 / sizeof(T), kU = 4;
+  using Elem = T;
+  struct Raw {
+    uint4 g, y;
+  };
+  const T *dy, *y;
+  T* dx;
+  __host__ __device__ bool aligned() const {
+    return ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(dx)) & 15) == 0;
+  }
+  __device__ Raw fetch(long long at) const {
+    return Raw{*reinterpret_cast<const uint4*>(dy + at), *reinterpret_cast<const uint4*>(y + at)};
+  }
+  __device__ void use(const Raw& r, long long at, float (&v)[kV]) const {
+    float s[kV];
+    unpack16<T>(r.g, v);
+    unpack16<T>(r.y, s);
+#pragma unroll
+    for (int i = 0; i < kV; ++i) v[i] = sizeof(T) == 4 ? unary_grad(v[i], s[i], OP, 0.f, 0.f) : unary_grad_fast(v[i], s[i], OP, 0.f, 0.f);
+    uint4 o;
+    if constexpr (sizeof(T) == 4) {
+      o = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
+    } else {
+      o = f32_to_bf16x8(v);
+      unpack16<T>(o, v);
+    }
+    *reinterpret_cast<uint4*>(dx + at) = o;
+  }
+  __device__ float one(long long at) const {
+    const float g = static_cast<float>(dy[at]), s = static_cast<float>(y[at]);
+    const T d = static_cast<T>(sizeof(T) == 4 ? unary_grad(g, s, OP, 0.f, 0.f) : unary_grad_fast(g, s, OP, 0.f, 0.f));
+    dx[at] = d;
+    return static_cast<float>(d);
+  }
+};
 
 template <int OP>
 __global__ void unary_fwd_bf16(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, long long n,
@@ -564,6 +605,32 @@ extern "C" int fb_unary_fwd(const void* x, void* y, long long n, int op, float a
     return -1;
   }
   return static_cast<int>(cudaGetLastError());
+}
+
+// dx = dy * act'(y) for an activation whose derivative is a function of its result (ReLU, tanh, sigmoid), [rows, cols], and
+// sums[cols] = its column sums.  -3: a shape whose column sums want a launch of their own.
+extern "C" int fb_unary_bwd_colsum(const void* dy, const void* y, void* dx, float* sums, long long rows, long long cols, int op,
+                                   int dtype, cudaStream_t stream) {
+  using namespace fb;
+  if (cols <= 0) return 0;
+  if (rows <= 0) return static_cast<int>(cudaMemsetAsync(sums, 0, static_cast<size_t>(cols) * sizeof(float), stream));
+  const auto run = [&](auto type) {
+    using T = decltype(type);
+    if (!column_cluster_fits<T>(rows, cols)) return -3;
+    const T *g = static_cast<const T*>(dy), *r = static_cast<const T*>(y);
+    T* d = static_cast<T*>(dx);
+    switch (op) {
+      case FB_ACT_RELU:
+        return launch_colsum(GradRows<T, FB_ACT_RELU>{g, r, d}, sums, rows, cols, 0, stream);
+      case FB_ACT_TANH:
+        return launch_colsum(GradRows<T, FB_ACT_TANH>{g, r, d}, sums, rows, cols, 0, stream);
+      case FB_ACT_SIGMOID:
+        return launch_colsum(GradRows<T, FB_ACT_SIGMOID>{g, r, d}, sums, rows, cols, 0, stream);
+      default:
+        return -1;
+    }
+  };
+  return dtype == FB_DT_F32 ? run(float{}) : dtype == FB_DT_BF16 ? run(__nv_bfloat16{}) : -1;
 }
 
 extern "C" int fb_unary_bwd(const void* dy, const void* saved, void* dx, long long n, int op, float alpha,

@@ -26,6 +26,7 @@
 #include "../common/ptx.cuh"
 #include "../common/status.h"
 #include "../include/ferrum_kernels.h"
+#include "column_sums.cuh"
 
 namespace fb {
 namespace {
@@ -954,14 +955,14 @@ ln_bwd_ring_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   }
 }
 
-// Fold partial[nblk][3*cols] into stats[3*cols] (accumulated into): block = 128 columns x a chunk of the
+// Fold partial[nblk][3*cols] into stats[3*cols] (written or added to): block = 128 columns x a chunk of the
 // nblk rows, lanes own 4 adjacent columns, partials leave with one atomicAdd per column per block.  kVec: 16-byte loads
 // (ncols a multiple of 4, partial on a 16-byte address).
 template <bool kVec>
 __global__ void __launch_bounds__(256)
 ln_fold_kernel(const float* __restrict__ partial, float* __restrict__ stats, int nblk, int ncols,
-               int rows_per_block) {
-  __shared__ float sm[8][128];
+               int rows_per_block, int add) {
+  __shared__ float sm[8][128], part[128];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c0 = blockIdx.x * 128 + lane * 4;
   const int r_lo = blockIdx.y * rows_per_block;
@@ -990,9 +991,12 @@ ln_fold_kernel(const float* __restrict__ partial, float* __restrict__ stats, int
     float s = 0.f;
 #pragma unroll
     for (int w = 0; w < 8; ++w) s += sm[w][threadIdx.x];
-    const int c = blockIdx.x * 128 + threadIdx.x;
-    if (c < ncols) atomicAdd(stats + c, s);
+    part[threadIdx.x] = s;
   }
+  cluster_sums(part, 128, [&](int i, float s) {
+    const int c = static_cast<int>(blockIdx.x) * 128 + i;
+    if (c < ncols) stats[c] = add ? stats[c] + s : s;
+  });
 }
 
 // ---------------------------------------------------------------- rows of any width and alignment in registers
@@ -1453,7 +1457,8 @@ bool launch_wide<__nv_bfloat16>(const __nv_bfloat16* dy, const __nv_bfloat16* x,
 template <typename T>
 int bwd_t(const void* dy, const void* x, const void* act_grad, const float* gamma, const float* mean,
           const float* rstd, void* dx, __nv_bfloat16* dx_low, float* partial, float* stats, long long rows, int cols,
-          int pre_act, int nblk, int want_colsum, cudaStream_t st) {
+          int pre_act, int nblk, int flags, cudaStream_t st) {
+  const int want_colsum = flags & 1, add = (flags & 2) == 0;
   const T* dyp = static_cast<const T*>(dy);
   const T* xp = static_cast<const T*>(x);
   const T* agp = static_cast<const T*>(act_grad);
@@ -1493,14 +1498,17 @@ int bwd_t(const void* dy, const void* x, const void* act_grad, const float* gamm
     }
     const int ncols = 3 * cols;
     const int col_blocks = (ncols + 127) / 128;
-    int row_blocks = (sm_count() * 2 + col_blocks - 1) / col_blocks;
-    const int max_rb = (used + 15) / 16;
-    if (row_blocks > max_rb) row_blocks = max_rb;
-    if (row_blocks < 1) row_blocks = 1;
+    int row_blocks = 1;  // one cluster to a column block
+    while (row_blocks < 8 && row_blocks * col_blocks < sm_count() * 2 && row_blocks * 16 < used) row_blocks *= 2;
     const int rpb = (used + row_blocks - 1) / row_blocks;
     const auto fold = ncols % 4 == 0 && aligned16(partial, nullptr, nullptr, nullptr) ? ln_fold_kernel<true> : ln_fold_kernel<false>;
-    fold<<<dim3(col_blocks, row_blocks), 256, 0, st>>>(partial, stats, used, ncols, rpb);
+    return launch_column_cluster(fold, dim3(col_blocks, row_blocks), st, static_cast<const float*>(partial), stats, used, ncols,
+                                 rpb, add);
   } else {
+    if (!add) {
+      const cudaError_t e = cudaMemsetAsync(stats, 0, 3 * static_cast<size_t>(cols) * sizeof(float), st);
+      if (e != cudaSuccess) return static_cast<int>(e);
+    }
     const int grid = static_cast<int>(rows < sm_count() * 4LL ? rows : sm_count() * 4LL);
     ln_bwd_generic<T><<<grid, 256, 0, st>>>(dyp, xp, agp, gamma, mean, rstd, dxp, stats, rows, cols, pre_act,
                                             want_colsum);
@@ -1538,15 +1546,19 @@ extern "C" int fb_layernorm_fwd(const void* x, const float* gamma, const float* 
   return -1;
 }
 
-// stats = [3][cols] fp32: d_gamma, d_beta and the column sum of dx.  All three are ACCUMULATED into
-// (zero the buffer for a fresh gradient); the column sum is produced only when want_colsum != 0.
+// stats = [3][cols] fp32: d_gamma, d_beta and the column sum of dx.  All three are ACCUMULATED into (zero the buffer for a
+// fresh gradient), or written where want_colsum has the bit 2; the column sum is produced only where it has the bit 1.
 // act_grad (optional, dtype of x): x then holds act(z) of an activation applied before the normalisation and
 // act_grad its derivative act'(z); dx is the gradient of z.  (pre_act instead re-evaluates a GELU from z.)
 extern "C" int fb_layernorm_bwd(const void* dy, const void* x, const void* act_grad, const float* gamma,
                                 const float* mean, const float* rstd, void* dx, float* partial, float* stats,
                                 long long rows, int cols, int pre_act, int dtype, int nblk, int want_colsum,
                                 cudaStream_t stream) {
-  if (rows <= 0 || cols <= 0) return 0;
+  if (cols <= 0) return 0;
+  if (rows <= 0)  // empty sums
+    return (want_colsum & 2) == 0 || stats == nullptr
+               ? 0
+               : static_cast<int>(cudaMemsetAsync(stats, 0, 3 * static_cast<size_t>(cols) * sizeof(float), stream));
   if (stats == nullptr) return -1;
   if (act_grad != nullptr && pre_act != FB_ACT_NONE) return -1;
   if (dtype == FB_DT_F32)
@@ -1573,12 +1585,12 @@ extern "C" int fb_add_layernorm_fwd(const float* x, const void* r, const float* 
   return -1;
 }
 
-// fb_layernorm_bwd of fp32 rows, whose dx also goes to dx_low (optional) in bf16.
+// fb_layernorm_bwd of fp32 rows, whose dx also goes to dx_low (optional) in bf16; stats are written.
 extern "C" int fb_add_layernorm_bwd(const float* dy, const float* sum, const float* gamma, const float* mean,
                                     const float* rstd, float* dx, void* dx_low, float* partial, float* stats,
                                     long long rows, int cols, int nblk, cudaStream_t stream) {
   if (rows <= 0 || cols <= 0) return 0;
   if (stats == nullptr) return -1;
   return bwd_t<float>(dy, sum, nullptr, gamma, mean, rstd, dx, static_cast<__nv_bfloat16*>(dx_low), partial, stats, rows,
-                      cols, FB_ACT_NONE, nblk, 0, stream);
+                      cols, FB_ACT_NONE, nblk, 2, stream);
 }

@@ -15,6 +15,7 @@
 #include <float.h>
 
 #include "../include/ferrum_kernels.h"
+#include "column_sums.cuh"
 
 namespace fb {
 namespace {
@@ -424,7 +425,14 @@ extern "C" int fb_arg_reduce(const float* x, long long* idx, float* val, long lo
 
 extern "C" int fb_colsum(const void* x, float* out, long long rows, long long cols, int dtype, int accumulate,
                          cudaStream_t stream) {
-  if (rows <= 0 || cols <= 0) return 0;
+  if (cols <= 0) return 0;
+  if (rows <= 0)  // an empty sum
+    return accumulate ? 0 : static_cast<int>(cudaMemsetAsync(out, 0, cols * sizeof(float), stream));
+  if (dtype == FB_DT_F32 && fb::column_cluster_fits<float>(rows, cols))
+    return fb::launch_colsum(fb::PlainRows<float>{static_cast<const float*>(x)}, out, rows, cols, accumulate, stream);
+  if (dtype == FB_DT_BF16 && fb::column_cluster_fits<__nv_bfloat16>(rows, cols))
+    return fb::launch_colsum(fb::PlainRows<__nv_bfloat16>{static_cast<const __nv_bfloat16*>(x)}, out, rows, cols, accumulate,
+                             stream);
   if (!accumulate) {
     cudaError_t e = cudaMemsetAsync(out, 0, cols * sizeof(float), stream);
     if (e != cudaSuccess) return static_cast<int>(e);

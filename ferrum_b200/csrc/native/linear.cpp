@@ -1,8 +1,6 @@
 // Linear layers: act(x W^T + b), LayerNorm(act(x W^T + b)) as one node, LayerNorm.
 #include "native.h"
 
-extern "C" int fb_rt_memset(void* p, int value, unsigned long long bytes, cudaStream_t stream);
-
 namespace fbn {
 namespace {
 
@@ -38,7 +36,7 @@ std::vector<int64_t> out_sizes(const Tensor& x, int64_t last) {
 // Gradient of a Linear's input, weight and bias from g2 [M, N], in the precision of the forward pass.
 void linear_grads(const Tensor& g2, const Tensor& x2, const Tensor& w, bool low, at::ScalarType x_dtype,
                   at::IntArrayRef x_sizes, const std::shared_ptr<Sink>& sink, bool need_x, bool need_w, bool need_b,
-                  variable_list& out) {
+                  variable_list& out, const Tensor& sums = Tensor()) {  // sums: the bias' gradient, if known
   const bool tf32 = !low && g_tf32.load(std::memory_order_relaxed);
   const int64_t N = w.size(0), K = w.size(1);
   if (need_x) {  // before the weight gradient: the weight may be overwritten once its bucket is reduced
@@ -55,7 +53,9 @@ void linear_grads(const Tensor& g2, const Tensor& x2, const Tensor& w, bool low,
       out[1] = gw;
     }
   }
-  if (need_b) {
+  if (need_b && sums.defined()) {
+    out[2] = sums;
+  } else if (need_b) {
     Tensor gb = empty({N}, g2, at::kFloat);
     FB_CALL(fb_colsum, g2.data_ptr(), gb.data_ptr<float>(), g2.size(0), N, dt(g2), 0, cur_stream());
     out[2] = gb;
@@ -83,14 +83,28 @@ struct LinearNode : Node {
     NoAutograd below;
     Tensor x2 = as2d(x), g2 = contig(as2d(grads[0]));
     g2 = low ? cast(g2, at::kBFloat16) : cast(g2, at::kFloat);
+    const bool need_b = has_bias && task_should_compute_output(2);
+    Tensor sums;
     if (act != kNone) {  // only activations whose derivative is a function of the output are fused
       y = as2d(y);
       Tensor d = empty(g2.sizes(), g2, g2.scalar_type());
-      FB_CALL(fb_unary_bwd, g2.data_ptr(), y.data_ptr(), d.data_ptr(), g2.numel(), act, 0.f, 0.f, dt(g2), cur_stream());
+      int rc = -3;
+      if (need_b && g2.numel() > 0) {  // with the bias' gradient, unless its sums want a launch of their own
+        sums = empty({g2.size(1)}, g2, at::kFloat);
+        launch("fb_unary_bwd_colsum", [&] {
+          rc = fb_unary_bwd_colsum(g2.data_ptr(), y.data_ptr(), d.data_ptr(), sums.data_ptr<float>(), g2.size(0), g2.size(1), act,
+                                   dt(g2), cur_stream());
+          return rc == -3 ? 0 : rc;
+        });
+      }
+      if (rc == -3) {
+        sums = Tensor();
+        FB_CALL(fb_unary_bwd, g2.data_ptr(), y.data_ptr(), d.data_ptr(), g2.numel(), act, 0.f, 0.f, dt(g2), cur_stream());
+      }
       g2 = d;
     }
-    linear_grads(g2, x2, w, low, x_dtype, x_sizes, sink, task_should_compute_output(0), task_should_compute_output(1),
-                 has_bias && task_should_compute_output(2), out);
+    linear_grads(g2, x2, w, low, x_dtype, x_sizes, sink, task_should_compute_output(0), task_should_compute_output(1), need_b,
+                 out, sums);
     return out;
   }
 };
@@ -139,10 +153,9 @@ Tensor norm_bwd(const Tensor& gy2, const Tensor& x2, const Tensor& dact, const T
   const int nblk = fb_layernorm_bwd_blocks(rows, static_cast<int>(cols));
   Tensor partial = empty({std::max(nblk, 1), 3, cols}, x2, at::kFloat);
   Tensor stats = empty({3, cols}, x2, at::kFloat);
-  fb_rt_memset(stats.data_ptr(), 0, stats.numel() * 4, cur_stream());
   FB_CALL(fb_layernorm_bwd, gy2.data_ptr(), x2.data_ptr(), ptr(dact), fptr(gamma), s.mean.data_ptr<float>(),
           s.rstd.data_ptr<float>(), dx.data_ptr(), partial.data_ptr<float>(), stats.data_ptr<float>(), rows,
-          static_cast<int>(cols), pre, dt(x2), nblk, colsum ? 1 : 0, cur_stream());
+          static_cast<int>(cols), pre, dt(x2), nblk, colsum ? 3 : 2, cur_stream());
   return stats;
 }
 
@@ -226,7 +239,6 @@ struct AddNormNode : Node {
       const int nblk = fb_layernorm_bwd_blocks(rows, static_cast<int>(cols));
       Tensor partial = empty({std::max(nblk, 1), 3, cols}, sum, at::kFloat);
       stats = empty({3, cols}, sum, at::kFloat);
-      fb_rt_memset(stats.data_ptr(), 0, stats.numel() * 4, cur_stream());
       FB_CALL(fb_add_layernorm_bwd, gy.data_ptr<float>(), sum.data_ptr<float>(), fptr(g), mean.data_ptr<float>(),
               rstd.data_ptr<float>(), dx.data_ptr<float>(), low.data_ptr(), partial.data_ptr<float>(),
               stats.data_ptr<float>(), rows, static_cast<int>(cols), nblk, cur_stream());

@@ -1,0 +1,80 @@
+"""Column sums of a matrix whose rows are divided over a cluster, against fp64: alone, behind the gradient of an activation and
+as the fold of the LayerNorm backward's partial sums.  Bound: partial sums of at most a few hundred fp32 additions each,
+2^-22 of the summed magnitudes; bf16 values are summed as they are stored."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(1, 1), (1, 4096), (63, 7), (64, 8), (65, 33), (128, 256), (511, 1000), (513, 1184), (777, 37), (1025, 1001), (4096, 2048),
+          (70000, 3), (20000, 64)]
+
+
+def _bound(x):
+    return 2.0 ** -22 * 8 * x.double().abs().sum(0) + 1e-30
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,cols", SHAPES)
+def test_sums(rows, cols, dtype):
+    from ferrum_b200.ops import functional as F
+
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    for off in (0, 1):  # behind a 16-byte boundary: one by one
+        x = torch.randn(rows * cols + 1, device="cuda", generator=g).to(dtype)[off:][:rows * cols].view(rows, cols)
+        out = torch.full((cols,), float("nan"), device="cuda")
+        F.raw_colsum(x, out)
+        assert ((out - x.double().sum(0)).abs() <= _bound(x)).all()
+        F.raw_colsum(x, out, accumulate=True)
+        assert ((out - 2 * x.double().sum(0)).abs() <= 3 * _bound(x)).all()
+        assert torch.equal(F.raw_colsum(x), F.raw_colsum(x)) or rows * cols >= 1 << 20
+
+
+@pytest.mark.parametrize("act", [1, 4, 5])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,cols", SHAPES[:-2])
+def test_behind_an_activation(rows, cols, dtype, act):
+    from ferrum_b200 import _lib
+    from ferrum_b200.ops import functional as F
+
+    lib, st = _lib.cuda(), torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    dt = F._dt(torch.empty(0, dtype=dtype))
+    for off in (0, 1):
+        dy, y, d, want = (torch.randn(rows * cols + 1, device="cuda", generator=g).to(dtype)[off:][:rows * cols].view(rows, cols)
+                          for _ in range(4))
+        sums = torch.full((cols,), float("nan"), device="cuda")
+        _lib.check(lib.fb_unary_bwd(dy.data_ptr(), y.data_ptr(), want.data_ptr(), rows * cols, act, 0.0, 0.0, dt, st), "two")
+        rc = lib.fb_unary_bwd_colsum(dy.data_ptr(), y.data_ptr(), d.data_ptr(), sums.data_ptr(), rows, cols, act, dt, st)
+        assert rc == 0 and torch.equal(d, want)
+        assert ((sums - d.double().sum(0)).abs() <= _bound(d)).all()
+    assert lib.fb_unary_bwd_colsum(dy.data_ptr(), y.data_ptr(), d.data_ptr(), sums.data_ptr(), rows, cols, 3, dt, st) == -1
+    assert lib.fb_unary_bwd_colsum(dy.data_ptr(), y.data_ptr(), d.data_ptr(), sums.data_ptr(), 10 ** 7, 3, act, dt, st) == -3
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 1001), (40, 96), (300, 1024), (777, 1001), (2049, 4096), (5, 9000)])
+def test_layernorm_statistics_are_written_or_added(rows, cols, dtype):
+    from ferrum_b200 import _lib
+    from ferrum_b200.ops import functional as F
+    from ferrum_b200.utils.runtime import check_status
+
+    lib, st = _lib.cuda(), torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x, dy = (torch.randn(rows, cols, device="cuda", generator=g).to(dtype) for _ in range(2))
+    gamma = torch.ones(cols, device="cuda")
+    mean, rstd = x.float().mean(1), (x.float().var(1, unbiased=False) + 1e-5).rsqrt()
+    dx, nblk = torch.empty_like(x), lib.fb_layernorm_bwd_blocks(rows, cols)
+    partial = torch.empty(max(nblk, 1), 3, cols, device="cuda")
+    ones, nan = torch.ones(3, cols, device="cuda"), torch.full((3, cols), float("nan"), device="cuda")
+    for stats, flags in ((ones, 1), (nan, 3)):
+        _lib.check(lib.fb_layernorm_bwd(dy.data_ptr(), x.data_ptr(), None, gamma.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
+                                        dx.data_ptr(), partial.data_ptr(), stats.data_ptr(), rows, cols, 0,
+                                        F._dt(x), nblk, flags, st), "ln")
+    check_status()
+    xh = (x.double() - mean.double()[:, None]) * rstd.double()[:, None]
+    terms = torch.stack([dy.double() * xh, dy.double(), dx.double()])
+    size = terms.abs().sum(1)
+    # the column sum of dx is that of the values before they are rounded to the type
+    tol = 2.0 ** -18 * size + torch.tensor([0.0, 0.0, 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20], device="cuda")[:, None] * size
+    assert ((nan - terms.sum(1)).abs() <= tol + 1e-6).all() and ((ones - 1 - terms.sum(1)).abs() <= tol + 1e-5).all()
