@@ -17,6 +17,8 @@
 // MMA) are half as many: 33 instead of 44 cycles each.  A programmatic dependent is let in when the last MMA has been issued,
 // not before: its CTAs, though they only wait, slowed the issue here from 54 to 81 cycles per MMA (16 x 4096 x 4096 in a
 // row 15.6 us, 12.6 so, 12.2 with 64 rows; eight layers of 4096 with their normalisations at 16 rows 183 -> 157).
+// Then the producer set the pace, a copy of 2 or 4 KB for every operand of a k-block: where K is whole k-blocks, one copy
+// brings a stage of an operand (3-D maps): 12.2 -> 11.0, the eight layers 157 -> 147.
 //
 // 192 threads: warp 0 TMA producer, warp 1 MMA issue, warps 2 - 5 read the accumulator; all of them write the output.
 #include <cooperative_groups.h>
@@ -62,6 +64,7 @@ struct Args {
   int kb_total, kb_per_split, tiles_p;
   int stages, block_bytes, body_bytes, p_bytes;  // block: a k-block of both operands
   int mma_rows;  // 128, or 64 where P has no more
+  int boxes;     // kGroup k-blocks of an operand in one copy (3-D maps: 64 of K, rows, k-blocks), else a copy each
   int prefetch;  // bring this CTA's rows of B into L2 before the kernel ahead has completed
   int32_t* status;
   unsigned long long timeout_ns;
@@ -133,8 +136,13 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  if (p.prefetch && warp == 2 && ptx::elect_one())
-    for (int kb = kb_lo; kb < kb_hi; ++kb) ptx::tma_prefetch_2d(kSwap ? &map_p : &map_q, kb * kBK, kSwap ? p0 : q0);
+  if (p.prefetch && warp == 2 && ptx::elect_one()) {
+    if (p.boxes) {
+      for (int kb = kb_lo; kb < kb_hi; kb += kGroup) ptx::tma_prefetch_3d(kSwap ? &map_p : &map_q, 0, kSwap ? p0 : q0, kb);
+    } else {
+      for (int kb = kb_lo; kb < kb_hi; ++kb) ptx::tma_prefetch_2d(kSwap ? &map_p : &map_q, kb * kBK, kSwap ? p0 : q0);
+    }
+  }
   ptx::grid_wait();
 
   if (warp == 0) {
@@ -148,11 +156,17 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
           ok = false;
           break;
         }
-        const int blocks = min(kGroup, kb_hi - kb);
-        ptx::mbar_arrive_expect_tx(&full_bar[s], blocks * p.block_bytes);
+        uint8_t* stage = smem + s * kGroup * p.block_bytes;  // the k-blocks of P, then those of Q
+        if (p.boxes) {  // k-blocks behind the last one arrive as zeros
+          ptx::mbar_arrive_expect_tx(&full_bar[s], kGroup * p.block_bytes);
+          ptx::tma_load_3d(stage, &map_p, &full_bar[s], 0, p0, kb);
+          ptx::tma_load_3d(stage + kGroup * p.p_bytes, &map_q, &full_bar[s], 0, q0, kb);
+        }
+        const int blocks = p.boxes ? 0 : min(kGroup, kb_hi - kb);
+        if (blocks > 0) ptx::mbar_arrive_expect_tx(&full_bar[s], blocks * p.block_bytes);
         for (int i = 0; i < blocks; ++i) {
-          uint8_t* sp = smem + (s * kGroup + i) * p.block_bytes;
-          uint8_t* sq = sp + p.p_bytes;
+          uint8_t* sp = stage + i * p.p_bytes;
+          uint8_t* sq = stage + kGroup * p.p_bytes + i * (p.block_bytes - p.p_bytes);
           const int k0 = (kb + i) * kBK;
           if (p.p_mn) {
 #pragma unroll
@@ -188,7 +202,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
       const uint32_t p_lbo = p.p_mn ? kChunk : 16, q_lbo = p.q_mn ? kChunk : 16;
       const uint32_t p_step = p.p_mn ? 16 * 128 : 32, q_step = p.q_mn ? 16 * 128 : 32;
       const uint64_t p_first = ptx::make_smem_desc_sw128(ptx::smem_u32(smem), p_lbo, 1024);
-      const uint64_t q_first = ptx::make_smem_desc_sw128(ptx::smem_u32(smem) + p.p_bytes, q_lbo, 1024);
+      const uint64_t q_first = ptx::make_smem_desc_sw128(ptx::smem_u32(smem) + kGroup * p.p_bytes, q_lbo, 1024);
       int s = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -200,8 +214,9 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
         }
         ptx::tc_fence_after();
         const auto block = [&](int i) {
-          const int at = (s * kGroup + i) * p.block_bytes;
-          const uint64_t dp = ptx::desc_advance(p_first, at), dq = ptx::desc_advance(q_first, at);
+          const int at = s * kGroup * p.block_bytes;
+          const uint64_t dp = ptx::desc_advance(p_first, at + i * p.p_bytes);
+          const uint64_t dq = ptx::desc_advance(q_first, at + i * (p.block_bytes - p.p_bytes));
 #pragma unroll
           for (int k = 0; k < kBK / 16; ++k)
             ptx::umma_f16(tmem, ptx::desc_advance(dp, k * p_step), ptx::desc_advance(dq, k * q_step), idesc,
@@ -359,6 +374,18 @@ bool make_map(CUtensorMap* map, const void* ptr, int rows, int K, long long ld, 
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The same of a K-major operand whose K is whole k-blocks, `blocks` of them in a box.
+bool make_map_blocks(CUtensorMap* map, const void* ptr, int rows, int K, long long ld, int box_rows, int blocks) {
+  const EncodeFn enc = encoder();
+  if (enc == nullptr || (reinterpret_cast<uintptr_t>(ptr) & 15) != 0 || ld % 8 != 0) return false;
+  const cuuint64_t dims[3] = {64, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(K / 64)};
+  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld) * 2, 128};
+  const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(blocks)}, estr[3] = {1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 int sm_count() {
   static const int n = [] {
     int dev = 0, v = 0;
@@ -463,11 +490,17 @@ int run(bool split, const void* a, const void* b, void* out, void* out2, const f
   // Few rows of A on the 128-row side: only they are loaded (what else the MMA reads there goes into rows of the
   // accumulator that nobody stores).
   const int box_p = swap || a_mn_major || M > 64 ? kRowsP : M <= 16 ? 16 : M <= 32 ? 32 : 64;
+  // Stages of four k-blocks while 98 KB hold three of them (boxes of 16 rows of A).
+  const bool four = !split && !(swap ? a_mn_major : b_mn_major) && box_p <= 16;
+  const int group = tile == 160 ? (four ? 4 : 2) : tile == 192 && four ? 2 : 1;
   CUtensorMap ma, mb;
-  if (!make_map(&ma, a, M, K, lda, a_mn_major != 0, swap ? bn : box_p) ||
+  Args g;
+  g.boxes = group > 1 && !a_mn_major && !b_mn_major && K % kBK == 0;
+  if (g.boxes) {
+    if (!make_map_blocks(&ma, a, M, K, lda, box_p, group) || !make_map_blocks(&mb, b, N, K, ldb, bn, group)) return -2;
+  } else if (!make_map(&ma, a, M, K, lda, a_mn_major != 0, swap ? bn : box_p) ||
       !make_map(&mb, b, N, K, ldb, b_mn_major != 0, swap ? kRowsP : bn))
     return -2;
-  Args g;
   g.out = out;
   g.out2 = out2;
   g.bias = bias;
@@ -482,8 +515,6 @@ int run(bool split, const void* a, const void* b, void* out, void* out2, const f
   g.kb_total = (K + kBK - 1) / kBK;
   g.status = status;
   g.timeout_ns = 2000000000ull;
-  // Stages of four k-blocks while 98 KB hold three of them (boxes of 16 rows of A).
-  const bool four = !split && !g.q_mn && box_p <= 16;
   switch (tile) {
     case 16: return launch<16, true, 1>(mb, ma, g, N, M, box_p, split, stream);
     case 32: return launch<32, true, 1>(mb, ma, g, N, M, box_p, split, stream);
