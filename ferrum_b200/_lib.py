@@ -127,6 +127,9 @@ _CUDA_SIGS = {
     "fb_conv_wgrad_splits": (I, [I] * 6),
     "fb_conv_wgrad": (I, [P, P, P] + [I] * 12 + [P, P]),
     "fb_conv_pack_input": (I, [P, P, P] + [I] * 12 + [LL, P]),
+    "fb_conv_pack_masked": (I, [P, P, P, I, I, I, I, LL, P]),
+    "fb_nhwc_to_nchw_masks": (I, [P, P, P, P, P, I, I, LL, LL, I, P]),
+    "fb_conv_igemm_epilogue": (I, [P] * 5 + [I] * 11 + [LL, I, I, I, P, P]),
     "fb_conv_pack_filters": (I, [P, P] + [I] * 10 + [P]),
     "fb_conv_fold_wgrad": (I, [P, P] + [I] * 10 + [P]),
     "fb_s2d_nhwc_to_nchw_f32": (I, [P, P] + [I] * 12 + [LL, P]),

@@ -14,6 +14,7 @@
 //   fb_conv_fold_wgrad    the splits of fb_conv_wgrad -> their sum as [O, C, kh, kw]
 //   fb_s2d_nhwc_to_nchw_f32  the data gradient of z -> that of x
 //   fb_nhwc_to_nchw_f32      a result [B, P, ld] -> [B, C, P], plus a residual, behind a ReLU
+//   fb_nhwc_to_nchw_masks, fb_conv_pack_masked  the same with the ReLU's mask as bytes: a quarter of what its result is
 //
 // All are bound by HBM if they do not spend too many instructions: a pixel a load and store they were bound by their issue
 // (ncu: 63 - 79 % of the slots, 23 - 39 % of the HBM rate), so rows of whole quads move four pixels at a time.  A residual
@@ -39,10 +40,17 @@ struct S2d {
 
 constexpr int kTileC = 64, kTileQ = 64;
 
+// Four values of a mask: floats, or bytes that say where.
+__device__ __forceinline__ float4 mask4(const float* m) { return __ldg(reinterpret_cast<const float4*>(m)); }
+__device__ __forceinline__ float4 mask4(const uint8_t* m) {
+  const uchar4 u = __ldg(reinterpret_cast<const uchar4*>(m));
+  return make_float4(u.x, u.y, u.z, u.w);
+}
+
 // kQuads: four pixels a load (rows of whole quads on 16-byte boundaries, no columns skipped).
-template <bool kVec, bool kQuads>
+template <bool kVec, bool kQuads, typename M>
 __global__ void __launch_bounds__(256)
-pack_input_kernel(const float* __restrict__ x, const float* __restrict__ mask, __nv_bfloat16* __restrict__ z, const S2d g,
+pack_input_kernel(const float* __restrict__ x, const M* __restrict__ mask, __nv_bfloat16* __restrict__ z, const S2d g,
                   int q_tiles) {
   __shared__ uint32_t tile[kTileC / 2][kTileQ + 1];
   const int q0 = static_cast<int>(blockIdx.x % q_tiles) * kTileQ;
@@ -76,7 +84,7 @@ pack_input_kernel(const float* __restrict__ x, const float* __restrict__ mask, _
           for (int e = 0; e < 2; ++e) {
             const int c = (pair0 + 16 * k) * 2 + e;
             m[k][e] = make_float4(1.f, 1.f, 1.f, 1.f);
-            if (in && c < nc) m[k][e] = __ldg(reinterpret_cast<const float4*>(mask + base + c * plane + j));
+            if (in && c < nc) m[k][e] = mask4(mask + base + c * plane + j);
           }
 #pragma unroll
         for (int k = 0; k < 2; ++k)
@@ -126,7 +134,7 @@ pack_input_kernel(const float* __restrict__ x, const float* __restrict__ mask, _
           const int c = (warp + 8 * k) * 2;
 #pragma unroll
           for (int e = 0; e < 2; ++e)
-            if (in && c + e < nc && !(__ldg(mask + base + (c + e) * plane + j) > 0.f)) v[e][k] = 0.f;
+            if (in && c + e < nc && !(static_cast<float>(__ldg(mask + base + (c + e) * plane + j)) > 0.f)) v[e][k] = 0.f;
         }
       }
 #pragma unroll
@@ -241,7 +249,8 @@ s2d_to_nchw_kernel(const float* __restrict__ z, float* __restrict__ x, const S2d
 // cost their reads beside the transposition, no pass of their own.
 __global__ void __launch_bounds__(256)
 nhwc_to_nchw_f32_kernel(const float* __restrict__ x, const float* __restrict__ add, float* __restrict__ y, int C, long long P,
-                        long long ld, int relu, int p_tiles, bool quads) {
+                        long long ld, int relu, int p_tiles, bool quads, const uint8_t* __restrict__ add_mask,
+                        uint8_t* __restrict__ mask) {
   __shared__ float tile[64][65];
   const long long b = blockIdx.x / p_tiles, p0 = static_cast<long long>(blockIdx.x % p_tiles) * 64;
   const int c0 = blockIdx.y * 64;
@@ -281,6 +290,10 @@ nhwc_to_nchw_f32_kernel(const float* __restrict__ x, const float* __restrict__ a
       const int c = cq + 16 * k;
       r[k] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (add != nullptr && c0 + c < C) r[k] = __ldg(reinterpret_cast<const float4*>(add + at + c * P));
+      if (add_mask != nullptr && c0 + c < C) {
+        const uchar4 u = __ldg(reinterpret_cast<const uchar4*>(add_mask + at + c * P));
+        r[k] = make_float4(u.x ? r[k].x : 0.f, u.y ? r[k].y : 0.f, u.z ? r[k].z : 0.f, u.w ? r[k].w : 0.f);
+      }
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -290,6 +303,8 @@ nhwc_to_nchw_f32_kernel(const float* __restrict__ x, const float* __restrict__ a
       if (add != nullptr) v = make_float4(v.x + r[k].x, v.y + r[k].y, v.z + r[k].z, v.w + r[k].w);
       if (relu) v = make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
       *reinterpret_cast<float4*>(y + at + c * P) = v;
+      if (mask != nullptr)
+        *reinterpret_cast<uchar4*>(mask + at + c * P) = make_uchar4(v.x > 0.f, v.y > 0.f, v.z > 0.f, v.w > 0.f);
     }
     return;
   }
@@ -304,6 +319,7 @@ nhwc_to_nchw_f32_kernel(const float* __restrict__ x, const float* __restrict__ a
     for (int k = 0; k < 8; ++k) {
       const int c = cr + 4 * (h * 8 + k);
       r[k] = add != nullptr && c0 + c < C ? __ldg(add + at + c * P) : 0.f;
+      if (add_mask != nullptr && c0 + c < C && !__ldg(add_mask + at + c * P)) r[k] = 0.f;
     }
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
@@ -313,6 +329,7 @@ nhwc_to_nchw_f32_kernel(const float* __restrict__ x, const float* __restrict__ a
       if (add != nullptr) v += r[k];
       if (relu) v = fmaxf(v, 0.f);
       y[at + c * P] = v;
+      if (mask != nullptr) mask[at + c * P] = v > 0.f;
     }
   }
 }
@@ -349,8 +366,10 @@ int for_each_tap(K32 k32, K64 k64, long long total, cudaStream_t stream, A... ar
 
 // x [B, C, H, W] fp32 -> z [B, Hz, Wz, ld] bf16, every element of it written.  mask (optional): x is the gradient behind
 // a ReLU whose result was mask.
-extern "C" int fb_conv_pack_input(const float* x, const float* mask, void* z, int B, int C, int H, int W, int sh, int sw,
-                                  int eh, int ew, int ph, int pw, int Hz, int Wz, long long ld, cudaStream_t stream) {
+namespace {
+template <typename M>
+int pack_input(const float* x, const M* mask, void* z, int B, int C, int H, int W, int sh, int sw, int eh, int ew, int ph, int pw,
+               int Hz, int Wz, long long ld, cudaStream_t stream) {
   fb::S2d g{C, H, W, sh, sw, eh, ew, ph, pw, Hz, Wz, ld};
   const bool plain = sh == 1 && sw == 1 && ph == 0 && pw == 0 && Hz == H && Wz == W;  // images and rows of any size
   if (!fb::s2d_ok(B, g) || (!plain && !fb::s2d_grid_ok(B, g))) return -1;
@@ -367,11 +386,22 @@ extern "C" int fb_conv_pack_input(const float* x, const float* mask, void* z, in
   const bool vec = ld == static_cast<long long>(eh) * ew * ((C + 7) / 8 * 8) && (C % 8 == 0 || eh * ew == 1) &&
                    reinterpret_cast<uintptr_t>(z) % 16 == 0;
   const bool quads = ew == sw && g.W % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 &&
-                     reinterpret_cast<uintptr_t>(mask) % 16 == 0;
-  const auto kernel = vec ? (quads ? fb::pack_input_kernel<true, true> : fb::pack_input_kernel<true, false>)
-                          : (quads ? fb::pack_input_kernel<false, true> : fb::pack_input_kernel<false, false>);
+                     reinterpret_cast<uintptr_t>(mask) % (4 * sizeof(M)) == 0;
+  const auto kernel = vec ? (quads ? fb::pack_input_kernel<true, true, M> : fb::pack_input_kernel<true, false, M>)
+                          : (quads ? fb::pack_input_kernel<false, true, M> : fb::pack_input_kernel<false, false, M>);
   kernel<<<grid, 256, 0, stream>>>(x, mask, static_cast<__nv_bfloat16*>(z), g, static_cast<int>(q_tiles));
   return static_cast<int>(cudaGetLastError());
+}
+}  // namespace
+
+extern "C" int fb_conv_pack_input(const float* x, const float* mask, void* z, int B, int C, int H, int W, int sh, int sw,
+                                  int eh, int ew, int ph, int pw, int Hz, int Wz, long long ld, cudaStream_t stream) {
+  return pack_input(x, mask, z, B, C, H, W, sh, sw, eh, ew, ph, pw, Hz, Wz, ld, stream);
+}
+// The mask as bytes (fb_nhwc_to_nchw_masks); stride 1, no padding.
+extern "C" int fb_conv_pack_masked(const float* x, const unsigned char* mask, void* z, int B, int C, int H, int W, long long ld,
+                                   cudaStream_t stream) {
+  return pack_input<uint8_t>(x, mask, z, B, C, H, W, 1, 1, 1, 1, 0, 0, H, W, ld, stream);
 }
 
 // dgrad = 0: out [O, k2h * k2w, pitch], dgrad = 1: out [eh * ew * C, k2h * k2w, pitch] with the taps in reverse order.
@@ -411,12 +441,19 @@ extern "C" int fb_s2d_nhwc_to_nchw_f32(const float* z, float* x, int B, int C, i
 }
 
 // y [B, C, P] = x [B, P, ld] (first C channels), plus add [B, C, P] (optional), behind a ReLU with relu = 1.
-extern "C" int fb_nhwc_to_nchw_f32(const float* x, const float* add, float* y, int B, int C, long long P, long long ld,
-                                   int relu, cudaStream_t stream) {
+// add_mask (optional, bytes laid out like add): add counts where it is set; mask (optional): set where y is above zero.
+extern "C" int fb_nhwc_to_nchw_masks(const float* x, const float* add, const unsigned char* add_mask, float* y,
+                                     unsigned char* mask, int B, int C, long long P, long long ld, int relu, cudaStream_t stream) {
   const long long tiles = (P + 63) / 64;
   if (B <= 0 || C <= 0 || P <= 0 || ld < C || tiles * B > 0x7fffffffll || (C + 63) / 64 > 65535) return -1;
   const dim3 grid(static_cast<unsigned>(tiles * B), static_cast<unsigned>((C + 63) / 64));
-  const bool quads = P % 4 == 0 && reinterpret_cast<uintptr_t>(add) % 16 == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0;
-  fb::nhwc_to_nchw_f32_kernel<<<grid, 256, 0, stream>>>(x, add, y, C, P, ld, relu, static_cast<int>(tiles), quads);
+  const bool quads = P % 4 == 0 && reinterpret_cast<uintptr_t>(add) % 16 == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0 &&
+                     reinterpret_cast<uintptr_t>(add_mask) % 4 == 0 && reinterpret_cast<uintptr_t>(mask) % 4 == 0;
+  fb::nhwc_to_nchw_f32_kernel<<<grid, 256, 0, stream>>>(x, add, y, C, P, ld, relu, static_cast<int>(tiles), quads,
+                                                       add_mask, mask);
   return static_cast<int>(cudaGetLastError());
+}
+extern "C" int fb_nhwc_to_nchw_f32(const float* x, const float* add, float* y, int B, int C, long long P, long long ld,
+                                   int relu, cudaStream_t stream) {
+  return fb_nhwc_to_nchw_masks(x, add, nullptr, y, nullptr, B, C, P, ld, relu, stream);
 }

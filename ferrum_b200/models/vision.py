@@ -7,7 +7,7 @@ from __future__ import annotations
 import torch
 
 from .. import nn
-from ..nn.conv import AdaptiveAvgPool2d, Conv2d, MaxPool2d, bare, conv_fused
+from ..nn.conv import AdaptiveAvgPool2d, Conv2d, MaxPool2d, bare, block_fused, conv_fused
 from ..ops import functional as F
 
 
@@ -25,6 +25,9 @@ class BasicBlock(nn.Module):
 
     @nn.tensor_io
     def forward(self, x):
+        y = block_fused(self.conv1, self.conv2, self.downsample, x)
+        if y is not None:
+            return y
         identity = self.downsample(x) if self.downsample is not None else x
         # the fused node reads its result in the backward pass: not where a hook of conv2 may write to it
         y = conv_fused(self.conv1, x, act="relu") if bare(self.conv2) else F.unary(self.conv1(x), "relu")

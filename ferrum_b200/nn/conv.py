@@ -119,6 +119,32 @@ def conv_fused(conv, x, add=None, act=None):
     return y if act is None else F.unary(y, act)
 
 
+def block_fused(conv1, conv2, down, x):
+    """``relu(conv2(relu(conv1(x))) + (down(x) or x))`` as one node where all of it runs as implicit GEMMs, else None."""
+    convs = [conv1, conv2] + ([down] if down is not None else [])
+    if not (all(bare(c) and c.bias is None and c.groups == 1 for c in convs) and x.dim() == 4 and x.dtype == torch.float32):
+        return None
+    w1, w2 = conv1.weight, conv2.weight
+    if not (x.shape[1] == w1.shape[1] and w1.shape[0] == w2.shape[1] and w1.shape[0] % 8 == 0
+            and tuple(conv2._stride) == (1, 1)):
+        return None
+    geometry = [(c._stride, c._padding, c.dilation) for c in convs]
+    for c in convs:  # the second one's operand is of x's kind
+        if not F.conv_igemm_ok(x, c._stride, c.dilation, c._padding, c.kernel_size, 1):
+            return None
+    mid = _out_hw(x, conv1.kernel_size, conv1._stride, conv1._padding, conv1.dilation)
+    out = tuple(F.conv_out_size(n, *(v[i] for v in (conv2.kernel_size, conv2._stride, conv2._padding, conv2.dilation)))
+                for i, n in enumerate(mid))
+    if down is None:
+        same = tuple(conv1._stride) == (1, 1) and (w2.shape[0],) + out == tuple(x.shape[1:])
+    else:
+        same = (down.weight.shape[1] == x.shape[1] and down.weight.shape[0] == w2.shape[0]
+                and tuple(_out_hw(x, down.kernel_size, down._stride, down._padding, down.dilation)) == out)
+    if not same or min(out) <= 0 or any(c.weight.device != x.device for c in convs):
+        return None
+    return F.conv_block(x, w1, w2, down.weight if down is not None else None, geometry)
+
+
 class Conv1d(Module):
     def __init__(self, in_channels, out_channels, kernel_size, stride=1, padding=0, dilation=1, groups=1,
                  bias=True, device=None):

@@ -1088,6 +1088,12 @@ def conv2d_igemm(x, weight, bias, padding=(0, 0), dilation=(1, 1), stride=(1, 1)
     return _lib.native().conv2d(x, weight, bias, add, stride, padding, dilation, _gemm.ACT[act])
 
 
+def conv_block(x, w1, w2, down, geometry):
+    """A residual block as one node (csrc/native/conv.cpp); ``geometry``: (stride, padding, dilation) of each convolution."""
+    g = [[list(v) for v in three] for three in geometry]
+    return _lib.native().conv_block(x, w1, w2, down, g[0], g[1], g[2] if down is not None else [])
+
+
 def im2col(x, kernel, stride=(1, 1), padding=(0, 0), dilation=(1, 1)):
     """Window matrix of a convolution with rows ordered (b, oh, ow) and columns (c, ki, kj)."""
     if _native(x):
