@@ -26,7 +26,6 @@
 #include "../common/ptx.cuh"
 #include "../common/status.h"
 #include "../include/ferrum_kernels.h"
-#include "column_sums.cuh"
 
 namespace fb {
 namespace {
@@ -130,6 +129,37 @@ __device__ __forceinline__ float row_sum(float v, float (*smem)[8]) {
   return t;
 }
 
+// A thread's columns of gamma and beta: kept over the rows where they are eight (registers), else read for each.
+template <bool kKeep>
+struct Affine {
+  float g[kKeep ? 8 : 1], b[kKeep ? 8 : 1];
+  __device__ Affine(const float* gamma, const float* beta, int at) {
+    if constexpr (kKeep) {
+      if (gamma && at >= 0) ld8f(gamma + at, g);
+      if (beta && at >= 0) ld8f(beta + at, b);
+    }
+  }
+  __device__ void get(const float* gamma, const float* beta, int at, float (&go)[8], float (&bo)[8]) const {
+    if constexpr (kKeep) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        go[i] = g[i];
+        bo[i] = b[i];
+      }
+    } else {
+      if (gamma) ld8f(gamma + at, go);
+      if (beta) ld8f(beta + at, bo);
+    }
+  }
+};
+
+// The column statistics that ln_fold_kernel adds to are cleared by the first block of the kernel ahead of it (NULL: they are
+// added to what is there): a launch and a gap of 3 us less than with a fill.
+__device__ __forceinline__ void clear_stats(float* stats, int cols) {
+  if (stats != nullptr && blockIdx.x == 0)
+    for (int i = threadIdx.x; i < 3 * cols; i += blockDim.x) stats[i] = 0.f;
+}
+
 // Forward.  A row lives in registers: TPR threads x K vectors of 8 elements.
 template <typename T, int TPR, int K>
 __global__ void __launch_bounds__(256)
@@ -144,6 +174,7 @@ ln_fwd_kernel(const T* __restrict__ x, const float* __restrict__ gamma, const fl
   const int nvec = cols >> 3;
   const float inv_n = 1.f / static_cast<float>(cols);
   const long long row_stride = static_cast<long long>(gridDim.x) * kRowsPerBlock;
+  const Affine<K == 1> par(gamma, beta, t < nvec ? t * 8 : -1);
   typename V8<T>::Raw raw[K], nxt[K];
   {
     const long long r0 = static_cast<long long>(blockIdx.x) * kRowsPerBlock + sub;
@@ -205,8 +236,7 @@ ln_fwd_kernel(const T* __restrict__ x, const float* __restrict__ gamma, const fl
       const int vi = t + k * TPR;
       if (live && vi < nvec) {
         float g[8], b[8], o[8];
-        if (gamma) ld8f(gamma + vi * 8, g);
-        if (beta) ld8f(beta + vi * 8, b);
+        par.get(gamma, beta, vi * 8, g, b);
 #pragma unroll
         for (int i = 0; i < 8; ++i)
           o[i] = (v[k][i] - mu) * rs * (gamma ? g[i] : 1.f) + (beta ? b[i] : 0.f);
@@ -233,6 +263,7 @@ ln_add_fwd_kernel(const float* __restrict__ x, const R* __restrict__ r, const fl
   const int nvec = cols >> 3;
   const float inv_n = 1.f / static_cast<float>(cols);
   const long long row_stride = static_cast<long long>(gridDim.x) * kRowsPerBlock;
+  const Affine<K == 1> par(gamma, beta, t < nvec ? t * 8 : -1);
   V8<float>::Raw raw[K], nxt[K];
   typename V8<R>::Raw res[K], res_nxt[K];
   {
@@ -304,8 +335,7 @@ ln_add_fwd_kernel(const float* __restrict__ x, const R* __restrict__ r, const fl
       const int vi = t + k * TPR;
       if (live && vi < nvec) {
         float g[8], b[8], o[8];
-        if (gamma) ld8f(gamma + vi * 8, g);
-        if (beta) ld8f(beta + vi * 8, b);
+        par.get(gamma, beta, vi * 8, g, b);
 #pragma unroll
         for (int i = 0; i < 8; ++i)
           o[i] = (v[k][i] - mu) * rs * (gamma ? g[i] : 1.f) + (beta ? b[i] : 0.f);
@@ -325,7 +355,10 @@ __device__ __forceinline__ void ld_pairs_f32(const float* p, float2 (&o)[4]);
 // Forward, one WARP per row (bf16, 1024..4096 columns): a lane keeps its K 16-byte vectors packed in registers,
 // all K loads are issued back to back (up to 8 KB in flight per warp), the statistics are one pass of shifted sums
 // (x - c with c = the row's first element) reduced by warp shuffles, and there is no block barrier at all: warps
-// stream rows independently.  Packed fp32x2 arithmetic; gamma / beta come through L1.
+// stream rows independently.  Packed fp32x2 arithmetic.  gamma and beta lie in shared memory, quads of columns side by
+// side (the even ones of a parameter, then the odd ones), so that a warp's 16-byte reads are free of bank conflicts: read
+// through L1 for each row, beside the rows that stream past, they were a third of the time.  8192 x 4096 36.1 -> 24.9 us (a copy
+// of the rows takes 22).
 // W > 1, few rows: a block per row.  Latency is all there is then, so W warps find the same statistics (the same sums in
 // the same order: the same bits) and each writes the vectors k % W of its number, whose gamma and beta it asks for
 // beforehand.
@@ -346,6 +379,15 @@ ln_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
   const long long nwarps = W > 1 ? gridDim.x : (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
   constexpr int kOwn = W > 1 ? K / W : 1;
   float2 own_g[kOwn][4], own_b[kOwn][4];
+  extern __shared__ float4 affine[];  // W == 1: gamma's even quads, odd quads, beta's even quads, odd quads
+  if constexpr (W == 1) {
+    for (int i = threadIdx.x; i < 2 * nvec; i += 256) {
+      const int at = (i & 1) * nvec + (i >> 1);
+      affine[at] = gamma ? *reinterpret_cast<const float4*>(gamma + 4 * i) : make_float4(1.f, 1.f, 1.f, 1.f);
+      affine[2 * nvec + at] = beta ? *reinterpret_cast<const float4*>(beta + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+  }
   for (long long row = warp_id; row < rows; row += nwarps) {
     const __nv_bfloat16* xr = x + row * cols;
     uint4 raw[K];
@@ -401,20 +443,18 @@ ln_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
       if (vi < nvec && (W == 1 || k % W == part)) {
         const uint32_t w[4] = {raw[k].x, raw[k].y, raw[k].z, raw[k].w};
         float2 g[4], b[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          g[e] = make_float2(1.f, 1.f);
-          b[e] = make_float2(0.f, 0.f);
-        }
         if constexpr (W > 1) {
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            if (gamma) g[e] = own_g[k / W][e];
-            if (beta) b[e] = own_b[k / W][e];
+            g[e] = gamma ? own_g[k / W][e] : make_float2(1.f, 1.f);
+            b[e] = beta ? own_b[k / W][e] : make_float2(0.f, 0.f);
           }
         } else {
-          if (gamma) ld_pairs_f32(gamma + vi * 8, g);
-          if (beta) ld_pairs_f32(beta + vi * 8, b);
+          const float4 g0 = affine[vi], g1 = affine[nvec + vi], b0 = affine[2 * nvec + vi], b1 = affine[3 * nvec + vi];
+          g[0] = make_float2(g0.x, g0.y); g[1] = make_float2(g0.z, g0.w);
+          g[2] = make_float2(g1.x, g1.y); g[3] = make_float2(g1.z, g1.w);
+          b[0] = make_float2(b0.x, b0.y); b[1] = make_float2(b0.z, b0.w);
+          b[2] = make_float2(b1.x, b1.y); b[3] = make_float2(b1.z, b1.w);
         }
         uint4 out;
         uint32_t* ow = reinterpret_cast<uint32_t*>(&out);
@@ -449,7 +489,8 @@ __global__ void __launch_bounds__(256, K == 1 ? 3 : 2)
 ln_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ act_grad,
               const float* __restrict__ gamma, const float* __restrict__ mean, const float* __restrict__ rstd,
               T* __restrict__ dx, __nv_bfloat16* __restrict__ dx_low, float* __restrict__ partial, long long rows,
-              int cols, int pre_act, int want_colsum) {
+              int cols, int pre_act, int want_colsum, float* __restrict__ clear) {
+  clear_stats(clear, cols);
   __shared__ float smem[8][8];
   constexpr int kRowsPerBlock = 256 / TPR;
   constexpr bool kFast = V8<T>::kFastMath;
@@ -822,7 +863,8 @@ ln_bwd_ring_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
                    const __nv_bfloat16* __restrict__ act_grad, const float* __restrict__ gamma,
                    const float* __restrict__ mean, const float* __restrict__ rstd, __nv_bfloat16* __restrict__ dx,
                    float* __restrict__ partial, long long rows, int cols, int want_colsum, int stages,
-                   int32_t* status) {
+                   int32_t* status, float* __restrict__ clear) {
+  clear_stats(clear, cols);
   using V = V8<__nv_bfloat16>;
   extern __shared__ __align__(128) uint8_t ring[];
   __shared__ RingCtl ctl;
@@ -955,14 +997,15 @@ ln_bwd_ring_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   }
 }
 
-// Fold partial[nblk][3*cols] into stats[3*cols] (written or added to): block = 128 columns x a chunk of the
-// nblk rows, lanes own 4 adjacent columns, partials leave with one atomicAdd per column per block.  kVec: 16-byte loads
+// Fold partial[nblk][3*cols] into stats[3*cols] (accumulated into): block = 128 columns x a chunk of the
+// nblk rows, lanes own 4 adjacent columns, partials leave with one atomicAdd per column per block.  (Without
+// atomics, a cluster or a block to a column range, it took 4.5 to 5.5 us for 1024 columns instead of 2.9: too few blocks.)  kVec: 16-byte loads
 // (ncols a multiple of 4, partial on a 16-byte address).
 template <bool kVec>
 __global__ void __launch_bounds__(256)
 ln_fold_kernel(const float* __restrict__ partial, float* __restrict__ stats, int nblk, int ncols,
-               int rows_per_block, int add) {
-  __shared__ float sm[8][128], part[128];
+               int rows_per_block) {
+  __shared__ float sm[8][128];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c0 = blockIdx.x * 128 + lane * 4;
   const int r_lo = blockIdx.y * rows_per_block;
@@ -991,12 +1034,9 @@ ln_fold_kernel(const float* __restrict__ partial, float* __restrict__ stats, int
     float s = 0.f;
 #pragma unroll
     for (int w = 0; w < 8; ++w) s += sm[w][threadIdx.x];
-    part[threadIdx.x] = s;
+    const int c = blockIdx.x * 128 + threadIdx.x;
+    if (c < ncols) atomicAdd(stats + c, s);
   }
-  cluster_sums(part, 128, [&](int i, float s) {
-    const int c = static_cast<int>(blockIdx.x) * 128 + i;
-    if (c < ncols) stats[c] = add ? stats[c] + s : s;
-  });
 }
 
 // ---------------------------------------------------------------- rows of any width and alignment in registers
@@ -1055,7 +1095,8 @@ __global__ void __launch_bounds__(256)
 ln_bwd_any_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ act_grad,
                   const float* __restrict__ gamma, const float* __restrict__ mean, const float* __restrict__ rstd,
                   T* __restrict__ dx, float* __restrict__ partial, long long rows, int cols, int pre_act,
-                  int want_colsum) {
+                  int want_colsum, float* __restrict__ clear) {
+  clear_stats(clear, cols);
   __shared__ float smem[8][8];
   constexpr int kRows = 256 / TPR;
   const int sub = threadIdx.x / TPR, t = threadIdx.x % TPR;
@@ -1333,12 +1374,13 @@ bool launch_fwd_warp<__nv_bfloat16>(const __nv_bfloat16* xp, const float* gamma,
   const long long want = (rows + 7) / 8;  // eight warps per block
   const long long cap = static_cast<long long>(sm_count()) * 2;
   const int grid = static_cast<int>(want < cap ? want : cap);
+  const size_t smem = static_cast<size_t>(cols) * 8;  // gamma and beta
   if (k <= 4)
-    ln_fwd_warp_kernel<4><<<grid, 256, 0, st>>>(xp, gamma, beta, yp, mean, rstd, rows, cols, eps);
+    ln_fwd_warp_kernel<4><<<grid, 256, smem, st>>>(xp, gamma, beta, yp, mean, rstd, rows, cols, eps);
   else if (k <= 8)
-    ln_fwd_warp_kernel<8><<<grid, 256, 0, st>>>(xp, gamma, beta, yp, mean, rstd, rows, cols, eps);
+    ln_fwd_warp_kernel<8><<<grid, 256, smem, st>>>(xp, gamma, beta, yp, mean, rstd, rows, cols, eps);
   else
-    ln_fwd_warp_kernel<16><<<grid, 256, 0, st>>>(xp, gamma, beta, yp, mean, rstd, rows, cols, eps);
+    ln_fwd_warp_kernel<16><<<grid, 256, smem, st>>>(xp, gamma, beta, yp, mean, rstd, rows, cols, eps);
   return true;
 }
 
@@ -1428,14 +1470,14 @@ int add_fwd_t(const float* x, const R* r, const float* gamma, const float* beta,
 
 template <typename T>
 bool launch_wide(const T*, const T*, const T*, const float*, const float*, const float*, T*, float*, long long, int,
-                 int, int, cudaStream_t) {
+                 int, int, float*, cudaStream_t) {
   return false;
 }
 // bf16 rows of 2 KB .. 8 KB with no activation to re-evaluate: the ring kernel, one block per SM.
 template <>
 bool launch_wide<__nv_bfloat16>(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* ag,
                                 const float* gamma, const float* mean, const float* rstd, __nv_bfloat16* dx,
-                                float* partial, long long rows, int cols, int blocks, int want_colsum,
+                                float* partial, long long rows, int cols, int blocks, int want_colsum, float* clear,
                                 cudaStream_t st) {
   const int stages = ring_stages(static_cast<size_t>(cols) * 2 * (ag != nullptr ? 3 : 2), 200u * 1024u);
   if (stages < 2) return false;
@@ -1450,7 +1492,7 @@ bool launch_wide<__nv_bfloat16>(const __nv_bfloat16* dy, const __nv_bfloat16* x,
     configured = smem;
   }
   ln_bwd_ring_kernel<<<blocks, kRingThreads, smem, st>>>(dy, x, ag, gamma, mean, rstd, dx, partial, rows, cols,
-                                                         want_colsum, stages, g_ln_status);
+                                                         want_colsum, stages, g_ln_status, clear);
   return true;
 }
 
@@ -1458,7 +1500,8 @@ template <typename T>
 int bwd_t(const void* dy, const void* x, const void* act_grad, const float* gamma, const float* mean,
           const float* rstd, void* dx, __nv_bfloat16* dx_low, float* partial, float* stats, long long rows, int cols,
           int pre_act, int nblk, int flags, cudaStream_t st) {
-  const int want_colsum = flags & 1, add = (flags & 2) == 0;
+  const int want_colsum = flags & 1;
+  float* clear = (flags & 2) != 0 ? stats : nullptr;
   const T* dyp = static_cast<const T*>(dy);
   const T* xp = static_cast<const T*>(x);
   const T* agp = static_cast<const T*>(act_grad);
@@ -1474,18 +1517,18 @@ int bwd_t(const void* dy, const void* x, const void* act_grad, const float* gamm
     const int wide_blocks = nblk / 2 < sm_count() ? nblk / 2 : sm_count();  // two rows of partial[] per block
     if (fast && dx_low == nullptr && ring_enabled() && pre_act == FB_ACT_NONE && cols * 2 >= 2048 && nvec <= 2 * kGroupThreads &&
         wide_blocks >= 1 &&
-        launch_wide<T>(dyp, xp, agp, gamma, mean, rstd, dxp, partial, rows, cols, wide_blocks, want_colsum, st)) {
+        launch_wide<T>(dyp, xp, agp, gamma, mean, rstd, dxp, partial, rows, cols, wide_blocks, want_colsum, clear, st)) {
       used = 2 * wide_blocks;
     } else if (!fast) {
 #define FB_LN_BWD(TPR, K) \
   ln_bwd_any_kernel<T, TPR, K><<<nblk, 256, 0, st>>>(dyp, xp, agp, gamma, mean, rstd, dxp, partial, rows, cols, pre_act, \
-                                                     want_colsum)
+                                                     want_colsum, clear)
       FB_LN_ANY(any, FB_LN_BWD, if constexpr (sizeof(T) == 4) FB_LN_BWD(256, 16));
 #undef FB_LN_BWD
     } else {
       const auto run = [&](auto plain, auto low) {
         (dx_low != nullptr ? low : plain)<<<nblk, 256, 0, st>>>(dyp, xp, agp, gamma, mean, rstd, dxp, dx_low, partial, rows,
-                                                                cols, pre_act, want_colsum);
+                                                                cols, pre_act, want_colsum, clear);
       };
 #define FB_LN_BWD(TPR, K) run(ln_bwd_kernel<T, TPR, K, K == 4>, ln_bwd_kernel<T, TPR, K, K == 4 || sizeof(T) == 4>)
     if (g.tpr == 32 && g.k == 1) FB_LN_BWD(32, 1);
@@ -1498,14 +1541,15 @@ int bwd_t(const void* dy, const void* x, const void* act_grad, const float* gamm
     }
     const int ncols = 3 * cols;
     const int col_blocks = (ncols + 127) / 128;
-    int row_blocks = 1;  // one cluster to a column block
-    while (row_blocks < 8 && row_blocks * col_blocks < sm_count() * 2 && row_blocks * 16 < used) row_blocks *= 2;
+    int row_blocks = (sm_count() * 2 + col_blocks - 1) / col_blocks;
+    const int max_rb = (used + 15) / 16;
+    if (row_blocks > max_rb) row_blocks = max_rb;
+    if (row_blocks < 1) row_blocks = 1;
     const int rpb = (used + row_blocks - 1) / row_blocks;
     const auto fold = ncols % 4 == 0 && aligned16(partial, nullptr, nullptr, nullptr) ? ln_fold_kernel<true> : ln_fold_kernel<false>;
-    return launch_column_cluster(fold, dim3(col_blocks, row_blocks), st, static_cast<const float*>(partial), stats, used, ncols,
-                                 rpb, add);
+    fold<<<dim3(col_blocks, row_blocks), 256, 0, st>>>(partial, stats, used, ncols, rpb);
   } else {
-    if (!add) {
+    if (clear != nullptr) {
       const cudaError_t e = cudaMemsetAsync(stats, 0, 3 * static_cast<size_t>(cols) * sizeof(float), st);
       if (e != cudaSuccess) return static_cast<int>(e);
     }
