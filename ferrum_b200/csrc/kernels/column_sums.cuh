@@ -1,8 +1,8 @@
 // Column sums of a matrix whose rows are divided among the blocks of a cluster (along y): every block's sums meet in the
 // first one through distributed shared memory, in the order of the blocks.  No atomics, so no result to clear first (a launch
-// and a gap of 3 us on the device, as much on the host where that is what bounds a step).  With the fill and its gap / so: 8192 x
-// 1024 bf16 9 / 7.6 us; ReLU gradient and column sums of 8192 x 4096 bf16 44 as three launches, 35.7 as one; a training step
-// of the 784-256-10 classifier 220 / 215.
+// and a gap of 3 us on the device, as much on the host where that is what bounds a step).  With a fill and atomics / so, us:
+// 128 x 256 bf16 5.9 / 3.0, 1024 x 1000 6.3 / 3.7, 8192 x 1000 10.3 / 7.8, 8192 x 1024 fp32 14.4 / 8.2; ReLU gradient and column
+// sums of 8192 x 4096 bf16 44 as three launches, 36 as one.
 #pragma once
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
@@ -51,12 +51,14 @@ inline int column_sms() {
   return n;
 }
 
+constexpr int kColumnThreads = 512;
+
 // A launch with clusters of grid.y blocks (at most 8).
 template <class... P, class... A>
 int launch_column_cluster(void (*kernel)(P...), dim3 grid, cudaStream_t stream, A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
-  cfg.blockDim = dim3(256);
+  cfg.blockDim = dim3(kColumnThreads);
   cfg.stream = stream;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -94,13 +96,14 @@ struct PlainRows {
   __device__ float one(long long at) const { return static_cast<float>(x[at]); }
 };
 
-// A block sums L lanes x 16 bytes of columns over its rows, 256 / L of them at a time with Rows::kU loads each in flight.
+// A block sums L lanes x 16 bytes of columns over its rows, 512 / L of them at a time with Rows::kU loads each in flight: there
+// are hardly more blocks than SMs, so a block keeps 64 KB on their way (with 32 KB, 256 threads: 8192 x 1000 bf16 10.5 us).
 template <class Rows, int L>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kColumnThreads)
 colsum_cluster_kernel(const Rows m, float* __restrict__ out, long long rows, long long cols, long long rows_per_block,
                       int accumulate) {
-  constexpr int kV = Rows::kV, kU = Rows::kU, kR = 256 / L, kCols = L * kV;
-  __shared__ float warps[8][kCols], part[kCols];
+  constexpr int kV = Rows::kV, kU = Rows::kU, kR = kColumnThreads / L, kCols = L * kV;
+  __shared__ float warps[kColumnThreads / 32][kCols], part[kCols];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l = threadIdx.x % L;
   const long long c0 = static_cast<long long>(blockIdx.x) * kCols + l * kV;
   const long long r_lo = static_cast<long long>(blockIdx.y) * rows_per_block, r_hi = min(rows, r_lo + rows_per_block);
@@ -139,10 +142,11 @@ colsum_cluster_kernel(const Rows m, float* __restrict__ out, long long rows, lon
     for (int i = 0; i < kV; ++i) warps[warp][l * kV + i] = acc[i];
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < kCols; t += 256) {
+  if (threadIdx.x < kCols) {
+    const int t = threadIdx.x;
     float s = 0.f;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) s += warps[w][t];
+    for (int w = 0; w < kColumnThreads / 32; ++w) s += warps[w][t];
     part[t] = s;
   }
   cluster_sums(part, kCols, [&](int i, float s) {
@@ -159,14 +163,16 @@ bool column_cluster_fits(long long rows, long long cols) {
 }
 template <class Rows>
 int launch_colsum(const Rows& m, float* out, long long rows, long long cols, int accumulate, cudaStream_t stream) {
-  // 128 bytes of a row to a block, or 64 or 32 where that would leave a third of the chip without one: 8192 x 1024 bf16 9.7 us
-  // with 32 bytes, 6.4 with 128 (memory is read by lines).
+  // 128 bytes of a row to a block, or 64 or 32 where that would leave a third of the chip without one (memory is read by
+  // lines: 8192 x 1024 bf16 9.7 us with 32 bytes, 7.6 with 128).
   int lanes = 8;
   while (lanes > 2 && (cols + lanes * Rows::kV - 1) / (lanes * Rows::kV) * 8 * 3 < column_sms() * 2) lanes /= 2;
   const long long per = lanes * Rows::kV;
+  // As many blocks to a range as give every SM one: with eight to each of 64 ranges they took turns (512 x 4096 bf16 7.5 us).
+  const long long ranges = (cols + per - 1) / per;
   int split = 1;
-  while (split < 8 && rows >= split * 64) split *= 2;
-  const dim3 grid(static_cast<unsigned>((cols + per - 1) / per), static_cast<unsigned>(split));
+  while (split < 8 && ranges * split < column_sms() && rows >= split * 64) split *= 2;
+  const dim3 grid(static_cast<unsigned>(ranges), static_cast<unsigned>(split));
   const long long rpb = (rows + split - 1) / split;
   const auto kernel = lanes == 8   ? colsum_cluster_kernel<Rows, 8>
                       : lanes == 4 ? colsum_cluster_kernel<Rows, 4>

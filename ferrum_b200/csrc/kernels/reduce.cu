@@ -430,7 +430,8 @@ extern "C" int fb_colsum(const void* x, float* out, long long rows, long long co
     return accumulate ? 0 : static_cast<int>(cudaMemsetAsync(out, 0, cols * sizeof(float), stream));
   if (dtype == FB_DT_F32 && fb::column_cluster_fits<float>(rows, cols))
     return fb::launch_colsum(fb::PlainRows<float>{static_cast<const float*>(x)}, out, rows, cols, accumulate, stream);
-  if (dtype == FB_DT_BF16 && fb::column_cluster_fits<__nv_bfloat16>(rows, cols))
+  // bf16 matrices past L2's half are read faster by more, smaller blocks: 16384 x 3072 22.1 us here, 20.6 with the fill.
+  if (dtype == FB_DT_BF16 && fb::column_cluster_fits<__nv_bfloat16>(rows, cols) && rows * cols <= (24LL << 20))
     return fb::launch_colsum(fb::PlainRows<__nv_bfloat16>{static_cast<const __nv_bfloat16*>(x)}, out, rows, cols, accumulate,
                              stream);
   if (!accumulate) {
