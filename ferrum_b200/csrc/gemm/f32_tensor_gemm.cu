@@ -41,6 +41,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cfloat>
 #include <cstdint>
 
@@ -695,6 +696,33 @@ int sm_count() {
   return n;
 }
 
+// Clusters of `size` CTAs that are on the chip at once: fewer than SMs / size, a cluster lies within one part of the chip.
+template <typename T, int BN>
+int resident_clusters(int size) {
+  static std::atomic<int> known[9];
+  int n = known[size].load(std::memory_order_relaxed);
+  if (n == 0) {
+    const auto kernel = gemm_split_kernel<T, BN, kVecK, kVecK>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(size));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = Cfg<T, BN>::kSmem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = size;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<T, BN>::kSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
+      cudaGetLastError();
+      n = sm_count() / size;
+    }
+    known[size].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
 template <typename T, int BN, int LA, int LB>
 int launch_one(const Args& args, int batch, int splits, cudaStream_t st) {
   constexpr int kSmem = Cfg<T, BN>::kSmem;
@@ -777,7 +805,8 @@ int gemm_split(const T* a, const T* b, void* out, int out_bf16, const float* bia
   g.status = status;
   g.timeout_ns = 2000000000ull;
   // Tile width and K splits: the wide tile where it alone fills the chip, else the narrow one; then as many splits
-  // as there are idle SMs, each with at least one k-block.
+  // as there are idle SMs, each with at least one k-block, but no more than leave all clusters on the chip at once (16 of
+  // eight CTAs do not fit: 1024 x 128 x 2048 took two turns, 21.8 us, and takes SPLITB with four).
   const long long tm = (M + kBM - 1) / kBM;
   const long long wide = tm * ((N + 127) / 128) * batch, narrow = tm * ((N + 63) / 64) * batch;
   constexpr int kBK = Cfg<T, 128>::kBK;
@@ -785,7 +814,8 @@ int gemm_split(const T* a, const T* b, void* out, int out_bf16, const float* bia
   const long long tiles = use_wide ? wide : narrow;
   g.kb_total = (K + kBK - 1) / kBK;
   int splits = 1;
-  while (splits < 8 && tiles * splits * 2 <= sm_count() && splits * 2 <= g.kb_total) splits *= 2;
+  const auto fits = [&](int n) { return tiles <= (use_wide ? resident_clusters<T, 128>(n) : resident_clusters<T, 64>(n)); };
+  while (splits < 8 && tiles * splits * 2 <= sm_count() && splits * 2 <= g.kb_total && fits(splits * 2)) splits *= 2;
   g.kb_per_split = (g.kb_total + splits - 1) / splits;
   const int la = layout_of<T>(g.a);
   int lb = layout_of<T>(g.b);
