@@ -13,7 +13,8 @@
 // A step is bound by latency: the product, two block barriers, the gates and the way to the other CTAs; everything a step
 // needs from global memory is fetched one step ahead.  How many clusters of eight are on the chip at once is asked of the
 // driver (it is fewer than SMs / 8, a cluster lies within one part of the chip): LSTM 256, batch 32, 64 steps ran as 16
-// clusters of which not all fitted, 270 us forward and 301 backward for two waves of 150 and 180; now 134 and 149.
+// clusters of which not all fitted, 270 us forward and 301 backward for two waves of 150 and 180; on 8 clusters 134 and
+// 149, on 11 (slices of three rows) 121 and 134 (GRU: 157 and 179 -> 122 and 123).
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -49,19 +50,23 @@ struct SeqArgs {
 
 // How a CTA's threads share the product of its `rows4` rows (a multiple of 4) with a vector v[k][BS] of K entries: a thread
 // takes four rows and a slice of k, the `ks_n` partial sums of an output meet in part[ks][b][row].
+constexpr int piece_k(int bs) { return bs == 3 ? 4 : 4 / bs; }    // weights in registers: k of a piece of the vector,
+constexpr int piece_vec(int bs) { return bs == 3 ? 3 : 1; }        // its 16-byte parts
 struct Tile {
   int quads, ks_n;        // row quads, slices
-  int vec4;               // weights in registers: 16-byte pieces of the vector per slice
+  int pieces;             // weights in registers: pieces of the vector per slice
   int threads, pitch;     // threads that add an output's slices (a power of two within a warp), floats per slice of part
-  __host__ __device__ int vec(int K, int bs, bool reg) const { return reg ? ks_n * vec4 * 4 : (K + 3) / 4 * 4 * bs; }
+  __host__ __device__ int vec(int K, int bs, bool reg) const {
+    return reg ? ks_n * pieces * piece_vec(bs) * 4 : (K + 3) / 4 * 4 * bs;
+  }
 };
 __host__ __device__ inline Tile tile_of(int rows4, int K, int bs, bool reg) {
   Tile t;
   t.quads = rows4 / 4;
   t.ks_n = kT / t.quads;
-  const int pieces = (K * bs + 3) / 4;
-  if (reg && t.ks_n > pieces) t.ks_n = pieces;
-  t.vec4 = (pieces + t.ks_n - 1) / t.ks_n;
+  const int all = bs == 3 ? (K + 3) / 4 : (K * bs + 3) / 4;
+  if (reg && t.ks_n > all) t.ks_n = all;
+  t.pieces = (all + t.ks_n - 1) / t.ks_n;
   const int n = rows4 * bs;
   t.threads = 1;
   while (t.threads < 32 && t.threads * 2 * n <= kT) t.threads *= 2;
@@ -119,22 +124,29 @@ __device__ __forceinline__ void matvec(const float* wsm, int k_res, int K, int r
 // The same product with the weights in registers: four rows and up to kKpt k per thread.  What a step then moves is the
 // vector, and a 16-byte read takes four cycles of the shared memory's 128 bytes per cycle even where all lanes read the
 // same address: with two rows and 32 k per thread that was 1470 cycles at LSTM 256 on 8 CTAs, two batch rows.  Slice ks
-// takes the 16-byte pieces ks, ks + ks_n, ...: neighbouring slices in a warp read neighbouring pieces.
+// takes the pieces ks, ks + ks_n, ... (16 bytes each, 48 for three batch rows): neighbouring slices in a warp read
+// neighbouring pieces.  The multiply-adds take as many cycles as those reads (1024 each of a step's 4180 at LSTM 256 with
+// four batch rows; two in one instruction run at half the rate), so a slice is no taller than the chip's clusters make it:
+// batch 32 in slices of three on 11 clusters, not of four on eight.
 constexpr int kKpt = 16;
 template <int BS>
 __device__ __forceinline__ void matvec_reg(const float (&w)[4][kKpt], const Tile& t, int rows4, int ks, int rq, const float* v,
                                            float* part) {
   if (ks >= t.ks_n) return;
-  constexpr int kPer = 4 / BS;  // k of a piece
+  constexpr int kPer = piece_k(BS), kVec = piece_vec(BS);
   float acc[4][BS];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int b = 0; b < BS; ++b) acc[i][b] = 0.f;
-  const float4* x = reinterpret_cast<const float4*>(v) + ks;
+  const float4* x = reinterpret_cast<const float4*>(v) + ks * kVec;
   auto piece = [&](int j) {
-    const float4 f = x[j * t.ks_n];
-    const float e[4] = {f.x, f.y, f.z, f.w};
+    float e[kVec * 4];
+#pragma unroll
+    for (int q = 0; q < kVec; ++q) {
+      const float4 f = x[j * t.ks_n * kVec + q];
+      e[q * 4] = f.x; e[q * 4 + 1] = f.y; e[q * 4 + 2] = f.z; e[q * 4 + 3] = f.w;
+    }
 #pragma unroll
     for (int k = 0; k < kPer; ++k)
 #pragma unroll
@@ -142,13 +154,13 @@ __device__ __forceinline__ void matvec_reg(const float (&w)[4][kKpt], const Tile
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[i][b] = fmaf(w[i][j * kPer + k], e[k * BS + b], acc[i][b]);
   };
-  if (t.vec4 == kKpt / kPer) {
+  if (t.pieces == kKpt / kPer) {
 #pragma unroll
     for (int j = 0; j < kKpt / kPer; ++j) piece(j);
   } else {
 #pragma unroll
     for (int j = 0; j < kKpt / kPer; ++j)
-      if (j < t.vec4) piece(j);
+      if (j < t.pieces) piece(j);
   }
   float* p = part + ks * t.pitch + rq * 4;
 #pragma unroll
@@ -158,14 +170,14 @@ __device__ __forceinline__ void matvec_reg(const float (&w)[4][kKpt], const Tile
 // This thread's weights: at(row) is the address of the row's first one or NULL, `step` the distance from k to k + 1.
 template <int BS, class At>
 __device__ __forceinline__ void load_weights(float (&w)[4][kKpt], const Tile& t, int K, int ks, int rq, long long step, At at) {
-  constexpr int kPer = 4 / BS;
+  constexpr int kPer = piece_k(BS);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const float* p = ks < t.ks_n ? at(rq * 4 + i) : nullptr;
 #pragma unroll
     for (int j = 0; j < kKpt; ++j) {
       const int k = (ks + j / kPer * t.ks_n) * kPer + j % kPer;
-      w[i][j] = p != nullptr && j / kPer < t.vec4 && k < K ? __ldg(p + k * step) : 0.f;
+      w[i][j] = p != nullptr && j / kPer < t.pieces && k < K ? __ldg(p + k * step) : 0.f;
     }
   }
 }
@@ -185,12 +197,16 @@ __device__ __forceinline__ Fold fold_of(const Tile& t, int n) {
   f.leader = f.part == 0;
   return f;
 }
+// kUnroll: slices in flight.  Registers are short beside the weights (64 of 128): forward with the weights there takes four
+// (LSTM 256, one batch row 96.7 -> 91.5 us; with sixteen two batch rows went from 106 to 112), the others, which have fewer
+// values to keep, eight (LSTM 256 backward, two batch rows: 97, with four 101; LSTM 512 forward: 988, with four 1014).
+template <int kUnroll>
 __device__ __forceinline__ float fold_sum(const Fold& f, const Tile& t, const float* part, int o, int n) {
   float s = 0.f;
   if (o < n) {
     const float* p = part + f.part * t.pitch + o;
     const int step = t.threads * t.pitch;
-#pragma unroll 8
+#pragma unroll kUnroll
     for (int ks = f.part; ks < t.ks_n; ks += t.threads, p += step) s += *p;
   }
   for (int d = t.threads >> 1; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
@@ -360,7 +376,7 @@ __global__ void __launch_bounds__(kT, 1) seq_fwd_kernel(const SeqArgs a) {
     __syncthreads();
     // gate activations in the threads that add the slices: the serial part below is the cell update alone
     for (int pass = 0, o = fd.out; pass < fd.passes; ++pass, o += fd.step) {
-      float s = fold_sum(fd, tile, part, o, n_out);
+      float s = fold_sum<kReg ? 4 : 8>(fd, tile, part, o, n_out);
       if (!fd.leader || o >= n_out) continue;
       int gate = gate0, u = uu0, b = bb0;
       bool ok = valid0;
@@ -534,7 +550,7 @@ __global__ void __launch_bounds__(kT, 1) seq_bwd_kernel(const SeqArgs a) {
       });
     __syncthreads();
     for (int pass = 0, o = fd.out; pass < fd.passes; ++pass, o += fd.step) {
-      const float s = fold_sum(fd, tile, part, o, n_out);
+      const float s = fold_sum<8>(fd, tile, part, o, n_out);
       if (fd.leader && o < n_out) dh[o] = s;
     }
     __syncthreads();
@@ -565,19 +581,22 @@ struct Plan {
 int cluster_slots(int ncl);
 
 // Cluster size: one CTA per 32 hidden units up to eight (a CTA's share of the weights is then what a step has to
-// stream from shared memory).  Batch slice: as small as keeps every cluster on the chip at once.
+// stream from shared memory).  Batch slice: as small as keeps every cluster on the chip at once; three rows only with the
+// weights in registers (where shared memory or L2 holds them a step costs what it reads of them, whatever the slice).
 bool plan(int G, int B, int H, bool backward, Plan* p) {
   if (H < 1 || H > 1024) return false;
   p->ncl = H >= 256 ? 8 : (H >= 128 ? 4 : (H >= 64 ? 2 : 1));
   const int slots = cluster_slots(p->ncl);
-  p->bs = B <= slots ? 1 : (B <= 2 * slots ? 2 : (B <= 4 * slots ? 4 : 8));
+  p->bs = B <= slots ? 1 : (B <= 2 * slots ? 2 : (B <= 3 * slots ? 3 : (B <= 4 * slots ? 4 : 8)));
   p->hs_units = (H + p->ncl - 1) / p->ncl;
   const int rows = backward ? p->hs_units : G * p->hs_units, K = backward ? G * H : H;
   p->rows4 = (rows + 3) / 4 * 4;
   if (p->rows4 / 4 > kT) return false;
   const size_t limit = static_cast<size_t>(smem_limit()) - 1024;
-  for (; p->bs >= 1; p->bs >>= 1) {  // a smaller slice leaves more shared memory to the weights
-    p->reg = p->bs <= 4 && tile_of(p->rows4, K, p->bs, true).vec4 * (4 / p->bs) <= kKpt;
+  auto in_registers = [&] { return p->bs <= 4 && tile_of(p->rows4, K, p->bs, true).pieces * piece_k(p->bs) <= kKpt; };
+  if (p->bs == 3 && !in_registers()) p->bs = 4;
+  for (; p->bs >= 1; p->bs = p->bs == 3 ? 2 : p->bs >> 1) {  // a smaller slice leaves more shared memory to the weights
+    p->reg = in_registers();
     const Tile t = tile_of(p->rows4, K, p->bs, p->reg);
     // two vectors, the partial sums, and the gates with their two input buffers
     const size_t fixed = (2 * static_cast<size_t>(t.vec(K, p->bs, p->reg)) + static_cast<size_t>(t.ks_n) * t.pitch +
@@ -656,6 +675,7 @@ int run_bs(bool backward, const SeqArgs& a, const Plan& p, cudaStream_t st) {
   switch (p.bs) {
     case 1: return run<G, 1>(backward, a, p, st);
     case 2: return run<G, 2>(backward, a, p, st);
+    case 3: return run<G, 3>(backward, a, p, st);
     case 4: return run<G, 4>(backward, a, p, st);
     default: return run<G, 8>(backward, a, p, st);
   }
@@ -674,7 +694,7 @@ extern "C" int fb_rnn_seq_supported(int gates, int B, int H) {
 extern "C" int fb_rnn_seq_plan(int gates, int B, int H, int backward) {
   Plan p;
   if ((gates != 3 && gates != 4) || B < 1 || !plan(gates, B, H, backward != 0, &p)) return 0;
-  const bool full = p.reg && tile_of(p.rows4, backward ? gates * H : H, p.bs, true).vec4 == kKpt / (4 / p.bs);
+  const bool full = p.reg && tile_of(p.rows4, backward ? gates * H : H, p.bs, true).pieces == kKpt / piece_k(p.bs);
   return p.bs + (p.reg ? 16 : 0) + (full ? 32 : 0);
 }
 

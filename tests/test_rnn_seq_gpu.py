@@ -51,7 +51,7 @@ def test_sequence(kind, T, B, I, H, L, state):
 
 
 @pytest.mark.parametrize("kind", ["LSTM", "GRU"])
-@pytest.mark.parametrize("H,bs", [(256, 1), (256, 2), (256, 4), (128, 4), (256, 8)])
+@pytest.mark.parametrize("H,bs", [(256, 1), (256, 2), (256, 3), (128, 3), (256, 4), (128, 4), (256, 8)])
 def test_batch_slices(kind, H, bs):
     """Every number of batch rows per cluster, the last slice whole and not; how many clusters the chip holds decides which
     batches that are."""
