@@ -178,6 +178,7 @@ _CUDA_SIGS = {
     "fb_embedding_keys": (I, [P, P, LL, LL, P]),
     "fb_embedding_pairs": (I, [P, P, P, LL, LL, LL, P]),
     "fb_embedding_bwd_pairs": (I, [P, P, P, P, LL, I, I, F, LL, LL, I, P]),
+    "fb_embedding_bwd_pairs_zeroed": (I, [P, P, P, P, LL, I, I, F, LL, LL, I, P]),
     "fb_gather_rows": (I, [P, P, P, LL, LL, LL, P, P]),
     "fb_attention_fwd": (I, [P, P, P, P, P, I, I, I, I, I, LL, LL, LL, LL, LL, LL, LL, LL, LL, F, I, P, P]),
     "fb_attention_bwd": (I, [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, LL, LL, LL, LL, LL, LL, LL, LL, LL, F, I, P, P]),

@@ -241,6 +241,10 @@ int fb_embedding_pairs(const long long* idx, int32_t* keys, int32_t* rows, long 
 int fb_embedding_bwd_pairs(const void* dout, const int32_t* keys, const int32_t* rows, float* dweight, long long n_idx,
                            int dim, int group, float scale, long long padding_idx, long long vocab, int dtype,
                            cudaStream_t stream);
+// The same into a table that holds zeros.
+int fb_embedding_bwd_pairs_zeroed(const void* dout, const int32_t* keys, const int32_t* rows, float* dweight, long long n_idx,
+                                  int dim, int group, float scale, long long padding_idx, long long vocab, int dtype,
+                                  cudaStream_t stream);
 int fb_embedding_keys(const long long* idx, int32_t* keys, long long n, long long vocab, cudaStream_t stream);
 int fb_embedding_bwd_sorted(const void* dout, const void* sorted_idx, int key_bytes, const long long* perm,
                             float* dweight, long long n_idx, int dim, int group, float scale, long long padding_idx,

@@ -36,11 +36,13 @@ struct EmbeddingNode : Node {
         std::tie(sorted, perm) = at::sort(idx.reshape({-1}), /*stable=*/true, /*dim=*/0, /*descending=*/false);
       }
     }
+    bool add = false;
     if (sink) {  // accumulate straight into the data-parallel gradient arena
       py::gil_scoped_acquire gil;
       py::tuple r = py::handle(sink->sink).attr("acquire")(py::handle(sink->param));
       dw = r[0].cast<Tensor>();
-      if (!r[1].cast<bool>()) dw.zero_();
+      add = r[1].cast<bool>();
+      if (!add) dw.zero_();
     } else {
       dw = at::zeros({vocab, dim}, g2.options().dtype(at::kFloat));
     }
@@ -49,10 +51,11 @@ struct EmbeddingNode : Node {
       FB_CALL(fb_embedding_bwd_sorted, g2.data_ptr(), sorted.data_ptr(), 8,
               reinterpret_cast<const ll*>(perm.data_ptr<int64_t>()), dw.data_ptr<float>(), n, static_cast<int>(dim),
               static_cast<int>(group), scale, padding, vocab, dt(g2), cur_stream());
-    else if (n > 0)
-      FB_CALL(fb_embedding_bwd_pairs, g2.data_ptr(), sorted.data_ptr<int32_t>(), sorted.data_ptr<int32_t>() + pitch,
-              dw.data_ptr<float>(), n, static_cast<int>(dim), static_cast<int>(group), scale, padding, vocab, dt(g2),
-              cur_stream());
+    else if (n > 0) {
+      const auto scatter = add ? fb_embedding_bwd_pairs : fb_embedding_bwd_pairs_zeroed;
+      FB_CALL(scatter, g2.data_ptr(), sorted.data_ptr<int32_t>(), sorted.data_ptr<int32_t>() + pitch, dw.data_ptr<float>(), n,
+              static_cast<int>(dim), static_cast<int>(group), scale, padding, vocab, dt(g2), cur_stream());
+    }
     if (sink) sink_ready(*sink);
     else out[0] = dw;
     return out;

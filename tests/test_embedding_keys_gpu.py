@@ -75,3 +75,39 @@ def test_pairs(vocab, batch, seq, dim):
         size.index_add_(0, idx.view(-1)[keep], per[keep].abs())
         check_status()
         assert ((w.grad - want).abs() <= 2.0 ** -22 * size * 8).all()
+
+
+@pytest.mark.parametrize("dim", [3, 8, 36, 1024, 1100])
+@pytest.mark.parametrize("vocab,n", [(1, 1), (1, 64), (15, 31), (17, 32), (40, 33), (40, 4000), (3000, 700), (33, 95), (5, 1000)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gradient_in_chunks(vocab, n, dim, dtype):
+    """Into a table of zeros and onto another: runs of an index within a chunk of 32, over its edges and over many chunks,
+    the same row of the gradient several times in a run, an index that is the padding, indices outside the table.  Sums of
+    32 bits within a chunk, then of the chunks, then the table's value."""
+    from ferrum_b200 import _lib
+    from ferrum_b200.ops import functional as F
+    from ferrum_b200.utils.runtime import check_status
+
+    g = torch.Generator(device="cuda").manual_seed(vocab + n + dim)
+    keys = torch.randint(0, vocab, (n,), device="cuda", generator=g)
+    keys[: n // 2] = vocab // 2
+    keys[-1] = vocab
+    for padding, zeroed in ((-1, True), (-1, False), (vocab // 2, True)):
+        group = 3
+        rows = torch.arange(n, device="cuda") // group
+        key, perm = torch.sort(keys, stable=True)
+        key, row = key.int(), rows[perm].int()
+        dout = torch.randn((n + group - 1) // group, dim, device="cuda", generator=g).to(dtype)
+        old = torch.randn(vocab, dim, device="cuda", generator=g) * (0 if zeroed else 1)
+        dw, lib = old.clone(), _lib.cuda()
+        _lib.check((lib.fb_embedding_bwd_pairs_zeroed if zeroed else lib.fb_embedding_bwd_pairs)(
+            dout.data_ptr(), key.data_ptr(), row.data_ptr(), dw.data_ptr(), n, dim, group, 0.5, padding, vocab,
+            F._dt(dout), torch.cuda.current_stream().cuda_stream), "grad")
+        check_status()
+        want, size = (torch.zeros(vocab + 1, dim, device="cuda", dtype=torch.float64) for _ in range(2))
+        want.index_add_(0, keys, dout.double()[rows] * 0.5)
+        size.index_add_(0, keys, dout.double()[rows].abs() * 0.5)
+        if padding >= 0:
+            want[padding] = 0
+        bound = 2.0 ** -24 * (40 + n / 32) * (size[:vocab] + old.abs())
+        assert ((dw - old.double() - want[:vocab]).abs() <= bound).all()
