@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("b_mn", [False, True])
 @pytest.mark.parametrize("M,N,K", [(1, 512, 512), (16, 520, 64), (17, 1000, 2056), (32, 4096, 520), (33, 4744, 1032),
-                                   (64, 9480, 512), (5, 96, 4104)])
+                                   (64, 9480, 512), (5, 96, 4104), (16, 640, 320), (30, 648, 448), (64, 520, 576)])
 def test_bits(M, N, K, b_mn):
     from ferrum_b200 import _lib
     from ferrum_b200.utils import runtime as rt
