@@ -461,12 +461,12 @@ int launch(const CUtensorMap& mp, const CUtensorMap& mq, Args& g, int rows_p, in
 }  // namespace
 }  // namespace fb
 
-// Where this kernel is the faster one by enough to repay another order of summation.  The persistent kernels take
-// 4.6 us and 4.3 ns per unit of K for any output that fits one wave (a chain of MMAs on one accumulator advances by
-// 16 of K in 69 ns however narrow the tile); this one has 5 to 6 us of launch, cluster and epilogue and then divides K
-// by the splits.  K 256: 6 against 5.7 us; K 1024: 7 against 9 at best; K 2048: 8 against 13.5 us with eight splits
-// (8 x 4096), 10.8 against 14 with four (96 x 4096); with two splits it needs a very long reduction
-// (512 x 4096 x 8192: 43 against 49 us, but 300 x 4096 x 4096: 26 against 24).
+// Where this kernel is the faster one by enough to repay another order of summation.  The persistent kernels take, for any
+// output that fits one wave, 4.6 us and 4.3 ns per unit of K on single CTAs and 5.2 us and 2.9 ns on pairs (512 x 512: K 1024
+// 8.1, K 4096 16.8 us); this one has 5 to 6 us of launch, cluster and epilogue and then divides K by the splits.  K 256: 6
+// against 5.7 us; K 1024: 7 against 9 at best; K 2048: 8 against 13.5 us with eight splits (8 x 4096), 10.8 against 14 with
+// four (96 x 4096).  Two splits of a very long reduction stay here although the pairs have caught up since (512 x 4096 x
+// 8192 was 43 against 49 us): half the chain of truncating additions, half the error.
 extern "C" int fb_gemm_bf16_splitk_use(int M, int N, int K) {
   using namespace fb;
   if (M <= 0 || N <= 0 || K < 2048) return 0;
@@ -544,7 +544,8 @@ extern "C" int fb_gemm_bf16_splitk(const void* a, const void* b, void* out, void
 // tiles of 128 columns of B (operands exchanged) / of 32, us: 16 x 4096 x 4096 29.7 / 22.7 / 17.1, 16 x 1024 x 4096
 // 29.0 / 20.0 / 13.8, 16 x 4096 x 1024 12.4 / 9.6 / 7.9, 64 x 1000 x 1024 12.8 / 11.0 / 8.4; 16 x 10000 x 1024, more
 // tiles of 32 than SMs: 13.0 / 11.3 / 14.9, with 64 columns 10.1.  16 x 128 x 512 was 12.3 on the persistent kernels and
-// 14.3 here, 128 x 512 x 512 18.4 on both.
+// 14.3 here, 128 x 512 x 512 18.4 on both.  Since then (copies of a whole stage, MMAs of 64 rows, dependents let in after the
+// last MMA), operands in L2: 16 x 4096 x 4096 15.6 -> 10.9, 16 x 4096 x 1024 7.2 -> 5.7, 64 x 1000 x 1024 7.3 -> 6.8.
 extern "C" int fb_gemm_bf16_narrow_use(int M, int N, int K) {
   return M > 0 && M <= 64 && N >= 512 && N <= fb::kRowsP * fb::sm_count() && K >= 512;
 }

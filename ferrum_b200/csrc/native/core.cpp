@@ -138,7 +138,8 @@ static bool copies_repay(const Op& a, const Op& b, bool rows_tma) {
 // 1e-7 against 1e-6 at K = 1001 and 4e-6 at K = 4095.  A row's bits may change when the rows beside it pass this line
 // (those of aligned operands never do).  In place against copy + product, us: 1024 x 1001 x 1001 19.1 / 3.7 + 13.8, 2048 x
 // 1001 x 1001 30.3 / 4.6 + 14.0, 777 x 2049 x 2049 49.2 / 6.3 + 20.4, 512 x 4095 x 4095 84.9 / 16.6 + 32.0, 8191 x 4095 x
-// 4095 1146 / 48 + 200; below 512 rows, without the pairs, 300 x 1001 x 4095 27.1 / 6.3 + 55.2.
+// 4095 1146 / 48 + 200; below 512 rows, without the pairs, 300 x 1001 x 4095 27.1 / 6.3 + 55.2.  (Both sides have become 5 - 15 %
+// faster since.)
 static bool repack_repays(const Op& a, const Op& b) {
   if (a.rows < 512 || b.rows < 128) return false;
   double cost = 14.;
