@@ -49,6 +49,7 @@
 
 #include "../common/ptx.cuh"
 #include "../common/status.h"
+#include "../common/tmem_share.h"
 #include "../include/ferrum_kernels.h"
 
 namespace fb {
@@ -96,7 +97,12 @@ struct Cfg {
   static constexpr int kTile = kBM * kPitch * 4;
   static constexpr int kBody = kStages * kStage > kTile ? kStages * kStage : kTile;
   static constexpr int kSmem = kBody + 1024 + 256;
+  // With splits: all of tensor memory is held over a cluster barrier (common/tmem_share.h).  The registers alone (96 x 544)
+  // kept other such CTAs off the SM until here.
+  static constexpr int kSmemSplit = kATmem && kSmem < kClusterAloneSmem ? kClusterAloneSmem : kSmem;
   static constexpr int kTmemCols = kATmem ? 512 : 2 * BN;  // two accumulators, then the stages of A
+  static_assert(kSmem >= kClusterLeastSmem, "tensor memory is held over a cluster barrier");
+  static_assert(kTmemCols < 512 || kSmemSplit + kClusterLeastSmem + 2 * kCtaSmem > kSmSmem, "no room for another one's columns");
   static constexpr int kPerThread = (kATmem ? BN : kBM + BN) * kPieces / kLoaders;  // pieces of a stage per thread
   static constexpr int kAcc = kBM * BN / kLoaders;                    // accumulators per thread: a quarter of a tile row
   // 16-byte chunk of a row, as the 128- / 64-byte swizzle of the matrix descriptors places it
@@ -708,14 +714,14 @@ int resident_clusters(int size) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(size));
     cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = Cfg<T, BN>::kSmem;
+    cfg.dynamicSmemBytes = Cfg<T, BN>::kSmemSplit;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = size;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<T, BN>::kSmem) != cudaSuccess ||
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<T, BN>::kSmemSplit) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
       n = sm_count() / size;
@@ -727,11 +733,10 @@ int resident_clusters(int size) {
 
 template <typename T, int BN, int LA, int LB>
 int launch_one(const Args& args, int batch, int splits, cudaStream_t st) {
-  constexpr int kSmem = Cfg<T, BN>::kSmem;
   static bool configured = false;
   if (!configured) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(gemm_split_kernel<T, BN, LA, LB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_split_kernel<T, BN, LA, LB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               Cfg<T, BN>::kSmemSplit);
     if (e != cudaSuccess) return static_cast<int>(e);
     configured = true;
   }
@@ -739,7 +744,7 @@ int launch_one(const Args& args, int batch, int splits, cudaStream_t st) {
   cfg.gridDim = dim3(static_cast<unsigned>((args.N + BN - 1) / BN * splits), static_cast<unsigned>((args.M + kBM - 1) / kBM),
                      static_cast<unsigned>(batch));
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = kSmem;
+  cfg.dynamicSmemBytes = splits > 1 ? Cfg<T, BN>::kSmemSplit : Cfg<T, BN>::kSmem;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;

@@ -30,6 +30,7 @@
 
 #include "../common/ptx.cuh"
 #include "../common/status.h"
+#include "../common/tmem_share.h"
 #include "../include/ferrum_kernels.h"
 #include "epilogue.cuh"
 
@@ -442,6 +443,7 @@ int launch(const CUtensorMap& mp, const CUtensorMap& mq, Args& g, int rows_p, in
   if (g.stages > need) g.stages = need;
   g.body_bytes = (g.stages * kGroup * g.block_bytes + tail + 1023) / 1024 * 1024;
   if (g.body_bytes < C::kTile) g.body_bytes = (C::kTile + 1023) / 1024 * 1024;
+  if (splits > 1 && g.body_bytes < kClusterLeastSmem) g.body_bytes = kClusterLeastSmem;  // never, with stages of 18 KB and more
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(tiles * splits));
   cfg.blockDim = dim3(kThreads);

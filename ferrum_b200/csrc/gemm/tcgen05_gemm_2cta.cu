@@ -45,6 +45,7 @@
 
 #include "../common/ptx.cuh"
 #include "../common/status.h"
+#include "../common/tmem_share.h"
 #include "../dist/dist_ctx.h"
 #include "../include/ferrum_kernels.h"
 #include "epilogue.cuh"
@@ -69,6 +70,7 @@ struct Cfg2 {
   // two output slabs per epilogue warp (the push mode uses a warp's 8 KB as a 32 x 33 fp32 transposing buffer)
   static constexpr int kStoreBytes = kEpilogueWarps * 2 * kSlabBytes;
   static constexpr int kSmemBytes = kStages * kStageBytes + kStoreBytes + 1024 + 256;
+  static_assert(kSmemBytes >= kClusterLeastSmem, "tensor memory is held over a cluster barrier");
   static constexpr int kTmemCols = 2 * BN;                    // two accumulators
 };
 
