@@ -151,6 +151,7 @@ _CUDA_SIGS = {
     "fb_reduce": (I, [P, P, LL, LL, LL, I, P, LL, P]),
     "fb_arg_reduce": (I, [P, P, P, LL, LL, LL, I, P]),
     "fb_colsum": (I, [P, P, LL, LL, I, I, P]),
+    "fb_colsum_clusters": (I, [LL, LL, I, I, I]),
     "fb_unary_bwd_colsum": (I, [P, P, P, P, LL, LL, I, I, P]),
     # norms
     "fb_layernorm_fwd": (I, [P, P, P, P, P, P, LL, I, F, I, I, P]),
@@ -222,7 +223,7 @@ class _CountingLib:
     """
 
     _NO_COUNT = ("fb_rt_", "fb_reduce_scratch_elems", "fb_layernorm_bwd_blocks", "fb_gemm_bf16_supported", "fb_gemm_bf16_2cta_pairs",
-                 "fb_dist_query_")
+                 "fb_colsum_clusters", "fb_dist_query_")
 
     def __init__(self, lib):
         self._lib = lib

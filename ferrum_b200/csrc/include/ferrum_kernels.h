@@ -133,10 +133,11 @@ int fb_reduce(const float* x, float* out, long long outer, long long R, long lon
               long long scratch_elems, cudaStream_t stream);
 int fb_arg_reduce(const float* x, long long* idx, float* val, long long outer, long long R, long long inner,
                   int is_max, cudaStream_t stream);
-// Column sums of a [rows, cols] matrix (fp32 or bf16 in, fp32 out): bias gradients.
-// dx = dy * act'(y) of a ReLU, tanh or sigmoid, and its column sums; -3: these want fb_colsum.
+// dx = dy * act'(y) of a ReLU, tanh or sigmoid, and its column sums; -3, nothing launched: these want fb_colsum.
 int fb_unary_bwd_colsum(const void* dy, const void* y, void* dx, float* sums, long long rows, long long cols, int op, int dtype,
                         cudaStream_t stream);
+// Column sums of a [rows, cols] matrix (fp32 or bf16 in, fp32 out): bias gradients.
+int fb_colsum_clusters(long long rows, long long cols, int dtype, int grad, int aligned);  // a query
 int fb_colsum(const void* x, float* out, long long rows, long long cols, int dtype, int accumulate,
               cudaStream_t stream);
 

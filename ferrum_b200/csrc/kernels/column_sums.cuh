@@ -87,7 +87,6 @@ __device__ __forceinline__ void unpack16(const uint4& u, float (&v)[16 / sizeof(
 template <typename T>
 struct PlainRows {
   static constexpr int kV = 16 / sizeof(T), kU = 8;
-  using Elem = T;
   using Raw = uint4;
   const T* x;
   __host__ __device__ bool aligned() const { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; }
@@ -155,28 +154,43 @@ colsum_cluster_kernel(const Rows m, float* __restrict__ out, long long rows, lon
   });
 }
 
-// Eight blocks to a column range: enough of them for the chip where there are many ranges, or little to read.
-template <typename T>
-bool column_cluster_fits(long long rows, long long cols) {
-  const long long ranges = (cols + 32 / sizeof(T) - 1) / (32 / sizeof(T));
-  return ranges <= 0x7fffffffLL && (ranges * 8 >= column_sms() || rows * cols * static_cast<long long>(sizeof(T)) <= (4LL << 20));
+struct ColumnPlan {
+  int lanes, split;  // 16-byte pieces of a row to a block, blocks to a column range
+  long long ranges;
+};
+inline ColumnPlan column_plan(long long rows, long long cols, int v) {  // v: elements of 16 bytes
+  // 128 bytes of a row to a block, or 64 or 32 where that would leave a third of the chip without one (memory is read by
+  // lines: 8192 x 1024 bf16 9.7 us with 32 bytes, 7.6 with 128).
+  ColumnPlan p{8, 1, 0};
+  while (p.lanes > 2 && (cols + p.lanes * v - 1) / (p.lanes * v) * 8 * 3 < column_sms() * 2) p.lanes /= 2;
+  p.ranges = (cols + p.lanes * v - 1) / (p.lanes * v);
+  // As many blocks to a range as give every SM one: with eight to each of 64 ranges they took turns (512 x 4096 bf16 7.5 us).
+  while (p.split < 8 && p.ranges * p.split < column_sms() && rows >= p.split * 64) p.split *= 2;
+  return p;
+}
+// Eight blocks to a column range: enough of them for the chip where there are many ranges, or little to read.  size: bytes of
+// an element; grad: behind an activation's gradient.
+inline bool column_cluster_pays(long long rows, long long cols, int size, bool grad, bool aligned) {
+  const int v = 16 / size;
+  const long long pieces = (cols + 2 * v - 1) / (2 * v);
+  if (pieces > 0x7fffffffLL) return false;
+  // Single loads of elements that lie 16 bytes apart in neighbouring lanes: with a gradient to store they repay the launches
+  // for one round of the block's threads (bf16, us, two launches / one: 512 x 1001 8.3 / 7.0, 1024 x 1001 12.3 / 14.2, 8191 x
+  // 4095 with the products around it 265 / 399).
+  if (grad && (cols % v != 0 || !aligned)) {
+    const ColumnPlan p = column_plan(rows, cols, v);
+    return (rows + p.split - 1) / p.split <= kColumnThreads / p.lanes;
+  }
+  return pieces * 8 >= column_sms() || rows * cols * size <= (4LL << 20);
 }
 template <class Rows>
 int launch_colsum(const Rows& m, float* out, long long rows, long long cols, int accumulate, cudaStream_t stream) {
-  // 128 bytes of a row to a block, or 64 or 32 where that would leave a third of the chip without one (memory is read by
-  // lines: 8192 x 1024 bf16 9.7 us with 32 bytes, 7.6 with 128).
-  int lanes = 8;
-  while (lanes > 2 && (cols + lanes * Rows::kV - 1) / (lanes * Rows::kV) * 8 * 3 < column_sms() * 2) lanes /= 2;
-  const long long per = lanes * Rows::kV;
-  // As many blocks to a range as give every SM one: with eight to each of 64 ranges they took turns (512 x 4096 bf16 7.5 us).
-  const long long ranges = (cols + per - 1) / per;
-  int split = 1;
-  while (split < 8 && ranges * split < column_sms() && rows >= split * 64) split *= 2;
-  const dim3 grid(static_cast<unsigned>(ranges), static_cast<unsigned>(split));
-  const long long rpb = (rows + split - 1) / split;
-  const auto kernel = lanes == 8   ? colsum_cluster_kernel<Rows, 8>
-                      : lanes == 4 ? colsum_cluster_kernel<Rows, 4>
-                                   : colsum_cluster_kernel<Rows, 2>;
+  const ColumnPlan p = column_plan(rows, cols, Rows::kV);
+  const dim3 grid(static_cast<unsigned>(p.ranges), static_cast<unsigned>(p.split));
+  const long long rpb = (rows + p.split - 1) / p.split;
+  const auto kernel = p.lanes == 8   ? colsum_cluster_kernel<Rows, 8>
+                      : p.lanes == 4 ? colsum_cluster_kernel<Rows, 4>
+                                     : colsum_cluster_kernel<Rows, 2>;
   return launch_column_cluster(kernel, grid, stream, m, out, rows, cols, rpb, accumulate);
 }
 

@@ -191,7 +191,6 @@ __global__ void unary_bwd_f32(const float* __restrict__ dy, const float* __restr
 template <typename T, int OP>
 struct GradRows {
   static constexpr int kV = 16 / sizeof(T), kU = 4;
-  using Elem = T;
   struct Raw {
     uint4 g, y;
   };
@@ -608,7 +607,7 @@ extern "C" int fb_unary_fwd(const void* x, void* y, long long n, int op, float a
 }
 
 // dx = dy * act'(y) for an activation whose derivative is a function of its result (ReLU, tanh, sigmoid), [rows, cols], and
-// sums[cols] = its column sums.  -3: a shape whose column sums want a launch of their own.
+// sums[cols] = its column sums.  -3, and nothing is launched: a shape or an address where a pass of each is faster.
 extern "C" int fb_unary_bwd_colsum(const void* dy, const void* y, void* dx, float* sums, long long rows, long long cols, int op,
                                    int dtype, cudaStream_t stream) {
   using namespace fb;
@@ -616,18 +615,17 @@ extern "C" int fb_unary_bwd_colsum(const void* dy, const void* y, void* dx, floa
   if (rows <= 0) return static_cast<int>(cudaMemsetAsync(sums, 0, static_cast<size_t>(cols) * sizeof(float), stream));
   const auto run = [&](auto type) {
     using T = decltype(type);
-    if (!column_cluster_fits<T>(rows, cols)) return -3;
     const T *g = static_cast<const T*>(dy), *r = static_cast<const T*>(y);
     T* d = static_cast<T*>(dx);
+    if (op != FB_ACT_RELU && op != FB_ACT_TANH && op != FB_ACT_SIGMOID) return -1;
+    if (!column_cluster_pays(rows, cols, sizeof(T), true, GradRows<T, FB_ACT_RELU>{g, r, d}.aligned())) return -3;
     switch (op) {
       case FB_ACT_RELU:
         return launch_colsum(GradRows<T, FB_ACT_RELU>{g, r, d}, sums, rows, cols, 0, stream);
       case FB_ACT_TANH:
         return launch_colsum(GradRows<T, FB_ACT_TANH>{g, r, d}, sums, rows, cols, 0, stream);
-      case FB_ACT_SIGMOID:
-        return launch_colsum(GradRows<T, FB_ACT_SIGMOID>{g, r, d}, sums, rows, cols, 0, stream);
       default:
-        return -1;
+        return launch_colsum(GradRows<T, FB_ACT_SIGMOID>{g, r, d}, sums, rows, cols, 0, stream);
     }
   };
   return dtype == FB_DT_F32 ? run(float{}) : dtype == FB_DT_BF16 ? run(__nv_bfloat16{}) : -1;

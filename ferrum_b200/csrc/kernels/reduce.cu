@@ -423,17 +423,23 @@ extern "C" int fb_arg_reduce(const float* x, long long* idx, float* val, long lo
   return static_cast<int>(cudaGetLastError());
 }
 
+// 1: one launch of clusters gives the sums (behind an activation's gradient: grad), 0: they are added up in a cleared buffer.
+extern "C" int fb_colsum_clusters(long long rows, long long cols, int dtype, int grad, int aligned) {
+  return rows > 0 && cols > 0 && fb::column_cluster_pays(rows, cols, dtype == FB_DT_BF16 ? 2 : 4, grad != 0, aligned != 0);
+}
+
 extern "C" int fb_colsum(const void* x, float* out, long long rows, long long cols, int dtype, int accumulate,
                          cudaStream_t stream) {
   if (cols <= 0) return 0;
   if (rows <= 0)  // an empty sum
     return accumulate ? 0 : static_cast<int>(cudaMemsetAsync(out, 0, cols * sizeof(float), stream));
-  if (dtype == FB_DT_F32 && fb::column_cluster_fits<float>(rows, cols))
-    return fb::launch_colsum(fb::PlainRows<float>{static_cast<const float*>(x)}, out, rows, cols, accumulate, stream);
   // bf16 matrices past L2's half are read faster by more, smaller blocks: 16384 x 3072 22.1 us here, 20.6 with the fill.
-  if (dtype == FB_DT_BF16 && fb::column_cluster_fits<__nv_bfloat16>(rows, cols) && rows * cols <= (24LL << 20))
-    return fb::launch_colsum(fb::PlainRows<__nv_bfloat16>{static_cast<const __nv_bfloat16*>(x)}, out, rows, cols, accumulate,
-                             stream);
+  const bool low = dtype == FB_DT_BF16, aligned = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  if ((low || dtype == FB_DT_F32) && fb::column_cluster_pays(rows, cols, low ? 2 : 4, false, aligned) &&
+      !(low && rows * cols > (24LL << 20)))
+    return low ? fb::launch_colsum(fb::PlainRows<__nv_bfloat16>{static_cast<const __nv_bfloat16*>(x)}, out, rows, cols,
+                                   accumulate, stream)
+               : fb::launch_colsum(fb::PlainRows<float>{static_cast<const float*>(x)}, out, rows, cols, accumulate, stream);
   if (!accumulate) {
     cudaError_t e = cudaMemsetAsync(out, 0, cols * sizeof(float), stream);
     if (e != cudaSuccess) return static_cast<int>(e);

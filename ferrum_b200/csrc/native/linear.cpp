@@ -88,17 +88,14 @@ struct LinearNode : Node {
     if (act != kNone) {  // only activations whose derivative is a function of the output are fused
       y = as2d(y);
       Tensor d = empty(g2.sizes(), g2, g2.scalar_type());
-      int rc = -3;
-      if (need_b && g2.numel() > 0) {  // with the bias' gradient, unless its sums want a launch of their own
+      const uintptr_t at = reinterpret_cast<uintptr_t>(g2.data_ptr()) | reinterpret_cast<uintptr_t>(y.data_ptr()) |
+                           reinterpret_cast<uintptr_t>(d.data_ptr());
+      // with the bias' gradient, unless its sums want a launch of their own
+      if (need_b && g2.numel() > 0 && fb_colsum_clusters(g2.size(0), g2.size(1), dt(g2), 1, at % 16 == 0)) {
         sums = empty({g2.size(1)}, g2, at::kFloat);
-        launch("fb_unary_bwd_colsum", [&] {
-          rc = fb_unary_bwd_colsum(g2.data_ptr(), y.data_ptr(), d.data_ptr(), sums.data_ptr<float>(), g2.size(0), g2.size(1), act,
-                                   dt(g2), cur_stream());
-          return rc == -3 ? 0 : rc;
-        });
-      }
-      if (rc == -3) {
-        sums = Tensor();
+        FB_CALL(fb_unary_bwd_colsum, g2.data_ptr(), y.data_ptr(), d.data_ptr(), sums.data_ptr<float>(), g2.size(0), g2.size(1),
+                act, dt(g2), cur_stream());
+      } else {
         FB_CALL(fb_unary_bwd, g2.data_ptr(), y.data_ptr(), d.data_ptr(), g2.numel(), act, 0.f, 0.f, dt(g2), cur_stream());
       }
       g2 = d;
