@@ -86,7 +86,7 @@ __device__ __forceinline__ void unpack16(const uint4& u, float (&v)[16 / sizeof(
 // The matrix as it is.
 template <typename T>
 struct PlainRows {
-  static constexpr int kV = 16 / sizeof(T), kU = 8;
+  static constexpr int kV = 16 / sizeof(T), kU = 8, kPerSm = 2;
   using Raw = uint4;
   const T* x;
   __host__ __device__ bool aligned() const { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; }
@@ -97,8 +97,11 @@ struct PlainRows {
 
 // A block sums L lanes x 16 bytes of columns over its rows, 512 / L of them at a time with Rows::kU loads each in flight: there
 // are hardly more blocks than SMs, so a block keeps 64 KB on their way (with 32 KB, 256 threads: 8192 x 1000 bf16 10.5 us).
+// Two blocks to an SM: a grid is up to twice the SMs, and with one of them at a time (90 registers for a gradient with four
+// loads of each operand) its second half took a turn of its own.  ReLU gradient and sums, bf16, us, two launches / one block /
+// two: 8192 x 2048 20.5 / 28.4 / 14.5, 16384 x 1024 21.0 / 27.1 / 21.8, 2048 x 2048 7.8 / 11.1 / 6.2.
 template <class Rows, int L>
-__global__ void __launch_bounds__(kColumnThreads)
+__global__ void __launch_bounds__(kColumnThreads, Rows::kPerSm)
 colsum_cluster_kernel(const Rows m, float* __restrict__ out, long long rows, long long cols, long long rows_per_block,
                       int accumulate) {
   constexpr int kV = Rows::kV, kU = Rows::kU, kR = kColumnThreads / L, kCols = L * kV;

@@ -190,7 +190,7 @@ __global__ void unary_bwd_f32(const float* __restrict__ dy, const float* __restr
 // sums those of the stored values.
 template <typename T, int OP>
 struct GradRows {
-  static constexpr int kV = 16 / sizeof(T), kU = 4;
+  static constexpr int kV = 16 / sizeof(T), kU = 2, kPerSm = 2;  // four loads of each operand: a block to an SM
   struct Raw {
     uint4 g, y;
   };
