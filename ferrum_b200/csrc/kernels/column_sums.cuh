@@ -1,8 +1,8 @@
 // Column sums of a matrix whose rows are divided among the blocks of a cluster (along y): every block's sums meet in the
-// first one through distributed shared memory, in the order of the blocks.  No atomics, so no result to clear first (a launch
-// and a gap of 3 us on the device, as much on the host where that is what bounds a step).  With a fill and atomics / so, us:
-// 128 x 256 bf16 5.9 / 3.0, 1024 x 1000 6.3 / 3.7, 8192 x 1000 10.3 / 7.8, 8192 x 1024 fp32 14.4 / 8.2; ReLU gradient and column
-// sums of 8192 x 4096 bf16 44 as three launches, 36 as one.
+// first one through distributed shared memory, in the order of the blocks.  No atomics, so no result to clear first: one launch
+// instead of two.  With a fill and atomics / so, us, one after another in a stream: 128 x 256 bf16 6.1 / 5.2 (as nodes of a graph
+// 6.0 / 3.4), 1024 x 1000 6.3 / 6.3 (6.3 / 4.2), 2048 x 4096 9.3 / 7.3, 8192 x 1024 fp32 out of memory 14.4 / 10.3; ReLU gradient
+// and column sums of 8192 x 4096 bf16 49 as three launches, 37 as one.
 #pragma once
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
@@ -96,7 +96,7 @@ struct PlainRows {
 };
 
 // A block sums L lanes x 16 bytes of columns over its rows, 512 / L of them at a time with Rows::kU loads each in flight: there
-// are hardly more blocks than SMs, so a block keeps 64 KB on their way (with 32 KB, 256 threads: 8192 x 1000 bf16 10.5 us).
+// are hardly more blocks than SMs, so a block of whole pieces keeps 64 KB on their way.
 // Two blocks to an SM: a grid is up to twice the SMs, and with one of them at a time (90 registers for a gradient with four
 // loads of each operand) its second half took a turn of its own.  ReLU gradient and sums, bf16, us, two launches / one block /
 // two: 8192 x 2048 20.5 / 28.4 / 14.5, 16384 x 1024 21.0 / 27.1 / 21.8, 2048 x 2048 7.8 / 11.1 / 6.2.
@@ -171,20 +171,34 @@ inline ColumnPlan column_plan(long long rows, long long cols, int v) {  // v: el
   while (p.split < 8 && p.ranges * p.split < column_sms() && rows >= p.split * 64) p.split *= 2;
   return p;
 }
-// Eight blocks to a column range: enough of them for the chip where there are many ranges, or little to read.  size: bytes of
-// an element; grad: behind an activation's gradient.
+// Whether one launch of clusters is faster than the sums in a cleared buffer (size: bytes of an element; grad: behind an
+// activation's gradient, then than a pass for each).  It saves a launch, or two; but a column range has eight blocks at most,
+// with fewer loads on their way than the four smaller ones to every SM there, so few blocks with much to read are slower.
+// us, otherwise / in one launch, one after another in a stream:
+//  - Never more than 4 MB in ranges of 32 bytes that leave SMs without a block.
+//  - Whole pieces: 96 KB to a block pay, and more where the ranges are wide (fp32 32768 x 1024 36 / 26, with a gradient bf16
+//    8192 x 2048 25.6 / 16.5).  Not where they are narrow (with a gradient bf16 32768 x 64 12.4 / 14.5, 32768 x 512 24.0 / 27.1,
+//    fp32 32768 x 160 18.5 / 22.6) nor for bf16 sums alone, which wait for instructions (16384 x 1024 8.3 / 12.4, 32768 x 512
+//    9.0 / 13.4), unless every SM has a block (8192 x 2048 out of memory 13.4 / 12.0).  Sums alone of up to 4 MB always
+//    (131072 x 8 fp32 12.4 / 10.4).
+//  - Single elements, 16 bytes apart in neighbouring lanes: a gradient to store repays its launches for one round of the
+//    block's threads (bf16 512 x 1001 12.4 / 10.4, 1024 x 1001 12.4 / 14.0, 8191 x 4095 with the products around it 265 / 399);
+//    sums alone for a few (fp32 16384 x 1 6.2 / 6.2, 32768 x 64 behind an odd address 8.0 / 13.1, bf16 8192 x 100 6.2 / 7.2), for
+//    eight times as many in wide ranges with a block to every SM (fp32 32768 x 1001 36 / 31, bf16 4096 x 4095 15.5 / 14.4).
 inline bool column_cluster_pays(long long rows, long long cols, int size, bool grad, bool aligned) {
   const int v = 16 / size;
-  const long long pieces = (cols + 2 * v - 1) / (2 * v);
-  if (pieces > 0x7fffffffLL) return false;
-  // Single loads of elements that lie 16 bytes apart in neighbouring lanes: with a gradient to store they repay the launches
-  // for one round of the block's threads (bf16, us, two launches / one: 512 x 1001 8.3 / 7.0, 1024 x 1001 12.3 / 14.2, 8191 x
-  // 4095 with the products around it 265 / 399).
-  if (grad && (cols % v != 0 || !aligned)) {
-    const ColumnPlan p = column_plan(rows, cols, v);
-    return (rows + p.split - 1) / p.split <= kColumnThreads / p.lanes;
+  const ColumnPlan p = column_plan(rows, cols, v);
+  const long long bytes = rows * cols * size, blocks = p.ranges * p.split, per_block = (bytes + blocks - 1) / blocks;
+  const long long narrow = (cols + 2 * v - 1) / (2 * v);  // ranges of 32 bytes
+  if (p.ranges > 0x7fffffffLL || (narrow * 8 < column_sms() && bytes > (4 << 20))) return false;
+  const bool full = blocks >= column_sms(), wide = p.lanes == 8;
+  if (cols % v != 0 || !aligned) {
+    const long long at_once = kColumnThreads / p.lanes, rounds = ((rows + p.split - 1) / p.split + at_once - 1) / at_once;
+    return rounds <= (grad ? 1 : (size == 4 ? 8 : 2) * (full && wide ? 8 : 1));
   }
-  return pieces * 8 >= column_sms() || rows * cols * size <= (4LL << 20);
+  if (per_block <= (96 << 10) || (!grad && bytes <= (4 << 20))) return true;
+  if (!grad && size == 2) return full && per_block <= (128 << 10);
+  return wide || (p.lanes == 4 && (full || size == 4));
 }
 template <class Rows>
 int launch_colsum(const Rows& m, float* out, long long rows, long long cols, int accumulate, cudaStream_t stream) {
