@@ -98,10 +98,11 @@ def test_scaled_products_of_other_ranks(lead_a, lead_b):
 
 
 @pytest.mark.parametrize("la", ["k", "rows", "odd"])
-@pytest.mark.parametrize("M,N,K", [(5, 4, 33), (130, 12, 64), (31, 68, 100), (128, 132, 257), (96, 1028, 1030)])
+@pytest.mark.parametrize("M,N,K", [(5, 4, 33), (130, 12, 64), (31, 68, 100), (128, 132, 257), (96, 1028, 1030),
+                                   (777, 1000, 333), (600, 1004, 520), (513, 904, 1030)])
 def test_rows_of_b_by_quads(la, M, N, K):
-    """B with its rows contiguous on 16-byte boundaries (read eight rows at a time) where the last eight are not whole, for each
-    way in which A reaches tensor memory; the operand ends where the last row of K does.  Bound as above."""
+    """B with its rows contiguous on 16-byte boundaries (read eight rows at a time) where the last eight are not whole or the
+    last tile has no more of them, for each way in which A reaches tensor memory; the operand ends where the last row of K does.  Bound as above."""
     from ferrum_b200.ops.gemm import gemm_f32
     from ferrum_b200.utils.runtime import check_status
 
