@@ -65,7 +65,6 @@ struct Args {
   int kb_total, kb_per_split, tiles_p;
   int stages, block_bytes, body_bytes, p_bytes;  // block: a k-block of both operands
   int mma_rows;  // 128, or 64 where P has no more
-  int boxes;     // kGroup k-blocks of an operand in one copy (3-D maps: 64 of K, rows, k-blocks), else a copy each
   int prefetch;  // bring this CTA's rows of B into L2 before the kernel ahead has completed
   int32_t* status;
   unsigned long long timeout_ns;
@@ -98,7 +97,10 @@ __device__ __forceinline__ void store_bf16(void* out, long long at, const float 
 
 // kSwap: P = B (rows are output columns), Q = A.  kGroup: k-blocks per stage.  One thread issues the MMAs, and a wait,
 // a commit and a loop around every four of them take it longer (400 cycles) than the MMAs of a narrow tile (160).
-template <int BN, bool kSwap, int kGroup>
+// kBoxes: the kGroup k-blocks of an operand arrive in one copy (3-D maps: 64 of K, rows, k-blocks), those of P, then those of Q;
+// else a copy or more for each.  Not a switch at run time: its test in the loops of the two issuing threads cost 35 ns per
+// k-block (64 x 64 x 65536 39.0 us, without it 34.5).
+template <int BN, bool kSwap, int kGroup, bool kBoxes>
 __global__ void __launch_bounds__(kThreads, 2)
 gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q,
                    const __grid_constant__ Args p) {
@@ -138,7 +140,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
   ptx::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   if (p.prefetch && warp == 2 && ptx::elect_one()) {
-    if (p.boxes) {
+    if constexpr (kBoxes) {
       for (int kb = kb_lo; kb < kb_hi; kb += kGroup) ptx::tma_prefetch_3d(kSwap ? &map_p : &map_q, 0, kSwap ? p0 : q0, kb);
     } else {
       for (int kb = kb_lo; kb < kb_hi; ++kb) ptx::tma_prefetch_2d(kSwap ? &map_p : &map_q, kb * kBK, kSwap ? p0 : q0);
@@ -157,17 +159,17 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
           ok = false;
           break;
         }
-        uint8_t* stage = smem + s * kGroup * p.block_bytes;  // the k-blocks of P, then those of Q
-        if (p.boxes) {  // k-blocks behind the last one arrive as zeros
+        if constexpr (kBoxes) {  // k-blocks behind the last one arrive as zeros
+          uint8_t* stage = smem + s * kGroup * p.block_bytes;
           ptx::mbar_arrive_expect_tx(&full_bar[s], kGroup * p.block_bytes);
           ptx::tma_load_3d(stage, &map_p, &full_bar[s], 0, p0, kb);
           ptx::tma_load_3d(stage + kGroup * p.p_bytes, &map_q, &full_bar[s], 0, q0, kb);
         }
-        const int blocks = p.boxes ? 0 : min(kGroup, kb_hi - kb);
-        if (blocks > 0) ptx::mbar_arrive_expect_tx(&full_bar[s], blocks * p.block_bytes);
+        const int blocks = kBoxes ? 0 : min(kGroup, kb_hi - kb);
+        if constexpr (!kBoxes) ptx::mbar_arrive_expect_tx(&full_bar[s], blocks * p.block_bytes);
         for (int i = 0; i < blocks; ++i) {
-          uint8_t* sp = stage + i * p.p_bytes;
-          uint8_t* sq = stage + kGroup * p.p_bytes + i * (p.block_bytes - p.p_bytes);
+          uint8_t* sp = smem + (s * kGroup + i) * p.block_bytes;
+          uint8_t* sq = sp + p.p_bytes;
           const int k0 = (kb + i) * kBK;
           if (p.p_mn) {
 #pragma unroll
@@ -203,7 +205,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
       const uint32_t p_lbo = p.p_mn ? kChunk : 16, q_lbo = p.q_mn ? kChunk : 16;
       const uint32_t p_step = p.p_mn ? 16 * 128 : 32, q_step = p.q_mn ? 16 * 128 : 32;
       const uint64_t p_first = ptx::make_smem_desc_sw128(ptx::smem_u32(smem), p_lbo, 1024);
-      const uint64_t q_first = ptx::make_smem_desc_sw128(ptx::smem_u32(smem) + kGroup * p.p_bytes, q_lbo, 1024);
+      const uint64_t q_first = ptx::make_smem_desc_sw128(ptx::smem_u32(smem) + (kBoxes ? kGroup : 1) * p.p_bytes, q_lbo, 1024);
       int s = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -215,9 +217,9 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_const
         }
         ptx::tc_fence_after();
         const auto block = [&](int i) {
-          const int at = s * kGroup * p.block_bytes;
-          const uint64_t dp = ptx::desc_advance(p_first, at + i * p.p_bytes);
-          const uint64_t dq = ptx::desc_advance(q_first, at + i * (p.block_bytes - p.p_bytes));
+          const int at = (s * kGroup + (kBoxes ? 0 : i)) * p.block_bytes;
+          const uint64_t dp = ptx::desc_advance(p_first, at + (kBoxes ? i * p.p_bytes : 0));
+          const uint64_t dq = ptx::desc_advance(q_first, at + (kBoxes ? i * (p.block_bytes - p.p_bytes) : 0));
 #pragma unroll
           for (int k = 0; k < kBK / 16; ++k)
             ptx::umma_f16(tmem, ptx::desc_advance(dp, k * p_step), ptx::desc_advance(dq, k * q_step), idesc,
@@ -418,13 +420,13 @@ int choose_splits(long long tiles, int kb_total) {
   return splits;
 }
 
-template <int BN, bool kSwap, int kGroup>
+template <int BN, bool kSwap, int kGroup, bool kBoxes = false>
 int launch(const CUtensorMap& mp, const CUtensorMap& mq, Args& g, int rows_p, int rows_q, int box_p, bool split,
            cudaStream_t st) {
   using C = Cfg<BN>;
   constexpr int kExtra = 1024 + 768;  // alignment, barriers
   static const cudaError_t configured = cudaFuncSetAttribute(
-      gemm_splitk_kernel<BN, kSwap, kGroup>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAlone + kExtra);
+      gemm_splitk_kernel<BN, kSwap, kGroup, kBoxes>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAlone + kExtra);
   if (configured != cudaSuccess) return static_cast<int>(configured);
   g.tiles_p = tiles_of(rows_p, kRowsP);
   const long long tiles = static_cast<long long>(g.tiles_p) * tiles_of(rows_q, BN);
@@ -457,7 +459,7 @@ int launch(const CUtensorMap& mp, const CUtensorMap& mq, Args& g, int rows_p, in
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = split ? 1 : 2;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, gemm_splitk_kernel<BN, kSwap, kGroup>, mp, mq, g));
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, gemm_splitk_kernel<BN, kSwap, kGroup, kBoxes>, mp, mq, g));
 }
 
 }  // namespace
@@ -497,8 +499,8 @@ int run(bool split, const void* a, const void* b, void* out, void* out2, const f
   const int group = tile == 160 ? (four ? 4 : 2) : tile == 192 && four ? 2 : 1;
   CUtensorMap ma, mb;
   Args g;
-  g.boxes = group > 1 && !a_mn_major && !b_mn_major && K % kBK == 0;
-  if (g.boxes) {
+  const bool boxes = group > 1 && !a_mn_major && !b_mn_major && K % kBK == 0;
+  if (boxes) {
     if (!make_map_blocks(&ma, a, M, K, lda, box_p, group) || !make_map_blocks(&mb, b, N, K, ldb, bn, group)) return -2;
   } else if (!make_map(&ma, a, M, K, lda, a_mn_major != 0, swap ? bn : box_p) ||
       !make_map(&mb, b, N, K, ldb, b_mn_major != 0, swap ? kRowsP : bn))
@@ -522,9 +524,13 @@ int run(bool split, const void* a, const void* b, void* out, void* out2, const f
     case 32: return launch<32, true, 1>(mb, ma, g, N, M, box_p, split, stream);
     case 64: return launch<64, true, 1>(mb, ma, g, N, M, box_p, split, stream);
     case 160:
+      if (boxes)
+        return four ? launch<32, false, 4, true>(ma, mb, g, M, N, box_p, split, stream)
+                    : launch<32, false, 2, true>(ma, mb, g, M, N, box_p, split, stream);
       return four ? launch<32, false, 4>(ma, mb, g, M, N, box_p, split, stream)
                   : launch<32, false, 2>(ma, mb, g, M, N, box_p, split, stream);
     case 192:
+      if (boxes) return launch<64, false, 2, true>(ma, mb, g, M, N, box_p, split, stream);
       return four ? launch<64, false, 2>(ma, mb, g, M, N, box_p, split, stream)
                   : launch<64, false, 1>(ma, mb, g, M, N, box_p, split, stream);
     default: return launch<128, false, 1>(ma, mb, g, M, N, box_p, split, stream);
