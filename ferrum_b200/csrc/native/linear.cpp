@@ -110,6 +110,7 @@ Tensor linear(const Tensor& x, const Tensor& weight, const c10::optional<Tensor>
               const c10::optional<Tensor>& w_low, py::object sink) {
   NoAutograd below;
   const Tensor bias = bias_.value_or(Tensor());
+  check_columns(weight, bias, weight.size(0), "the bias");
   Operands o = operands(x, weight, w_low.value_or(Tensor()), low);
   const int64_t N = weight.size(0);
   Tensor y = empty(out_sizes(x, N), o.x2, low ? at::kBFloat16 : at::kFloat);
@@ -192,6 +193,8 @@ Tensor layer_norm(const Tensor& x, const c10::optional<Tensor>& gamma_, const c1
   if (!norm_evaluates(pre)) return layer_norm(unary(x, pre, 0., 0.), gamma_, beta_, eps, kNone);
   NoAutograd below;
   const Tensor gamma = gamma_.value_or(Tensor()), beta = beta_.value_or(Tensor());
+  check_columns(x, gamma, x.size(-1), "the scale");
+  check_columns(x, beta, x.size(-1), "the shift");
   Tensor xc = contig(x);
   Tensor g = gamma.defined() ? contig(gamma) : gamma, b = beta.defined() ? contig(beta) : beta;
   Tensor y = empty(xc.sizes(), xc, xc.scalar_type());
@@ -332,6 +335,9 @@ Tensor linear_act_norm(const Tensor& x, const Tensor& weight, const c10::optiona
   if (!low && !norm_evaluates(act))
     return layer_norm(linear(x, weight, bias_, kNone, low, tf32, w_low, sink), gamma, beta, eps, act);
   const Tensor bias = bias_.value_or(Tensor());
+  check_columns(weight, bias, weight.size(0), "the bias");
+  check_columns(weight, gamma, weight.size(0), "the scale");
+  check_columns(weight, beta, weight.size(0), "the shift");
   Operands o;
   {
     NoAutograd below;

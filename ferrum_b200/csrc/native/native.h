@@ -73,6 +73,12 @@ inline Tensor f32c(const Tensor& t) { return contig(is_f32(t) ? t : cast(t, at::
 inline void check_on(const Tensor& input, const Tensor& t, const char* what) {
   TORCH_CHECK_VALUE(t.device() == input.device(), what, " is on ", t.device(), ", the input on ", input.device());
 }
+// A bias or a scale: a value for each of the n columns.
+inline void check_columns(const Tensor& input, const Tensor& t, int64_t n, const char* what) {
+  if (!t.defined()) return;
+  check_on(input, t, what);
+  TORCH_CHECK_VALUE(t.numel() == n, what, " has ", t.numel(), " values, expected ", n);
+}
 inline Tensor as2d(const Tensor& t) { return t.dim() == 2 ? t : t.reshape({-1, t.size(-1)}); }
 
 // ------------------------------------------------------------------------------------------------ autograd

@@ -80,3 +80,17 @@ def test_products_that_no_kernel_has():
                                 (f, f, f, 6, False)):
         with pytest.raises(RuntimeError, match="gemm"):
             _native().gemm_nt(a, b, None, act, out, acc, False)
+
+
+def test_biases_and_scales():
+    """A bias or a scale on another device than the weight, or of another size, in the three ops that read one by a pointer."""
+    x, w, ok = torch.zeros(4, 6), torch.zeros(5, 6), torch.zeros(5)
+    for bad, what in ((torch.zeros(5, device="meta"), "on meta"), (torch.zeros(4), "expected 5"), (torch.zeros(6), "expected 5")):
+        with pytest.raises(ValueError, match=what):
+            _native().linear(x, w, bad, 0, False, False, None, None)
+        for args in ((bad, ok, ok), (ok, bad, ok), (ok, ok, bad)):
+            with pytest.raises(ValueError, match=what):
+                _native().linear_act_norm(x, w, *args, 1e-5, 0, False, False, None, None)
+        for args in ((bad, ok), (ok, bad), (None, bad)):
+            with pytest.raises(ValueError, match=what):
+                _native().layer_norm(torch.zeros(4, 5), *args, 1e-5, 0)
