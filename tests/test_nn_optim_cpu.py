@@ -343,3 +343,26 @@ def test_causal_attention_ignores_later_positions():
     y, y2, z, z2 = (t.torch() if hasattr(t, "torch") else t for t in (y, y2, z, z2))
     assert float((y[:, :4] - y2[:, :4]).abs().max()) == 0.0
     assert float((z[:, :4] - z2[:, :4]).abs().max()) > 0.0
+
+
+@pytest.mark.parametrize("name", ["weight", "bias"])
+def test_layers_use_the_weights_that_their_attributes_give(name):
+    """An attribute of the instance, a property of a subclass and a parametrization come before the table of parameters."""
+    x = torch.randn(3, 4)
+    for make in (lambda: nn.Linear(4, 4), lambda: nn.LayerNorm([4])):
+        plain = make()
+        want = make()
+        want.load_state_dict(plain.state_dict())
+        with torch.no_grad():
+            getattr(want, name).mul_(2.0).add_(1.0)
+        changed = getattr(want, name).detach()
+
+        instance, below, parametrized = (make() for _ in range(3))
+        for m in (instance, below, parametrized):
+            m.load_state_dict(plain.state_dict())
+        instance.__dict__[name] = changed
+        below.__class__ = type("Below", (type(below),), {name: property(lambda m: changed)})
+        double = type("Double", (torch.nn.Module,), {"forward": lambda m, t: 2.0 * t + 1.0})()
+        torch.nn.utils.parametrize.register_parametrization(parametrized, name, double)
+        for m in (instance, below, parametrized):
+            assert torch.allclose(m(x), want(x), atol=1e-6) and not torch.allclose(m(x), plain(x), atol=1e-3)
