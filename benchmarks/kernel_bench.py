@@ -110,13 +110,17 @@ def _cases(small: bool):
     idx = torch.from_numpy(zipf_indices(V, 1.1, Bt * S, seed=0)).to(dev).reshape(Bt, S)
     case("embedding_meanpool_fwd", lambda: F.embedding_mean_pool(w, idx, bf), Bt * S * D * 4, "K10 gather+pool")
     gout = torch.randn(Bt, D, device=dev).to(bf)
-    keys = torch.empty(Bt * S, device=dev, dtype=torch.int32)  # 32-bit sort keys, as the backward pass makes them
-    lib.fb_embedding_keys(idx.data_ptr(), keys.data_ptr(), Bt * S, V, st())
+    keys, rows = (torch.empty(Bt * S, device=dev, dtype=torch.int32) for _ in range(2))  # as the backward pass makes them
+    lib.fb_embedding_pairs(idx.data_ptr(), keys.data_ptr(), rows.data_ptr(), Bt * S, V, S, st())
     sidx, perm = torch.sort(keys, stable=True)
-    dw = torch.zeros(V, D, device=dev)
-    case("embedding_scatter_add_bwd",
-         lambda: lib.fb_embedding_bwd_sorted(gout.data_ptr(), sidx.data_ptr(), 4, perm.data_ptr(), dw.data_ptr(),
-                                             Bt * S, D, S, 1.0 / S, -1, V, 3, st()), Bt * S * D * 2, "K10 bwd")
+    rows, dw = rows[perm], torch.empty(V, D, device=dev)
+
+    def scatter():  # with the clearing that it relies on
+        dw.zero_()
+        lib.fb_embedding_bwd_pairs_zeroed(gout.data_ptr(), sidx.data_ptr(), rows.data_ptr(), dw.data_ptr(), Bt * S, D, S,
+                                          1.0 / S, -1, V, 3, st())
+
+    case("embedding_scatter_add_bwd", scatter, Bt * S * D * 2 + V * D * 4, "K10 bwd")
     gi = torch.randint(0, R, (R,), device=dev)
     case("gather_rows_f32", lambda: F.gather_rows(x32, gi), n * 8, "K18 collate")
 

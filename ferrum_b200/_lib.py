@@ -175,8 +175,7 @@ _CUDA_SIGS = {
     "fb_dropout_bwd": (I, [P, P, P, LL, F, I, P]),
     "fb_embedding_fwd": (I, [P, P, P, LL, I, LL, LL, I, P, P]),
     "fb_embedding_meanpool_fwd": (I, [P, P, P, LL, I, I, LL, I, P]),
-    "fb_embedding_bwd_sorted": (I, [P, P, I, P, P, LL, I, I, F, LL, LL, I, P]),
-    "fb_embedding_keys": (I, [P, P, LL, LL, P]),
+    "fb_embedding_bwd_sorted": (I, [P, P, P, P, LL, I, I, F, LL, LL, I, P]),
     "fb_embedding_pairs": (I, [P, P, P, LL, LL, LL, P]),
     "fb_embedding_bwd_pairs": (I, [P, P, P, P, LL, I, I, F, LL, LL, I, P]),
     "fb_embedding_bwd_pairs_zeroed": (I, [P, P, P, P, LL, I, I, F, LL, LL, I, P]),

@@ -236,7 +236,8 @@ int fb_embedding_fwd(const float* weight, const long long* idx, void* out, long 
 // Mean over `seq` consecutive indices: out[b] = mean_s W[idx[b, s]].
 int fb_embedding_meanpool_fwd(const float* weight, const long long* idx, void* out, long long batch, int seq,
                               int dim, long long vocab, int out_dtype, cudaStream_t stream);
-// dW[idx[i]] += scale * dout[i / group] ; `sorted_idx/perm` come from a radix sort of idx.
+// dW[idx[i]] += scale * dout[i / group].  Pairs of an index (vocab where it is no row of the table) and its row of dout, i / group,
+// sorted by index:
 int fb_embedding_pairs(const long long* idx, int32_t* keys, int32_t* rows, long long n, long long vocab, long long group,
                        cudaStream_t stream);
 int fb_embedding_bwd_pairs(const void* dout, const int32_t* keys, const int32_t* rows, float* dweight, long long n_idx,
@@ -246,10 +247,10 @@ int fb_embedding_bwd_pairs(const void* dout, const int32_t* keys, const int32_t*
 int fb_embedding_bwd_pairs_zeroed(const void* dout, const int32_t* keys, const int32_t* rows, float* dweight, long long n_idx,
                                   int dim, int group, float scale, long long padding_idx, long long vocab, int dtype,
                                   cudaStream_t stream);
-int fb_embedding_keys(const long long* idx, int32_t* keys, long long n, long long vocab, cudaStream_t stream);
-int fb_embedding_bwd_sorted(const void* dout, const void* sorted_idx, int key_bytes, const long long* perm,
-                            float* dweight, long long n_idx, int dim, int group, float scale, long long padding_idx,
-                            long long vocab, int dtype, cudaStream_t stream);
+// The same for sorted indices of 64 bits and their original positions.
+int fb_embedding_bwd_sorted(const void* dout, const long long* sorted_idx, const long long* perm, float* dweight, long long n_idx,
+                            int dim, int group, float scale, long long padding_idx, long long vocab, int dtype,
+                            cudaStream_t stream);
 // Blockwise attention forward (tcgen05, head dimension 64, bf16): out[B, Sq, H, 64] = softmax(scale q k^T) v for
 // [B, H, S, 64] views given by element strides; lse (optional) [B, H, Sq].  -2: operand not describable by TMA.
 int fb_attention_fwd(const void* q, const void* k, const void* v, void* out, float* lse, int B, int H, int Sq, int Skv,

@@ -246,15 +246,15 @@ __global__ void embedding_meanpool_kernel(const float* __restrict__ w, const lon
 }
 
 // Row numbers as 32-bit sort keys: half the bytes and half the passes of a radix sort of the 64-bit indices.  Indices
-// outside the table (reported by the forward pass) become `vocab`, which the scatter drops.  rows (optional): the row of
-// the gradient that position i adds, i / group.
+// outside the table (reported by the forward pass) become `vocab`, which the scatter drops.  rows: the row of the gradient
+// that position i adds, i / group.
 __global__ void embedding_keys_kernel(const long long* __restrict__ idx, int32_t* __restrict__ keys,
                                       int32_t* __restrict__ rows, long long n, long long vocab, long long group) {
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
     const long long id = __ldg(idx + i);
     keys[i] = static_cast<int32_t>(id < 0 || id > vocab ? vocab : id);
-    if (rows != nullptr) rows[i] = static_cast<int32_t>(i / group);
+    rows[i] = static_cast<int32_t>(i / group);
   }
 }
 
@@ -723,10 +723,6 @@ extern "C" int fb_embedding_pairs(const long long* idx, int32_t* keys, int32_t* 
   embedding_keys_kernel<<<static_cast<int>(want < cap ? want : cap), 256, 0, stream>>>(idx, keys, rows, n, vocab, group);
   return static_cast<int>(cudaGetLastError());
 }
-extern "C" int fb_embedding_keys(const long long* idx, int32_t* keys, long long n, long long vocab, cudaStream_t stream) {
-  if (n <= 0) return 0;
-  return fb_embedding_pairs(idx, keys, nullptr, n, vocab, n, stream);
-}
 
 namespace {
 template <bool kZeroed, typename Key, typename At>
@@ -748,17 +744,12 @@ int embedding_bwd(const void* dout, const void* sorted_idx, const void* at, floa
 }
 }  // namespace
 
-// sorted_idx: 32-bit (key_bytes = 4) or 64-bit (8) row numbers; perm: their original positions.
-extern "C" int fb_embedding_bwd_sorted(const void* dout, const void* sorted_idx, int key_bytes, const long long* perm,
-                                       float* dweight, long long n_idx, int dim, int group, float scale,
-                                       long long padding_idx, long long vocab, int dtype, cudaStream_t stream) {
-  if (key_bytes == 4)
-    return embedding_bwd<false, int32_t, long long>(dout, sorted_idx, perm, dweight, n_idx, dim, group, scale, padding_idx, vocab,
-                                             dtype, stream);
-  if (key_bytes == 8)
-    return embedding_bwd<false, long long, long long>(dout, sorted_idx, perm, dweight, n_idx, dim, group, scale, padding_idx, vocab,
-                                               dtype, stream);
-  return n_idx <= 0 || dim <= 0 ? 0 : -1;
+// Sorted row numbers of 64 bits (tables that pairs do not reach); perm: their original positions.
+extern "C" int fb_embedding_bwd_sorted(const void* dout, const long long* sorted_idx, const long long* perm, float* dweight,
+                                       long long n_idx, int dim, int group, float scale, long long padding_idx,
+                                       long long vocab, int dtype, cudaStream_t stream) {
+  return embedding_bwd<false, long long, long long>(dout, sorted_idx, perm, dweight, n_idx, dim, group, scale, padding_idx, vocab,
+                                                    dtype, stream);
 }
 // The same for pairs of fb_embedding_pairs, sorted by key: rows are rows of dout, `group` of the indices to each.
 extern "C" int fb_embedding_bwd_pairs(const void* dout, const int32_t* keys, const int32_t* rows, float* dweight,

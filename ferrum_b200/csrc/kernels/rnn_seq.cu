@@ -668,7 +668,8 @@ int run(bool backward, const SeqArgs& a, const Plan& p, cudaStream_t st) {
   if constexpr (BS <= 4) {
     if (p.reg) return run_one<G, BS, true>(backward, a, p, st);
   }
-  return run_one<G, BS, false>(backward, a, p, st);
+  if constexpr (BS == 3) return -1;  // plan() has three rows with the weights in registers alone
+  else return run_one<G, BS, false>(backward, a, p, st);
 }
 template <int G>
 int run_bs(bool backward, const SeqArgs& a, const Plan& p, cudaStream_t st) {

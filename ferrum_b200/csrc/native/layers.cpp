@@ -48,7 +48,7 @@ struct EmbeddingNode : Node {
     }
     const float scale = 1.f / static_cast<float>(group);
     if (!pairs)
-      FB_CALL(fb_embedding_bwd_sorted, g2.data_ptr(), sorted.data_ptr(), 8,
+      FB_CALL(fb_embedding_bwd_sorted, g2.data_ptr(), reinterpret_cast<const ll*>(sorted.data_ptr<int64_t>()),
               reinterpret_cast<const ll*>(perm.data_ptr<int64_t>()), dw.data_ptr<float>(), n, static_cast<int>(dim),
               static_cast<int>(group), scale, padding, vocab, dt(g2), cur_stream());
     else if (n > 0) {

@@ -19,8 +19,8 @@ def test_gradient(vocab, n, dim, padding):
     dout = torch.randn(n, dim, device="cuda", generator=g)
     lib, st = _lib.cuda(), torch.cuda.current_stream().cuda_stream
     for ids in (idx, bad):
-        keys = torch.empty(n, dtype=torch.int32, device="cuda")
-        _lib.check(lib.fb_embedding_keys(ids.data_ptr(), keys.data_ptr(), n, vocab, st), "fb_embedding_keys")
+        keys, rows = (torch.empty(n, dtype=torch.int32, device="cuda") for _ in range(2))
+        _lib.check(lib.fb_embedding_pairs(ids.data_ptr(), keys.data_ptr(), rows.data_ptr(), n, vocab, 1, st), "fb_embedding_pairs")
         ok = (ids >= 0) & (ids < vocab)
         assert torch.equal(keys.long(), torch.where(ok, ids, vocab))
         ok_grad = ok & (ids != padding)
@@ -30,9 +30,10 @@ def test_gradient(vocab, n, dim, padding):
         for unsorted in (keys, torch.where(ok, ids, vocab)):  # 64 bits: tables of 2^31 - 1 rows and more
             key, perm = torch.sort(unsorted, stable=True)
             dw = torch.zeros(vocab, dim, device="cuda")
-            _lib.check(lib.fb_embedding_bwd_sorted(dout.data_ptr(), key.data_ptr(), key.element_size(), perm.data_ptr(),
-                                                   dw.data_ptr(), n, dim, 1, 1.0, padding, vocab, 0, st),
-                       "fb_embedding_bwd_sorted")
+            pairs = key.dtype == torch.int32
+            scatter, at = (lib.fb_embedding_bwd_pairs, rows[perm]) if pairs else (lib.fb_embedding_bwd_sorted, perm)
+            _lib.check(scatter(dout.data_ptr(), key.data_ptr(), at.data_ptr(), dw.data_ptr(), n, dim, 1, 1.0, padding, vocab, 0,
+                               st), "scatter")
             check_status()
             assert ((dw - want).abs() <= 2.0 ** -22 * size * 8).all()
 
