@@ -133,6 +133,7 @@ _CUDA_SIGS = {
     "fb_conv_pack_filters": (I, [P, P] + [I] * 10 + [P]),
     "fb_conv_fold_wgrad": (I, [P, P] + [I] * 10 + [P]),
     "fb_s2d_nhwc_to_nchw_f32": (I, [P, P] + [I] * 12 + [LL, P]),
+    "fb_s2d_nhwc_to_nchw_add": (I, [P, P, P] + [I] * 12 + [LL, P]),
     "fb_nhwc_to_nchw_f32": (I, [P, P, P, I, I, LL, LL, I, P]),
     "fb_attention_bwd_map_error": (I, []),
     "fb_col2im": (I, [P, P] + [I] * 14 + [LL, P]),

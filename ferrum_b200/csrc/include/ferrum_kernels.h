@@ -270,27 +270,32 @@ int fb_attention_bwd_map_error(void);
 int fb_conv_igemm(const void* x, const void* w, void* y, const float* bias, int B, int H, int W, int Cp, int O, int kh,
                   int kw, int ph, int pw, int dh, int dw, long long ldy, int out_bf16, int32_t* status,
                   cudaStream_t stream);
+// With an activation, a mask (bf16, laid out like y: results count where it is above zero) or an fp32 y that is added to.
+int fb_conv_igemm_epilogue(const void* x, const void* w, void* y, const float* bias, const void* mask, int B, int H, int W,
+                           int Cp, int O, int kh, int kw, int ph, int pw, int dh, int dw, long long ldy, int out_bf16, int act,
+                           int beta, int32_t* status, cudaStream_t stream);
 int fb_conv_wgrad_splits(int B, int Ho, int Wo, int O, int Cp, int taps);
 int fb_conv_wgrad(const void* dy, const void* x, float* out, int B, int H, int W, int Cp, int O, int Op, int kh, int kw,
                   int ph, int pw, int dh, int dw, int32_t* status, cudaStream_t stream);
 // A convolution of any stride becomes one of stride 1 by a space-to-depth arrangement (conv_layout.cu).
-int fb_conv_pack_masked(const float* x, const unsigned char* mask, void* z, int B, int C, int H, int W, long long ld,
-                        cudaStream_t stream);
-int fb_nhwc_to_nchw_masks(const float* x, const float* add, const unsigned char* add_mask, float* y, unsigned char* mask, int B,
-                          int C, long long P, long long ld, int relu, cudaStream_t stream);
-int fb_conv_igemm_epilogue(const void* x, const void* w, void* y, const float* bias, const void* mask, int B, int H, int W,
-                           int Cp, int O, int kh, int kw, int ph, int pw, int dh, int dw, long long ldy, int out_bf16, int act,
-                           int beta, int32_t* status, cudaStream_t stream);
 int fb_conv_pack_input(const float* x, const float* mask, void* z, int B, int C, int H, int W, int sh, int sw, int eh,
                        int ew, int ph, int pw, int Hz, int Wz, long long ld, cudaStream_t stream);
+// The same of a gradient behind a ReLU whose mask is bytes (fb_nhwc_to_nchw_masks); stride 1, no padding.
+int fb_conv_pack_masked(const float* x, const unsigned char* mask, void* z, int B, int C, int H, int W, long long ld,
+                        cudaStream_t stream);
 int fb_conv_pack_filters(const float* w, void* out, int O, int C, int kh, int kw, int sh, int sw, int eh, int ew, int pitch,
                          int dgrad, cudaStream_t stream);
 int fb_conv_fold_wgrad(const float* part, float* dw, int splits, int O, int C, int kh, int kw, int sh, int sw, int eh,
                        int ew, int pitch, cudaStream_t stream);
 int fb_s2d_nhwc_to_nchw_f32(const float* z, float* x, int B, int C, int H, int W, int sh, int sw, int eh, int ew, int ph,
                             int pw, int Hz, int Wz, long long ld, cudaStream_t stream);
+int fb_s2d_nhwc_to_nchw_add(const float* z, const float* add, float* x, int B, int C, int H, int W, int sh, int sw, int eh, int ew,
+                            int ph, int pw, int Hz, int Wz, long long ld, cudaStream_t stream);
 int fb_nhwc_to_nchw_f32(const float* x, const float* add, float* y, int B, int C, long long P, long long ld, int relu,
                         cudaStream_t stream);
+// add counts where add_mask is set; mask is set where y is above zero (both optional, bytes).
+int fb_nhwc_to_nchw_masks(const float* x, const float* add, const unsigned char* add_mask, float* y, unsigned char* mask, int B,
+                          int C, long long P, long long ld, int relu, cudaStream_t stream);
 int fb_gather_rows(const void* src, const long long* idx, void* dst, long long n_idx, long long row_bytes,
                    long long n_rows, int32_t* status, cudaStream_t stream);
 

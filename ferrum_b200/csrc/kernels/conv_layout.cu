@@ -217,7 +217,7 @@ fold_wgrad_kernel(const float* __restrict__ part, float* __restrict__ dw, const 
 }
 
 __global__ void __launch_bounds__(256)
-s2d_to_nchw_kernel(const float* __restrict__ z, float* __restrict__ x, const S2d g) {
+s2d_to_nchw_kernel(const float* __restrict__ z, const float* __restrict__ add, float* __restrict__ x, const S2d g) {
   __shared__ float tile[32][33];
   const long long bi = blockIdx.x;
   const long long b = bi / g.H;
@@ -237,11 +237,20 @@ s2d_to_nchw_kernel(const float* __restrict__ z, float* __restrict__ x, const S2d
     tile[ty + 8 * k][tx] = v;
   }
   __syncthreads();
-  float* xr = x + (b * g.C * g.H + i) * static_cast<long long>(g.W);
+  const long long row = (b * g.C * g.H + i) * static_cast<long long>(g.W);
+  float r[4] = {0.f, 0.f, 0.f, 0.f};
+  if (add != nullptr) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int c = c0 + ty + 8 * k, j = j0 + tx;
+      if (c < g.C && j < g.W) r[k] = __ldg(add + row + static_cast<long long>(c) * g.H * g.W + j);
+    }
+  }
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int c = c0 + ty + 8 * k, j = j0 + tx;
-    if (c < g.C && j < g.W) xr[static_cast<long long>(c) * g.H * g.W + j] = tile[tx][ty + 8 * k];
+    const float v = tile[tx][ty + 8 * k];
+    if (c < g.C && j < g.W) x[row + static_cast<long long>(c) * g.H * g.W + j] = add != nullptr ? v + r[k] : v;
   }
 }
 
@@ -430,14 +439,18 @@ extern "C" int fb_conv_fold_wgrad(const float* part, float* dw, int splits, int 
 }
 
 // x[b, c, i, j] = z[b, (i + ph) / sh, (j + pw) / sw, (((i + ph) % sh) * ew + (j + pw) % sw) * C + c], zero where no
-// window reaches.
-extern "C" int fb_s2d_nhwc_to_nchw_f32(const float* z, float* x, int B, int C, int H, int W, int sh, int sw, int eh,
-                                       int ew, int ph, int pw, int Hz, int Wz, long long ld, cudaStream_t stream) {
+// window reaches; plus add (optional, laid out like x).
+extern "C" int fb_s2d_nhwc_to_nchw_add(const float* z, const float* add, float* x, int B, int C, int H, int W, int sh, int sw,
+                                       int eh, int ew, int ph, int pw, int Hz, int Wz, long long ld, cudaStream_t stream) {
   const fb::S2d g{C, H, W, sh, sw, eh, ew, ph, pw, Hz, Wz, ld};
   if (!fb::s2d_ok(B, g) || !fb::s2d_grid_ok(B, g)) return -1;
   dim3 grid(static_cast<unsigned>(B) * H, static_cast<unsigned>((W + 31) / 32), static_cast<unsigned>((C + 31) / 32));
-  fb::s2d_to_nchw_kernel<<<grid, 256, 0, stream>>>(z, x, g);
+  fb::s2d_to_nchw_kernel<<<grid, 256, 0, stream>>>(z, add, x, g);
   return static_cast<int>(cudaGetLastError());
+}
+extern "C" int fb_s2d_nhwc_to_nchw_f32(const float* z, float* x, int B, int C, int H, int W, int sh, int sw, int eh,
+                                       int ew, int ph, int pw, int Hz, int Wz, long long ld, cudaStream_t stream) {
+  return fb_s2d_nhwc_to_nchw_add(z, nullptr, x, B, C, H, W, sh, sw, eh, ew, ph, pw, Hz, Wz, ld, stream);
 }
 
 // y [B, C, P] = x [B, P, ld] (first C channels), plus add [B, C, P] (optional), behind a ReLU with relu = 1.

@@ -73,13 +73,13 @@ Tensor input_product(const Tensor& gh, const Tensor& w, const Shape& s, const Te
           cur_stream());
   return dz;
 }
-// That of x, plus add (stride 1; add_mask: where that is set).
+// That of x, plus add (add_mask: where that is set; stride 1).
 Tensor input_grad(const Tensor& gh, const Tensor& w, const Shape& s, const Tensor& add = Tensor(), const Tensor& add_mask = Tensor()) {
   Tensor dz = input_product(gh, w, s), dx = empty({s.B, s.C, s.H, s.W}, gh, at::kFloat);
   const int rows = s.eh * s.ew * s.C;
   if (s.strided)
-    FB_CALL(fb_s2d_nhwc_to_nchw_f32, dz.data_ptr<float>(), dx.data_ptr<float>(), s.B, s.C, s.H, s.W, s.sh, s.sw, s.eh, s.ew, s.ph,
-            s.pw, s.Hz, s.Wz, rows, cur_stream());
+    FB_CALL(fb_s2d_nhwc_to_nchw_add, dz.data_ptr<float>(), fptr(add), dx.data_ptr<float>(), s.B, s.C, s.H, s.W, s.sh, s.sw, s.eh,
+            s.ew, s.ph, s.pw, s.Hz, s.Wz, rows, cur_stream());
   else
     FB_CALL(fb_nhwc_to_nchw_masks, dz.data_ptr<float>(), fptr(add), static_cast<const unsigned char*>(ptr(add_mask)),
             dx.data_ptr<float>(), nullptr, s.B, s.C, static_cast<ll>(s.H) * s.W, rows, 0, cur_stream());
@@ -220,7 +220,7 @@ struct BlockNode : Node {
       if (need_1) out[1] = filter_grad(g1, z1, s1);
       if (need_x) dx = down ? input_grad(g1, w1, s1) : input_grad(g1, w1, s1, dy, mask);
     }
-    if (need_x && down) dx = sd.strided ? input_grad(gh, wd, sd).add_(dx) : input_grad(gh, wd, sd, dx);
+    if (need_x && down) dx = input_grad(gh, wd, sd, dx);
     out[0] = dx;
     return out;
   }
