@@ -1633,8 +1633,9 @@ extern "C" int fb_add_layernorm_fwd(const float* x, const void* r, const float* 
 extern "C" int fb_add_layernorm_bwd(const float* dy, const float* sum, const float* gamma, const float* mean,
                                     const float* rstd, float* dx, void* dx_low, float* partial, float* stats,
                                     long long rows, int cols, int nblk, cudaStream_t stream) {
-  if (rows <= 0 || cols <= 0) return 0;
+  if (cols <= 0) return 0;
   if (stats == nullptr) return -1;
+  if (rows <= 0) return static_cast<int>(cudaMemsetAsync(stats, 0, 3 * static_cast<size_t>(cols) * sizeof(float), stream));
   return bwd_t<float>(dy, sum, nullptr, gamma, mean, rstd, dx, static_cast<__nv_bfloat16*>(dx_low), partial, stats, rows,
                       cols, FB_ACT_NONE, nblk, 2, stream);
 }

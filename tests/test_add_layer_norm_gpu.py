@@ -48,3 +48,16 @@ def test_values_that_are_not_finite(r_dtype):
     for a, b in zip(*got):
         assert torch.equal(torch.isnan(a).any(1).nonzero().flatten().cpu(), torch.tensor([1, 4, 6]))
         assert torch.equal(torch.nan_to_num(a), torch.nan_to_num(b))
+
+
+def test_no_rows_have_empty_sums():
+    from ferrum_b200 import _lib
+
+    lib, st = _lib.cuda(), torch.cuda.current_stream().cuda_stream
+    for added in (False, True):
+        stats = torch.full((3, 24), float("nan"), device="cuda")
+        if added:
+            rc = lib.fb_add_layernorm_bwd(None, None, None, None, None, None, None, None, stats.data_ptr(), 0, 24, 1, st)
+        else:
+            rc = lib.fb_layernorm_bwd(None, None, None, None, None, None, None, None, stats.data_ptr(), 0, 24, 0, 0, 1, 2, st)
+        assert rc == 0 and not stats.any()
