@@ -15,6 +15,7 @@ import math
 
 import torch
 
+from .. import config
 from ..core import ShapeMismatch, _as_device
 from ..ops import functional as F
 from .modules import Module, _param, tensor_io
@@ -121,6 +122,8 @@ def conv_fused(conv, x, add=None, act=None):
 
 def block_fused(conv1, conv2, down, x):
     """``relu(conv2(relu(conv1(x))) + (down(x) or x))`` as one node where all of it runs as implicit GEMMs, else None."""
+    if not (F._native(x) and config.low_precision_active()):  # first: all that follows takes 10 us of the host
+        return None
     convs = [conv1, conv2] + ([down] if down is not None else [])
     if not (all(bare(c) and c.bias is None and c.groups == 1 for c in convs) and x.dim() == 4 and x.dtype == torch.float32):
         return None
