@@ -122,9 +122,9 @@ def _own(m, cls):
     """``m.weight`` and ``m.bias`` of a layer of class ``cls``, straight from its table of parameters, where a module's attribute
     is looked up last: unless an attribute of the instance or of a subclass (a parametrization) comes before it."""
     d = m.__dict__
-    if type(m) is cls and "weight" not in d and "bias" not in d:
-        own = d["_parameters"]
+    if m.__class__ is cls and "weight" not in d and "bias" not in d:
         try:
+            own = d["_parameters"]
             return own["weight"], own["bias"]
         except KeyError:  # a buffer
             pass
