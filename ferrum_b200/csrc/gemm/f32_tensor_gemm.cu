@@ -37,8 +37,10 @@
 // on their way before barriers and tensor memory are set up, tiles without splits meet without a cluster barrier, and the
 // partial sums are asked for several at a time.  us before all this and now: 1024 x 1024 x 64 8.8 / 6.2, 1024^3 21.1 / 19.2, 2048^3
 // 114 / 104, 591 x 1536 x 384 15.4 / 13.0, 128 x 256 x 784 8.8 / 7.6, 1 x 256 x 784 7.6 / 6.6.  Large products run into the
-// power limit: 8192 x 4096 x 4096 1549 / 1482 by itself, 1547 / 1606 in an unbroken row of twelve; a training step of three
-// layers of 4096 over 8192 rows 14.7 / 13.9 ms.
+// power limit.  8192 x 4096 x 4096, forward, input gradient and weight gradient: 1549 / 1482 by itself; in rows of sixty at the
+// limit, the two sides taking turns, 1820 / 1756, 1983 / 1726 and 1905 / 1940 (whoever comes first on a cool chip is 5 % faster);
+// a training step of three layers of 4096 over 8192 rows 14.7 / 13.9 ms.  Seventeen warps leave 96 registers: with A's rows
+// contiguous (weight gradients) tiles of 128 spill 36 - 40 bytes, 20 - 28 before.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

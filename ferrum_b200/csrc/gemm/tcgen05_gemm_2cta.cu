@@ -35,7 +35,7 @@
 // some 600 cycles or more.  Picked the new way in the MMA warp alone: large products 10 % faster, small ones up to 2 us
 // slower; in both warps, us before and after: 512 x 512 x 4096 25.8 / 17.6, 512 x 4096 x 1024 11.3 / 8.8, 8192 x 1024 x
 // 1024 18.7 / 16.2, 8192 x 2048 x 2048 53 / 48, 8192 x 4096 x 4096 183 - 190 / 169, weight gradient 4096 x 4096 x 8192
-// 208 - 232 / 204.
+// 208 - 232 / 204 (194 with the last round in halves: launch2).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
